@@ -149,3 +149,25 @@ def test_seeded_contract_determinism_and_distribution(cuda):
     assert np.abs(freq - prob).max() < 0.02, (freq, prob)   # Gumbel-max samples the softmax
     ids3, _, _ = run(cuda, x, [1.0] * B, [O.sampler_row_seed(1235, i, 3) for i in range(B)])
     assert (ids3 != ids1).mean() > 0.3
+
+
+@pytest.mark.parametrize("V", [1000, 20001, 70000, 151936])   # 20001: rows off 16 bytes
+def test_short_cuts_select_what_the_radix_selection_selects(cuda, V):
+    """Logits and temperature times 2^24 give the same scaled values to the bit, but lie beyond the range of temperatures that the
+    candidate and linear-bin short cuts take: survivors and tokens have to be identical."""
+    rng = np.random.default_rng(V)
+    combos = [(k, p) for k in (0, 1, 50, 255, 256, 257) for p in (0.0, 0.1, 0.9, 0.999)]
+    B = len(combos)
+    x = (rng.standard_normal((B, V)) * 3).astype(np.float32)
+    x[::3] = np.round(x[::3] * 4) / 4           # tie groups at both cuts
+    x[1::6] = np.sort(x[1::6], -1)              # the largest values in one place
+    x[4, : V // 2] = -np.inf
+    x[5, 3] = np.nan                            # left to the radix selection
+    x[7] = 0.5
+    temps = (0.4 + 0.1 * np.arange(B)).astype(np.float32)
+    ks, ps = [k for k, _ in combos], [p for _, p in combos]
+    seeds = seeds_for(B, 21)
+    a = run(cuda, x, temps, seeds, top_k=ks, top_p=ps)
+    b = run(cuda, x * np.float32(2 ** 24), temps * np.float32(2 ** 24), seeds, top_k=ks, top_p=ps)
+    for got, want in zip(a, b):
+        assert (got == want).all()
