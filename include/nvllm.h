@@ -529,8 +529,10 @@ int nvllm_window_attention(void* out, int64_t ldo, const void* q, int64_t ldq, c
                            const int32_t* cu_tokens, int32_t n_seqs, int32_t dtype, void* stream);
 /* nvllm_latent_attention with a sliding window (window > 0: keys p - window + 1 .. p), sinks (f32 [heads], nullable, as
  * above) and a gate per head (f32 [n, heads], ldg apart, nullable: out[t, h, :] *= sigmoid(gate[t, h])).
- * workspace (nullable, f32): with it, single tokens in a long window (1000 keys and more) whose CTAs would not fill the SMs
- * split their key tiles over up to 4 CTAs; needs n * heads * 4 * (kv_rank + 2) * 4 bytes for n <= 256 (larger batches never split). */
+ * workspace (nullable, f32): with it, up to 256 tokens whose CTAs would not fill the SMs split their key tiles over several
+ * CTAs: over up to 4 in a long window (1000 keys and more; n * heads * 4 * (kv_rank + 2) * 4 bytes), without a window over as many
+ * as the workspace holds (nvllm_latent_workspace_bytes: enough for every split the kernel would choose; 0: none). */
+size_t nvllm_latent_workspace_bytes(int32_t n, int32_t heads, int32_t kv_rank);
 int nvllm_latent_window_attention(void* out, int64_t ldo, const float* q_abs, int64_t ldqa, const void* q, int64_t ldq,
                                   const int32_t* tok_seq, const int64_t* positions, const int32_t* block_tables,
                                   int32_t table_cap, int32_t block_size, const void* cache, int64_t cache_row, int32_t n,

@@ -120,6 +120,7 @@ PROTOTYPES = {
     "nvllm_ff_activation_params": (i32, [vp, vp, i32, i32, i32, vp, i32, vp]),
     "nvllm_embedding_stream": (i32, [vp, vp, i32, vp, vp, i32, i32, i32, f32, i32, vp]),
     "nvllm_moe_route_logits": (i32, [vp, vp, vp, i64, vp, i32, i32, i32, vp]),
+    "nvllm_latent_workspace_bytes": (sz, [i32, i32, i32]),
     "nvllm_latent_window_attention": (i32, [vp, i64, vp, i64, vp, i64, vp, vp, vp, i32, i32, vp, i64, i32, i32, i32, i32, i32, f32, i32,
                                             vp, vp, i64, vp, sz, i32, vp]),
     "nvllm_delta_prepare": (i32, [vp, i64, vp, i64, vp, i64, vp, i64, vp, vp, i32, i32, i32, i32, f32, f32, vp]),

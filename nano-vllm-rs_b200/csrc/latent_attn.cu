@@ -15,9 +15,11 @@
 // Options of the attention (nvllm_latent_window_attention): a sliding window (position p sees p - window + 1 .. p), a sink
 // per head whose exponential joins the softmax denominator, and a gate per head (out *= sigmoid(gate)); the rotated part
 // may be absent (rot_dim = 0).
+#include <algorithm>
 #include <cmath>
 
 #include "common.cuh"
+#include "latent_attn.cuh"
 
 namespace nvllm {
 namespace {
@@ -223,19 +225,9 @@ __global__ void __launch_bounds__(128) latent_prepare_kernel(const PrepArgs a) {
   }
 }
 
-struct AttnArgs {
-  void* out; int64_t ldo;           // [n, heads, kv_rank]
-  const float* q_abs; int64_t ldqa;  // [n, heads, kv_rank] f32
-  const void* q; int64_t ldq;        // [n, heads, dim + rot_dim]: only the rotated part is read
-  const int32_t* tok_seq; const int64_t* positions;
-  const int32_t* tables; int table_cap, block_size;
-  const void* cache; int64_t cache_row;
-  int n, heads, dim, rot_dim, kv_rank;
-  float scale;
-  int window; const float* sinks; const float* gate; int64_t ldg;   // 0 / null: none
-  int splits; float* part;   // splits > 1: CTAs along z share a token's key tiles; partial (acc[kv_rank], m, l) per (token, head, split)
-};
+using AttnArgs = LatentAttnArgs;
 
+constexpr int kMaxLatentSplits = 32;
 constexpr int kKeyTile = 32;
 
 // CTA = one query token x up to 8 heads (one warp per head).  Key tiles of 32 cache rows are staged once in shared memory
@@ -369,7 +361,15 @@ __global__ void __launch_bounds__(kMmaThreads) latent_attn_mma_kernel(const Attn
       for (int e = tid; e < (16 - heads_here) * pad0; e += kMmaThreads)
         Qs[(q * 16 + heads_here + e / pad0) * DPS + e % pad0] = __float2bfloat16_rn(0.f);
   }
-  const int tfirst = blockIdx.x * TQ;
+  if (a.skip_dense) {   // usually every tile of the batch is dense: nothing to do
+    int left = 0;
+    for (int t = tid; t * kLatentTileTokens < a.n; t += kMmaThreads) left |= !latent_tile_dense(a.tok_seq, a.n, t);
+    if (!__syncthreads_or(left)) return;
+  }
+  const int items = (a.n + TQ - 1) / TQ;
+  for (int item = blockIdx.x; item < items; item += gridDim.x) {
+  const int tfirst = item * TQ;
+  if (a.skip_dense && latent_tile_dense(a.tok_seq, a.n, tfirst / kLatentTileTokens)) continue;
   bool together = false;
   if (TQ == 2 && tfirst + 1 < a.n) together = a.tok_seq[tfirst] == a.tok_seq[tfirst + 1];
   const int npass = (TQ == 1 || together || tfirst + 1 >= a.n) ? 1 : 2;
@@ -627,6 +627,7 @@ __global__ void __launch_bounds__(kMmaThreads) latent_attn_mma_kernel(const Attn
       }
     }
   }
+  }
 }
 
 // One warp per (token, head): merges the splits' partial softmaxes, adds the sink to the denominator, applies the gate.
@@ -635,6 +636,7 @@ __global__ void __launch_bounds__(128) latent_attn_merge_kernel(const AttnArgs a
   const int64_t item = static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5);
   if (item >= static_cast<int64_t>(a.n) * a.heads) return;
   const int64_t t = item / a.heads;
+  if (a.skip_dense && latent_tile_dense(a.tok_seq, a.n, static_cast<int>(t / kLatentTileTokens))) return;
   const int h = static_cast<int>(item - t * a.heads), W = a.kv_rank + 2;
   const float* pr = a.part + item * a.splits * W;
   float mx = a.sinks ? a.sinks[h] : -INFINITY;
@@ -664,7 +666,9 @@ int launch_attn_mma_tq(const AttnArgs& a, cudaStream_t st) {
   const size_t smem = static_cast<size_t>(TQ * 16 + 2 * kMmaKeys) * DPS * 2 + TQ * 16 * kPsStride * 2 +
                       (TQ * 2 * 16 * kSsStride + TQ * 48) * 4;
   NVLLM_SMEM_ATTR_ONCE((latent_attn_mma_kernel<NT2, TQ>), 225 * 1024);
-  dim3 grid((a.n + TQ - 1) / TQ, (a.heads + 15) / 16, TQ == 1 && a.splits > 1 ? a.splits : 1);
+  const int items = (a.n + TQ - 1) / TQ, groups = (a.heads + 15) / 16;
+  // behind the tcgen05 kernel a launch with nothing to do should cost little: no more CTAs than run at once
+  dim3 grid(a.skip_dense ? std::min(items, std::max(1, sm_count() / groups)) : items, groups, TQ == 1 && a.splits > 1 ? a.splits : 1);
   latent_attn_mma_kernel<NT2, TQ><<<grid, kMmaThreads, smem, st>>>(a, DPS, DP16);
   NVLLM_LAUNCH_CHECK("latent_attn_mma_kernel");
   if (TQ == 1 && a.splits > 1) {
@@ -814,6 +818,12 @@ extern "C" int nvllm_latent_attention(void* out, int64_t ldo, const float* q_abs
                                        cache_row, n, heads, dim, rot_dim, kv_rank, scale, 0, nullptr, nullptr, 0, nullptr, 0, dtype, stream);
 }
 
+extern "C" size_t nvllm_latent_workspace_bytes(int32_t n, int32_t heads, int32_t kv_rank) {
+  if (n <= 0 || n > 256 || heads <= 0 || kv_rank <= 0) return 0;
+  const int splits = std::min(kMaxLatentSplits, sm_count() / (n * ((heads + 15) / 16)));
+  return splits > 1 ? static_cast<size_t>(n) * heads * splits * (kv_rank + 2) * sizeof(float) : 0;
+}
+
 extern "C" int nvllm_latent_window_attention(void* out, int64_t ldo, const float* q_abs, int64_t ldqa, const void* q, int64_t ldq,
                                              const int32_t* tok_seq, const int64_t* positions, const int32_t* block_tables,
                                              int32_t table_cap, int32_t block_size, const void* cache, int64_t cache_row, int32_t n,
@@ -826,24 +836,29 @@ extern "C" int nvllm_latent_window_attention(void* out, int64_t ldo, const float
   if (n == 0) return 0;
   NVLLM_CHECK_ARG(out && q_abs && (q || rot_dim == 0) && tok_seq && positions && block_tables && cache, NVLLM_ERR_ARG, "latent_attention: NULL");
   const AttnArgs a{out, ldo, q_abs, ldqa, q ? q : q_abs, ldq, tok_seq, positions, block_tables, table_cap, block_size, cache, cache_row,
-                   n, heads, dim, rot_dim, kv_rank, scale, window > 0 ? window : 0, sinks, gate, ldg, 1, static_cast<float*>(workspace)};
+                   n, heads, dim, rot_dim, kv_rank, scale, window > 0 ? window : 0, sinks, gate, ldg, 1, static_cast<float*>(workspace), 0};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // bf16 caches with a 16-byte row pitch and kv_rank <= 512 run on the tensor cores (NVLLM_LATENT_MMA=0: the CUDA-core kernel)
   const int dp16 = (static_cast<int>(cache_row) + 15) / 16 * 16;
   if (dtype == NVLLM_BF16 && knobs().latent_mma != 0 && kv_rank <= 512 && cache_row % 8 == 0 && dp16 <= 704 &&
       (reinterpret_cast<uintptr_t>(cache) & 15u) == 0) {
-    // Single tokens with a bounded key range (a window) and fewer CTAs than SMs: split every token's key tiles over up to 4
-    // CTAs, as many as fill the SMs once and leave each at least eight tiles; the partials meet in latent_attn_merge_kernel.
-    // (Measured, 64 tokens x 16 heads, rank 512: a window of 2048 keys 118 -> 79 us; at 512 keys the second launch costs what
-    // the shorter loop saves, 39 -> 37 us, so short windows stay on one CTA.)
     AttnArgs b = a;
-    if (workspace != nullptr && n <= 256 && window > 0) {
+    if (knobs().latent_mma == 1 && latent_attn_tc_applies(a)) {
+      if (int rc = latent_attn_tc_launch(a, st)) return rc;
+      b.skip_dense = 1;   // single tokens (tiles of many sequences) are left to the kernel below
+    }
+    // Single tokens on fewer CTAs than SMs: the key tiles of a token are split over CTAs along z, as many as fill the SMs once and
+    // leave each (at the longest context the tables or the window allow) at least four tiles; the partials meet in
+    // latent_attn_merge_kernel.  Measured, 32 tokens x 16 heads at 4001 keys, rank 512: 223 -> 104 us.  64 tokens in a window of 2048 keys 118 -> 79 us; in one of 512 the second launch costs what the shorter loop saves (39 -> 37 us), hence eight
+    // tiles for windows.
+    if (workspace != nullptr && n <= 256) {
       const int64_t ctas = static_cast<int64_t>(n) * ((heads + 15) / 16);
+      const int64_t reach = window > 0 ? window + kMmaKeys - 1 : static_cast<int64_t>(table_cap) * block_size;
+      const int tiles = static_cast<int>(std::min<int64_t>((reach + kMmaKeys - 1) / kMmaKeys, 1 << 20));
       int splits = static_cast<int>(sm_count() / (ctas > 0 ? ctas : 1));
-      const int tiles = (window + 2 * kMmaKeys - 2) / kMmaKeys;   // tiles a window can touch
-      splits = splits > 4 ? 4 : splits;
-      splits = splits > tiles / 8 ? tiles / 8 : splits;
-      if (splits > 1 && static_cast<size_t>(n) * heads * splits * (kv_rank + 2) * sizeof(float) <= workspace_bytes) b.splits = splits;
+      splits = std::min(splits, window > 0 ? std::min(4, tiles / 8) : std::min(kMaxLatentSplits, tiles / 4));
+      splits = static_cast<int>(std::min<size_t>(splits, workspace_bytes / (static_cast<size_t>(n) * heads * (kv_rank + 2) * sizeof(float))));
+      if (splits > 1) b.splits = splits;
     }
     if (kv_rank <= 128) return launch_attn_mma<1>(b, st);
     if (kv_rank <= 256) return launch_attn_mma<2>(b, st);

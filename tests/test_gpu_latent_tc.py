@@ -1,0 +1,78 @@
+"""Latent attention of prompts and portions on tcgen05 (kv_rank 512), the split of single tokens' keys, and what falls to the
+mma.sync kernel beside them, against the attention in 64 bits."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from tests.arch_util import paged
+
+RANK = 512
+
+
+def reference(q_abs, q_rot, cache, spans, pos, tables, bs, heads, rot, scale, window, sinks, gate):
+    out = torch.empty(q_abs.shape[0], heads, RANK, dtype=torch.float64, device=q_abs.device)
+    for s, (a, b) in enumerate(spans):
+        L = int(pos[a:b].max()) + 1
+        j = torch.arange(L, device=q_abs.device)
+        rows = cache[(tables[s].long()[j // bs] * bs + j % bs)].double()
+        x = torch.cat([q_abs[a:b].to(torch.bfloat16).double().reshape(b - a, heads, RANK), q_rot[a:b].double()], -1)
+        sc = x @ rows[:, :RANK + rot].T * scale
+        hidden = j[None] > pos[a:b, None]
+        if window:
+            hidden |= j[None] <= pos[a:b, None] - window
+        sc = sc.masked_fill(hidden[:, None], -math.inf)
+        if sinks is not None:
+            sc = torch.cat([sc, sinks.double()[None, :, None].expand(b - a, heads, 1)], -1)
+        p = torch.softmax(sc, -1)[..., :L]
+        o = p @ rows[:, :RANK]
+        out[a:b] = o if gate is None else o * torch.sigmoid(gate[a:b].double())[..., None]
+    return out.reshape(q_abs.shape[0], -1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,rot,bs,window,extras,portions", [
+    (16, 64, 16, 0, False, [(0, 64), (0, 1), (130, 9), (3, 70)]),      # prompts, a single token, portions behind cached keys
+    (16, 64, 256, 0, False, [(0, 8), (0, 8), (0, 8), (0, 8)]),         # every tile one sequence
+    (32, 8, 48, 100, True, [(0, 63), (500, 65), (63, 1), (64, 2)]),    # two head groups, a window, sinks and a gate
+    (16, 0, 16, 33, True, [(0, 129), (0, 127)]),                       # no rotated part
+    (16, 64, 64, 0, False, [(k * 17, 1) for k in range(40)]),          # single tokens alone: no dense tile
+    (16, 64, 64, 0, False, [(40, 1), (0, 100), (700, 1), (5, 1), (9, 1), (2, 1), (1000, 30)]),
+    (16, 64, 256, 0, False, [(1500, 1), (700, 1), (0, 1)]),            # few single tokens: their keys are split over CTAs
+])
+def test_latent_prompts_portions_and_single_tokens(cuda, heads, rot, bs, window, extras, portions):
+    from nano_vllm_rs_b200 import _ffi, ops
+    rng = np.random.default_rng(len(portions) + heads + rot)
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    randn = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    dim, row = 24, RANK + rot
+    ctx = [c + n for c, n in portions]
+    tables, _, nslots = paged(rng, ctx, bs)
+    cache = randn(nslots, row).to(torch.bfloat16)
+    counts = [n for _, n in portions]
+    N = sum(counts)
+    starts = np.concatenate([[0], np.cumsum(counts)])
+    spans = [(int(starts[i]), int(starts[i + 1])) for i in range(len(counts))]
+    pos = torch.cat([torch.arange(c, c + n) for c, n in portions]).cuda()
+    tok_seq = torch.repeat_interleave(torch.arange(len(counts)), torch.tensor(counts)).to(torch.int32).cuda()
+    tabs = torch.from_numpy(tables).cuda()
+    q_abs = randn(N, heads * RANK) * 0.5
+    q = randn(N, heads, dim + rot).to(torch.bfloat16)
+    scale = 0.11
+    sinks = randn(heads) if extras else None
+    gate = randn(N, heads) if extras else None
+    if extras:
+        got = out = torch.empty((N, heads * RANK), dtype=torch.bfloat16, device="cuda")
+        p = lambda t: t.data_ptr()
+        _ffi.check(_ffi.lib().nvllm_latent_window_attention(p(out), out.stride(0), p(q_abs), q_abs.stride(0), p(q), q.stride(0), p(tok_seq), p(pos), p(tabs),
+                                                            tabs.shape[1], bs, p(cache), cache.stride(0), N, heads, dim, rot, RANK, scale, window,
+                                                            p(sinks), p(gate), heads, None, 0, 0, torch.cuda.current_stream().cuda_stream))
+    else:
+        got = ops.latent_attention(q_abs, q.reshape(N, -1), tok_seq, pos, tabs, bs, cache, heads, dim, rot, RANK, scale)
+    ref = reference(q_abs, q[..., dim:], cache, spans, pos, tabs, bs, heads, rot, scale, window, sinks, gate)
+    # bf16 probabilities (2^-9 each) against exact ones, and a bf16 output (2^-9): per value of O(1)
+    err = (got.double() - ref).abs()
+    assert torch.isfinite(got.float()).all()
+    assert float((err / (ref.abs() + 0.25 * ref.pow(2).mean().sqrt())).max()) < 0.06, float(err.max())
+    assert float(err.norm() / ref.norm()) < 6e-3
