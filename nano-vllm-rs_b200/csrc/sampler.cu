@@ -454,13 +454,13 @@ __device__ bool select_mass_linear(Shared& sh, const float* __restrict__ row, in
   return true;
 }
 
-// u of the seeded contract (sampler.rs:211-212 clamps it) as Gumbel noise
-__device__ __forceinline__ float gumbel(uint64_t seed, uint32_t i) {
+// u of the seeded contract, and the Gumbel noise it stands for
+__device__ __forceinline__ float uniform(uint64_t seed, uint32_t i) {
   const uint64_t h = mix64(seed + static_cast<uint64_t>(i + 1) * kGolden);
   const float u = (static_cast<float>(h >> 41) + 0.5f) * 1.1920928955078125e-07f;  // 2^-23; in (0, 1)
-  const float uc = fminf(fmaxf(u, 1e-8f), 1.0f - 1e-8f);
-  return -logf(-logf(uc));
+  return fminf(fmaxf(u, 1e-8f), 1.0f - 1e-8f);                                     // sampler.rs:211-212
 }
+__device__ __forceinline__ float gumbel_of(float u) { return -logf(-logf(u)); }
 
 __device__ float block_max(Shared& sh, float v) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -528,7 +528,7 @@ sample_kernel(int64_t* __restrict__ out_ids, const float* __restrict__ logits, i
       int bidx = 0x7fffffff;
       for (int j = tid; j < r; j += kThreads) {
         const uint32_t i = static_cast<uint32_t>(sh.hist[j]);
-        const float score = okey_inv(candidate_key(sh.hist[j])) + gumbel(row_seeds[b], i);
+        const float score = okey_inv(candidate_key(sh.hist[j])) + gumbel_of(uniform(row_seeds[b], i));
         if (kept_mask != nullptr) kept_mask[static_cast<int64_t>(b) * V + i] = 1;
         if (score > best || (score == best && static_cast<int>(i) < bidx)) { best = score; bidx = static_cast<int>(i); }
       }
@@ -586,28 +586,48 @@ sample_kernel(int64_t* __restrict__ out_ids, const float* __restrict__ logits, i
   const uint64_t seed = greedy ? 0ull : row_seeds[b];
   float best = -INFINITY;
   int bidx = 0x7fffffff, kept = 0;
-  for_each4(row, V, [&](const float (&v)[4], int i0, int n) {
+  if (kept_mask == nullptr && kept_count == nullptr) {
+    // g = -log(w), w = -log(u) >= 1 - u:  the value cannot win where 1 - u > exp(s - best), which costs one fast exponential of an
+    // approximate quotient instead of a division and two logarithms (1 % is far beyond the approximations' error; 1e4 bounds
+    // the rounding of s + g against it).
+    const float inv_t = 1.0f / T;
+    for_each4_free(row, V, 1, [&](const float (&v)[4], int i0, int n) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      if (e < n) {
-        const int i = i0 + e;
-        float score;
-        bool keep = true;
-        if (greedy) {
-          score = v[e];
-        } else {
-          const float s = scaled(v[e], T);
-          const uint32_t key = okey(s);
-          keep = keeps(sk, key, static_cast<uint32_t>(i)) && keeps(sp, key, static_cast<uint32_t>(i));
-          score = -INFINITY;
-          if (keep) score = s + gumbel(seed, static_cast<uint32_t>(i));  // the noise is only needed for survivors
+      for (int e = 0; e < 4; ++e)
+        if (e < n) {
+          const int i = i0 + e;
+          float score = v[e];
+          if (!greedy) {
+            const float near = v[e] * inv_t, u = uniform(seed, static_cast<uint32_t>(i));
+            if (fabsf(near) < 1e4f && 1.0f - u > 1.01f * __expf(near - best)) continue;
+            const float s = scaled(v[e], T);
+            const uint32_t key = okey(s);
+            if (!keeps(sk, key, static_cast<uint32_t>(i)) || !keeps(sp, key, static_cast<uint32_t>(i))) continue;
+            score = s + gumbel_of(u);
+          }
+          if (score > best || (score == best && i < bidx)) { best = score; bidx = i; }
         }
-        if (kept_mask != nullptr) kept_mask[static_cast<int64_t>(b) * V + i] = keep ? 1 : 0;
-        kept += keep ? 1 : 0;
-        if (score > best || (score == best && i < bidx)) { best = score; bidx = i; }
-      }
-    }
-  });
+    });
+  } else {
+    for_each4_free(row, V, 1, [&](const float (&v)[4], int i0, int n) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (e < n) {
+          const int i = i0 + e;
+          float score = v[e];
+          bool keep = true;
+          if (!greedy) {
+            const float s = scaled(v[e], T);
+            const uint32_t key = okey(s);
+            keep = keeps(sk, key, static_cast<uint32_t>(i)) && keeps(sp, key, static_cast<uint32_t>(i));
+            score = keep ? s + gumbel_of(uniform(seed, static_cast<uint32_t>(i))) : -INFINITY;
+          }
+          if (kept_mask != nullptr) kept_mask[static_cast<int64_t>(b) * V + i] = keep ? 1 : 0;
+          kept += keep ? 1 : 0;
+          if (score > best || (score == best && i < bidx)) { best = score; bidx = i; }
+        }
+    });
+  }
   finish_row(sh, best, bidx, kept, out_ids + b, kept_count != nullptr ? kept_count + b : nullptr);
 }
 
