@@ -31,8 +31,9 @@
 namespace nvllm {
 namespace {
 
-constexpr int kThreads = 512;   // two CTAs (rows) per SM
-constexpr int kWarps = kThreads / 32;
+// A row per CTA: 1024 threads while every row has an SM to itself (148 rows x 151936 without filters: 82 us, with 512 threads 91;
+// 32768 values 24 against 41), two CTAs of 512 on an SM beyond that (256 rows x 151936: 140 us).
+constexpr int kMaxThreads = 1024;
 constexpr int kBins = 4096;  // three selection passes over 8 + 12 + 12 key bits (see radix_select)
 constexpr uint64_t kGolden = 0x9E3779B97F4A7C15ull;
 constexpr unsigned kFull = 0xffffffffu;
@@ -75,7 +76,7 @@ struct Shared {
   unsigned long long need, eq;
   float redf[32];
   int redi[32];
-  uint32_t cnt[kWarps];
+  uint32_t cnt[kMaxThreads / 32];
   int sel_bin;
   uint32_t cut;
   int ncand, odd;
@@ -90,14 +91,14 @@ __device__ __forceinline__ void for_each4(const float* __restrict__ row, int V, 
   if ((reinterpret_cast<uintptr_t>(row) & 15u) == 0) {
     const int nvec = V >> 2;
     const float4* r4 = reinterpret_cast<const float4*>(row);
-    for (int base = 0; base < nvec; base += 2 * kThreads) {
-      const int j0 = base + tid, j1 = j0 + kThreads;
+    for (int base = 0; base < nvec; base += 2 * static_cast<int>(blockDim.x)) {
+      const int j0 = base + tid, j1 = j0 + static_cast<int>(blockDim.x);
       float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0;
       if (j0 < nvec) q0 = __ldg(r4 + j0);
       if (j1 < nvec) q1 = __ldg(r4 + j1);
       const float v0[4] = {q0.x, q0.y, q0.z, q0.w}, v1[4] = {q1.x, q1.y, q1.z, q1.w};
       f(v0, 4 * j0, j0 < nvec ? 4 : 0);
-      if (base + kThreads < nvec) f(v1, 4 * j1, j1 < nvec ? 4 : 0);  // block-uniform condition
+      if (base + static_cast<int>(blockDim.x) < nvec) f(v1, 4 * j1, j1 < nvec ? 4 : 0);  // block-uniform condition
     }
     const int t0 = nvec << 2;
     if (t0 < V) {  // V % 4 trailing elements: thread 0 takes them, everybody makes the call
@@ -107,7 +108,7 @@ __device__ __forceinline__ void for_each4(const float* __restrict__ row, int V, 
       f(v, t0, n);
     }
   } else {
-    for (int base = 0; base < V; base += kThreads) {
+    for (int base = 0; base < V; base += static_cast<int>(blockDim.x)) {
       const int i = base + tid;
       float v[4] = {0.f, 0.f, 0.f, 0.f};
       if (i < V) v[0] = row[i];
@@ -136,7 +137,7 @@ __device__ void radix_select(Shared& sh, const float* __restrict__ row, int V, f
     // update costs ~ the number of DISTINCT bins in a warp (a handful at this width); later passes see few candidates.
     const int shift = pass == 0 ? 24 : (pass == 1 ? 12 : 0);
     const int nbins = pass == 0 ? 256 : 4096;
-    for (int b = tid; b < nbins; b += kThreads) sh.hist[b] = 0ull;
+    for (int b = tid; b < nbins; b += static_cast<int>(blockDim.x)) sh.hist[b] = 0ull;
     __syncthreads();
     for_each4(row, V, [&](const float (&v)[4], int i0, int n) {
 #pragma unroll
@@ -208,7 +209,7 @@ __device__ void radix_select(Shared& sh, const float* __restrict__ row, int V, f
 template <typename PF>
 __device__ uint32_t ordered_cut(Shared& sh, int V, PF pred, uint32_t need) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int chunk = ((V + kWarps - 1) / kWarps + 31) & ~31;
+  const int chunk = ((V + static_cast<int>(blockDim.x >> 5) - 1) / static_cast<int>(blockDim.x >> 5) + 31) & ~31;
   const int start = warp * chunk, end = min(V, start + chunk);
   uint32_t cnt = 0;
   for (int base = start; base < end; base += 32) {
@@ -220,7 +221,7 @@ __device__ uint32_t ordered_cut(Shared& sh, int V, PF pred, uint32_t need) {
   __syncthreads();
   uint32_t run = 0;
   int wsel = -1;
-  for (int w = 0; w < kWarps; ++w) {
+  for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) {
     if (wsel < 0) {
       if (run + sh.cnt[w] >= need) wsel = w; else run += sh.cnt[w];
     }
@@ -251,11 +252,11 @@ __device__ void sort_candidates(Shared& sh, int n) {
   const int tid = threadIdx.x;
   int n2 = 2;
   while (n2 < n) n2 <<= 1;
-  for (int i = n + tid; i < n2; i += kThreads) sh.hist[i] = ~0ull;
+  for (int i = n + tid; i < n2; i += static_cast<int>(blockDim.x)) sh.hist[i] = ~0ull;
   __syncthreads();
   for (int size = 2; size <= n2; size <<= 1)
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int i = tid; i < n2 / 2; i += kThreads) {
+      for (int i = tid; i < n2 / 2; i += static_cast<int>(blockDim.x)) {
         const int lo = 2 * i - (i & (stride - 1)), hi = lo + stride;
         const bool up = (lo & size) == 0;
         const unsigned long long x = sh.hist[lo], y = sh.hist[hi];
@@ -307,7 +308,7 @@ __device__ int mass_position(Shared& sh, int n, float m, unsigned long long need
 }
 
 // Visits the row like for_each4 with four loads in flight per thread; f(v, i0, n) may be called different numbers of times by
-// different threads.  Blocks of 4 kThreads values; every `step`-th block is visited (1: all of them).
+// different threads.  Blocks of 4 static_cast<int>(blockDim.x) values; every `step`-th block is visited (1: all of them).
 template <typename F>
 __device__ __forceinline__ void for_each4_free(const float* __restrict__ row, int V, int step, F f) {
   const int tid = threadIdx.x;
@@ -315,7 +316,7 @@ __device__ __forceinline__ void for_each4_free(const float* __restrict__ row, in
     const int nvec = V >> 2;
     const float4* r4 = reinterpret_cast<const float4*>(row);
     int j = tid;
-    const int hop = step * kThreads;
+    const int hop = step * static_cast<int>(blockDim.x);
     for (; j + 3 * hop < nvec; j += 4 * hop) {
       float4 q[4];
 #pragma unroll
@@ -327,7 +328,7 @@ __device__ __forceinline__ void for_each4_free(const float* __restrict__ row, in
     const int t0 = nvec << 2;
     if (step == 1 && t0 + tid < V) { const float v[4] = {row[t0 + tid], 0.f, 0.f, 0.f}; f(v, t0 + tid, 1); }
   } else {
-    for (int i = tid; i < V; i += step * kThreads) { const float v[4] = {row[i], 0.f, 0.f, 0.f}; f(v, i, 1); }
+    for (int i = tid; i < V; i += step * static_cast<int>(blockDim.x)) { const float v[4] = {row[i], 0.f, 0.f, 0.f}; f(v, i, 1); }
   }
 }
 
@@ -381,7 +382,7 @@ __device__ int rank_top_k(Shared& sh, const float* __restrict__ row, int V, floa
 __device__ bool select_mass_linear(Shared& sh, const float* __restrict__ row, int V, float T, double p, float m, Sel& sp) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (!(T >= 9.5e-7f && T <= 1.05e6f) || !(fabsf(m) <= 1e30f)) return false;
-  for (int b = tid; b < kBins; b += kThreads) sh.hist[b] = 0ull;
+  for (int b = tid; b < kBins; b += static_cast<int>(blockDim.x)) sh.hist[b] = 0ull;
   if (tid == 0) { sh.ncand = 0; sh.odd = 0; }
   __syncthreads();
   // a mass is zero once the value lies 32 ln 2 = 22.18 below the maximum; equal values share a bin, larger ones are in lower bins
@@ -468,7 +469,7 @@ __device__ float block_max(Shared& sh, float v) {
   if (lane == 0) sh.redf[warp] = v;
   __syncthreads();
   float r = sh.redf[0];
-  for (int w = 1; w < kWarps; ++w) r = fmaxf(r, sh.redf[w]);
+  for (int w = 1; w < static_cast<int>(blockDim.x >> 5); ++w) r = fmaxf(r, sh.redf[w]);
   __syncthreads();
   return r;
 }
@@ -487,7 +488,7 @@ __device__ void finish_row(Shared& sh, float best, int bidx, int kept, int64_t* 
   __syncthreads();
   if (tid == 0) {
     int total = 0;
-    for (int w = 0; w < kWarps; ++w) {
+    for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) {
       total += static_cast<int>(sh.cnt[w]);
       if (sh.redf[w] > best || (sh.redf[w] == best && sh.redi[w] < bidx)) { best = sh.redf[w]; bidx = sh.redi[w]; }
     }
@@ -496,7 +497,8 @@ __device__ void finish_row(Shared& sh, float best, int bidx, int kept, int64_t* 
   }
 }
 
-__global__ void __launch_bounds__(kThreads, 2)
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, kMaxThreads / THREADS)
 sample_kernel(int64_t* __restrict__ out_ids, const float* __restrict__ logits, int V, int64_t ld,
               const float* __restrict__ temperatures, const int32_t* __restrict__ top_k, const float* __restrict__ top_p,
               const uint64_t* __restrict__ row_seeds, int32_t* __restrict__ kept_count, uint8_t* __restrict__ kept_mask) {
@@ -521,12 +523,12 @@ sample_kernel(int64_t* __restrict__ out_ids, const float* __restrict__ logits, i
       int r = k;
       if (do_p) r = mass_position(sh, k, okey_inv(candidate_key(sh.hist[0])), 0ull, true, static_cast<double>(p)) + 1;
       if (kept_mask != nullptr) {
-        for (int i = tid; i < V; i += kThreads) kept_mask[static_cast<int64_t>(b) * V + i] = 0;
+        for (int i = tid; i < V; i += static_cast<int>(blockDim.x)) kept_mask[static_cast<int64_t>(b) * V + i] = 0;
         __syncthreads();
       }
       float best = -INFINITY;
       int bidx = 0x7fffffff;
-      for (int j = tid; j < r; j += kThreads) {
+      for (int j = tid; j < r; j += static_cast<int>(blockDim.x)) {
         const uint32_t i = static_cast<uint32_t>(sh.hist[j]);
         const float score = okey_inv(candidate_key(sh.hist[j])) + gumbel_of(uniform(row_seeds[b], i));
         if (kept_mask != nullptr) kept_mask[static_cast<int64_t>(b) * V + i] = 1;
@@ -643,7 +645,9 @@ extern "C" int nvllm_sample(int64_t* out_ids, const float* logits, int32_t batch
                   (long long)ld);
   if (batch == 0) return 0;
   NVLLM_CHECK_ARG(out_ids && logits && temperatures && row_seeds, NVLLM_ERR_ARG, "sample: NULL pointer");
-  NVLLM_CUDA(launch_pdl(sample_kernel, dim3(batch), dim3(kThreads), 0, static_cast<cudaStream_t>(stream), out_ids, logits,
-                        static_cast<int>(vocab), ld, temperatures, top_k, top_p, row_seeds, kept_count, kept_mask));
+  const int threads = batch <= sm_count() ? kMaxThreads : kMaxThreads / 2;
+  NVLLM_CUDA(launch_pdl(threads == kMaxThreads ? sample_kernel<kMaxThreads> : sample_kernel<kMaxThreads / 2>, dim3(batch), dim3(threads), 0,
+                        static_cast<cudaStream_t>(stream), out_ids, logits, static_cast<int>(vocab), ld, temperatures, top_k, top_p, row_seeds,
+                        kept_count, kept_mask));
   return 0;
 }
