@@ -43,6 +43,7 @@ struct DecodeParams {
   float* ws_o;   // [B, H, S, D]
   float* ws_ml;  // [B, H, S, 2]
   int batch, H, Hkv, g, ngrp, max_blocks, block_size, num_splits;
+  int cluster;  // the splits of an item are one cluster and merge over distributed shared memory (no partials in memory, no second kernel)
   int64_t q_stride, out_stride, blk_stride, tok_stride, head_stride;
   float scale_log2;
   // FUSE only (nvllm_paged_decode_attention_fused): q points at the packed [q | k | v] rows of this step; the kernel applies
@@ -57,6 +58,19 @@ struct DecodeParams {
   float eps;
   int max_position;
 };
+
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+// the f32 at this shared-memory address in CTA `rank` of the cluster
+__device__ __forceinline__ float ld_peer_f32(uint32_t addr, int rank) {
+  uint32_t peer;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(peer) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(peer) : "memory");
+  return v;
+}
 
 template <int D, int STAGES, int NWARPS>
 struct DecodeCfg {
@@ -86,7 +100,6 @@ paged_decode_kernel(const DecodeParams p) {
   constexpr int KS = D / 16;  // k-steps of QK^T == m-tiles of PV
   extern __shared__ __align__(128) uint8_t smem[];
 
-  pdl_launch_dependents();
   const int split = blockIdx.x;
   const int kvh = blockIdx.y / p.ngrp;
   const int grp = blockIdx.y - kvh * p.ngrp;
@@ -94,6 +107,7 @@ paged_decode_kernel(const DecodeParams p) {
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   pdl_wait();  // q and the newest KV row were written by the previous kernel
+  pdl_launch_dependents();   // (not earlier: see gemm_skinny.cu)
   const int ctx_all = __ldg(p.ctx + b);        // tokens attended to, including (FUSE) this step's own
   const int ctx = FUSE ? max(ctx_all - 1, 0) : ctx_all;  // tokens read from the cache
   const int gvalid = min(8, p.g - grp * 8);   // q heads handled by this CTA
@@ -400,6 +414,10 @@ paged_decode_kernel(const DecodeParams p) {
     if (p.num_splits == 1) {
       p.out[b * p.out_stride + static_cast<int64_t>(qh) * D + d] =
           __float2bfloat16_rn(L > 0.f ? o / L : 0.f);
+    } else if (p.cluster) {
+      float* part = reinterpret_cast<float*>(smem + C::kMergeBytes);   // [8][D] and [8][2] behind the merge buffer
+      part[idx] = o;
+      if (d == 0) { part[8 * D + 2 * hn] = M; part[8 * D + 2 * hn + 1] = L; }
     } else {
       const int64_t slot = (static_cast<int64_t>(b) * p.H + qh) * p.num_splits + split;
       p.ws_o[slot * D + d] = o;
@@ -409,6 +427,27 @@ paged_decode_kernel(const DecodeParams p) {
       }
     }
   }
+  if (!p.cluster) return;
+  // the cluster's CTAs share the item's outputs; the splits are summed in rank order (as paged_decode_reduce_kernel does)
+  static_assert(C::kMergeBytes + (8 * D + 16) * 4 <= C::kSmemBytes, "the partial state fits behind the merge buffer");
+  cluster_sync();
+  const uint32_t mine = smem_u32(smem) + C::kMergeBytes;
+  for (int idx = split * NWARPS * 32 + threadIdx.x; idx < gvalid * D; idx += p.num_splits * NWARPS * 32) {
+    const int hn = idx / D;
+    float M = -INFINITY;
+    for (int s = 0; s < p.num_splits; ++s) M = fmaxf(M, ld_peer_f32(mine + (8 * D + 2 * hn) * 4, s));
+    float o = 0.f, L = 0.f;
+    if (M != -INFINITY)
+      for (int s = 0; s < p.num_splits; ++s) {
+        const float ms = ld_peer_f32(mine + (8 * D + 2 * hn) * 4, s);
+        if (ms == -INFINITY) continue;
+        const float f = fast_exp2(ms - M);
+        o += ld_peer_f32(mine + idx * 4, s) * f;
+        L += ld_peer_f32(mine + (8 * D + 2 * hn + 1) * 4, s) * f;
+      }
+    p.out[b * p.out_stride + static_cast<int64_t>(qh0) * D + idx] = __float2bfloat16_rn(L > 0.f ? o / L : 0.f);
+  }
+  cluster_sync();   // nobody leaves while a peer still reads its partial state
 }
 
 // ------------------------------------------------------------------------------------------------------------------
@@ -682,6 +721,8 @@ __global__ void __launch_bounds__(D) paged_decode_reduce_kernel(const DecodePara
 // ------------------------------------------------------------------------------------------------
 namespace nvllm {
 
+constexpr int kMaxClusterSplits = 16;
+
 template <int D, int STAGES, int NWARPS, bool FUSE = false>
 static int launch_decode(const DecodeParams& p, cudaStream_t stream) {
   using C = DecodeCfg<D, STAGES, NWARPS>;
@@ -689,6 +730,30 @@ static int launch_decode(const DecodeParams& p, cudaStream_t stream) {
   constexpr int kBytes = C::kSmemBytes + (FUSE ? 2 * C::kSubTileBytes : 0);  // + the step's own K/V sub-tile
   NVLLM_SMEM_ATTR_ONCE(kern, kBytes);
   dim3 grid(p.num_splits, p.Hkv * p.ngrp, p.batch);
+  // Few splits: a cluster per item, one launch instead of two (a launch in a chain of dependent kernels costs 4-6 us: a step of one
+  // token over 28 layers 1002 -> 954 us together with the norm, rotation and store inside this kernel).
+  if (p.num_splits > 1 && p.num_splits <= kMaxClusterSplits) {
+    static std::once_flag once;
+    static cudaError_t once_err = cudaSuccess;
+    std::call_once(once, [&] { once_err = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1); });
+    NVLLM_CUDA(once_err);
+    DecodeParams q = p;
+    q.cluster = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(NWARPS * 32);
+    cfg.dynamicSmemBytes = kBytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = p.num_splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    NVLLM_CUDA(cudaLaunchKernelEx(&cfg, kern, q));
+    return 0;
+  }
   NVLLM_CUDA(launch_pdl(kern, grid, dim3(NWARPS * 32), kBytes, stream, p));
   if (p.num_splits > 1)
     NVLLM_CUDA(launch_pdl(paged_decode_reduce_kernel<D>, dim3(p.H, p.batch), dim3(D), 0, stream, p));
@@ -830,6 +895,7 @@ static int decode_dispatch(void* out, const void* q, void* k_cache, void* v_cach
   p.max_blocks = max_blocks_per_seq;
   p.block_size = layout->block_size;
   p.num_splits = num_splits;
+  p.cluster = 0;
   p.q_stride = q_token_stride;
   p.out_stride = out_token_stride;
   p.blk_stride = layout->block_stride;
