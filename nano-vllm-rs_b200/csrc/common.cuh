@@ -48,6 +48,12 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 
 int sm_count();  // api.cu (cached)
 
+// Projections of up to 16 tokens (gemm_skinny.cu): y = x . w^T as nvllm_gemm_bf16 / nvllm_gemm_silu_mul_bf16; norm_w: x is normed
+// first (bf16 weights, k columns); residual: y += the bf16 product, in place.
+bool gemm_skinny_applies(int m, int n, int k, int64_t ldx, int64_t ldw);
+int gemm_skinny(void* y, const void* x, const void* w, int m, int n, int k, int64_t ldx, int64_t ldw, int64_t ldy, int out_dtype, bool silu_gate,
+                const void* norm_w, float eps, bool residual, cudaStream_t st);
+
 // The NVLLM_* environment knobs (A/B measurements), parsed ONCE per process — never on a dispatch
 // path.  nvllm_reload_env() (benchmark tools that sweep knobs inside one process) re-parses them.
 struct Knobs {
@@ -56,6 +62,7 @@ struct Knobs {
                             // behaviour: ~1 in 10 tiny-model runs at 8 ranks ends with rank 0 one call behind)
   int gemm_bn = 0;          // NVLLM_GEMM_BN: forced tile width (0 = heuristic)
   int gemm_2cta = 1;        // NVLLM_GEMM_2CTA: 0 never, 1 default (M > 512), 2 every M > 128
+  int gemm_skinny = 1;      // NVLLM_GEMM_SKINNY: 0 keeps products of up to 16 rows on the tcgen05 kernels
   int gemm_mcast = 0;       // NVLLM_GEMM_MCAST: 1 enables the x-multicast clusters
   int gemm_stages = 0;      // NVLLM_GEMM_STAGES: ring depth cap of single-wave launches (0 = deepest)
   int sk_stages = 0;        // NVLLM_GEMM_SK_STAGES: ring depth of the split-K kernel (0 = deepest)
@@ -227,6 +234,13 @@ __device__ __forceinline__ bf16* push_row(const RowPush& ps, int row) {
   const uint32_t b = ld_state(ps.ctrl + 131);
   return reinterpret_cast<bf16*>(base + ps.ll_off + static_cast<size_t>(b) * 2 * ps.ll_cap +
                                  (static_cast<size_t>(ps.rank) * ps.R + (row - owner * ps.R)) * ps.hidden * 2);
+}
+
+// 16 bytes of data that no running kernel writes and nothing reads twice (weights)
+__device__ __forceinline__ uint4 ld_nc_stream(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.L2::128B.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
 }
 
 // ---- cp.async (LDGSTS) ---------------------------------------------------------------------------

@@ -1,0 +1,208 @@
+// gemm_skinny.cu — projections of a few tokens (M <= 16): decode steps of small batches, bound by reading the weights once.
+//
+// The tcgen05 kernels stage 128-row tiles of x for one token and are bound by their fixed steps (operand ring, TMEM, split-K
+// exchange: 6-20 us a launch however small M is).  Here the weight rows are the M side of mma.sync m16n8k16 and the tokens the N side:
+// a warp loads its weight fragments straight from global memory into registers (a lane owns 8 neighbouring values of a row, one
+// 16-byte load; the product does not care in which order k is visited, so both operands use that order), all of a CTA's loads are in
+// flight at once, and they start BEFORE the wait for the predecessor kernel.  8 warps share a CTA's 16 (or, for narrow outputs, 8)
+// rows and split K; their f32 partial sums meet in shared memory in fixed order.
+// Fused around it, with the roundings of the separate kernels:
+//   norm_w    x is the residual stream and every CTA normalises its own copy of the few rows (rms(x) * w rounded to bf16)
+//   GATE      w = [gate | up]; the CTA computes the matching rows of both and writes silu(gate) * up
+//   residual  y = bf16(y + bf16(x . w^T)): the projection's output goes into the stream in place
+// Measured, a decode step of one token (Qwen3-0.6B, 28 layers, graph replay): 1408 us on the tcgen05 kernels, 862 with these; 28 layers of
+// weights and the head take 180 us at the copy rate, the rest is latency: 143 dependent launches of 5-6 us.
+#include "tc.cuh"
+
+namespace nvllm {
+namespace {
+
+constexpr int kSkThreads = 256, kSkWarps = 8;
+
+struct SkinnyArgs {
+  void* y; const bf16* x; const bf16* w; const bf16* norm_w;
+  int64_t ldx, ldw, ldy;
+  int m, n, k;
+  float eps;
+  int residual;
+};
+
+// NT: tokens / 8; ROWS: weight rows of a CTA (16, or 8 with the upper half of the MMA rows unused); PRE: 32-wide k-blocks a warp
+// loads ahead.
+template <int NT, int ROWS, int PRE, bool GATE, bool NORM, typename OutT>
+__global__ void __launch_bounds__(kSkThreads, sizeof(OutT) == 4 && NT == 1 ? 4 : 1) gemm_skinny_kernel(const SkinnyArgs a) {
+  constexpr int MATS = GATE ? 2 : 1, HV = ROWS / 8;   // 8-row halves
+  __shared__ float red[kSkWarps][MATS][NT * 8][ROWS + 1];
+  __shared__ float ssq[kSkWarps][NT * 8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+  const int n0 = blockIdx.x * ROWS, nkb = a.k / 32;
+  const bf16* wrow[MATS][HV];
+#pragma unroll
+  for (int i = 0; i < MATS; ++i)
+#pragma unroll
+    for (int h = 0; h < HV; ++h) {
+      const int r = n0 + 8 * h + g;
+      wrow[i][h] = r < a.n ? a.w + (static_cast<int64_t>(i) * a.n + r) * a.ldw + 8 * t4 : nullptr;
+    }
+  uint4 wf[PRE][MATS][HV];
+  auto load_w = [&](int kb, uint4 (&f)[MATS][HV]) {
+#pragma unroll
+    for (int i = 0; i < MATS; ++i)
+#pragma unroll
+      for (int h = 0; h < HV; ++h)
+        f[i][h] = (kb < nkb && wrow[i][h] != nullptr) ? ld_nc_stream(wrow[i][h] + kb * 32) : make_uint4(0, 0, 0, 0);
+  };
+#pragma unroll
+  for (int p = 0; p < PRE; ++p) load_w(warp + p * kSkWarps, wf[p]);
+  uint4 nk[PRE];
+  if (NORM) {
+#pragma unroll
+    for (int p = 0; p < PRE; ++p)
+      nk[p] = warp + p * kSkWarps < nkb ? __ldg(reinterpret_cast<const uint4*>(a.norm_w + (warp + p * kSkWarps) * 32 + 8 * t4)) : make_uint4(0, 0, 0, 0);
+  }
+  pdl_wait();   // the weights are in flight; x (and a residual y) come from the predecessor
+  // Only now may the successor start: launched any earlier, several kernels of the chain sit on the SMs at once and a step of one
+  // token is slower than without the overlap (28 layers: 925 us, 914 without, 836 so).
+  pdl_launch_dependents();
+  const bf16* xrow[NT];
+#pragma unroll
+  for (int j = 0; j < NT; ++j) xrow[j] = 8 * j + g < a.m ? a.x + (8 * j + g) * a.ldx + 8 * t4 : nullptr;
+  // the first PRE blocks of x stay in registers between the norm's sum and the products
+  uint4 xk[PRE][NT];
+#pragma unroll
+  for (int p = 0; p < PRE; ++p)
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      const int kb = warp + p * kSkWarps;
+      xk[p][j] = (xrow[j] != nullptr && kb < nkb) ? *reinterpret_cast<const uint4*>(xrow[j] + kb * 32) : make_uint4(0, 0, 0, 0);
+    }
+  float inv[NT];
+  if (NORM) {
+    auto squares = [](const uint4& v) {
+      const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+      float s = 0.f;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s += bf16_lo(u[e]) * bf16_lo(u[e]) + bf16_hi(u[e]) * bf16_hi(u[e]);
+      return s;
+    };
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      inv[j] = 0.f;
+#pragma unroll
+      for (int p = 0; p < PRE; ++p) inv[j] += squares(xk[p][j]);
+      if (xrow[j] != nullptr)
+        for (int kb = warp + PRE * kSkWarps; kb < nkb; kb += kSkWarps) inv[j] += squares(*reinterpret_cast<const uint4*>(xrow[j] + kb * 32));
+      inv[j] += __shfl_xor_sync(0xffffffffu, inv[j], 1);
+      inv[j] += __shfl_xor_sync(0xffffffffu, inv[j], 2);
+      if (t4 == 0) ssq[warp][8 * j + g] = inv[j];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      float s = 0.f;
+#pragma unroll
+      for (int i = 0; i < kSkWarps; ++i) s += ssq[i][8 * j + g];
+      inv[j] = 1.0f / sqrtf(s / static_cast<float>(a.k) + a.eps);
+    }
+  }
+  float acc[MATS][NT][4];
+#pragma unroll
+  for (int i = 0; i < MATS; ++i)
+#pragma unroll
+    for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.f;
+  for (int kb0 = warp; kb0 < nkb; kb0 += kSkWarps * PRE) {
+#pragma unroll
+    for (int p = 0; p < PRE; ++p) {
+      const int kb = kb0 + p * kSkWarps;
+      if (kb >= nkb) break;
+      uint4 xf[NT];
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+        xf[j] = kb0 == warp ? xk[p][j] : (xrow[j] != nullptr ? *reinterpret_cast<const uint4*>(xrow[j] + kb * 32) : make_uint4(0, 0, 0, 0));
+      if (NORM) {
+        const uint4 nv = kb0 == warp ? nk[p] : __ldg(reinterpret_cast<const uint4*>(a.norm_w + kb * 32 + 8 * t4));
+        const uint32_t nw[4] = {nv.x, nv.y, nv.z, nv.w};
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+          uint32_t u[4] = {xf[j].x, xf[j].y, xf[j].z, xf[j].w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) u[e] = pack_bf16x2(bf16_lo(u[e]) * inv[j] * bf16_lo(nw[e]), bf16_hi(u[e]) * inv[j] * bf16_hi(nw[e]));
+          xf[j] = make_uint4(u[0], u[1], u[2], u[3]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < MATS; ++i) {
+        const uint4 lo = wf[p][i][0], hi = HV == 2 ? wf[p][i][HV - 1] : make_uint4(0, 0, 0, 0);
+        const uint32_t a0[4] = {lo.x, hi.x, lo.y, hi.y}, a1[4] = {lo.z, hi.z, lo.w, hi.w};
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+          mma_bf16_16816(acc[i][j], a0, xf[j].x, xf[j].y);
+          mma_bf16_16816(acc[i][j], a1, xf[j].z, xf[j].w);
+        }
+      }
+      load_w(kb + kSkWarps * PRE, wf[p]);   // (nothing beyond the last block)
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < MATS; ++i)
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (e < 2 || HV == 2) red[warp][i][8 * j + 2 * t4 + (e & 1)][g + 8 * (e >> 1)] = acc[i][j][e];
+  __syncthreads();
+  for (int e = threadIdx.x; e < ROWS * NT * 8; e += kSkThreads) {
+    const int t = e / ROWS, r = e - t * ROWS;
+    if (t >= a.m || n0 + r >= a.n) continue;
+    float s[MATS];
+#pragma unroll
+    for (int i = 0; i < MATS; ++i) {
+      s[i] = 0.f;
+#pragma unroll
+      for (int wv = 0; wv < kSkWarps; ++wv) s[i] += red[wv][i][t][r];
+    }
+    OutT* dst = static_cast<OutT*>(a.y) + t * a.ldy + n0 + r;
+    if constexpr (GATE) {
+      const float2 p = gated_pair<kGateSilu>(pack_bf16x2(s[0], 0.f), pack_bf16x2(s[MATS - 1], 0.f), 0.f);
+      *dst = __float2bfloat16_rn(p.x);
+    } else if constexpr (sizeof(OutT) == 4) {
+      *dst = s[0];
+    } else {
+      float v = s[0];
+      if (a.residual) v = __bfloat162float(*dst) + __bfloat162float(__float2bfloat16_rn(v));
+      *dst = __float2bfloat16_rn(v);
+    }
+  }
+}
+
+template <int NT, int ROWS, int PRE, bool GATE, typename OutT>
+int skinny_run(const SkinnyArgs& a, cudaStream_t st) {
+  const dim3 grid((a.n + ROWS - 1) / ROWS);
+  NVLLM_CUDA(launch_pdl(a.norm_w != nullptr ? gemm_skinny_kernel<NT, ROWS, PRE, GATE, true, OutT> : gemm_skinny_kernel<NT, ROWS, PRE, GATE, false, OutT>,
+                        grid, dim3(kSkThreads), 0, st, a));
+  return 0;
+}
+
+template <int NT>
+int skinny_rows(const SkinnyArgs& a, bool gate, int out_dtype, cudaStream_t st) {
+  // 8-row CTAs where 16-row ones would leave SMs without work; k-blocks ahead: all of a warp's up to K = 1024 (narrow outputs: 3072)
+  if (gate) return skinny_run<NT, 16, 4, true, bf16>(a, st);
+  if (out_dtype == NVLLM_F32) return skinny_run<NT, 16, 4, false, float>(a, st);
+  if ((a.n + 15) / 16 < sm_count()) return skinny_run<NT, 8, 12, false, bf16>(a, st);
+  return skinny_run<NT, 16, 4, false, bf16>(a, st);
+}
+
+}  // namespace
+
+// Where these kernels take over: up to 16 tokens (beyond, the x fragments every CTA reads from L2 outweigh the weights), 16-byte rows.
+bool gemm_skinny_applies(int m, int n, int k, int64_t ldx, int64_t ldw) {
+  return knobs().gemm_skinny && m >= 1 && m <= 16 && k % 32 == 0 && ldx % 8 == 0 && ldw % 8 == 0 && n > 0;
+}
+
+int gemm_skinny(void* y, const void* x, const void* w, int m, int n, int k, int64_t ldx, int64_t ldw, int64_t ldy, int out_dtype, bool silu_gate,
+                const void* norm_w, float eps, bool residual, cudaStream_t st) {
+  const SkinnyArgs a{y, static_cast<const bf16*>(x), static_cast<const bf16*>(w), static_cast<const bf16*>(norm_w), ldx, ldw, ldy, m, n, k, eps, residual ? 1 : 0};
+  return m <= 8 ? skinny_rows<1>(a, silu_gate, out_dtype, st) : skinny_rows<2>(a, silu_gate, out_dtype, st);
+}
+
+}  // namespace nvllm

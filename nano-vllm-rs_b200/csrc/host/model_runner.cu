@@ -650,6 +650,15 @@ int nvllm_runner::forward(int N, int S, bool is_prefill, bool paged_prefill, con
     mark("add_rmsnorm");
     return rc;
   };
+  // Up to 16 tokens: every norm rides in the projection behind it, every residual add in the one before it (gemm_skinny.cu), so h is
+  // the stream itself throughout.
+  const bool few = tp == 1 && gemm_skinny_applies(N, hidden, hidden, hidden, hidden) && inter % 32 == 0 && HD % 32 == 0;
+  auto few_gemm = [&](void* y, const void* x, const void* w, int rows_n, int n, int k, int64_t ldy, int out_dt, bool gate, const bf16* norm, bool residual, const char* what) {
+    ++launches;
+    const int rc = gemm_skinny(y, x, w, rows_n, n, k, k, k, ldy, out_dt, gate, norm, eps, residual, stream);
+    mark(what);
+    return rc;
+  };
   RUN(nvllm_embedding_gather(h, embed, d_ids, N, hidden, vocab, NVLLM_BF16, st)); ++launches; mark("embedding_gather");
   const int splits = is_prefill ? 1 : nvllm_paged_decode_choose_splits(N, H, Hkv, table_cap * layout.block_size);
   if (!is_prefill) last_decode_splits = splits;
@@ -657,12 +666,13 @@ int nvllm_runner::forward(int N, int S, bool is_prefill, bool paged_prefill, con
     const LayerWeights& w = lw[l];
     // input_layernorm; for l > 0 fused with the residual add of the previous MLP output (qwen3.rs:389 -> :378)
     // (and, under TP, with the all-reduce of that output: see add_norm below)
-    if (l == 0) { RUN(nvllm_add_rmsnorm(normed, h, nullptr, w.input_ln, N, hidden, eps, NVLLM_BF16, st)); ++launches; mark("add_rmsnorm"); }
+    if (few) {}
+    else if (l == 0) { RUN(nvllm_add_rmsnorm(normed, h, nullptr, w.input_ln, N, hidden, eps, NVLLM_BF16, st)); ++launches; mark("add_rmsnorm"); }
     else RUN(add_norm(w.input_ln));
     const bf16* qnw = cfg.qk_norm ? w.q_norm : nullptr;
     const bf16* knw = cfg.qk_norm ? w.k_norm : nullptr;
     bool roped = false;  // q/k-norm + RoPE + KV store already applied to the qkv buffer / cache
-    if (fuse_rope && D == 128 && N <= 256) {
+    if (fuse_rope && !few && D == 128 && N <= 256) {
       // decode-sized batches: qkv GEMM with q/k norm + RoPE + KV-cache store in its epilogue (one head per 128-wide tile)
       ++launches;
       RUN(nvllm_gemm_qkv_rope_store(qkv, normed, w.qkv, N, hidden, hidden, hidden, d_pos, rope, qnw, knw, eps, H, Hkv, D,
@@ -670,8 +680,9 @@ int nvllm_runner::forward(int N, int S, bool is_prefill, bool paged_prefill, con
       mark("qkv_proj GEMM + rope/store epilogue");
       roped = true;
     } else {
-      RUN(gemm(qkv, normed, w.qkv, qkv_dim, hidden, qkv_dim, NVLLM_BF16, "qkv_proj GEMM"));
-      if (is_prefill || !fuse_decode) {
+      if (few) RUN(few_gemm(qkv, h, w.qkv, N, qkv_dim, hidden, qkv_dim, NVLLM_BF16, false, w.input_ln, false, "norm + qkv_proj"));
+      else RUN(gemm(qkv, normed, w.qkv, qkv_dim, hidden, qkv_dim, NVLLM_BF16, "qkv_proj GEMM"));
+      if (is_prefill || !(fuse_decode || (few && D == 128))) {   // (few: a launch costs more than the attention's longer prologue)
         // q/k norm + RoPE in place, K/V of this step into the cache (store before attention: note N2)
         RUN(nvllm_qknorm_rope_store(qkv, d_pos, rope, qnw, knw, eps, N, H, Hkv, D, cfg.max_position_embeddings, kc[l], vc[l],
                                     d_slots, &layout, NVLLM_BF16, st)); ++launches;
@@ -688,7 +699,7 @@ int nvllm_runner::forward(int N, int S, bool is_prefill, bool paged_prefill, con
         RUN(nvllm_paged_decode_attention(attn, qkv, kc[l], vc[l], d_tables, d_ctx, N, H, table_cap, qkv_dim, HD, &layout,
                                          scale, decode_ws, decode_ws_bytes, splits, NVLLM_BF16, st));
       }
-      launches += splits > 1 ? 2 : 1;
+      launches += splits > 16 ? 2 : 1;   // (up to 16 splits merge inside the kernel)
       mark(roped ? "paged_decode_attention" : "paged_decode_attention (+ q/k-norm, RoPE, KV store)");
     } else {
       RUN(nvllm_varlen_prefill_attention(attn, qkv, qkv + HD, qkv + HD + Hkv * D, d_cu_q, d_cu_k, S, N, N, b.max_seqlen_q,
@@ -696,6 +707,12 @@ int nvllm_runner::forward(int N, int S, bool is_prefill, bool paged_prefill, con
                                          paged_prefill ? vc[l] : nullptr, paged_prefill ? d_tables : nullptr, table_cap,
                                          &layout, scale, NVLLM_BF16, st)); ++launches;
       mark(paged_prefill ? "prefill_attention (paged prefix)" : "prefill_attention");
+    }
+    if (few) {
+      RUN(few_gemm(h, attn, w.o, N, hidden, HD, hidden, NVLLM_BF16, false, nullptr, true, "o_proj + residual"));
+      RUN(few_gemm(act, h, w.gate_up, N, inter, hidden, inter, NVLLM_BF16, true, w.post_ln, false, "norm + gate_up_proj + SiLU*mul"));
+      RUN(few_gemm(h, act, w.down, N, hidden, inter, hidden, NVLLM_BF16, false, nullptr, true, "down_proj + residual"));
+      continue;
     }
     RUN(row_gemm(attn, w.o, HD, "o_proj GEMM"));
     RUN(add_norm(w.post_ln));                                                                                          // qwen3.rs:382-385
@@ -706,22 +723,27 @@ int nvllm_runner::forward(int N, int S, bool is_prefill, bool paged_prefill, con
     mark("gate_up_proj GEMM + SiLU*mul");
     RUN(row_gemm(act, w.down, inter, "down_proj GEMM"));
   }
-  RUN(add_norm(final_norm));                                                                                           // qwen3.rs:389,501
-  const bf16* head_in = normed;
+  if (!few) RUN(add_norm(final_norm));                                                                                           // qwen3.rs:389,501
+  const bf16* last_rows = few ? h : normed;   // few: the final norm rides in the head's projection
+  const bf16* head_in = last_rows;
   int rows = N;
   if (is_prefill && explicit_rows) {  // the caller named the tokens whose logits it wants
     NVLLM_CHECK_ARG(n_logit_rows > 0 && n_logit_rows <= max_seqs, NVLLM_ERR_ARG, "execute: %d logit rows (1..max_num_seqs for this architecture)", n_logit_rows);
-    RUN(nvllm_gather_rows(last_hidden, normed, d_logit_rows, n_logit_rows, hidden, N, NVLLM_BF16, st)); ++launches; mark("gather_rows");
+    RUN(nvllm_gather_rows(last_hidden, last_rows, d_logit_rows, n_logit_rows, hidden, N, NVLLM_BF16, st)); ++launches; mark("gather_rows");
     head_in = last_hidden;
     rows = n_logit_rows;
   } else if (is_prefill) {  // only the last token of each sequence feeds the head (embed_head.rs:250-289)
-    RUN(nvllm_gather_last_tokens(last_hidden, normed, d_cu_q, S, hidden, NVLLM_BF16, st)); ++launches; mark("gather_last_tokens");
+    RUN(nvllm_gather_last_tokens(last_hidden, last_rows, d_cu_q, S, hidden, NVLLM_BF16, st)); ++launches; mark("gather_last_tokens");
     head_in = last_hidden;
     rows = S;
   }
-  ++launches;
-  RUN(nvllm_gemm_bf16(logits, head_in, lm_head, rows, vshard, hidden, hidden, hidden, vshard, NVLLM_F32, nullptr, 0, st));
-  mark("lm_head GEMM");
+  if (few) {
+    RUN(few_gemm(logits, head_in, lm_head, rows, vshard, hidden, vshard, NVLLM_F32, false, final_norm, false, "norm + lm_head"));
+  } else {
+    ++launches;
+    RUN(nvllm_gemm_bf16(logits, head_in, lm_head, rows, vshard, hidden, hidden, hidden, vshard, NVLLM_F32, nullptr, 0, st));
+    mark("lm_head GEMM");
+  }
   if (tp == 1) {
     RUN(nvllm_argmax(tokens, nullptr, logits, rows, vshard, vshard, 0, NVLLM_F32, st)); ++launches; mark("argmax");
   } else {  // sharded argmax: local (max, id) -> all-gather -> first-max combine

@@ -236,3 +236,23 @@ def test_gemm_x_multicast_clusters_opt_in(cuda, m, n, k, monkeypatch):
     r = ops.gemm_bf16(x, w, out_dtype=torch.float32, simt=True)
     torch.cuda.synchronize()
     assert_close(to_np_f32(y), to_np_f32(r), ATOL, RTOL, f"mcast gemm {m}x{n}x{k}")
+
+
+@pytest.mark.parametrize("m", [1, 7, 8, 9, 16])
+@pytest.mark.parametrize("n,k", [(8, 64), (1000, 192), (1024, 3072), (4104, 1024), (3072, 4096)])
+def test_products_of_a_few_rows(cuda, m, n, k):
+    """m <= 16: weight rows on the M side of mma.sync, K split over the warps of a CTA (8- and 16-row CTAs, remainders of both)."""
+    from nano_vllm_rs_b200 import ops
+    g = torch.Generator(device=cuda).manual_seed(m * n + k)
+    wide = torch.randn((m, k + 24), generator=g, device=cuda).to(torch.bfloat16)
+    x, w = wide[:, :k], (torch.randn((2 * n, k), generator=g, device=cuda) * k ** -0.5).to(torch.bfloat16)
+    want = x.double() @ w.double().T
+    # f32 sums of k exact products: k 2^-24 of sum |x w| is far above what any order of summation shows
+    bound = k * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+    got = ops.gemm_bf16(x, w[:n], out_dtype=torch.float32)
+    assert ((got.double() - want[:, :n]).abs() <= bound[:, :n]).all()
+    got = ops.gemm_bf16(x, w[:n])
+    assert ((got.double() - want[:, :n]).abs() <= bound[:, :n] + 2.0 ** -8 * want[:, :n].abs()).all()
+    if n % 128 == 0:
+        fused = ops.gemm_silu_mul(x, w)
+        assert torch.equal(fused, ops.silu_mul(ops.gemm_bf16(x, w)))
