@@ -101,6 +101,8 @@ struct nvllm_runner {
   // sampler parameters of the current step (only used when some sequence has temperature != 0):
   // [temperature f32 | top_k i32 | top_p f32 | row_seed u64] x max_seqs, pinned staging + device copy
   uint8_t *d_samp = nullptr, *h_samp = nullptr;
+  uint8_t* h_logit_stage = nullptr;  // pinned: logits on their way to the caller
+  size_t logit_stage_bytes = 0;
   // pointers into d_meta for the current step
   int64_t *d_ids = nullptr, *d_pos = nullptr;
   int32_t *d_slots = nullptr, *d_cu_q = nullptr, *d_cu_k = nullptr, *d_ctx = nullptr, *d_tables = nullptr;
@@ -144,6 +146,7 @@ struct nvllm_runner {
     if (h_meta) cudaFreeHost(h_meta);
     if (h_tokens) cudaFreeHost(h_tokens);
     if (h_samp) cudaFreeHost(h_samp);
+    if (h_logit_stage) cudaFreeHost(h_logit_stage);
     if (stream) cudaStreamDestroy(stream);
   }
 
@@ -165,6 +168,7 @@ struct nvllm_runner {
   int create_for_model(const nvllm_config& c);
   int forward_model(int n_tokens, int n_seqs);
   int ensure_logit_rows(int rows);
+  int stage_logits();
   int init_weights(uint64_t seed, float std);
   int load_weight(const char* name, const void* h_bf16, int64_t rows, int64_t cols);
   int upload(const nvllm_batch& b, int padded);
@@ -236,7 +240,15 @@ int nvllm_runner::create_for_model(const nvllm_config& c) {
   NVLLM_CUDA(cudaMallocHost(reinterpret_cast<void**>(&h_tokens), sizeof(int64_t) * S));
   RUN(dalloc(&d_samp, 24 * S));
   NVLLM_CUDA(cudaMallocHost(reinterpret_cast<void**>(&h_samp), 24 * S));
+  RUN(stage_logits());
   NVLLM_CUDA(cudaStreamSynchronize(stream));
+  return 0;
+}
+
+int nvllm_runner::stage_logits() {
+  const size_t bytes = std::min<size_t>(sizeof(float) * max_seqs * static_cast<size_t>(vshard), 4 << 20);
+  NVLLM_CUDA(cudaMallocHost(reinterpret_cast<void**>(&h_logit_stage), bytes));
+  logit_stage_bytes = bytes;
   return 0;
 }
 
@@ -371,6 +383,7 @@ int nvllm_runner::create(const nvllm_config& c, nvllm_comm* cm) {
   NVLLM_CUDA(cudaMallocHost(reinterpret_cast<void**>(&h_tokens), sizeof(int64_t) * S));
   RUN(dalloc(&d_samp, 24 * S));
   NVLLM_CUDA(cudaMallocHost(reinterpret_cast<void**>(&h_samp), 24 * S));
+  RUN(stage_logits());
   NVLLM_CUDA(cudaStreamSynchronize(stream));
   return 0;
 }
@@ -942,9 +955,15 @@ int nvllm_runner_execute(nvllm_runner* r, const nvllm_batch* b, int64_t* h_token
   NVLLM_CHECK_ARG(r && b, NVLLM_ERR_ARG, "runner_execute: NULL");
   RUN(r->execute_async(*b));
   const size_t logit_rows = (b->is_prefill && r->explicit_rows) ? r->n_logit_rows : b->num_seqs;
-  if (h_logits && logit_rows > 0)
-    NVLLM_CUDA(cudaMemcpyAsync(h_logits, r->logits, sizeof(float) * logit_rows * r->vshard, cudaMemcpyDeviceToHost, r->stream));
-  return r->fetch(h_tokens, b->num_seqs);
+  if (h_logits == nullptr || logit_rows == 0) return r->fetch(h_tokens, b->num_seqs);
+  // Logits of a few MB pass through the runner's pinned buffer: one DMA beside the step's other copies and one memcpy, instead of the
+  // driver's chunked copy into pageable memory.
+  const size_t bytes = sizeof(float) * logit_rows * r->vshard;
+  void* dst = bytes <= r->logit_stage_bytes ? static_cast<void*>(r->h_logit_stage) : h_logits;
+  NVLLM_CUDA(cudaMemcpyAsync(dst, r->logits, bytes, cudaMemcpyDeviceToHost, r->stream));
+  RUN(r->fetch(h_tokens, b->num_seqs));
+  if (dst != h_logits) memcpy(h_logits, dst, bytes);
+  return 0;
 }
 void* nvllm_runner_stream(nvllm_runner* r) { return r ? r->stream : nullptr; }
 int nvllm_runner_profile(nvllm_runner* r, int32_t enable) {

@@ -401,7 +401,7 @@ class ModelRunner:
             batch.c.num_logit_rows = self._rows.size
             self._rows_keep = keep
             rows = self._rows.size
-        logits = np.zeros((rows, self.vshard), np.float32) if return_logits else None
+        logits = np.empty((rows, self.vshard), np.float32) if return_logits else None   # written whole
         check(lib().nvllm_runner_execute(self.h, C.byref(batch.c), toks.ctypes.data,
                                          logits.ctypes.data if (return_logits and rows) else None))
         return (toks, logits) if return_logits else toks
@@ -526,7 +526,7 @@ class LLMEngine:
         ids = np.ascontiguousarray(seq_ids, dtype=np.int64)
         cnt = np.ascontiguousarray(counts, dtype=np.int32)
         rows = np.ascontiguousarray(logit_rows, dtype=np.int32)
-        out = np.zeros((rows.size, self.model_runner.vshard), np.float32)
+        out = np.empty((rows.size, self.model_runner.vshard), np.float32)   # written whole
         check(lib().nvllm_engine_step_chunks(self.h, ids.ctypes.data, cnt.ctypes.data, ids.size,
                                              rows.ctypes.data if rows.size else None, rows.size,
                                              out.ctypes.data if rows.size else None))
