@@ -35,6 +35,8 @@ __global__ void attn_bias_store_kernel(T* __restrict__ q, int64_t ldq, T* __rest
                                        const float* __restrict__ proj, int64_t ldp, const float* __restrict__ qb,
                                        const float* __restrict__ kb, const float* __restrict__ vb, const int32_t* __restrict__ slots,
                                        int qn, int kn, int vn) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int64_t t = blockIdx.x;
   const float* p = proj + t * ldp;
   for (int c = threadIdx.x; c < qn; c += blockDim.x) stv(q + t * ldq + c, p[c] + (qb ? qb[c] : 0.f));
@@ -48,6 +50,8 @@ __global__ void attn_bias_store_kernel(T* __restrict__ q, int64_t ldq, T* __rest
 template <typename T>
 __global__ void __launch_bounds__(256) attn_store_vec_kernel(T* __restrict__ q, int64_t ldq, T* __restrict__ kc, T* __restrict__ vc, int64_t k_row, int64_t v_row,
                                                              const float* __restrict__ proj, int64_t ldp, const int32_t* __restrict__ slots, int qn, int kn, int vn) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int64_t t = blockIdx.x;
   const float4* p = reinterpret_cast<const float4*>(proj + t * ldp);
   const int32_t slot = slots[t];
@@ -69,6 +73,8 @@ __global__ void __launch_bounds__(256) attn_wide_norm_store_kernel(T* __restrict
                                                                    int64_t k_row, int64_t v_row, const float* __restrict__ proj, int64_t ldp,
                                                                    const float* __restrict__ qw, const float* __restrict__ kw,
                                                                    const int32_t* __restrict__ slots, int qn, int kn, int vn, float eps) {
+  pdl_wait();
+  pdl_launch_dependents();
   __shared__ float red[2][8];
   const int64_t t = blockIdx.x;
   const float* p = proj + t * ldp;
@@ -129,6 +135,8 @@ __device__ __forceinline__ void head_norm_store(F value, T* dst, int dim, float 
 // v_from_k the value head IS the key head as projected (bias added, neither rotated nor normed).
 template <typename T>
 __global__ void __launch_bounds__(128) attn_rope_norm_store_kernel(const RopeStoreArgs a) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int per = a.heads + a.kv_heads + (a.v_from_k ? 0 : a.kv_heads);
   const int64_t item = static_cast<int64_t>(blockIdx.x) * 4 + warp;
@@ -209,6 +217,8 @@ __global__ void __launch_bounds__(128) attn_rope_norm_store_kernel(const RopeSto
 // The same with 16-byte accesses (dim a multiple of 4, at most 512; aligned rows): the head stays in registers, one pass.
 template <typename T>
 __global__ void __launch_bounds__(128) attn_rope_norm_store_vec_kernel(const RopeStoreArgs a) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int per = a.heads + a.kv_heads;
   const int64_t item = static_cast<int64_t>(blockIdx.x) * 4 + warp;
@@ -260,6 +270,8 @@ __global__ void __launch_bounds__(128) attn_rope_norm_store_vec_kernel(const Rop
 // rotation is the chunk half the rotated part away (read again: it is in L1), so nothing crosses lanes but the norm's sum.
 template <typename T>
 __global__ void __launch_bounds__(128) attn_rotary_store_halves_vec_kernel(const RopeStoreArgs a) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int per = a.heads + 2 * a.kv_heads;
   const int64_t item = static_cast<int64_t>(blockIdx.x) * 4 + warp;
@@ -331,6 +343,8 @@ struct NormStoreArgs {
 // One warp per (token, head) over the heads [q heads | key heads | value heads]; any sizes, both pairings.
 template <typename T>
 __global__ void __launch_bounds__(128) attn_norm_rotary_store_kernel(const NormStoreArgs a) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int lane = threadIdx.x & 31, per = a.heads + 2 * a.kv_heads;
   const int64_t item = static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5);
   if (item >= static_cast<int64_t>(a.n) * per) return;
@@ -383,6 +397,8 @@ __global__ void __launch_bounds__(128) attn_norm_rotary_store_kernel(const NormS
 // head stays in registers; a chunk's partner in the rotation is read again (it is in L1).
 template <typename T>
 __global__ void __launch_bounds__(128) attn_norm_rotary_store_vec_kernel(const NormStoreArgs a) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int lane = threadIdx.x & 31, per = a.heads + 2 * a.kv_heads;
   const int64_t item = static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5);
   if (item >= static_cast<int64_t>(a.n) * per) return;
@@ -499,6 +515,8 @@ constexpr int kMaxVPerLane = 16;  // vdim <= 512
 // the online-softmax statistics, then every lane accumulates its output dimensions over the 32 keys.
 template <typename T>
 __global__ void __launch_bounds__(128) capped_attn_warp_kernel(const AttnArgs a) {
+  pdl_wait();
+  pdl_launch_dependents();
   extern __shared__ float qs[];  // [4 warps][max(dim, vdim)]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t item = static_cast<int64_t>(blockIdx.x) * 4 + warp;
@@ -716,6 +734,8 @@ __device__ __forceinline__ void attn_tile(float (&o)[VMAX / 8][4], float (&m)[2]
 template <int DMAX, int VMAX, int EXT, int WARPS>
 __global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) capped_attn_mma_kernel(const AttnArgs a, const int32_t* __restrict__ cu_tokens, int n_seqs, int tq,
                                                               int group) {
+  pdl_wait();
+  pdl_launch_dependents();
   constexpr int kRows = 16 * WARPS, kThreads = 32 * WARPS;
   constexpr int QS = DMAX + 8, VS = VMAX + 8;       // shared-memory row strides (elements): 16-byte rows, conflict-free ldmatrix
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -973,7 +993,7 @@ int launch_mma(AttnArgs a, const int32_t* cu_tokens, int n_seqs, cudaStream_t st
   const size_t smem = tiles + (a.bias_staged ? bias_bytes : 0);
   NVLLM_SMEM_ATTR_ONCE((capped_attn_mma_kernel<DMAX, VMAX, EXT, WARPS>), tiles + (EXT == kExtTable ? kBiasSmemBytes : 0));
   dim3 grid((a.n + tq - 1) / tq + n_seqs, a.kv_heads);
-  capped_attn_mma_kernel<DMAX, VMAX, EXT, WARPS><<<grid, kThreads, smem, st>>>(a, cu_tokens, n_seqs, tq, group);
+  NVLLM_CUDA(launch_plain(capped_attn_mma_kernel<DMAX, VMAX, EXT, WARPS>, dim3(grid), dim3(kThreads), smem, st, a, cu_tokens, n_seqs, tq, group));
   NVLLM_LAUNCH_CHECK("capped_attn_mma_kernel");
   return 0;
 }
@@ -996,20 +1016,20 @@ extern "C" int nvllm_attn_bias_store(void* q, int64_t ldq, void* k_cache, void* 
   if (!q_bias && !k_bias && !v_bias && q_cols % 4 == 0 && k_cols % 4 == 0 && v_cols % 4 == 0 && ldq % 4 == 0 && k_row % 4 == 0 && v_row % 4 == 0 &&
       ldp % 4 == 0 && aligned16(q) && aligned16(k_cache) && aligned16(v_cache) && aligned16(proj)) {
     if (dtype == NVLLM_BF16)
-      attn_store_vec_kernel<bf16><<<n, 256, 0, st>>>(static_cast<bf16*>(q), ldq, static_cast<bf16*>(k_cache), static_cast<bf16*>(v_cache), k_row, v_row, proj,
-                                                     ldp, slots, q_cols, k_cols, v_cols);
+      NVLLM_CUDA(launch_pdl(attn_store_vec_kernel<bf16>, dim3(n), dim3(256), 0, st, static_cast<bf16*>(q), ldq, static_cast<bf16*>(k_cache), static_cast<bf16*>(v_cache), k_row, v_row, proj,
+                                                     ldp, slots, q_cols, k_cols, v_cols));
     else
-      attn_store_vec_kernel<float><<<n, 256, 0, st>>>(static_cast<float*>(q), ldq, static_cast<float*>(k_cache), static_cast<float*>(v_cache), k_row, v_row,
-                                                      proj, ldp, slots, q_cols, k_cols, v_cols);
+      NVLLM_CUDA(launch_pdl(attn_store_vec_kernel<float>, dim3(n), dim3(256), 0, st, static_cast<float*>(q), ldq, static_cast<float*>(k_cache), static_cast<float*>(v_cache), k_row, v_row,
+                                                      proj, ldp, slots, q_cols, k_cols, v_cols));
     NVLLM_LAUNCH_CHECK("attn_store_vec_kernel");
     return 0;
   }
   if (dtype == NVLLM_BF16)
-    attn_bias_store_kernel<bf16><<<n, 256, 0, st>>>(static_cast<bf16*>(q), ldq, static_cast<bf16*>(k_cache), static_cast<bf16*>(v_cache), k_row,
-                                                    v_row, proj, ldp, q_bias, k_bias, v_bias, slots, q_cols, k_cols, v_cols);
+    NVLLM_CUDA(launch_pdl(attn_bias_store_kernel<bf16>, dim3(n), dim3(256), 0, st, static_cast<bf16*>(q), ldq, static_cast<bf16*>(k_cache), static_cast<bf16*>(v_cache), k_row,
+                                                    v_row, proj, ldp, q_bias, k_bias, v_bias, slots, q_cols, k_cols, v_cols));
   else
-    attn_bias_store_kernel<float><<<n, 256, 0, st>>>(static_cast<float*>(q), ldq, static_cast<float*>(k_cache), static_cast<float*>(v_cache),
-                                                     k_row, v_row, proj, ldp, q_bias, k_bias, v_bias, slots, q_cols, k_cols, v_cols);
+    NVLLM_CUDA(launch_pdl(attn_bias_store_kernel<float>, dim3(n), dim3(256), 0, st, static_cast<float*>(q), ldq, static_cast<float*>(k_cache), static_cast<float*>(v_cache),
+                                                     k_row, v_row, proj, ldp, q_bias, k_bias, v_bias, slots, q_cols, k_cols, v_cols));
   NVLLM_LAUNCH_CHECK("attn_bias_store_kernel");
   return 0;
 }
@@ -1025,11 +1045,11 @@ extern "C" int nvllm_attn_wide_norm_store(void* q, int64_t ldq, void* k_cache, v
   NVLLM_CHECK_ARG(q && proj && slots && (k_cols == 0 || (k_cache && v_cache)), NVLLM_ERR_ARG, "attn_wide_norm_store: NULL");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (dtype == NVLLM_BF16)
-    attn_wide_norm_store_kernel<bf16><<<n, 256, 0, st>>>(static_cast<bf16*>(q), ldq, static_cast<bf16*>(k_cache), static_cast<bf16*>(v_cache),
-                                                         k_row, v_row, proj, ldp, q_norm_w, k_norm_w, slots, q_cols, k_cols, v_cols, eps);
+    NVLLM_CUDA(launch_pdl(attn_wide_norm_store_kernel<bf16>, dim3(n), dim3(256), 0, st, static_cast<bf16*>(q), ldq, static_cast<bf16*>(k_cache), static_cast<bf16*>(v_cache),
+                                                         k_row, v_row, proj, ldp, q_norm_w, k_norm_w, slots, q_cols, k_cols, v_cols, eps));
   else
-    attn_wide_norm_store_kernel<float><<<n, 256, 0, st>>>(static_cast<float*>(q), ldq, static_cast<float*>(k_cache), static_cast<float*>(v_cache),
-                                                          k_row, v_row, proj, ldp, q_norm_w, k_norm_w, slots, q_cols, k_cols, v_cols, eps);
+    NVLLM_CUDA(launch_pdl(attn_wide_norm_store_kernel<float>, dim3(n), dim3(256), 0, st, static_cast<float*>(q), ldq, static_cast<float*>(k_cache), static_cast<float*>(v_cache),
+                                                          k_row, v_row, proj, ldp, q_norm_w, k_norm_w, slots, q_cols, k_cols, v_cols, eps));
   NVLLM_LAUNCH_CHECK("attn_wide_norm_store_kernel");
   return 0;
 }
@@ -1071,8 +1091,8 @@ extern "C" int nvllm_attn_rotary_store(void* q, int64_t ldq, void* k_cache, void
   if (v_from_k && !halves && dim % 4 == 0 && dim <= 512 && ldp % 4 == 0 && ldq % 4 == 0 && k_row % 4 == 0 && v_row % 4 == 0 && aligned16(proj) && aligned16(q) &&
       aligned16(k_cache) && aligned16(v_cache) && aligned16(q_bias) && aligned16(k_bias)) {
     const int64_t vitems = static_cast<int64_t>(n) * (heads + kv_heads);
-    if (dtype == NVLLM_BF16) attn_rope_norm_store_vec_kernel<bf16><<<static_cast<unsigned>((vitems + 3) / 4), 128, 0, st>>>(a);
-    else attn_rope_norm_store_vec_kernel<float><<<static_cast<unsigned>((vitems + 3) / 4), 128, 0, st>>>(a);
+    if (dtype == NVLLM_BF16) NVLLM_CUDA(launch_pdl(attn_rope_norm_store_vec_kernel<bf16>, dim3(static_cast<unsigned>((vitems + 3) / 4)), dim3(128), 0, st, a));
+    else NVLLM_CUDA(launch_pdl(attn_rope_norm_store_vec_kernel<float>, dim3(static_cast<unsigned>((vitems + 3) / 4)), dim3(128), 0, st, a));
     NVLLM_LAUNCH_CHECK("attn_rope_norm_store_vec_kernel");
     return 0;
   }
@@ -1080,13 +1100,13 @@ extern "C" int nvllm_attn_rotary_store(void* q, int64_t ldq, void* k_cache, void
   if (halves && !v_from_k && !q_bias && !k_bias && !v_bias && dim % 4 == 0 && vdim % 4 == 0 && dim <= 512 && vdim <= 512 && rot_dims % 8 == 0 &&
       (v_rope_table == nullptr || vdim % 8 == 0) && ldp % 4 == 0 && ldq % 4 == 0 && k_row % 4 == 0 && v_row % 4 == 0 && aligned16(proj) && aligned16(q) &&
       aligned16(k_cache) && aligned16(v_cache) && aligned16(rope_table) && aligned16(v_rope_table)) {
-    if (dtype == NVLLM_BF16) attn_rotary_store_halves_vec_kernel<bf16><<<static_cast<unsigned>((items + 3) / 4), 128, 0, st>>>(a);
-    else attn_rotary_store_halves_vec_kernel<float><<<static_cast<unsigned>((items + 3) / 4), 128, 0, st>>>(a);
+    if (dtype == NVLLM_BF16) NVLLM_CUDA(launch_pdl(attn_rotary_store_halves_vec_kernel<bf16>, dim3(static_cast<unsigned>((items + 3) / 4)), dim3(128), 0, st, a));
+    else NVLLM_CUDA(launch_pdl(attn_rotary_store_halves_vec_kernel<float>, dim3(static_cast<unsigned>((items + 3) / 4)), dim3(128), 0, st, a));
     NVLLM_LAUNCH_CHECK("attn_rotary_store_halves_vec_kernel");
     return 0;
   }
-  if (dtype == NVLLM_BF16) attn_rope_norm_store_kernel<bf16><<<static_cast<unsigned>((items + 3) / 4), 128, 0, st>>>(a);
-  else attn_rope_norm_store_kernel<float><<<static_cast<unsigned>((items + 3) / 4), 128, 0, st>>>(a);
+  if (dtype == NVLLM_BF16) NVLLM_CUDA(launch_pdl(attn_rope_norm_store_kernel<bf16>, dim3(static_cast<unsigned>((items + 3) / 4)), dim3(128), 0, st, a));
+  else NVLLM_CUDA(launch_pdl(attn_rope_norm_store_kernel<float>, dim3(static_cast<unsigned>((items + 3) / 4)), dim3(128), 0, st, a));
   NVLLM_LAUNCH_CHECK("attn_rope_norm_store_kernel");
   return 0;
 }
@@ -1116,13 +1136,13 @@ extern "C" int nvllm_attn_norm_rotary_store(void* q, int64_t ldq, void* k_cache,
   if (halves && dim % 4 == 0 && vdim % 4 == 0 && dim <= 512 && rot_dims % 8 == 0 && ldp % 4 == 0 && ldq % 4 == 0 && k_row % 4 == 0 && v_row % 4 == 0 &&
       ldvf % 4 == 0 && aligned16(proj) && aligned16(q) && aligned16(k_cache) && aligned16(v_cache) && aligned16(rope_table) && aligned16(q_norm_w) &&
       aligned16(k_norm_w) && aligned16(v_first)) {
-    if (dtype == NVLLM_BF16) attn_norm_rotary_store_vec_kernel<bf16><<<grid, 128, 0, st>>>(a);
-    else attn_norm_rotary_store_vec_kernel<float><<<grid, 128, 0, st>>>(a);
+    if (dtype == NVLLM_BF16) NVLLM_CUDA(launch_pdl(attn_norm_rotary_store_vec_kernel<bf16>, dim3(grid), dim3(128), 0, st, a));
+    else NVLLM_CUDA(launch_pdl(attn_norm_rotary_store_vec_kernel<float>, dim3(grid), dim3(128), 0, st, a));
     NVLLM_LAUNCH_CHECK("attn_norm_rotary_store_vec_kernel");
     return 0;
   }
-  if (dtype == NVLLM_BF16) attn_norm_rotary_store_kernel<bf16><<<grid, 128, 0, st>>>(a);
-  else attn_norm_rotary_store_kernel<float><<<grid, 128, 0, st>>>(a);
+  if (dtype == NVLLM_BF16) NVLLM_CUDA(launch_pdl(attn_norm_rotary_store_kernel<bf16>, dim3(grid), dim3(128), 0, st, a));
+  else NVLLM_CUDA(launch_pdl(attn_norm_rotary_store_kernel<float>, dim3(grid), dim3(128), 0, st, a));
   NVLLM_LAUNCH_CHECK("attn_norm_rotary_store_kernel");
   return 0;
 }
@@ -1225,8 +1245,8 @@ extern "C" int nvllm_extended_attention(void* out, int64_t ldo, const void* q, i
   }
   const unsigned grid = static_cast<unsigned>((static_cast<int64_t>(n) * heads + 3) / 4);
   const size_t smem = static_cast<size_t>(4) * (dim > vdim ? dim : vdim) * sizeof(float);
-  if (dtype == NVLLM_BF16) capped_attn_warp_kernel<bf16><<<grid, 128, smem, st>>>(a);
-  else capped_attn_warp_kernel<float><<<grid, 128, smem, st>>>(a);
+  if (dtype == NVLLM_BF16) NVLLM_CUDA(launch_pdl(capped_attn_warp_kernel<bf16>, dim3(grid), dim3(128), smem, st, a));
+  else NVLLM_CUDA(launch_pdl(capped_attn_warp_kernel<float>, dim3(grid), dim3(128), smem, st, a));
   NVLLM_LAUNCH_CHECK("capped_attn_warp_kernel");
   return 0;
 }

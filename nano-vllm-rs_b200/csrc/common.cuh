@@ -133,6 +133,18 @@ __device__ __forceinline__ uint32_t ld_state(const uint32_t* p) {
   return v;
 }
 
+// A plain launch in the same form: for kernels that are bound by one or two long-lived CTAs per SM.  Launched early, such CTAs take the
+// slots the predecessor has freed by then, two on one SM and none on another, and the doubled SM decides the kernel's time.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_plain(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                               Args&&... args) {

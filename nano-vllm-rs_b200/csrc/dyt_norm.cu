@@ -31,6 +31,8 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 // bf16 rows whose length is a multiple of 8: 16-byte vectors (the residual as two float4)
 __global__ void dyt_residual_norm_vec8_kernel(bf16* __restrict__ out, float* __restrict__ h, const bf16* __restrict__ y,
                                               DytParams post, DytParams pre, int64_t total8, int hidden8) {
+  pdl_wait();
+  pdl_launch_dependents();
   const float a_post = y ? *post.alpha : 0.f, a_pre = out ? *pre.alpha : 0.f;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total8;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -58,6 +60,8 @@ __global__ void dyt_residual_norm_vec8_kernel(bf16* __restrict__ out, float* __r
 template <typename T>
 __global__ void dyt_residual_norm_kernel(T* __restrict__ out, float* __restrict__ h, const T* __restrict__ y, DytParams post,
                                          DytParams pre, int64_t total, int hidden) {
+  pdl_wait();
+  pdl_launch_dependents();
   const float a_post = y ? *post.alpha : 0.f, a_pre = out ? *pre.alpha : 0.f;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -74,6 +78,8 @@ __global__ void dyt_residual_norm_kernel(T* __restrict__ out, float* __restrict_
 template <typename T>
 __global__ void embedding_f32_kernel(float* __restrict__ h, const T* __restrict__ table, const int64_t* __restrict__ ids,
                                      int n, int hidden, int vocab) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int64_t total = static_cast<int64_t>(n) * hidden;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -87,6 +93,8 @@ __global__ void embedding_f32_kernel(float* __restrict__ h, const T* __restrict_
 // rows whose byte length is a multiple of 16: plain 16-byte copies
 __global__ void gather_rows_vec_kernel(uint4* __restrict__ out, const uint4* __restrict__ x, const int32_t* __restrict__ rows, int n,
                                        int vecs, int n_src) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int64_t total = static_cast<int64_t>(n) * vecs;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -100,6 +108,8 @@ __global__ void gather_rows_vec_kernel(uint4* __restrict__ out, const uint4* __r
 template <typename T>
 __global__ void gather_rows_kernel(T* __restrict__ out, const T* __restrict__ x, const int32_t* __restrict__ rows, int n,
                                    int hidden, int n_src) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int64_t total = static_cast<int64_t>(n) * hidden;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -134,12 +144,12 @@ extern "C" int nvllm_dyt_residual_norm(void* out, float* h, const void* y, const
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const DytParams post{post_alpha, post_w, post_b}, pre{pre_alpha, pre_w, pre_b};
   if (dtype == NVLLM_BF16 && hidden % 8 == 0 && aligned16(h) && aligned16(out) && aligned16(y))
-    dyt_residual_norm_vec8_kernel<<<blocks_for(total / 8), 256, 0, st>>>(static_cast<bf16*>(out), h, static_cast<const bf16*>(y), post, pre,
-                                                                          total / 8, hidden / 8);
+    NVLLM_CUDA(launch_pdl(dyt_residual_norm_vec8_kernel, dim3(blocks_for(total / 8)), dim3(256), 0, st, static_cast<bf16*>(out), h, static_cast<const bf16*>(y), post, pre,
+                                                                          total / 8, hidden / 8));
   else if (dtype == NVLLM_BF16)
-    dyt_residual_norm_kernel<bf16><<<blocks_for(total), 256, 0, st>>>(static_cast<bf16*>(out), h, static_cast<const bf16*>(y), post, pre, total, hidden);
+    NVLLM_CUDA(launch_pdl(dyt_residual_norm_kernel<bf16>, dim3(blocks_for(total)), dim3(256), 0, st, static_cast<bf16*>(out), h, static_cast<const bf16*>(y), post, pre, total, hidden));
   else
-    dyt_residual_norm_kernel<float><<<blocks_for(total), 256, 0, st>>>(static_cast<float*>(out), h, static_cast<const float*>(y), post, pre, total, hidden);
+    NVLLM_CUDA(launch_pdl(dyt_residual_norm_kernel<float>, dim3(blocks_for(total)), dim3(256), 0, st, static_cast<float*>(out), h, static_cast<const float*>(y), post, pre, total, hidden));
   NVLLM_LAUNCH_CHECK("dyt_residual_norm_kernel");
   return 0;
 }
@@ -153,9 +163,9 @@ extern "C" int nvllm_embedding_gather_f32(float* h, const void* table, const int
   const int64_t total = static_cast<int64_t>(n) * hidden;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (table_dtype == NVLLM_BF16)
-    embedding_f32_kernel<bf16><<<blocks_for(total), 256, 0, st>>>(h, static_cast<const bf16*>(table), ids, n, hidden, vocab);
+    NVLLM_CUDA(launch_pdl(embedding_f32_kernel<bf16>, dim3(blocks_for(total)), dim3(256), 0, st, h, static_cast<const bf16*>(table), ids, n, hidden, vocab));
   else
-    embedding_f32_kernel<float><<<blocks_for(total), 256, 0, st>>>(h, static_cast<const float*>(table), ids, n, hidden, vocab);
+    NVLLM_CUDA(launch_pdl(embedding_f32_kernel<float>, dim3(blocks_for(total)), dim3(256), 0, st, h, static_cast<const float*>(table), ids, n, hidden, vocab));
   NVLLM_LAUNCH_CHECK("embedding_f32_kernel");
   return 0;
 }
@@ -171,14 +181,14 @@ extern "C" int nvllm_gather_rows(void* out, const void* x, const int32_t* rows, 
   const int64_t row_bytes = static_cast<int64_t>(hidden) * (dtype == NVLLM_BF16 ? 2 : 4);
   if (row_bytes % 16 == 0 && aligned16(out) && aligned16(x)) {
     const int vecs = static_cast<int>(row_bytes / 16);
-    gather_rows_vec_kernel<<<blocks_for(static_cast<int64_t>(n) * vecs), 256, 0, st>>>(static_cast<uint4*>(out), static_cast<const uint4*>(x), rows, n, vecs, n_src);
+    NVLLM_CUDA(launch_pdl(gather_rows_vec_kernel, dim3(blocks_for(static_cast<int64_t>(n) * vecs)), dim3(256), 0, st, static_cast<uint4*>(out), static_cast<const uint4*>(x), rows, n, vecs, n_src));
     NVLLM_LAUNCH_CHECK("gather_rows_vec_kernel");
     return 0;
   }
   if (dtype == NVLLM_BF16)
-    gather_rows_kernel<bf16><<<blocks_for(total), 256, 0, st>>>(static_cast<bf16*>(out), static_cast<const bf16*>(x), rows, n, hidden, n_src);
+    NVLLM_CUDA(launch_pdl(gather_rows_kernel<bf16>, dim3(blocks_for(total)), dim3(256), 0, st, static_cast<bf16*>(out), static_cast<const bf16*>(x), rows, n, hidden, n_src));
   else
-    gather_rows_kernel<float><<<blocks_for(total), 256, 0, st>>>(static_cast<float*>(out), static_cast<const float*>(x), rows, n, hidden, n_src);
+    NVLLM_CUDA(launch_pdl(gather_rows_kernel<float>, dim3(blocks_for(total)), dim3(256), 0, st, static_cast<float*>(out), static_cast<const float*>(x), rows, n, hidden, n_src));
   NVLLM_LAUNCH_CHECK("gather_rows_kernel");
   return 0;
 }

@@ -86,6 +86,8 @@ struct NormStoreArgs {
 
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(128) latent_norm_store_kernel(const NormStoreArgs a) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int lane = threadIdx.x & 31;
   const int64_t item = static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5);
   if (item >= 2 * static_cast<int64_t>(a.n)) return;
@@ -147,6 +149,8 @@ __global__ void __launch_bounds__(128) latent_norm_store_kernel(const NormStoreA
 template <typename T, int PAIRS>
 __global__ void __launch_bounds__(256) rotate_tail_kernel(T* __restrict__ x, int64_t ldx, const int64_t* __restrict__ positions, const float2* __restrict__ table,
                                                           int max_pos, int64_t n, int heads, int dim, int rot_dim, int half) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int per = half / PAIRS;
   const int64_t total = n * heads * per;
   for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total; e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -188,6 +192,8 @@ struct PrepArgs {
 // rotated part) on dkv[kv_rank:] -> cache row, and in place on the rotated part of every query head.
 template <typename T>
 __global__ void __launch_bounds__(128) latent_prepare_kernel(const PrepArgs a) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * 4 + warp;
   if (t >= a.n) return;
@@ -234,6 +240,8 @@ constexpr int kKeyTile = 32;
 // (f32) and shared by the CTA's heads; lane j scores key j, then every lane owns kv_rank/32 output columns.
 template <typename T, int RI>
 __global__ void __launch_bounds__(256) latent_attn_kernel(const AttnArgs a) {
+  pdl_wait();
+  pdl_launch_dependents();
   extern __shared__ float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   const int t = blockIdx.x, h = blockIdx.y * nwarps + warp;
@@ -314,7 +322,7 @@ int launch_attn(const AttnArgs& a, cudaStream_t st) {
   NVLLM_CHECK_ARG(smem <= 220 * 1024, NVLLM_ERR_ARG, "latent_attention: kv_rank + rot_dim = %d needs %zu bytes of shared memory", D, smem);
   NVLLM_SMEM_ATTR_ONCE((latent_attn_kernel<T, RI>), 220 * 1024);
   dim3 grid(a.n, (a.heads + hpb - 1) / hpb);
-  latent_attn_kernel<T, RI><<<grid, 32 * hpb, smem, st>>>(a);
+  NVLLM_CUDA(launch_pdl(latent_attn_kernel<T, RI>, dim3(grid), dim3(32 * hpb), smem, st, a));
   NVLLM_LAUNCH_CHECK("latent_attn_kernel");
   return 0;
 }
@@ -338,6 +346,8 @@ constexpr int kMmaKeys = 64, kPsStride = 72, kSsStride = 68, kMmaThreads = 256;
 // the CTA runs them one after the other.
 template <int NT2, int TQ>  // kv_rank padded to NT2 * 128
 __global__ void __launch_bounds__(kMmaThreads) latent_attn_mma_kernel(const AttnArgs a, int DPS, int DP16) {
+  pdl_wait();
+  pdl_launch_dependents();
   extern __shared__ __align__(16) uint8_t smraw[];
   bf16* Qs = reinterpret_cast<bf16*>(smraw);          // TQ x [16][DPS]
   bf16* Kbuf = Qs + TQ * 16 * DPS;                    // 2 x [64][DPS]: the next tile lands while this one is used
@@ -632,6 +642,8 @@ __global__ void __launch_bounds__(kMmaThreads) latent_attn_mma_kernel(const Attn
 
 // One warp per (token, head): merges the splits' partial softmaxes, adds the sink to the denominator, applies the gate.
 __global__ void __launch_bounds__(128) latent_attn_merge_kernel(const AttnArgs a) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int lane = threadIdx.x & 31;
   const int64_t item = static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5);
   if (item >= static_cast<int64_t>(a.n) * a.heads) return;
@@ -669,10 +681,10 @@ int launch_attn_mma_tq(const AttnArgs& a, cudaStream_t st) {
   const int items = (a.n + TQ - 1) / TQ, groups = (a.heads + 15) / 16;
   // behind the tcgen05 kernel a launch with nothing to do should cost little: no more CTAs than run at once
   dim3 grid(a.skip_dense ? std::min(items, std::max(1, sm_count() / groups)) : items, groups, TQ == 1 && a.splits > 1 ? a.splits : 1);
-  latent_attn_mma_kernel<NT2, TQ><<<grid, kMmaThreads, smem, st>>>(a, DPS, DP16);
+  NVLLM_CUDA(launch_plain(latent_attn_mma_kernel<NT2, TQ>, dim3(grid), dim3(kMmaThreads), smem, st, a, DPS, DP16));
   NVLLM_LAUNCH_CHECK("latent_attn_mma_kernel");
   if (TQ == 1 && a.splits > 1) {
-    latent_attn_merge_kernel<<<static_cast<unsigned>((static_cast<int64_t>(a.n) * a.heads + 3) / 4), 128, 0, st>>>(a);
+    NVLLM_CUDA(launch_pdl(latent_attn_merge_kernel, dim3(static_cast<unsigned>((static_cast<int64_t>(a.n) * a.heads + 3) / 4)), dim3(128), 0, st, a));
     NVLLM_LAUNCH_CHECK("latent_attn_merge_kernel");
   }
   return 0;
@@ -756,11 +768,11 @@ extern "C" int nvllm_latent_norm_store(void* cq, int64_t ldcq, const float* proj
   const bool vec = q_rank % 4 == 0 && kv_rank % 4 == 0 && kv_off % 4 == 0 && ldp % 4 == 0 && ldcq % 4 == 0 && cache_row % 4 == 0 && aligned16(proj) &&
                    aligned16(cq) && aligned16(cache) && aligned16(dense) && aligned16(dq_norm_w) && aligned16(c_norm_w);
   if (dtype == NVLLM_BF16) {
-    if (vec) latent_norm_store_kernel<bf16, true><<<grid, 128, 0, st>>>(a);
-    else latent_norm_store_kernel<bf16, false><<<grid, 128, 0, st>>>(a);
+    if (vec) NVLLM_CUDA(launch_pdl(latent_norm_store_kernel<bf16, true>, dim3(grid), dim3(128), 0, st, a));
+    else NVLLM_CUDA(launch_pdl(latent_norm_store_kernel<bf16, false>, dim3(grid), dim3(128), 0, st, a));
   } else {
-    if (vec) latent_norm_store_kernel<float, true><<<grid, 128, 0, st>>>(a);
-    else latent_norm_store_kernel<float, false><<<grid, 128, 0, st>>>(a);
+    if (vec) NVLLM_CUDA(launch_pdl(latent_norm_store_kernel<float, true>, dim3(grid), dim3(128), 0, st, a));
+    else NVLLM_CUDA(launch_pdl(latent_norm_store_kernel<float, false>, dim3(grid), dim3(128), 0, st, a));
   }
   NVLLM_LAUNCH_CHECK("latent_norm_store_kernel");
   return 0;
@@ -781,9 +793,9 @@ extern "C" int nvllm_rotate_tail(void* x, int64_t ldx, const int64_t* positions,
   const unsigned grid = static_cast<unsigned>(blocks);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const float2* tab = reinterpret_cast<const float2*>(rope_table);
-  if (vec) rotate_tail_kernel<bf16, 4><<<grid, 256, 0, st>>>(static_cast<bf16*>(x), ldx, positions, tab, max_pos, n, heads, dim, rot_dim, half);
-  else if (dtype == NVLLM_BF16) rotate_tail_kernel<bf16, 1><<<grid, 256, 0, st>>>(static_cast<bf16*>(x), ldx, positions, tab, max_pos, n, heads, dim, rot_dim, half);
-  else rotate_tail_kernel<float, 1><<<grid, 256, 0, st>>>(static_cast<float*>(x), ldx, positions, tab, max_pos, n, heads, dim, rot_dim, half);
+  if (vec) NVLLM_CUDA(launch_pdl(rotate_tail_kernel<bf16, 4>, dim3(grid), dim3(256), 0, st, static_cast<bf16*>(x), ldx, positions, tab, max_pos, n, heads, dim, rot_dim, half));
+  else if (dtype == NVLLM_BF16) NVLLM_CUDA(launch_pdl(rotate_tail_kernel<bf16, 1>, dim3(grid), dim3(256), 0, st, static_cast<bf16*>(x), ldx, positions, tab, max_pos, n, heads, dim, rot_dim, half));
+  else NVLLM_CUDA(launch_pdl(rotate_tail_kernel<float, 1>, dim3(grid), dim3(256), 0, st, static_cast<float*>(x), ldx, positions, tab, max_pos, n, heads, dim, rot_dim, half));
   NVLLM_LAUNCH_CHECK("rotate_tail_kernel");
   return 0;
 }
@@ -803,8 +815,8 @@ extern "C" int nvllm_latent_prepare(void* q, int64_t ldq, const void* dkv, int64
   const PrepArgs a{q, ldq, dkv, lddkv, c_norm_w, eps, positions, reinterpret_cast<const float2*>(rope_table), rot_dims, max_pos,
                    n, heads, dim, rot_dim, kv_rank, cache, cache_row, slots};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (dtype == NVLLM_BF16) latent_prepare_kernel<bf16><<<(n + 3) / 4, 128, 0, st>>>(a);
-  else latent_prepare_kernel<float><<<(n + 3) / 4, 128, 0, st>>>(a);
+  if (dtype == NVLLM_BF16) NVLLM_CUDA(launch_pdl(latent_prepare_kernel<bf16>, dim3((n + 3) / 4), dim3(128), 0, st, a));
+  else NVLLM_CUDA(launch_pdl(latent_prepare_kernel<float>, dim3((n + 3) / 4), dim3(128), 0, st, a));
   NVLLM_LAUNCH_CHECK("latent_prepare_kernel");
   return 0;
 }
@@ -849,8 +861,9 @@ extern "C" int nvllm_latent_window_attention(void* out, int64_t ldo, const float
     }
     // Single tokens on fewer CTAs than SMs: the key tiles of a token are split over CTAs along z, as many as fill the SMs once and
     // leave each (at the longest context the tables or the window allow) at least four tiles; the partials meet in
-    // latent_attn_merge_kernel.  Measured, 32 tokens x 16 heads at 4001 keys, rank 512: 223 -> 104 us.  64 tokens in a window of 2048 keys 118 -> 79 us; in one of 512 the second launch costs what the shorter loop saves (39 -> 37 us), hence eight
-    // tiles for windows.
+    // latent_attn_merge_kernel.  Measured, 32 tokens x 16 heads at 4001 keys, rank 512: 223 -> 104 us.  64 tokens in a window of
+    // 2048 keys 118 -> 79 us; in one of 512 the second launch costs what the shorter loop saves (39 -> 37 us), hence eight tiles for
+    // windows.
     if (workspace != nullptr && n <= 256) {
       const int64_t ctas = static_cast<int64_t>(n) * ((heads + 15) / 16);
       const int64_t reach = window > 0 ? window + kMmaKeys - 1 : static_cast<int64_t>(table_cap) * block_size;

@@ -56,6 +56,8 @@ __device__ __forceinline__ Span span_of(const LatentAttnArgs& a, int t0, int ten
 }
 
 __global__ void __launch_bounds__(kThreads, 1) latent_attn_tc_kernel(const LatentAttnArgs a, int halves) {
+  pdl_wait();
+  pdl_launch_dependents();
   extern __shared__ uint8_t smem_raw[];
   const int tile = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);   // late tokens of the batch (most keys) first
   if (!latent_tile_dense(a.tok_seq, a.n, tile)) return;
@@ -223,9 +225,9 @@ __global__ void __launch_bounds__(kThreads, 1) latent_attn_tc_kernel(const Laten
       int js = 0, jp = 0;
       long long t0 = clock64();
       while (jp < total) {
-        if (js < total && js <= jp + 1 && mbar_try_wait(k_full(js & 1), (js >> 1) & 1)) {
+        if (js < total && js <= jp + 1 && mbar_test_wait(k_full(js & 1), (js >> 1) & 1)) {
           issue_s(js++);
-        } else if (jp < js && mbar_try_wait(p_ready(jp & 1), (jp >> 1) & 1)) {
+        } else if (jp < js && mbar_test_wait(p_ready(jp & 1), (jp >> 1) & 1)) {
           const int in1 = jp - halves * tiles[0], span_tiles = in1 < 0 ? tiles[0] : tiles[1], in = in1 < 0 ? jp : in1;
           issue_pv(jp, half0 + in / span_tiles, in % span_tiles == 0);
           ++jp;
@@ -371,7 +373,7 @@ int latent_attn_tc_launch(const LatentAttnArgs& a, cudaStream_t st) {
   // One CTA per (tile, head group) walks both halves of the latent values on one copy of the queries; where that leaves SMs without
   // a CTA the halves are CTAs of their own.
   const bool split = static_cast<int64_t>(tiles) * groups * 2 <= sm_count();
-  latent_attn_tc_kernel<<<dim3(tiles, groups, split ? 2 : 1), kThreads, kSmemBytes, st>>>(a, split ? 1 : 2);
+  NVLLM_CUDA(launch_pdl(latent_attn_tc_kernel, dim3(tiles, groups, split ? 2 : 1), dim3(kThreads), kSmemBytes, st, a, split ? 1 : 2));
   NVLLM_LAUNCH_CHECK("latent_attn_tc_kernel");
   return 0;
 }

@@ -34,6 +34,8 @@ constexpr int BM = 32, BN = 64, BK = 32;
 
 template <typename TI, typename TO, bool GLU>
 __global__ void __launch_bounds__(256) linear_tile_kernel(const LinArgs a) {
+  pdl_wait();
+  pdl_launch_dependents();
   __shared__ float xs[BM][BK + 1];
   __shared__ float ws[BN][BK + 1];
   __shared__ float us[GLU ? BN : 1][BK + 1];
@@ -118,6 +120,8 @@ __global__ void __launch_bounds__(256) linear_tile_kernel(const LinArgs a) {
 
 template <typename T>
 __global__ void glu_clamped_kernel(T* __restrict__ out, const T* __restrict__ gate_up, int64_t n, int ff, float limit) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int64_t total = n * ff;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -137,6 +141,8 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 }
 
 __global__ void glu_clamped_vec8_kernel(bf16* __restrict__ out, const bf16* __restrict__ gate_up, int64_t n, int ff8, float limit) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int64_t total = n * ff8;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -159,6 +165,8 @@ __device__ __forceinline__ float softplus_f(float x) { return fmaxf(x, 0.f) + lo
 // kind 3: out[i, c] = gelu_tanh(in[i, c]) * in[i, ff + c] (in: [n, 2 ff])
 template <typename T>
 __global__ void ff_activation_kernel(T* __restrict__ out, const T* __restrict__ in, int64_t n, int ff, int kind, const float* __restrict__ params) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int64_t total = n * ff;
   const float ap = kind == 2 ? softplus_f(params[0]) : 0.f, an = kind == 2 ? 0.5f + softplus_f(params[1]) : 0.f;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
@@ -182,6 +190,8 @@ __global__ void ff_activation_kernel(T* __restrict__ out, const T* __restrict__ 
 // The same for bf16 rows of 16-byte multiples: 8 values per thread and access, no division per element.
 __global__ void __launch_bounds__(256) ff_activation_vec8_kernel(bf16* __restrict__ out, const bf16* __restrict__ in, int64_t n, int ff8, int kind,
                                                                  const float* __restrict__ params) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int64_t total = n * ff8;
   const float ap = kind == 2 ? softplus_f(params[0]) : 0.f, an = kind == 2 ? 0.5f + softplus_f(params[1]) : 0.f;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
@@ -209,6 +219,8 @@ __global__ void __launch_bounds__(256) ff_activation_vec8_kernel(bf16* __restric
 // y *= sigmoid(gate), element by element, in place (y in the operand type, gate f32): VEC values per access.
 template <typename T, int VEC>
 __global__ void __launch_bounds__(256) sigmoid_gate_kernel(T* __restrict__ y, int64_t ldy, const float* __restrict__ gate, int64_t ldg, int64_t n, int cols) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int64_t total = n * (cols / VEC);
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total; i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int64_t r = i / (cols / VEC);
@@ -233,6 +245,8 @@ __global__ void __launch_bounds__(256) sigmoid_gate_kernel(T* __restrict__ y, in
 template <typename T>
 __global__ void __launch_bounds__(256) token_gate_kernel(T* __restrict__ out, const float* __restrict__ gate, int64_t ldg, const T* __restrict__ table,
                                                          int64_t ld_table, int64_t col0, const int64_t* __restrict__ ids, int vocab, int64_t n, int dim) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int64_t total = n * dim;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total; i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int64_t t = i / dim;
@@ -246,6 +260,8 @@ __global__ void __launch_bounds__(256) token_gate_kernel(T* __restrict__ out, co
 __global__ void __launch_bounds__(256) token_gate_vec8_kernel(bf16* __restrict__ out, const float* __restrict__ gate, int64_t ldg,
                                                               const bf16* __restrict__ table, int64_t ld_table, int64_t col0,
                                                               const int64_t* __restrict__ ids, int vocab, int64_t n, int dim8) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int64_t total = n * dim8;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total; i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int64_t t = i / dim8;
@@ -271,6 +287,8 @@ constexpr int MK = 64, MS = MK + 8;   // k step and the shared-memory row stride
 
 template <int BNT, typename TO>
 __global__ void __launch_bounds__(128) linear_mma_kernel(const LinArgs a) {
+  pdl_wait();
+  pdl_launch_dependents();
   __shared__ __align__(16) bf16 xs[2][64][MS];
   __shared__ __align__(16) bf16 ws[2][BNT][MS];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, tq4 = lane & 3;
@@ -340,12 +358,12 @@ int launch_mma(const LinArgs& a, int batch, int out_dtype, cudaStream_t st) {
   const int64_t ctas64 = static_cast<int64_t>((a.N + 63) / 64) * ((a.M + 63) / 64) * batch;
   if (ctas64 >= sm_count() || a.N <= 32) {
     dim3 grid((a.N + 63) / 64, (a.M + 63) / 64, batch);
-    if (out_dtype == NVLLM_BF16) linear_mma_kernel<64, bf16><<<grid, 128, 0, st>>>(a);
-    else linear_mma_kernel<64, float><<<grid, 128, 0, st>>>(a);
+    if (out_dtype == NVLLM_BF16) NVLLM_CUDA(launch_pdl(linear_mma_kernel<64, bf16>, dim3(grid), dim3(128), 0, st, a));
+    else NVLLM_CUDA(launch_pdl(linear_mma_kernel<64, float>, dim3(grid), dim3(128), 0, st, a));
   } else {
     dim3 grid((a.N + 31) / 32, (a.M + 63) / 64, batch);
-    if (out_dtype == NVLLM_BF16) linear_mma_kernel<32, bf16><<<grid, 128, 0, st>>>(a);
-    else linear_mma_kernel<32, float><<<grid, 128, 0, st>>>(a);
+    if (out_dtype == NVLLM_BF16) NVLLM_CUDA(launch_pdl(linear_mma_kernel<32, bf16>, dim3(grid), dim3(128), 0, st, a));
+    else NVLLM_CUDA(launch_pdl(linear_mma_kernel<32, float>, dim3(grid), dim3(128), 0, st, a));
   }
   NVLLM_LAUNCH_CHECK("linear_mma_kernel");
   return 0;
@@ -354,9 +372,9 @@ int launch_mma(const LinArgs& a, int batch, int out_dtype, cudaStream_t st) {
 template <bool GLU>
 int launch_tile(const LinArgs& a, int m_tiles, int batch, int dtype, int out_dtype, cudaStream_t st) {
   dim3 grid((a.N + BN - 1) / BN, m_tiles, batch);
-  if (dtype == NVLLM_BF16 && out_dtype == NVLLM_BF16) linear_tile_kernel<bf16, bf16, GLU><<<grid, 256, 0, st>>>(a);
-  else if (dtype == NVLLM_BF16) linear_tile_kernel<bf16, float, GLU><<<grid, 256, 0, st>>>(a);
-  else if (out_dtype == NVLLM_F32) linear_tile_kernel<float, float, GLU><<<grid, 256, 0, st>>>(a);
+  if (dtype == NVLLM_BF16 && out_dtype == NVLLM_BF16) NVLLM_CUDA(launch_pdl(linear_tile_kernel<bf16, bf16, GLU>, dim3(grid), dim3(256), 0, st, a));
+  else if (dtype == NVLLM_BF16) NVLLM_CUDA(launch_pdl(linear_tile_kernel<bf16, float, GLU>, dim3(grid), dim3(256), 0, st, a));
+  else if (out_dtype == NVLLM_F32) NVLLM_CUDA(launch_pdl(linear_tile_kernel<float, float, GLU>, dim3(grid), dim3(256), 0, st, a));
   else { set_error("linear: f32 operands need an f32 output"); return NVLLM_ERR_DTYPE; }
   NVLLM_LAUNCH_CHECK("linear_tile_kernel");
   return 0;
@@ -431,11 +449,11 @@ extern "C" int nvllm_glu_clamped(void* out, const void* gate_up, int32_t n, int3
   if (dtype == NVLLM_BF16 && ff % 8 == 0 && aligned16(out) && aligned16(gate_up)) {
     int64_t b8 = (total / 8 + 255) / 256;
     if (b8 > sm_count() * 16) b8 = sm_count() * 16;
-    glu_clamped_vec8_kernel<<<static_cast<unsigned>(b8), 256, 0, st>>>(static_cast<bf16*>(out), static_cast<const bf16*>(gate_up), n, ff / 8, limit);
+    NVLLM_CUDA(launch_pdl(glu_clamped_vec8_kernel, dim3(static_cast<unsigned>(b8)), dim3(256), 0, st, static_cast<bf16*>(out), static_cast<const bf16*>(gate_up), n, ff / 8, limit));
   } else if (dtype == NVLLM_BF16)
-    glu_clamped_kernel<bf16><<<static_cast<unsigned>(blocks), 256, 0, st>>>(static_cast<bf16*>(out), static_cast<const bf16*>(gate_up), n, ff, limit);
+    NVLLM_CUDA(launch_pdl(glu_clamped_kernel<bf16>, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, st, static_cast<bf16*>(out), static_cast<const bf16*>(gate_up), n, ff, limit));
   else if (dtype == NVLLM_F32)
-    glu_clamped_kernel<float><<<static_cast<unsigned>(blocks), 256, 0, st>>>(static_cast<float*>(out), static_cast<const float*>(gate_up), n, ff, limit);
+    NVLLM_CUDA(launch_pdl(glu_clamped_kernel<float>, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, st, static_cast<float*>(out), static_cast<const float*>(gate_up), n, ff, limit));
   else NVLLM_CHECK_ARG(false, NVLLM_ERR_DTYPE, "glu_clamped: dtype %d", dtype);
   NVLLM_LAUNCH_CHECK("glu_clamped_kernel");
   return 0;
@@ -460,12 +478,12 @@ extern "C" int nvllm_ff_activation_params(void* out, const void* in, int32_t n, 
   if (dtype == NVLLM_BF16 && ff % 8 == 0 && aligned16(out) && aligned16(in)) {
     int64_t b8 = (total / 8 + 255) / 256;
     if (b8 > sm_count() * 16) b8 = sm_count() * 16;
-    ff_activation_vec8_kernel<<<static_cast<unsigned>(b8), 256, 0, st>>>(static_cast<bf16*>(out), static_cast<const bf16*>(in), n, ff / 8, kind, params);
+    NVLLM_CUDA(launch_pdl(ff_activation_vec8_kernel, dim3(static_cast<unsigned>(b8)), dim3(256), 0, st, static_cast<bf16*>(out), static_cast<const bf16*>(in), n, ff / 8, kind, params));
     NVLLM_LAUNCH_CHECK("ff_activation_vec8_kernel");
     return 0;
   }
-  if (dtype == NVLLM_BF16) ff_activation_kernel<bf16><<<static_cast<unsigned>(blocks), 256, 0, st>>>(static_cast<bf16*>(out), static_cast<const bf16*>(in), n, ff, kind, params);
-  else ff_activation_kernel<float><<<static_cast<unsigned>(blocks), 256, 0, st>>>(static_cast<float*>(out), static_cast<const float*>(in), n, ff, kind, params);
+  if (dtype == NVLLM_BF16) NVLLM_CUDA(launch_pdl(ff_activation_kernel<bf16>, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, st, static_cast<bf16*>(out), static_cast<const bf16*>(in), n, ff, kind, params));
+  else NVLLM_CUDA(launch_pdl(ff_activation_kernel<float>, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, st, static_cast<float*>(out), static_cast<const float*>(in), n, ff, kind, params));
   NVLLM_LAUNCH_CHECK("ff_activation_kernel");
   return 0;
 }
@@ -480,9 +498,9 @@ extern "C" int nvllm_sigmoid_gate(void* y, int64_t ldy, const float* gate, int64
   if (blocks > sm_count() * 16) blocks = sm_count() * 16;
   const unsigned grid = static_cast<unsigned>(blocks);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (vec) sigmoid_gate_kernel<bf16, 8><<<grid, 256, 0, st>>>(static_cast<bf16*>(y), ldy, gate, ldg, n, cols);
-  else if (dtype == NVLLM_BF16) sigmoid_gate_kernel<bf16, 1><<<grid, 256, 0, st>>>(static_cast<bf16*>(y), ldy, gate, ldg, n, cols);
-  else sigmoid_gate_kernel<float, 1><<<grid, 256, 0, st>>>(static_cast<float*>(y), ldy, gate, ldg, n, cols);
+  if (vec) NVLLM_CUDA(launch_pdl(sigmoid_gate_kernel<bf16, 8>, dim3(grid), dim3(256), 0, st, static_cast<bf16*>(y), ldy, gate, ldg, n, cols));
+  else if (dtype == NVLLM_BF16) NVLLM_CUDA(launch_pdl(sigmoid_gate_kernel<bf16, 1>, dim3(grid), dim3(256), 0, st, static_cast<bf16*>(y), ldy, gate, ldg, n, cols));
+  else NVLLM_CUDA(launch_pdl(sigmoid_gate_kernel<float, 1>, dim3(grid), dim3(256), 0, st, static_cast<float*>(y), ldy, gate, ldg, n, cols));
   NVLLM_LAUNCH_CHECK("sigmoid_gate_kernel");
   return 0;
 }
@@ -500,11 +518,11 @@ extern "C" int nvllm_token_gate(void* out, const float* gate, int64_t ldg, const
   const unsigned grid = static_cast<unsigned>(blocks);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (vec)
-    token_gate_vec8_kernel<<<grid, 256, 0, st>>>(static_cast<bf16*>(out), gate, ldg, static_cast<const bf16*>(table), ld_table, col0, ids, vocab, n, dim / 8);
+    NVLLM_CUDA(launch_pdl(token_gate_vec8_kernel, dim3(grid), dim3(256), 0, st, static_cast<bf16*>(out), gate, ldg, static_cast<const bf16*>(table), ld_table, col0, ids, vocab, n, dim / 8));
   else if (dtype == NVLLM_BF16)
-    token_gate_kernel<bf16><<<grid, 256, 0, st>>>(static_cast<bf16*>(out), gate, ldg, static_cast<const bf16*>(table), ld_table, col0, ids, vocab, n, dim);
+    NVLLM_CUDA(launch_pdl(token_gate_kernel<bf16>, dim3(grid), dim3(256), 0, st, static_cast<bf16*>(out), gate, ldg, static_cast<const bf16*>(table), ld_table, col0, ids, vocab, n, dim));
   else
-    token_gate_kernel<float><<<grid, 256, 0, st>>>(static_cast<float*>(out), gate, ldg, static_cast<const float*>(table), ld_table, col0, ids, vocab, n, dim);
+    NVLLM_CUDA(launch_pdl(token_gate_kernel<float>, dim3(grid), dim3(256), 0, st, static_cast<float*>(out), gate, ldg, static_cast<const float*>(table), ld_table, col0, ids, vocab, n, dim));
   NVLLM_LAUNCH_CHECK("token_gate_kernel");
   return 0;
 }

@@ -24,6 +24,8 @@ template <> __device__ __forceinline__ void stf<bf16>(bf16* p, float v) { *p = _
 __global__ void __launch_bounds__(128) moe_route_kernel(int32_t* __restrict__ idx, float* __restrict__ wts,
                                                         const float* __restrict__ logits, const float* __restrict__ bias,
                                                         int n, int e_total, int top, float scale) {
+  pdl_wait();
+  pdl_launch_dependents();
   extern __shared__ float sm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * 4 + warp;
@@ -73,6 +75,8 @@ __global__ void __launch_bounds__(128) moe_route_kernel(int32_t* __restrict__ id
 __global__ void __launch_bounds__(128) moe_route_logits_kernel(int32_t* __restrict__ idx, float* __restrict__ wts,
                                                                const float* __restrict__ logits, const float* __restrict__ bias,
                                                                int64_t ld, int n, int e_total, int top) {
+  pdl_wait();
+  pdl_launch_dependents();
   extern __shared__ float sm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * 4 + warp;
@@ -117,6 +121,8 @@ __global__ void __launch_bounds__(128) moe_route_logits_kernel(int32_t* __restri
 __global__ void __launch_bounds__(128) moe_route_sigmoid_kernel(int32_t* __restrict__ idx, float* __restrict__ wts,
                                                                 const float* __restrict__ logits, const float* __restrict__ bias,
                                                                 int64_t ld, int n, int e_total, int top) {
+  pdl_wait();
+  pdl_launch_dependents();
   extern __shared__ float sm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * 4 + warp;
@@ -158,6 +164,8 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(int32_t* __restrict__ ro
                                                         int32_t* __restrict__ slot_row, float* __restrict__ row_weight,
                                                         const int32_t* __restrict__ idx, const float* __restrict__ wts,
                                                         int n_assign, int top, int experts, int max_rows, int tile) {
+  pdl_wait();
+  pdl_launch_dependents();
   extern __shared__ int32_t sh[];
   int32_t* cnt = sh;             // [experts]
   int32_t* off = sh + experts;   // [experts + 1]
@@ -200,6 +208,8 @@ __global__ void moe_combine_kernel(T* __restrict__ out, const T* __restrict__ ex
                                    const T* __restrict__ shared_out, const int32_t* __restrict__ idx,
                                    const float* __restrict__ wts, const int32_t* __restrict__ slot_row, int n, int hidden,
                                    int top, int experts) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int64_t total = static_cast<int64_t>(n) * hidden;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -230,6 +240,8 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 __global__ void moe_combine_vec8_kernel(bf16* __restrict__ out, const bf16* __restrict__ expert_out, const bf16* __restrict__ x,
                                         const bf16* __restrict__ shared_out, const float* __restrict__ wts,
                                         const int32_t* __restrict__ slot_row, int n, int hidden8, int top) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int64_t total = static_cast<int64_t>(n) * hidden8;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -255,6 +267,8 @@ __global__ void moe_combine_vec8_kernel(bf16* __restrict__ out, const bf16* __re
 // Routing without a router: row ids[t] of a table names the experts of token t, each with the same weight.
 __global__ void moe_table_route_kernel(int32_t* __restrict__ topk_idx, float* __restrict__ topk_w, const int32_t* __restrict__ table,
                                        const int64_t* __restrict__ ids, int64_t n, int top, int rows, float weight) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int64_t total = n * top;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total; i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int64_t t = i / top;
@@ -276,8 +290,8 @@ extern "C" int nvllm_moe_table_route(int32_t* topk_idx, float* topk_w, const int
   if (n == 0) return 0;
   NVLLM_CHECK_ARG(topk_idx && topk_w && table && ids, NVLLM_ERR_ARG, "moe_table_route: NULL");
   const int64_t total = static_cast<int64_t>(n) * top;
-  moe_table_route_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(topk_idx, topk_w, table, ids, n,
-                                                                                                               top, table_rows, 1.0f / top);
+  NVLLM_CUDA(launch_pdl(moe_table_route_kernel, dim3(static_cast<unsigned>((total + 255) / 256)), dim3(256), 0, static_cast<cudaStream_t>(stream), topk_idx, topk_w, table, ids, n,
+                                                                                                               top, table_rows, 1.0f / top));
   NVLLM_LAUNCH_CHECK("moe_table_route_kernel");
   return 0;
 }
@@ -289,7 +303,7 @@ extern "C" int nvllm_moe_route(int32_t* topk_idx, float* topk_w, const float* lo
   if (n == 0) return 0;
   NVLLM_CHECK_ARG(topk_idx && topk_w && logits, NVLLM_ERR_ARG, "moe_route: NULL");
   const size_t smem = static_cast<size_t>(4) * 2 * e_total * sizeof(float);
-  moe_route_kernel<<<(n + 3) / 4, 128, smem, static_cast<cudaStream_t>(stream)>>>(topk_idx, topk_w, logits, bias, n, e_total, top, scale);
+  NVLLM_CUDA(launch_pdl(moe_route_kernel, dim3((n + 3) / 4), dim3(128), smem, static_cast<cudaStream_t>(stream), topk_idx, topk_w, logits, bias, n, e_total, top, scale));
   NVLLM_LAUNCH_CHECK("moe_route_kernel");
   return 0;
 }
@@ -301,7 +315,7 @@ extern "C" int nvllm_moe_route_logits(int32_t* topk_idx, float* topk_w, const fl
   if (n == 0) return 0;
   NVLLM_CHECK_ARG(topk_idx && topk_w && logits, NVLLM_ERR_ARG, "moe_route_logits: NULL");
   const size_t smem = static_cast<size_t>(4) * experts * sizeof(float);
-  moe_route_logits_kernel<<<(n + 3) / 4, 128, smem, static_cast<cudaStream_t>(stream)>>>(topk_idx, topk_w, logits, bias, ld, n, experts, top);
+  NVLLM_CUDA(launch_pdl(moe_route_logits_kernel, dim3((n + 3) / 4), dim3(128), smem, static_cast<cudaStream_t>(stream), topk_idx, topk_w, logits, bias, ld, n, experts, top));
   NVLLM_LAUNCH_CHECK("moe_route_logits_kernel");
   return 0;
 }
@@ -313,7 +327,7 @@ extern "C" int nvllm_moe_route_sigmoid(int32_t* topk_idx, float* topk_w, const f
   if (n == 0) return 0;
   NVLLM_CHECK_ARG(topk_idx && topk_w && logits, NVLLM_ERR_ARG, "moe_route_sigmoid: NULL");
   const size_t smem = static_cast<size_t>(4) * experts * sizeof(float);
-  moe_route_sigmoid_kernel<<<(n + 3) / 4, 128, smem, static_cast<cudaStream_t>(stream)>>>(topk_idx, topk_w, logits, bias, ld, n, experts, top);
+  NVLLM_CUDA(launch_pdl(moe_route_sigmoid_kernel, dim3((n + 3) / 4), dim3(128), smem, static_cast<cudaStream_t>(stream), topk_idx, topk_w, logits, bias, ld, n, experts, top));
   NVLLM_LAUNCH_CHECK("moe_route_sigmoid_kernel");
   return 0;
 }
@@ -339,8 +353,8 @@ extern "C" int nvllm_moe_sort_weighted(int32_t* row_token, float* row_weight, in
   if (n == 0) return 0;
   NVLLM_CHECK_ARG(row_token && tile_expert && slot_row && topk_idx, NVLLM_ERR_ARG, "moe_sort: NULL");
   const size_t smem = (2 * static_cast<size_t>(experts) + 1) * sizeof(int32_t);
-  moe_sort_kernel<<<1, 1024, smem, static_cast<cudaStream_t>(stream)>>>(row_token, tile_expert, slot_row, row_weight, topk_idx, topk_w, n * top, top,
-                                                                      experts, max_rows, tile_rows);
+  NVLLM_CUDA(launch_pdl(moe_sort_kernel, dim3(1), dim3(1024), smem, static_cast<cudaStream_t>(stream), row_token, tile_expert, slot_row, row_weight, topk_idx, topk_w, n * top, top,
+                                                                      experts, max_rows, tile_rows));
   NVLLM_LAUNCH_CHECK("moe_sort_kernel");
   return 0;
 }
@@ -359,17 +373,17 @@ extern "C" int nvllm_moe_combine(void* out, const void* expert_out, const void* 
   if (dtype == NVLLM_BF16 && hidden % 8 == 0 && aligned16(out) && aligned16(expert_out) && aligned16(x) && aligned16(shared_out)) {
     int64_t b8 = (total / 8 + 255) / 256;
     if (b8 > sm_count() * 16) b8 = sm_count() * 16;
-    moe_combine_vec8_kernel<<<static_cast<unsigned>(b8), 256, 0, st>>>(static_cast<bf16*>(out), static_cast<const bf16*>(expert_out),
+    NVLLM_CUDA(launch_pdl(moe_combine_vec8_kernel, dim3(static_cast<unsigned>(b8)), dim3(256), 0, st, static_cast<bf16*>(out), static_cast<const bf16*>(expert_out),
                                                                       static_cast<const bf16*>(x), static_cast<const bf16*>(shared_out),
-                                                                      topk_w, slot_row, n, hidden / 8, top);
+                                                                      topk_w, slot_row, n, hidden / 8, top));
   } else if (dtype == NVLLM_BF16)
-    moe_combine_kernel<bf16><<<static_cast<unsigned>(blocks), 256, 0, st>>>(
+    NVLLM_CUDA(launch_pdl(moe_combine_kernel<bf16>, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, st, 
         static_cast<bf16*>(out), static_cast<const bf16*>(expert_out), static_cast<const bf16*>(x),
-        static_cast<const bf16*>(shared_out), topk_idx, topk_w, slot_row, n, hidden, top, experts);
+        static_cast<const bf16*>(shared_out), topk_idx, topk_w, slot_row, n, hidden, top, experts));
   else
-    moe_combine_kernel<float><<<static_cast<unsigned>(blocks), 256, 0, st>>>(
+    NVLLM_CUDA(launch_pdl(moe_combine_kernel<float>, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, st, 
         static_cast<float*>(out), static_cast<const float*>(expert_out), static_cast<const float*>(x),
-        static_cast<const float*>(shared_out), topk_idx, topk_w, slot_row, n, hidden, top, experts);
+        static_cast<const float*>(shared_out), topk_idx, topk_w, slot_row, n, hidden, top, experts));
   NVLLM_LAUNCH_CHECK("moe_combine_kernel");
   return 0;
 }
