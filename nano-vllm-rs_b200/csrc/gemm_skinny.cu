@@ -10,7 +10,7 @@
 //   norm_w    x is the residual stream and every CTA normalises its own copy of the few rows (rms(x) * w rounded to bf16)
 //   GATE      w = [gate | up]; the CTA computes the matching rows of both and writes silu(gate) * up
 //   residual  y = bf16(y + bf16(x . w^T)): the projection's output goes into the stream in place
-// Measured, a decode step of one token (Qwen3-0.6B, 28 layers, graph replay): 1408 us on the tcgen05 kernels, 862 with these; 28 layers of
+// Measured, a decode step of one token (Qwen3-0.6B, 28 layers, graph replay): 1408 us on the tcgen05 kernels, 825 with these; 28 layers of
 // weights and the head take 180 us at the copy rate, the rest is latency: 143 dependent launches of 5-6 us.
 #include "tc.cuh"
 
@@ -187,7 +187,7 @@ template <int NT>
 int skinny_rows(const SkinnyArgs& a, bool gate, int out_dtype, cudaStream_t st) {
   // 8-row CTAs where 16-row ones would leave SMs without work; k-blocks ahead: all of a warp's up to K = 1024 (narrow outputs: 3072)
   if (gate) return skinny_run<NT, 16, 4, true, bf16>(a, st);
-  if (out_dtype == NVLLM_F32) return skinny_run<NT, 16, 4, false, float>(a, st);
+  if (out_dtype == NVLLM_F32) return skinny_run<NT, 16, 2, false, float>(a, st);   // heads: many CTAs, bound by bytes in flight: four on an SM
   if ((a.n + 15) / 16 < sm_count()) return skinny_run<NT, 8, 12, false, bf16>(a, st);
   return skinny_run<NT, 16, 4, false, bf16>(a, st);
 }
