@@ -664,8 +664,10 @@ int nvllm_runner::forward(int N, int S, bool is_prefill, bool paged_prefill, con
     return rc;
   };
   // Up to 16 tokens: every norm rides in the projection behind it, every residual add in the one before it (gemm_skinny.cu), so h is
-  // the stream itself throughout.
-  const bool few = tp == 1 && gemm_skinny_applies(N, hidden, hidden, hidden, hidden) && inter % 32 == 0 && HD % 32 == 0;
+  // the stream itself throughout.  The widths are those that the general path takes (it reports the others), and no more rows than
+  // tokens reach the head (a prefill batch may hold sequences without tokens).
+  const bool few = tp == 1 && gemm_skinny_applies(N, hidden, hidden, hidden, hidden) && hidden % 64 == 0 && inter % 64 == 0 && HD % 64 == 0 &&
+                   vshard % 8 == 0 && S <= N;
   auto few_gemm = [&](void* y, const void* x, const void* w, int rows_n, int n, int k, int64_t ldy, int out_dt, bool gate, const bf16* norm, bool residual, const char* what) {
     ++launches;
     const int rc = gemm_skinny(y, x, w, rows_n, n, k, k, k, ldy, out_dt, gate, norm, eps, residual, stream);
