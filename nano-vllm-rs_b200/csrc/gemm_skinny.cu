@@ -10,7 +10,7 @@
 //   norm_w    x is the residual stream and every CTA normalises its own copy of the few rows (rms(x) * w rounded to bf16)
 //   GATE      w = [gate | up]; the CTA computes the matching rows of both and writes silu(gate) * up
 //   residual  y = bf16(y + bf16(x . w^T)): the projection's output goes into the stream in place
-// Measured, a decode step of one token (Qwen3-0.6B, 28 layers, graph replay): 1408 us on the tcgen05 kernels, 825 with these; 28 layers of
+// Measured, a decode step of one token (Qwen3-0.6B, 28 layers, graph replay): 1408 us on the tcgen05 kernels, 791 with these; 28 layers of
 // weights and the head take 180 us at the copy rate, the rest is latency: 143 dependent launches of 5-6 us.
 #include "tc.cuh"
 
@@ -175,6 +175,124 @@ __global__ void __launch_bounds__(kSkThreads, sizeof(OutT) == 4 && NT == 1 ? 4 :
   }
 }
 
+// Heads (f32 out, many rows): the same products by CTAs that stay.  x is normed once per CTA and kept in shared memory, and a warp's
+// weight loads run kHeadPre blocks ahead across the edges of its 16-row tiles, so that HBM never waits for a tile's prologue or its sum.
+// Bound by HBM.  Measured, 1 x 1024 by 151936 rows (311 MB, 47 us at the copy rate): 81 us with a CTA per tile, 54 so.  Launched
+// plainly: CTAs that stay and start early share SMs unevenly (a decode step of one token 838 us early, 797 plainly, 824 before).
+constexpr int kHeadPre = 4, kHeadCtas = 3, kHeadSmem = 72 * 1024;
+template <int NT>
+constexpr int head_red_bytes() { return 2 * kSkWarps * NT * 8 * 17 * 4; }
+
+template <int NT>
+__global__ void __launch_bounds__(kSkThreads, kHeadCtas) gemm_skinny_head_kernel(const SkinnyArgs a) {
+  extern __shared__ __align__(16) uint8_t head_smem[];
+  __shared__ float ssq[kSkWarps][NT * 8];
+  float* red = reinterpret_cast<float*>(head_smem);   // [2][warp][token][17]: one barrier a tile
+  bf16* xs = reinterpret_cast<bf16*>(head_smem + head_red_bytes<NT>());
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+  const int nkb = a.k / 32, nb = (nkb + kSkWarps - 1) / kSkWarps, tiles = (a.n + 15) / 16, step = static_cast<int>(gridDim.x);
+  const int pitch = a.k + 32;   // rows 64 bytes apart in the banks
+  int lt = blockIdx.x, lb = 0;  // the next block to load
+  auto load = [&](uint4 (&f)[2]) {
+    const int kb = warp + lb * kSkWarps;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = 16 * lt + 8 * h + g;
+      f[h] = (lt < tiles && r < a.n && kb < nkb) ? ld_nc_stream(a.w + static_cast<int64_t>(r) * a.ldw + kb * 32 + 8 * t4) : make_uint4(0, 0, 0, 0);
+    }
+    if (++lb == nb) { lb = 0; lt += step; }
+  };
+  uint4 wf[kHeadPre][2];
+#pragma unroll
+  for (int p = 0; p < kHeadPre; ++p) load(wf[p]);
+  pdl_launch_dependents();
+#pragma unroll
+  for (int j = 0; j < NT; ++j) {
+    float ss = 0.f;
+    if (8 * j + g < a.m)
+      for (int kb = warp; kb < nkb; kb += kSkWarps) {
+        const uint4 v = *reinterpret_cast<const uint4*>(a.x + (8 * j + g) * a.ldx + kb * 32 + 8 * t4);
+        *reinterpret_cast<uint4*>(xs + (8 * j + g) * pitch + kb * 32 + 8 * t4) = v;
+        const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+        float s = 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s += bf16_lo(u[e]) * bf16_lo(u[e]) + bf16_hi(u[e]) * bf16_hi(u[e]);
+        ss += s;
+      }
+    ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+    ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+    if (t4 == 0) ssq[warp][8 * j + g] = ss;
+  }
+  __syncthreads();
+  if (a.norm_w != nullptr) {   // every thread norms the values that it stored
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      if (8 * j + g >= a.m) continue;
+      float s = 0.f;
+#pragma unroll
+      for (int i = 0; i < kSkWarps; ++i) s += ssq[i][8 * j + g];
+      const float inv = 1.0f / sqrtf(s / static_cast<float>(a.k) + a.eps);
+      for (int kb = warp; kb < nkb; kb += kSkWarps) {
+        uint4* at = reinterpret_cast<uint4*>(xs + (8 * j + g) * pitch + kb * 32 + 8 * t4);
+        const uint4 v = *at, nv = __ldg(reinterpret_cast<const uint4*>(a.norm_w + kb * 32 + 8 * t4));
+        uint32_t u[4] = {v.x, v.y, v.z, v.w};
+        const uint32_t nw[4] = {nv.x, nv.y, nv.z, nv.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) u[e] = pack_bf16x2(bf16_lo(u[e]) * inv * bf16_lo(nw[e]), bf16_hi(u[e]) * inv * bf16_hi(nw[e]));
+        *at = make_uint4(u[0], u[1], u[2], u[3]);
+      }
+    }
+  }
+  // (a lane reads back, below, only blocks that it stored itself)
+  float acc[NT][4] = {};
+  int tile = blockIdx.x, b = 0, buf = 0;
+  while (tile < tiles) {
+#pragma unroll
+    for (int p = 0; p < kHeadPre; ++p) {
+      if (tile >= tiles) break;   // (the same for all threads of the CTA)
+      const int kb = warp + b * kSkWarps;
+      if (kb < nkb) {
+        const uint32_t a0[4] = {wf[p][0].x, wf[p][1].x, wf[p][0].y, wf[p][1].y}, a1[4] = {wf[p][0].z, wf[p][1].z, wf[p][0].w, wf[p][1].w};
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+          const uint4 xf = 8 * j + g < a.m ? *reinterpret_cast<const uint4*>(xs + (8 * j + g) * pitch + kb * 32 + 8 * t4) : make_uint4(0, 0, 0, 0);
+          mma_bf16_16816(acc[j], a0, xf.x, xf.y);
+          mma_bf16_16816(acc[j], a1, xf.z, xf.w);
+        }
+      }
+      load(wf[p]);   // (nothing beyond the last tile)
+      if (++b < nb) continue;
+      float* rb = red + buf * kSkWarps * NT * 8 * 17;
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          rb[(warp * NT * 8 + 8 * j + 2 * t4 + (e & 1)) * 17 + g + 8 * (e >> 1)] = acc[j][e];
+          acc[j][e] = 0.f;
+        }
+      __syncthreads();
+      for (int e = threadIdx.x; e < 16 * a.m; e += kSkThreads) {
+        const int t = e / 16, r = e - t * 16;
+        if (16 * tile + r >= a.n) continue;
+        float s = 0.f;
+#pragma unroll
+        for (int wv = 0; wv < kSkWarps; ++wv) s += rb[(wv * NT * 8 + t) * 17 + r];
+        static_cast<float*>(a.y)[t * a.ldy + 16 * tile + r] = s;
+      }
+      b = 0;
+      buf ^= 1;
+      tile += step;
+    }
+  }
+}
+
+template <int NT>
+int skinny_head(const SkinnyArgs& a, cudaStream_t st) {
+  NVLLM_SMEM_ATTR_ONCE(gemm_skinny_head_kernel<NT>, kHeadSmem);
+  NVLLM_CUDA(launch_plain(gemm_skinny_head_kernel<NT>, dim3(kHeadCtas * sm_count()), dim3(kSkThreads), head_red_bytes<NT>() + a.m * (a.k + 32) * 2, st, a));
+  return 0;
+}
+
 template <int NT, int ROWS, int PRE, bool GATE, typename OutT>
 int skinny_run(const SkinnyArgs& a, cudaStream_t st) {
   const dim3 grid((a.n + ROWS - 1) / ROWS);
@@ -187,6 +305,9 @@ template <int NT>
 int skinny_rows(const SkinnyArgs& a, bool gate, int out_dtype, cudaStream_t st) {
   // 8-row CTAs where 16-row ones would leave SMs without work; k-blocks ahead: all of a warp's up to K = 1024 (narrow outputs: 3072)
   if (gate) return skinny_run<NT, 16, 4, true, bf16>(a, st);
+  // heads: CTAs that stay where each has two tiles or more and the rows of x fit three times into an SM's shared memory
+  if (out_dtype == NVLLM_F32 && a.n >= 2 * 16 * kHeadCtas * sm_count() && head_red_bytes<NT>() + a.m * (static_cast<int64_t>(a.k) + 32) * 2 <= kHeadSmem)
+    return skinny_head<NT>(a, st);
   if (out_dtype == NVLLM_F32) return skinny_run<NT, 16, 2, false, float>(a, st);   // heads: many CTAs, bound by bytes in flight: four on an SM
   if ((a.n + 15) / 16 < sm_count()) return skinny_run<NT, 8, 12, false, bf16>(a, st);
   return skinny_run<NT, 16, 4, false, bf16>(a, st);

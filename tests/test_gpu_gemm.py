@@ -239,9 +239,10 @@ def test_gemm_x_multicast_clusters_opt_in(cuda, m, n, k, monkeypatch):
 
 
 @pytest.mark.parametrize("m", [1, 7, 8, 9, 16])
-@pytest.mark.parametrize("n,k", [(8, 64), (1000, 192), (1024, 3072), (4104, 1024), (3072, 4096)])
+@pytest.mark.parametrize("n,k", [(8, 64), (1000, 192), (1024, 3072), (4104, 1024), (3072, 4096), (14208, 96 * 2), (14216, 1024), (31000, 1088), (14224, 4096)])
 def test_products_of_a_few_rows(cuda, m, n, k):
-    """m <= 16: weight rows on the M side of mma.sync, K split over the warps of a CTA (8- and 16-row CTAs, remainders of both)."""
+    """m <= 16: weight rows on the M side of mma.sync, K split over the warps of a CTA (8- and 16-row CTAs, remainders of both; from
+    14208 rows f32 results by CTAs that take several tiles, and rows of x that are too long for those)."""
     from nano_vllm_rs_b200 import ops
     g = torch.Generator(device=cuda).manual_seed(m * n + k)
     wide = torch.randn((m, k + 24), generator=g, device=cuda).to(torch.bfloat16)
