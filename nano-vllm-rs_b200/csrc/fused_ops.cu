@@ -342,13 +342,17 @@ __device__ __forceinline__ float to_f32(T v);
 template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; }
 template <> __device__ __forceinline__ float to_f32<bf16>(bf16 v) { return __bfloat162float(v); }
 
-template <typename T>
+// SPLIT > 1: a cluster shares a row, its first CTA merges.  Bound by what one SM reads: a row of 151936 f32 takes one CTA 16 us and
+// eight 10 (launches included).
+template <typename T, int SPLIT>
 __global__ void __launch_bounds__(1024)
 argmax_kernel(int64_t* __restrict__ out_ids, float* __restrict__ out_max, const T* __restrict__ logits,
               int vocab, int64_t ld, int64_t vocab_offset) {
   pdl_launch_dependents();
   pdl_wait();
-  const T* row = logits + blockIdx.x * ld;
+  const int part = static_cast<int>(blockIdx.x) % SPLIT, tid = part * blockDim.x + threadIdx.x, stride = SPLIT * blockDim.x;
+  const int64_t b = blockIdx.x / SPLIT;
+  const T* row = logits + b * ld;
   float best = -INFINITY;
   int bidx = 0x7fffffff;
   constexpr int VEC = 16 / sizeof(T);  // elements per 16-byte load
@@ -357,13 +361,13 @@ argmax_kernel(int64_t* __restrict__ out_ids, float* __restrict__ out_max, const 
     const uintptr_t a = reinterpret_cast<uintptr_t>(row) & 15u;
     if (a) head = min(vocab, static_cast<int>((16 - a) / sizeof(T)));
   }
-  for (int i = threadIdx.x; i < head; i += blockDim.x) {
+  for (int i = tid; i < head; i += stride) {
     const float v = to_f32<T>(row[i]);
     if (v > best || (v == best && i < bidx)) { best = v; bidx = i; }
   }
   const int nvec = (vocab - head) / VEC;
   const uint4* rv = reinterpret_cast<const uint4*>(row + head);
-  for (int j = threadIdx.x; j < nvec; j += blockDim.x) {
+  for (int j = tid; j < nvec; j += stride) {
     const uint4 q = ld_nc_16(rv + j);
     T e[VEC];
     *reinterpret_cast<uint4*>(e) = q;
@@ -374,7 +378,7 @@ argmax_kernel(int64_t* __restrict__ out_ids, float* __restrict__ out_max, const 
       if (v > best || (v == best && i < bidx)) { best = v; bidx = i; }
     }
   }
-  for (int i = head + nvec * VEC + threadIdx.x; i < vocab; i += blockDim.x) {
+  for (int i = head + nvec * VEC + tid; i < vocab; i += stride) {
     const float v = to_f32<T>(row[i]);
     if (v > best || (v == best && i < bidx)) { best = v; bidx = i; }
   }
@@ -398,11 +402,24 @@ argmax_kernel(int64_t* __restrict__ out_ids, float* __restrict__ out_max, const 
       const int oi = __shfl_xor_sync(0xffffffffu, bidx, o);
       if (ov > best || (ov == best && oi < bidx)) { best = ov; bidx = oi; }
     }
-    if (threadIdx.x == 0) {
-      if (bidx == 0x7fffffff) bidx = 0;  // all -inf / NaN row
-      out_ids[blockIdx.x] = static_cast<int64_t>(bidx) + vocab_offset;
-      if (out_max) out_max[blockIdx.x] = best;
-    }
+    if (SPLIT > 1 && threadIdx.x == 0) { sv[0] = best; si[0] = bidx; }
+  }
+  if (SPLIT > 1) {
+    __syncwarp();
+    cluster_sync();
+    if (part == 0 && threadIdx.x == 0)
+      for (int r = 1; r < SPLIT; ++r) {
+        const float ov = ld_peer_f32(smem_u32(sv), r);
+        const int oi = __float_as_int(ld_peer_f32(smem_u32(si), r));
+        if (ov > best || (ov == best && oi < bidx)) { best = ov; bidx = oi; }
+      }
+    __syncwarp();
+    cluster_sync();   // nobody leaves before its result has been read
+  }
+  if (part == 0 && threadIdx.x == 0) {
+    if (bidx == 0x7fffffff) bidx = 0;  // all -inf / NaN row
+    out_ids[b] = static_cast<int64_t>(bidx) + vocab_offset;
+    if (out_max) out_max[b] = best;
   }
 }
 
@@ -581,12 +598,19 @@ extern "C" int nvllm_argmax(int64_t* out_ids, float* out_max, const void* logits
   if (batch == 0) return 0;
   NVLLM_CHECK_ARG(out_ids && logits, NVLLM_ERR_ARG, "argmax: NULL pointer");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (logits_dtype == NVLLM_F32)
-    NVLLM_CUDA(launch_pdl(argmax_kernel<float>, dim3(batch), dim3(1024), 0, st, out_ids, out_max, static_cast<const float*>(logits), vocab, ld, vocab_offset));
-  else if (logits_dtype == NVLLM_BF16)
-    NVLLM_CUDA(launch_pdl(argmax_kernel<bf16>, dim3(batch), dim3(1024), 0, st, out_ids, out_max, static_cast<const bf16*>(logits), vocab, ld, vocab_offset));
-  else
-    NVLLM_CHECK_ARG(false, NVLLM_ERR_DTYPE, "argmax: dtype %d", logits_dtype);
+  NVLLM_CHECK_ARG(logits_dtype == NVLLM_F32 || logits_dtype == NVLLM_BF16, NVLLM_ERR_DTYPE, "argmax: dtype %d", logits_dtype);
+  const float* lf = static_cast<const float*>(logits);
+  const bf16* lb = static_cast<const bf16*>(logits);
+  constexpr int kSplit = 8;
+  // A cluster per row while all of them find an SM each and every thread has a vector to read; beyond that the rows alone fill the SMs.
+  if (batch * kSplit <= sm_count() && vocab >= kSplit * 1024 * 8) {
+    if (logits_dtype == NVLLM_F32) NVLLM_CUDA(launch_pdl_cluster(argmax_kernel<float, kSplit>, dim3(batch * kSplit), dim3(1024), kSplit, 0, st, out_ids, out_max, lf, vocab, ld, vocab_offset));
+    else NVLLM_CUDA(launch_pdl_cluster(argmax_kernel<bf16, kSplit>, dim3(batch * kSplit), dim3(1024), kSplit, 0, st, out_ids, out_max, lb, vocab, ld, vocab_offset));
+  } else if (logits_dtype == NVLLM_F32) {
+    NVLLM_CUDA(launch_pdl(argmax_kernel<float, 1>, dim3(batch), dim3(1024), 0, st, out_ids, out_max, lf, vocab, ld, vocab_offset));
+  } else {
+    NVLLM_CUDA(launch_pdl(argmax_kernel<bf16, 1>, dim3(batch), dim3(1024), 0, st, out_ids, out_max, lb, vocab, ld, vocab_offset));
+  }
   NVLLM_LAUNCH_CHECK("argmax_kernel");
   return 0;
 }

@@ -59,19 +59,6 @@ struct DecodeParams {
   int max_position;
 };
 
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-}
-// the f32 at this shared-memory address in CTA `rank` of the cluster
-__device__ __forceinline__ float ld_peer_f32(uint32_t addr, int rank) {
-  uint32_t peer;
-  float v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(peer) : "r"(addr), "r"(rank));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(peer) : "memory");
-  return v;
-}
-
 template <int D, int STAGES, int NWARPS>
 struct DecodeCfg {
   static constexpr int kChunks = D / 8;                // 16-byte chunks per row
@@ -739,19 +726,7 @@ static int launch_decode(const DecodeParams& p, cudaStream_t stream) {
     NVLLM_CUDA(once_err);
     DecodeParams q = p;
     q.cluster = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(NWARPS * 32);
-    cfg.dynamicSmemBytes = kBytes;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = p.num_splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    NVLLM_CUDA(cudaLaunchKernelEx(&cfg, kern, q));
+    NVLLM_CUDA(launch_pdl_cluster(kern, grid, dim3(NWARPS * 32), static_cast<unsigned>(p.num_splits), kBytes, stream, q));
     return 0;
   }
   NVLLM_CUDA(launch_pdl(kern, grid, dim3(NWARPS * 32), kBytes, stream, p));

@@ -77,6 +77,24 @@ def test_paged_decode_attention_vs_oracle(cuda, kind, case):
     assert_close(to_np_f32(out), ref, ATT_ATOL, ATT_RTOL, f"paged decode {case}")
 
 
+@pytest.mark.parametrize("D", [64, 128])
+def test_paged_decode_splits_merge_alike(cuda, D):
+    """Every cluster size (2 to 16 splits merge inside the kernel) and the separate merge beyond it, with empty splits and an empty row."""
+    from nano_vllm_rs_b200 import ops
+    ctx, H, Hkv, bs = [1, 777, 0, 64], 8, 4, 32
+    rng = np.random.default_rng(D)
+    kc, vc, tables, _, _ = make_paged_kv(rng, ctx, bs, Hkv, D)
+    q = randn_bf16(rng, (len(ctx), H, D))
+    scale = 1.0 / np.sqrt(D)
+    ref = O.flash_attention_decode(q, kc, vc, tables, np.asarray(ctx, np.int32), scale)
+    args = (to_dev_bf16(q, cuda), cache_to_layout(kc, "head_major", cuda), cache_to_layout(vc, "head_major", cuda),
+            torch.from_numpy(tables).to(cuda), torch.tensor(ctx, dtype=torch.int32, device=cuda), _layout("head_major", bs, Hkv, D))
+    for splits in range(2, 19):
+        out = ops.paged_decode_attention(*args, scale=scale, num_splits=splits)
+        torch.cuda.synchronize()
+        assert_close(to_np_f32(out), ref, ATT_ATOL, ATT_RTOL, f"{splits} splits")
+
+
 PERSIST_CASES = [
     # (batch, max_ctx, H, Hkv, block_size): more (sequence, kv head, group) items than resident CTAs -> the persistent kernel
     (80, 700, 16, 8, 256),      # 640 items, Qwen3-0.6B heads, ragged contexts incl. empty rows
@@ -327,6 +345,25 @@ def test_argmax_first_max_bit_exact(cuda, dtype):
     comb = ops.argmax_combine(torch.stack(am), torch.stack(ai))
     torch.cuda.synchronize()
     assert np.array_equal(comb.cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,vocab", [(1, 65536), (18, 65541), (19, 65541), (3, 151936), (2, 65535)])
+def test_argmax_of_few_rows(cuda, dtype, rows, vocab):
+    """A row shared by a cluster (up to 18 rows of 65536 or more values) and its neighbours: ties over parts, winners at both ends, rows of
+    any alignment, rows without a winner."""
+    from nano_vllm_rs_b200 import ops
+    g = torch.Generator(device=cuda).manual_seed(vocab + rows)
+    t = torch.randn((rows, vocab), generator=g, device=cuda).to(dtype)
+    t[0, 0] = t[0, vocab - 1] = 60.0
+    if rows > 1:
+        t[1, vocab - 1] = 60.0
+    if rows > 2:
+        t[2] = float("-inf")
+    ids, mx = ops.argmax(t, return_max=True)
+    h = t.float().cpu().numpy()
+    assert np.array_equal(ids.cpu().numpy(), h.argmax(-1))
+    assert np.array_equal(mx.cpu().numpy(), h.max(-1))
 
 
 def test_init_weight_matches_oracle_bit_exact(cuda):
