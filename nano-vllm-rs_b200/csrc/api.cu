@@ -41,7 +41,6 @@ static void parse_knobs() {
   k.gemm_bn = num("NVLLM_GEMM_BN", 0);
   k.gemm_2cta = num("NVLLM_GEMM_2CTA", 1);
   k.gemm_skinny = num("NVLLM_GEMM_SKINNY", 1);
-  k.gemm_mcast = num("NVLLM_GEMM_MCAST", 0) == 1;
   k.gemm_stages = num("NVLLM_GEMM_STAGES", 0);
   k.sk_stages = num("NVLLM_GEMM_SK_STAGES", 0);
   if (const char* e = getenv("NVLLM_GEMM_SPLITK")) {

@@ -63,7 +63,6 @@ struct Knobs {
   int gemm_bn = 0;          // NVLLM_GEMM_BN: forced tile width (0 = heuristic)
   int gemm_2cta = 1;        // NVLLM_GEMM_2CTA: 0 never, 1 default (M > 512), 2 every M > 128
   int gemm_skinny = 1;      // NVLLM_GEMM_SKINNY: 0 keeps products of up to 16 rows on the tcgen05 kernels
-  int gemm_mcast = 0;       // NVLLM_GEMM_MCAST: 1 enables the x-multicast clusters
   int gemm_stages = 0;      // NVLLM_GEMM_STAGES: ring depth cap of single-wave launches (0 = deepest)
   int sk_stages = 0;        // NVLLM_GEMM_SK_STAGES: ring depth of the split-K kernel (0 = deepest)
   int splitk_mode = 1;      // NVLLM_GEMM_SPLITK: 0 never, 1 cost model, 2 forced (splitk_bn, splitk_sk)

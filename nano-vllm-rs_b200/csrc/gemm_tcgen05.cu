@@ -93,10 +93,7 @@ struct RopeEpi {
   float eps;
 };
 
-// CN > 1: clusters of CN CTAs along N work on the same 128-row x tile.  Each CTA loads 128/CN rows of it and MULTICASTS
-// them into all CN shared memories (L2 -> SM traffic for x drops by CN: the bound for small-N, long-K shards such as the
-// TP=8 qkv / o / down projections); a stage is released only when all CN CTAs' MMAs have retired (multicast commit).
-template <int BN, typename OutT, int GATE, int CN, bool ROPE = false>
+template <int BN, typename OutT, int GATE, bool ROPE = false>
 __global__ void __launch_bounds__(256, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                     OutT* __restrict__ y, int M, int N, int K, int64_t ldy, int num_m_tiles, int num_tiles,
@@ -121,10 +118,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int num_kb = K / C::BK;
-  // num_tiles counts CLUSTER tiles: (m_tile, group of CN consecutive n-tiles); this CTA owns n-tile group*CN + rank
-  const int rank = CN > 1 ? static_cast<int>(cluster_ctarank()) : 0;
-  const int cta0 = static_cast<int>(blockIdx.x) / CN, cta_stride = static_cast<int>(gridDim.x) / CN;
-  constexpr uint16_t kMask = static_cast<uint16_t>((1u << CN) - 1u);
+  const int cta0 = static_cast<int>(blockIdx.x), cta_stride = static_cast<int>(gridDim.x);
   pdl_launch_dependents();  // everything up to pdl_wait() below is independent of the previous kernel
 
   if (warp == 0 && lane == 0) {
@@ -134,7 +128,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
   if (warp == 1 && lane == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(full_bar(s), 1);
-      mbar_init(empty_bar(s), CN);  // every CTA of the cluster must have drained the stage before it is refilled
+      mbar_init(empty_bar(s), 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tfull_bar(a), 1);
@@ -144,7 +138,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
   }
   if (warp == 2) tmem_alloc<C::kTmemCols>(tmem_slot);
   tc_fence_before();
-  if constexpr (CN > 1) cluster_sync_all(); else __syncthreads();
+  __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
 
@@ -161,18 +155,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
       }
     };
     auto load_x = [&](int stage, int kb, int m_tile) {
-      if constexpr (CN > 1) {
-        constexpr int kRows = C::BM / CN;  // this CTA's share of the x tile, multicast to the whole cluster
-        tma_load_2d_mcast(sA + stage * C::kABytes + rank * kRows * 128, &tmap_x, full_bar(stage), kb * C::BK,
-                          m_tile * C::BM + rank * kRows, kMask);
-      } else {
-        tma_load_2d(sA + stage * C::kABytes, &tmap_x, full_bar(stage), kb * C::BK, m_tile * C::BM);
-      }
+      tma_load_2d(sA + stage * C::kABytes, &tmap_x, full_bar(stage), kb * C::BK, m_tile * C::BM);
     };
     // (grouped launches read the tile's group, which the previous kernel wrote: no weight tile before the wait)
     const int pre = tile_group != nullptr ? 0 : (num_kb < STAGES ? num_kb : STAGES);
     {
-      const int n_tile0 = (cta0 / num_m_tiles) * CN + rank;
+      const int n_tile0 = cta0 / num_m_tiles;
       for (int kb = 0; kb < pre; ++kb) {
         mbar_expect_tx(full_bar(kb), C::kStageBytes);
         load_w(kb, kb, n_tile0);
@@ -183,7 +171,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     uint32_t phase = 0;
     bool first = true;
     for (int tile = cta0; tile < num_tiles; tile += cta_stride) {
-      const int m_tile = tile % num_m_tiles, n_tile = (tile / num_m_tiles) * CN + rank;
+      const int m_tile = tile % num_m_tiles, n_tile = tile / num_m_tiles;
       int goff = 0;
       if (tile_group != nullptr) { const int g = tile_group[m_tile]; goff = (g > 0 ? g : 0) * group_rows; }
       for (int kb = 0; kb < num_kb; ++kb) {
@@ -219,8 +207,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
           const uint64_t bdesc = umma_desc_sw128(b0 + k * 32, 16, 1024);
           umma_bf16_ss(tmem_d, adesc, bdesc, idesc, (kb | k) != 0 ? 1u : 0u);
         }
-        if constexpr (CN > 1) umma_commit_mcast(empty_bar(stage), kMask);  // tell every producer of the cluster
-        else umma_commit(empty_bar(stage));                 // smem stage reusable once these MMAs retire
+        umma_commit(empty_bar(stage));                      // smem stage reusable once these MMAs retire
         if (kb == num_kb - 1) umma_commit(tfull_bar(acc));  // accumulator complete
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
@@ -233,7 +220,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int tile = cta0; tile < num_tiles; tile += cta_stride) {
-      const int m_tile = tile % num_m_tiles, n_tile = (tile / num_m_tiles) * CN + rank;
+      const int m_tile = tile % num_m_tiles, n_tile = tile / num_m_tiles;
       mbar_wait(tfull_bar(acc), acc_phase);
       tc_fence_after();
       const int row = m_tile * C::BM + q * 32 + lane;
@@ -347,53 +334,35 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
   }
 
   tc_fence_before();
-  if constexpr (CN > 1) cluster_sync_all(); else __syncthreads();  // peers may still multicast into / signal this CTA
+  __syncthreads();
   if (warp == 2) {
     tc_fence_after();
     tmem_dealloc<C::kTmemCols>(tmem_base);
   }
 }
 
-template <int BN, typename OutT, int GATE = kGateNone, int CN = 1, bool ROPE = false>
+template <int BN, typename OutT, int GATE = kGateNone, bool ROPE = false>
 static int launch_gemm(const CUtensorMap& tx, const CUtensorMap& tw, void* y, int M, int N, int K, int64_t ldy,
                        cudaStream_t st, const RopeEpi& re = RopeEpi{}, const RowPush& ps = RowPush{},
                        const int32_t* tile_group = nullptr, int group_rows = 0, float glu_limit = 0.f, const float* row_scale = nullptr) {
   using C = GemmCfg<BN>;
-  auto kern = gemm_tcgen05_kernel<BN, OutT, GATE, CN, ROPE>;
+  auto kern = gemm_tcgen05_kernel<BN, OutT, GATE, ROPE>;
   NVLLM_SMEM_ATTR_ONCE(kern, C::kSmemBytes);
   const int num_m_tiles = (M + C::BM - 1) / C::BM;
   const int num_n_tiles = GATE != kGateNone ? (N + BN / 2 - 1) / (BN / 2) : (N + BN - 1) / BN;
-  const int num_tiles = num_m_tiles * (num_n_tiles / CN);  // cluster tiles (the caller guarantees num_n_tiles % CN == 0)
-  const int max_clusters = sm_count() / CN;
-  const int clusters = num_tiles < max_clusters ? num_tiles : max_clusters;
+  const int num_tiles = num_m_tiles * num_n_tiles;
+  const int ctas = num_tiles < sm_count() ? num_tiles : sm_count();
   // Ring depth: NVLLM_GEMM_STAGES (benchmark knob) caps it for single-wave (decode-sized) launches: with <= ~100 KB of
   // shared memory two CTAs fit on an SM, so the NEXT kernel's CTAs become resident (prologue + weight prefetch under PDL)
   // while this kernel's are still running.
   int stages = C::kStages;
-  if (CN == 1 && num_tiles <= max_clusters) {
+  if (num_tiles <= sm_count()) {
     const int want = knobs().gemm_stages;
     if (want >= 2 && want < stages) stages = want;
   }
   const int smem = C::kSmemBytes - (C::kStages - stages) * C::kStageBytes;
-  if constexpr (CN == 1) {
-    NVLLM_CUDA(launch_pdl(kern, dim3(clusters), dim3(256), smem, st, tx, tw, static_cast<OutT*>(y), M, N, K, ldy,
-                          num_m_tiles, num_tiles, re, stages, ps, tile_group, group_rows, glu_limit, row_scale));
-  } else {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(clusters * CN);
-    cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = C::kSmemBytes;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = CN; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    NVLLM_CUDA(cudaLaunchKernelEx(&cfg, kern, tx, tw, static_cast<OutT*>(y), M, N, K, ldy, num_m_tiles, num_tiles, re,
-                                  static_cast<int>(C::kStages), ps, tile_group, group_rows, glu_limit, row_scale));
-  }
+  NVLLM_CUDA(launch_pdl(kern, dim3(ctas), dim3(256), smem, st, tx, tw, static_cast<OutT*>(y), M, N, K, ldy,
+                        num_m_tiles, num_tiles, re, stages, ps, tile_group, group_rows, glu_limit, row_scale));
   return 0;
 }
 
@@ -459,13 +428,6 @@ static bool want_2cta(int m, int n, int k) {
   return true;
 }
 
-static bool use_mcast() {
-  // x-multicast clusters: OFF by default.  In-graph they measured 5-7 % SLOWER than plain tiles on every shape they
-  // apply to (the bytes still have to enter every SM; the bound is the SM's TMA ingest, not L2 reads) and the long-K
-  // narrow-N projections they were built for now go to the cluster split-K kernel.  NVLLM_GEMM_MCAST=1 enables them.
-  return knobs().gemm_mcast != 0;
-}
-
 static bool use_2cta() {
   return knobs().gemm_2cta != 0;  // A/B knob: 0 keeps every shape on the single-CTA kernel
 }
@@ -498,14 +460,6 @@ int gemm_bf16_impl(void* y, const void* x, const void* w, int32_t m, int32_t n, 
   if (!push && want_2cta(m, n, k)) return gemm_2cta_dispatch(y, x, w, m, n, k, ldx, ldw, ldy, out_dtype, st);
   const int bn = pick_bn(m, n);
   CUtensorMap tx, tw;
-  // x-multicast clusters of 4 along N: worth it when x (re-read once per n-tile) dominates the L2 -> SM traffic,
-  // i.e. several n-tiles of a narrow width and a long K.
-  if (!push && use_mcast() && bn <= 64 && n % (4 * bn) == 0 && k >= 2048 && out_dtype == NVLLM_BF16) {
-    if (int rc = make_tmap_bf16_2d(&tx, x, m, k, ldx, 32)) return rc;
-    if (int rc = make_tmap_bf16_2d(&tw, w, n, k, ldw, bn)) return rc;
-    return bn == 64 ? launch_gemm<64, bf16, kGateNone, 4>(tx, tw, y, m, n, k, ldy, st)
-                    : launch_gemm<32, bf16, kGateNone, 4>(tx, tw, y, m, n, k, ldy, st);
-  }
   if (int rc = make_tmap_bf16_2d(&tx, x, m, k, ldx, 128)) return rc;
   if (int rc = make_tmap_bf16_2d(&tw, w, n, k, ldw, bn)) return rc;
 #define NVLLM_GEMM_CASE(BNV)                                                                     \
@@ -681,5 +635,5 @@ extern "C" int nvllm_gemm_qkv_rope_store(void* qkv, const void* x, const void* w
   CUtensorMap tx, tw;
   if (int rc = make_tmap_bf16_2d(&tx, x, m, k, ldx, 128)) return rc;
   if (int rc = make_tmap_bf16_2d(&tw, w_qkv, n, k, ldw, 128)) return rc;
-  return launch_gemm<128, bf16, kGateNone, 1, true>(tx, tw, qkv, m, n, k, n, static_cast<cudaStream_t>(stream), re);
+  return launch_gemm<128, bf16, kGateNone, true>(tx, tw, qkv, m, n, k, n, static_cast<cudaStream_t>(stream), re);
 }

@@ -16,7 +16,7 @@ ATOL, RTOL = 2e-2, 2 ** -7
 SHAPES = [
     (128, 128, 64), (1, 8, 64), (5, 40, 128), (129, 136, 192), (256, 4096, 1024), (300, 1024, 2048),
     (256, 6144, 1024), (64, 1024, 3072), (7, 264, 4096), (512, 512, 512),
-    (512, 768, 4096), (256, 1024, 3072), (130, 256, 2048),   # x-multicast clusters (narrow N, long K: TP shards)
+    (512, 768, 4096), (256, 1024, 3072), (130, 256, 2048),   # narrow N, long K: TP shards
 ]
 
 
@@ -224,18 +224,17 @@ def test_gemm_splitk_auto_decode_shapes(cuda, m, n, k):
 
 
 @pytest.mark.parametrize("m,n,k", [(512, 768, 4096), (256, 1024, 3072), (130, 256, 2048)])
-def test_gemm_x_multicast_clusters_opt_in(cuda, m, n, k, monkeypatch):
-    """The x-multicast cluster mode (off by default since the in-graph measurements) still computes the same GEMM."""
+def test_gemm_narrow_tiles_without_split_k(cuda, m, n, k, monkeypatch):
+    """Narrow outputs with a long K on the plain tiles (what they run on where no split is legal)."""
     from nano_vllm_rs_b200 import ops
     monkeypatch.setenv("NVLLM_GEMM_SPLITK", "0")
-    monkeypatch.setenv("NVLLM_GEMM_MCAST", "1")
     g = torch.Generator(device="cuda").manual_seed(m + n + k)
     x = torch.randn((m, k), generator=g, device=cuda).to(torch.bfloat16)
     w = (torch.randn((n, k), generator=g, device=cuda) * 0.02).to(torch.bfloat16)
     y = ops.gemm_bf16(x, w)
     r = ops.gemm_bf16(x, w, out_dtype=torch.float32, simt=True)
     torch.cuda.synchronize()
-    assert_close(to_np_f32(y), to_np_f32(r), ATOL, RTOL, f"mcast gemm {m}x{n}x{k}")
+    assert_close(to_np_f32(y), to_np_f32(r), ATOL, RTOL, f"narrow gemm {m}x{n}x{k}")
 
 
 @pytest.mark.parametrize("m", [1, 7, 8, 9, 16])

@@ -1,7 +1,7 @@
 """In-graph cost of the decode-step GEMMs (K5): each shape is captured `layers` times back to back into one CUDA graph
 (a different weight tensor per launch, > L2 in total, PDL edges kept — exactly how the decode step issues them) and the
 graph is replayed; us/launch = replay time / launches.  Per-launch event timing from Python cannot resolve these
-(~25 us floor); this can.  Sweeps the dispatch knobs (NVLLM_GEMM_BN / MCAST / 2CTA / SPLITK) in one process."""
+(~25 us floor); this can.  Sweeps the dispatch knobs (NVLLM_GEMM_BN / 2CTA / SPLITK) in one process."""
 import argparse, json, os, sys
 import torch
 sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
@@ -25,9 +25,9 @@ SHAPES = {  # name: (M, N, K, kind)
 }
 S, T, G = "NVLLM_GEMM_SPLITK", "NVLLM_GEMM_SK_STAGES", "NVLLM_GEMM_STAGES"
 KNOBS = [{}, {S: "0"}, {S: "64,4"}, {S: "64,2"}, {S: "128,4"}, {S: "128,2"}, {S: "256,4"}, {S: "256,2"},
-         {S: "0", "NVLLM_GEMM_MCAST": "1"}, {S: "0", "NVLLM_GEMM_2CTA": "2"},
+         {S: "0", "NVLLM_GEMM_2CTA": "2"},
          {S: "0", "NVLLM_GEMM_BN": "128"}, {S: "0", "NVLLM_GEMM_BN": "192"}, {S: "0", "NVLLM_GEMM_BN": "256"}, {S: "128,8"}, {S: "256,8"}]
-ALL = ("NVLLM_GEMM_BN", "NVLLM_GEMM_MCAST", "NVLLM_GEMM_2CTA", S, T, G)
+ALL = ("NVLLM_GEMM_BN", "NVLLM_GEMM_2CTA", S, T, G)
 
 
 def run(name, M, N, K, kind, layers, reps):
