@@ -21,10 +21,12 @@ struct LatentAttnArgs {
 
 constexpr int kLatentTileTokens = 8;
 
-// A tile of 8 consecutive tokens of the batch is dense when it holds tokens of at most two sequences: prompts and portions of
-// prompts, not a run of single decoded tokens.
+// A tile of 8 consecutive tokens of the batch is dense when the 8 tokens that end with its last one belong to at most two sequences:
+// prompts and portions of prompts, not single decoded tokens.  (A short last tile is judged with the tokens in front of it: one or two
+// tokens are always of two sequences at most, and 33 single tokens at 4001 keys took 311 us with the last one walking its keys alone
+// on the tcgen05 kernel, 105 so; the end of a prompt stays dense.)
 __device__ __forceinline__ bool latent_tile_dense(const int32_t* __restrict__ tok_seq, int n, int tile) {
-  const int t0 = tile * kLatentTileTokens, t1 = min(n, t0 + kLatentTileTokens);
+  const int t1 = min(n, (tile + 1) * kLatentTileTokens), t0 = max(0, t1 - kLatentTileTokens);
   int runs = 1;
   for (int t = t0 + 1; t < t1; ++t) runs += tok_seq[t] != tok_seq[t - 1];
   return runs <= 2;

@@ -76,3 +76,35 @@ def test_latent_prompts_portions_and_single_tokens(cuda, heads, rot, bs, window,
     assert torch.isfinite(got.float()).all()
     assert float((err / (ref.abs() + 0.25 * ref.pow(2).mean().sqrt())).max()) < 0.06, float(err.max())
     assert float(err.norm() / ref.norm()) < 6e-3
+
+
+def call(q_abs, q, tok_seq, pos, tabs, bs, cache, heads, dim, rot, scale, window=0):
+    """The C entry without a workspace: nothing is split."""
+    from nano_vllm_rs_b200 import _ffi
+    out = torch.empty((q.shape[0], heads * RANK), dtype=torch.bfloat16, device="cuda")
+    p = lambda t: t.data_ptr()
+    _ffi.check(_ffi.lib().nvllm_latent_window_attention(p(out), out.stride(0), p(q_abs), q_abs.stride(0), p(q), q.stride(0), p(tok_seq), p(pos), p(tabs), tabs.shape[1],
+                                                        bs, p(cache), cache.stride(0), q.shape[0], heads, dim, rot, RANK, scale, window, None, None, 0, None, 0, 0,
+                                                        torch.cuda.current_stream().cuda_stream))
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [32, 33, 34, 40, 41, 42])
+def test_single_tokens_are_what_each_gives_alone(cuda, n):
+    """Single tokens keep to the kernel of single tokens whatever their number is (a last tile of one or two is no prompt): without a
+    split every row is, to the bit, what its token gives alone."""
+    heads, dim, rot, bs, scale = 16, 24, 64, 64, 0.11
+    rng = np.random.default_rng(n)
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    randn = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    ctx = rng.integers(1, 700, n)
+    ctx[-2:] = 650, 333
+    tables, _, nslots = paged(rng, [int(c) for c in ctx], bs)
+    cache, tabs = randn(nslots, RANK + rot).to(torch.bfloat16), torch.from_numpy(tables).cuda()
+    q_abs, q = randn(n, heads * RANK) * 0.5, randn(n, heads * (dim + rot)).to(torch.bfloat16)
+    seq, pos = torch.arange(n, dtype=torch.int32, device="cuda"), torch.from_numpy(ctx - 1).cuda()
+    got = call(q_abs, q, seq, pos, tabs, bs, cache, heads, dim, rot, scale)
+    for t in range(n):
+        alone = call(q_abs[t:t + 1], q[t:t + 1], seq[t:t + 1], pos[t:t + 1], tabs, bs, cache, heads, dim, rot, scale)
+        assert torch.equal(alone[0], got[t]), t
