@@ -55,6 +55,66 @@ __device__ __forceinline__ Span span_of(const LatentAttnArgs& a, int t0, int ten
   return s;
 }
 
+// The factor on a row's accumulated values, from its running maximum (log2 units) and sum.
+__device__ __forceinline__ float row_factor(const LatentAttnArgs& a, int tok, int head, float m, float l) {
+  float oc = 1.0f, den = l;
+  if (a.sinks) {   // the sink joins the denominator only
+    const float sk = a.sinks[head] * 1.4426950408889634f, mn = fmaxf(m, sk);
+    oc = fast_exp2(m - mn);
+    den = l * oc + fast_exp2(sk - mn);
+  }
+  float inv = den > 0.f ? oc / den : 0.f;
+  if (a.gate) inv *= 1.0f / (1.0f + expf(-a.gate[static_cast<int64_t>(tok) * a.ldg + head]));
+  return inv;
+}
+
+// One row by one warp, over the keys [lo, hi) that it sees and no others: a NaN or an infinity in a cached row that a query of the tile
+// does not see would reach it through P = 0 (0 x Inf) in the tile's products.  Such rows are computed again here, for one half of the
+// values (8 neighbouring ones a lane); caches that hold numbers never get here.
+__device__ __noinline__ void row_alone(const LatentAttnArgs& a, int tok, int head, int lo, int hi, int half, int lane) {
+  const float* qa = a.q_abs + static_cast<int64_t>(tok) * a.ldqa + static_cast<int64_t>(head) * kRank + 8 * lane;
+  const bf16* qr = static_cast<const bf16*>(a.q) + static_cast<int64_t>(tok) * a.ldq + static_cast<int64_t>(head) * (a.dim + a.rot_dim) + a.dim + 2 * lane;
+  const bool rot = 2 * lane < a.rot_dim;
+  float q[2][8], acc[8] = {};
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) q[i][e] = __bfloat162float(__float2bfloat16_rn(qa[i * kHalf + e]));
+  const float r0 = rot ? __bfloat162float(qr[0]) : 0.f, r1 = rot ? __bfloat162float(qr[1]) : 0.f;
+  const int32_t* table = a.tables + static_cast<int64_t>(a.tok_seq[tok]) * a.table_cap;
+  float m = -INFINITY, l = 0.f;
+#pragma unroll 4
+  for (int j = lo; j < hi; ++j) {
+    const bf16* row = static_cast<const bf16*>(a.cache) + (static_cast<int64_t>(table[j / a.block_size]) * a.block_size + j % a.block_size) * a.cache_row;
+    float v[2][8], s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uint4 x = *reinterpret_cast<const uint4*>(row + i * kHalf + 8 * lane);
+      const uint32_t u[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) { v[i][2 * e] = bf16_lo(u[e]); v[i][2 * e + 1] = bf16_hi(u[e]); }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) s = fmaf(q[i][e], v[i][e], s);
+    }
+    if (rot) s = fmaf(r0, __bfloat162float(row[kRank + 2 * lane]), fmaf(r1, __bfloat162float(row[kRank + 2 * lane + 1]), s));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    s *= a.scale * 1.4426950408889634f;
+    const float mn = fmaxf(m, s), corr = m == -INFINITY ? 0.f : fast_exp2(m - mn), p = fast_exp2(s - (mn == -INFINITY ? 0.f : mn));
+    m = mn;
+    l = l * corr + p;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[e] = fmaf(p, half ? v[1][e] : v[0][e], j == lo ? 0.f : acc[e] * corr);
+  }
+  const float inv = row_factor(a, tok, head, m, l);
+  uint4 w;
+  w.x = pack_bf16x2(acc[0] * inv, acc[1] * inv);
+  w.y = pack_bf16x2(acc[2] * inv, acc[3] * inv);
+  w.z = pack_bf16x2(acc[4] * inv, acc[5] * inv);
+  w.w = pack_bf16x2(acc[6] * inv, acc[7] * inv);
+  *reinterpret_cast<uint4*>(static_cast<bf16*>(a.out) + static_cast<int64_t>(tok) * a.ldo + static_cast<int64_t>(head) * kRank + half * kHalf + 8 * lane) = w;
+}
+
 __global__ void __launch_bounds__(kThreads, 1) latent_attn_tc_kernel(const LatentAttnArgs a, int halves) {
   pdl_wait();
   pdl_launch_dependents();
@@ -242,7 +302,8 @@ __global__ void __launch_bounds__(kThreads, 1) latent_attn_tc_kernel(const Laten
     const float scale2 = a.scale * 1.4426950408889634f;
     const uint32_t tO = tmem + lane_off + kColO;
     constexpr float kRescale = 8.0f;   // log2 units: O is rescaled only when a row's maximum grows by more
-    int it = 0;
+    int it = 0, again_lo = 0, again_hi = 0;
+    bool again = false;
     for (int t = tile0; t < tend;) {
       const Span s = span_of(a, t, tend);
       const bool mine = my_tok >= s.t0 && my_tok < s.t1;
@@ -250,6 +311,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_attn_tc_kernel(const Laten
       const int hi = min(pos + 1, s.nkeys), lo = a.window > 0 && pos + 1 > a.window ? pos + 1 - a.window : 0;   // the row sees the keys [lo, hi)
       for (int h = 0; h < halves; ++h) {
         float m = -INFINITY, l = 0.f;
+        bool odd = false;   // the score of a key that the row does not see is no number: nor is its cached row
         const int it0 = it;
         for (int j0 = s.jstart; j0 < s.nkeys; j0 += kKeys, ++it) {
           const int b = it & 1;
@@ -266,7 +328,10 @@ __global__ void __launch_bounds__(kThreads, 1) latent_attn_tc_kernel(const Laten
           if (j0 + kKeys > hi || j0 < lo) {
 #pragma unroll
             for (int c = 0; c < kKeys; ++c)
-              if (j0 + c >= hi || j0 + c < lo) sr[c >> 5][c & 31] = 0xff800000u;
+              if (j0 + c >= hi || j0 + c < lo) {
+                odd |= (sr[c >> 5][c & 31] & 0x7f800000u) == 0x7f800000u;
+                sr[c >> 5][c & 31] = 0xff800000u;
+              }
           }
           float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -306,17 +371,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_attn_tc_kernel(const Laten
           tc_fence_before();
           mbar_arrive(p_ready(b));
         }
-        float inv = 0.f;
-        if (mine) {
-          float oc = 1.0f, den = l;
-          if (a.sinks) {   // the sink joins the denominator only
-            const float sk = a.sinks[my_head] * 1.4426950408889634f, mn = fmaxf(m, sk);
-            oc = fast_exp2(m - mn);
-            den = l * oc + fast_exp2(sk - mn);
-          }
-          inv = den > 0.f ? oc / den : 0.f;
-          if (a.gate) inv *= 1.0f / (1.0f + expf(-a.gate[static_cast<int64_t>(my_tok) * a.ldg + my_head]));
-        }
+        const float inv = mine ? row_factor(a, my_tok, my_head, m, l) : 0.f;
         bf16* out = static_cast<bf16*>(a.out) + static_cast<int64_t>(mine ? my_tok : tile0) * a.ldo + static_cast<int64_t>(my_head) * kRank + (half0 + h) * kHalf;
         if (it > it0) {
           mbar_wait(o_done, (it - 1) & 1);
@@ -344,9 +399,17 @@ __global__ void __launch_bounds__(kThreads, 1) latent_attn_tc_kernel(const Laten
             }
           }
         }
+        // (l is no number where a key that the row does see is none: the row's values are none, whatever the others hold)
+        if (mine && odd && fabsf(l) < INFINITY) { again = true; again_lo = lo; again_hi = hi; }
         tc_fence_before();   // the next half's first PV overwrites O: it waits for this group's next p_ready
       }
       t = s.t1;
+    }
+    __syncwarp();   // other lanes write a row that its owner has written
+    for (unsigned rows = __ballot_sync(0xffffffffu, again); rows != 0; rows &= rows - 1) {   // (no other role waits for this one any more)
+      const int src = __ffs(rows) - 1, tok = __shfl_sync(0xffffffffu, my_tok, src), head = __shfl_sync(0xffffffffu, my_head, src);
+      const int lo = __shfl_sync(0xffffffffu, again_lo, src), hi = __shfl_sync(0xffffffffu, again_hi, src);
+      for (int h = 0; h < halves; ++h) row_alone(a, tok, head, lo, hi, half0 + h, lane);
     }
   }
   tc_fence_before();

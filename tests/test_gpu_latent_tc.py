@@ -108,3 +108,27 @@ def test_single_tokens_are_what_each_gives_alone(cuda, n):
     for t in range(n):
         alone = call(q_abs[t:t + 1], q[t:t + 1], seq[t:t + 1], pos[t:t + 1], tabs, bs, cache, heads, dim, rot, scale)
         assert torch.equal(alone[0], got[t]), t
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("value", [math.nan, math.inf, -math.inf])
+@pytest.mark.parametrize("column", [3, 300, RANK + 5])   # either half of the latent values, the rotated part
+@pytest.mark.parametrize("window,tokens", [(0, 129), (33, 129), (0, 1200)])   # 1200: both halves in one CTA
+def test_a_cached_value_that_is_no_number_stays_with_the_tokens_that_see_it(cuda, value, column, window, tokens):
+    """Tokens of a tile share the key tiles; a key that a token does not see must not reach it through 0 x Inf."""
+    heads, dim, rot, bs, scale, at = 16, 24, 64, 64, 0.11, 50
+    gen = torch.Generator(device="cuda").manual_seed(tokens + column)
+    randn = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    tables, _, nslots = paged(np.random.default_rng(1), [tokens], bs)
+    cache, tabs = randn(nslots, RANK + rot).to(torch.bfloat16), torch.from_numpy(tables).cuda()
+    q_abs, q = randn(tokens, heads * RANK) * 0.5, randn(tokens, heads, dim + rot).to(torch.bfloat16)
+    seq, pos = torch.zeros(tokens, dtype=torch.int32, device="cuda"), torch.arange(tokens, device="cuda")
+    ref = reference(q_abs, q[..., dim:], cache, [(0, tokens)], pos, tabs, bs, heads, rot, scale, window, None, None)
+    cache[int(tables[0, at // bs]) * bs + at % bs, column] = value
+    got = call(q_abs, q.reshape(tokens, -1), seq, pos, tabs, bs, cache, heads, dim, rot, scale, window).double()
+    sees = (pos >= at) & ((pos < at + window) if window else True)
+    err = (got - ref)[~sees]
+    assert torch.isfinite(got[~sees]).all()
+    assert float(err.norm() / ref[~sees].norm()) < 6e-3 and float((err.abs() / (ref[~sees].abs() + 0.25 * ref.pow(2).mean().sqrt())).max()) < 0.06
+    if value != value:
+        assert not torch.isfinite(got[sees]).any()
