@@ -539,6 +539,14 @@ int nvllm_latent_window_attention(void* out, int64_t ldo, const float* q_abs, in
                                   int32_t heads, int32_t dim, int32_t rot_dim, int32_t kv_rank, float scale, int32_t window,
                                   const float* sinks, const float* gate, int64_t ldg, void* workspace, size_t workspace_bytes,
                                   int32_t dtype, void* stream);
+/* The same for a batch in which (nearly) every sequence has one token, as in a decode step: the kernel for prompts is not tried.
+ * (Any batch may be given; prompts run slower here.) */
+int nvllm_latent_token_attention(void* out, int64_t ldo, const float* q_abs, int64_t ldqa, const void* q, int64_t ldq,
+                                 const int32_t* tok_seq, const int64_t* positions, const int32_t* block_tables,
+                                 int32_t table_cap, int32_t block_size, const void* cache, int64_t cache_row, int32_t n,
+                                 int32_t heads, int32_t dim, int32_t rot_dim, int32_t kv_rank, float scale,
+                                 int32_t window, const float* sinks, const float* gate, int64_t ldg, void* workspace,
+                                 size_t workspace_bytes, int32_t dtype, void* stream);
 /* Per-token preparation of the gated delta rule, in place, all f32:
  *   q, k: [n, groups * dk] -> every head divided by sqrt(sum of squares + unit_eps), q also times q_scale;
  *   beta: [n, heads] -> sigmoid;   decay: [n, heads * dk] -> exp(-exp(a_log[h]) * softplus(decay + dt_bias[h, c])). */

@@ -435,7 +435,7 @@ class Kosazen : public ModelImpl {
       } else {
         NVLLM_CUDA(cudaMemsetAsync(q_abs_, 0, static_cast<size_t>(N) * HR * 4, static_cast<cudaStream_t>(st)));
       }
-      RUN(nvllm_latent_window_attention(o_lat_, HR, q_abs_, HR, qd_, ldqd, v.tok_seq, v.positions, v.tables, v.table_cap, lim_.block_size,
+      RUN((v.n_tokens <= v.n_seqs ? nvllm_latent_token_attention : nvllm_latent_window_attention)(o_lat_, HR, q_abs_, HR, qd_, ldqd, v.tok_seq, v.positions, v.tables, v.table_cap, lim_.block_size,
                                         cache_[r], L.cache_row(), N, L.heads, L.dim, L.rot_dim, L.kv_rank, L.scale, 0, nullptr, nullptr, 0,
                                         lat_ws_, lat_ws_bytes_, dt_, st)); ++launches; mk("latent_attention");
       // values: per head Uv_h applied to the attended latent, then the output projection

@@ -836,12 +836,46 @@ extern "C" size_t nvllm_latent_workspace_bytes(int32_t n, int32_t heads, int32_t
   return splits > 1 ? static_cast<size_t>(n) * heads * splits * (kv_rank + 2) * sizeof(float) : 0;
 }
 
-extern "C" int nvllm_latent_window_attention(void* out, int64_t ldo, const float* q_abs, int64_t ldqa, const void* q, int64_t ldq,
-                                             const int32_t* tok_seq, const int64_t* positions, const int32_t* block_tables,
-                                             int32_t table_cap, int32_t block_size, const void* cache, int64_t cache_row, int32_t n,
-                                             int32_t heads, int32_t dim, int32_t rot_dim, int32_t kv_rank, float scale,
-                                             int32_t window, const float* sinks, const float* gate, int64_t ldg, void* workspace,
-                                             size_t workspace_bytes, int32_t dtype, void* stream) {
+namespace {
+// single_tokens: the caller knows that (nearly) every sequence has one token in the batch.  A batch of 32 and more of them would be
+// offered to the tcgen05 kernel first, a launch that finds no dense tile and that the next one waits for.
+int run_attention(const AttnArgs& a, size_t workspace_bytes, int dtype, bool single_tokens, cudaStream_t st) {
+  // bf16 caches with a 16-byte row pitch and kv_rank <= 512 run on the tensor cores (NVLLM_LATENT_MMA=0: the CUDA-core kernel)
+  const int dp16 = (static_cast<int>(a.cache_row) + 15) / 16 * 16;
+  if (dtype == NVLLM_BF16 && knobs().latent_mma != 0 && a.kv_rank <= 512 && a.cache_row % 8 == 0 && dp16 <= 704 &&
+      (reinterpret_cast<uintptr_t>(a.cache) & 15u) == 0) {
+    AttnArgs b = a;
+    if (!single_tokens && knobs().latent_mma == 1 && latent_attn_tc_applies(a)) {
+      if (int rc = latent_attn_tc_launch(a, st)) return rc;
+      b.skip_dense = 1;   // tiles of many sequences are left to the kernel below
+    }
+    // Single tokens on fewer CTAs than SMs: the key tiles of a token are split over CTAs along z, as many as fill the SMs once and
+    // leave each (at the longest context the tables or the window allow) at least four tiles; the partials meet in
+    // latent_attn_merge_kernel.  Measured, 32 tokens x 16 heads at 4001 keys, rank 512: 223 -> 104 us.  64 tokens in a window of
+    // 2048 keys 118 -> 79 us; in one of 512 the second launch costs what the shorter loop saves (39 -> 37 us), hence eight tiles for
+    // windows.
+    if (a.part != nullptr && a.n <= 256) {
+      const int64_t ctas = static_cast<int64_t>(a.n) * ((a.heads + 15) / 16);
+      const int64_t reach = a.window > 0 ? a.window + kMmaKeys - 1 : static_cast<int64_t>(a.table_cap) * a.block_size;
+      const int tiles = static_cast<int>(std::min<int64_t>((reach + kMmaKeys - 1) / kMmaKeys, 1 << 20));
+      int splits = static_cast<int>(sm_count() / (ctas > 0 ? ctas : 1));
+      splits = std::min(splits, a.window > 0 ? std::min(4, tiles / 8) : std::min(kMaxLatentSplits, tiles / 4));
+      splits = static_cast<int>(std::min<size_t>(splits, workspace_bytes / (static_cast<size_t>(a.n) * a.heads * (a.kv_rank + 2) * sizeof(float))));
+      if (splits > 1) b.splits = splits;
+    }
+    if (a.kv_rank <= 128) return launch_attn_mma<1>(b, st);
+    if (a.kv_rank <= 256) return launch_attn_mma<2>(b, st);
+    if (a.kv_rank <= 384) return launch_attn_mma<3>(b, st);
+    return launch_attn_mma<4>(b, st);
+  }
+  return dtype == NVLLM_BF16 ? dispatch_attn<bf16>(a, st) : dispatch_attn<float>(a, st);
+}
+
+int window_attention(void* out, int64_t ldo, const float* q_abs, int64_t ldqa, const void* q, int64_t ldq, const int32_t* tok_seq,
+                     const int64_t* positions, const int32_t* block_tables, int32_t table_cap, int32_t block_size, const void* cache,
+                     int64_t cache_row, int32_t n, int32_t heads, int32_t dim, int32_t rot_dim, int32_t kv_rank, float scale, int32_t window,
+                     const float* sinks, const float* gate, int64_t ldg, void* workspace, size_t workspace_bytes, int32_t dtype, bool single_tokens,
+                     void* stream) {
   NVLLM_CHECK_ARG(n >= 0 && heads > 0 && dim >= 0 && rot_dim >= 0 && kv_rank > 0 && kv_rank <= 1024 && table_cap > 0 && block_size > 0,
                   NVLLM_ERR_ARG, "latent_attention: sizes (kv_rank <= 1024)");
   NVLLM_CHECK_ARG(dtype == NVLLM_BF16 || dtype == NVLLM_F32, NVLLM_ERR_DTYPE, "latent_attention: dtype %d", dtype);
@@ -849,34 +883,26 @@ extern "C" int nvllm_latent_window_attention(void* out, int64_t ldo, const float
   NVLLM_CHECK_ARG(out && q_abs && (q || rot_dim == 0) && tok_seq && positions && block_tables && cache, NVLLM_ERR_ARG, "latent_attention: NULL");
   const AttnArgs a{out, ldo, q_abs, ldqa, q ? q : q_abs, ldq, tok_seq, positions, block_tables, table_cap, block_size, cache, cache_row,
                    n, heads, dim, rot_dim, kv_rank, scale, window > 0 ? window : 0, sinks, gate, ldg, 1, static_cast<float*>(workspace), 0};
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // bf16 caches with a 16-byte row pitch and kv_rank <= 512 run on the tensor cores (NVLLM_LATENT_MMA=0: the CUDA-core kernel)
-  const int dp16 = (static_cast<int>(cache_row) + 15) / 16 * 16;
-  if (dtype == NVLLM_BF16 && knobs().latent_mma != 0 && kv_rank <= 512 && cache_row % 8 == 0 && dp16 <= 704 &&
-      (reinterpret_cast<uintptr_t>(cache) & 15u) == 0) {
-    AttnArgs b = a;
-    if (knobs().latent_mma == 1 && latent_attn_tc_applies(a)) {
-      if (int rc = latent_attn_tc_launch(a, st)) return rc;
-      b.skip_dense = 1;   // single tokens (tiles of many sequences) are left to the kernel below
-    }
-    // Single tokens on fewer CTAs than SMs: the key tiles of a token are split over CTAs along z, as many as fill the SMs once and
-    // leave each (at the longest context the tables or the window allow) at least four tiles; the partials meet in
-    // latent_attn_merge_kernel.  Measured, 32 tokens x 16 heads at 4001 keys, rank 512: 223 -> 104 us.  64 tokens in a window of
-    // 2048 keys 118 -> 79 us; in one of 512 the second launch costs what the shorter loop saves (39 -> 37 us), hence eight tiles for
-    // windows.
-    if (workspace != nullptr && n <= 256) {
-      const int64_t ctas = static_cast<int64_t>(n) * ((heads + 15) / 16);
-      const int64_t reach = window > 0 ? window + kMmaKeys - 1 : static_cast<int64_t>(table_cap) * block_size;
-      const int tiles = static_cast<int>(std::min<int64_t>((reach + kMmaKeys - 1) / kMmaKeys, 1 << 20));
-      int splits = static_cast<int>(sm_count() / (ctas > 0 ? ctas : 1));
-      splits = std::min(splits, window > 0 ? std::min(4, tiles / 8) : std::min(kMaxLatentSplits, tiles / 4));
-      splits = static_cast<int>(std::min<size_t>(splits, workspace_bytes / (static_cast<size_t>(n) * heads * (kv_rank + 2) * sizeof(float))));
-      if (splits > 1) b.splits = splits;
-    }
-    if (kv_rank <= 128) return launch_attn_mma<1>(b, st);
-    if (kv_rank <= 256) return launch_attn_mma<2>(b, st);
-    if (kv_rank <= 384) return launch_attn_mma<3>(b, st);
-    return launch_attn_mma<4>(b, st);
-  }
-  return dtype == NVLLM_BF16 ? dispatch_attn<bf16>(a, st) : dispatch_attn<float>(a, st);
+  return run_attention(a, workspace_bytes, dtype, single_tokens, static_cast<cudaStream_t>(stream));
+}
+}  // namespace
+
+extern "C" int nvllm_latent_window_attention(void* out, int64_t ldo, const float* q_abs, int64_t ldqa, const void* q, int64_t ldq,
+                                             const int32_t* tok_seq, const int64_t* positions, const int32_t* block_tables,
+                                             int32_t table_cap, int32_t block_size, const void* cache, int64_t cache_row,
+                                             int32_t n, int32_t heads, int32_t dim, int32_t rot_dim, int32_t kv_rank, float scale,
+                                             int32_t window, const float* sinks, const float* gate, int64_t ldg, void* workspace,
+                                             size_t workspace_bytes, int32_t dtype, void* stream) {
+  return window_attention(out, ldo, q_abs, ldqa, q, ldq, tok_seq, positions, block_tables, table_cap, block_size, cache, cache_row, n, heads, dim,
+                          rot_dim, kv_rank, scale, window, sinks, gate, ldg, workspace, workspace_bytes, dtype, false, stream);
+}
+
+extern "C" int nvllm_latent_token_attention(void* out, int64_t ldo, const float* q_abs, int64_t ldqa, const void* q, int64_t ldq,
+                                            const int32_t* tok_seq, const int64_t* positions, const int32_t* block_tables,
+                                            int32_t table_cap, int32_t block_size, const void* cache, int64_t cache_row, int32_t n,
+                                            int32_t heads, int32_t dim, int32_t rot_dim, int32_t kv_rank, float scale,
+                                            int32_t window, const float* sinks, const float* gate, int64_t ldg, void* workspace,
+                                            size_t workspace_bytes, int32_t dtype, void* stream) {
+  return window_attention(out, ldo, q_abs, ldqa, q, ldq, tok_seq, positions, block_tables, table_cap, block_size, cache, cache_row, n, heads, dim,
+                          rot_dim, kv_rank, scale, window, sinks, gate, ldg, workspace, workspace_bytes, dtype, true, stream);
 }

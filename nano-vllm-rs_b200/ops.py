@@ -324,10 +324,10 @@ def latent_attention(q_abs, q, tok_seq, positions, tables, block_size, cache, he
     out = torch.empty((n, heads * kv_rank), dtype=q.dtype, device=q.device)
     need = _ffi.lib().nvllm_latent_workspace_bytes(n, heads, kv_rank)   # of single tokens whose keys are split over CTAs
     ws = torch.empty(need, dtype=torch.uint8, device=q.device) if need and q.dtype == torch.bfloat16 else None
-    check(_ffi.lib().nvllm_latent_window_attention(_p(out), out.stride(0), _p(q_abs), q_abs.stride(0), _p(q), q.stride(0), _p(tok_seq),
-                                                   _p(positions), _p(tables), tables.shape[1], block_size, _p(cache), cache.stride(0), n,
-                                                   heads, dim, rot_dim, kv_rank, scale, 0, None, None, 0, _p(ws), need if ws is not None else 0,
-                                                   _dt(q), _stream()))
+    check(_latent_entry(n, tables)(_p(out), out.stride(0), _p(q_abs), q_abs.stride(0), _p(q), q.stride(0), _p(tok_seq),
+                                   _p(positions), _p(tables), tables.shape[1], block_size, _p(cache), cache.stride(0), n,
+                                   heads, dim, rot_dim, kv_rank, scale, 0, None, None, 0, _p(ws), need if ws is not None else 0,
+                                   _dt(q), _stream()))
     return out
 
 
@@ -540,15 +540,20 @@ def window_attention(q, gate, k_cache, v_cache, tok_seq, positions, tables, bloc
     return out
 
 
+def _latent_entry(n, tables):
+    """As many sequences as tokens: single tokens, as in a decode step."""
+    return _ffi.lib().nvllm_latent_token_attention if n <= tables.shape[0] else _ffi.lib().nvllm_latent_window_attention
+
+
 def latent_window_attention(q_abs, tok_seq, positions, tables, block_size, cache, heads, kv_rank, scale, dtype, window=0, sinks=None,
                             gate=None, workspace=None):
     """q_abs f32 [n, heads * kv_rank] (the key map folded into the query); cache [slots, row >= kv_rank] in `dtype`."""
     n = q_abs.shape[0]
     out = torch.empty((n, heads * kv_rank), dtype=dtype, device=q_abs.device)
-    check(_ffi.lib().nvllm_latent_window_attention(_p(out), out.stride(0), _p(q_abs), q_abs.stride(0), None, 0, _p(tok_seq), _p(positions),
-                                                   _p(tables), tables.shape[1], block_size, _p(cache), cache.stride(0), n, heads, 0, 0,
-                                                   kv_rank, scale, window, _p(sinks), _p(gate), gate.stride(0) if gate is not None else 0,
-                                                   _p(workspace), workspace.numel() * 4 if workspace is not None else 0, _dt(out), _stream()))
+    check(_latent_entry(n, tables)(_p(out), out.stride(0), _p(q_abs), q_abs.stride(0), None, 0, _p(tok_seq), _p(positions),
+                                   _p(tables), tables.shape[1], block_size, _p(cache), cache.stride(0), n, heads, 0, 0,
+                                   kv_rank, scale, window, _p(sinks), _p(gate), gate.stride(0) if gate is not None else 0,
+                                   _p(workspace), workspace.numel() * 4 if workspace is not None else 0, _dt(out), _stream()))
     return out
 
 
@@ -818,10 +823,10 @@ def latent_rotary_attention(q_abs, q, tok_seq, positions, tables, block_size, ca
     """latent_window_attention whose cache rows also hold a rotated key part; q [n, heads * (dim + rot_dim)]."""
     n = q_abs.shape[0]
     out = torch.empty((n, heads * kv_rank), dtype=q.dtype, device=q_abs.device)
-    check(_ffi.lib().nvllm_latent_window_attention(_p(out), out.stride(0), _p(q_abs), q_abs.stride(0), _p(q), q.stride(0), _p(tok_seq), _p(positions),
-                                                   _p(tables), tables.shape[1], block_size, _p(cache), cache.stride(0), n, heads, dim, rot_dim, kv_rank,
-                                                   scale, window, None, None, 0, _p(workspace), workspace.numel() * 4 if workspace is not None else 0,
-                                                   _dt(out), _stream()))
+    check(_latent_entry(n, tables)(_p(out), out.stride(0), _p(q_abs), q_abs.stride(0), _p(q), q.stride(0), _p(tok_seq), _p(positions),
+                                   _p(tables), tables.shape[1], block_size, _p(cache), cache.stride(0), n, heads, dim, rot_dim, kv_rank,
+                                   scale, window, None, None, 0, _p(workspace), workspace.numel() * 4 if workspace is not None else 0,
+                                   _dt(out), _stream()))
     return out
 
 

@@ -132,3 +132,55 @@ def test_a_cached_value_that_is_no_number_stays_with_the_tokens_that_see_it(cuda
     assert float(err.norm() / ref[~sees].norm()) < 6e-3 and float((err.abs() / (ref[~sees].abs() + 0.25 * ref.pow(2).mean().sqrt())).max()) < 0.06
     if value != value:
         assert not torch.isfinite(got[sees]).any()
+
+
+def kernels_of(f):
+    """How many kernels f launches: the nodes of its graph."""
+    from cuda.bindings import runtime
+    f()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        f()
+    err, _, count = runtime.cudaGraphGetNodes(runtime.cudaGraph_t(graph.raw_cuda_graph()))
+    assert int(err) == 0
+    return int(count)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,context,launches", [(8, 300, 1), (40, 300, 1), (40, 3000, 2), (300, 300, 1)])
+def test_a_batch_of_single_tokens_launches_no_kernel_for_prompts(cuda, n, context, launches):
+    from nano_vllm_rs_b200 import ops
+    heads, dim, rot, bs, scale = 16, 24, 64, 64, 0.11
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    randn = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    tables, _, nslots = paged(np.random.default_rng(n), [context] * n, bs)
+    cache, tabs = randn(nslots, RANK + rot).to(torch.bfloat16), torch.from_numpy(tables).cuda()
+    q_abs, q = randn(n, heads * RANK) * 0.5, randn(n, heads * (dim + rot)).to(torch.bfloat16)
+    seq, pos = torch.arange(n, dtype=torch.int32, device="cuda"), torch.full((n,), context - 1, device="cuda")
+    run = lambda: ops.latent_attention(q_abs, q, seq, pos, tabs, bs, cache, heads, dim, rot, RANK, scale)
+    assert kernels_of(run) == launches
+    if launches == 1:
+        assert torch.equal(run(), call(q_abs, q, seq, pos, tabs, bs, cache, heads, dim, rot, scale))
+
+
+@pytest.mark.gpu
+def test_the_entry_of_single_tokens_takes_any_batch(cuda, monkeypatch):
+    """Prompts and portions given to nvllm_latent_token_attention run on the mma.sync kernel."""
+    from nano_vllm_rs_b200 import _ffi
+    heads, dim, rot, bs, scale = 16, 24, 64, 64, 0.11
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    randn = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    counts = [70, 1, 30]
+    n = sum(counts)
+    tables, _, nslots = paged(np.random.default_rng(3), counts, bs)
+    cache, tabs = randn(nslots, RANK + rot).to(torch.bfloat16), torch.from_numpy(tables).cuda()
+    q_abs, q = randn(n, heads * RANK) * 0.5, randn(n, heads * (dim + rot)).to(torch.bfloat16)
+    seq = torch.repeat_interleave(torch.arange(3), torch.tensor(counts)).to(torch.int32).cuda()
+    pos = torch.cat([torch.arange(c) for c in counts]).cuda()
+    args = (q_abs, q, seq, pos, tabs, bs, cache, heads, dim, rot, scale)
+    prompts = call(*args)
+    with monkeypatch.context() as m:
+        m.setattr(_ffi.lib(), "nvllm_latent_window_attention", _ffi.lib().nvllm_latent_token_attention)
+        single = call(*args)
+    monkeypatch.setenv("NVLLM_LATENT_MMA", "2")
+    assert torch.equal(single, call(*args)) and not torch.equal(single, prompts)
