@@ -322,12 +322,13 @@ def latent_prepare(q, dkv, c_norm_w, eps, positions, table, rot_dims, heads, dim
 def latent_attention(q_abs, q, tok_seq, positions, tables, block_size, cache, heads, dim, rot_dim, kv_rank, scale):
     n = q.shape[0]
     out = torch.empty((n, heads * kv_rank), dtype=q.dtype, device=q.device)
-    need = _ffi.lib().nvllm_latent_workspace_bytes(n, heads, kv_rank)   # of single tokens whose keys are split over CTAs
-    ws = torch.empty(need, dtype=torch.uint8, device=q.device) if need and q.dtype == torch.bfloat16 else None
+    need, ws = 0, None   # of single tokens whose keys are split over CTAs: four tiles of 64 keys or more each, so none below eight tiles
+    if tables.shape[1] * block_size > 448 and n <= 256 and q.dtype == torch.bfloat16:
+        need = _ffi.lib().nvllm_latent_workspace_bytes(n, heads, kv_rank)
+        ws = torch.empty(need, dtype=torch.uint8, device=q.device) if need else None
     check(_latent_entry(n, tables)(_p(out), out.stride(0), _p(q_abs), q_abs.stride(0), _p(q), q.stride(0), _p(tok_seq),
                                    _p(positions), _p(tables), tables.shape[1], block_size, _p(cache), cache.stride(0), n,
-                                   heads, dim, rot_dim, kv_rank, scale, 0, None, None, 0, _p(ws), need if ws is not None else 0,
-                                   _dt(q), _stream()))
+                                   heads, dim, rot_dim, kv_rank, scale, 0, None, None, 0, _p(ws), need, _dt(q), _stream()))
     return out
 
 

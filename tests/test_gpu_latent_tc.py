@@ -184,3 +184,24 @@ def test_the_entry_of_single_tokens_takes_any_batch(cuda, monkeypatch):
         single = call(*args)
     monkeypatch.setenv("NVLLM_LATENT_MMA", "2")
     assert torch.equal(single, call(*args)) and not torch.equal(single, prompts)
+
+
+@pytest.mark.gpu
+def test_a_workspace_is_asked_for_where_keys_can_be_split(cuda, monkeypatch):
+    """Eight tiles of 64 keys are the fewest that two CTAs share; the split never lies below."""
+    from nano_vllm_rs_b200 import _ffi, ops
+    heads, dim, rot, scale, n = 16, 24, 64, 0.11, 4
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    randn = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    asked = []
+    entry = _ffi.lib().nvllm_latent_workspace_bytes
+    monkeypatch.setattr(_ffi.lib(), "nvllm_latent_workspace_bytes", lambda *a: asked.append(a) or entry(*a))
+    q_abs, q, seq = randn(n, heads * RANK) * 0.5, randn(n, heads * (dim + rot)).to(torch.bfloat16), torch.arange(n, dtype=torch.int32, device="cuda")
+    for blocks, launches in ((7, 1), (8, 2)):
+        tabs = torch.arange(n * blocks, dtype=torch.int32, device="cuda").reshape(n, blocks)
+        cache, pos = randn(n * blocks * 64, RANK + rot).to(torch.bfloat16), torch.full((n,), blocks * 64 - 1, device="cuda")
+        ws = torch.empty(entry(n, heads, RANK) // 4, device="cuda")
+        asked.clear()
+        assert kernels_of(lambda: ops.latent_attention(q_abs, q, seq, pos, tabs, 64, cache, heads, dim, rot, RANK, scale)) == launches
+        assert bool(asked) == (launches == 2)
+        assert kernels_of(lambda: ops.latent_rotary_attention(q_abs, q, seq, pos, tabs, 64, cache, heads, dim, rot, RANK, scale, workspace=ws)) == launches
