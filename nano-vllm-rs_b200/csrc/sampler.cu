@@ -393,7 +393,7 @@ __device__ bool select_mass_linear(Shared& sh, const float* __restrict__ row, in
     for (int e = 0; e < 4; ++e)
       if (e < n) {
         const float s = scaled(v[e], T);
-        if (s > m - 22.5f) {
+        if (m - s < 22.5f) {   // (the difference is exact where it matters; m - 22.5 is not, for large m)
           const uint32_t w = fx_exp(s, m);
           if (w != 0u) atomicAdd(&sh.hist[bin_of(s)], static_cast<unsigned long long>(w));
         } else if (!(s <= m)) {
@@ -438,7 +438,7 @@ __device__ bool select_mass_linear(Shared& sh, const float* __restrict__ row, in
     for (int e = 0; e < 4; ++e)
       if (e < n) {
         const float s = scaled(v[e], T);
-        if (s > m - 22.5f && bin_of(s) == bin && fx_exp(s, m) != 0u) {
+        if (m - s < 22.5f && bin_of(s) == bin && fx_exp(s, m) != 0u) {
           const int at = atomicAdd(&sh.ncand, 1);
           if (at < kCand) sh.hist[at] = pack_candidate(okey(s), static_cast<uint32_t>(i0 + e));
         }

@@ -171,3 +171,28 @@ def test_short_cuts_select_what_the_radix_selection_selects(cuda, V):
     b = run(cuda, x * np.float32(2 ** 24), temps * np.float32(2 ** 24), seeds, top_k=ks, top_p=ps)
     for got, want in zip(a, b):
         assert (got == want).all()
+
+
+@pytest.mark.parametrize("top", [3.0, 25.0, 100.0, 150.0, -150.0])
+def test_masses_of_large_scaled_values(cuda, top):
+    """At a temperature of 1e-6 neighbouring logits lie whole units apart: 100 000 values some steps below the maximum have a mass (one of
+    2^32 at 22 below) that decides the cut.  Times 2^44 the same scaled values go to the radix selection."""
+    V = 120000
+    steps = [1, 2, 3, 5, 6, 7, 11, 12, 23, 90, 180]
+    ps = [0.5, 0.995, 0.99999]
+    rows = []
+    for s in steps:
+        x = np.full(V, top - 1.0, np.float32)
+        below = np.float32(top)
+        for _ in range(s):
+            below = np.nextafter(below, np.float32(-np.inf), dtype=np.float32)
+        x[10:100010] = below
+        x[7] = top
+        rows.append(x)
+    x = np.repeat(np.stack(rows), len(ps), 0)
+    B = len(x)
+    top_p, temps, seeds = ps * len(steps), np.full(B, 1e-6, np.float32), seeds_for(B, 5)
+    a = run(cuda, x, temps, seeds, top_p=top_p)
+    b = run(cuda, x * np.float32(2.0 ** 44), temps * np.float32(2.0 ** 44), seeds, top_p=top_p)
+    for got, want in zip(a, b):
+        assert (got == want).all()
