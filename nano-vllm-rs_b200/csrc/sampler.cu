@@ -604,8 +604,8 @@ sample_kernel(int64_t* __restrict__ out_ids, const float* __restrict__ logits, i
             if (fabsf(near) < 1e4f && 1.0f - u > 1.01f * __expf(near - best)) continue;
             const float s = scaled(v[e], T);
             const uint32_t key = okey(s);
-            if (!keeps(sk, key, static_cast<uint32_t>(i)) || !keeps(sp, key, static_cast<uint32_t>(i))) continue;
-            score = s + gumbel_of(u);
+            // (a value that is filtered out still wins where every survivor is NaN, as in the body below)
+            score = keeps(sk, key, static_cast<uint32_t>(i)) && keeps(sp, key, static_cast<uint32_t>(i)) ? s + gumbel_of(u) : -INFINITY;
           }
           if (score > best || (score == best && i < bidx)) { best = score; bidx = i; }
         }

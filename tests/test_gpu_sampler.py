@@ -196,3 +196,30 @@ def test_masses_of_large_scaled_values(cuda, top):
     b = run(cuda, x * np.float32(2.0 ** 44), temps * np.float32(2.0 ** 44), seeds, top_p=top_p)
     for got, want in zip(a, b):
         assert (got == want).all()
+
+
+@pytest.mark.parametrize("rows", [24, 168])        # 1024 threads a row, and 512 beyond one row per SM
+@pytest.mark.parametrize("V", [4096, 20001, 151936])
+def test_tokens_do_not_depend_on_what_else_is_asked_for(cuda, rows, V):
+    """Without the survivors' count and mask, a value that cannot win is skipped before its noise is computed: the tokens are the same."""
+    from nano_vllm_rs_b200 import ops
+    g = torch.Generator(device=cuda).manual_seed(V + rows)
+    x = 2.5 * torch.randn((rows, V), generator=g, device=cuda)
+    T = torch.tensor([0.1, 0.5, 1.0, 1.7, 3.0, 0.0], device=cuda).repeat(rows // 6)
+    x[1::12] *= 400.0                                      # quotients on both sides of 1e4, where the skip ends
+    x[2::12] = torch.round(x[2::12])                       # ties
+    x[3::24] = x[3::24].sort(-1).values                    # the winner comes last
+    x[4::24] = x[4::24].sort(-1, descending=True).values
+    x[7::24, : V // 2] = float("-inf")
+    x[8::24, 5] = float("inf")
+    x[9::24, 3] = float("nan")
+    x[10::24, 100:200] = float("nan")                      # with top-k 50 every survivor is NaN
+    x[13::24] = float("nan")
+    x[14::24] = float("-inf")
+    T[13::24], T[15::24] = 1e-6, 1e6
+    seeds = torch.randint(-(1 << 62), 1 << 62, (rows,), generator=g, device=cuda)
+    for k, p in ((None, None), (50, None), (300, None), (None, 0.9), (300, 0.9), (50, 0.9)):
+        tk = None if k is None else torch.full((rows,), k, dtype=torch.int32, device=cuda)
+        tp = None if p is None else torch.full((rows,), p, device=cuda)
+        ids, _, _ = ops.sample(x, T, seeds, tk, tp, debug=True)
+        assert torch.equal(ids, ops.sample(x, T, seeds, tk, tp)), (k, p)
