@@ -8,15 +8,20 @@
 //   both CTAs, warp 0 lane 0   TMA producer (cp.async.bulk.tensor ... cta_group::2: bytes complete on the LEADER's barrier)
 //   leader,    warp 1 lane 0   MMA issuer; tcgen05.commit ... multicast releases the smem stage / publishes the tile in BOTH CTAs
 //   both CTAs, warp 2          TMEM allocator (cta_group::2)
-//   both CTAs, warps 4-11      epilogue on the CTA's own 128 TMEM lanes, warps 8-11 the upper half of the columns; drained-signal goes
-//                              to the leader (remote mbarrier arrive).  With four warps the gated epilogue (an exponential and a
-//                              division per output, one warp per scheduler) outlasted a tile's 16 k-blocks at K = 1024: 13.4 K x 6144 x 1024
-//                              215 us, with eight 157 (K = 4096: no difference).
+//   both CTAs, warps 4-7       epilogue on the CTA's own 128 TMEM lanes; drained-signal goes to the leader (remote mbarrier arrive).
+//                              Gated outputs have warps 8-11 besides, on the upper half of the columns: with four warps their epilogue
+//                              (an exponential and a division per output, one warp per scheduler) outlasted a tile's 16 k-blocks at
+//                              K = 1024: 13.4 K x 6144 x 1024 215 us, with eight 157 (K = 4096: no difference).  A plain epilogue only
+//                              stores, and eight warps storing at once are slower than four: 32768 x 6144 x 1024 f32 512 us with four,
+//                              560 with eight; 13.4 K x 4096 x 1024 bf16 94 and 99.
 #include "tc.cuh"
 
 namespace nvllm {
 
-constexpr int kGemm2Threads = 384;
+template <int GATE>
+constexpr int gemm2_epilogue_warps() { return GATE != kGateNone ? 8 : 4; }
+template <int GATE>
+constexpr int gemm2_threads() { return 128 + 32 * gemm2_epilogue_warps<GATE>(); }
 
 template <int BN>
 struct Gemm2Cfg {
@@ -56,7 +61,7 @@ __device__ __forceinline__ void store_row32_2(OutT* dst, const uint32_t (&r)[32]
 // [BN/2, BN) are up for the same BN/2 output features, and the epilogue writes y[:, n_tile*BN/2 + c] = silu(gate)*up
 // (SiluAndMul::forward, activation.rs:46-63; or another gate of gated_pair) without the [M, 2N] intermediate ever reaching HBM.  N = output features.
 template <int BN, typename OutT, int GATE>
-__global__ void __launch_bounds__(kGemm2Threads, 1)
+__global__ void __launch_bounds__(gemm2_threads<GATE>(), 1)
 gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                          OutT* __restrict__ y, int M, int N, int K, int64_t ldy, int num_m_tiles, int num_tiles, float glu_limit) {
   using C = Gemm2Cfg<BN>;
@@ -91,7 +96,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tfull_bar(a), 1);     // each CTA: multicast commit
-      mbar_init(tempty_bar(a), 512);  // leader: 256 epilogue threads of each CTA
+      mbar_init(tempty_bar(a), 64 * gemm2_epilogue_warps<GATE>());  // leader: the epilogue threads of both CTAs
     }
     fence_barrier_init();
   }
@@ -146,7 +151,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
   } else if (warp >= 4) {
     // ===== epilogue (both CTAs): own 128 TMEM lanes -> global =====
     pdl_wait();
-    const int q = warp & 3, upper = (warp - 4) >> 2;
+    const int q = warp & 3;
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int tile = cluster_id; tile < num_tiles; tile += num_clusters) {
@@ -157,7 +162,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
       if constexpr (GATE != kGateNone) {
 #pragma unroll 1
-        for (int c = upper * (BN / 128); c < (upper ? BN / 64 : BN / 128); ++c) {
+        for (int c = warp < 8 ? 0 : BN / 128; c < (warp < 8 ? BN / 128 : BN / 64); ++c) {
           uint32_t g[32], u[32];
           tmem_ld_32x32b_x32(taddr + c * 32, g);
           tmem_ld_32x32b_x32(taddr + BN / 2 + c * 32, u);
@@ -176,7 +181,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
         }
       } else {
 #pragma unroll 1
-        for (int c = upper * (BN / 64); c < (upper + 1) * (BN / 64); ++c) {
+        for (int c = 0; c < BN / 32; ++c) {
           uint32_t r[32];
           tmem_ld_32x32b_x32(taddr + c * 32, r);
           tmem_ld_wait();
@@ -211,7 +216,7 @@ static int launch_gemm2(const CUtensorMap& tx, const CUtensorMap& tw, void* y, i
   const int clusters = num_tiles < max_clusters ? num_tiles : max_clusters;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(2 * clusters);
-  cfg.blockDim = dim3(kGemm2Threads);
+  cfg.blockDim = dim3(gemm2_threads<GATE>());
   cfg.dynamicSmemBytes = C::kSmemBytes;
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
