@@ -172,6 +172,18 @@ struct nvllm_runner {
   int init_weights(uint64_t seed, float std);
   int load_weight(const char* name, const void* h_bf16, int64_t rows, int64_t cols);
   int upload(const nvllm_batch& b, int padded);
+  // Up to 16 tokens: every norm rides in the projection behind it, every residual add in the one before it (gemm_skinny.cu), so h is
+  // the stream itself throughout.  The widths are those that the general path takes (it reports the others), and no more rows than
+  // tokens reach the head (a prefill batch may hold sequences without tokens).
+  bool few_tokens(int N, int S) const {
+    const int HD = H * D;
+    return tp == 1 && gemm_skinny_applies(N, hidden, hidden, hidden, hidden) && hidden % 64 == 0 && inter % 64 == 0 && HD % 64 == 0 &&
+           vshard % 8 == 0 && S <= N;
+  }
+  // where the q/k norm, the rotation and the store of a step's keys happen: in the qkv projection, or (decode) in the attention
+  // (few tokens: a launch costs more than the attention's longer prologue)
+  bool rope_in_qkv(int N, int S) const { return fuse_rope && !few_tokens(N, S) && D == 128 && N <= 256; }
+  bool rope_in_decode(int N, int S) const { return !rope_in_qkv(N, S) && (fuse_decode || (few_tokens(N, S) && D == 128)); }
   int forward(int n_tokens, int n_seqs, bool is_prefill, bool paged_prefill, const nvllm_batch& b);
   int execute_async(const nvllm_batch& b);
   int fetch(int64_t* out, int n);
@@ -663,11 +675,7 @@ int nvllm_runner::forward(int N, int S, bool is_prefill, bool paged_prefill, con
     mark("add_rmsnorm");
     return rc;
   };
-  // Up to 16 tokens: every norm rides in the projection behind it, every residual add in the one before it (gemm_skinny.cu), so h is
-  // the stream itself throughout.  The widths are those that the general path takes (it reports the others), and no more rows than
-  // tokens reach the head (a prefill batch may hold sequences without tokens).
-  const bool few = tp == 1 && gemm_skinny_applies(N, hidden, hidden, hidden, hidden) && hidden % 64 == 0 && inter % 64 == 0 && HD % 64 == 0 &&
-                   vshard % 8 == 0 && S <= N;
+  const bool few = few_tokens(N, S);   // no norm and no residual add of its own
   auto few_gemm = [&](void* y, const void* x, const void* w, int rows_n, int n, int k, int64_t ldy, int out_dt, bool gate, const bf16* norm, bool residual, const char* what) {
     ++launches;
     const int rc = gemm_skinny(y, x, w, rows_n, n, k, k, k, ldy, out_dt, gate, norm, eps, residual, stream);
@@ -687,7 +695,7 @@ int nvllm_runner::forward(int N, int S, bool is_prefill, bool paged_prefill, con
     const bf16* qnw = cfg.qk_norm ? w.q_norm : nullptr;
     const bf16* knw = cfg.qk_norm ? w.k_norm : nullptr;
     bool roped = false;  // q/k-norm + RoPE + KV store already applied to the qkv buffer / cache
-    if (fuse_rope && !few && D == 128 && N <= 256) {
+    if (rope_in_qkv(N, S)) {
       // decode-sized batches: qkv GEMM with q/k norm + RoPE + KV-cache store in its epilogue (one head per 128-wide tile)
       ++launches;
       RUN(nvllm_gemm_qkv_rope_store(qkv, normed, w.qkv, N, hidden, hidden, hidden, d_pos, rope, qnw, knw, eps, H, Hkv, D,
@@ -697,7 +705,7 @@ int nvllm_runner::forward(int N, int S, bool is_prefill, bool paged_prefill, con
     } else {
       if (few) RUN(few_gemm(qkv, h, w.qkv, N, qkv_dim, hidden, qkv_dim, NVLLM_BF16, false, w.input_ln, false, "norm + qkv_proj"));
       else RUN(gemm(qkv, normed, w.qkv, qkv_dim, hidden, qkv_dim, NVLLM_BF16, "qkv_proj GEMM"));
-      if (is_prefill || !(fuse_decode || (few && D == 128))) {   // (few: a launch costs more than the attention's longer prologue)
+      if (is_prefill || !rope_in_decode(N, S)) {
         // q/k norm + RoPE in place, K/V of this step into the cache (store before attention: note N2)
         RUN(nvllm_qknorm_rope_store(qkv, d_pos, rope, qnw, knw, eps, N, H, Hkv, D, cfg.max_position_embeddings, kc[l], vc[l],
                                     d_slots, &layout, NVLLM_BF16, st)); ++launches;
@@ -1040,7 +1048,7 @@ int nvllm_runner_time_decode_attention(nvllm_runner* r, int32_t iters, float* ms
   NVLLM_CHECK_ARG(r->last_decode_b > 0 && r->d_ctx != nullptr, NVLLM_ERR_STATE, "time_decode_attention: no decode step has run yet");
   const int B = r->last_decode_b, HD = r->H * r->D;
   const float scale = 1.0f / sqrtf(static_cast<float>(r->D));
-  const bool fused = r->fuse_decode && !(r->fuse_rope && r->D == 128 && B <= 256);  // the kernel the decode step launches
+  const bool fused = r->rope_in_decode(B, B);  // the kernel the decode step launches
   auto launch = [&](int l) {
     if (fused) {  // re-stores the step's K/V rows into the same slots: idempotent
       const auto& w = r->lw[l];

@@ -268,3 +268,55 @@ def test_gpu_engine_vs_hf_transformers_golden(cuda, which, arch, fixture):
         assert (err <= tol).all(), f"step {step}: GPU vs HF off by {(err / sig).max():.4f} sigma"
         sched.postprocess([f[step] if step < n_dec else 0 for f in gold["forced"]])
     print("max |GPU - HF| =", worst, "sigma")
+
+
+@pytest.mark.parametrize("arch,seqs", [("qwen3-0.6b", 3), ("qwen3-0.6b", 9), ("qwen3-0.6b", 16), ("qwen3-8b", 9), ("qwen3-8b", 16)])
+def test_fused_projections_of_few_tokens(cuda, arch, seqs, monkeypatch):
+    """Steps of up to 16 tokens norm inside the projections and add the residual in them (one and two groups of 8 tokens, hidden sizes
+    whose blocks of x stay in registers or do not, a head of CTAs that stay): the logits of the general path, up to the roundings that
+    another order of the sums flips."""
+    import torch
+    from nano_vllm_rs_b200 import engine as E
+    W, H, ff, tied = {"qwen3-0.6b": (1024, 16, 3072, True), "qwen3-8b": (4096, 32, 12288, False)}[arch]
+    layers, vocab, kv = 2, 15000, 8
+    rng = np.random.default_rng(seqs + W)
+    prompts = [rng.integers(0, vocab, 1).tolist() for _ in range(seqs)]
+    forced = rng.integers(0, vocab, (4, seqs))
+    shapes = {"model.embed_tokens.weight": (vocab, W), "model.norm.weight": (W,)}
+    if not tied:
+        shapes["lm_head.weight"] = (vocab, W)
+    for l in range(layers):
+        p = f"model.layers.{l}."
+        shapes.update({p + "input_layernorm.weight": (W,), p + "post_attention_layernorm.weight": (W,), p + "self_attn.q_norm.weight": (128,),
+                       p + "self_attn.k_norm.weight": (128,), p + "self_attn.q_proj.weight": (H * 128, W), p + "self_attn.k_proj.weight": (kv * 128, W),
+                       p + "self_attn.v_proj.weight": (kv * 128, W), p + "self_attn.o_proj.weight": (W, H * 128), p + "mlp.gate_proj.weight": (ff, W),
+                       p + "mlp.up_proj.weight": (ff, W), p + "mlp.down_proj.weight": (W, ff)})
+    gen = torch.Generator(device=cuda).manual_seed(seqs)
+    weights = {}
+    for name, shape in shapes.items():
+        x = torch.randn(shape, generator=gen, device=cuda)
+        x = 1.0 + 0.3 * x if "norm" in name else (x if "embed" in name else x * shape[-1] ** -0.5)
+        weights[name] = x.to(torch.bfloat16).view(torch.int16).cpu().numpy().view(np.uint16)
+    got = {}
+    for skinny in ("0", "1"):
+        monkeypatch.setenv("NVLLM_GEMM_SKINNY", skinny)
+        cfg = E.Config(arch, vocab_size=vocab, num_hidden_layers=layers, max_num_seqs=seqs, max_model_len=64, kvcache_block_size=16,
+                       num_kvcache_blocks=2 * seqs, enforce_eager=1).validate()
+        sched, runner = E.Scheduler(cfg), E.ModelRunner(cfg)
+        for name, w in weights.items():
+            runner.load_weight(name, w)
+        for p in prompts:
+            sched.add_sequence(p, E.SamplingParams(temperature=0.0, max_tokens=8, ignore_eos=True))
+        out = []
+        runner.profile()
+        for step in range(4):   # a prefill of one token a sequence, three decode steps
+            b = sched.schedule()
+            out.append(runner.execute_model(b, return_logits=True)[1])
+            sched.postprocess([int(t) for t in forced[step]])
+        assert ("norm + qkv_proj" in runner.profile_report()) == (skinny == "1")
+        got[skinny] = np.stack(out)
+    sig = got["0"].std(-1, keepdims=True)
+    err = np.abs(got["1"] - got["0"])
+    tol = LOGIT_SIGMA_PER_SQRT_LAYER * np.sqrt(layers) * sig + LOGIT_RTOL * np.abs(got["0"])
+    print((err / sig).max())
+    assert (err <= tol).all(), float((err / sig).max())

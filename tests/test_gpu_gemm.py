@@ -211,9 +211,10 @@ def test_gemm_splitk_silu_every_config_vs_oracle(cuda, cfg, monkeypatch):
 
 @pytest.mark.parametrize("m,n,k", [(256, 1024, 3072), (256, 1024, 2048), (4, 1024, 3072), (64, 2048, 4096), (1, 1024, 2048),
                                    (512, 768, 4096), (512, 4096, 6144), (300, 4096, 2048)])
-def test_gemm_splitk_auto_decode_shapes(cuda, m, n, k):
+def test_gemm_splitk_auto_decode_shapes(cuda, m, n, k, monkeypatch):
     """The shapes the cost model sends to split-K by default (Qwen3-0.6B o_proj / down_proj at decode) vs the check kernel."""
     from nano_vllm_rs_b200 import ops
+    monkeypatch.setenv("NVLLM_GEMM_SKINNY", "0")   # up to 16 rows they go elsewhere by default
     g = torch.Generator(device="cuda").manual_seed(m + n + k)
     x = torch.randn((m, k), generator=g, device=cuda).to(torch.bfloat16)
     w = (torch.randn((n, k), generator=g, device=cuda) * 0.02).to(torch.bfloat16)
