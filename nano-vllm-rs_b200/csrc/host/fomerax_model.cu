@@ -487,7 +487,7 @@ class Fomerax : public ModelBase {
             RUN(nvllm_linear(q_abs_, q_, L.ukT, N, R, L.D, HQ, L.D, HR, L.H, L.q_head(), static_cast<int64_t>(R) * L.D, R, dt_, NVLLM_F32, st));
             mk("q absorb (per-head linear)");
           }
-          RUN((v.n_tokens <= v.n_seqs ? nvllm_latent_token_attention : nvllm_latent_window_attention)(o_lat_, HR, q_abs_, HR, q_, HQ, v.tok_seq, v.positions, v.tables, v.table_cap, lim_.block_size, kv.lat, row, N,
+          RUN(nvllm_latent_step_attention(o_lat_, HR, q_abs_, HR, q_, HQ, v.tok_seq, v.positions, v.tables, v.table_cap, lim_.block_size, kv.lat, row, N, v.n_seqs,
                                             L.H, L.D, L.rot, R, L.scale, L.window, nullptr, nullptr, 0, lat_ws_, lat_ws_bytes_, dt_, st));
           mk("latent_window_attention");
           if (head_gemms) {

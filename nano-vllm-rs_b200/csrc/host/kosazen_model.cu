@@ -69,8 +69,7 @@ class Kosazen : public ModelImpl {
   std::vector<void*> cache_;  // per run
   std::map<std::pair<double, int>, float*> rope_tables_;
   // activations
-  float *h_ = nullptr, *q_abs_ = nullptr, *router_logits_ = nullptr, *topk_w_ = nullptr, *lat_ws_ = nullptr;
-  size_t lat_ws_bytes_ = 0;
+  float *h_ = nullptr, *q_abs_ = nullptr, *router_logits_ = nullptr, *topk_w_ = nullptr;
   void *normed_ = nullptr, *qd_ = nullptr, *o_lat_ = nullptr, *attn_ = nullptr, *proj_ = nullptr, *act_ = nullptr,
        *eout_ = nullptr, *xg_ = nullptr, *egu_buf_ = nullptr, *sgu_buf_ = nullptr, *sact_ = nullptr, *sout_ = nullptr, *moe_out_ = nullptr, *head_in_ = nullptr;
   int32_t *topk_idx_ = nullptr, *row_token_ = nullptr, *tile_expert_ = nullptr, *slot_row_ = nullptr;
@@ -223,9 +222,6 @@ class Kosazen : public ModelImpl {
       NVLLM_CUDA(cudaMemsetAsync(cache_[r], 0, n * esz_, stream));
     }
     RUN(dalloc(&h_, T * W)); RUN(oalloc(&normed_, T * W)); RUN(oalloc(&qd_, T * m_qd));
-    for (const Layer& L : layers_)   // partial softmaxes of single tokens whose keys are split over CTAs
-      for (int n = 1; n <= 256 && n <= static_cast<int>(T); ++n) lat_ws_bytes_ = std::max(lat_ws_bytes_, nvllm_latent_workspace_bytes(n, L.heads, L.kv_rank));
-    if (lat_ws_bytes_ > 0) RUN(dalloc(&lat_ws_, lat_ws_bytes_ / sizeof(float)));
     RUN(dalloc(&q_abs_, T * m_hr)); RUN(oalloc(&o_lat_, T * m_hr)); RUN(oalloc(&attn_, T * m_hv)); RUN(oalloc(&proj_, T * W));
     if (m_et > 0) {
       RUN(dalloc(&router_logits_, T * m_et)); RUN(dalloc(&topk_w_, T * m_top)); RUN(dalloc(&topk_idx_, T * m_top));
@@ -435,9 +431,9 @@ class Kosazen : public ModelImpl {
       } else {
         NVLLM_CUDA(cudaMemsetAsync(q_abs_, 0, static_cast<size_t>(N) * HR * 4, static_cast<cudaStream_t>(st)));
       }
-      RUN((v.n_tokens <= v.n_seqs ? nvllm_latent_token_attention : nvllm_latent_window_attention)(o_lat_, HR, q_abs_, HR, qd_, ldqd, v.tok_seq, v.positions, v.tables, v.table_cap, lim_.block_size,
-                                        cache_[r], L.cache_row(), N, L.heads, L.dim, L.rot_dim, L.kv_rank, L.scale, 0, nullptr, nullptr, 0,
-                                        lat_ws_, lat_ws_bytes_, dt_, st)); ++launches; mk("latent_attention");
+      RUN(nvllm_latent_step_attention(o_lat_, HR, q_abs_, HR, qd_, ldqd, v.tok_seq, v.positions, v.tables, v.table_cap, lim_.block_size,
+                                        cache_[r], L.cache_row(), N, v.n_seqs, L.heads, L.dim, L.rot_dim, L.kv_rank, L.scale, 0, nullptr, nullptr, 0,
+                                        nullptr, 0, dt_, st)); ++launches; mk("latent_attention");
       // values: per head Uv_h applied to the attended latent, then the output projection
       if (head_gemms) {
         for (int hh = 0; hh < L.heads; ++hh) {

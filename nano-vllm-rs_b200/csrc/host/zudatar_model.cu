@@ -592,8 +592,8 @@ class Zudatar : public ModelImpl {
             RUN(nvllm_linear(q_abs_, q_, L.ukT, N, R, L.D, HD, L.D, HR, L.H, L.D, static_cast<int64_t>(R) * L.D, R, dt_, NVLLM_F32, st)); ++launches;
             mk("q absorb (per-head linear)");
           }
-          RUN((v.n_tokens <= v.n_seqs ? nvllm_latent_token_attention : nvllm_latent_window_attention)(o_lat_, HR, q_abs_, HR, nullptr, 0, v.tok_seq, v.positions, v.tables, v.table_cap, lim_.block_size, cache,
-                                            L.cache_row(), N, L.H, L.D, 0, R, L.scale, L.window, L.sink, proj_ + L.q_rank + own, ldl, lat_ws_, lat_ws_bytes_,
+          RUN(nvllm_latent_step_attention(o_lat_, HR, q_abs_, HR, nullptr, 0, v.tok_seq, v.positions, v.tables, v.table_cap, lim_.block_size, cache,
+                                            L.cache_row(), N, v.n_seqs, L.H, L.D, 0, R, L.scale, L.window, L.sink, proj_ + L.q_rank + own, ldl, lat_ws_, lat_ws_bytes_,
                                             dt_, st));
           ++launches; mk("latent_window_attention");
           if (head_gemms) {

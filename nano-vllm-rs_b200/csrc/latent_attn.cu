@@ -233,7 +233,8 @@ __global__ void __launch_bounds__(128) latent_prepare_kernel(const PrepArgs a) {
 
 using AttnArgs = LatentAttnArgs;
 
-constexpr int kMaxLatentSplits = 32;
+constexpr int kMaxCluster = 8;        // the portable size
+constexpr int kShareTiles = 2;        // key tiles of a CTA of one, at least
 constexpr int kKeyTile = 32;
 
 // CTA = one query token x up to 8 heads (one warp per head).  Key tiles of 32 cache rows are staged once in shared memory
@@ -344,7 +345,9 @@ constexpr int kMmaKeys = 64, kPsStride = 72, kSsStride = 68, kMmaThreads = 256;
 // tokens of the batch; when they belong to the same sequence they share every key tile and every B fragment (the kernel is
 // bound by instruction issue and latency, not by the tensor pipe, so the second token is almost free); when they do not,
 // the CTA runs them one after the other.
-template <int NT2, int TQ>  // kv_rank padded to NT2 * 128
+// SKIP: behind the tcgen05 kernel, whose dense tiles are left out; a CTA may take several items.  (One instantiation with a loop for both
+// cost 1.5 us a launch: 40 tokens x 33 keys 8.8 -> 10.4 us.)
+template <int NT2, int TQ, bool SKIP>  // kv_rank padded to NT2 * 128
 __global__ void __launch_bounds__(kMmaThreads) latent_attn_mma_kernel(const AttnArgs a, int DPS, int DP16) {
   pdl_wait();
   pdl_launch_dependents();
@@ -371,15 +374,16 @@ __global__ void __launch_bounds__(kMmaThreads) latent_attn_mma_kernel(const Attn
       for (int e = tid; e < (16 - heads_here) * pad0; e += kMmaThreads)
         Qs[(q * 16 + heads_here + e / pad0) * DPS + e % pad0] = __float2bfloat16_rn(0.f);
   }
-  if (a.skip_dense) {   // usually every tile of the batch is dense: nothing to do
+  if (SKIP) {   // usually every tile of the batch is dense: nothing to do
     int left = 0;
     for (int t = tid; t * kLatentTileTokens < a.n; t += kMmaThreads) left |= !latent_tile_dense(a.tok_seq, a.n, t);
     if (!__syncthreads_or(left)) return;
   }
   const int items = (a.n + TQ - 1) / TQ;
-  for (int item = blockIdx.x; item < items; item += gridDim.x) {
+  int item = static_cast<int>(blockIdx.x);
+  do {
   const int tfirst = item * TQ;
-  if (a.skip_dense && latent_tile_dense(a.tok_seq, a.n, tfirst / kLatentTileTokens)) continue;
+  if (SKIP && latent_tile_dense(a.tok_seq, a.n, tfirst / kLatentTileTokens)) continue;
   bool together = false;
   if (TQ == 2 && tfirst + 1 < a.n) together = a.tok_seq[tfirst] == a.tok_seq[tfirst + 1];
   const int npass = (TQ == 1 || together || tfirst + 1 >= a.n) ? 1 : 2;
@@ -412,6 +416,18 @@ __global__ void __launch_bounds__(kMmaThreads) latent_attn_mma_kernel(const Attn
       if (jstart > nkeys) jstart = nkeys;
 #pragma unroll
       for (int q = 0; q < TQ; ++q) nk[q] = nk[q] < nkeys ? nk[q] : nkeys;
+    }
+    int shares = 1;   // CTAs of the cluster that have key tiles of this token (TQ == 1): the host only knows how long contexts may get
+    if (TQ == 1 && a.cluster > 1) {
+      const int tiles = (nkeys - jstart + kMmaKeys - 1) / kMmaKeys, most = max(1, min(a.cluster, tiles / kShareTiles));
+      const int per = (tiles + most - 1) / most, z = static_cast<int>(blockIdx.z);
+      shares = per > 0 ? (tiles + per - 1) / per : 1;
+      if (shares == 1 && z > 0) continue;   // (the whole cluster agrees: nobody waits for this CTA)
+      if (shares > 1) {
+        jstart = min(jstart + z * per * kMmaKeys, nkeys);
+        nkeys = min(nkeys, jstart + per * kMmaKeys);
+        nk[0] = min(nk[0], nkeys);
+      }
     }
     __syncthreads();   // previous pass done with every buffer; the zero fill above is ordered before the copies below
     if (tid < TQ * 16) { m_s[tid] = -INFINITY; l_s[tid] = 0.f; c_s[tid] = 1.f; }
@@ -611,6 +627,66 @@ __global__ void __launch_bounds__(kMmaThreads) latent_attn_mma_kernel(const Attn
       }
       continue;
     }
+    if (TQ == 1 && shares > 1) {   // the partial softmaxes of the cluster meet in distributed shared memory, summed in rank order
+      constexpr int PW = RC * 8 + 8;   // row pitch of the parked values
+      float* part = reinterpret_cast<float*>(Kbuf);
+      cp_async_wait<0>();
+      __syncthreads();   // a share without tiles never entered the loop: its first copy (zeros) may still be on its way
+#pragma unroll
+      for (int nt = 0; nt < 2 * NT2; ++nt) {
+        const int col = warp * RC + nt * 8 + 2 * t4;
+        *reinterpret_cast<float2*>(part + g * PW + col) = make_float2(acc[0][nt][0], acc[0][nt][1]);
+        *reinterpret_cast<float2*>(part + (g + 8) * PW + col) = make_float2(acc[0][nt][2], acc[0][nt][3]);
+      }
+      cluster_sync();
+      if (tid < 16) {   // Ss: the factor of every share on row tid
+        const uint32_t m_at = smem_u32(m_s + tid), l_at = smem_u32(l_s + tid);
+        const int h = hbase + tid;
+        const float sk = a.sinks && h < a.heads ? a.sinks[h] : -INFINITY;
+        float mx = sk, ms[kMaxCluster], ls[kMaxCluster];
+#pragma unroll
+        for (int s = 0; s < kMaxCluster; ++s)
+          if (s < shares) { ms[s] = ld_peer_f32(m_at, s); ls[s] = ld_peer_f32(l_at, s); }
+#pragma unroll
+        for (int s = 0; s < kMaxCluster; ++s)
+          if (s < shares) mx = fmaxf(mx, ms[s]);
+        float den = a.sinks ? expf(sk - mx) : 0.f;
+#pragma unroll
+        for (int s = 0; s < kMaxCluster; ++s) {
+          if (s >= shares) continue;
+          const float fs = ms[s] != -INFINITY ? expf(ms[s] - mx) : -1.f;   // -1: the share has no key of this row
+          if (ms[s] != -INFINITY) den = fmaf(fs, ls[s], den);
+          Ss[s * 16 + tid] = fs;
+        }
+        float inv = den > 0.f ? 1.0f / den : 0.f;
+        if (a.gate && h < a.heads) inv *= 1.0f / (1.0f + expf(-a.gate[static_cast<int64_t>(tq[0]) * a.ldg + h]));
+        c_s[tid] = inv;
+      }
+      __syncthreads();
+      const int cols4 = (a.kv_rank + 3) / 4;
+      for (int e = static_cast<int>(blockIdx.z) * kMmaThreads + tid; e < heads_here * cols4; e += a.cluster * kMmaThreads) {
+        const int r = e / cols4, c = 4 * (e - r * cols4);
+        const uint32_t at = smem_u32(part + r * PW + c);
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f), x[kMaxCluster];
+#pragma unroll
+        for (int s = 0; s < kMaxCluster; ++s)
+          if (s < shares) x[s] = ld_peer_f32x4(at, s);
+#pragma unroll
+        for (int s = 0; s < kMaxCluster; ++s) {
+          const float fs = s < shares ? Ss[s * 16 + r] : -1.f;
+          if (!(fs < 0.f)) v = make_float4(fmaf(fs, x[s].x, v.x), fmaf(fs, x[s].y, v.y), fmaf(fs, x[s].z, v.z), fmaf(fs, x[s].w, v.w));
+        }
+        const float inv = c_s[r], o[4] = {v.x * inv, v.y * inv, v.z * inv, v.w * inv};
+        bf16* dst = static_cast<bf16*>(a.out) + static_cast<int64_t>(tq[0]) * a.ldo + static_cast<int64_t>(hbase + r) * a.kv_rank + c;
+        if (c + 4 <= a.kv_rank && (reinterpret_cast<uintptr_t>(dst) & 7u) == 0) {
+          *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
+        } else {
+          for (int i = 0; i < 4 && c + i < a.kv_rank; ++i) dst[i] = __float2bfloat16_rn(o[i]);
+        }
+      }
+      cluster_sync();   // nobody leaves, or parks its next token, while a peer still reads
+      continue;
+    }
 #pragma unroll
     for (int q = 0; q < TQ; ++q) {
       if (tq[q] < 0) continue;
@@ -637,7 +713,7 @@ __global__ void __launch_bounds__(kMmaThreads) latent_attn_mma_kernel(const Attn
       }
     }
   }
-  }
+  } while (SKIP && (item += static_cast<int>(gridDim.x)) < items);
 }
 
 // One warp per (token, head): merges the splits' partial softmaxes, adds the sink to the denominator, applies the gate.
@@ -671,23 +747,52 @@ __global__ void __launch_bounds__(128) latent_attn_merge_kernel(const AttnArgs a
   }
 }
 
-template <int NT2, int TQ>
+template <int NT2, int TQ, bool SKIP>
 int launch_attn_mma_tq(const AttnArgs& a, cudaStream_t st) {
   const int DP16 = (static_cast<int>(a.cache_row) + 15) / 16 * 16, RP = NT2 * 128;
   const int DPS = (DP16 > RP ? DP16 : RP) + 8;
   const size_t smem = static_cast<size_t>(TQ * 16 + 2 * kMmaKeys) * DPS * 2 + TQ * 16 * kPsStride * 2 +
                       (TQ * 2 * 16 * kSsStride + TQ * 48) * 4;
-  NVLLM_SMEM_ATTR_ONCE((latent_attn_mma_kernel<NT2, TQ>), 225 * 1024);
+  auto kern = latent_attn_mma_kernel<NT2, TQ, SKIP>;
+  NVLLM_SMEM_ATTR_ONCE(kern, 225 * 1024);
   const int items = (a.n + TQ - 1) / TQ, groups = (a.heads + 15) / 16;
   // behind the tcgen05 kernel a launch with nothing to do should cost little: no more CTAs than run at once
-  dim3 grid(a.skip_dense ? std::min(items, std::max(1, sm_count() / groups)) : items, groups, TQ == 1 && a.splits > 1 ? a.splits : 1);
-  NVLLM_CUDA(launch_plain(latent_attn_mma_kernel<NT2, TQ>, dim3(grid), dim3(kMmaThreads), smem, st, a, DPS, DP16));
+  const dim3 grid(SKIP ? std::min(items, std::max(1, sm_count() / groups)) : items, groups, TQ == 1 ? std::max(a.splits, a.cluster) : 1);
+  if (TQ == 1 && a.cluster > 1) NVLLM_CUDA(launch_plain_cluster_z(kern, grid, dim3(kMmaThreads), smem, st, a, DPS, DP16));
+  else NVLLM_CUDA(launch_plain(kern, grid, dim3(kMmaThreads), smem, st, a, DPS, DP16));
   NVLLM_LAUNCH_CHECK("latent_attn_mma_kernel");
   if (TQ == 1 && a.splits > 1) {
     NVLLM_CUDA(launch_pdl(latent_attn_merge_kernel, dim3(static_cast<unsigned>((static_cast<int64_t>(a.n) * a.heads + 3) / 4)), dim3(128), 0, st, a));
     NVLLM_LAUNCH_CHECK("latent_attn_merge_kernel");
   }
   return 0;
+}
+
+// The largest cluster (at most 8, the portable size) of which `clusters` run at once, one CTA an SM: what the GPCs hold, not what the
+// SMs add up to (a cluster that waits for another one's end doubles the kernel's time).
+template <int NT2>
+int cluster_that_fits(int64_t clusters) {
+  static std::once_flag once;
+  static int room[kMaxCluster + 1];
+  std::call_once(once, [] {
+    auto kern = latent_attn_mma_kernel<NT2, 1, false>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024) != cudaSuccess) { (void)cudaGetLastError(); return; }
+    for (int s = 2; s <= kMaxCluster; ++s) {
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3(1, 1, s);
+      cfg.blockDim = dim3(kMmaThreads);
+      cfg.dynamicSmemBytes = 225 * 1024;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = s;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&room[s], kern, &cfg) != cudaSuccess) { (void)cudaGetLastError(); room[s] = 0; }
+    }
+  });
+  int s = kMaxCluster;
+  while (s > 1 && room[s] < clusters) --s;
+  return s;
 }
 
 // Two tokens per CTA for batches that are mostly prompt portions (more than 256 tokens: a decode batch holds one token per
@@ -697,8 +802,21 @@ int launch_attn_mma(const AttnArgs& a, cudaStream_t st) {
   const int DP16 = (static_cast<int>(a.cache_row) + 15) / 16 * 16, RP = NT2 * 128;
   const int DPS = (DP16 > RP ? DP16 : RP) + 8;
   const size_t smem2 = static_cast<size_t>(32 + 2 * kMmaKeys) * DPS * 2 + 32 * kPsStride * 2 + (4 * 16 * kSsStride + 96) * 4;
-  if (a.n > 256 && knobs().latent_mma != 2 && smem2 <= 225 * 1024) { AttnArgs b = a; b.splits = 1; return launch_attn_mma_tq<NT2, 2>(b, st); }
-  return launch_attn_mma_tq<NT2, 1>(a, st);
+  if (a.n > 256 && knobs().latent_mma != 2 && smem2 <= 225 * 1024) {
+    AttnArgs b = a;
+    b.splits = 1;
+    return a.skip_dense ? launch_attn_mma_tq<NT2, 2, true>(b, st) : launch_attn_mma_tq<NT2, 2, false>(b, st);
+  }
+  // Single tokens without a window on fewer CTAs than SMs: a cluster shares the key tiles of a token, as many CTAs as give each (at the
+  // longest context the tables allow; the kernel looks at the token's own) kShareTiles tiles.  Measured, 16 heads, rank 512 (us, one CTA a
+  // token -> so): 1 token at 4001 keys 218 -> 36, 32 at 4001 221 -> 68, 11 at 279 22.0 -> 16.2, 40 at 33 9.0 -> 9.2.  With partials in
+  // memory and a second kernel, whose cost follows the splits that the tables allow, 1 token at 33 keys in tables for 4096 took 36.
+  AttnArgs b = a;
+  if (a.n <= 256 && a.window == 0) {
+    const int64_t tiles = (static_cast<int64_t>(a.table_cap) * a.block_size + kMmaKeys - 1) / kMmaKeys;
+    b.cluster = static_cast<int>(std::min<int64_t>(cluster_that_fits<NT2>(static_cast<int64_t>(a.n) * ((a.heads + 15) / 16)), std::max<int64_t>(1, tiles / kShareTiles)));
+  }
+  return a.skip_dense ? launch_attn_mma_tq<NT2, 1, true>(b, st) : launch_attn_mma_tq<NT2, 1, false>(b, st);
 }
 
 template <typename T>
@@ -830,38 +948,38 @@ extern "C" int nvllm_latent_attention(void* out, int64_t ldo, const float* q_abs
                                        cache_row, n, heads, dim, rot_dim, kv_rank, scale, 0, nullptr, nullptr, 0, nullptr, 0, dtype, stream);
 }
 
-extern "C" size_t nvllm_latent_workspace_bytes(int32_t n, int32_t heads, int32_t kv_rank) {
-  if (n <= 0 || n > 256 || heads <= 0 || kv_rank <= 0) return 0;
-  const int splits = std::min(kMaxLatentSplits, sm_count() / (n * ((heads + 15) / 16)));
-  return splits > 1 ? static_cast<size_t>(n) * heads * splits * (kv_rank + 2) * sizeof(float) : 0;
-}
+extern "C" size_t nvllm_latent_workspace_bytes(int32_t, int32_t, int32_t) { return 0; }
 
 namespace {
-// single_tokens: the caller knows that (nearly) every sequence has one token in the batch.  A batch of 32 and more of them would be
-// offered to the tcgen05 kernel first, a launch that finds no dense tile and that the next one waits for.
-int run_attention(const AttnArgs& a, size_t workspace_bytes, int dtype, bool single_tokens, cudaStream_t st) {
+// n_seqs: how many sequences the batch holds, 0 if the caller does not say.  The tcgen05 kernel takes batches whose tokens would need more
+// than one round of CTAs here (with fewer, the clusters of the mma.sync kernel are done sooner: 64 tokens of a prompt at 1000 keys 56 us
+// there, 34 here; 256 tokens 56 and 113), and whose sequences have a tile of tokens each: single tokens and short portions leave it no
+// dense tile, and tiles of two sequences walk both (9 x 14 tokens x 32 heads at 1000 keys 132 us there, 119 here).
+bool prompts_worth_a_launch(const AttnArgs& a, int n_seqs) {
+  const int64_t ctas = static_cast<int64_t>(a.n) * ((a.heads + 15) / 16);
+  return ctas > sm_count() && (n_seqs <= 0 || a.n / n_seqs >= 16 || (a.n / n_seqs >= 8 && ctas > 2 * sm_count()));
+}
+
+int run_attention(const AttnArgs& a, size_t workspace_bytes, int dtype, int n_seqs, cudaStream_t st) {
   // bf16 caches with a 16-byte row pitch and kv_rank <= 512 run on the tensor cores (NVLLM_LATENT_MMA=0: the CUDA-core kernel)
   const int dp16 = (static_cast<int>(a.cache_row) + 15) / 16 * 16;
   if (dtype == NVLLM_BF16 && knobs().latent_mma != 0 && a.kv_rank <= 512 && a.cache_row % 8 == 0 && dp16 <= 704 &&
       (reinterpret_cast<uintptr_t>(a.cache) & 15u) == 0) {
     AttnArgs b = a;
-    if (!single_tokens && knobs().latent_mma == 1 && latent_attn_tc_applies(a)) {
+    if (knobs().latent_mma == 1 && prompts_worth_a_launch(a, n_seqs) && latent_attn_tc_applies(a)) {
       if (int rc = latent_attn_tc_launch(a, st)) return rc;
       b.skip_dense = 1;   // tiles of many sequences are left to the kernel below
     }
-    // Single tokens on fewer CTAs than SMs: the key tiles of a token are split over CTAs along z, as many as fill the SMs once and
-    // leave each (at the longest context the tables or the window allow) at least four tiles; the partials meet in
-    // latent_attn_merge_kernel.  Measured, 32 tokens x 16 heads at 4001 keys, rank 512: 223 -> 104 us.  64 tokens in a window of
-    // 2048 keys 118 -> 79 us; in one of 512 the second launch costs what the shorter loop saves (39 -> 37 us), hence eight tiles for
-    // windows.
-    if (a.part != nullptr && a.n <= 256) {
+    // Single tokens with a bounded key range (a window) and fewer CTAs than SMs: split every token's key tiles over up to 4
+    // CTAs, as many as fill the SMs once and leave each at least eight tiles; the partials meet in latent_attn_merge_kernel.
+    // (Measured, 64 tokens x 16 heads, rank 512: a window of 2048 keys 118 -> 79 us; at 512 keys the second launch costs what
+    // the shorter loop saves, 39 -> 37 us, so short windows stay on one CTA.)
+    if (a.part != nullptr && a.n <= 256 && a.window > 0) {
       const int64_t ctas = static_cast<int64_t>(a.n) * ((a.heads + 15) / 16);
-      const int64_t reach = a.window > 0 ? a.window + kMmaKeys - 1 : static_cast<int64_t>(a.table_cap) * a.block_size;
-      const int tiles = static_cast<int>(std::min<int64_t>((reach + kMmaKeys - 1) / kMmaKeys, 1 << 20));
       int splits = static_cast<int>(sm_count() / (ctas > 0 ? ctas : 1));
-      splits = std::min(splits, a.window > 0 ? std::min(4, tiles / 8) : std::min(kMaxLatentSplits, tiles / 4));
-      splits = static_cast<int>(std::min<size_t>(splits, workspace_bytes / (static_cast<size_t>(a.n) * a.heads * (a.kv_rank + 2) * sizeof(float))));
-      if (splits > 1) b.splits = splits;
+      const int tiles = (a.window + 2 * kMmaKeys - 2) / kMmaKeys;   // tiles a window can touch
+      splits = std::min(4, std::min(splits, tiles / 8));
+      if (splits > 1 && static_cast<size_t>(a.n) * a.heads * splits * (a.kv_rank + 2) * sizeof(float) <= workspace_bytes) b.splits = splits;
     }
     if (a.kv_rank <= 128) return launch_attn_mma<1>(b, st);
     if (a.kv_rank <= 256) return launch_attn_mma<2>(b, st);
@@ -874,7 +992,7 @@ int run_attention(const AttnArgs& a, size_t workspace_bytes, int dtype, bool sin
 int window_attention(void* out, int64_t ldo, const float* q_abs, int64_t ldqa, const void* q, int64_t ldq, const int32_t* tok_seq,
                      const int64_t* positions, const int32_t* block_tables, int32_t table_cap, int32_t block_size, const void* cache,
                      int64_t cache_row, int32_t n, int32_t heads, int32_t dim, int32_t rot_dim, int32_t kv_rank, float scale, int32_t window,
-                     const float* sinks, const float* gate, int64_t ldg, void* workspace, size_t workspace_bytes, int32_t dtype, bool single_tokens,
+                     const float* sinks, const float* gate, int64_t ldg, void* workspace, size_t workspace_bytes, int32_t dtype, int n_seqs,
                      void* stream) {
   NVLLM_CHECK_ARG(n >= 0 && heads > 0 && dim >= 0 && rot_dim >= 0 && kv_rank > 0 && kv_rank <= 1024 && table_cap > 0 && block_size > 0,
                   NVLLM_ERR_ARG, "latent_attention: sizes (kv_rank <= 1024)");
@@ -882,8 +1000,8 @@ int window_attention(void* out, int64_t ldo, const float* q_abs, int64_t ldqa, c
   if (n == 0) return 0;
   NVLLM_CHECK_ARG(out && q_abs && (q || rot_dim == 0) && tok_seq && positions && block_tables && cache, NVLLM_ERR_ARG, "latent_attention: NULL");
   const AttnArgs a{out, ldo, q_abs, ldqa, q ? q : q_abs, ldq, tok_seq, positions, block_tables, table_cap, block_size, cache, cache_row,
-                   n, heads, dim, rot_dim, kv_rank, scale, window > 0 ? window : 0, sinks, gate, ldg, 1, static_cast<float*>(workspace), 0};
-  return run_attention(a, workspace_bytes, dtype, single_tokens, static_cast<cudaStream_t>(stream));
+                   n, heads, dim, rot_dim, kv_rank, scale, window > 0 ? window : 0, sinks, gate, ldg, 1, static_cast<float*>(workspace), 1, 0};
+  return run_attention(a, workspace_bytes, dtype, n_seqs, static_cast<cudaStream_t>(stream));
 }
 }  // namespace
 
@@ -894,15 +1012,16 @@ extern "C" int nvllm_latent_window_attention(void* out, int64_t ldo, const float
                                              int32_t window, const float* sinks, const float* gate, int64_t ldg, void* workspace,
                                              size_t workspace_bytes, int32_t dtype, void* stream) {
   return window_attention(out, ldo, q_abs, ldqa, q, ldq, tok_seq, positions, block_tables, table_cap, block_size, cache, cache_row, n, heads, dim,
-                          rot_dim, kv_rank, scale, window, sinks, gate, ldg, workspace, workspace_bytes, dtype, false, stream);
+                          rot_dim, kv_rank, scale, window, sinks, gate, ldg, workspace, workspace_bytes, dtype, 0, stream);
 }
 
-extern "C" int nvllm_latent_token_attention(void* out, int64_t ldo, const float* q_abs, int64_t ldqa, const void* q, int64_t ldq,
-                                            const int32_t* tok_seq, const int64_t* positions, const int32_t* block_tables,
-                                            int32_t table_cap, int32_t block_size, const void* cache, int64_t cache_row, int32_t n,
-                                            int32_t heads, int32_t dim, int32_t rot_dim, int32_t kv_rank, float scale,
-                                            int32_t window, const float* sinks, const float* gate, int64_t ldg, void* workspace,
-                                            size_t workspace_bytes, int32_t dtype, void* stream) {
+extern "C" int nvllm_latent_step_attention(void* out, int64_t ldo, const float* q_abs, int64_t ldqa, const void* q,
+                                           int64_t ldq, const int32_t* tok_seq, const int64_t* positions,
+                                           const int32_t* block_tables, int32_t table_cap, int32_t block_size,
+                                           const void* cache, int64_t cache_row, int32_t n, int32_t n_seqs,
+                                           int32_t heads, int32_t dim, int32_t rot_dim, int32_t kv_rank, float scale,
+                                           int32_t window, const float* sinks, const float* gate, int64_t ldg,
+                                           void* workspace, size_t workspace_bytes, int32_t dtype, void* stream) {
   return window_attention(out, ldo, q_abs, ldqa, q, ldq, tok_seq, positions, block_tables, table_cap, block_size, cache, cache_row, n, heads, dim,
-                          rot_dim, kv_rank, scale, window, sinks, gate, ldg, workspace, workspace_bytes, dtype, true, stream);
+                          rot_dim, kv_rank, scale, window, sinks, gate, ldg, workspace, workspace_bytes, dtype, n_seqs, stream);
 }

@@ -16,6 +16,7 @@ struct LatentAttnArgs {
   float scale;
   int window; const float* sinks; const float* gate; int64_t ldg;   // 0 / null: none
   int splits; float* part;   // splits > 1: CTAs along z share a token's key tiles; partial (acc[kv_rank], m, l) per (token, head, split)
+  int cluster;               // cluster > 1: so does a cluster of that many CTAs along z, without partials in memory
   int skip_dense;            // the tcgen05 kernel takes the dense 8-token tiles of the batch (latent_tile_dense), this launch the others
 };
 
@@ -23,8 +24,8 @@ constexpr int kLatentTileTokens = 8;
 
 // A tile of 8 consecutive tokens of the batch is dense when the 8 tokens that end with its last one belong to at most two sequences:
 // prompts and portions of prompts, not single decoded tokens.  (A short last tile is judged with the tokens in front of it: one or two
-// tokens are always of two sequences at most, and 33 single tokens at 4001 keys took 311 us with the last one walking its keys alone
-// on the tcgen05 kernel, 105 so; the end of a prompt stays dense.)
+// tokens are always of two sequences at most, and 33 single tokens at 4001 keys took 290 us, 34 477, with the last ones walking their
+// keys alone on the tcgen05 kernel, 32 took 98; the end of a prompt stays dense.)
 __device__ __forceinline__ bool latent_tile_dense(const int32_t* __restrict__ tok_seq, int n, int tile) {
   const int t1 = min(n, (tile + 1) * kLatentTileTokens), t0 = max(0, t1 - kLatentTileTokens);
   int runs = 1;

@@ -322,13 +322,9 @@ def latent_prepare(q, dkv, c_norm_w, eps, positions, table, rot_dims, heads, dim
 def latent_attention(q_abs, q, tok_seq, positions, tables, block_size, cache, heads, dim, rot_dim, kv_rank, scale):
     n = q.shape[0]
     out = torch.empty((n, heads * kv_rank), dtype=q.dtype, device=q.device)
-    need, ws = 0, None   # of single tokens whose keys are split over CTAs: four tiles of 64 keys or more each, so none below eight tiles
-    if tables.shape[1] * block_size > 448 and n <= 256 and q.dtype == torch.bfloat16:
-        need = _ffi.lib().nvllm_latent_workspace_bytes(n, heads, kv_rank)
-        ws = torch.empty(need, dtype=torch.uint8, device=q.device) if need else None
-    check(_latent_entry(n, tables)(_p(out), out.stride(0), _p(q_abs), q_abs.stride(0), _p(q), q.stride(0), _p(tok_seq),
-                                   _p(positions), _p(tables), tables.shape[1], block_size, _p(cache), cache.stride(0), n,
-                                   heads, dim, rot_dim, kv_rank, scale, 0, None, None, 0, _p(ws), need, _dt(q), _stream()))
+    check(_ffi.lib().nvllm_latent_step_attention(_p(out), out.stride(0), _p(q_abs), q_abs.stride(0), _p(q), q.stride(0), _p(tok_seq),
+                                                 _p(positions), _p(tables), tables.shape[1], block_size, _p(cache), cache.stride(0), n, tables.shape[0],
+                                                 heads, dim, rot_dim, kv_rank, scale, 0, None, None, 0, None, 0, _dt(q), _stream()))
     return out
 
 
@@ -541,20 +537,15 @@ def window_attention(q, gate, k_cache, v_cache, tok_seq, positions, tables, bloc
     return out
 
 
-def _latent_entry(n, tables):
-    """As many sequences as tokens: single tokens, as in a decode step."""
-    return _ffi.lib().nvllm_latent_token_attention if n <= tables.shape[0] else _ffi.lib().nvllm_latent_window_attention
-
-
 def latent_window_attention(q_abs, tok_seq, positions, tables, block_size, cache, heads, kv_rank, scale, dtype, window=0, sinks=None,
                             gate=None, workspace=None):
     """q_abs f32 [n, heads * kv_rank] (the key map folded into the query); cache [slots, row >= kv_rank] in `dtype`."""
     n = q_abs.shape[0]
     out = torch.empty((n, heads * kv_rank), dtype=dtype, device=q_abs.device)
-    check(_latent_entry(n, tables)(_p(out), out.stride(0), _p(q_abs), q_abs.stride(0), None, 0, _p(tok_seq), _p(positions),
-                                   _p(tables), tables.shape[1], block_size, _p(cache), cache.stride(0), n, heads, 0, 0,
-                                   kv_rank, scale, window, _p(sinks), _p(gate), gate.stride(0) if gate is not None else 0,
-                                   _p(workspace), workspace.numel() * 4 if workspace is not None else 0, _dt(out), _stream()))
+    check(_ffi.lib().nvllm_latent_step_attention(_p(out), out.stride(0), _p(q_abs), q_abs.stride(0), None, 0, _p(tok_seq), _p(positions),
+                                                 _p(tables), tables.shape[1], block_size, _p(cache), cache.stride(0), n, tables.shape[0], heads, 0, 0,
+                                                 kv_rank, scale, window, _p(sinks), _p(gate), gate.stride(0) if gate is not None else 0,
+                                                 _p(workspace), workspace.numel() * 4 if workspace is not None else 0, _dt(out), _stream()))
     return out
 
 
@@ -824,10 +815,10 @@ def latent_rotary_attention(q_abs, q, tok_seq, positions, tables, block_size, ca
     """latent_window_attention whose cache rows also hold a rotated key part; q [n, heads * (dim + rot_dim)]."""
     n = q_abs.shape[0]
     out = torch.empty((n, heads * kv_rank), dtype=q.dtype, device=q_abs.device)
-    check(_latent_entry(n, tables)(_p(out), out.stride(0), _p(q_abs), q_abs.stride(0), _p(q), q.stride(0), _p(tok_seq), _p(positions),
-                                   _p(tables), tables.shape[1], block_size, _p(cache), cache.stride(0), n, heads, dim, rot_dim, kv_rank,
-                                   scale, window, None, None, 0, _p(workspace), workspace.numel() * 4 if workspace is not None else 0,
-                                   _dt(out), _stream()))
+    check(_ffi.lib().nvllm_latent_step_attention(_p(out), out.stride(0), _p(q_abs), q_abs.stride(0), _p(q), q.stride(0), _p(tok_seq), _p(positions),
+                                                 _p(tables), tables.shape[1], block_size, _p(cache), cache.stride(0), n, tables.shape[0], heads, dim, rot_dim, kv_rank,
+                                                 scale, window, None, None, 0, _p(workspace), workspace.numel() * 4 if workspace is not None else 0,
+                                                 _dt(out), _stream()))
     return out
 
 
