@@ -48,6 +48,9 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 
 int sm_count();  // api.cu (cached)
 
+// Kernels that a paged decode attention of these sizes launches (paged_decode.cu; one, or two with partials in memory)
+int paged_decode_launches(int batch, int heads, int kv_heads, int splits, bool fused);
+
 // Projections of up to 16 tokens (gemm_skinny.cu): y = x . w^T as nvllm_gemm_bf16 / nvllm_gemm_silu_mul_bf16; norm_w: x is normed
 // first (bf16 weights, k columns); residual: y += the bf16 product, in place.
 bool gemm_skinny_applies(int m, int n, int k, int64_t ldx, int64_t ldw);

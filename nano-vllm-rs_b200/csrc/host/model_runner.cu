@@ -722,7 +722,7 @@ int nvllm_runner::forward(int N, int S, bool is_prefill, bool paged_prefill, con
         RUN(nvllm_paged_decode_attention(attn, qkv, kc[l], vc[l], d_tables, d_ctx, N, H, table_cap, qkv_dim, HD, &layout,
                                          scale, decode_ws, decode_ws_bytes, splits, NVLLM_BF16, st));
       }
-      launches += splits > 16 ? 2 : 1;   // (up to 16 splits merge inside the kernel)
+      launches += paged_decode_launches(N, H, Hkv, splits, !roped);
       mark(roped ? "paged_decode_attention" : "paged_decode_attention (+ q/k-norm, RoPE, KV store)");
     } else {
       RUN(nvllm_varlen_prefill_attention(attn, qkv, qkv + HD, qkv + HD + Hkv * D, d_cu_q, d_cu_k, S, N, N, b.max_seqlen_q,

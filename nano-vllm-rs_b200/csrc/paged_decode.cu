@@ -19,8 +19,9 @@
 //   P^T -> B operand through movmatrix.trans (8x8 b16 transpose inside the warp)
 //   O^T[D x 8 heads] += V^T[D x 16 tok] . P^T[16 x 8]        (A = V via ldmatrix.trans)
 //   No padding waste for g = 8, 2x for g = 4, 4x for g = 2 — the tensor pipe is idle otherwise.
-// Epilogue: warps merge (m, l, O) through shared memory; with one split the CTA writes bf16 output,
-//   otherwise fp32 partials + (m, l) go to the workspace and paged_decode_reduce_kernel combines.
+// Epilogue: warps merge (m, l, O) through shared memory; with one split the CTA writes bf16 output.  Up to 16 splits that fit the
+//   GPCs are a cluster (FUSE) and meet in distributed shared memory; otherwise fp32 partials + (m, l) go to the workspace and
+//   paged_decode_reduce_kernel combines them.
 //
 // Algorithmic bytes per launch: sum_b 2*L_b*Hkv*D*2 + 2*B*H*D*2 + 4*sum_b ceil(L_b/bs) + 4*B.
 #include <math.h>
@@ -43,7 +44,6 @@ struct DecodeParams {
   float* ws_o;   // [B, H, S, D]
   float* ws_ml;  // [B, H, S, 2]
   int batch, H, Hkv, g, ngrp, max_blocks, block_size, num_splits;
-  int cluster;  // the splits of an item are one cluster and merge over distributed shared memory (no partials in memory, no second kernel)
   int64_t q_stride, out_stride, blk_stride, tok_stride, head_stride;
   float scale_log2;
   // FUSE only (nvllm_paged_decode_attention_fused): q points at the packed [q | k | v] rows of this step; the kernel applies
@@ -57,6 +57,7 @@ struct DecodeParams {
   const int32_t* slots;
   float eps;
   int max_position;
+  int cluster = 0;  // FUSE: the splits of an item are one cluster and merge over distributed shared memory (no partials, no second kernel)
 };
 
 template <int D, int STAGES, int NWARPS>
@@ -87,6 +88,7 @@ paged_decode_kernel(const DecodeParams p) {
   constexpr int KS = D / 16;  // k-steps of QK^T == m-tiles of PV
   extern __shared__ __align__(128) uint8_t smem[];
 
+  if (!FUSE) pdl_launch_dependents();
   const int split = blockIdx.x;
   const int kvh = blockIdx.y / p.ngrp;
   const int grp = blockIdx.y - kvh * p.ngrp;
@@ -94,7 +96,7 @@ paged_decode_kernel(const DecodeParams p) {
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   pdl_wait();  // q and the newest KV row were written by the previous kernel
-  pdl_launch_dependents();   // (not earlier: see gemm_skinny.cu)
+  if (FUSE) pdl_launch_dependents();   // (steps of few tokens: not earlier, see gemm_skinny.cu)
   const int ctx_all = __ldg(p.ctx + b);        // tokens attended to, including (FUSE) this step's own
   const int ctx = FUSE ? max(ctx_all - 1, 0) : ctx_all;  // tokens read from the cache
   const int gvalid = min(8, p.g - grp * 8);   // q heads handled by this CTA
@@ -401,7 +403,7 @@ paged_decode_kernel(const DecodeParams p) {
     if (p.num_splits == 1) {
       p.out[b * p.out_stride + static_cast<int64_t>(qh) * D + d] =
           __float2bfloat16_rn(L > 0.f ? o / L : 0.f);
-    } else if (p.cluster) {
+    } else if (FUSE && p.cluster) {
       float* part = reinterpret_cast<float*>(smem + C::kMergeBytes);   // [8][D] and [8][2] behind the merge buffer
       part[idx] = o;
       if (d == 0) { part[8 * D + 2 * hn] = M; part[8 * D + 2 * hn + 1] = L; }
@@ -414,27 +416,29 @@ paged_decode_kernel(const DecodeParams p) {
       }
     }
   }
-  if (!p.cluster) return;
-  // the cluster's CTAs share the item's outputs; the splits are summed in rank order (as paged_decode_reduce_kernel does)
-  static_assert(C::kMergeBytes + (8 * D + 16) * 4 <= C::kSmemBytes, "the partial state fits behind the merge buffer");
-  cluster_sync();
-  const uint32_t mine = smem_u32(smem) + C::kMergeBytes;
-  for (int idx = split * NWARPS * 32 + threadIdx.x; idx < gvalid * D; idx += p.num_splits * NWARPS * 32) {
-    const int hn = idx / D;
-    float M = -INFINITY;
-    for (int s = 0; s < p.num_splits; ++s) M = fmaxf(M, ld_peer_f32(mine + (8 * D + 2 * hn) * 4, s));
-    float o = 0.f, L = 0.f;
-    if (M != -INFINITY)
-      for (int s = 0; s < p.num_splits; ++s) {
-        const float ms = ld_peer_f32(mine + (8 * D + 2 * hn) * 4, s);
-        if (ms == -INFINITY) continue;
-        const float f = fast_exp2(ms - M);
-        o += ld_peer_f32(mine + idx * 4, s) * f;
-        L += ld_peer_f32(mine + (8 * D + 2 * hn + 1) * 4, s) * f;
-      }
-    p.out[b * p.out_stride + static_cast<int64_t>(qh0) * D + idx] = __float2bfloat16_rn(L > 0.f ? o / L : 0.f);
+  if constexpr (FUSE) {
+    if (!p.cluster) return;
+    // the cluster's CTAs share the item's outputs; the splits are summed in rank order (as paged_decode_reduce_kernel does)
+    static_assert(C::kMergeBytes + (8 * D + 16) * 4 <= C::kSmemBytes, "the partial state fits behind the merge buffer");
+    cluster_sync();
+    const uint32_t mine = smem_u32(smem) + C::kMergeBytes;
+    for (int idx = split * NWARPS * 32 + threadIdx.x; idx < gvalid * D; idx += p.num_splits * NWARPS * 32) {
+      const int hn = idx / D;
+      float M = -INFINITY;
+      for (int s = 0; s < p.num_splits; ++s) M = fmaxf(M, ld_peer_f32(mine + (8 * D + 2 * hn) * 4, s));
+      float o = 0.f, L = 0.f;
+      if (M != -INFINITY)
+        for (int s = 0; s < p.num_splits; ++s) {
+          const float ms = ld_peer_f32(mine + (8 * D + 2 * hn) * 4, s);
+          if (ms == -INFINITY) continue;
+          const float f = fast_exp2(ms - M);
+          o += ld_peer_f32(mine + idx * 4, s) * f;
+          L += ld_peer_f32(mine + (8 * D + 2 * hn + 1) * 4, s) * f;
+        }
+      p.out[b * p.out_stride + static_cast<int64_t>(qh0) * D + idx] = __float2bfloat16_rn(L > 0.f ? o / L : 0.f);
+    }
+    cluster_sync();   // nobody leaves while a peer still reads its partial state
   }
-  cluster_sync();   // nobody leaves while a peer still reads its partial state
 }
 
 // ------------------------------------------------------------------------------------------------------------------
@@ -710,6 +714,39 @@ namespace nvllm {
 
 constexpr int kMaxClusterSplits = 16;
 
+// Whether clusters of `splits` CTAs merge inside the kernel: steps of few tokens (FUSE; in a chain of other kernels the second launch is
+// hidden), few splits, and clusters that all run at once.  A GPC holds whole clusters only, so that the grid may not fit although its
+// CTAs do: 4 x 4000 tokens x 8 KV heads in 9 splits took 20.4 us as clusters (two waves), 11.8 with partials in memory and a second
+// kernel.
+static bool splits_merge_inside(int splits, long items) {
+  if (splits < 2 || splits > kMaxClusterSplits) return false;
+  using C = DecodeCfg<128, 3, 4>;
+  static std::once_flag once;
+  static int room[kMaxClusterSplits + 1];
+  std::call_once(once, [] {
+    auto kern = paged_decode_kernel<128, 3, 4, true>;
+    constexpr int kBytes = C::kSmemBytes + 2 * C::kSubTileBytes;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes) != cudaSuccess ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return;
+    }
+    for (int s = 2; s <= kMaxClusterSplits; ++s) {
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3(s);
+      cfg.blockDim = dim3(128);
+      cfg.dynamicSmemBytes = kBytes;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = s; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&room[s], kern, &cfg) != cudaSuccess) { (void)cudaGetLastError(); room[s] = 0; }
+    }
+  });
+  return items <= room[splits];
+}
+
 template <int D, int STAGES, int NWARPS, bool FUSE = false>
 static int launch_decode(const DecodeParams& p, cudaStream_t stream) {
   using C = DecodeCfg<D, STAGES, NWARPS>;
@@ -717,17 +754,16 @@ static int launch_decode(const DecodeParams& p, cudaStream_t stream) {
   constexpr int kBytes = C::kSmemBytes + (FUSE ? 2 * C::kSubTileBytes : 0);  // + the step's own K/V sub-tile
   NVLLM_SMEM_ATTR_ONCE(kern, kBytes);
   dim3 grid(p.num_splits, p.Hkv * p.ngrp, p.batch);
-  // Few splits: a cluster per item, one launch instead of two (a launch in a chain of dependent kernels costs 4-6 us: a step of one
-  // token over 28 layers 1002 -> 954 us together with the norm, rotation and store inside this kernel).
-  if (p.num_splits > 1 && p.num_splits <= kMaxClusterSplits) {
-    static std::once_flag once;
-    static cudaError_t once_err = cudaSuccess;
-    std::call_once(once, [&] { once_err = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1); });
-    NVLLM_CUDA(once_err);
-    DecodeParams q = p;
-    q.cluster = 1;
-    NVLLM_CUDA(launch_pdl_cluster(kern, grid, dim3(NWARPS * 32), static_cast<unsigned>(p.num_splits), kBytes, stream, q));
-    return 0;
+  // A cluster per item, one launch instead of two (a step of one token over 28 layers 1002 -> 954 us together with the norm, rotation and
+  // store inside this kernel).
+  if constexpr (FUSE) {
+    static_assert(D == 128 && STAGES == 3 && NWARPS == 4, "splits_merge_inside asks about this form");
+    if (splits_merge_inside(p.num_splits, static_cast<long>(p.Hkv) * p.ngrp * p.batch)) {
+      DecodeParams q = p;
+      q.cluster = 1;
+      NVLLM_CUDA(launch_pdl_cluster(kern, grid, dim3(NWARPS * 32), static_cast<unsigned>(p.num_splits), kBytes, stream, q));
+      return 0;
+    }
   }
   NVLLM_CUDA(launch_pdl(kern, grid, dim3(NWARPS * 32), kBytes, stream, p));
   if (p.num_splits > 1)
@@ -752,6 +788,10 @@ static int launch_decode_persist(const DecodeParams& p, cudaStream_t stream) {
   const long slots = static_cast<long>(per_sm) * sm_count();
   NVLLM_CUDA(launch_pdl(kern, dim3(static_cast<unsigned>(items < slots ? items : slots)), dim3(NWARPS * 32), kBytes, stream, p));
   return 0;
+}
+
+int paged_decode_launches(int batch, int heads, int kv_heads, int splits, bool fused) {
+  return splits > 1 && !(fused && splits_merge_inside(splits, static_cast<long>(batch) * kv_heads * ((heads / kv_heads + 7) / 8))) ? 2 : 1;
 }
 
 // Tuning knob for benchmarking only (bench.py --decode-cfg): 0 = default.
@@ -870,7 +910,6 @@ static int decode_dispatch(void* out, const void* q, void* k_cache, void* v_cach
   p.max_blocks = max_blocks_per_seq;
   p.block_size = layout->block_size;
   p.num_splits = num_splits;
-  p.cluster = 0;
   p.q_stride = q_token_stride;
   p.out_stride = out_token_stride;
   p.blk_stride = layout->block_stride;

@@ -79,7 +79,7 @@ def test_paged_decode_attention_vs_oracle(cuda, kind, case):
 
 @pytest.mark.parametrize("D", [64, 128])
 def test_paged_decode_splits_merge_alike(cuda, D):
-    """Every cluster size (2 to 16 splits merge inside the kernel) and the separate merge beyond it, with empty splits and an empty row."""
+    """2 to 18 splits, with empty splits and an empty row (the fused kernel's merge inside clusters has a test of its own)."""
     from nano_vllm_rs_b200 import ops
     ctx, H, Hkv, bs = [1, 777, 0, 64], 8, 4, 32
     rng = np.random.default_rng(D)
@@ -191,6 +191,34 @@ def test_paged_decode_attention_fused_vs_oracle(cuda, kind, case):
             mask[slots[b] // bs, slots[b] % bs] = True
     assert np.array_equal(kc_got[~mask], kc[~mask]), "only the new tokens' slots may change"
     assert_close(kc_got[mask], kc_ref[mask], 2e-3, 2 ** -6, "stored K rows (norm + RoPE)")
+
+
+def test_paged_decode_fused_splits_merge_alike(cuda):
+    """Every cluster size of the fused kernel (2 to 16 splits merge inside it), batches whose clusters do not all fit (partials in memory and
+    a second kernel), and more splits than a cluster takes: the step without a split, with empty splits and an empty row."""
+    from nano_vllm_rs_b200 import ops
+    D, H, Hkv, bs = 128, 16, 8, 32
+    for B, splits in [(4, range(2, 19)), (16, (2, 3, 9, 16))]:
+        ctx = ([1, 777, 0, 64] * B)[:B]
+        rng = np.random.default_rng(B)
+        kc, vc, tables, _, _ = make_paged_kv(rng, [c + 1 for c in ctx], bs, Hkv, D)
+        qkv = to_dev_bf16(randn_bf16(rng, (B, (H + 2 * Hkv) * D)), cuda)
+        pos = np.asarray([max(c - 1, 0) for c in ctx], np.int64)
+        slots = np.asarray([(tables[b, pos[b] // bs] * bs + pos[b] % bs) if ctx[b] else -1 for b in range(B)], np.int32)
+        w = to_dev_bf16(round_bf16(1.0 + 0.1 * rng.standard_normal(D).astype(np.float32)), cuda)
+        args = (torch.from_numpy(pos).to(cuda), torch.from_numpy(O.rope_cos_sin_table(2048, D, 1e6)).to(cuda), w, w, 1e-6)
+        rest = (torch.from_numpy(slots).to(cuda), torch.from_numpy(tables).to(cuda), torch.tensor(ctx, dtype=torch.int32, device=cuda), H,
+                _layout("head_major", bs, Hkv, D))
+
+        def step(n):
+            kd, vd = cache_to_layout(kc, "head_major", cuda), cache_to_layout(vc, "head_major", cuda)
+            return to_np_f32(ops.paged_decode_attention_fused(qkv, *args, kd, vd, *rest, num_splits=n)), kd, vd
+
+        want, k1, v1 = step(1)
+        for n in splits:
+            got, k2, v2 = step(n)
+            assert_close(got, want, ATT_ATOL, ATT_RTOL, f"{B} rows, {n} splits")
+            assert torch.equal(k1, k2) and torch.equal(v1, v2)
 
 
 def test_paged_decode_full_size_properties(cuda):
