@@ -53,7 +53,7 @@ int paged_decode_launches(int batch, int heads, int kv_heads, int splits, bool f
 
 // Projections of up to 16 tokens (gemm_skinny.cu): y = x . w^T as nvllm_gemm_bf16 / nvllm_gemm_silu_mul_bf16; norm_w: x is normed
 // first (bf16 weights, k columns); residual: y += the bf16 product, in place.
-bool gemm_skinny_applies(int m, int n, int k, int64_t ldx, int64_t ldw);
+bool gemm_skinny_applies(int m, int n, int k, int64_t ldx, int64_t ldw, bool f32_out, bool gate);
 int gemm_skinny(void* y, const void* x, const void* w, int m, int n, int k, int64_t ldx, int64_t ldw, int64_t ldy, int out_dtype, bool silu_gate,
                 const void* norm_w, float eps, bool residual, cudaStream_t st);
 
@@ -147,9 +147,6 @@ inline cudaError_t launch_plain(void (*kernel)(KArgs...), dim3 grid, dim3 block,
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                              Args&&... args) {
 // ... as clusters of grid.z CTAs along z
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_plain_cluster_z(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
@@ -166,6 +163,9 @@ inline cudaError_t launch_plain_cluster_z(void (*kernel)(KArgs...), dim3 grid, d
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                              Args&&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -210,9 +210,6 @@ __device__ __forceinline__ float ld_peer_f32(uint32_t addr, int rank) {
   asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(peer) : "memory");
   return v;
 }
-
-typedef __nv_bfloat16 bf16;
-typedef __nv_bfloat162 bf162;
 __device__ __forceinline__ float4 ld_peer_f32x4(uint32_t addr, int rank) {   // 16-byte aligned
   uint32_t peer;
   float4 v;
@@ -220,6 +217,9 @@ __device__ __forceinline__ float4 ld_peer_f32x4(uint32_t addr, int rank) {   // 
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(peer) : "memory");
   return v;
 }
+
+typedef __nv_bfloat16 bf16;
+typedef __nv_bfloat162 bf162;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));

@@ -303,21 +303,33 @@ int skinny_run(const SkinnyArgs& a, cudaStream_t st) {
 
 template <int NT>
 int skinny_rows(const SkinnyArgs& a, bool gate, int out_dtype, cudaStream_t st) {
-  // 8-row CTAs where 16-row ones would leave SMs without work; k-blocks ahead: all of a warp's up to K = 1024 (narrow outputs: 3072)
+  // 8-row CTAs while all of them run at once (two rounds of them lose to one of 16-row ones); k-blocks ahead: all of a warp's up to
+  // K = 1024 (narrow outputs: 3072)
   if (gate) return skinny_run<NT, 16, 4, true, bf16>(a, st);
-  // heads: CTAs that stay where each has two tiles or more and the rows of x fit three times into an SM's shared memory
-  if (out_dtype == NVLLM_F32 && a.n >= 2 * 16 * kHeadCtas * sm_count() && head_red_bytes<NT>() + a.m * (static_cast<int64_t>(a.k) + 32) * 2 <= kHeadSmem)
-    return skinny_head<NT>(a, st);
+  if constexpr (NT == 1)   // heads: CTAs that stay where each has two tiles or more (gemm_skinny_applies lets no more than 8 rows of 2560 come here)
+    if (out_dtype == NVLLM_F32 && a.n >= 2 * 16 * kHeadCtas * sm_count()) return skinny_head<NT>(a, st);
   if (out_dtype == NVLLM_F32) return skinny_run<NT, 16, 2, false, float>(a, st);   // heads: many CTAs, bound by bytes in flight: four on an SM
-  if ((a.n + 15) / 16 < sm_count()) return skinny_run<NT, 8, 12, false, bf16>(a, st);
+  if ((a.n + 7) / 8 <= sm_count()) return skinny_run<NT, 8, 12, false, bf16>(a, st);
   return skinny_run<NT, 16, 4, false, bf16>(a, st);
 }
 
 }  // namespace
 
-// Where these kernels take over: up to 16 tokens (beyond, the x fragments every CTA reads from L2 outweigh the weights), 16-byte rows.
-bool gemm_skinny_applies(int m, int n, int k, int64_t ldx, int64_t ldw) {
-  return knobs().gemm_skinny && m >= 1 && m <= 16 && k % 32 == 0 && ldx % 8 == 0 && ldw % 8 == 0 && n > 0;
+// Where these kernels take over: up to 16 rows of x, and matrices small enough that the fixed steps of the general kernels decide their
+// time.  A warp asks for x block by block behind the first ones, so long rows lose, and CTAs that end and start anew do not keep HBM busy
+// over a large matrix.  Measured beside the general path with weights from HBM (us, general -> here, 1 and 16 rows):
+//   bf16   4096 x 1024  7.2 -> 3.3, 4.1    1024 x 3072  6.5 -> 3.4, 5.2    4096 x 2048  9.2 -> 6.7, 7.7    | 8192 x 2048 0.95, 1.11 of it
+//          2560 x 4096 10.7 -> 12.0, 13.1  6144 x 4096 13.7 -> 22.8, 25.4  2048 x 8192 14.3 -> 35, 40
+//   gate   3072 x 1024 16.0 -> 5.0, 6.5    8192 x 2048 31.9 -> 25.5, 28.8  | 16384 x 2304 1.00, 1.10 of it  12288 x 4096 61 -> 76, 83
+//   f32    4096 x 2048  9.2 -> 6.8, 7.8    151936 x 2560 139 -> 119, 215   1024 x 3072 7.3 -> 8.2, 8.7
+bool gemm_skinny_applies(int m, int n, int k, int64_t ldx, int64_t ldw, bool f32_out, bool gate) {
+  if (!knobs().gemm_skinny || m < 1 || m > 16 || k % 32 != 0 || ldx % 8 != 0 || ldw % 8 != 0 || n < 1) return false;
+  if (gate) return k <= 2048;
+  if (f32_out)
+    return m <= 8 ? k <= (n <= 1024 ? 2048 : 2560) && (n <= 8192 || k >= 1024) : (n <= 4096 && k <= (n <= 1024 ? 1536 : 2048)) || (n <= 8192 && k <= 1024);
+  // (8-row CTAs up to 8 rows an SM; then 16-row ones, first too few of them to fill the SMs)
+  const int most = n <= 8 * sm_count() ? 3072 : (n <= 16 * sm_count() ? (m <= 8 ? 2048 : 1536) : (m <= 8 ? 3072 : 2304));
+  return (n <= 4096 && k <= most) || (n <= 8192 && k <= 1024);
 }
 
 int gemm_skinny(void* y, const void* x, const void* w, int m, int n, int k, int64_t ldx, int64_t ldw, int64_t ldy, int out_dtype, bool silu_gate,

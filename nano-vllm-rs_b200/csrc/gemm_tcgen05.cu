@@ -450,7 +450,7 @@ int gemm_bf16_impl(void* y, const void* x, const void* w, int32_t m, int32_t n, 
   if (m == 0) return 0;
   NVLLM_CHECK_ARG(y && x && w && aligned16(y) && aligned16(x) && aligned16(w), NVLLM_ERR_ALIGN, "gemm: pointers");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (!push && gemm_skinny_applies(m, n, k, ldx, ldw))
+  if (!push && gemm_skinny_applies(m, n, k, ldx, ldw, out_dtype == NVLLM_F32, false))
     return gemm_skinny(y, x, w, m, n, k, ldx, ldw, ldy, out_dtype, false, nullptr, 0.f, false, st);
   {  // decode-sized, long-K projections: split K over a cluster (gemm_splitk.cu)
     int sbn = 0, ssk = 0;
@@ -573,7 +573,7 @@ extern "C" int nvllm_gemm_gated_bf16(void* out, const void* x, const void* w_gat
   (void)workspace; (void)workspace_bytes;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (inter % 128 == 0) {  // fused epilogue: the [m, 2*inter] tensor never exists
-    if (gate == NVLLM_GATE_SILU && gemm_skinny_applies(m, inter, k, ldx, ldw))
+    if (gate == NVLLM_GATE_SILU && gemm_skinny_applies(m, inter, k, ldx, ldw, false, true))
       return gemm_skinny(out, x, w_gate_up, m, inter, k, ldx, ldw, ldout, NVLLM_BF16, true, nullptr, 0.f, false, st);
     const int bn = pick_bn(m, 2 * inter) < 64 ? 64 : pick_bn(m, 2 * inter);
     {

@@ -172,13 +172,14 @@ struct nvllm_runner {
   int init_weights(uint64_t seed, float std);
   int load_weight(const char* name, const void* h_bf16, int64_t rows, int64_t cols);
   int upload(const nvllm_batch& b, int padded);
-  // Up to 16 tokens: every norm rides in the projection behind it, every residual add in the one before it (gemm_skinny.cu), so h is
-  // the stream itself throughout.  The widths are those that the general path takes (it reports the others), and no more rows than
-  // tokens reach the head (a prefill batch may hold sequences without tokens).
+  // Up to 16 tokens on matrices that gemm_skinny.cu takes over: every norm rides in the projection behind it, every residual add in the one
+  // before it, so h is the stream itself throughout.  The widths are those that the general path takes (it reports the others), and no
+  // more rows than tokens reach the head (a prefill batch may hold sequences without tokens).
   bool few_tokens(int N, int S) const {
     const int HD = H * D;
-    return tp == 1 && gemm_skinny_applies(N, hidden, hidden, hidden, hidden) && hidden % 64 == 0 && inter % 64 == 0 && HD % 64 == 0 &&
-           vshard % 8 == 0 && S <= N;
+    return tp == 1 && hidden % 64 == 0 && inter % 64 == 0 && HD % 64 == 0 && vshard % 8 == 0 && S <= N &&
+           gemm_skinny_applies(N, qkv_dim, hidden, hidden, hidden, false, false) && gemm_skinny_applies(N, hidden, HD, HD, HD, false, false) &&
+           gemm_skinny_applies(N, inter, hidden, hidden, hidden, false, true) && gemm_skinny_applies(N, hidden, inter, inter, inter, false, false);
   }
   // where the q/k norm, the rotation and the store of a step's keys happen: in the qkv projection, or (decode) in the attention
   // (few tokens: a launch costs more than the attention's longer prologue)
@@ -760,9 +761,13 @@ int nvllm_runner::forward(int N, int S, bool is_prefill, bool paged_prefill, con
     head_in = last_hidden;
     rows = S;
   }
-  if (few) {
+  if (few && gemm_skinny_applies(rows, vshard, hidden, hidden, hidden, true, false)) {
     RUN(few_gemm(logits, head_in, lm_head, rows, vshard, hidden, vshard, NVLLM_F32, false, final_norm, false, "norm + lm_head"));
   } else {
+    if (few) {
+      RUN(nvllm_add_rmsnorm(normed, head_in, nullptr, final_norm, rows, hidden, eps, NVLLM_BF16, st)); ++launches; mark("add_rmsnorm");
+      head_in = normed;
+    }
     ++launches;
     RUN(nvllm_gemm_bf16(logits, head_in, lm_head, rows, vshard, hidden, hidden, hidden, vshard, NVLLM_F32, nullptr, 0, st));
     mark("lm_head GEMM");

@@ -270,14 +270,16 @@ def test_gpu_engine_vs_hf_transformers_golden(cuda, which, arch, fixture):
     print("max |GPU - HF| =", worst, "sigma")
 
 
-@pytest.mark.parametrize("arch,seqs", [("qwen3-0.6b", 3), ("qwen3-0.6b", 9), ("qwen3-0.6b", 16), ("qwen3-8b", 9), ("qwen3-8b", 16)])
-def test_fused_projections_of_few_tokens(cuda, arch, seqs, monkeypatch):
-    """Steps of up to 16 tokens norm inside the projections and add the residual in them (one and two groups of 8 tokens, hidden sizes
-    whose blocks of x stay in registers or do not, a head of CTAs that stay): the logits of the general path, up to the roundings that
-    another order of the sums flips."""
+@pytest.mark.parametrize("W,H,ff,tied,seqs,fused", [
+    (1024, 16, 3072, True, 3, True), (1024, 16, 3072, True, 9, True), (1024, 16, 3072, True, 16, True),
+    (2048, 16, 2048, False, 8, True), (1536, 8, 1536, False, 16, True),       # blocks of x that do not stay in registers
+    (4096, 32, 12288, False, 1, False), (4096, 32, 12288, False, 16, False),   # matrices that the general kernels read faster
+])
+def test_fused_projections_of_few_tokens(cuda, W, H, ff, tied, seqs, fused, monkeypatch):
+    """Steps of up to 16 tokens norm inside the projections and add the residual in them (one and two groups of 8 tokens; up to 8 rows the
+    head's CTAs stay): the logits of the general path, up to the roundings that another order of the sums flips."""
     import torch
     from nano_vllm_rs_b200 import engine as E
-    W, H, ff, tied = {"qwen3-0.6b": (1024, 16, 3072, True), "qwen3-8b": (4096, 32, 12288, False)}[arch]
     layers, vocab, kv = 2, 15000, 8
     rng = np.random.default_rng(seqs + W)
     prompts = [rng.integers(0, vocab, 1).tolist() for _ in range(seqs)]
@@ -300,7 +302,8 @@ def test_fused_projections_of_few_tokens(cuda, arch, seqs, monkeypatch):
     got = {}
     for skinny in ("0", "1"):
         monkeypatch.setenv("NVLLM_GEMM_SKINNY", skinny)
-        cfg = E.Config(arch, vocab_size=vocab, num_hidden_layers=layers, max_num_seqs=seqs, max_model_len=64, kvcache_block_size=16,
+        cfg = E.Config("qwen3-0.6b", hidden_size=W, num_attention_heads=H, intermediate_size=ff, tie_word_embeddings=int(tied), vocab_size=vocab,
+                       num_hidden_layers=layers, max_num_seqs=seqs, max_model_len=64, kvcache_block_size=16,
                        num_kvcache_blocks=2 * seqs, enforce_eager=1).validate()
         sched, runner = E.Scheduler(cfg), E.ModelRunner(cfg)
         for name, w in weights.items():
@@ -313,8 +316,10 @@ def test_fused_projections_of_few_tokens(cuda, arch, seqs, monkeypatch):
             b = sched.schedule()
             out.append(runner.execute_model(b, return_logits=True)[1])
             sched.postprocess([int(t) for t in forced[step]])
-        assert ("norm + qkv_proj" in runner.profile_report()) == (skinny == "1")
+        assert ("norm + qkv_proj" in runner.profile_report()) == (fused and skinny == "1")
         got[skinny] = np.stack(out)
+    if not fused:
+        assert np.array_equal(got["0"], got["1"])
     sig = got["0"].std(-1, keepdims=True)
     err = np.abs(got["1"] - got["0"])
     tol = LOGIT_SIGMA_PER_SQRT_LAYER * np.sqrt(layers) * sig + LOGIT_RTOL * np.abs(got["0"])

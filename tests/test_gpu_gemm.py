@@ -239,10 +239,12 @@ def test_gemm_narrow_tiles_without_split_k(cuda, m, n, k, monkeypatch):
 
 
 @pytest.mark.parametrize("m", [1, 7, 8, 9, 16])
-@pytest.mark.parametrize("n,k", [(8, 64), (1000, 192), (1024, 3072), (4104, 1024), (3072, 4096), (14208, 96 * 2), (14216, 1024), (31000, 1088), (14224, 4096)])
+@pytest.mark.parametrize("n,k", [(8, 64), (1000, 192), (1024, 3072), (4104, 1024), (3072, 4096), (14208, 96 * 2), (14216, 1024), (31000, 1088), (14224, 4096),
+                                 (1184, 3072), (1192, 3072), (4096, 2304), (4096, 2048), (8192, 1024), (8200, 1024), (16000, 2560), (512, 2560)])
 def test_products_of_a_few_rows(cuda, m, n, k):
     """m <= 16: weight rows on the M side of mma.sync, K split over the warps of a CTA (8- and 16-row CTAs, remainders of both; from
-    14208 rows f32 results by CTAs that take several tiles, and rows of x that are too long for those)."""
+    14208 rows f32 results by CTAs that take several tiles), and sizes on both sides of the rule that keeps large matrices on the
+    general kernels."""
     from nano_vllm_rs_b200 import ops
     g = torch.Generator(device=cuda).manual_seed(m * n + k)
     wide = torch.randn((m, k + 24), generator=g, device=cuda).to(torch.bfloat16)
@@ -256,4 +258,10 @@ def test_products_of_a_few_rows(cuda, m, n, k):
     assert ((got.double() - want[:, :n]).abs() <= bound[:, :n] + 2.0 ** -8 * want[:, :n].abs()).all()
     if n % 128 == 0:
         fused = ops.gemm_silu_mul(x, w)
-        assert torch.equal(fused, ops.silu_mul(ops.gemm_bf16(x, w)))
+        if k <= 2048 and n <= 4096:   # both products run here; otherwise one is on the general kernels, which sum in another order
+            assert torch.equal(fused, ops.silu_mul(torch.cat([ops.gemm_bf16(x, w[:n]), ops.gemm_bf16(x, w[n:])], 1)))
+        # gate and up rounded to bf16 (8 significant bits: 2^-8 each; |silu'| < 1.1), silu and the product rounded once more
+        g, u = want[:, :n], want[:, n:]
+        silu = g * torch.sigmoid(g)
+        eg, eu = 2.0 ** -8 * g.abs() + bound[:, :n], 2.0 ** -8 * u.abs() + bound[:, n:]
+        assert ((fused.double() - silu * u).abs() <= 1.1 * eg * (u.abs() + eu) + silu.abs() * eu + 2.0 ** -7 * (silu * u).abs() + 1e-6).all()
