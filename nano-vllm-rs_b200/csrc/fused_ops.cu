@@ -350,8 +350,9 @@ argmax_kernel(int64_t* __restrict__ out_ids, float* __restrict__ out_max, const 
               int vocab, int64_t ld, int64_t vocab_offset) {
   pdl_launch_dependents();
   pdl_wait();
-  const int part = static_cast<int>(blockIdx.x) % SPLIT, tid = part * blockDim.x + threadIdx.x, stride = SPLIT * blockDim.x;
-  const int64_t b = blockIdx.x / SPLIT;
+  const int part = SPLIT > 1 ? static_cast<int>(blockIdx.x) % SPLIT : 0, tid = SPLIT > 1 ? part * blockDim.x + threadIdx.x : threadIdx.x;
+  const unsigned stride = SPLIT * blockDim.x;
+  const unsigned b = blockIdx.x / SPLIT;
   const T* row = logits + b * ld;
   float best = -INFINITY;
   int bidx = 0x7fffffff;
@@ -402,24 +403,32 @@ argmax_kernel(int64_t* __restrict__ out_ids, float* __restrict__ out_max, const 
       const int oi = __shfl_xor_sync(0xffffffffu, bidx, o);
       if (ov > best || (ov == best && oi < bidx)) { best = ov; bidx = oi; }
     }
-    if (SPLIT > 1 && threadIdx.x == 0) { sv[0] = best; si[0] = bidx; }
+    if (threadIdx.x == 0) {
+      if constexpr (SPLIT > 1) {
+        sv[0] = best;
+        si[0] = bidx;
+      } else {
+        if (bidx == 0x7fffffff) bidx = 0;  // all -inf / NaN row
+        out_ids[blockIdx.x] = static_cast<int64_t>(bidx) + vocab_offset;
+        if (out_max) out_max[blockIdx.x] = best;
+      }
+    }
   }
-  if (SPLIT > 1) {
+  if constexpr (SPLIT > 1) {
     __syncwarp();
     cluster_sync();
-    if (part == 0 && threadIdx.x == 0)
+    if (part == 0 && threadIdx.x == 0) {
       for (int r = 1; r < SPLIT; ++r) {
         const float ov = ld_peer_f32(smem_u32(sv), r);
         const int oi = __float_as_int(ld_peer_f32(smem_u32(si), r));
         if (ov > best || (ov == best && oi < bidx)) { best = ov; bidx = oi; }
       }
+      if (bidx == 0x7fffffff) bidx = 0;
+      out_ids[b] = static_cast<int64_t>(bidx) + vocab_offset;
+      if (out_max) out_max[b] = best;
+    }
     __syncwarp();
     cluster_sync();   // nobody leaves before its result has been read
-  }
-  if (part == 0 && threadIdx.x == 0) {
-    if (bidx == 0x7fffffff) bidx = 0;  // all -inf / NaN row
-    out_ids[b] = static_cast<int64_t>(bidx) + vocab_offset;
-    if (out_max) out_max[b] = best;
   }
 }
 
@@ -520,7 +529,9 @@ extern "C" int nvllm_qknorm_rope_store(void* qkv, const int64_t* positions, cons
     s_head = layout->head_stride;
   }
   const int heads = num_heads + 2 * num_kv_heads;
-  const bool vec = aligned16(qkv) && aligned16(cos_sin) && aligned16(q_norm_w) && aligned16(k_norm_w) && aligned16(k_cache) && aligned16(v_cache) &&
+  // Few heads do not fill the SMs four to a lane group: a warp per head is done sooner (64 tokens x 32 heads of 128 3.5 us so, 2.6 with warps;
+  // 2000 tokens 8.8 and 14.5; the lines cross near 128 heads an SM).
+  const bool vec = static_cast<int64_t>(num_tokens) * heads >= 128ll * sm_count() && aligned16(qkv) && aligned16(cos_sin) && aligned16(q_norm_w) && aligned16(k_norm_w) && aligned16(k_cache) && aligned16(v_cache) &&
                    s_blk % 8 == 0 && s_tok % 8 == 0 && s_head % 8 == 0;
   const int64_t threads = vec ? static_cast<int64_t>(num_tokens) * ((heads + kRopeHeads - 1) / kRopeHeads) * (head_dim / 8)
                               : static_cast<int64_t>(num_tokens) * heads * 32;
@@ -602,8 +613,9 @@ extern "C" int nvllm_argmax(int64_t* out_ids, float* out_max, const void* logits
   const float* lf = static_cast<const float*>(logits);
   const bf16* lb = static_cast<const bf16*>(logits);
   constexpr int kSplit = 8;
-  // A cluster per row while all of them find an SM each and every thread has a vector to read; beyond that the rows alone fill the SMs.
-  if (batch * kSplit <= sm_count() && vocab >= kSplit * 1024 * 8) {
+  // A cluster per row while all of them find an SM each and every thread has a vector to read, or two where the clusters take more than half
+  // of the SMs (18 rows of 65536 f32: 6.5 us as clusters, 5.6 with a CTA each; 4 rows 3.3 and 5.5); beyond that the rows alone fill the SMs.
+  if (batch <= sm_count() / kSplit && vocab >= kSplit * 1024 * (batch * kSplit > sm_count() / 2 ? 16 : 8)) {
     if (logits_dtype == NVLLM_F32) NVLLM_CUDA(launch_pdl_cluster(argmax_kernel<float, kSplit>, dim3(batch * kSplit), dim3(1024), kSplit, 0, st, out_ids, out_max, lf, vocab, ld, vocab_offset));
     else NVLLM_CUDA(launch_pdl_cluster(argmax_kernel<bf16, kSplit>, dim3(batch * kSplit), dim3(1024), kSplit, 0, st, out_ids, out_max, lb, vocab, ld, vocab_offset));
   } else if (logits_dtype == NVLLM_F32) {

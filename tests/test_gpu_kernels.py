@@ -288,7 +288,8 @@ def test_rope_table_vs_oracle(cuda):
 
 
 @pytest.mark.parametrize("kind", ["reference", "head_major"])
-@pytest.mark.parametrize("n,H,Hkv,D,qknorm", [(64, 16, 8, 128, True), (7, 32, 8, 128, False), (33, 4, 2, 64, True), (1, 8, 1, 128, True)])
+@pytest.mark.parametrize("n,H,Hkv,D,qknorm", [(64, 16, 8, 128, True), (7, 32, 8, 128, False), (33, 4, 2, 64, True), (1, 8, 1, 128, True),
+                                                (620, 16, 8, 128, True), (1101, 14, 2, 128, False), (2401, 4, 2, 64, True)])   # lane groups of four heads
 def test_qknorm_rope_store_vs_oracle(cuda, kind, n, H, Hkv, D, qknorm):
     from nano_vllm_rs_b200 import ops
     rng = np.random.default_rng(n + H)
