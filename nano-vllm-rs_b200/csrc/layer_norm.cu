@@ -58,9 +58,9 @@ __global__ void __launch_bounds__(256) residual_layernorm_kernel(TO* __restrict_
   }
 }
 
-// The same for rows of up to 1024 NK values (NK 2, 4, 8) in 16-byte vectors: the row stays in registers and everything it is made of is
+// The same for rows of up to 1024 NK values (NK 2, 3, 4) in 16-byte vectors: the row stays in registers and everything it is made of is
 // requested before the first reduction (8192 rows of 2048, up to three f32 addends: 77 -> 47 us on average; 288 MB with two, 43 us
-// at the copy rate).
+// at the copy rate).  Longer rows keep the kernel above: their registers leave too few warps (8192 rows of 5120: 119 us there, 152 so).
 __device__ __forceinline__ float4 ld4_any(const Addend& a, int64_t i) {
   if (a.dt == NVLLM_F32) return *reinterpret_cast<const float4*>(static_cast<const float*>(a.p) + i);
   const uint2 u = *reinterpret_cast<const uint2*>(static_cast<const bf16*>(a.p) + i);
@@ -127,8 +127,8 @@ template <typename TO>
 int launch_layernorm_vec(TO* out, float* h, const Addend& a0, const Addend& a1, const Addend& a2, const float* bias, float sb, const float* w, int n,
                          int hidden, float eps, cudaStream_t st) {
   NVLLM_CUDA(launch_pdl(hidden <= 2048   ? residual_layernorm_vec_kernel<2, TO>
-                        : hidden <= 4096 ? residual_layernorm_vec_kernel<4, TO>
-                                         : residual_layernorm_vec_kernel<8, TO>,
+                        : hidden <= 3072 ? residual_layernorm_vec_kernel<3, TO>
+                                         : residual_layernorm_vec_kernel<4, TO>,
                         dim3(n), dim3(256), 0, st, out, h, a0, a1, a2, bias, sb, w, hidden, eps));
   NVLLM_LAUNCH_CHECK("residual_layernorm_vec_kernel");
   return 0;
@@ -189,15 +189,16 @@ extern "C" int nvllm_residual_layernorm(void* out, float* h, const void* a0, flo
   const size_t smem = static_cast<size_t>(hidden) * sizeof(float);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const Addend A0{a0, s0, dt0}, A1{a1, s1, dt1}, A2{a2, s2, dt2};
-  if (hidden % 4 == 0 && hidden <= 8192 && aligned16(h) && aligned16(out) && aligned16(a0) && aligned16(a1) && aligned16(a2) && aligned16(bias) && aligned16(w))
+  if (hidden % 4 == 0 && hidden <= 4096 && aligned16(h) && aligned16(out) && aligned16(a0) && aligned16(a1) && aligned16(a2) && aligned16(bias) && aligned16(w))
     return out_dtype == NVLLM_BF16 ? launch_layernorm_vec(static_cast<bf16*>(out), h, A0, A1, A2, bias, bias_scale, w, n, hidden, eps, st)
                                    : launch_layernorm_vec(static_cast<float*>(out), h, A0, A1, A2, bias, bias_scale, w, n, hidden, eps, st);
+  // (plainly: 16 to 256 rows of 5120 with addends took 11.7-12.2 us launched early, 10.3-10.7 so)
   if (out_dtype == NVLLM_BF16) {
     if (smem > 48 * 1024) NVLLM_CUDA(cudaFuncSetAttribute(residual_layernorm_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 192 * 1024));
-    NVLLM_CUDA(launch_pdl(residual_layernorm_kernel<bf16>, dim3(n), dim3(256), smem, st, static_cast<bf16*>(out), h, A0, A1, A2, bias, bias_scale, w, hidden, eps));
+    NVLLM_CUDA(launch_plain(residual_layernorm_kernel<bf16>, dim3(n), dim3(256), smem, st, static_cast<bf16*>(out), h, A0, A1, A2, bias, bias_scale, w, hidden, eps));
   } else {
     if (smem > 48 * 1024) NVLLM_CUDA(cudaFuncSetAttribute(residual_layernorm_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 192 * 1024));
-    NVLLM_CUDA(launch_pdl(residual_layernorm_kernel<float>, dim3(n), dim3(256), smem, st, static_cast<float*>(out), h, A0, A1, A2, bias, bias_scale, w, hidden, eps));
+    NVLLM_CUDA(launch_plain(residual_layernorm_kernel<float>, dim3(n), dim3(256), smem, st, static_cast<float*>(out), h, A0, A1, A2, bias, bias_scale, w, hidden, eps));
   }
   NVLLM_LAUNCH_CHECK("residual_layernorm_kernel");
   return 0;

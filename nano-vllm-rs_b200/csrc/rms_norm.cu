@@ -82,8 +82,9 @@ __global__ void __launch_bounds__(256) rms_residual_norm_kernel(TO* __restrict__
 }
 
 // The same for rows of up to 1024 NK values (NK 2, 4, 8) in 16-byte vectors: the row stays in registers (one global pass), y and out in f32
-// or bf16.  y and h are both requested before the first reduction: read after it, h was a second round trip to HBM in every CTA
-// (8192 rows of 2048: 52 -> 36 us; 192 MB, 29 us at the copy rate).
+// or bf16.  Up to 4096 values y and h are both requested before the first reduction: read after it, h was a second round trip to HBM in
+// every CTA (8192 rows of 2048: 52 -> 36 us; 192 MB, 29 us at the copy rate).  Longer rows have enough in flight, and the registers
+// of a second row cost more than the round trip (8192 rows of 5120, f32: 140 us with h ahead, 109 without).
 template <int NK, typename TY, typename TO>
 __global__ void __launch_bounds__(256) rms_residual_norm_vec_kernel(TO* __restrict__ out, float* __restrict__ h, const TY* __restrict__ y,
                                                                     const float* __restrict__ post_w, const float* __restrict__ pre_w, int hidden,
@@ -93,13 +94,17 @@ __global__ void __launch_bounds__(256) rms_residual_norm_vec_kernel(TO* __restri
   __shared__ float red[8];
   const int nv = hidden / 4;
   const int64_t base = static_cast<int64_t>(blockIdx.x) * hidden;
-  float4 v[NK], hv[NK];
+  constexpr bool AHEAD = NK <= 4;
+  float4 v[NK], hv[AHEAD ? NK : 1];
   float sq = 0.f;
+  if constexpr (AHEAD) {
 #pragma unroll
-  for (int k = 0; k < NK; ++k) {
-    const int c = threadIdx.x + 256 * k;
-    if (c < nv) hv[k] = reinterpret_cast<const float4*>(h + base)[c];
+    for (int k = 0; k < NK; ++k) {
+      const int c = threadIdx.x + 256 * k;
+      if (c < nv) hv[k] = reinterpret_cast<const float4*>(h + base)[c];
+    }
   }
+  auto stream_at = [&](int k, int c) { if constexpr (AHEAD) return hv[k]; else return reinterpret_cast<const float4*>(h + base)[c]; };
   if (y != nullptr) {
 #pragma unroll
     for (int k = 0; k < NK; ++k) {
@@ -120,8 +125,8 @@ __global__ void __launch_bounds__(256) rms_residual_norm_vec_kernel(TO* __restri
     for (int k = 0; k < NK; ++k) {
       const int c = threadIdx.x + 256 * k;
       if (c < nv) {
-        const float4 w = reinterpret_cast<const float4*>(post_w)[c];
-        v[k] = make_float4(hv[k].x + v[k].x * r * w.x, hv[k].y + v[k].y * r * w.y, hv[k].z + v[k].z * r * w.z, hv[k].w + v[k].w * r * w.w);
+        const float4 x = stream_at(k, c), w = reinterpret_cast<const float4*>(post_w)[c];
+        v[k] = make_float4(x.x + v[k].x * r * w.x, x.y + v[k].y * r * w.y, x.z + v[k].z * r * w.z, x.w + v[k].w * r * w.w);
         reinterpret_cast<float4*>(h + base)[c] = v[k];
         sq += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
       }
@@ -131,7 +136,7 @@ __global__ void __launch_bounds__(256) rms_residual_norm_vec_kernel(TO* __restri
     for (int k = 0; k < NK; ++k) {
       const int c = threadIdx.x + 256 * k;
       if (c < nv) {
-        v[k] = hv[k];
+        v[k] = stream_at(k, c);
         sq += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
       }
     }

@@ -48,7 +48,7 @@ def rel_err(got, ref):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("hid", [50, 256, 1])
+@pytest.mark.parametrize("hid", [50, 256, 1, 1500, 2048, 2052, 3072, 4096, 4100])   # rows in registers up to 4096
 def test_residual_layernorm(cuda, dtype, hid):
     from nano_vllm_rs_b200 import ops
     rng = np.random.default_rng(hid)
@@ -235,6 +235,31 @@ def test_causal_conv_carries_its_last_inputs(cuda, taps):
             got[s].append(out[o:o + n]); o += n; at[s] += n
     for s in (0, 1):
         np.testing.assert_allclose(np.vstack(got[s]), ref[s], rtol=2e-5, atol=2e-5)
+
+
+@pytest.mark.parametrize("taps", [2, 3, 4])
+@pytest.mark.parametrize("ch", [12, 260])
+def test_causal_conv_long_portions(cuda, taps, ch):
+    """Portions of 16 and more tokens (four channels a thread, eight tokens a step, runs of 32 that cross from one sequence to the next):
+    equal to the convolution of the whole sequence."""
+    from nano_vllm_rs_b200 import ops
+    rng = np.random.default_rng(taps + ch)
+    lens, cuts = [107, 83], [[40, 17, 50], [33, 47, 3]]
+    x = [rng.standard_normal((n, ch + 4)) for n in lens]
+    w, b = rng.standard_normal((ch, taps)), rng.standard_normal(ch)
+    state = torch.full((4, taps - 1, ch), 9.0, device=cuda)
+    at, got = [0, 0], [[], []]
+    for k in range(3):
+        ls = [cuts[s][k] for s in (0, 1)]
+        xin = dev_t(np.vstack([x[s][at[s]:at[s] + n] for s, n in enumerate(ls)]), cuda)
+        out = ops.causal_conv(xin[:, :ch], dev_t(w, cuda), dev_t(b, cuda), state, *_steps_meta(ls, at, [3, 1], cuda)).cpu().numpy()
+        for s, n in enumerate(ls):
+            got[s].append(out[sum(ls[:s]):sum(ls[:s]) + n])
+            at[s] += n
+    for s in (0, 1):
+        pad = np.vstack([np.zeros((taps - 1, ch)), x[s][:, :ch]])
+        ref = T.silu(np.stack([(pad[t:t + taps] * w.T).sum(0) + b for t in range(lens[s])]))
+        np.testing.assert_allclose(np.vstack(got[s]), ref, rtol=2e-5, atol=2e-5)
 
 
 @pytest.mark.parametrize("heads,groups,dk,dv", [(4, 2, 5, 4), (3, 3, 16, 7), (2, 1, 48, 40), (1, 1, 130, 33), (2, 2, 64, 64), (1, 1, 300, 6)])

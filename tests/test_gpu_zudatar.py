@@ -52,7 +52,7 @@ f32r = lambda x: np.asarray(x, np.float32).astype(np.float64)
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("hid", [50, 256, 1, 3000])
+@pytest.mark.parametrize("hid", [50, 256, 1, 3000, 2048, 4096, 4100, 8192])   # the stream is asked for ahead up to 4096
 def test_rms_residual_norm(cuda, dtype, hid):
     from nano_vllm_rs_b200 import ops
     rng = np.random.default_rng(hid)
