@@ -6,14 +6,14 @@
 
 A "step" is one decode step of the whole model over one batch (embedding -> 28/36 layers of norm / qkv GEMM / qk-norm
 + RoPE + KV store / split-K paged decode attention / o_proj / MLP -> LM head -> greedy argmax).
-  N == 1 : BASELINE.json configs[1] — Qwen3-0.6B bf16, 256 concurrent seqs, paged KV block 256, 512-token prompts +
+  N == 1 : Qwen3-0.6B bf16, 256 concurrent seqs, paged KV block 256, 512-token prompts +
            512 decode steps.  The K timed steps are centred on the workload's mean context (768 tokens): the synthetic
            prompts are 768 - W - K/2 tokens long (the cost of a step depends on the context only through its length);
            with K >= 480 the prompts are exactly 512 tokens and the run IS the workload.
-  N  > 1 : BASELINE.json configs[2] — Qwen3-8B bf16 tensor-parallel TP=N, 512 seqs x (1K prompt + 1K decode), timed
+  N  > 1 : Qwen3-8B bf16 tensor-parallel TP=N, 512 seqs x (1K prompt + 1K decode), timed
            window centred on context 1536; "scaling": "strong" (same job on more GPUs; the 1-GPU point of the same job is
            `--gpus 1 --model qwen3-8b`, kept in profiles/ and quoted in every N > 1 line).
-  --workload prefix : BASELINE.json configs[3] — Qwen3-8B, 256 seqs sharing a 4096-token prefix (+ 256 unique tokens),
+  --workload prefix : Qwen3-8B, 256 seqs sharing a 4096-token prefix (+ 256 unique tokens),
            N = 1: prefix-cached varlen prefill (block dedup, paged-prefix attention) then decode at context 4353+.
 value  : decode tokens/s with the step's inputs already resident in HBM (CUDA events around K replays of the step).
 e2e    : the same metric through the public API (LLMEngine.step: schedule -> H2D metadata -> graph -> D2H tokens ->
@@ -26,7 +26,7 @@ parity : checked INSIDE the run, before the timed region, exit code 1 on failure
          oracle (vocab-sharded logits gathered on rank 0), and the sampled tokens of every warm-up step of the real
          workload compared across ranks.
 cpu_baseline / --impl reference: the CPU oracle (numpy port of the reference's algorithm; the reference itself cannot
-         be built — DESIGN.md) timed on the host cores on a bounded sample of the same workload."""
+         be built) timed on the host cores on a bounded sample of the same workload."""
 import argparse
 import json
 import os
@@ -40,9 +40,9 @@ sys.path.insert(0, ROOT)
 
 MODELS = {"qwen3-0.6b": dict(seqs=256, prompt=512, decode=512, blocks_per_seq=4),
           "qwen3-8b": dict(seqs=512, prompt=1024, decode=1024, blocks_per_seq=8),
-          # BASELINE.json configs[4]: Qwen3-32B TP=8, 64 seqs at 32K context (long-context split-K paged decode stress)
+          # Qwen3-32B TP=8, 64 seqs at 32K context (long-context split-K paged decode stress)
           "qwen3-32b": dict(seqs=64, prompt=32256, decode=512, blocks_per_seq=129)}
-# BASELINE.json configs[3]: 256 seqs = one shared 4096-token prefix (seed 4321) + 256 unique tokens each (SURVEY Appendix B)
+# 256 seqs = one shared 4096-token prefix (seed 4321) + 256 unique tokens each
 PREFIX = dict(model="qwen3-8b", seqs=256, shared=4096, unique=256)
 
 
@@ -207,7 +207,7 @@ def cpu_decode_sample(model, ctx, seqs, steps, warmup, budget_s=None, distinct=N
 
 def tensor_kernels(peak_tflops):
     """Secondary rooflines (north_star (c)): the tensor-core kernels of the workload's PREFILL step, timed live with CUDA
-    events on torch's stream at the shapes of configs[1] (64 sequences x 512 tokens per prefill step of Qwen3-0.6B).
+    events on torch's stream at the shapes of the decode workload (64 sequences x 512 tokens per prefill step of Qwen3-0.6B).
     Returns None on any failure — the headline line never depends on it."""
     try:
         import torch
@@ -269,8 +269,8 @@ def workload_name(model, wl):
 
 def reference_arm(args):
     """bench.py --impl reference: the reference's own CPU implementation of the path.  The Rust crate cannot be built
-    here (no toolchain, invalid manifest, type errors on the path — DESIGN.md), so this times the oracle port, on the SAME
-    workload string as our arm: the full decode batch of configs[1] (256 sequences) for 2 timed steps after 1 warm-up
+    here (no toolchain, invalid manifest, type errors on the path), so this times the oracle port, on the SAME
+    workload string as our arm: the full decode batch of that workload (256 sequences) for 2 timed steps after 1 warm-up
     (~10 s each); for the 8B / 32B workloads a bounded number of the batch's sequences (stated in `sample`)."""
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
@@ -451,7 +451,7 @@ def run_decode(args, model, wl, prompt, K, W, rank, world, local, want_parity, w
     progress(f"building the engine: {model}, tp={world}, {B} sequences, {nblk} KV blocks")
     eng = E.LLMEngine(cfg, comm=comm, seed=seed, std=std)
     progress("engine ready (weights initialised, KV cache allocated); prefilling")
-    rng = np.random.default_rng(1234)                      # SURVEY.md §8d: token stream seed 1234, ids mod vocab
+    rng = np.random.default_rng(1234)                      # token stream seed 1234, ids mod vocab
     sp = E.SamplingParams(temperature=0.0, max_tokens=W + 2 * K + 64, ignore_eos=True)
     sids = [eng.add_request(rng.integers(0, cfg.vocab_size, prompt), sp) for _ in range(B)]
 
@@ -596,18 +596,18 @@ def run_decode(args, model, wl, prompt, K, W, rank, world, local, want_parity, w
     return line
 
 
-# ------------------------------------------------------------------------------------------------ configs[3]: prefix caching
+# ------------------------------------------------------------------------------------------------ prefix caching
 def run_prefix(args, rank, world, local):
-    """BASELINE.json configs[3] on ONE GPU: Qwen3-8B, 256 sequences = one shared 4096-token prefix (seed 4321) + 256 unique
+    """Prefix caching on ONE GPU: Qwen3-8B, 256 sequences = one shared 4096-token prefix (seed 4321) + 256 unique
     tokens.  Prefill: sequence 0 computes all 4352 tokens, every other sequence hits the 16 shared blocks (ref_count 256)
     and computes only its 256-token suffix against the paged prefix (attention.rs:211-222, block_manager.rs:157-219);
-    then decode at context 4353+.  The block accounting of SURVEY.md Appendix B is asserted (272 blocks after prefill,
+    then decode at context 4353+.  The block accounting is asserted (272 blocks after prefill,
     + 256 at the first decode step)."""
     import numpy as np
     import torch
 
     from nano_vllm_rs_b200 import engine as E
-    assert world == 1, "--workload prefix is the single-GPU configs[3] run"
+    assert world == 1, "--workload prefix is a single-GPU run"
     model, B, shared, unique = PREFIX["model"], args.seqs or PREFIX["seqs"], PREFIX["shared"], PREFIX["unique"]
     K, W = args.steps, max(args.warmup, 3)
     L = shared + unique
@@ -684,13 +684,13 @@ def run_prefix(args, rank, world, local):
         "steps": K, "warmup": W, "ms_per_step": round(dev_ms / K, 4), "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "bf16", "data": "synthetic",
         "config": {"workload": f"{model} bf16 prefix caching: {B} seqs sharing a {shared}-token prefix + {unique} unique tokens "
-                               f"(BASELINE.json configs[3]), paged KV block 256; decode timed at context {ctx_first}..{ctx_last}",
+                               f"each, paged KV block 256; decode timed at context {ctx_first}..{ctx_last}",
                    "seqs": B, "parallelism": "tp1", "cuda_graphs": not args.eager,
                    "l2_note": f"inputs larger than L2: one decode step reads {round(att_bytes * layers / 1e9, 1)} GB of KV"},
         "prefill": prefill,
         "blocks": {"after_prefill": blocks_after_prefill, "after_first_decode_step": blocks_after_first_decode,
                    "expected": [expect_prefill_blocks, expect_prefill_blocks + B], "ok": ok_blocks,
-                   "what": "SURVEY.md Appendix B cfg4: 16 shared blocks at ref_count 256 + one private block per sequence, "
+                   "what": "16 shared blocks at ref_count 256 + one private block per sequence, "
                            "then one more per sequence at len 4353"},
         "e2e": {"value": round(B * K / e2e_s, 1), "unit": "tokens/s", "ms_per_step": round(e2e_s / K * 1e3, 4),
                 "h2d_bytes_per_step": B * (24 + 4 * cap), "d2h_bytes_per_step": 8 * B, "api": "LLMEngine.step"},

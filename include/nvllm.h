@@ -47,7 +47,7 @@ int nvllm_version(void);
 const char* nvllm_last_error(void);
 /* 1 when a CUDA device of compute capability 10.x is visible, else 0 (never throws). */
 int nvllm_device_ok(void);
-/* The NVLLM_* environment knobs (A/B measurement switches, DESIGN.md appendix) are parsed once per process, never on a
+/* The NVLLM_* environment knobs (A/B measurement switches) are parsed once per process, never on a
  * dispatch path; benchmark tools that sweep a knob inside one process call this after changing the environment.
  * NOT re-entrant, unlike every other entry point: it rewrites the knob set in place, so call it only while no other thread
  * is inside the library (a dispatch running concurrently could see half of the old set and half of the new). */
@@ -155,7 +155,7 @@ int nvllm_paged_decode_attention_fused(void* out, const void* qkv, const int64_t
  * keys 0 .. Lk-Lq+j), which is the plain causal mask when Lq == Lk.
  * If block_tables == NULL keys/values come from the dense k, v: [total_k, Hkv, D];
  * otherwise (prefix-cache prefill) they are read from the paged cache through block_tables[i,:]
- * (the new K/V of this step must already have been stored — note N2 in SURVEY.md §8).
+ * (the new K/V of this step must already have been stored).
  * total_q / total_k: rows of q / of the dense k, v (bounds of the TMA descriptors; total_k is ignored when paged).
  * Requires Lk >= Lq per sequence and head_dim == 128; runs on tcgen05 tensor cores. */
 int nvllm_varlen_prefill_attention(void* out, const void* q, const void* k, const void* v,
@@ -214,7 +214,7 @@ int nvllm_add_rmsnorm(void* out, const void* x, void* residual, const void* weig
 
 /* K7 (+K1 fused) — replaces RotaryEmbedding::forward / apply_rotary_emb_single
  * (src/layers/rotary_embedding.rs:23-48,136-158), the per-head q_norm/k_norm of the named Qwen3
- * architecture (absent in the reference, SURVEY.md §8 note N1) and, when k_cache != NULL, the
+ * architecture (absent in the reference) and, when k_cache != NULL, the
  * store_kv_cache call that follows (attention.rs:78-81).
  * In place on the packed qkv buffer [num_tokens, (H + 2*Hkv) * D] (q | k | v, linear.rs:331-340):
  *   q_h <- rope(rmsnorm_D(q_h) * q_norm_w),  k_h <- rope(rmsnorm_D(k_h) * k_norm_w)
@@ -228,7 +228,7 @@ int nvllm_qknorm_rope_store(void* qkv, const int64_t* positions, const float* co
                             const int32_t* slot_mapping, const nvllm_kv_layout* layout,
                             int32_t dtype, void* stream);
 /* Fills cos_sin [max_position, D] fp32 exactly as the oracle does (f64 inv_freq and angle, rounded
- * to f32) — rotary_embedding.rs:82-110 with the table kept in f32 (note N1). */
+ * to f32) — rotary_embedding.rs:82-110 with the table kept in f32. */
 int nvllm_rope_table(float* cos_sin, int32_t max_position, int32_t head_dim, double theta,
                      void* stream);
 

@@ -19,7 +19,7 @@ extern "C" {
 #endif
 
 /* Config (config.rs:16-71) + Qwen3Config (models/qwen3.rs:26-68) with the named-architecture fields the
- * reference lacks (head_dim, qk_norm — SURVEY.md §8 note N1). */
+ * reference lacks (head_dim, qk_norm). */
 typedef struct nvllm_config {
   /* Config */
   int32_t max_num_batched_tokens; /* 32768 */
@@ -203,7 +203,7 @@ int nvllm_runner_time_decode_attention(nvllm_runner* r, int32_t iters, float* ms
 int nvllm_runner_replay_decode(nvllm_runner* r, int32_t iters, float* ms_total);
 
 /* LLMEngine (llm_engine.rs:23-362): scheduler + runner; step() = schedule -> execute_model -> sample_tokens ->
- * postprocess (llm_engine.rs:155-197).  The async/streaming/tokeniser facade is out of scope (SURVEY.md §8f #4). */
+ * postprocess (llm_engine.rs:155-197).  The async/streaming/tokeniser facade is out of scope. */
 typedef struct nvllm_engine nvllm_engine;
 int nvllm_engine_create(nvllm_engine** e, const nvllm_config* cfg, nvllm_comm* comm);
 int nvllm_engine_create_for_model(nvllm_engine** e, const nvllm_config* cfg, const char* model_config_json, int32_t dtype,

@@ -6,7 +6,7 @@ import ctypes as C
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
-# NVLLM_LIB_PATH: debug builds only (e.g. lib/libnvllm_timeline.so for tools/gemm_timeline.py); a missing file still raises
+# NVLLM_LIB_PATH: another build of the library; a missing file still raises
 LIB_PATH = os.environ.get("NVLLM_LIB_PATH") or os.path.join(_HERE, "lib", "libnvllm.so")
 _lib = None
 

@@ -124,7 +124,7 @@ __device__ __forceinline__ void st_release_sys(uint32_t* p, uint32_t v) {
 }
 // 16-byte COHERENT load of data another GPU wrote while this kernel may already be running (ordered after the flag
 // acquire): never through the non-coherent path, never from L1 — ld.global.nc is outside the PTX memory model for
-// memory that changes during the kernel's lifetime (ADVICE r1).
+// memory that changes during the kernel's lifetime.
 __device__ __forceinline__ uint4 ld_sys_16(const void* p) {
   uint4 r;
   asm volatile("ld.relaxed.sys.global.v4.u32 {%0,%1,%2,%3}, [%4];\n"
@@ -173,8 +173,8 @@ struct FusedArParams {
 // Two-shot all-reduce fused with the residual add and the RMSNorm that always follow it (qwen3.rs:382-385,389):
 //   shot 1  rank r owns rows [r*R, (r+1)*R): it reads those rows of every rank's partial sums over NVLink — WORLD is a
 //           template parameter and a thread's WORLD x min(VPT, 2) 16-byte peer loads are all issued before the first add,
-//           so one CTA keeps up to 64 KiB in flight per row (the round-1 kernel issued its peer loads one behind the other
-//           through a run-time loop: ~8x less memory-level parallelism on a ~2 us NVLink round trip).  Fixed rank order of
+//           so one CTA keeps up to 64 KiB in flight per row (one behind the other through
+//           a run-time loop they have ~8x less memory-level parallelism on a ~2 us NVLink round trip).  Fixed rank order of
 //           the adds -> bit-identical on every rank.  The sum is rounded to bf16 (the all-reduced tensor), the residual
 //           added (bf16 tensor add), the row normalised in f32;
 //   shot 2  it writes the normed rows into EVERY rank's buffer (peer stores); the new residual rows stay on the owner
@@ -323,20 +323,6 @@ allreduce_add_rmsnorm_kernel(const FusedArParams p) {
 // Every CTA waits for remote CTAs that may not have started: the grid must be co-resident (launch_fused_ar_ll sizes it
 // from the occupancy calculator), and phase A comes first in every CTA, unconditionally.
 
-#ifdef NVLLM_TIMELINE
-// Debug build only (make timeline, tools/ar_timeline.py): thread 0 of every CTA stamps %globaltimer at the phase boundaries.
-__device__ unsigned long long* g_ar_tl_buf = nullptr;   // [cap][12]: {blockIdx, t0..t8, rows reduced, smid}
-__device__ unsigned int g_ar_tl_cursor = 0;
-__device__ unsigned int g_ar_tl_cap = 0;
-__device__ __forceinline__ unsigned long long ar_tl_now() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;\n" : "=l"(t));
-  return t;
-}
-#define ATL(i) do { if (threadIdx.x == 0) atl[i] = ar_tl_now(); } while (0)
-#else
-#define ATL(i) do { } while (0)
-#endif
 
 __device__ __forceinline__ bool ll_arrived(const uint4& v) {
   return v.x != kLLEmpty && v.y != kLLEmpty && v.z != kLLEmpty && v.w != kLLEmpty;
@@ -365,14 +351,8 @@ __device__ __forceinline__ uint8_t* peer_of(const LLArParams& p, unsigned q) {
 template <int WORLD, int VPT>
 __global__ void __launch_bounds__(512)
 allreduce_add_rmsnorm_ll_kernel(const LLArParams p) {
-#ifdef NVLLM_TIMELINE
-  unsigned long long atl[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  unsigned int atl_rows = 0;
-#endif
-  ATL(0);
   pdl_launch_dependents();
   pdl_wait();
-  ATL(1);
   uint32_t* ctrl = reinterpret_cast<uint32_t*>(p.self);
   const uint32_t b = ld_state(ctrl + 131);                  // pair of this call; advanced by the last CTA of the call
   const uint32_t bclr = b >= 1 ? b - 1 : 2;              // (b + 2) % 3
@@ -403,7 +383,6 @@ allreduce_add_rmsnorm_ll_kernel(const LLArParams p) {
       if (i < nvec) st_sys_16(dst + i * 16, ll_scrub(v[k]));
     }
   }
-  ATL(2);  // partial rows pushed (stores issued)
   // ---- housekeeping while the pushes fly: clear the pair two calls ahead ------------------------------------------
   {
     uint4* c0 = reinterpret_cast<uint4*>(p.self + p.ll_off + static_cast<size_t>(bclr) * 2 * p.ll_cap);
@@ -412,7 +391,6 @@ allreduce_add_rmsnorm_ll_kernel(const LLArParams p) {
     const uint32_t n16 = clr_bytes >> 4;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n16; i += gridDim.x * blockDim.x) { c0[i] = e; c1[i] = e; }
   }
-  ATL(3);  // clear issued
   // ---- B: reduce + add + norm the rows I own, broadcast them -----------------------------------------------------
   const int row0 = p.rank * R;
   const int row1 = min(p.num_tokens, row0 + R);
@@ -449,7 +427,7 @@ allreduce_add_rmsnorm_ll_kernel(const LLArParams p) {
         // Re-poll in ROUNDS: every vector that has not arrived is re-loaded in the same round (all in flight together), so
         // a round costs one L2 round trip however many of the KCH x (WORLD-1) vectors are still missing (spinning on them
         // one after the other could cost up to 14 round trips per thread at 8 ranks; measured it made no difference on an
-        // idle box — 14.4 us per 640 KiB call either way, profiles/r02_scaling.md — but it bounds the worst case).
+        // idle box — 14.4 us per 640 KiB call either way — but it bounds the worst case).
         long long t0 = 0;
         while (true) {
           bool miss = false;
@@ -508,9 +486,6 @@ allreduce_add_rmsnorm_ll_kernel(const LLArParams p) {
     ss = warp_sum(ss);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
     __syncthreads();
-#ifdef NVLLM_TIMELINE
-    if (atl_rows++ == 0) ATL(4);  // first owned row: every staged vector of the CTA has arrived
-#endif
     if (threadIdx.x < 32) {
       float t = (threadIdx.x < (blockDim.x >> 5)) ? red[threadIdx.x] : 0.f;
       t = warp_sum(t);
@@ -538,7 +513,6 @@ allreduce_add_rmsnorm_ll_kernel(const LLArParams p) {
     }
     __syncthreads();  // red / s_inv reuse
   }
-  ATL(5);  // owned rows reduced and broadcast
   // ---- C: gather the rows the other ranks own ----------------------------------------------------------------------
   for (int row = blockIdx.x; row < p.num_tokens; row += gridDim.x) {
     if (row / R == p.rank) continue;
@@ -576,24 +550,8 @@ allreduce_add_rmsnorm_ll_kernel(const LLArParams p) {
       if (i < nvec) *reinterpret_cast<uint4*>(p.out + row * row_bytes + i * 16) = v[k];
     }
   }
-  ATL(6);  // foreign rows gathered
   // ---- the last CTA rotates the pair -------------------------------------------------------------------------------
   __syncthreads();
-  ATL(7);
-#ifdef NVLLM_TIMELINE
-  if (threadIdx.x == 0 && g_ar_tl_buf != nullptr) {
-    const unsigned int slot = atomicAdd(&g_ar_tl_cursor, 1u);
-    if (slot < g_ar_tl_cap) {
-      unsigned long long* e = g_ar_tl_buf + static_cast<size_t>(slot) * 12;
-      unsigned int smid;
-      asm volatile("mov.u32 %0, %%smid;\n" : "=r"(smid));
-      e[0] = blockIdx.x;
-      for (int i = 0; i < 9; ++i) e[1 + i] = atl[i];
-      e[10] = atl_rows;
-      e[11] = smid;
-    }
-  }
-#endif
   if (threadIdx.x == 0) {
     __threadfence();
     if (atomicAdd(ctrl + 135, 1u) == gridDim.x - 1) {
@@ -695,7 +653,7 @@ int nvllm_comm_symm_alloc(nvllm_comm* comm, size_t bytes, void** local_base) {
   cudaIpcMemHandle_t* d_all = nullptr;
   cudaStream_t st = nullptr;
   bool stream_busy = false;  // a collective that never finished may still write d_all: leak it rather than free it
-  // Every early exit below releases what was taken so far (base, d_all and the opened peer mappings leaked).
+  // Every early exit below releases what was taken so far (base, d_all and the opened peer mappings).
   auto fail = [&](int rc) {
     for (int r = 0; r < comm->world; ++r) {
       if (r != comm->rank && comm->sym_peer[r]) cudaIpcCloseMemHandle(comm->sym_peer[r]);
@@ -856,15 +814,6 @@ static int allreduce_add_rmsnorm_any(nvllm_comm* comm, void* out, void* x, void*
   NVLLM_CHECK_ARG(false, NVLLM_ERR_ARG, "allreduce_add_rmsnorm: world %d (2, 4 or 8)", comm->world);
 }
 
-#ifdef NVLLM_TIMELINE
-int nvllmdbg_ar_timeline(unsigned long long* d_buf, unsigned int cap) {
-  unsigned int zero = 0;
-  if (cudaMemcpyToSymbol(nvllm::g_ar_tl_buf, &d_buf, sizeof(d_buf)) != cudaSuccess) return 1;
-  if (cudaMemcpyToSymbol(nvllm::g_ar_tl_cap, &cap, sizeof(cap)) != cudaSuccess) return 1;
-  if (cudaMemcpyToSymbol(nvllm::g_ar_tl_cursor, &zero, sizeof(zero)) != cudaSuccess) return 1;
-  return 0;
-}
-#endif
 
 // 0, or NVLLM_ERR_COMM once a fused kernel of this communicator has given up waiting for a peer (sticky).
 int nvllm_comm_error(const nvllm_comm* comm) {

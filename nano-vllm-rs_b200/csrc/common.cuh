@@ -57,12 +57,12 @@ bool gemm_skinny_applies(int m, int n, int k, int64_t ldx, int64_t ldw, bool f32
 int gemm_skinny(void* y, const void* x, const void* w, int m, int n, int k, int64_t ldx, int64_t ldw, int64_t ldy, int out_dtype, bool silu_gate,
                 const void* norm_w, float eps, bool residual, cudaStream_t st);
 
-// The NVLLM_* environment knobs (A/B measurements; DESIGN.md appendix), parsed ONCE per process — never on a dispatch
+// The NVLLM_* environment knobs (A/B measurements), parsed ONCE per process — never on a dispatch
 // path.  nvllm_reload_env() (benchmark tools that sweep knobs inside one process) re-parses them.
 struct Knobs {
   int pdl = 1;              // NVLLM_PDL: 0 disables programmatic dependent launch
-  int pdl_tp = 0;           // NVLLM_PDL_TP: 1 keeps programmatic dependent launch while a TP symmetric region is live (round-2
-                            // behaviour: ~1 in 10 tiny-model runs at 8 ranks ends with rank 0 one call behind)
+  int pdl_tp = 0;           // NVLLM_PDL_TP: 1 keeps programmatic dependent launch while a TP symmetric region is live (about 1 in 10
+                            // tiny-model runs at 8 ranks then ends with rank 0 one call behind)
   int gemm_bn = 0;          // NVLLM_GEMM_BN: forced tile width (0 = heuristic)
   int gemm_2cta = 1;        // NVLLM_GEMM_2CTA: 0 never, 1 default (M > 512), 2 every M > 128
   int gemm_skinny = 1;      // NVLLM_GEMM_SKINNY: 0 keeps products of up to 16 rows on the tcgen05 kernels
@@ -92,7 +92,7 @@ extern std::atomic<int> g_live_symm_regions;  // api.cu; nvllm_comm_symm_alloc +
 // Programmatic dependent launch is OFF while this process holds a tensor-parallel symmetric region, unless NVLLM_PDL_TP=1:
 // with it on, the fused all-reduce kernels' per-call device state (buffer pair / epoch, handed from one call to the next
 // through the control block) was observed one call stale on the rank whose kernels never spin (8 ranks, 4-CTA grids, about
-// one run in ten; tools/tp_parity_soak.py); with it off, 50 consecutive runs were clean.  Root cause open.
+// one run in ten; tools/tp_parity_soak.py); with it off, 50 consecutive runs were clean.  The root cause is open.
 inline bool pdl_enabled() {
   return knobs().pdl != 0 && (knobs().pdl_tp != 0 || g_live_symm_regions.load(std::memory_order_relaxed) == 0);
 }
@@ -117,18 +117,19 @@ inline bool pdl_enabled() {
 namespace nvllm {
 
 // ---- Programmatic dependent launch (PDL) -----------------------------------------------------------
-// Every kernel of the step is launched with cudaLaunchAttributeProgrammaticStreamSerialization: it may start while
-// its predecessor is still running.  Contract inside each kernel: pdl_launch_dependents() first (lets the successor
-// be scheduled), then only predecessor-independent work (barrier init, TMEM alloc, descriptor / weight prefetch),
-// then pdl_wait() before the first access to anything a previous kernel wrote or still reads.
+// Most kernels of a step are launched with cudaLaunchAttributeProgrammaticStreamSerialization (launch_pdl): such a kernel may start while
+// its predecessor is still running.  Contract: before pdl_wait() only work that does not depend on the predecessor (barrier init, TMEM
+// alloc, descriptor / weight prefetch), after it everything that a previous kernel wrote or still reads.  pdl_launch_dependents() lets the
+// successor be scheduled: first thing in most kernels; after pdl_wait() where CTAs of several kernels of the chain on one SM cost more than
+// the overlap gives (the kernel says so).  Kernels that launch_plain starts wait for their predecessor in stream order; pdl_wait()
+// returns at once in them.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-// A word of per-communicator device state that ONE CTA of an earlier kernel rewrites and EVERY CTA of a later kernel reads
-// (call counters, buffer-pair index, dead flag in the symmetric region's control block).  Read it past L1: with
-// programmatic dependent launch a CTA of the later kernel can be resident on an SM (launched early, parked in
-// griddepcontrol.wait) BEFORE a CTA of the earlier kernel on the same SM pulls the old value of the line into that SM's
-// L1 — the later kernel's ordinary ld.global then hits the stale line.  Observed as a rank that re-used the previous
-// call's buffer pair / epoch (the round-2 8-GPU hang); a gpu-scope load always goes to L2.
+// A word of per-communicator device state that ONE CTA of an earlier kernel rewrites and EVERY CTA of a later kernel reads (call counters,
+// buffer-pair index, dead flag in the symmetric region's control block): read at gpu scope, from L2, so that its value depends on no line
+// that an earlier CTA brought into this SM's L1.  (Ordinary loads of data are sound behind pdl_wait(): griddepcontrol.wait makes the
+// predecessors' writes visible to them, in-place updates included.  The stale counters that pdl_enabled() tells of came back with
+// these loads too, so L1 was not their cause.)
 __device__ __forceinline__ uint32_t ld_state(const uint32_t* p) {
   uint32_t v;
   asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");

@@ -1,6 +1,6 @@
 // gemm_splitk.cu — K5'': split-K variant of the tcgen05 GEMM for the decode-sized projections (M <= 512 rows).
 //
-// Why: measured in-graph (profiles/r01_gemm_ingraph_v1.jsonl) the small-M GEMMs cost ~0.31 us per 64-wide k-block per
+// Why: measured in-graph the small-M GEMMs cost ~0.31 us per 64-wide k-block per
 // CTA whatever the tile width — each SM can only ingest ~35-45 B/clk through TMA, and every CTA of a 128 x BN tile has
 // to pull (128 + BN) x K x 2 bytes on its own (the x tile is re-read by every n-tile; multicasting it does not help,
 // the bytes still have to enter each SM).  o_proj / down_proj of Qwen3-0.6B (N = 1024, K = 2048 / 3072) run on only
@@ -15,23 +15,6 @@
 #include "tc.cuh"
 
 namespace nvllm {
-#ifdef NVLLM_TIMELINE
-// Debug build only (make timeline -> lib/libnvllm_timeline.so, tools/gemm_timeline.py): every CTA records %globaltimer at
-// its phase boundaries into a host-provided buffer, to decompose the fixed per-launch cost of the decode-sized GEMMs.
-__device__ unsigned long long* g_tl_buf = nullptr;   // [cap][12]: {blockIdx, t0..t9, smid}
-__device__ unsigned int g_tl_cursor = 0;
-__device__ unsigned int g_tl_cap = 0;
-__device__ __forceinline__ unsigned long long tl_now() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;\n" : "=l"(t));
-  return t;
-}
-#define TL_DECL __shared__ unsigned long long tl_s[12];
-#define TL(i) do { tl_s[i] = tl_now(); } while (0)
-#else
-#define TL_DECL
-#define TL(i) do { } while (0)
-#endif
 namespace {
 
 template <int BN>
@@ -43,7 +26,7 @@ struct SkCfg {
   static constexpr int kMaxStages = (192 * 1024) / kStageBytes > 8 ? 8 : (192 * 1024) / kStageBytes;
   // f32 partial tile, column-major [BN][128]: a warp (32 consecutive rows of one column) touches 128 contiguous bytes, for
   // the local stores (conflict-free) and for the DSMEM loads (one coalesced request per warp — strided 16-byte DSMEM
-  // loads measured 2.4 us slower per kernel, profiles/r01_gemm_ingraph_v3_splitk_v2.jsonl)
+  // loads measured 2.4 us slower per kernel)
   static constexpr int kColPitch = BM * 4;
   static constexpr int kPartialBytes = BN * kColPitch;
   static constexpr int kTmemCols = BN < 32 ? 32 : BN;
@@ -95,8 +78,6 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
   const int tile = static_cast<int>(blockIdx.x) / SK;
   const int m_tile = tile % num_m_tiles, n_tile = tile / num_m_tiles;
   const int kb_per = (K / C::BK) / SK, kb0 = rank * kb_per;
-  TL_DECL
-  if (threadIdx.x == 0) TL(0);   // kernel entry
   pdl_launch_dependents();
 
   if (warp == 0 && lane == 0) {
@@ -113,7 +94,6 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
-  if (threadIdx.x == 0) TL(1);   // prologue (barrier init, TMEM alloc) done
 
   if (warp == 0 && lane == 0) {
     // ===== TMA producer: weights first (independent of the predecessor kernel), x after the dependency wait =====
@@ -131,7 +111,6 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
       load_w(i, kb0 + i);
     }
     pdl_wait();
-    TL(2);   // predecessor kernel complete (x may be loaded)
     int stage = 0;
     uint32_t phase = 0;
     for (int i = 0; i < kb_per; ++i) {
@@ -151,8 +130,6 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     pdl_wait();  // keep the wait for the predecessor out of the bounded mbarrier waits
     for (int i = 0; i < kb_per; ++i) {
       mbar_wait(full_bar(stage), phase);
-      if (i == 0) TL(3);             // first operand stage landed
-      if (i == kb_per - 1) TL(4);    // last operand stage landed
       tc_fence_after();
       const uint32_t a0 = sA + stage * C::kABytes, b0 = sB + stage * C::kBBytes;
 #pragma unroll
@@ -168,7 +145,6 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     const int q = warp & 3;
     pdl_wait();               // (also needed below: y may still be read by an earlier kernel)
     mbar_wait(tfull_bar, 0);  // every MMA has retired: the operand ring is dead and can be overwritten
-    if (threadIdx.x == 128) TL(5);   // accumulator complete
     tc_fence_after();
     const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
     const uint32_t prow = smem_base + (q * 32 + lane) * 4;
@@ -183,9 +159,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     tc_fence_before();
   }
   __syncwarp();
-  if (threadIdx.x == 128) TL(6);     // partial tile parked in shared memory
   cluster_sync_all();  // all SK partial tiles are parked and visible cluster-wide
-  if (threadIdx.x == 128) TL(7);     // first cluster barrier passed
 
   if (warp >= 4) {
     // ===== reduce this CTA's column slice over the cluster in fixed rank order, then the usual epilogue =====
@@ -274,27 +248,11 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     }
   }
   __syncwarp();
-  if (threadIdx.x == 128) TL(8);     // DSMEM reduce + global stores done
   cluster_sync_all();  // nobody leaves while a peer may still read its partial tile
   if (warp == 2) {
     tc_fence_after();
     tmem_dealloc<C::kTmemCols>(tmem_base);
   }
-#ifdef NVLLM_TIMELINE
-  if (threadIdx.x == 128) TL(9);
-  __syncthreads();
-  if (threadIdx.x == 0 && g_tl_buf != nullptr) {
-    const unsigned int slot = atomicAdd(&g_tl_cursor, 1u);
-    if (slot < g_tl_cap) {
-      unsigned long long* e = g_tl_buf + static_cast<size_t>(slot) * 12;
-      unsigned int smid;
-      asm volatile("mov.u32 %0, %%smid;\n" : "=r"(smid));
-      e[0] = blockIdx.x;
-      for (int i = 0; i < 10; ++i) e[1 + i] = tl_s[i];
-      e[11] = smid;
-    }
-  }
-#endif
 }
 
 // Stages of the operand ring: NVLLM_GEMM_SK_STAGES (benchmark knob) or the deepest that fits, never more than the
@@ -335,7 +293,6 @@ int launch_splitk(const CUtensorMap& tx, const CUtensorMap& tw, void* y, int M, 
 // partial tile over DSMEM — (SK-1)/SK of a BN x 128 f32 tile per CTA at ~20 B/clk (B300_MICROARCH.md: 17-21 B/clk), i.e.
 // weighted x4 — which is why narrow tiles with SK = 4 win for the 0.6B projections.  Clusters of 8 measured 3-6 us
 // slower than clusters of 4 at equal bytes (fewer can be co-scheduled per GPC): flat penalty.
-// Data: profiles/r01_gemm_ingraph_v2_splitk.jsonl, r01_gemm_ingraph_v3_splitk_v2.jsonl.
 long splitk_cost(int bn, int sk, int k) {
   return 2l * (128 + bn) * (k / sk) + (sk > 1 ? 4l * 512 * bn * (sk - 1) / sk : 0) + (sk >= 8 ? 600l * 1024 : 0);
 }
@@ -377,17 +334,6 @@ bool splitk_choose(int m, int n_acc, int k, bool silu, int bn_default, int* out_
   return best * 10 < splitk_cost(bn_default, 1, k) * waves_d * 9;  // at least 10 % fewer bytes per SM
 }
 
-#ifdef NVLLM_TIMELINE
-}  // namespace nvllm
-extern "C" int nvllmdbg_timeline(unsigned long long* d_buf, unsigned int cap) {
-  unsigned int zero = 0;
-  if (cudaMemcpyToSymbol(nvllm::g_tl_buf, &d_buf, sizeof(d_buf)) != cudaSuccess) return 1;
-  if (cudaMemcpyToSymbol(nvllm::g_tl_cap, &cap, sizeof(cap)) != cudaSuccess) return 1;
-  if (cudaMemcpyToSymbol(nvllm::g_tl_cursor, &zero, sizeof(zero)) != cudaSuccess) return 1;
-  return 0;
-}
-namespace nvllm {
-#endif
 
 int gemm_splitk_dispatch(void* y, const void* x, const void* w, int m, int n, int k, int64_t ldx, int64_t ldw, int64_t ldy,
                          int gate, int bn, int sk, cudaStream_t st, const RowPush& ps, float glu_limit, int out_dtype) {

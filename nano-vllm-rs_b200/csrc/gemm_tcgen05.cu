@@ -421,7 +421,7 @@ static bool use_2cta();
 static bool want_2cta(int m, int n, int k) {
   if (m <= 128 || !use_2cta()) return false;
   if (knobs().gemm_2cta == 2) return true;  // benchmark knob: CTA pairs for every m > 128
-  // In-graph measurements (profiles/r01_gemm_ingraph_v2_splitk.jsonl): at M = 512 (the TP decode batches) the single-CTA
+  // In-graph measurements: at M = 512 (the TP decode batches) the single-CTA
   // kernel is 7-17 % faster on all four projections; CTA pairs pay off from two 256-row tile rows upwards (prefill).
   if (m <= 512) return false;
   (void)n; (void)k;

@@ -32,7 +32,7 @@ int nvllm_config_init(nvllm_config* c, const char* arch) {
   c->max_num_batched_tokens = 32768; c->max_num_seqs = 512; c->max_model_len = 4096;
   c->tensor_parallel_size = 1; c->enforce_eager = 0; c->kvcache_block_size = 256; c->num_kvcache_blocks = 0;
   c->tp_rank = 0; c->eos_token_id = -1;
-  // common Qwen3 values (SURVEY.md §8): vocab 151936, eps 1e-6, head_dim 128, qk-norm, theta 1e6
+  // common Qwen3 values: vocab 151936, eps 1e-6, head_dim 128, qk-norm, theta 1e6
   c->vocab_size = 151936; c->head_dim = 128; c->max_position_embeddings = 40960; c->qk_norm = 1;
   c->rms_norm_eps = 1e-6f; c->rope_theta = 1e6; c->kv_layout = 0;
   if (!strcmp(arch, "qwen3-0.6b")) {

@@ -403,7 +403,7 @@ int nvllm_runner::create(const nvllm_config& c, nvllm_comm* cm) {
 
 // ------------------------------------------------------------------------------------------------ weights
 // Logical tensor ids of the seeded init (mirrored by oracle/qwen3.py): 1 embed, 2 lm_head, 16*(l+1) + {0 q, 1 k,
-// 2 v, 3 o, 4 gate, 5 up, 6 down}.  Norm weights are 1 (SURVEY.md §8d).
+// 2 v, 3 o, 4 gate, 5 up, 6 down}.  Norm weights are 1.
 int nvllm_runner::init_weights(uint64_t seed, float std) {
   if (model) {
     RUN(model->init_weights(seed, std, stream));
@@ -707,7 +707,7 @@ int nvllm_runner::forward(int N, int S, bool is_prefill, bool paged_prefill, con
       if (few) RUN(few_gemm(qkv, h, w.qkv, N, qkv_dim, hidden, qkv_dim, NVLLM_BF16, false, w.input_ln, false, "norm + qkv_proj"));
       else RUN(gemm(qkv, normed, w.qkv, qkv_dim, hidden, qkv_dim, NVLLM_BF16, "qkv_proj GEMM"));
       if (is_prefill || !rope_in_decode(N, S)) {
-        // q/k norm + RoPE in place, K/V of this step into the cache (store before attention: note N2)
+        // q/k norm + RoPE in place, K/V of this step into the cache (stored before the attention reads it)
         RUN(nvllm_qknorm_rope_store(qkv, d_pos, rope, qnw, knw, eps, N, H, Hkv, D, cfg.max_position_embeddings, kc[l], vc[l],
                                     d_slots, &layout, NVLLM_BF16, st)); ++launches;
         mark("qknorm_rope_store");
@@ -1080,7 +1080,7 @@ int nvllm_runner_time_decode_attention(nvllm_runner* r, int32_t iters, float* ms
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   *ms_per_launch = ms / iters;
-  if (alg_bytes) {  // SURVEY.md §8d: sum_b 2*L_b*Hkv*D*2 + 2*B*H*D*2 + 4*sum_b ceil(L_b/bs) + 4*B
+  if (alg_bytes) {  // sum_b 2*L_b*Hkv*D*2 + 2*B*H*D*2 + 4*sum_b ceil(L_b/bs) + 4*B
     int64_t bytes = 0;
     for (int32_t L : r->last_ctx)
       bytes += 2ll * L * r->Hkv * r->D * 2 + 4ll * ((L + r->layout.block_size - 1) / r->layout.block_size);

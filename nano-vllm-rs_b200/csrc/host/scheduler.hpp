@@ -326,7 +326,7 @@ class Scheduler {
   }
 
   // prepare_prefill_inputs + create_prefill_context (model_runner.rs:172-193,222-263) with the intended slot
-  // mapping and cached-prefix handling (SURVEY.md §8 a14; oracle/host.py prepare_prefill).
+  // mapping and cached-prefix handling (oracle/host.py prepare_prefill).
   void build_prefill(nvllm_batch* out) {
     fill_common(out, true);
     BatchArrays& a = arrays_;

@@ -23,7 +23,7 @@
 //   GPCs are a cluster (FUSE) and meet in distributed shared memory; otherwise fp32 partials + (m, l) go to the workspace and
 //   paged_decode_reduce_kernel combines them.
 //
-// Algorithmic bytes per launch (SURVEY.md §8d): sum_b 2*L_b*Hkv*D*2 + 2*B*H*D*2 + 4*sum_b ceil(L_b/bs) + 4*B.
+// Algorithmic bytes per launch: sum_b 2*L_b*Hkv*D*2 + 2*B*H*D*2 + 4*sum_b ceil(L_b/bs) + 4*B.
 #include <math.h>
 
 #include <atomic>
@@ -818,9 +818,9 @@ extern "C" int nvllm_paged_decode_choose_splits(int32_t batch, int32_t num_heads
   long max_s = max_context_len / 256;          // keep >= 256 tokens per split
   if (max_s < 1) max_s = 1;
   if (max_s > 64) max_s = 64;
-  // Measured (profiles/r02_decode_split_sweep.jsonl, 512 seqs x 1536 tokens, Hkv = 1 / 2 / 4 / 8 per rank): once the grid
+  // Measured (512 seqs x 1536 tokens, Hkv = 1 / 2 / 4 / 8 per rank): once the grid
   // holds a full wave, ONE split wins at every shard shape — 5.94 vs 5.16 TB/s at Hkv = 1 (512 CTAs = 1.73 waves), where
-  // round 1's wave-filling model picked 4.  A split costs its f32 partials, a second launch and shorter CTAs (6-24 % at
+  // a model that fills waves picks 4.  A split costs its f32 partials, a second launch and shorter CTAs (6-24 % at
   // 2-8 splits); dynamic CTA scheduling already hides most of a ragged last wave.  Split only to FILL the first wave
   // (few sequences x long contexts: 64 x 32.5K at Hkv = 1 -> 4 splits = 256 CTAs, the measured best).
   if (base >= slots) return 1;

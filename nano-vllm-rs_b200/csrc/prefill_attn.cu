@@ -48,7 +48,7 @@ struct PrefillParams {
 
 // POLY: how many of every 4 exponentials go to a polynomial instead of MUFU.EX2 (NVLLM_PREFILL_POLY): 1 / 2 / 3 with the
 // floor-based polynomial (the first version; its floor and float-to-int also run on the XU pipe, so 2 and 3 gain nothing over 1),
-// 4 / 5 / 6 = 1/4, 1/2, 3/4 with the XU-free polynomial.  Default 4 (measured best: profiles/r01_prefill_microbench_v5_polysplit.jsonl).
+// 4 / 5 / 6 = 1/4, 1/2, 3/4 with the XU-free polynomial.  Default 4 (measured best).
 template <int POLY>
 __global__ void __launch_bounds__(pf::kThreads, 1)
 prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,

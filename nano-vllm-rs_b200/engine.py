@@ -1,6 +1,6 @@
 """Python mirror of the reference's public API over the C++ host runtime (include/nvllm_engine.h).
 
-Names, fields and defaults follow the reference crate (SURVEY.md Appendix A): Config (config.rs:16-186),
+Names, fields and defaults follow the reference crate: Config (config.rs:16-186),
 SamplingParams (sampling_params.rs:10-120), Scheduler (scheduler.rs), ModelRunner (model_runner.rs), LLMEngine /
 LLMEngineBuilder (llm_engine.rs:39-483).  All state and logic live in libnvllm.so; this file only marshals."""
 import ctypes as C

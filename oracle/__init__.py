@@ -5,7 +5,7 @@ paged-attention decode hot path of ssvgopal/nano-vllm-rs.  Each function cites t
 file:line it follows.  Only tests/, __graft_entry__.smoke() and bench.py's cpu_baseline / --impl reference
 legs may import this package; the product (nano-vllm-rs_b200/) never does.
 
-Parity pinning (SURVEY.md §8c): the reference cannot be compiled or run here (no Rust toolchain, invalid
+Parity pinning: the reference cannot be compiled or run here (no Rust toolchain, invalid
 manifest, type errors on the path), and it holds NO numeric golden vectors for attention outputs, logits or
 tokens.  What it does pin, and what tests/test_oracle_*.py check this oracle against:
   * block accounting / scheduler / sequence / runner-input known answers of the reference's in-file unit tests

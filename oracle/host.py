@@ -2,8 +2,8 @@
 
 Everything here must be reproduced BIT-EXACTLY by the C++ host (csrc/host/): block ids, ref-counts, hashes,
 block tables, slot mappings, context lengths, cu_seqlens, scheduling order.  Citations are file:line under
-/root/reference/src/engine/.  Where the reference is internally inconsistent or does not compile, the INTENT
-stated in SURVEY.md §8 (notes N1-N3, row a14) is followed and marked "intent:"."""
+the reference's src/engine/.  Where the reference is internally inconsistent or does not compile, the INTENT
+stated beside it is followed and marked "intent:"."""
 from collections import deque
 from dataclasses import dataclass, field
 from typing import List, Optional
@@ -123,7 +123,7 @@ class Block:
 
 
 class BlockManager:
-    """block_manager.rs:69-331.  Quirks kept on purpose (SURVEY.md §8 note N3): FIFO free list taken from the
+    """block_manager.rs:69-331.  Quirks kept on purpose: FIFO free list taken from the
     front, freed ids appended at the back in reverse table order; the hash->block entry is dropped when a block
     is freed; a cache hit does not re-`update` the block; can_allocate demands free >= num_blocks(seq) even when
     most blocks will be hits."""
@@ -374,7 +374,7 @@ def _padded_tables(sequences, width=None):
 
 def prepare_prefill(sequences, block_size) -> StepInputs:
     """prepare_prefill_inputs + create_prefill_context, model_runner.rs:172-193,222-263.
-    intent (SURVEY.md §8 a14): the reference's slot_mapping is a placeholder (:241-243) and it ignores
+    intent: the reference's slot_mapping is a placeholder (:241-243) and it ignores
     num_cached_tokens (:177); intended: only the uncached suffix [start, len) is computed, positions are absolute,
     slot = table[p / bs] * bs + p % bs, cu_seqlens_k counts the whole sequence, and block tables are passed iff some
     sequence has a cached prefix (attention.rs:85-91 branch).  start = min(num_cached_tokens, len - 1): a fully

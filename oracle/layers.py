@@ -2,7 +2,7 @@
 
 All tensors are float32 numpy arrays holding bf16-representable values ("bf16 tensors"); `round_bf16`
 is applied wherever the reference materialises a tensor in the model dtype.  Citations are
-file:line in /root/reference/src."""
+file:line of the reference, under src/."""
 import numpy as np
 
 from .bf16 import round_bf16
@@ -49,7 +49,7 @@ def softmax_last_dim(x):
 
 def compute_attention(q, k, v, scale, causal):
     """Attention::compute_attention, attention.rs:238-261, per head (the reference's transpose(1,2) on
-    [L,H,D] batches over tokens — SURVEY.md §8 a4; the intent, per-head attention, is restated).
+    [L,H,D] batches over tokens; the intent, per-head attention, is restated).
     q: [Lq, H, D], k, v: [Lk, Hkv, D]; GQA map h -> h // (H/Hkv) (expand_kv_heads, attention.rs:419-435).
     f32 math on bf16 inputs, output rounded to bf16."""
     lq, H, D = q.shape
@@ -71,7 +71,7 @@ def compute_attention(q, k, v, scale, causal):
 def gather_cached_kv(k_cache, v_cache, block_table, context_len=None):
     """Attention::gather_cached_kv, attention.rs:293-318: concatenate the blocks listed in the table,
     skipping ids < 0 (:306).  The reference then attends to every slot of the last block including
-    unwritten zeros; the intent (note N1) truncates to context_len."""
+    unwritten zeros; the intent truncates to context_len."""
     ks, vs = [], []
     for bid in block_table:
         bid = int(bid)
@@ -114,7 +114,7 @@ def flash_attention_varlen(q, k, v, cu_seqlens_q, cu_seqlens_k, scale):
 
 
 def flash_attention_varlen_with_cache(q, k_cache, v_cache, block_tables, cu_seqlens_q, cu_seqlens_k, scale):
-    """Attention::flash_attention_varlen_with_cache, attention.rs:211-222 (intent, SURVEY.md §8 a5): the
+    """Attention::flash_attention_varlen_with_cache, attention.rs:211-222 (its intent): the
     uncached suffix of each sequence attends, bottom-right causally, to prefix + itself read back from the
     paged cache through block_tables (this step's K/V already stored — note N2)."""
     outs = []
@@ -217,7 +217,7 @@ def greedy_sample(logits):
     return np.argmax(logits, axis=-1).astype(np.int64)
 
 
-# ---------------------------------------------------------------------------- sampler (SURVEY.md §8f #3)
+# ---------------------------------------------------------------------------- sampler
 #
 # Sampler::forward / sample_single / apply_top_k / apply_top_p / multinomial_sample / sample_gumbel, sampler.rs:26-219.
 # The reference draws its uniforms from an UNSEEDED Tensor::rand (sampler.rs:208), so its random draws cannot be

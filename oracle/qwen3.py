@@ -4,7 +4,7 @@ Qwen3Model::forward (models/qwen3.rs:487-505) -> Qwen3Layer::forward (:372-392) 
 (:208-240) -> Attention::forward (layers/attention.rs:65-99) / Qwen3MLP::forward (qwen3.rs:305-314) ->
 ParallelLMHead::forward (layers/embed_head.rs:250-306) -> Sampler::greedy_sample (layers/sampler.rs:109-112).
 f32 math on bf16-representable values, rounded to bf16 wherever the reference materialises a model-dtype tensor.
-Deviations N1 of SURVEY.md §8 (qk-norm, explicit head_dim, f32 RoPE table, context_lens truncation, seeded weights
+Deviations (qk-norm, explicit head_dim, f32 RoPE table, context_lens truncation, seeded weights
 incl. the LM head) are flag-controlled / stated in oracle/layers.py."""
 import numpy as np
 

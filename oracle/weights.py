@@ -1,7 +1,7 @@
 """Seeded synthetic weights shared bit-for-bit with the device (nvllm_init_weight, csrc/fused_ops.cu).
 
 The reference leaves weight init unspecified (linear.rs:37 calls a candle overload that does not exist;
-the LM head is re-randomised on every call, embed_head.rs:309-318).  SURVEY.md §8d: seeded N(0, 0.02^2),
+the LM head is re-randomised on every call, embed_head.rs:309-318).  Here: seeded N(0, 0.02^2),
 identical bytes for oracle and GPU.  To be reproducible without transcendental functions the normal is
 approximated by an Irwin-Hall sum: the four 16-bit fields of splitmix64(key + (i+1)*golden), minus their
 mean 131070, times std/37837.23 — integer arithmetic and one exact int->f32 multiply."""

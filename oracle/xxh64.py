@@ -1,6 +1,6 @@
 """XXH64 restated from the published algorithm (xxHash specification, "XXH64 algorithm description").
 
-Third-party arithmetic that is NOT under /root/reference: the reference calls `xxhash_rust::xxh64::xxh64(&data, 0)`
+Third-party arithmetic, not part of the reference itself: the reference calls `xxhash_rust::xxh64::xxh64(&data, 0)`
 (Cargo.toml:39 `xxhash-rust = "0.8"` feature xxh64, unpinned — no Cargo.lock; call site
 src/engine/block_manager.rs:7,122).  xxhash-rust implements canonical XXH64, so parity is anchored on the
 canonical known-answer vectors (tests/golden/xxh64.json) and on the reference's own call site semantics:

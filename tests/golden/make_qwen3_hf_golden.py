@@ -2,7 +2,7 @@
 `transformers` Qwen3ForCausalLM (fp32, CPU, eager attention) — on a tiny random Qwen3 (2 layers, GQA 4/2 heads, head_dim 128,
 per-head q/k RMSNorm, half-split RoPE theta 1e6, untied head) whose weights (bf16-representable, norm weights != 1) are
 stored in the fixture's seed.  tests/test_oracle_model.py checks oracle/qwen3.py (paged KV cache, prefill + decode steps,
-bf16 rounding at the tensor boundaries) against it: this pins the model WIRING of SURVEY.md §8 note N1 (q/k-norm placement,
+bf16 rounding at the tensor boundaries) against it: this pins the model WIRING (q/k-norm placement,
 RoPE convention, GQA mapping, residual / norm order) that the reference itself leaves unpinned.  Run from the repo root."""
 import json
 import os
@@ -23,7 +23,7 @@ CFGS = {"tiny": (CFG, "qwen3_hf.json"), "wide": (CFG_WIDE, "qwen3_hf_wide.json")
 SEED, STD = 20261104, 0.05
 PROMPTS = [[5, 17, 900, 3, 44], [1023, 0, 7, 7, 512, 64, 33, 2, 81, 300, 11, 640]]
 FORCED = [[10, 20, 30], [700, 5, 999]]   # tokens appended at the three decode steps (teacher forcing)
-# prefix caching (SURVEY.md §8 a5): two prompts sharing a 32-token prefix (= 2 full blocks of 16), different suffixes
+# prefix caching: two prompts sharing a 32-token prefix (= 2 full blocks of 16), different suffixes
 PREFIX = [(i * 37 + 11) % 1024 for i in range(32)]
 SUFFIXES = [[3, 1, 4, 1, 5], [9, 2, 6, 5, 3, 5, 8, 9, 7]]
 

@@ -1,6 +1,6 @@
 """CPU tests of bench.py: the reference arm (`--impl reference`, the CPU oracle port timed on the host cores) prints one JSON
-line with the keys the driver's contract names, on the same metric / unit / workload wording as the GPU arm; the workload
-window arithmetic follows BASELINE.json's configs.  (The GPU arm itself is exercised on the GPU box by the driver.)"""
+line with the contract's keys, on the same metric / unit / workload wording as the GPU arm; the workload window arithmetic
+follows the declared workloads.  (The GPU arm itself needs a GPU.)"""
 import json
 import os
 import subprocess
@@ -48,7 +48,7 @@ def test_workload_windows_follow_the_baseline_configs():
     args.model = "qwen3-32b"
     model, wl, prompt, K, W = bench.workload(args)
     assert wl["seqs"] == 64 and wl["blocks_per_seq"] == 129
-    assert "decode" in base["metric"] or "token" in base["metric"]              # the metric bench.py prints is BASELINE.json's
+    assert "decode" in base["metric"] or "token" in base["metric"]              # the metric bench.py prints is the declared one
 
 
 def test_watchdog_names_the_stalled_phase_on_stdout():

@@ -155,8 +155,8 @@ def test_engine_sampling_is_reproducible_and_seeded(cuda):
 
 
 def test_cfg1_qwen3_0_6b_4x128_prompts_64_decode_steps(cuda):
-    """BASELINE config 1: Qwen3-0.6B random-init, batch 4 x 128-token synthetic prompts (seed 1234), 64 greedy decode
-    steps (max_tokens = 65: 1 prefill + 64 decode forwards, SURVEY.md Appendix B), KV block 256."""
+    """Qwen3-0.6B random-init, batch 4 x 128-token synthetic prompts (seed 1234), 64 greedy decode
+    steps (max_tokens = 65: 1 prefill + 64 decode forwards), KV block 256."""
     rng = np.random.default_rng(1234)
     prompts = [rng.integers(0, 151936, 128).tolist() for _ in range(4)]
     stats, _ = run_lockstep("qwen3-0.6b", prompts, max_tokens=65, bs=256, num_blocks=16, std=0.02, max_num_seqs=8,
@@ -167,7 +167,7 @@ def test_cfg1_qwen3_0_6b_4x128_prompts_64_decode_steps(cuda):
 
 
 def test_cfg4_shape_prefix_cached_prefill_then_decode_qwen3_0_6b(cuda):
-    """BASELINE configs[3] shape on Qwen3-0.6B dimensions (the 8B oracle would take hours on the CPU): a 4096-token shared
+    """Prefix caching on Qwen3-0.6B dimensions (the 8B oracle would take hours on the CPU): a 4096-token shared
     prefix (seed 4321, 16 full blocks of 256) + 256 unique tokens, three sequences — sequence 0 computes all 4352 tokens,
     the two sharers hit its 16 blocks in the SAME prefill batch (note N2: K/V stored before attention reads the cache) and
     compute only their suffix against the paged prefix (attention.rs:211-222, block_manager.rs:157-219) — then one decode

@@ -12,7 +12,7 @@ from tests.util import (assert_close, cache_from_layout, cache_to_layout, make_p
 
 pytestmark = pytest.mark.gpu
 
-# attention tolerance (SURVEY.md §8c): |d| <= 1e-2 + 1.6e-2 |ref|  (~2 bf16 ulps of the output + P rounding)
+# attention tolerance: |d| <= 1e-2 + 1.6e-2 |ref|  (~2 bf16 ulps of the output + P rounding)
 ATT_ATOL, ATT_RTOL = 1e-2, 1.6e-2
 
 
@@ -222,7 +222,7 @@ def test_paged_decode_fused_splits_merge_alike(cuda):
 
 
 def test_paged_decode_full_size_properties(cuda):
-    """BASELINE config 2 shape (256 seqs x 1024 ctx, 16/8 heads): size-independent checks —
+    """256 seqs x 1024 ctx, 16/8 heads: size-independent checks —
     (i) V == const c per head  =>  out == c exactly representable in bf16;  (ii) split-K invariance;
     (iii) layout invariance (reference vs head-major physical layouts give identical bits)."""
     from nano_vllm_rs_b200 import ops

@@ -9,7 +9,7 @@ from oracle import layers as O
 from tests.util import assert_close, cache_to_layout, make_paged_kv, randn_bf16, to_dev_bf16, to_np_f32
 
 pytestmark = pytest.mark.gpu
-ATT_ATOL, ATT_RTOL = 1e-2, 1.6e-2   # SURVEY.md §8c attention tolerance
+ATT_ATOL, ATT_RTOL = 1e-2, 1.6e-2   # attention tolerance (2 bf16 ulps of the output + P rounding)
 
 
 def _cu(lens):
@@ -18,7 +18,7 @@ def _cu(lens):
 
 DENSE = [
     ([1], 4, 2), ([5], 16, 8), ([64], 4, 4), ([65, 1, 128], 4, 2), ([129, 256, 257], 8, 2), ([300, 513, 7], 16, 8),
-    ([1024], 32, 8), ([128] * 4, 16, 8),   # the last one is BASELINE config 1's prefill shape
+    ([1024], 32, 8), ([128] * 4, 16, 8),   # the last one is the 4 x 128-token prefill of Qwen3-0.6B
 ]
 
 
@@ -77,7 +77,7 @@ def test_varlen_prefill_paged_prefix_vs_oracle(cuda, kind, case):
 
 
 def test_varlen_prefill_full_size_vs_torch(cuda):
-    """BASELINE config 2 prefill step: 64 seqs x 512 tokens, 16/8 heads — against torch SDPA (fp32 math on the
+    """A full prefill step: 64 seqs x 512 tokens, 16/8 heads — against torch SDPA (fp32 math on the
     device) on sampled sequences, plus the paged == dense consistency property."""
     from nano_vllm_rs_b200 import ops
     B, L, H, Hkv, D = 64, 512, 16, 8, 128

@@ -1,5 +1,5 @@
 """CPU tests of launch heuristics that are plain host arithmetic (no compute call): the split count of the paged decode
-attention.  The expectations are the measured optima of profiles/r02_decode_split_sweep.jsonl (B200, 148 SMs, two resident
+attention.  The expectations are the measured optima of a sweep over split counts (B200, 148 SMs, two resident
 CTAs per SM): one split once the grid holds a wave; otherwise as many as fill the first wave, never below 256 tokens each."""
 import pytest
 
@@ -8,7 +8,7 @@ import pytest
     (512, 4, 1, 2048, 1),      # Qwen3-8B TP=8 shard: 512 CTAs = 1.73 waves — one split measured 5.94 vs 5.16 TB/s for four
     (512, 8, 2, 2048, 1),      # TP=4 shard
     (512, 32, 8, 2048, 1),     # one GPU
-    (256, 16, 8, 1024, 1),     # configs[1]
+    (256, 16, 8, 1024, 1),     # the decode workload
     (64, 8, 1, 33024, 4),      # Qwen3-32B TP=8, 64 x 32.5K: 4 x 64 = 256 CTAs fill the first wave (measured best)
     (1, 16, 8, 4096, 16),      # one sequence: bounded by 256 tokens per split
     (1, 16, 8, 100, 1),        # short context: nothing to split

@@ -1,6 +1,6 @@
 """CPU tests (no GPU): the C++ host layer behind include/nvllm_engine.h against the Python oracle, BIT-EXACT —
 XXH64 digests, block ids / ref-counts / hashes, free-list order, block tables, slot mappings, context lengths,
-cu_seqlens, prefill/decode order and preemption — every step of randomised and Appendix-B workloads."""
+cu_seqlens, prefill/decode order and preemption — every step of randomised workloads and of two full traces."""
 import json
 import os
 
@@ -143,7 +143,7 @@ def test_config_defaults_and_validate():
 
 
 def test_cfg2_full_size_trace_appendix_b():
-    """BASELINE configs[1] at FULL size through the C++ scheduler: 256 x 512-token prompts,
+    """The plain decode workload at FULL size through the C++ scheduler: 256 x 512-token prompts,
     512 new tokens, block 256 — 4 prefill steps of 64 sequences, seq j owns blocks [2j, 2j+1], takes block 512+j at the
     first decode step and 768+j at length 769; 1024 blocks in total; slot mapping / context lengths follow."""
     rng = np.random.default_rng(1234)
@@ -182,7 +182,7 @@ def test_cfg2_full_size_trace_appendix_b():
 
 
 def test_cfg4_full_size_shared_prefix_trace_appendix_b():
-    """BASELINE configs[3] at FULL size (Appendix B, cfg4): 256 sequences = one shared 4096-token prefix + 256 unique tokens;
+    """The prefix-caching workload at FULL size: 256 sequences = one shared 4096-token prefix + 256 unique tokens;
     17 full blocks each; sequence 0 allocates blocks 0..16, sequence k >= 1 hits blocks 0..15 (ref_count -> k + 1,
     num_cached_tokens = 4096) and misses the 17th (chained hash differs) -> new block 16 + k; 7 sequences per prefill step
     (admission counts the full 4352 tokens), 37 prefill steps, 272 blocks after prefill, + 256 at the first decode step."""
@@ -225,7 +225,7 @@ def test_cfg4_full_size_shared_prefix_trace_appendix_b():
 
 
 def test_max_model_len_is_enforced_at_admission():
-    """nothing bounded prompt + max_tokens by max_model_len (the reference carries the field, config.rs:27,60, and
+    """Nothing else bounds prompt + max_tokens by max_model_len (the reference carries the field, config.rs:27,60, and
     never reads it): a sequence could outgrow the runner's block tables mid-run.  Now the prompt is refused (no state
     change) when it cannot fit, and max_tokens is clamped so the sequence ends with len == max_model_len + 1 at the latest —
     in lockstep with the oracle scheduler given the clamped max_tokens explicitly."""

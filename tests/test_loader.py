@@ -1,4 +1,4 @@
-"""Safetensors loading (SURVEY.md §8f row 1; reference src/utils/loader.rs).  CPU: format round-trip, dtype conversion,
+"""Safetensors loading (reference src/utils/loader.rs).  CPU: format round-trip, dtype conversion,
 packed-module mapping.  GPU: a checkpoint written from the oracle's seeded tensors and loaded through
 nvllm_runner_load_weight produces exactly the logits of the engine's own seeded init (same bytes, same slices)."""
 import numpy as np

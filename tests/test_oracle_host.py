@@ -1,5 +1,5 @@
 """CPU tests: the oracle's integer host layer against every known answer the reference's own unit tests hold for
-this path plus the worked traces of SURVEY.md Appendix B.  These pin the oracle before anything
+this path plus worked traces of two full workloads.  These pin the oracle before anything
 is compared with it."""
 import ctypes
 import json
@@ -250,7 +250,7 @@ def test_block_table_padding_minus_one():
     assert d.block_tables.tolist() == [[3, 9, 2], [7, -1, -1]]
 
 
-# ---------------------------------------------------------------------------- Appendix B traces
+# ---------------------------------------------------------------------------- worked traces
 
 def run_trace(prompts, bs, num_blocks, max_tokens, max_batched=32768, max_seqs=512, token_fn=lambda s, step: 7):
     cfg = H.Config(kvcache_block_size=bs, num_kvcache_blocks=num_blocks, max_num_batched_tokens=max_batched, max_num_seqs=max_seqs)

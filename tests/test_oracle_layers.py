@@ -1,5 +1,5 @@
 """CPU tests pinning the oracle's floating-point layer functions: (i) every formula-level known answer the reference's
-in-file unit tests state (SURVEY.md §8c), (ii) an independent torch-CPU fp32 implementation of the same math, and
+in-file unit tests state, (ii) an independent torch-CPU fp32 implementation of the same math, and
 (iii) the committed golden vectors under tests/golden/ (generator: tests/golden/make_layers_golden.py).
 The reference holds no numeric golden outputs for attention / logits, so (ii)+(iii) are cross-checks, not reference pins."""
 import json

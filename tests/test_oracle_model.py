@@ -1,7 +1,7 @@
 """CPU test: the oracle MODEL (oracle/qwen3.py: paged KV cache, prefill then decode steps driven by the oracle scheduler,
 bf16 rounding at tensor boundaries) against logits of an independent implementation of the named architecture — Hugging
 Face transformers' Qwen3ForCausalLM in fp32 (fixture tests/golden/qwen3_hf.json, generator make_qwen3_hf_golden.py).
-The reference pins none of this (no numeric golden vectors; it lacks q/k-norm and an explicit head_dim, SURVEY.md §8 N1)."""
+The reference pins none of this (no numeric golden vectors; it lacks q/k-norm and an explicit head_dim)."""
 import importlib.util
 import json
 import os
@@ -68,7 +68,7 @@ def test_oracle_model_matches_hf_qwen3_prefill_and_decode(which):
 
 
 def test_wiring_errors_would_be_caught():
-    """Sensitivity of the check above: dropping the q/k-norm (the reference's own wiring, SURVEY.md N1) moves the logits by
+    """Sensitivity of the check above: dropping the q/k-norm (the reference's own wiring) moves the logits by
     far more than the tolerance — the fixture does discriminate between the two architectures."""
     cfg = dict(GOLD["config"], qk_norm=False)
     bs = 16
@@ -81,7 +81,7 @@ def test_wiring_errors_would_be_caught():
 
 
 def test_oracle_prefix_cached_prefill_matches_hf_full_recompute():
-    """SURVEY.md §8 a5 (flash_attention_varlen_with_cache, attention.rs:211-222): the second prompt shares two full blocks
+    """flash_attention_varlen_with_cache (attention.rs:211-222): the second prompt shares two full blocks
     with the first; the scheduler's prefix cache hits them, only the suffix is computed (bottom-right causal mask over the
     paged prefix), and the logits equal HF's full recompute of the whole prompt."""
     cfg = dict(GOLD["config"], qk_norm=True)

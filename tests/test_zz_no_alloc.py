@@ -18,7 +18,7 @@ from tests.util import assert_close, cache_to_layout, make_paged_kv, randn_bf16,
 
 pytestmark = pytest.mark.gpu
 
-# Same attention tolerance as tests/test_gpu_kernels.py (SURVEY.md §8c); the two entry points run the same kernels on
+# Same attention tolerance as tests/test_gpu_kernels.py; the two entry points run the same kernels on
 # the same inputs, so they are in fact expected to agree bit for bit, which is asserted as well.
 ATT_ATOL, ATT_RTOL = 1e-2, 1.6e-2
 

@@ -2,7 +2,7 @@
 
   python tools/bench_decode.py [--batch 256 --ctx 1024 --heads 16 --kv-heads 8 --layout head_major --splits 0]
 
-Algorithmic bytes per launch (SURVEY.md §8d):
+Algorithmic bytes per launch:
   sum_b 2*L_b*Hkv*D*2 + 2*B*H*D*2 + 4*sum_b ceil(L_b/bs) + 4*B      (split-K partials excluded)
 KV (>= 1 GiB at the default shape) is far larger than the 126 MB L2, so every iteration streams from HBM."""
 import argparse

@@ -1,5 +1,5 @@
 """Summarise an `ncu --metrics gpu__time_duration.sum --csv` launch list: launches, total time and share per kernel.
-usage: python tools/summarize_launches.py gpurun_out/launches.csv [header text] > profiles/rNN_launch_summary.txt"""
+usage: python tools/summarize_launches.py launches.csv [header text] > launch_summary.txt"""
 import csv, re, sys
 from collections import defaultdict
 
