@@ -73,7 +73,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
   const uint32_t tmem_slot = bars + (2 * STAGES + 1) * 8;
   uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // (uniform)
   const int rank = static_cast<int>(cluster_ctarank());
   const int tile = static_cast<int>(blockIdx.x) / SK;
   const int m_tile = tile % num_m_tiles, n_tile = tile / num_m_tiles;
@@ -122,8 +122,9 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
       tma_load_2d(sA + stage * C::kABytes, &tmap_x, full_bar(stage), (kb0 + i) * C::BK, m_tile * C::BM);
       if (++stage == STAGES) { stage = 0; phase ^= 1; }
     }
-  } else if (warp == 1 && lane == 0) {
-    // ===== MMA issuer =====
+  } else if (warp == 1) {
+    // ===== MMA issuer: the whole warp walks the k-blocks, one lane issues =====
+    const uint32_t el = elect_one() ? 1u : 0u, tm = __reduce_max_sync(0xffffffffu, tmem_base);   // (read from shared memory: uniform from here on)
     constexpr uint32_t idesc = umma_idesc_bf16(C::BM, BN, 0, 0);
     int stage = 0;
     uint32_t phase = 0;
@@ -134,10 +135,10 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
       const uint32_t a0 = sA + stage * C::kABytes, b0 = sB + stage * C::kBBytes;
 #pragma unroll
       for (int k = 0; k < C::BK / 16; ++k)
-        umma_bf16_ss(tmem_base, umma_desc_sw128(a0 + k * 32, 16, 1024), umma_desc_sw128(b0 + k * 32, 16, 1024), idesc,
-                     (i | k) != 0 ? 1u : 0u);
-      umma_commit(empty_bar(stage));
-      if (i == kb_per - 1) umma_commit(tfull_bar);
+        umma_bf16_ss_warp(tm, umma_desc_lo(a0, 16) + k * 2, umma_desc_lo(b0, 16) + k * 2, idesc,
+                          (i | k) != 0 ? 1u : 0u, el);
+      umma_commit_warp(empty_bar(stage), el);
+      if (i == kb_per - 1) umma_commit_warp(tfull_bar, el);
       if (++stage == STAGES) { stage = 0; phase ^= 1; }
     }
   } else if (warp >= 4) {

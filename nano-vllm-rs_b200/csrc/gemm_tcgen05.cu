@@ -115,7 +115,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
   const uint32_t tmem_slot = bars + (2 * STAGES + 4) * 8;
   uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // (uniform)
   const int lane = threadIdx.x & 31;
   const int num_kb = K / C::BK;
   const int cta0 = static_cast<int>(blockIdx.x), cta_stride = static_cast<int>(gridDim.x);
@@ -187,8 +187,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
       }
       first = false;
     }
-  } else if (warp == 1 && lane == 0) {
-    // ===== MMA issuer (single thread) =====
+  } else if (warp == 1) {
+    // ===== MMA issuer: the whole warp walks the tiles, one lane issues =====
+    const uint32_t el = elect_one() ? 1u : 0u, tm = __reduce_max_sync(0xffffffffu, tmem_base);   // (read from shared memory: uniform from here on)
     constexpr uint32_t idesc = umma_idesc_bf16(C::BM, BN, 0, 0);
     int stage = 0, acc = 0;
     uint32_t phase = 0, acc_phase = 0;
@@ -196,19 +197,19 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     for (int tile = cta0; tile < num_tiles; tile += cta_stride) {
       mbar_wait(tempty_bar(acc), acc_phase ^ 1);  // epilogue has drained this TMEM buffer
       tc_fence_after();
-      const uint32_t tmem_d = tmem_base + acc * BN;
+      const uint32_t tmem_d = tm + acc * BN;
       for (int kb = 0; kb < num_kb; ++kb) {
         mbar_wait(full_bar(stage), phase);
         tc_fence_after();
         const uint32_t a0 = sA + stage * C::kABytes, b0 = sB + stage * C::kBBytes;
 #pragma unroll
         for (int k = 0; k < C::BK / 16; ++k) {
-          const uint64_t adesc = umma_desc_sw128(a0 + k * 32, 16, 1024);
-          const uint64_t bdesc = umma_desc_sw128(b0 + k * 32, 16, 1024);
-          umma_bf16_ss(tmem_d, adesc, bdesc, idesc, (kb | k) != 0 ? 1u : 0u);
+          const uint32_t adesc = umma_desc_lo(a0, 16) + k * 2;
+          const uint32_t bdesc = umma_desc_lo(b0, 16) + k * 2;
+          umma_bf16_ss_warp(tmem_d, adesc, bdesc, idesc, (kb | k) != 0 ? 1u : 0u, el);
         }
-        umma_commit(empty_bar(stage));                      // smem stage reusable once these MMAs retire
-        if (kb == num_kb - 1) umma_commit(tfull_bar(acc));  // accumulator complete
+        umma_commit_warp(empty_bar(stage), el);                      // smem stage reusable once these MMAs retire
+        if (kb == num_kb - 1) umma_commit_warp(tfull_bar(acc), el);  // accumulator complete
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }

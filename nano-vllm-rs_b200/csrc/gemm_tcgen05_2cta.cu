@@ -78,7 +78,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
   const uint32_t tmem_slot = bars + (2 * STAGES + 4) * 8;
   uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // (uniform)
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
   const int num_kb = K / C::BK;
@@ -122,8 +122,9 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
-  } else if (warp == 1 && lane == 0 && leader) {
-    // ===== MMA issuer (leader CTA, single thread) =====
+  } else if (warp == 1 && leader) {
+    // ===== MMA issuer (leader CTA): the whole warp walks the tiles, one lane issues =====
+    const uint32_t el = elect_one() ? 1u : 0u, tm = __reduce_max_sync(0xffffffffu, tmem_base);   // (read from shared memory: uniform from here on)
     constexpr uint32_t idesc = umma_idesc_bf16(C::BM, BN, 0, 0);
     int stage = 0, acc = 0;
     uint32_t phase = 0, acc_phase = 0;
@@ -131,19 +132,19 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
     for (int tile = cluster_id; tile < num_tiles; tile += num_clusters) {
       mbar_wait(tempty_bar(acc), acc_phase ^ 1);
       tc_fence_after();
-      const uint32_t tmem_d = tmem_base + acc * BN;
+      const uint32_t tmem_d = tm + acc * BN;
       for (int kb = 0; kb < num_kb; ++kb) {
         mbar_wait(full_bar(stage), phase);
         tc_fence_after();
         const uint32_t a0 = sA + stage * C::kABytes, b0 = sB + stage * C::kBBytes;
 #pragma unroll
         for (int k = 0; k < C::BK / 16; ++k) {
-          const uint64_t adesc = umma_desc_sw128(a0 + k * 32, 16, 1024);
-          const uint64_t bdesc = umma_desc_sw128(b0 + k * 32, 16, 1024);
-          umma_bf16_ss_cg2(tmem_d, adesc, bdesc, idesc, (kb | k) != 0 ? 1u : 0u);
+          const uint32_t adesc = umma_desc_lo(a0, 16) + k * 2;
+          const uint32_t bdesc = umma_desc_lo(b0, 16) + k * 2;
+          umma_bf16_ss_cg2_warp(tmem_d, adesc, bdesc, idesc, (kb | k) != 0 ? 1u : 0u, el);
         }
-        umma_commit_cg2(empty_bar(stage), 0b11);
-        if (kb == num_kb - 1) umma_commit_cg2(tfull_bar(acc), 0b11);
+        umma_commit_cg2_warp(empty_bar(stage), 0b11, el);
+        if (kb == num_kb - 1) umma_commit_cg2_warp(tfull_bar(acc), 0b11, el);
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }

@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_attn_tc_kernel(const __gri
   auto p_ready = [&](int b) { return bars + (6 + b) * 8; };   // 128 arrivals: P is in TMEM (and O rescaled where it had to be)
   const uint32_t o_done = bars + 8 * 8;
   const uint32_t tmem_slot = bars + 9 * 8;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;   // (warp: uniform)
   const int tile0 = tile * kLatentTileTokens, tend = min(a.n, tile0 + kLatentTileTokens);
   const int hbase = blockIdx.y * kHeads;
   const int half0 = halves == 2 ? 0 : static_cast<int>(blockIdx.z);   // this CTA's halves of the latent values: half0 .. half0 + halves - 1
@@ -243,24 +243,28 @@ __global__ void __launch_bounds__(kThreads, 1) latent_attn_tc_kernel(const __gri
       t = s.t1;
     }
   } else if (warp == 8) {
-    if (lane == 0) {
+    {   // the whole warp walks the tiles, one lane issues
+      const uint32_t el = elect_one() ? 1u : 0u;
+      auto uni = [](uint32_t v) { return __reduce_max_sync(0xffffffffu, v); };   // a value that is uniform for the compiler too
+      auto test = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_test_wait(bar, parity)) != 0; };
+      const uint32_t tm = uni(tmem);
       constexpr uint32_t idesc_s = umma_idesc_bf16(kRows, kKeys, 0, 0), idesc_o = umma_idesc_bf16(kRows, kHalf, 0, 1);
       const int rot_steps = (a.rot_dim + 15) / 16;
       auto issue_s = [&](int it) {   // S_it = Q . K_it^T
         const int b = it & 1;
-        const uint32_t k0 = sK + b * kTileBytes, d = tmem + kColS + b * kKeys;
+        const uint32_t k0 = sK + b * kTileBytes, d = tm + kColS + b * kKeys;
         tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < kQTmem / 16; ++ks)
-          umma_bf16_ts(d, tmem + kColQ + ks * 8, umma_desc_sw128(k0 + (ks >> 2) * kKChunkBytes + (ks & 3) * 32, 16, 1024), idesc_s, ks != 0);
+          umma_bf16_ts_warp(d, tm + kColQ + ks * 8, umma_desc_lo(k0, 16) + (((ks >> 2) * kKChunkBytes + (ks & 3) * 32) >> 4), idesc_s, ks != 0, el);
 #pragma unroll
         for (int ks = 0; ks < (kRank - kQTmem) / 16; ++ks)
-          umma_bf16_ss(d, umma_desc_sw128(sQ + (ks >> 2) * kQChunkBytes + (ks & 3) * 32, 16, 1024),
-                       umma_desc_sw128(k0 + (kQTmem / 64 + (ks >> 2)) * kKChunkBytes + (ks & 3) * 32, 16, 1024), idesc_s, 1);
+          umma_bf16_ss_warp(d, umma_desc_lo(sQ, 16) + (((ks >> 2) * kQChunkBytes + (ks & 3) * 32) >> 4),
+                       umma_desc_lo(k0, 16) + (((kQTmem / 64 + (ks >> 2)) * kKChunkBytes + (ks & 3) * 32) >> 4), idesc_s, 1, el);
         for (int ks = 0; ks < rot_steps; ++ks)
-          umma_bf16_ss(d, umma_desc_sw128(sQ + (kQChunks - 1) * kQChunkBytes + ks * 32, 16, 1024),
-                       umma_desc_sw128(k0 + (kChunks - 1) * kKChunkBytes + ks * 32, 16, 1024), idesc_s, 1);
-        umma_commit(s_full(b));
+          umma_bf16_ss_warp(d, umma_desc_lo(sQ, 16) + (((kQChunks - 1) * kQChunkBytes + ks * 32) >> 4),
+                       umma_desc_lo(k0, 16) + (((kChunks - 1) * kKChunkBytes + ks * 32) >> 4), idesc_s, 1, el);
+        umma_commit_warp(s_full(b), el);
       };
       auto issue_pv = [&](int it, int half, bool first) {   // O (+)= P_it . C_it
         const int b = it & 1;
@@ -268,16 +272,16 @@ __global__ void __launch_bounds__(kThreads, 1) latent_attn_tc_kernel(const __gri
         tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < kKeys / 16; ++ks)
-          umma_bf16_ts(tmem + kColO, tmem + kColS + b * kKeys + ks * 8, umma_desc_sw128(v0 + ks * 2048, kKChunkBytes, 1024), idesc_o, !first || ks != 0);
-        umma_commit(o_done);
-        umma_commit(k_empty(b));
+          umma_bf16_ts_warp(tm + kColO, tm + kColS + b * kKeys + ks * 8, umma_desc_lo(v0, kKChunkBytes) + ((ks * 2048) >> 4), idesc_o, !first || ks != 0, el);
+        umma_commit_warp(o_done, el);
+        umma_commit_warp(k_empty(b), el);
       };
       // The key tiles of the two spans (the second may be empty), each walked once per half of the values.
       int tiles[2] = {0, 0}, ns = 0;
       for (int t = tile0; t < tend; ++ns) {
         const Span s = span_of(a, t, tend);
-        tiles[ns] = (s.nkeys - s.jstart + kKeys - 1) / kKeys;
-        t = s.t1;
+        tiles[ns] = static_cast<int>(uni((s.nkeys - s.jstart + kKeys - 1) / kKeys));
+        t = static_cast<int>(uni(s.t1));
       }
       const int total = halves * (tiles[0] + tiles[1]);
       // S of the next tile goes first when its keys are there (it runs while this tile's softmax does), PV of this tile otherwise.
@@ -285,9 +289,9 @@ __global__ void __launch_bounds__(kThreads, 1) latent_attn_tc_kernel(const __gri
       int js = 0, jp = 0;
       long long t0 = clock64();
       while (jp < total) {
-        if (js < total && js <= jp + 1 && mbar_test_wait(k_full(js & 1), (js >> 1) & 1)) {
+        if (js < total && js <= jp + 1 && test(k_full(js & 1), (js >> 1) & 1)) {
           issue_s(js++);
-        } else if (jp < js && mbar_test_wait(p_ready(jp & 1), (jp >> 1) & 1)) {
+        } else if (jp < js && test(p_ready(jp & 1), (jp >> 1) & 1)) {
           const int in1 = jp - halves * tiles[0], span_tiles = in1 < 0 ? tiles[0] : tiles[1], in = in1 < 0 ? jp : in1;
           issue_pv(jp, half0 + in / span_tiles, in % span_tiles == 0);
           ++jp;
