@@ -75,24 +75,8 @@ __device__ __forceinline__ void store_row32<float>(float* dst, const uint32_t (&
 
 // GATE != kGateNone: w = [gate (N rows) | up (N rows)]; the B tile is staged as BN/2 gate rows + the matching BN/2 up rows and
 // the epilogue writes y[:, n_tile*BN/2 + c] = silu(gate) * up, or another gate of gated_pair (see gemm_tcgen05_2cta.cu for the CTA-pair variant).
-// Optional qkv epilogue (ROPE mode, BN == 128 == head_dim): each output tile is one head of the packed [q | k | v] row,
-// and each epilogue thread owns that head for one token.  It applies what Qwen3Attention::forward does between qkv_proj
-// and Attention::forward (qwen3.rs:219-229) plus Attention::store_kv_cache (attention.rs:150-174): round to bf16 (the
-// qkv tensor), per-head RMSNorm (q/k), bf16, half-split RoPE from the f32 table, bf16; q/k/v rows go to the qkv buffer
-// and k/v additionally into the paged cache at slot_mapping[token] — same rounding points as the stand-alone kernel.
-struct RopeEpi {
-  const int64_t* positions;
-  const float* cos_sin;     // [max_position, 128]
-  const bf16* q_norm_w;     // may be NULL (no qk-norm)
-  const bf16* k_norm_w;
-  bf16* k_cache;
-  bf16* v_cache;
-  const int32_t* slot_mapping;
-  int H, Hkv, max_position, block_size;
-  int64_t blk_stride, tok_stride, head_stride;
-  float eps;
-};
-
+// ROPE mode (BN == 128 == head_dim): the qkv epilogue that RopeEpi describes; each output tile is one head of the packed [q | k | v]
+// row, and each epilogue thread owns that head for one token.
 template <int BN, typename OutT, int GATE, bool ROPE = false>
 __global__ void __launch_bounds__(256, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
@@ -406,6 +390,8 @@ static int pick_bn(int M, int N) {
 int gemm_2cta_dispatch(void* y, const void* x, const void* w, int m, int n, int k, int64_t ldx, int64_t ldw,
                        int64_t ldy, int out_dtype, cudaStream_t st);  // gemm_tcgen05_2cta.cu
 
+int gemm_qkv_2cta_dispatch(void* qkv, const void* x, const void* w, int m, int n, int k, int64_t ldx, int64_t ldw, const RopeEpi& re,
+                           cudaStream_t st);  // gemm_tcgen05_2cta.cu
 int gemm_silu_2cta_dispatch(void* y, const void* x, const void* w, int m, int inter, int k, int64_t ldx, int64_t ldw,
                             int64_t ldy, int gate, float glu_limit, cudaStream_t st);  // gemm_tcgen05_2cta.cu
 
@@ -633,6 +619,8 @@ extern "C" int nvllm_gemm_qkv_rope_store(void* qkv, const void* x, const void* w
     re.head_stride = layout->head_stride;
   }
   const int n = (num_heads + 2 * num_kv_heads) * 128;
+  if (want_2cta(m, n, k) && n % 256 == 0 && aligned16(cos_sin) && aligned16(q_norm_w) && aligned16(k_norm_w) && aligned16(k_cache) && aligned16(v_cache))
+    return gemm_qkv_2cta_dispatch(qkv, x, w_qkv, m, n, k, ldx, ldw, re, static_cast<cudaStream_t>(stream));
   CUtensorMap tx, tw;
   if (int rc = make_tmap_bf16_2d(&tx, x, m, k, ldx, 128)) return rc;
   if (int rc = make_tmap_bf16_2d(&tw, w_qkv, n, k, ldw, 128)) return rc;

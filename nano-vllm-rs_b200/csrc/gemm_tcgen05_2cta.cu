@@ -18,10 +18,12 @@
 
 namespace nvllm {
 
-template <int GATE>
-constexpr int gemm2_epilogue_warps() { return GATE != kGateNone ? 8 : 4; }
-template <int GATE>
-constexpr int gemm2_threads() { return 128 + 32 * gemm2_epilogue_warps<GATE>(); }
+template <int GATE, bool ROPE = false>
+constexpr int gemm2_epilogue_warps() { return GATE != kGateNone || ROPE ? 8 : 4; }
+template <int GATE, bool ROPE = false>
+constexpr int gemm2_threads() { return 128 + 32 * gemm2_epilogue_warps<GATE, ROPE>(); }
+
+constexpr int kRopeStage = 2 * 16 * 256;   // bytes of shared memory of an epilogue warp of the qkv form
 
 template <int BN>
 struct Gemm2Cfg {
@@ -56,21 +58,120 @@ __device__ __forceinline__ void store_row32_2(OutT* dst, const uint32_t (&r)[32]
   }
 }
 
+// The qkv epilogue of a warp: 16 tokens (from row0 on) of the tile's two heads.  In the accumulator's layout (a lane per token) it is bound
+// by the LSU: angles and rows are then 16-byte accesses to 32 different lines each (13.4 K tokens x 4096 x 1024: 168 us, against 96 + 67 for
+// the projection and a pass of its own; as here 113; 8192 x 6144 x 4096: 315 against 315 + 69).  So the tokens go through shared memory (per head 16 rows of 256 bytes; the 16-byte piece c of row r
+// lies at c ^ (r & 7)) and come back with 8 lanes a token, 8 neighbouring values of each half of the head a lane: a rotation
+// then needs no other lane, and every access covers whole lines.  The angles serve both heads (the table does not fit the L1 that the
+// operand ring leaves, and L2 -> SM is what binds the GEMM) and are requested before the accumulator is ready.
+struct RopeAngles { float4 c[4][2], s[4][2]; int slot; };
+
+__device__ __forceinline__ void rope_angles(RopeAngles& an, const RopeEpi& re, int row0, int M, bool rotate) {
+  const int lane = threadIdx.x & 31, row = row0 + (lane & 15);
+  int64_t pos = row < M ? re.positions[row] : 0;
+  pos = pos < 0 ? 0 : (pos >= re.max_position ? re.max_position - 1 : pos);
+  an.slot = row < M && re.k_cache != nullptr ? __ldg(re.slot_mapping + row) : -1;
+  if (!rotate) return;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int64_t p = __shfl_sync(0xffffffffu, static_cast<int>(pos), 4 * i + (lane >> 3));
+    const float4* cs = reinterpret_cast<const float4*>(re.cos_sin + p * 128) + 2 * (lane & 7);
+    an.c[i][0] = __ldg(cs); an.c[i][1] = __ldg(cs + 1); an.s[i][0] = __ldg(cs + 16); an.s[i][1] = __ldg(cs + 17);
+  }
+}
+__device__ __forceinline__ void rope_rows(bf16* __restrict__ y, int64_t ldy, const RopeEpi& re, const RopeAngles& an, uint32_t taddr, uint8_t* stage,
+                                          int row0, int M, int head0, int half) {
+  const int lane = threadIdx.x & 31, l = lane & 15, j = lane & 7;
+#pragma unroll 1
+  for (int c = 0; c < 8; ++c) {      // 32 columns at a time; the warp's tokens are the lanes of its half
+    uint32_t r[32];
+    tmem_ld_32x32b_x32(taddr + c * 32, r);
+    tmem_ld_wait();
+    if ((lane >> 4) == half) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)    // bf16 qkv
+        *reinterpret_cast<uint4*>(stage + (c >> 2) * 4096 + l * 256 + ((((c & 3) * 4 + e) ^ (l & 7)) * 16)) =
+            make_uint4(pack_bf16x2(__uint_as_float(r[8 * e]), __uint_as_float(r[8 * e + 1])), pack_bf16x2(__uint_as_float(r[8 * e + 2]), __uint_as_float(r[8 * e + 3])),
+                       pack_bf16x2(__uint_as_float(r[8 * e + 4]), __uint_as_float(r[8 * e + 5])), pack_bf16x2(__uint_as_float(r[8 * e + 6]), __uint_as_float(r[8 * e + 7])));
+    }
+  }
+  __syncwarp();
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {
+    const int head = head0 + h;                                               // packed row: H q heads, Hkv k heads, Hkv v heads
+    const int kind = head < re.H ? 0 : (head < re.H + re.Hkv ? 1 : 2);
+    const bf16* w = kind == 0 ? re.q_norm_w : (kind == 1 ? re.k_norm_w : nullptr);
+    bf16* const cache = kind == 1 ? re.k_cache + (head - re.H) * re.head_stride : re.v_cache + (head - re.H - re.Hkv) * re.head_stride;
+    uint4 wa = make_uint4(0, 0, 0, 0), wb = wa;
+    if (w != nullptr) { wa = __ldg(reinterpret_cast<const uint4*>(w) + j); wb = __ldg(reinterpret_cast<const uint4*>(w) + 8 + j); }
+    const uint32_t w1[4] = {wa.x, wa.y, wa.z, wa.w}, w2[4] = {wb.x, wb.y, wb.z, wb.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int rr = 4 * i + (lane >> 3), row = row0 + rr;
+      const uint8_t* src = stage + h * 4096 + rr * 256;
+      const uint4 a4 = *reinterpret_cast<const uint4*>(src + ((j ^ (rr & 7)) * 16)), b4 = *reinterpret_cast<const uint4*>(src + (((8 + j) ^ (rr & 7)) * 16));
+      uint32_t a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
+      const int slot = __shfl_sync(0xffffffffu, an.slot, rr);
+      if (kind < 2) {
+        if (w != nullptr) {
+          float ss[2] = {0.f, 0.f};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            ss[0] = fmaf(bf16_lo(a[e]), bf16_lo(a[e]), fmaf(bf16_hi(a[e]), bf16_hi(a[e]), ss[0]));
+            ss[1] = fmaf(bf16_lo(b[e]), bf16_lo(b[e]), fmaf(bf16_hi(b[e]), bf16_hi(b[e]), ss[1]));
+          }
+          float t = ss[0] + ss[1];
+#pragma unroll
+          for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+          const float inv = 1.0f / sqrtf(t * (1.0f / 128.0f) + re.eps);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            a[e] = pack_bf16x2(bf16_lo(a[e]) * inv * bf16_lo(w1[e]), bf16_hi(a[e]) * inv * bf16_hi(w1[e]));
+            b[e] = pack_bf16x2(bf16_lo(b[e]) * inv * bf16_lo(w2[e]), bf16_hi(b[e]) * inv * bf16_hi(w2[e]));
+          }
+        }
+        const float c[8] = {an.c[i][0].x, an.c[i][0].y, an.c[i][0].z, an.c[i][0].w, an.c[i][1].x, an.c[i][1].y, an.c[i][1].z, an.c[i][1].w};
+        const float s[8] = {an.s[i][0].x, an.s[i][0].y, an.s[i][0].z, an.s[i][0].w, an.s[i][1].x, an.s[i][1].y, an.s[i][1].z, an.s[i][1].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float x0 = bf16_lo(a[e]), x1 = bf16_hi(a[e]), z0 = bf16_lo(b[e]), z1 = bf16_hi(b[e]);
+          a[e] = pack_bf16x2(x0 * c[2 * e] - z0 * s[2 * e], x1 * c[2 * e + 1] - z1 * s[2 * e + 1]);
+          b[e] = pack_bf16x2(z0 * c[2 * e] + x0 * s[2 * e], z1 * c[2 * e + 1] + x1 * s[2 * e + 1]);
+        }
+      }
+      if (row < M) {
+        auto store = [&](bf16* dst) {
+          reinterpret_cast<uint4*>(dst)[j] = make_uint4(a[0], a[1], a[2], a[3]);
+          reinterpret_cast<uint4*>(dst)[8 + j] = make_uint4(b[0], b[1], b[2], b[3]);
+        };
+        store(y + row * ldy + head * 128);
+        if (kind >= 1 && slot >= 0) {
+          const int blk = slot / re.block_size;
+          store(cache + blk * re.blk_stride + (slot - blk * re.block_size) * re.tok_stride);
+        }
+      }
+    }
+  }
+  __syncwarp();
+}
+
 // GATE != kGateNone: w is the packed [gate (N rows) | up (N rows)] matrix of MergedColumnParallelLinear (linear.rs:421-433);
 // the leader CTA stages BN/2 gate rows, its peer the matching BN/2 up rows, so accumulator columns [0, BN/2) are gate and
 // [BN/2, BN) are up for the same BN/2 output features, and the epilogue writes y[:, n_tile*BN/2 + c] = silu(gate)*up
 // (SiluAndMul::forward, activation.rs:46-63; or another gate of gated_pair) without the [M, 2N] intermediate ever reaching HBM.  N = output features.
-template <int BN, typename OutT, int GATE>
-__global__ void __launch_bounds__(gemm2_threads<GATE>(), 1)
+// ROPE: the qkv epilogue that RopeEpi describes, on the two heads of a tile; see rope_rows.
+template <int BN, typename OutT, int GATE, bool ROPE>
+__global__ void __launch_bounds__(gemm2_threads<GATE, ROPE>(), 1)
 gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
-                         OutT* __restrict__ y, int M, int N, int K, int64_t ldy, int num_m_tiles, int num_tiles, float glu_limit) {
+                         OutT* __restrict__ y, int M, int N, int K, int64_t ldy, int num_m_tiles, int num_tiles, float glu_limit,
+                         const RopeEpi re) {
   using C = Gemm2Cfg<BN>;
-  constexpr int STAGES = C::kStages;
+  constexpr int STAGES = C::kStages - (ROPE ? 1 : 0);   // (the qkv epilogue takes a stage's room)
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t sA = smem_base;
   const uint32_t sB = smem_base + STAGES * C::kABytes;
-  const uint32_t bars = smem_base + STAGES * C::kStageBytes;
+  const uint32_t bars = smem_base + STAGES * C::kStageBytes + (ROPE ? 8 * kRopeStage : 0);
   auto full_bar = [&](int s) { return bars + s * 8; };
   auto empty_bar = [&](int s) { return bars + (STAGES + s) * 8; };
   auto tfull_bar = [&](int a) { return bars + (2 * STAGES + a) * 8; };
@@ -96,7 +197,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tfull_bar(a), 1);     // each CTA: multicast commit
-      mbar_init(tempty_bar(a), 64 * gemm2_epilogue_warps<GATE>());  // leader: the epilogue threads of both CTAs
+      mbar_init(tempty_bar(a), 64 * gemm2_epilogue_warps<GATE, ROPE>());  // leader: the epilogue threads of both CTAs
     }
     fence_barrier_init();
   }
@@ -157,11 +258,20 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
     uint32_t acc_phase = 0;
     for (int tile = cluster_id; tile < num_tiles; tile += num_clusters) {
       const int m_tile = tile % num_m_tiles, n_tile = tile / num_m_tiles;
+      [[maybe_unused]] RopeAngles angles;
+      [[maybe_unused]] const int rope_row0 = m_tile * C::BM + static_cast<int>(rank) * C::BM_CTA + q * 32 + (warp < 8 ? 0 : 16);
+      if constexpr (ROPE) {
+        static_assert(!ROPE || BN == 256, "two heads a tile");
+        rope_angles(angles, re, rope_row0, M, n_tile * 2 < re.H + re.Hkv);
+      }
       mbar_wait(tfull_bar(acc), acc_phase);
       tc_fence_after();
       const int row = m_tile * C::BM + rank * C::BM_CTA + q * 32 + lane;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
-      if constexpr (GATE != kGateNone) {
+      if constexpr (ROPE) {
+        rope_rows(y, ldy, re, angles, taddr, smem_raw + (smem_base - smem_u32(smem_raw)) + STAGES * C::kStageBytes + (warp - 4) * kRopeStage, rope_row0, M,
+                  n_tile * 2, warp < 8 ? 0 : 1);
+      } else if constexpr (GATE != kGateNone) {
 #pragma unroll 1
         for (int c = warp < 8 ? 0 : BN / 128; c < (warp < 8 ? BN / 128 : BN / 64); ++c) {
           uint32_t g[32], u[32];
@@ -204,12 +314,13 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
   }
 }
 
-template <int BN, typename OutT, int GATE = kGateNone>
+template <int BN, typename OutT, int GATE = kGateNone, bool ROPE = false>
 static int launch_gemm2(const CUtensorMap& tx, const CUtensorMap& tw, void* y, int M, int N, int K, int64_t ldy,
-                        cudaStream_t st, float glu_limit = 0.f) {
+                        cudaStream_t st, float glu_limit = 0.f, const RopeEpi& re = RopeEpi{}) {
   using C = Gemm2Cfg<BN>;
-  auto kern = gemm_tcgen05_2cta_kernel<BN, OutT, GATE>;
-  NVLLM_SMEM_ATTR_ONCE(kern, C::kSmemBytes);
+  auto kern = gemm_tcgen05_2cta_kernel<BN, OutT, GATE, ROPE>;
+  constexpr int smem = C::kSmemBytes + (ROPE ? 8 * kRopeStage - C::kStageBytes : 0);
+  NVLLM_SMEM_ATTR_ONCE(kern, smem);
   const int num_m_tiles = (M + C::BM - 1) / C::BM;
   const int num_n_tiles = GATE != kGateNone ? (N + BN / 2 - 1) / (BN / 2) : (N + BN - 1) / BN;
   const int num_tiles = num_m_tiles * num_n_tiles;
@@ -217,8 +328,8 @@ static int launch_gemm2(const CUtensorMap& tx, const CUtensorMap& tw, void* y, i
   const int clusters = num_tiles < max_clusters ? num_tiles : max_clusters;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(2 * clusters);
-  cfg.blockDim = dim3(gemm2_threads<GATE>());
-  cfg.dynamicSmemBytes = C::kSmemBytes;
+  cfg.blockDim = dim3(gemm2_threads<GATE, ROPE>());
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -227,7 +338,7 @@ static int launch_gemm2(const CUtensorMap& tx, const CUtensorMap& tw, void* y, i
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  NVLLM_CUDA(cudaLaunchKernelEx(&cfg, kern, tx, tw, static_cast<OutT*>(y), M, N, K, ldy, num_m_tiles, num_tiles, glu_limit));
+  NVLLM_CUDA(cudaLaunchKernelEx(&cfg, kern, tx, tw, static_cast<OutT*>(y), M, N, K, ldy, num_m_tiles, num_tiles, glu_limit, re));
   return 0;
 }
 
@@ -270,6 +381,14 @@ int gemm_2cta_dispatch(void* y, const void* x, const void* w, int m, int n, int 
       NVLLM_G2(64);
   }
 #undef NVLLM_G2
+}
+
+// qkv = x . Wqkv^T with the qkv epilogue; n = 128 x heads, a multiple of 256.
+int gemm_qkv_2cta_dispatch(void* qkv, const void* x, const void* w, int m, int n, int k, int64_t ldx, int64_t ldw, const RopeEpi& re, cudaStream_t st) {
+  CUtensorMap tx, tw;
+  if (int rc = make_tmap_bf16_2d(&tx, x, m, k, ldx, 128)) return rc;
+  if (int rc = make_tmap_bf16_2d(&tw, w, n, k, ldw, 128)) return rc;
+  return launch_gemm2<256, bf16, kGateNone, true>(tx, tw, qkv, m, n, k, n, st, 0.f, re);
 }
 
 // y[M, inter] = silu(x . Wgate^T) * (x . Wup^T) (or another gate) with w = [Wgate | Wup] packed row-wise ([2*inter, K]).

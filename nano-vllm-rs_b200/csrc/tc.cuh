@@ -17,6 +17,25 @@ int make_tmap_bf16_2d(CUtensorMap* map, const void* base, int64_t rows, int64_t 
 int make_tmap_bf16_nd(CUtensorMap* map, const void* base, int rank, const uint64_t* dims,
                       const uint64_t* strides_bytes, const uint32_t* box);  // tc_host.cu
 
+// ---- qkv epilogue of the GEMMs ---------------------------------------------------------------------
+// What Qwen3Attention::forward does between qkv_proj and Attention::forward (qwen3.rs:219-229) plus Attention::store_kv_cache
+// (attention.rs:150-174), on the accumulators of x . Wqkv^T: round to bf16 (the qkv tensor), per-head RMSNorm (q/k), bf16, half-split
+// RoPE from the f32 table, bf16; q/k/v rows go to the qkv buffer and k/v additionally into the paged cache at slot_mapping[token] —
+// same rounding points as the stand-alone kernel.
+struct RopeEpi {
+  const int64_t* positions;
+  const float* cos_sin;     // [max_position, 128]
+  const bf16* q_norm_w;     // may be NULL (no qk-norm)
+  const bf16* k_norm_w;
+  bf16* k_cache;
+  bf16* v_cache;
+  const int32_t* slot_mapping;
+  int H, Hkv, max_position, block_size;
+  int64_t blk_stride, tok_stride, head_stride;
+  float eps;
+};
+
+
 #ifdef __CUDACC__
 
 // ---- mbarrier ------------------------------------------------------------------------------------

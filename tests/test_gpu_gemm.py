@@ -125,7 +125,8 @@ def test_gemm_192_wide_tiles(cuda, m, n, k, silu, monkeypatch):
 
 
 @pytest.mark.parametrize("kind", ["reference", "head_major"])
-@pytest.mark.parametrize("m,H,Hkv,k,qknorm", [(256, 16, 8, 1024, True), (37, 4, 1, 512, True), (130, 8, 2, 256, False)])
+@pytest.mark.parametrize("m,H,Hkv,k,qknorm", [(256, 16, 8, 1024, True), (37, 4, 1, 512, True), (130, 8, 2, 256, False),
+                                                  (700, 16, 8, 1024, True), (1300, 16, 8, 512, True), (513, 4, 2, 256, False)])   # CTA pairs
 def test_gemm_qkv_rope_store_fused_equals_unfused(cuda, kind, m, H, Hkv, k, qknorm, monkeypatch):
     """qkv GEMM with the q/k-norm + RoPE + KV-store epilogue vs nvllm_gemm_bf16 followed by nvllm_qknorm_rope_store
     (same rounding points; split-K off so that both GEMMs sum in the same order), for both cache layouts."""
