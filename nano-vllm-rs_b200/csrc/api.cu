@@ -49,7 +49,6 @@ static void parse_knobs() {
     else if (sscanf(e, "%d,%d", &bn, &sk) == 2) { k.splitk_mode = 2; k.splitk_bn = bn; k.splitk_sk = sk; }
   }
   k.decode_cfg = num("NVLLM_DECODE_CFG", 0);
-  k.prefill_poly = num("NVLLM_PREFILL_POLY", 4);
   k.fuse_rope = num("NVLLM_FUSE_ROPE", 0) == 1;
   k.fuse_decode = num("NVLLM_FUSE_DECODE", 0);
   k.fused_tp = num("NVLLM_FUSED_TP", 1);

@@ -4,20 +4,34 @@
 // 321-339: per-sequence loop, O(L^2) host-built mask, dense matmul) and flash_attention_varlen_with_cache
 // (:211-222, prefill of the uncached suffix against the paged prefix).
 //
-// One CTA = 256 query rows of one (sequence, head): two row groups (RG) of 128 threads, one query row per thread
-// (== one TMEM lane), sharing the K/V tiles of the KV head; KV tiles of 128 keys.
-//   warp 8 (one lane)   TMA producer: Q once (2 x 128 x 128), then K_0, V_0, K_1, V_1, ... through a ring of NSLOT
-//                       32 KiB slots; dense K/V via a 2-D map, paged K/V via a 4-D map (d, token, head, block) + block_tables
-//   warp 9 (one lane)   MMA issuer for both groups: S = Q . K^T (8 x tcgen05.mma M128 N128 K16, both operands K-major in
-//                       shared memory) and O += P . V (8 x tcgen05.mma with A = P read from TENSOR MEMORY, V MN-major)
-//   RG threads          tcgen05.ld S row -> row max -> exp2 (3/4 on MUFU, 1/4 by an XU-free polynomial on the FMA pipe) ->
-//                       P as packed bf16 written BACK INTO TMEM over the S columns (tcgen05.st; each thread only touches its
-//                       own lane, so no cross-thread hazard) -> mbarrier arrive.  No shared-memory round trip for P.
-//                       O accumulates in TMEM across tiles; the reference maximum is refreshed lazily (only when a tile
-//                       exceeds it by 2^8), and only then is O read, scaled and written back.
-// While one group runs its softmax the tensor core executes the other group's MMAs.
-// TMEM: 512 columns = 2 RG x (S/P 128 + O 128).  Causal mask is bottom-right aligned (row r of Lq sees keys <= Lk - Lq + r)
-// so the same kernel serves Lq == Lk and suffix-over-prefix.  CTAs are ordered longest-first.
+// One work item = two row groups (RG) of 128 threads, one query row per thread (== one TMEM lane), that share the K/V tiles
+// (64 keys) of a KV head: the same 128 rows of two of its query heads where the heads pair up (both groups then end at the
+// same tile and a block of rows reads half the keys of its diagonal), else 256 rows of one head.
+// CTAs stay: each starts with its own block index and takes further ones from the grid's not yet started CTAs
+// (clusterlaunchcontrol), so that the loads and the first S of the next item run under the last softmax and the output of
+// this one, and barriers, TMEM and the launch are paid once.
+//   warp 8              TMA producer: per item K_0, Q (2 x 128 x 128), V_0, K_1, V_1, ... through a ring of NSLOT 16 KiB slots.  Maps see a
+//                       head's 128 values as two halves of 64 (128 bytes each): one copy brings a tile, [half][row][64] in shared memory;
+//                       dense K/V (64, token, half), paged K/V (64, token, half, head, block) + block_tables
+//   warps 9, 11         MMAs of group 0, 1: S = Q . K^T (8 x tcgen05.mma M128 N64 K16, both operands K-major in shared memory) and
+//                       O += P . V (4 x M128 N128 K16 with A = P read from TENSOR MEMORY, V MN-major).  Warps 8, 9 and 11 stay converged, one
+//                       elected lane issues: a diverged one takes over 100 clocks for every copy or MMA, and a converged one 50 to 76
+//                       where the pipe takes 48, hence a warp for each group.
+//   warp 10 (one lane)  claims the next item while this one is worked on
+//   RG threads          tcgen05.ld S row -> row max -> exp2 (MUFU) -> P as packed bf16 written BACK INTO TMEM over the S columns
+//                       (tcgen05.st; each thread only touches its own lane, so no cross-thread hazard) -> mbarrier arrive -> row sum.
+//                       O accumulates in TMEM across tiles; the reference maximum is refreshed lazily (only when a tile exceeds it
+//                       by 2^8), and only then is O read, scaled and written back.
+// Each group has two S buffers: S of tile j + 2 follows P.V of tile j, so a group's softmax finds its next S ready and waits for no MMA;
+// with one buffer of 128 keys every tile waited 850 of 3870 clocks for P.V and S of its own.
+// TMEM: 512 columns = 2 RG x (2 x S/P 64 + O 128).  Causal mask is bottom-right aligned (row r of Lq sees keys <= Lk - Lq + r)
+// so the same kernel serves Lq == Lk and suffix-over-prefix.  Items are ordered by their distance from the last rows of their
+// sequence: longest first within a sequence, and the empty ones of short sequences at the end.
+// Bound by the exponentials and the MMAs' issue side by side.  Measured, against one CTA per 256 rows with 128-key tiles and diverged issuing
+// lanes (us): 24 prompts of up to 1021 tokens, 16/8 heads 128 and 80; 64 x 512 213 and 131; 2 x 4096, 32/8 heads 354 and 246; 16384 tokens 1140
+// and 877 (1.25 PFLOP/s); 32 suffixes behind 2048 shared keys, paged 184 and 132; 64 x 5 47 and 20; 1 x 300 15 and 15.
+#include <type_traits>
+
 #include "tc.cuh"
 
 namespace nvllm {
@@ -25,15 +39,20 @@ namespace nvllm {
 int check_layout(const nvllm_kv_layout* L);  // store_kvcache.cu
 
 namespace pf {
-constexpr int D = 128, BM = 128, BN = 128, NSLOT = 4;
+constexpr int D = 128, BM = 128, BN = 64, NSLOT = 8;
 constexpr int kQBytes = BM * D * 2;          // one RG's Q tile: 2 halves of [128 x 64]
-constexpr int kTileBytes = BN * D * 2;       // one K (or V) tile: 2 halves of [128 x 64]
+constexpr int kTileBytes = BN * D * 2;       // one K (or V) tile: 2 halves of [64 x 64]
 constexpr int kSmemQ = 0;
 constexpr int kSmemKV = kSmemQ + 2 * kQBytes;
 constexpr int kSmemBar = kSmemKV + NSLOT * kTileBytes;
-constexpr int kNumBars = 1 + 2 * NSLOT + 6;
-constexpr int kSmemBytes = kSmemBar + kNumBars * 8 + 16 + 1024;
-constexpr int kThreads = 384;  // 2 softmax warpgroups + 1 warpgroup holding the TMA and MMA warps (2 idle warps)
+constexpr int kNumBars = 2 + 2 * NSLOT + 12 + 4;        // even: what follows lies on 16 bytes
+constexpr int kSmemClaim = kSmemBar + kNumBars * 8;   // 16-byte answer to a claim
+constexpr int kSmemItem = kSmemClaim + 16;            // block index of the next item and whether there is one
+constexpr int kSmemTmem = kSmemItem + 16;
+constexpr int kSmemBytes = kSmemTmem + 16 + 1024;
+constexpr int kThreads = 384;   // 2 softmax warpgroups + 1 warpgroup holding the TMA, claim and two MMA warps
+constexpr int kReaders = 3 + 8; // of the next item: one lane of the TMA warp, the MMA warps and the softmax warps
+static_assert(kSmemClaim % 16 == 0, "the claim's answer is written as 16 bytes");
 }  // namespace pf
 
 struct PrefillParams {
@@ -41,283 +60,440 @@ struct PrefillParams {
   const int32_t* cu_q;
   const int32_t* cu_k;
   const int32_t* tables;  // NULL: dense K/V
-  int H, Hkv, max_blocks, block_size, box_tok;
+  int H, Hkv, max_blocks, block_size;
+  int box_tok;   // tokens of a K / V copy: 0 dense, else min(64, block size)
+  int pair;      // 1: row group g = query head 2u + g of the same 128 rows; 0: rows [128 g, 128 g + 128) of 256 rows of head u
+  int units;     // grid.x = units * (row blocks per grid.z step)
+  int z_blocks;
   int64_t out_stride;
   float scale_log2;
 };
 
-// POLY: how many of every 4 exponentials go to a polynomial instead of MUFU.EX2 (NVLLM_PREFILL_POLY): 1 / 2 / 3 with the
-// floor-based polynomial (the first version; its floor and float-to-int also run on the XU pipe, so 2 and 3 gain nothing over 1),
-// 4 / 5 / 6 = 1/4, 1/2, 3/4 with the XU-free polynomial.  Default 4 (measured best).
-template <int POLY>
+namespace pf {
+
+struct Item {
+  int seq, head[2], first[2], n[2];  // per row group: query head, first row within the sequence's queries, KV tiles
+  int kvh, q0, k0, Lq, Lk, n_cta;
+};
+
+// The item of a block index; false if the sequence has no such rows.
+__device__ __forceinline__ bool decode_item(const PrefillParams& p, int bx, int by, int bz, Item& it) {
+  const int unit = bx % p.units, zz = bz * p.z_blocks + bx / p.units;
+  it.seq = by;
+  it.q0 = __ldg(p.cu_q + by);
+  it.Lq = __ldg(p.cu_q + by + 1) - it.q0;
+  it.k0 = __ldg(p.cu_k + by);
+  it.Lk = __ldg(p.cu_k + by + 1) - it.k0;
+  const int rows = p.pair ? BM : 2 * BM;
+  const int qblk = (it.Lq + rows - 1) / rows - 1 - zz;  // zz counts from the sequence's last rows
+  it.n_cta = 0;
+  if (qblk < 0) return false;
+  it.kvh = (p.pair ? 2 * unit : unit) / (p.H / p.Hkv);
+#pragma unroll
+  for (int g = 0; g < 2; ++g) {
+    it.head[g] = p.pair ? 2 * unit + g : unit;
+    it.first[g] = qblk * rows + (p.pair ? 0 : g * BM);
+    // KV tiles the row group needs (0 when it has no valid row); bottom-right aligned
+    const int last = min(it.first[g] + BM, it.Lq) - 1;
+    const int visible = max(1, min(it.Lk, it.Lk - it.Lq + last + 1));
+    it.n[g] = it.first[g] >= it.Lq ? 0 : (visible + BN - 1) / BN;
+    it.n_cta = max(it.n_cta, it.n[g]);
+  }
+  return true;
+}
+
+// Asks for the block index of a CTA of this grid that has not started (it then never will); 16 bytes arrive at `dst`.
+__device__ __forceinline__ void claim_next(uint32_t dst, uint32_t bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];\n" ::"r"(dst), "r"(bar) : "memory");
+}
+__device__ __forceinline__ bool claim_read(uint32_t src, int& bx, int& by, int& bz) {
+  uint32_t ok, x = 0, y = 0, z = 0;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 h;\n\t"
+      "mov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\t"
+      "ld.shared.b128 h, [%4];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+      "selp.u32 %3, 1, 0, p;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%0, %1, %2, _}, h;\n\t}\n"
+      : "=&r"(x), "=&r"(y), "=&r"(z), "=&r"(ok)
+      : "r"(src)
+      : "memory");
+  bx = static_cast<int>(x); by = static_cast<int>(y); bz = static_cast<int>(z);
+  return ok != 0;
+}
+
+// pairs of f32 in one 64-bit register: one instruction slot for two values
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;\n" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// Exponentials of 32 scores (in place, f32) and the packed bf16 of them.
+__device__ __forceinline__ void exp_chunk(uint32_t (&s)[32], uint32_t (&pk)[16], uint64_t scale2, uint64_t off2) {
+#pragma unroll
+  for (int e = 0; e < 16; ++e) {
+    float p0, p1;
+    unpack2(fma2(pack2(__uint_as_float(s[2 * e]), __uint_as_float(s[2 * e + 1])), scale2, off2), p0, p1);
+    p0 = fast_exp2(p0);
+    p1 = fast_exp2(p1);
+    s[2 * e] = __float_as_uint(p0);
+    s[2 * e + 1] = __float_as_uint(p1);
+    pk[e] = pack_bf16x2(p0, p1);      // low half = even key: consecutive K elements share a 32-bit column
+  }
+}
+__device__ __forceinline__ float max3(uint32_t a, uint32_t b, float m) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;\n" : "=f"(r) : "f"(__uint_as_float(a)), "f"(__uint_as_float(b)), "f"(m));
+  return r;
+}
+__device__ __forceinline__ float max32(const uint32_t (&s)[32]) {
+  float a[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+  for (int e = 0; e < 16; ++e) a[e & 3] = max3(s[2 * e], s[2 * e + 1], a[e & 3]);
+  return fmaxf(fmaxf(a[0], a[1]), fmaxf(a[2], a[3]));
+}
+__device__ __forceinline__ uint64_t sum32(const uint32_t (&s)[32], uint64_t acc) {
+  uint64_t b = pack2(0.f, 0.f);
+#pragma unroll
+  for (int e = 0; e < 16; e += 2) {
+    acc = add2(acc, pack2(__uint_as_float(s[2 * e]), __uint_as_float(s[2 * e + 1])));
+    b = add2(b, pack2(__uint_as_float(s[2 * e + 2]), __uint_as_float(s[2 * e + 3])));
+  }
+  return add2(acc, b);
+}
+}  // namespace pf
+
 __global__ void __launch_bounds__(pf::kThreads, 1)
 prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const PrefillParams p) {
   using namespace pf;
   pdl_launch_dependents();
-  pdl_wait();  // q / k / v (and the cache) come from the previous kernel
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
   const uint32_t bars = smem_base + kSmemBar;
-  const uint32_t q_full = bars;
-  auto slot_full = [&](int s) { return bars + (1 + s) * 8; };
-  auto slot_empty = [&](int s) { return bars + (1 + NSLOT + s) * 8; };
-  auto s_full = [&](int g) { return bars + (1 + 2 * NSLOT + g) * 8; };       // S_j of group g is in TMEM
-  auto p_ready = [&](int g) { return bars + (1 + 2 * NSLOT + 2 + g) * 8; };  // P_j of group g is in TMEM (128 arrivals)
-  auto o_done = [&](int g) { return bars + (1 + 2 * NSLOT + 4 + g) * 8; };   // PV_j of group g has retired
-  const uint32_t tmem_slot = bars + kNumBars * 8;
+  const uint32_t q_full = bars, q_empty = bars + 8;
+  auto slot_full = [&](int s) { return bars + (2 + s) * 8; };
+  auto slot_empty = [&](int s) { return bars + (2 + NSLOT + s) * 8; };
+  auto s_full = [&](int g, int b) { return bars + (2 + 2 * NSLOT + 2 * g + b) * 8; };       // S is in buffer b of group g
+  auto p_ready = [&](int g, int b) { return bars + (2 + 2 * NSLOT + 4 + 2 * g + b) * 8; };  // P is in buffer b of group g (128 arrivals)
+  auto o_done = [&](int g, int b) { return bars + (2 + 2 * NSLOT + 8 + 2 * g + b) * 8; };   // P.V with buffer b of group g has retired
+  const uint32_t item_full = bars + (2 + 2 * NSLOT + 12) * 8, item_empty = item_full + 8, answered = item_full + 16;
+  const uint32_t claim = smem_base + kSmemClaim, tmem_slot = smem_base + kSmemTmem;
+  volatile int* item_smem = reinterpret_cast<volatile int*>(smem_gen + kSmemItem);
 
-  const int seq = blockIdx.z, head = blockIdx.y;
-  const int qblk = gridDim.x - 1 - blockIdx.x;  // longest (latest rows) first: shorter tail
-  const int kvh = head / (p.H / p.Hkv);
-  const int q0 = __ldg(p.cu_q + seq), Lq = __ldg(p.cu_q + seq + 1) - q0;
-  const int k0 = __ldg(p.cu_k + seq), Lk = __ldg(p.cu_k + seq + 1) - k0;
-  if (qblk * 2 * BM >= Lq) return;  // uniform per CTA: nothing allocated yet
-  const int shift = Lk - Lq;        // bottom-right alignment
-  auto tiles_for = [&](int g) {     // number of KV tiles a row group needs (0 when it has no valid row)
-    const int first = qblk * 2 * BM + g * BM;
-    if (first >= Lq) return 0;
-    const int last = min(first + BM, Lq) - 1;
-    const int visible = max(1, min(Lk, shift + last + 1));
-    return (visible + BN - 1) / BN;
-  };
-  const int n_rg[2] = {tiles_for(0), tiles_for(1)};
-  const int n_cta = max(n_rg[0], n_rg[1]);
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // (uniform: the roles below stay converged)
   if (warp == 8 && lane == 0) {
     tma_prefetch_desc(&tmap_q); tma_prefetch_desc(&tmap_k); tma_prefetch_desc(&tmap_v);
-    mbar_init(q_full, 1);
-    for (int s = 0; s < NSLOT; ++s) { mbar_init(slot_full(s), 1); mbar_init(slot_empty(s), 1); }
-    for (int g = 0; g < 2; ++g) { mbar_init(s_full(g), 1); mbar_init(p_ready(g), BM); mbar_init(o_done(g), 1); }
+    mbar_init(q_full, 1); mbar_init(q_empty, 2);
+    for (int s = 0; s < NSLOT; ++s) { mbar_init(slot_full(s), 1); mbar_init(slot_empty(s), 2); }
+    for (int g = 0; g < 2; ++g)
+      for (int b = 0; b < 2; ++b) { mbar_init(s_full(g, b), 1); mbar_init(p_ready(g, b), BM); mbar_init(o_done(g, b), 1); }
+    mbar_init(item_full, 1); mbar_init(item_empty, kReaders); mbar_init(answered, 1);
     fence_barrier_init();
   }
   if (warp == 0) tmem_alloc<512>(tmem_slot);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *reinterpret_cast<uint32_t*>(smem_gen + kSmemBar + kNumBars * 8);
+  const uint32_t tmem_base = *reinterpret_cast<uint32_t*>(smem_gen + kSmemTmem);
+  pdl_wait();  // q / k / v (and the cache) come from the previous kernel
 
-  // Register reallocation (setmaxnreg, per warpgroup): the producer / MMA warpgroup keeps 88 registers per thread and
-  // donates the rest; each softmax thread holds a full 128-key S row (128 registers) and gets 208.
+  // Every role walks the same list of items: its own block index, then what warp 10 publishes.
+  uint32_t item_phase = 0;
+  auto take_item = [&](Item& it) {       // the item behind a completed item_full
+    item_phase ^= 1;
+    const int x = item_smem[0], y = item_smem[1], z = item_smem[2], ok = item_smem[3];
+    return ok != 0 && decode_item(p, x, y, z, it);
+  };
+  auto next_item = [&](Item& it) {       // a whole warp
+    mbar_wait(item_full, item_phase);
+    const bool ok = take_item(it);
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(item_empty);
+    return ok;
+  };
+  // what the control flow and the addresses of a converged warp depend on, as values that are uniform for the compiler too
+  auto uni = [](int v) { return static_cast<int>(__reduce_max_sync(0xffffffffu, static_cast<uint32_t>(v))); };
+  Item it;
+  const bool own = decode_item(p, blockIdx.x, blockIdx.y, blockIdx.z, it);
+
+  // Register reallocation (setmaxnreg, per warpgroup): the producer / MMA warpgroup keeps 120 registers per thread and
+  // donates the rest: 192 for a softmax thread.
   if (warp >= 8) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 88;\n");  // must dominate the role code below (and only it)
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 120;\n");  // must dominate the role code below (and only it)
   }
-  if (warp >= 10) {
-    // idle warps of the third warpgroup
+  if (warp == 10) {
+    if (lane == 0) {
+      // ===== claims: one item ahead of the softmax; empty items end here =====
+      // The next claim goes out once every role has read the last item, which no role puts off until another item is done.
+      uint32_t ph = 0, answer_phase = 0;
+      int x, y, z;
+      bool ok = true;
+      while (true) {
+        do {
+          mbar_expect_tx(answered, 16);
+          claim_next(claim, answered);
+          mbar_wait(answered, answer_phase);
+          answer_phase ^= 1;
+          ok = claim_read(claim, x, y, z);
+          fence_proxy_async();             // the next answer is written by the async proxy
+        } while (ok && !decode_item(p, x, y, z, it));
+        item_smem[0] = x; item_smem[1] = y; item_smem[2] = z; item_smem[3] = ok;
+        mbar_arrive(item_full);
+        if (!ok) break;
+        mbar_wait(item_empty, ph);
+        ph ^= 1;
+      }
+    }
   } else if (warp == 8) {
-    if (lane == 0) {
-      // ===== TMA producer =====
-      mbar_expect_tx(q_full, 2 * kQBytes);
-      for (int g = 0; g < 2; ++g)
-        for (int hf = 0; hf < 2; ++hf)
-          tma_load_2d(smem_base + kSmemQ + g * kQBytes + hf * (BM * 128), &tmap_q, q_full, head * D + hf * 64,
-                      q0 + qblk * 2 * BM + g * BM);
-      const int32_t* table = p.tables ? p.tables + static_cast<int64_t>(seq) * p.max_blocks : nullptr;
-      for (int t = 0; t < 2 * n_cta; ++t) {  // t even: K_{t/2}, t odd: V_{t/2}
-        const int j = t >> 1, slot = t % NSLOT;
-        const CUtensorMap* map = (t & 1) ? &tmap_v : &tmap_k;
-        mbar_wait(slot_empty(slot), ((t / NSLOT) & 1) ^ 1);
-        mbar_expect_tx(slot_full(slot), kTileBytes);
-        const uint32_t dst = smem_base + kSmemKV + slot * kTileBytes;
-        if (table == nullptr) {
-          for (int hf = 0; hf < 2; ++hf)
-            tma_load_2d(dst + hf * (BN * 128), map, slot_full(slot), kvh * D + hf * 64, k0 + j * BN);
-        } else {
-          for (int c = 0; c < BN / p.box_tok; ++c) {  // box_tok = min(128, block_size) tokens per TMA box
-            const int tok = j * BN + c * p.box_tok;
-            const int bi = tok / p.block_size;
-            const int blk = bi < p.max_blocks ? __ldg(table + bi) : -1;
-            const int blk_c = blk < 0 ? 0x3fffff : blk;  // past the sequence end: far out of bounds -> TMA zero-fills
-            for (int hf = 0; hf < 2; ++hf)
-              tma_load_4d(dst + hf * (BN * 128) + c * p.box_tok * 128, map, slot_full(slot), hf * 64,
-                          tok - bi * p.block_size, kvh, blk_c);
-          }
-        }
-      }
-    }
-  } else if (warp == 9) {
-    if (lane == 0) {
-      // ===== MMA issuer (both row groups) =====
-      constexpr uint32_t idesc_s = umma_idesc_bf16(BM, BN, 0, 0);  // Q K-major, K K-major
-      constexpr uint32_t idesc_o = umma_idesc_bf16(BM, D, 0, 1);   // P K-major (TMEM), V MN-major
-      auto tile_full = [&](int t) { mbar_wait(slot_full(t % NSLOT), (t / NSLOT) & 1); tc_fence_after(); };
-      auto issue_s = [&](int g, int j) {  // S_j^g = Q^g . K_j^T
-        const uint32_t sQ = smem_base + kSmemQ + g * kQBytes;
-        const uint32_t sK = smem_base + kSmemKV + ((2 * j) % NSLOT) * kTileBytes;
-#pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks) {
-          const uint64_t ad = umma_desc_sw128(sQ + (ks >> 2) * (BM * 128) + (ks & 3) * 32, 16, 1024);
-          const uint64_t bd = umma_desc_sw128(sK + (ks >> 2) * (BN * 128) + (ks & 3) * 32, 16, 1024);
-          umma_bf16_ss(tmem_base + g * 256, ad, bd, idesc_s, ks != 0);
-        }
-        umma_commit(s_full(g));
-      };
-      mbar_wait(q_full, 0);
-      if (n_cta > 0) {
-        tile_full(0);
-        for (int g = 0; g < 2; ++g)
-          if (n_rg[g] > 0) issue_s(g, 0);
-        umma_commit(slot_empty(0));  // K_0 consumed once these MMAs retire
-      }
+    // ===== TMA producer =====
+    const uint32_t el = elect_one() ? 1u : 0u;
+    int t = 0;            // tiles through the ring so far
+    uint32_t q_phase = 1; // the first item finds Q's buffer empty
+    for (bool more = uni(own) != 0 || uni(next_item(it)) != 0; more; more = uni(next_item(it)) != 0) {
+      const int n_cta = uni(it.n_cta), kvh = uni(it.kvh), k0 = uni(it.k0);
+      const int32_t* table = p.tables ? p.tables + static_cast<int64_t>(it.seq) * p.max_blocks : nullptr;
+      // whole-tile boxes: a lane holds one of 32 consecutive entries of the table, entry `bi` is the present tile's
+      int bi = 0, in_block = 0, entry = -1;
       for (int j = 0; j < n_cta; ++j) {
-        bool v_waited = false, k_waited = false;
-        for (int g = 0; g < 2; ++g) {
-          if (j >= n_rg[g]) continue;
-          mbar_wait(p_ready(g), j & 1);  // softmax of group g wrote P_j (and rescaled O if it had to)
-          tc_fence_after();
-          if (!v_waited) { tile_full(2 * j + 1); v_waited = true; }
-          const uint32_t sV = smem_base + kSmemKV + ((2 * j + 1) % NSLOT) * kTileBytes;
-#pragma unroll
-          for (int ks = 0; ks < BN / 16; ++ks) {
-            // P: 16 keys = 8 packed columns per step.  V tile: rows = keys, 64 contiguous d per row; the two d halves
-            // (MN groups) are 16 KiB apart, 8 keys per 1 KiB.
-            const uint64_t bd = umma_desc_sw128(sV + ks * 2048, BN * 128, 1024);
-            umma_bf16_ts(tmem_base + g * 256 + 128, tmem_base + g * 256 + ks * 8, bd, idesc_o, (j | ks) != 0);
+        int blk = 0;
+        if (p.box_tok == BN) {
+          if ((bi & 31) == 0 && in_block == 0) entry = bi + lane < p.max_blocks ? __ldg(table + bi + lane) : -1;
+          blk = __shfl_sync(0xffffffffu, entry, bi & 31);
+          blk = uni(blk < 0 ? 0x3fffff : blk);  // past the sequence end: far out of bounds -> TMA zero-fills
+        }
+        for (int kv = 0; kv < 2; ++kv, ++t) {  // K_j, V_j
+          const int slot = t & (NSLOT - 1);
+          const CUtensorMap* map = kv ? &tmap_v : &tmap_k;
+          mbar_wait(slot_empty(slot), ((t / NSLOT) & 1) ^ 1);
+          mbar_expect_tx_warp(slot_full(slot), kTileBytes, el);
+          const uint32_t dst = smem_base + kSmemKV + slot * kTileBytes;
+          if (p.box_tok == 0) {                 // dense
+            tma_load_3d_warp(dst, map, slot_full(slot), 0, k0 + j * BN, kvh * 2, el);
+          } else if (p.box_tok == BN) {
+            tma_load_5d_warp(dst, map, slot_full(slot), 0, in_block, 0, kvh, blk, el);
+          } else {                              // blocks smaller than a tile: a copy for each block and half
+            for (int c = 0; c < BN / p.box_tok; ++c) {
+              const int tok = j * BN + c * p.box_tok, b = tok / p.block_size;
+              const int e = b < p.max_blocks ? __ldg(table + b) : -1;
+              for (int hf = 0; hf < 2; ++hf)
+                tma_load_5d_warp(dst + hf * (BN * 128) + c * p.box_tok * 128, map, slot_full(slot), 0, tok - b * p.block_size, hf, kvh, uni(e < 0 ? 0x3fffff : e), el);
+            }
           }
-          umma_commit(o_done(g));
-          if (j + 1 < n_rg[g]) {
-            if (!k_waited) { tile_full(2 * j + 2); k_waited = true; }
-            issue_s(g, j + 1);  // executes after PV_j^g in the pipe: P_j (aliased with S) is no longer needed by then
+          if (j == 0 && kv == 0) {
+            mbar_wait(q_empty, q_phase);
+            q_phase ^= 1;
+            mbar_expect_tx_warp(q_full, 2 * kQBytes, el);
+            for (int g = 0; g < 2; ++g)
+              tma_load_3d_warp(smem_base + kSmemQ + g * kQBytes, &tmap_q, q_full, 0, uni(it.q0 + it.first[g]), uni(it.head[g]) * 2, el);
           }
         }
-        // both groups' uses of V_j and K_{j+1} are issued: release the slots once they retire
-        umma_commit(slot_empty((2 * j + 1) % NSLOT));
-        if (j + 1 < n_cta) umma_commit(slot_empty((2 * j + 2) % NSLOT));
+        in_block += BN;
+        if (in_block >= p.block_size) { in_block = 0; ++bi; }
       }
     }
+  } else if (warp == 9 || warp == 11) {
+    // ===== MMA issuers, a warp for each row group =====
+    constexpr uint32_t idesc_s = umma_idesc_bf16(BM, BN, 0, 0);  // Q K-major, K K-major
+    constexpr uint32_t idesc_o = umma_idesc_bf16(BM, D, 0, 1);   // P K-major (TMEM), V MN-major
+    const uint32_t el = elect_one() ? 1u : 0u;
+    auto test = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_test_wait(bar, parity)) != 0; };
+    auto slot_of = [&](int t) { return t & (NSLOT - 1); };
+    auto tile_full = [&](int t) { mbar_wait(slot_full(slot_of(t)), (t / NSLOT) & 1); tc_fence_after(); };
+    auto run = [&](auto group) {
+      constexpr int g = decltype(group)::value;
+      const uint32_t tm = __reduce_max_sync(0xffffffffu, tmem_base) + g * 256;
+      struct Tiles { int n, n_cta; };  // of this group, of the item
+      auto tiles_of = [&](const Item& it) { return Tiles{uni(it.n[g]), uni(it.n_cta)}; };
+      auto next = [&](Tiles& nt) {
+        const bool ok = uni(next_item(it)) != 0;
+        nt = tiles_of(it);
+        return ok;
+      };
+      uint32_t q_phase = 0, s_cnt = 0, p_cnt = 0;   // S and P.V issued so far: tile n of the group uses buffer n & 1
+      // S = Q . K^T of tile `tile` of an item whose K_0 is number `base` of the ring; a group that does not need the tile lets it go
+      auto s_of = [&](const Tiles& ti, int base, int tile) {
+        const int t = base + 2 * tile;
+        if (tile == 0) { mbar_wait(q_full, q_phase); q_phase ^= 1; }
+        tile_full(t);
+        if (tile < ti.n) {
+          const uint32_t ad = umma_desc_lo(smem_base + kSmemQ + g * kQBytes, 16), bd = umma_desc_lo(smem_base + kSmemKV, 16) + slot_of(t) * (kTileBytes >> 4);
+          const uint32_t b = s_cnt++ & 1;
+#pragma unroll
+          for (int ks = 0; ks < D / 16; ++ks)
+            umma_bf16_ss_warp(tm + b * BN, ad + (((ks >> 2) * (BM * 128) + (ks & 3) * 32) >> 4), bd + (((ks >> 2) * (BN * 128) + (ks & 3) * 32) >> 4), idesc_s,
+                              ks != 0, el);   // executes after P.V of the buffer's last tile, which has been issued
+          umma_commit_warp(s_full(g, b), el);
+        }
+        umma_commit_warp(slot_empty(slot_of(t)), el);
+        if (tile + 1 == ti.n_cta) umma_commit_warp(q_empty, el);   // that was the last S of its item
+      };
+      auto pv_of = [&](const Tiles& ti, int base, int j) {   // O (+)= P_j . V_j
+        const int t = base + 2 * j + 1;
+        if (j < ti.n) {
+          const uint32_t b = p_cnt & 1;
+          mbar_wait(p_ready(g, b), (p_cnt >> 1) & 1);  // the softmax wrote P_j (and rescaled O if it had to)
+          ++p_cnt;
+          tile_full(t);
+          // P: 16 keys = 8 packed columns per step.  V tile: rows = keys, 64 contiguous d per row; the two d halves
+          // (MN groups) are 8 KiB apart, 8 keys per 1 KiB.
+          const uint32_t vd = umma_desc_lo(smem_base + kSmemKV, BN * 128) + slot_of(t) * (kTileBytes >> 4);
+#pragma unroll
+          for (int ks = 0; ks < BN / 16; ++ks)
+            umma_bf16_ts_warp(tm + 2 * BN, tm + b * BN + ks * 8, vd + ((ks * 2048) >> 4), idesc_o, ks != 0 ? 1u : (j == 0 ? 0u : 1u), el);
+          umma_commit_warp(o_done(g, b), el);
+        } else {
+          tile_full(t);
+        }
+        umma_commit_warp(slot_empty(slot_of(t)), el);
+      };
+      int base = 0;                    // ring number of the present item's K_0; its V_j is base + 2 j + 1, K_j base + 2 j
+      int s_now = 0;                   // tiles of the present item whose S has been issued
+      Tiles cur{}, nxt{};
+      bool more = uni(own) != 0;
+      if (more) cur = tiles_of(it); else more = next(cur);
+      while (more) {
+        for (; s_now < min(2, cur.n_cta); ++s_now) s_of(cur, base, s_now);
+        bool known = false;
+        int s_next = 0;                // tiles of the next item whose S has been issued
+        const int base_next = base + 2 * cur.n_cta;
+        for (int j = 0; j < cur.n_cta; ++j) {
+          pv_of(cur, base, j);
+          // the S behind this tile's P.V: of the tile after next, or of the next item's first ones if nothing of it has to be waited for
+          if (s_now < cur.n_cta) {
+            s_of(cur, base, s_now++);
+          } else {
+            if (!known && test(item_full, item_phase)) { more = next(nxt); known = true; }
+            const int kt = base_next + 2 * s_next;
+            if (known && more && s_next < min(2, nxt.n_cta) && (s_next > 0 || test(q_full, q_phase)) && test(slot_full(slot_of(kt)), (kt / NSLOT) & 1))
+              s_of(nxt, base_next, s_next++);
+          }
+        }
+        if (!known) more = next(nxt);
+        base = base_next;
+        cur = nxt;
+        s_now = s_next;
+      }
+    };
+    if (warp == 9) run(std::integral_constant<int, 0>{}); else run(std::integral_constant<int, 1>{});
   } else {
     // ===== row groups: softmax + output =====
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 208;\n");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 192;\n");
     const int g = warp >> 2;               // row group 0 / 1
     const int t = threadIdx.x & 127;       // row within the group's tile == TMEM lane
-    const int n_my = n_rg[g];
-    const int row = qblk * 2 * BM + g * BM + t;  // row within the sequence's queries
-    const int limit = shift + row;               // last visible key index
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const uint32_t tS = tmem_base + g * 256 + lane_off;  // S (fp32, 128 columns) / P (packed bf16, first 64 columns)
-    const uint32_t tO = tS + 128;
+    const uint32_t tS0 = tmem_base + g * 256 + lane_off;  // two buffers of S (fp32, 64 columns) / P (packed bf16, first 32 columns)
+    const uint32_t tO = tS0 + 2 * BN;
     constexpr float kRescaleThreshold = 8.0f;  // log2 units: P stays <= 2^8 between refreshes
-    // 2^x for x <= 0 on the FMA pipe: x = n + f, f in [0, 1); 2^f by a degree-3 polynomial (rel. err 2.3e-4, far below
-    // bf16's 2^-9), 2^n by adding n to the exponent field.
-    auto exp2_poly = [](float x) {
-      x = fmaxf(x, -126.f);
-      const float n = floorf(x);
-      const float f = x - n;
-      float pfr = fmaf(f, 0.0790209f, 0.2241543f);
-      pfr = fmaf(pfr, f, 0.6965186f);
-      pfr = fmaf(pfr, f, 0.9998430f);
-      return __int_as_float(__float_as_int(pfr) + (static_cast<int>(n) << 23));
-    };
-
-    // The same without any XU-pipe instruction (the floor and float-to-int of the version above run on the
-    // XU pipe next to the exponentials, whose counter is saturated — it relieves nothing): round-to-nearest by the 1.5 * 2^23 magic add,
-    // f in [-0.5, 0.5], degree-3 minimax polynomial (rel. err 7.5e-5), n taken from the low mantissa bits of the sum.
-    auto exp2_poly2 = [](float x) {
-      x = fmaxf(x, -126.f);
-      const float t = x + 12582912.f;
-      const float f = x - (t - 12582912.f);
-      float pfr = fmaf(f, 0.05517210811376572f, 0.24261118471622467f);
-      pfr = fmaf(pfr, f, 0.693260908126831f);
-      pfr = fmaf(pfr, f, 0.9999280571937561f);
-      return __int_as_float(__float_as_int(pfr) + (__float_as_int(t) << 23));
-    };
-
-    float m_ref = -INFINITY, l_run = 0.f;  // m_ref: the (stale-by-design) maximum the exponentials are taken against
-    for (int j = 0; j < n_my; ++j) {
-      mbar_wait(s_full(g), j & 1);
-      // S_j was issued after PV_{j-1} and MMAs of one thread retire in order: this wait is free.  It consumes the o_done
-      // phases strictly in order (a parity wait may never lag two phases behind), and O is quiescent from here on.
-      if (j > 0) mbar_wait(o_done(g), (j - 1) & 1);
-      tc_fence_after();
-      uint32_t sr[4][32];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x32(tS + c * 32, sr[c]);
-      tmem_ld_wait();
-      const int kbase = j * BN;
-      if ((kbase + BN - 1 > limit) || (kbase + BN > Lk)) {
-#pragma unroll
-        for (int c = 0; c < BN; ++c)
-          if (kbase + c > limit || kbase + c >= Lk) sr[c >> 5][c & 31] = 0xff800000u;  // -inf
+    const uint64_t scale2 = pack2(p.scale_log2, p.scale_log2);
+    uint32_t tile = 0;                         // tiles of this group so far
+    bool more = own;
+    while (true) {
+      if (!more) {
+        mbar_wait(item_full, item_phase);
+        const bool ok = take_item(it);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(item_empty);
+        if (!ok) break;
       }
-      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // 4 independent chains
+      more = false;
+      const int n_my = g ? it.n[1] : it.n[0], Lk = it.Lk;
+      const int row = (g ? it.first[1] : it.first[0]) + t;             // row within the sequence's queries
+      const int vis = min(Lk, Lk - it.Lq + row + 1);       // keys [0, vis) are visible
+      const int vis_lo = min(Lk, Lk - it.Lq + row - lane + 1);   // ... to the warp's first row
+      float m_ref = -INFINITY, l_run = 0.f;  // m_ref: the (stale-by-design) maximum the exponentials are taken against
+      for (int j = 0; j < n_my; ++j, ++tile) {
+        const int kbase = j * BN;
+        const int b = tile & 1;
+        const uint32_t tS = tS0 + b * BN;
+        mbar_wait(s_full(g, b), (tile >> 1) & 1);
+        tc_fence_after();
+        uint32_t sr[2][32], pk[16];
+        tmem_ld_32x32b_x32(tS, sr[0]);
+        tmem_ld_32x32b_x32(tS + 32, sr[1]);
+        tmem_ld_wait(sr[0]);
+        tmem_ld_wait(sr[1]);
+        if (vis_lo < kbase + BN) {     // some row of the warp has a hidden key in this tile
 #pragma unroll
-      for (int c = 0; c < BN; ++c) mx4[c & 3] = fmaxf(mx4[c & 3], __uint_as_float(sr[c >> 5][c & 31]));
-      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-      // lazy rescale: refresh the reference maximum only when this tile exceeds it by more than the threshold
-      const bool refresh = (mx - m_ref) * p.scale_log2 > kRescaleThreshold;  // also true for the first finite tile
-      float corr = 1.f;
-      if (refresh) {
-        corr = (m_ref == -INFINITY) ? 0.f : fast_exp2((m_ref - mx) * p.scale_log2);
-        m_ref = mx;
-        l_run *= corr;
+          for (int c = 0; c < BN; ++c)
+            if (kbase + c >= vis) sr[c >> 5][c & 31] = 0xff800000u;  // -inf
+        }
+        const float mx = fmaxf(max32(sr[0]), max32(sr[1]));
+        // lazy rescale: refresh the reference maximum only when this tile exceeds it by more than the threshold
+        const bool refresh = (mx - m_ref) * p.scale_log2 > kRescaleThreshold;  // also true for the first finite tile
+        float corr = 1.f;
+        if (refresh) {
+          corr = (m_ref == -INFINITY) ? 0.f : fast_exp2((m_ref - mx) * p.scale_log2);
+          m_ref = mx;
+          l_run *= corr;
+        }
+        if (j > 0 && __any_sync(0xffffffffu, refresh)) {  // tcgen05.ld/st are warp-collective: the whole warp takes part
+          // O rests once P.V of the tile before has retired.  (That of two tiles before has: S of this tile was issued after it.  So the
+          // barrier is at most one phase ahead of what is waited for here.)
+          mbar_wait(o_done(g, b ^ 1), ((tile - 1) >> 1) & 1);
+          tc_fence_after();
+#pragma unroll 1
+          for (int c = 0; c < D / 16; ++c) {
+            uint32_t orr[16];
+            tmem_ld_32x32b_x16(tO + c * 16, orr);
+            tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < 16; ++e) orr[e] = __float_as_uint(__uint_as_float(orr[e]) * corr);
+            tmem_st_32x32b_x16(tO + c * 16, orr);
+          }
+        }
+        const float moff = (m_ref == -INFINITY) ? 0.f : -m_ref * p.scale_log2;
+        const uint64_t off2 = pack2(moff, moff);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          exp_chunk(sr[c], pk, scale2, off2);
+          tmem_st_32x32b_x16(tS + c * 16, pk);  // P over this thread's own S lane
+        }
+        tmem_st_wait();
+        tc_fence_before();
+        mbar_arrive(p_ready(g, b));
+        uint64_t ls = sum32(sr[1], sum32(sr[0], pack2(0.f, 0.f)));
+        float l0, l1;
+        unpack2(ls, l0, l1);
+        l_run += l0 + l1;
       }
-      if (j > 0 && __any_sync(0xffffffffu, refresh)) {  // tcgen05.ld/st are warp-collective: the whole warp takes part
+      // ---- output -----------------------------------------------------------------------------------
+      if (n_my > 0) {
+        mbar_wait(o_done(g, (tile - 1) & 1), ((tile - 1) >> 1) & 1);
+        tc_fence_after();
+        const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
+        bf16* orow = p.out + static_cast<int64_t>(it.q0 + row) * p.out_stride + (g ? it.head[1] : it.head[0]) * D;
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
           uint32_t orr[32];
           tmem_ld_32x32b_x32(tO + c * 32, orr);
           tmem_ld_wait();
+          if (row < it.Lq) {
 #pragma unroll
-          for (int e = 0; e < 32; ++e) orr[e] = __float_as_uint(__uint_as_float(orr[e]) * corr);
-          tmem_st_32x32b_x32(tO + c * 32, orr);
-        }
-      }
-      const float moff = (m_ref == -INFINITY) ? 0.f : m_ref * p.scale_log2;
-      float ls4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int h2 = 0; h2 < 2; ++h2) {  // 2 x 64 keys -> 2 x 32 packed columns
-        uint32_t pk[32];
-#pragma unroll
-        for (int e = 0; e < 32; ++e) {
-          const int c = h2 * 64 + e * 2;
-          const float a0 = fmaf(__uint_as_float(sr[c >> 5][c & 31]), p.scale_log2, -moff);
-          const float a1 = fmaf(__uint_as_float(sr[(c + 1) >> 5][(c + 1) & 31]), p.scale_log2, -moff);
-          float p0, p1;
-          if constexpr (POLY <= 3) {
-            p0 = (POLY >= 3 && (e & 1)) ? exp2_poly(a0) : fast_exp2(a0);               // MUFU (POLY 3: half of them FMA)
-            p1 = (POLY >= 2 || (POLY == 1 && (e & 1))) ? exp2_poly(a1) : fast_exp2(a1);  // FMA-pipe share per POLY
-          } else {  // POLY 4 / 5 / 6: 1/4, 1/2, 3/4 of the exponentials on the XU-free polynomial
-            p0 = (POLY >= 6 && (e & 1)) ? exp2_poly2(a0) : fast_exp2(a0);
-            p1 = (POLY >= 5 || (e & 1)) ? exp2_poly2(a1) : fast_exp2(a1);
+            for (int e = 0; e < 32; e += 8) {
+              uint4 v;
+              v.x = pack_bf16x2(__uint_as_float(orr[e]) * inv, __uint_as_float(orr[e + 1]) * inv);
+              v.y = pack_bf16x2(__uint_as_float(orr[e + 2]) * inv, __uint_as_float(orr[e + 3]) * inv);
+              v.z = pack_bf16x2(__uint_as_float(orr[e + 4]) * inv, __uint_as_float(orr[e + 5]) * inv);
+              v.w = pack_bf16x2(__uint_as_float(orr[e + 6]) * inv, __uint_as_float(orr[e + 7]) * inv);
+              *reinterpret_cast<uint4*>(orow + c * 32 + e) = v;
+            }
           }
-          ls4[e & 3] += p0 + p1;
-          pk[e] = pack_bf16x2(p0, p1);      // low half = even key: consecutive K elements share a 32-bit column
         }
-        tmem_st_32x32b_x32(tS + h2 * 32, pk);  // P over this thread's own S lane
-      }
-      l_run += (ls4[0] + ls4[1]) + (ls4[2] + ls4[3]);
-      tmem_st_wait();
-      tc_fence_before();
-      mbar_arrive(p_ready(g));
-    }
-    float acc[D];
-    if (n_my > 0) {
-      mbar_wait(o_done(g), (n_my - 1) & 1);
-      tc_fence_after();
-#pragma unroll
-      for (int c = 0; c < D / 32; ++c) {
-        uint32_t orr[32];
-        tmem_ld_32x32b_x32(tO + c * 32, orr);
-        tmem_ld_wait();
-#pragma unroll
-        for (int e = 0; e < 32; ++e) acc[c * 32 + e] = __uint_as_float(orr[e]);
-      }
-      tc_fence_before();
-    }
-    // ---- output -------------------------------------------------------------------------------------
-    if (n_my > 0 && row < Lq) {
-      const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
-      bf16* orow = p.out + static_cast<int64_t>(q0 + row) * p.out_stride + head * D;
-#pragma unroll
-      for (int c = 0; c < D / 8; ++c) {
-        uint4 v;
-        v.x = pack_bf16x2(acc[c * 8 + 0] * inv, acc[c * 8 + 1] * inv);
-        v.y = pack_bf16x2(acc[c * 8 + 2] * inv, acc[c * 8 + 3] * inv);
-        v.z = pack_bf16x2(acc[c * 8 + 4] * inv, acc[c * 8 + 5] * inv);
-        v.w = pack_bf16x2(acc[c * 8 + 6] * inv, acc[c * 8 + 7] * inv);
-        *reinterpret_cast<uint4*>(orow + c * 8) = v;
+        tc_fence_before();   // ordered before the first P of the next item, whose P.V overwrites O
       }
     }
   }
@@ -355,13 +531,20 @@ extern "C" int nvllm_varlen_prefill_attention(void* out, const void* q, const vo
                   NVLLM_ERR_ALIGN, "prefill_attention: out alignment / stride");
   const bool paged = block_tables != nullptr;
   CUtensorMap tq, tk, tv;
-  if (int rc = make_tmap_bf16_2d(&tq, q, total_q, (int64_t)num_heads * head_dim, q_token_stride, pf::BM)) return rc;
+  // (64 values, row, half of a head): a head's two halves come in one copy
+  auto rows_map = [](CUtensorMap* map, const void* base, int64_t rows, int heads, int64_t ld, int box_rows) -> int {
+    NVLLM_CHECK_ARG(ld % 8 == 0, NVLLM_ERR_ALIGN, "TMA: base must be 16-byte aligned and the row pitch a multiple of 16 bytes");
+    const uint64_t dims[3] = {64, (uint64_t)rows, 2 * (uint64_t)heads}, strides[2] = {(uint64_t)ld * 2, 128};
+    const uint32_t box[3] = {64, (uint32_t)box_rows, 2};
+    return make_tmap_bf16_nd(map, base, 3, dims, strides, box);
+  };
+  if (int rc = rows_map(&tq, q, total_q, num_heads, q_token_stride, pf::BM)) return rc;
   PrefillParams p;
-  p.box_tok = pf::BN;
+  p.box_tok = 0;
   if (!paged) {
     NVLLM_CHECK_ARG(k && v && total_k > 0, NVLLM_ERR_ARG, "prefill_attention: dense k/v missing");
-    if (int rc = make_tmap_bf16_2d(&tk, k, total_k, (int64_t)num_kv_heads * head_dim, kv_token_stride, pf::BN)) return rc;
-    if (int rc = make_tmap_bf16_2d(&tv, v, total_k, (int64_t)num_kv_heads * head_dim, kv_token_stride, pf::BN)) return rc;
+    if (int rc = rows_map(&tk, k, total_k, num_kv_heads, kv_token_stride, pf::BN)) return rc;
+    if (int rc = rows_map(&tv, v, total_k, num_kv_heads, kv_token_stride, pf::BN)) return rc;
     p.block_size = 1;
     p.max_blocks = 0;
   } else {
@@ -370,15 +553,15 @@ extern "C" int nvllm_varlen_prefill_attention(void* out, const void* q, const vo
     NVLLM_CHECK_ARG(layout->num_kv_heads == num_kv_heads && layout->head_dim == head_dim, NVLLM_ERR_ARG,
                     "prefill_attention: layout heads/dim mismatch");
     const int bs = layout->block_size;
-    NVLLM_CHECK_ARG(bs % 16 == 0 && (bs >= pf::BN ? bs % pf::BN == 0 : pf::BN % bs == 0), NVLLM_ERR_ARG,
-                    "prefill_attention: block_size %d must divide or be a multiple of %d", bs, pf::BN);
+    constexpr int kUnit = 128;
+    NVLLM_CHECK_ARG(bs % 16 == 0 && (bs >= kUnit ? bs % kUnit == 0 : kUnit % bs == 0), NVLLM_ERR_ARG,
+                    "prefill_attention: block_size %d must divide or be a multiple of %d", bs, kUnit);
     p.box_tok = bs < pf::BN ? bs : pf::BN;
-    const uint64_t dims[4] = {(uint64_t)head_dim, (uint64_t)bs, (uint64_t)num_kv_heads, 0x3fffffull};
-    const uint64_t strides[3] = {(uint64_t)layout->token_stride * 2, (uint64_t)layout->head_stride * 2,
-                                 (uint64_t)layout->block_stride * 2};
-    const uint32_t box[4] = {64, (uint32_t)p.box_tok, 1, 1};
-    if (int rc = make_tmap_bf16_nd(&tk, k_cache, 4, dims, strides, box)) return rc;
-    if (int rc = make_tmap_bf16_nd(&tv, v_cache, 4, dims, strides, box)) return rc;
+    const uint64_t dims[5] = {64, (uint64_t)bs, 2, (uint64_t)num_kv_heads, 0x3fffffull};
+    const uint64_t strides[4] = {(uint64_t)layout->token_stride * 2, 128, (uint64_t)layout->head_stride * 2, (uint64_t)layout->block_stride * 2};
+    const uint32_t box[5] = {64, (uint32_t)p.box_tok, p.box_tok == pf::BN ? 2u : 1u, 1, 1};
+    if (int rc = make_tmap_bf16_nd(&tk, k_cache, 5, dims, strides, box)) return rc;
+    if (int rc = make_tmap_bf16_nd(&tv, v_cache, 5, dims, strides, box)) return rc;
     p.block_size = bs;
     p.max_blocks = max_blocks_per_seq;
   }
@@ -390,30 +573,15 @@ extern "C" int nvllm_varlen_prefill_attention(void* out, const void* q, const vo
   p.Hkv = num_kv_heads;
   p.out_stride = out_token_stride;
   p.scale_log2 = scale * 1.4426950408889634f;
-  {
-    static std::once_flag once;
-    static cudaError_t once_err = cudaSuccess;
-    std::call_once(once, [] {
-      const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-      cudaError_t e = cudaFuncSetAttribute(prefill_attn_kernel<1>, attr, pf::kSmemBytes);
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(prefill_attn_kernel<2>, attr, pf::kSmemBytes);
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(prefill_attn_kernel<3>, attr, pf::kSmemBytes);
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(prefill_attn_kernel<4>, attr, pf::kSmemBytes);
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(prefill_attn_kernel<5>, attr, pf::kSmemBytes);
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(prefill_attn_kernel<6>, attr, pf::kSmemBytes);
-      once_err = e;
-    });
-    NVLLM_CUDA(once_err);
-  }
+  const bool pair = (num_heads / num_kv_heads) % 2 == 0;
+  p.pair = pair ? 1 : 0;
+  p.units = pair ? num_heads / 2 : num_heads;
+  const int rows = pair ? pf::BM : 2 * pf::BM;
+  const int blocks = (max_seqlen_q + rows - 1) / rows;
+  p.z_blocks = (blocks + 65534) / 65535;
   (void)max_seqlen_k;
-  dim3 grid((max_seqlen_q + 2 * pf::BM - 1) / (2 * pf::BM), num_heads, batch);
-  const int poly = knobs().prefill_poly;  // XU-free polynomial on 1/4 of the exponentials: +26 % at 4K, 1060 TFLOP/s at 32K
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (poly == 2) NVLLM_CUDA(launch_pdl(prefill_attn_kernel<2>, grid, dim3(pf::kThreads), pf::kSmemBytes, st, tq, tk, tv, p));
-  else if (poly == 3) NVLLM_CUDA(launch_pdl(prefill_attn_kernel<3>, grid, dim3(pf::kThreads), pf::kSmemBytes, st, tq, tk, tv, p));
-  else if (poly == 4) NVLLM_CUDA(launch_pdl(prefill_attn_kernel<4>, grid, dim3(pf::kThreads), pf::kSmemBytes, st, tq, tk, tv, p));
-  else if (poly == 5) NVLLM_CUDA(launch_pdl(prefill_attn_kernel<5>, grid, dim3(pf::kThreads), pf::kSmemBytes, st, tq, tk, tv, p));
-  else if (poly == 6) NVLLM_CUDA(launch_pdl(prefill_attn_kernel<6>, grid, dim3(pf::kThreads), pf::kSmemBytes, st, tq, tk, tv, p));
-  else NVLLM_CUDA(launch_pdl(prefill_attn_kernel<1>, grid, dim3(pf::kThreads), pf::kSmemBytes, st, tq, tk, tv, p));
+  const dim3 grid(p.units * p.z_blocks, batch, (blocks + p.z_blocks - 1) / p.z_blocks);
+  NVLLM_SMEM_ATTR_ONCE(prefill_attn_kernel, pf::kSmemBytes);
+  NVLLM_CUDA(launch_pdl(prefill_attn_kernel, grid, dim3(pf::kThreads), pf::kSmemBytes, static_cast<cudaStream_t>(stream), tq, tk, tv, p));
   return 0;
 }

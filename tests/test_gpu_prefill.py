@@ -94,3 +94,47 @@ def test_varlen_prefill_full_size_vs_torch(cuda):
         vv = v[sl].float().permute(1, 0, 2).repeat_interleave(H // Hkv, 0)
         ref = torch.nn.functional.scaled_dot_product_attention(qq, kk, vv, is_causal=True).permute(1, 0, 2)
         assert_close(to_np_f32(out[sl]), to_np_f32(ref), ATT_ATOL, ATT_RTOL, f"prefill full-size seq {b}")
+
+
+@pytest.mark.parametrize("H,Hkv,top,paged", [(16, 8, 700, 0), (6, 2, 500, 0), (8, 8, 300, 0), (16, 8, 300, 64), (6, 2, 200, 256), (8, 2, 130, 16)])
+def test_varlen_prefill_many_ragged_items(cuda, H, Hkv, top, paged):
+    """More work items than SMs, most of them claimed by CTAs that stay, many of them empty: 60 sequences of 0 .. top new tokens (heads that pair
+    up and heads that do not, tiles of one to a dozen), dense and behind a paged prefix, against torch in f32."""
+    from nano_vllm_rs_b200 import ops
+    from nano_vllm_rs_b200._ffi import KvLayout
+    D, B = 128, 60
+    rng = np.random.default_rng(H + top)
+    lens = [int(top * u * u) for u in rng.random(B)]
+    lens[5], lens[17], lens[40] = 0, top, 1
+    pre = [int(rng.integers(0, 300)) if paged else 0 for _ in lens]
+    tot = [a + b for a, b in zip(pre, lens)]
+    g = torch.Generator(device="cuda").manual_seed(top)
+    rand = lambda *s: torch.randn(*s, generator=g, device=cuda).to(torch.bfloat16)
+    q = rand(sum(lens), H, D)
+    ks, vs = [rand(n, Hkv, D) for n in tot], [rand(n, Hkv, D) for n in tot]
+    cu_q, cu_k = torch.from_numpy(_cu(lens)).to(cuda), torch.from_numpy(_cu(tot)).to(cuda)
+    if not paged:
+        out = ops.varlen_prefill_attention(q, torch.cat(ks), torch.cat(vs), cu_q, cu_k, max(lens), max(tot))
+    else:
+        per = [-(-n // paged) for n in tot]
+        ids = iter(torch.randperm(sum(per), generator=torch.Generator().manual_seed(1)).tolist())
+        tables = torch.full((B, max(per)), -1, dtype=torch.int32)
+        kc, vc = (torch.zeros(sum(per), Hkv, paged, D, dtype=torch.bfloat16, device=cuda) for _ in range(2))
+        for b in range(B):
+            for i in range(per[b]):
+                blk = next(ids)
+                tables[b, i] = blk
+                n = min(paged, tot[b] - i * paged)
+                kc[blk, :, :n] = ks[b][i * paged:i * paged + n].transpose(0, 1)
+                vc[blk, :, :n] = vs[b][i * paged:i * paged + n].transpose(0, 1)
+        out = ops.varlen_prefill_attention(q, None, None, cu_q, cu_k, max(lens), max(tot), k_cache=kc, v_cache=vc, block_tables=tables.to(cuda),
+                                           layout=KvLayout.head_major(paged, Hkv, D))
+    torch.cuda.synchronize()
+    at = 0
+    for b, n in enumerate(lens):
+        if n:
+            s = torch.einsum("qhd,khd->hqk", q[at:at + n].float(), ks[b].float().repeat_interleave(H // Hkv, 1)) * D ** -0.5
+            hidden = torch.arange(tot[b], device=cuda)[None, :] > torch.arange(n, device=cuda)[:, None] + pre[b]
+            ref = torch.einsum("hqk,khd->qhd", s.masked_fill(hidden, -float("inf")).softmax(-1), vs[b].float().repeat_interleave(H // Hkv, 1))
+            assert_close(to_np_f32(out[at:at + n]), to_np_f32(ref), ATT_ATOL, ATT_RTOL, f"sequence {b}: {n} of {tot[b]}")
+        at += n
