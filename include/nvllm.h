@@ -469,6 +469,13 @@ int nvllm_linear_recurrence(float* y, int64_t ldy, const float* q, int64_t ldq, 
                             int32_t step_per_token, const float* skip, float* state, const int32_t* seq_slot,
                             const int32_t* cu_tokens, const int64_t* positions, int32_t n_seqs, int32_t heads,
                             int32_t groups, int32_t dk, int32_t dv, void* stream);
+/* The same for a caller that knows how many tokens the batch holds (n; 0: not known): prompts are taken 32 tokens at a time as
+ * matrix products. */
+int nvllm_linear_recurrence_step(float* y, int64_t ldy, const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v,
+                                 int64_t ldv, const float* decay, int32_t decay_per_token, const float* step,
+                                 int32_t step_per_token, const float* skip, float* state, const int32_t* seq_slot,
+                                 const int32_t* cu_tokens, const int64_t* positions, int32_t n, int32_t n_seqs, int32_t heads,
+                                 int32_t groups, int32_t dk, int32_t dv, void* stream);
 /* out[t, c] = act(bias[c] + sum_j w[c, j] * in[token at position(t) - (taps - 1 - j), c]) (zero before the sequence; act =
  * SiLU when silu != 0); state: [slots, taps - 1, channels] = the raw inputs of the last taps - 1 tokens, read for inputs
  * before the portion and rewritten afterwards.  taps <= 16; out != in. */

@@ -87,6 +87,8 @@ PROTOTYPES = {
                                      f32, f32, f32, i32, vp, i32, i32, vp]),
     "nvllm_linear_recurrence": (i32, [vp, i64, vp, i64, vp, i64, vp, i64, vp, i32, vp, i32, vp, vp, vp, vp, vp, i32, i32, i32, i32,
                                       i32, vp]),
+    "nvllm_linear_recurrence_step": (i32, [vp, i64, vp, i64, vp, i64, vp, i64, vp, i32, vp, i32, vp, vp, vp, vp, vp, i32, i32, i32, i32,
+                                           i32, i32, vp]),
     "nvllm_causal_conv": (i32, [vp, i64, vp, i64, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp]),
     "nvllm_ssd_prepare": (i32, [vp, vp, vp, i64, vp, vp, i32, i32, vp]),
     "nvllm_rotate_half": (i32, [vp, i64, vp, vp, i32, i32, i32, i32, i32, f32, vp]),

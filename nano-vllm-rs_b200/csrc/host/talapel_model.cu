@@ -536,8 +536,8 @@ class Talapel : public ModelImpl {
         RUN(nvllm_causal_conv(conv_out_, ch, proj_ + inner, lds, L.conv_w, L.conv_b, rs.conv, v.tok_seq, v.seq_slots, v.cu_tokens, v.positions, N, S,
                               ch, L.taps, 1, st)); launches += L.taps > 1 ? 2 : 1; mk("causal_conv");
         RUN(nvllm_ssd_prepare(step_, decay_t_, proj_ + inner + ch, lds, L.dt_bias, L.a_log, N, L.sH, st)); ++launches; mk("ssd_prepare");
-        RUN(nvllm_linear_recurrence(y_, inner, conv_out_ + inner + gns, ch, conv_out_ + inner, ch, conv_out_, ch, decay_t_, 1, step_, 1, L.skip,
-                                    rs.ssd, v.seq_slots, v.cu_tokens, v.positions, S, L.sH, L.sG, L.sN, L.sP, st)); ++launches; mk("linear_recurrence (ssd)");
+        RUN(nvllm_linear_recurrence_step(y_, inner, conv_out_ + inner + gns, ch, conv_out_ + inner, ch, conv_out_, ch, decay_t_, 1, step_, 1, L.skip,
+                                    rs.ssd, v.seq_slots, v.cu_tokens, v.positions, N, S, L.sH, L.sG, L.sN, L.sP, st)); ++launches; mk("linear_recurrence (ssd)");
         RUN(nvllm_gated_group_norm(mix_in_, inner, y_, inner, proj_, lds, L.s_norm, N, inner, L.norm_groups, eps_, 1, dt_, st)); ++launches; mk("gated_group_norm");
         RUN(lin(right_out_, mix_in_, L.s_o, W, inner, W, NVLLM_F32, "ssd output projection"));
         pend.a[0] = left_out_; pend.s[0] = L.left_scale;
@@ -549,8 +549,8 @@ class Talapel : public ModelImpl {
         RUN(lin(proj_, normed_, L.r_in, ldr, W, ldr, NVLLM_F32, "retention q k v g projection"));
         // q and k heads lie side by side: one launch rotates both; the key scale dim^-1/2 rides in the recurrence as its step
         RUN(nvllm_rotate_half(proj_, ldr, v.positions, L.rope, lim_.max_positions, N, 2 * L.rH, L.rD, L.rot_dims, 1.0f, st)); ++launches; mk("rotate_half (q, k)");
-        RUN(nvllm_linear_recurrence(y_, vn, proj_, ldr, proj_ + qn, ldr, proj_ + 2 * qn, ldr, L.decay, 0, L.kscale, 0, nullptr, rs.ret, v.seq_slots,
-                                    v.cu_tokens, v.positions, S, L.rH, L.rH, L.rD, L.rV, st)); ++launches; mk("linear_recurrence (retention)");
+        RUN(nvllm_linear_recurrence_step(y_, vn, proj_, ldr, proj_ + qn, ldr, proj_ + 2 * qn, ldr, L.decay, 0, L.kscale, 0, nullptr, rs.ret, v.seq_slots,
+                                    v.cu_tokens, v.positions, N, S, L.rH, L.rH, L.rD, L.rV, st)); ++launches; mk("linear_recurrence (retention)");
         RUN(nvllm_gated_group_norm(mix_in_, vn, y_, vn, proj_ + 2 * qn + vn, ldr, nullptr, N, vn, L.rH, eps_, 0, dt_, st)); ++launches; mk("gated_group_norm");
         RUN(lin(left_out_, mix_in_, L.r_o, W, vn, W, NVLLM_F32, "retention output projection"));
         pend.a[0] = left_out_; pend.s[0] = 1.0f;

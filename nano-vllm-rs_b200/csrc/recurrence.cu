@@ -21,23 +21,10 @@
 // feeds a projection).
 #include <algorithm>
 
-#include "common.cuh"
+#include "recurrence.cuh"
 
 namespace nvllm {
 namespace {
-
-struct RecArgs {
-  float* y; int64_t ldy;
-  const float *q, *k, *v; int64_t ldq, ldk, ldv;
-  int group_div;                 // head h reads q / k of group h / group_div
-  const float* decay; int64_t decay_ld;   // [n, heads] (decay_ld = heads) or [heads] (decay_ld = 0); per channel: [n, heads * dk], rows decay_ld apart
-  const float* step; int step_ld;     // same, or null (1)
-  const float* skip;                  // [heads] or null (0)
-  float* state;                       // [slots, heads, dk, dv]
-  const int32_t *seq_slot, *cu_tokens; const int64_t* positions;
-  int heads, dk, dv;
-  float q_scale;                      // factor on the read-out (a constant scale of the queries)
-};
 
 constexpr int kRecTile = 16;  // tokens per stage
 
@@ -1000,11 +987,11 @@ extern "C" int nvllm_channel_recurrence(float* y, int64_t ldy, const float* q, i
   return launch_recurrence<true>(a, n_seqs, static_cast<cudaStream_t>(stream));
 }
 
-extern "C" int nvllm_linear_recurrence(float* y, int64_t ldy, const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v,
-                                       int64_t ldv, const float* decay, int32_t decay_per_token, const float* step,
-                                       int32_t step_per_token, const float* skip, float* state, const int32_t* seq_slot,
-                                       const int32_t* cu_tokens, const int64_t* positions, int32_t n_seqs, int32_t heads,
-                                       int32_t groups, int32_t dk, int32_t dv, void* stream) {
+extern "C" int nvllm_linear_recurrence_step(float* y, int64_t ldy, const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v,
+                                            int64_t ldv, const float* decay, int32_t decay_per_token, const float* step,
+                                            int32_t step_per_token, const float* skip, float* state, const int32_t* seq_slot,
+                                            const int32_t* cu_tokens, const int64_t* positions, int32_t n, int32_t n_seqs, int32_t heads,
+                                            int32_t groups, int32_t dk, int32_t dv, void* stream) {
   NVLLM_CHECK_ARG(n_seqs >= 0 && heads > 0 && groups > 0 && heads % groups == 0 && dk > 0 && dk <= 512 && dv > 0, NVLLM_ERR_ARG,
                   "linear_recurrence: seqs=%d heads=%d groups=%d dk=%d (<= 512) dv=%d", n_seqs, heads, groups, dk, dv);
   if (n_seqs == 0) return 0;
@@ -1012,7 +999,17 @@ extern "C" int nvllm_linear_recurrence(float* y, int64_t ldy, const float* q, in
   RecArgs a{y, ldy, q, k, v, ldq, ldk, ldv, heads / groups, decay, decay_per_token ? heads : 0, step, step_per_token ? heads : 0,
             skip, state, seq_slot, cu_tokens, positions, heads, dk, dv, 1.0f};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (linear_recurrence_chunked_applies(a, n_seqs, n)) return linear_recurrence_chunked(a, n_seqs, st);
   return launch_recurrence<false>(a, n_seqs, st);
+}
+
+extern "C" int nvllm_linear_recurrence(float* y, int64_t ldy, const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v,
+                                       int64_t ldv, const float* decay, int32_t decay_per_token, const float* step,
+                                       int32_t step_per_token, const float* skip, float* state, const int32_t* seq_slot,
+                                       const int32_t* cu_tokens, const int64_t* positions, int32_t n_seqs, int32_t heads,
+                                       int32_t groups, int32_t dk, int32_t dv, void* stream) {
+  return nvllm_linear_recurrence_step(y, ldy, q, ldq, k, ldk, v, ldv, decay, decay_per_token, step, step_per_token, skip, state, seq_slot,
+                                      cu_tokens, positions, 0, n_seqs, heads, groups, dk, dv, stream);
 }
 
 extern "C" int nvllm_causal_conv(float* out, int64_t ldo, const float* in, int64_t ldi, const float* w, const float* bias, float* state,

@@ -441,9 +441,9 @@ def linear_recurrence(q, k, v, decay, state, seq_slot, cu_tokens, positions, hea
     decay / step: [n, heads] (per token) or [heads]."""
     n = v.shape[0]
     y = torch.empty((n, heads * dv), dtype=torch.float32, device=v.device)
-    check(_ffi.lib().nvllm_linear_recurrence(_p(y), y.stride(0), _p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(decay),
+    check(_ffi.lib().nvllm_linear_recurrence_step(_p(y), y.stride(0), _p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(decay),
                                              int(decay.dim() == 2), _p(step), int(step is not None and step.dim() == 2), _p(skip),
-                                             _p(state), _p(seq_slot), _p(cu_tokens), _p(positions), seq_slot.shape[0], heads, groups, dk,
+                                             _p(state), _p(seq_slot), _p(cu_tokens), _p(positions), n, seq_slot.shape[0], heads, groups, dk,
                                              dv, _stream()))
     return y
 
