@@ -18,6 +18,7 @@
 // nvllm_attn_norm_rotary_store: a weighted per-head RMS norm before the rotation, values mixed with an earlier layer's.
 // Scores, softmax and the accumulation of P.V are f32.
 #include "common.cuh"
+#include "prefill_attn.cuh"
 
 namespace nvllm {
 namespace {
@@ -1221,6 +1222,13 @@ extern "C" int nvllm_extended_attention(void* out, int64_t ldo, const void* q, i
              keep_first, chunk, head_scale, dist_bias, dist_rows, reinterpret_cast<const float2*>(out_rot_table), max_pos, 0,
              slopes, k_shared, ks_row, shared_dim};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  // bf16 prompts with heads of 128 values and none of the options beyond a window, a cap, a temperature, sinks and a gate: the prompt kernel
+  if (dtype == NVLLM_BF16 && cu_tokens != nullptr && n_seqs > 0 && knobs().capped_mma == 1 && keep_first == 0 && chunk == 0 && head_scale == nullptr &&
+      dist_bias == nullptr && out_rot_table == nullptr && slopes == nullptr && shared_dim == 0) {
+    const PromptAttn e{positions, gate, ldg, gate_per_head, sinks, scale, softcap, temp_coef, temp_every, a.window, n_seqs};
+    if (prompt_attention_applies(e, n, heads, kv_heads, dim, vdim, ldq, k_row, v_row, ldo, out, q, k_cache, v_cache, block_tables != nullptr, block_size))
+      return prompt_attention(e, out, ldo, q, ldq, k_cache, v_cache, k_row, v_row, cu_tokens, block_tables, table_cap, block_size, n, heads, kv_heads, st);
+  }
   // bf16 with 16-byte rows and a token range per sequence: tensor cores; everything else (f32, odd sizes): one warp per row
   const int group = heads / kv_heads;
   if (dtype == NVLLM_BF16 && cu_tokens != nullptr && n_seqs > 0 && knobs().capped_mma && group <= kRows && dim % 8 == 0 && vdim % 8 == 0 &&

@@ -82,7 +82,7 @@ struct Knobs {
   int delta_cfg = 0;        // NVLLM_DELTA_CFG: alternative thread layouts of the gated delta rule for key sizes 65..128
   int latent_unfold = 1;    // NVLLM_LATENT_UNFOLD: 0 = whole prompts of a latent-attention layer also take the folded (multi-query) form
   int linear_mma = 1;       // NVLLM_LINEAR_MMA: 0 = batched / odd-sized bf16 products always on the CUDA-core tile kernel
-  int capped_mma = 1;       // NVLLM_CAPPED_MMA: 0 = capped attention always on the CUDA-core kernel (A/B against the tensor-core one)
+  int capped_mma = 1;       // NVLLM_CAPPED_MMA: 0 = capped attention always on the CUDA-core kernel, 2 = prompts on the mma.sync kernel too (A/B)
   int profile = 0;          // NVLLM_PROFILE: 1 = the runner times every launch of eager steps with CUDA events
   long long comm_timeout_ms = 20000;   // NVLLM_COMM_TIMEOUT_MS: how long a fused TP kernel (or a set-up / tear-down collective) waits for a peer
 };

@@ -17,7 +17,7 @@
 //                       O += P . V (4 x M128 N128 K16 with A = P read from TENSOR MEMORY, V MN-major).  Warps 8, 9 and 11 stay converged, one
 //                       elected lane issues: a diverged one takes over 100 clocks for every copy or MMA, and a converged one 50 to 76
 //                       where the pipe takes 48, hence a warp for each group.
-//   warp 10 (one lane)  claims the next item while this one is worked on
+//   warp 10             claims the next item while this one is worked on
 //   RG threads          tcgen05.ld S row -> row max -> exp2 (MUFU) -> P as packed bf16 written BACK INTO TMEM over the S columns
 //                       (tcgen05.st; each thread only touches its own lane, so no cross-thread hazard) -> mbarrier arrive -> row sum.
 //                       O accumulates in TMEM across tiles; the reference maximum is refreshed lazily (only when a tile exceeds it
@@ -32,6 +32,7 @@
 // and 877 (1.25 PFLOP/s); 32 suffixes behind 2048 shared keys, paged 184 and 132; 64 x 5 47 and 20; 1 x 300 15 and 15.
 #include <type_traits>
 
+#include "prefill_attn.cuh"
 #include "tc.cuh"
 
 namespace nvllm {
@@ -47,9 +48,11 @@ constexpr int kSmemKV = kSmemQ + 2 * kQBytes;
 constexpr int kSmemBar = kSmemKV + NSLOT * kTileBytes;
 constexpr int kNumBars = 2 + 2 * NSLOT + 12 + 4;        // even: what follows lies on 16 bytes
 constexpr int kSmemClaim = kSmemBar + kNumBars * 8;   // 16-byte answer to a claim
-constexpr int kSmemItem = kSmemClaim + 16;            // block index of the next item and whether there is one
-constexpr int kSmemTmem = kSmemItem + 16;
+constexpr int kSmemItem = kSmemClaim + 16;            // the next item and whether there is one
+constexpr int kSmemTmem = kSmemItem + 64;
+constexpr int kSmemGate = kSmemTmem + 16;             // EXT: 4 KiB for each softmax warp
 constexpr int kSmemBytes = kSmemTmem + 16 + 1024;
+constexpr int kSmemBytesExt = kSmemBytes + 8 * 4096;
 constexpr int kThreads = 384;   // 2 softmax warpgroups + 1 warpgroup holding the TMA, claim and two MMA warps
 constexpr int kReaders = 3 + 8; // of the next item: one lane of the TMA warp, the MMA warps and the softmax warps
 static_assert(kSmemClaim % 16 == 0, "the claim's answer is written as 16 bytes");
@@ -67,6 +70,7 @@ struct PrefillParams {
   int z_blocks;
   int64_t out_stride;
   float scale_log2;
+  PromptAttn e;  // EXT only
 };
 
 namespace pf {
@@ -74,6 +78,7 @@ namespace pf {
 struct Item {
   int seq, head[2], first[2], n[2];  // per row group: query head, first row within the sequence's queries, KV tiles
   int kvh, q0, k0, Lq, Lk, n_cta;
+  int kt0;  // EXT: the key tile that tile 0 of the item is
 };
 
 // The item of a block index; false if the sequence has no such rows.
@@ -99,6 +104,48 @@ __device__ __forceinline__ bool decode_item(const PrefillParams& p, int bx, int 
     it.n[g] = it.first[g] >= it.Lq ? 0 : (visible + BN - 1) / BN;
     it.n_cta = max(it.n_cta, it.n[g]);
   }
+  return true;
+}
+
+// EXT: blocks of all sequences in one row (by), the last block of the last sequence first.  A whole converged warp; lane i looks at sequence i of 32.
+__device__ __forceinline__ bool decode_prompt_item(const PrefillParams& p, int bx, int by, Item& it) {
+  const int lane = threadIdx.x & 31, rows = p.pair ? BM : 2 * BM;
+  auto blocks_of = [&](int s) { return s < p.e.n_seqs ? (__ldg(p.cu_q + s + 1) - __ldg(p.cu_q + s) + rows - 1) / rows : 0; };
+  int total = 0;
+  for (int s = lane; s < p.e.n_seqs; s += 32) total += blocks_of(s);
+  int tile = static_cast<int>(__reduce_add_sync(0xffffffffu, static_cast<unsigned>(total))) - 1 - by, qblk = 0;
+  it.n_cta = 0;
+  if (tile < 0) return false;
+  it.seq = -1;
+  for (int s0 = 0; s0 < p.e.n_seqs; s0 += 32) {
+    int end = blocks_of(s0 + lane);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, end, o); end += lane >= o ? v : 0; }
+    const unsigned behind = __ballot_sync(0xffffffffu, tile < end);
+    if (behind != 0u) {
+      const int l = __ffs(behind) - 1, before = __shfl_sync(0xffffffffu, end, l > 0 ? l - 1 : 0);
+      it.seq = s0 + l;
+      qblk = tile - (l > 0 ? before : 0);
+      break;
+    }
+    tile -= __shfl_sync(0xffffffffu, end, 31);
+  }
+  if (it.seq < 0) return false;
+  it.q0 = __ldg(p.cu_q + it.seq);
+  it.Lq = __ldg(p.cu_q + it.seq + 1) - it.q0;
+  it.k0 = it.q0;                              // keys that are not paged are the sequence's own rows
+  it.kvh = (p.pair ? 2 * bx : bx) / (p.H / p.Hkv);
+  const int p0 = static_cast<int>(__ldg(p.e.positions + it.q0 + qblk * rows));
+  it.kt0 = p.e.window > 0 ? max(0, p0 - p.e.window + 1) / BN : 0;
+#pragma unroll
+  for (int g = 0; g < 2; ++g) {
+    it.head[g] = p.pair ? 2 * bx + g : bx;
+    it.first[g] = qblk * rows + (p.pair ? 0 : g * BM);
+    const int last = min(it.first[g] + BM, it.Lq) - 1;
+    it.n[g] = it.first[g] >= it.Lq ? 0 : max(1, static_cast<int>(__ldg(p.e.positions + it.q0 + last)) / BN + 1 - it.kt0);
+    it.n_cta = max(it.n_cta, it.n[g]);
+  }
+  it.Lk = 0;
   return true;
 }
 
@@ -153,6 +200,9 @@ __device__ __forceinline__ void exp_chunk(uint32_t (&s)[32], uint32_t (&pk)[16],
     pk[e] = pack_bf16x2(p0, p1);      // low half = even key: consecutive K elements share a 32-bit column
   }
 }
+// tanh(x) = 1 - 2 / (2^(2 x log2 e) + 1): absolute error ~1e-6, exact at both saturations (as in the kernels of capped_attn.cu)
+__device__ __forceinline__ float ratio_tanh(float x) { return 1.0f - __fdividef(2.0f, fast_exp2(x * 2.8853900817779268f) + 1.0f); }
+
 __device__ __forceinline__ float max3(uint32_t a, uint32_t b, float m) {
   float r;
   asm("max.f32 %0, %1, %2, %3;\n" : "=f"(r) : "f"(__uint_as_float(a)), "f"(__uint_as_float(b)), "f"(m));
@@ -175,6 +225,8 @@ __device__ __forceinline__ uint64_t sum32(const uint32_t (&s)[32], uint64_t acc)
 }
 }  // namespace pf
 
+// EXT: what PromptAttn adds.
+template <bool EXT>
 __global__ void __launch_bounds__(pf::kThreads, 1)
 prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const PrefillParams p) {
@@ -192,7 +244,9 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   auto o_done = [&](int g, int b) { return bars + (2 + 2 * NSLOT + 8 + 2 * g + b) * 8; };   // P.V with buffer b of group g has retired
   const uint32_t item_full = bars + (2 + 2 * NSLOT + 12) * 8, item_empty = item_full + 8, answered = item_full + 16;
   const uint32_t claim = smem_base + kSmemClaim, tmem_slot = smem_base + kSmemTmem;
-  volatile int* item_smem = reinterpret_cast<volatile int*>(smem_gen + kSmemItem);
+  Item* const item_smem = reinterpret_cast<Item*>(smem_gen + kSmemItem);
+  static_assert(sizeof(Item) + 4 <= 64 && kSmemItem % 4 == 0, "an item and a word beside it fit their 64 bytes");
+  int* const item_ok = reinterpret_cast<int*>(item_smem + 1);
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // (uniform: the roles below stay converged)
   if (warp == 8 && lane == 0) {
@@ -211,12 +265,16 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   const uint32_t tmem_base = *reinterpret_cast<uint32_t*>(smem_gen + kSmemTmem);
   pdl_wait();  // q / k / v (and the cache) come from the previous kernel
 
+  auto item_of = [&](int x, int y, int z, Item& it) {
+    if constexpr (EXT) return decode_prompt_item(p, x, y, it);
+    else return decode_item(p, x, y, z, it);
+  };
   // Every role walks the same list of items: its own block index, then what warp 10 publishes.
   uint32_t item_phase = 0;
   auto take_item = [&](Item& it) {       // the item behind a completed item_full
     item_phase ^= 1;
-    const int x = item_smem[0], y = item_smem[1], z = item_smem[2], ok = item_smem[3];
-    return ok != 0 && decode_item(p, x, y, z, it);
+    it = *item_smem;
+    return *reinterpret_cast<volatile int*>(item_ok) != 0;
   };
   auto next_item = [&](Item& it) {       // a whole warp
     mbar_wait(item_full, item_phase);
@@ -228,7 +286,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   // what the control flow and the addresses of a converged warp depend on, as values that are uniform for the compiler too
   auto uni = [](int v) { return static_cast<int>(__reduce_max_sync(0xffffffffu, static_cast<uint32_t>(v))); };
   Item it;
-  const bool own = decode_item(p, blockIdx.x, blockIdx.y, blockIdx.z, it);
+  const bool own = item_of(blockIdx.x, blockIdx.y, blockIdx.z, it);
 
   // Register reallocation (setmaxnreg, per warpgroup): the producer / MMA warpgroup keeps 120 registers per thread and
   // donates the rest: 192 for a softmax thread.
@@ -236,27 +294,31 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     asm volatile("setmaxnreg.dec.sync.aligned.u32 120;\n");  // must dominate the role code below (and only it)
   }
   if (warp == 10) {
-    if (lane == 0) {
-      // ===== claims: one item ahead of the softmax; empty items end here =====
-      // The next claim goes out once every role has read the last item, which no role puts off until another item is done.
-      uint32_t ph = 0, answer_phase = 0;
-      int x, y, z;
-      bool ok = true;
-      while (true) {
-        do {
+    // ===== claims: one item ahead of the softmax; empty items end here, the others go out decoded =====
+    // The next claim goes out once every role has read the last item, which no role puts off until another item is done.
+    uint32_t ph = 0, answer_phase = 0;
+    int x, y, z;
+    bool ok = true;
+    while (true) {
+      do {
+        if (lane == 0) {
           mbar_expect_tx(answered, 16);
           claim_next(claim, answered);
-          mbar_wait(answered, answer_phase);
-          answer_phase ^= 1;
-          ok = claim_read(claim, x, y, z);
-          fence_proxy_async();             // the next answer is written by the async proxy
-        } while (ok && !decode_item(p, x, y, z, it));
-        item_smem[0] = x; item_smem[1] = y; item_smem[2] = z; item_smem[3] = ok;
+        }
+        mbar_wait(answered, answer_phase);
+        answer_phase ^= 1;
+        ok = claim_read(claim, x, y, z);
+        fence_proxy_async();             // the next answer is written by the async proxy
+        __syncwarp();
+      } while (ok && !item_of(x, y, z, it));
+      if (lane == 0) {
+        *item_smem = it;
+        *item_ok = ok;
         mbar_arrive(item_full);
-        if (!ok) break;
-        mbar_wait(item_empty, ph);
-        ph ^= 1;
       }
+      if (!ok) break;
+      mbar_wait(item_empty, ph);
+      ph ^= 1;
     }
   } else if (warp == 8) {
     // ===== TMA producer =====
@@ -264,14 +326,14 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     int t = 0;            // tiles through the ring so far
     uint32_t q_phase = 1; // the first item finds Q's buffer empty
     for (bool more = uni(own) != 0 || uni(next_item(it)) != 0; more; more = uni(next_item(it)) != 0) {
-      const int n_cta = uni(it.n_cta), kvh = uni(it.kvh), k0 = uni(it.k0);
+      const int n_cta = uni(it.n_cta), kvh = uni(it.kvh), kt0 = EXT ? uni(it.kt0) : 0, k0 = uni(it.k0) + kt0 * BN;
       const int32_t* table = p.tables ? p.tables + static_cast<int64_t>(it.seq) * p.max_blocks : nullptr;
       // whole-tile boxes: a lane holds one of 32 consecutive entries of the table, entry `bi` is the present tile's
-      int bi = 0, in_block = 0, entry = -1;
+      int bi = kt0 * BN / p.block_size, in_block = kt0 * BN % p.block_size, entry = -1;
       for (int j = 0; j < n_cta; ++j) {
         int blk = 0;
         if (p.box_tok == BN) {
-          if ((bi & 31) == 0 && in_block == 0) entry = bi + lane < p.max_blocks ? __ldg(table + bi + lane) : -1;
+          if (j == 0 || ((bi & 31) == 0 && in_block == 0)) entry = (bi & ~31) + lane < p.max_blocks ? __ldg(table + (bi & ~31) + lane) : -1;
           blk = __shfl_sync(0xffffffffu, entry, bi & 31);
           blk = uni(blk < 0 ? 0x3fffff : blk);  // past the sequence end: far out of bounds -> TMA zero-fills
         }
@@ -287,7 +349,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             tma_load_5d_warp(dst, map, slot_full(slot), 0, in_block, 0, kvh, blk, el);
           } else {                              // blocks smaller than a tile: a copy for each block and half
             for (int c = 0; c < BN / p.box_tok; ++c) {
-              const int tok = j * BN + c * p.box_tok, b = tok / p.block_size;
+              const int tok = (kt0 + j) * BN + c * p.box_tok, b = tok / p.block_size;
               const int e = b < p.max_blocks ? __ldg(table + b) : -1;
               for (int hf = 0; hf < 2; ++hf)
                 tma_load_5d_warp(dst + hf * (BN * 128) + c * p.box_tok * 128, map, slot_full(slot), 0, tok - b * p.block_size, hf, kvh, uni(e < 0 ? 0x3fffff : e), el);
@@ -398,7 +460,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     const uint32_t tS0 = tmem_base + g * 256 + lane_off;  // two buffers of S (fp32, 64 columns) / P (packed bf16, first 32 columns)
     const uint32_t tO = tS0 + 2 * BN;
     constexpr float kRescaleThreshold = 8.0f;  // log2 units: P stays <= 2^8 between refreshes
-    const uint64_t scale2 = pack2(p.scale_log2, p.scale_log2);
+    const uint64_t scale2 = EXT ? pack2(1.f, 1.f) : pack2(p.scale_log2, p.scale_log2);
     uint32_t tile = 0;                         // tiles of this group so far
     bool more = own;
     while (true) {
@@ -412,11 +474,24 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       more = false;
       const int n_my = g ? it.n[1] : it.n[0], Lk = it.Lk;
       const int row = (g ? it.first[1] : it.first[0]) + t;             // row within the sequence's queries
-      const int vis = min(Lk, Lk - it.Lq + row + 1);       // keys [0, vis) are visible
-      const int vis_lo = min(Lk, Lk - it.Lq + row - lane + 1);   // ... to the warp's first row
+      int vis, vis_lo, from = 0, from_hi = 0;       // keys [from, vis) are visible; vis_lo, from_hi: to all rows of the warp
+      float qscale = 0.f;                           // EXT: factor on the score: over the cap, or to log2 units
+      if constexpr (EXT) {
+        const int pos = static_cast<int>(__ldg(p.e.positions + it.q0 + min(row, it.Lq - 1)));
+        vis = pos + 1;
+        from = p.e.window > 0 ? max(0, pos - p.e.window + 1) : 0;
+        vis_lo = __reduce_min_sync(0xffffffffu, vis);
+        from_hi = __reduce_max_sync(0xffffffffu, from);
+        qscale = p.e.scale * (1.0f + p.e.temp_coef * logf(floorf(static_cast<float>((pos + 1) / p.e.temp_every)) + 1.0f)) *
+                 (p.e.softcap > 0.f ? 1.0f / p.e.softcap : 1.4426950408889634f);
+      } else {
+        vis = min(Lk, Lk - it.Lq + row + 1);
+        vis_lo = min(Lk, Lk - it.Lq + row - lane + 1);
+      }
+      const float to_log2 = EXT ? 1.f : p.scale_log2;   // EXT scores are in log2 units before the maximum
       float m_ref = -INFINITY, l_run = 0.f;  // m_ref: the (stale-by-design) maximum the exponentials are taken against
       for (int j = 0; j < n_my; ++j, ++tile) {
-        const int kbase = j * BN;
+        const int kbase = EXT ? (it.kt0 + j) * BN : j * BN;
         const int b = tile & 1;
         const uint32_t tS = tS0 + b * BN;
         mbar_wait(s_full(g, b), (tile >> 1) & 1);
@@ -426,6 +501,21 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         tmem_ld_32x32b_x32(tS + 32, sr[1]);
         tmem_ld_wait(sr[0]);
         tmem_ld_wait(sr[1]);
+        if constexpr (EXT) {
+          if (p.e.softcap > 0.f) {
+            const float cap2 = p.e.softcap * 1.4426950408889634f;
+#pragma unroll
+            for (int c = 0; c < BN; ++c) sr[c >> 5][c & 31] = __float_as_uint(cap2 * ratio_tanh(__uint_as_float(sr[c >> 5][c & 31]) * qscale));
+          } else {
+#pragma unroll
+            for (int c = 0; c < BN; ++c) sr[c >> 5][c & 31] = __float_as_uint(__uint_as_float(sr[c >> 5][c & 31]) * qscale);
+          }
+          if (from_hi > kbase) {
+#pragma unroll
+            for (int c = 0; c < BN; ++c)
+              if (kbase + c < from) sr[c >> 5][c & 31] = 0xff800000u;  // -inf
+          }
+        }
         if (vis_lo < kbase + BN) {     // some row of the warp has a hidden key in this tile
 #pragma unroll
           for (int c = 0; c < BN; ++c)
@@ -433,10 +523,10 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         }
         const float mx = fmaxf(max32(sr[0]), max32(sr[1]));
         // lazy rescale: refresh the reference maximum only when this tile exceeds it by more than the threshold
-        const bool refresh = (mx - m_ref) * p.scale_log2 > kRescaleThreshold;  // also true for the first finite tile
+        const bool refresh = (mx - m_ref) * to_log2 > kRescaleThreshold;  // also true for the first finite tile
         float corr = 1.f;
         if (refresh) {
-          corr = (m_ref == -INFINITY) ? 0.f : fast_exp2((m_ref - mx) * p.scale_log2);
+          corr = (m_ref == -INFINITY) ? 0.f : fast_exp2((m_ref - mx) * to_log2);
           m_ref = mx;
           l_run *= corr;
         }
@@ -455,7 +545,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             tmem_st_32x32b_x16(tO + c * 16, orr);
           }
         }
-        const float moff = (m_ref == -INFINITY) ? 0.f : -m_ref * p.scale_log2;
+        const float moff = (m_ref == -INFINITY) ? 0.f : -m_ref * to_log2;
         const uint64_t off2 = pack2(moff, moff);
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
@@ -474,13 +564,56 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       if (n_my > 0) {
         mbar_wait(o_done(g, (tile - 1) & 1), ((tile - 1) >> 1) & 1);
         tc_fence_after();
-        const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
-        bf16* orow = p.out + static_cast<int64_t>(it.q0 + row) * p.out_stride + (g ? it.head[1] : it.head[0]) * D;
+        float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
+        const int head = g ? it.head[1] : it.head[0];
+        // EXT: the gate of one head and 32 columns of the warp's rows, read along the rows (8 lanes a row) and passed through shared memory
+        // (the 16-byte piece c of row r lies at c ^ (r & 7))
+        [[maybe_unused]] float4 gate4[8];
+        [[maybe_unused]] uint8_t* const stage = smem_gen + kSmemGate + warp * 4096;
+        [[maybe_unused]] auto load_gate = [&](int c) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int r = row - lane + i * 4 + (lane >> 3);
+            gate4[i] = r < it.Lq ? __ldg(reinterpret_cast<const float4*>(p.e.gate + static_cast<int64_t>(it.q0 + r) * p.e.ldg + head * D + c * 32) + (lane & 7))
+                                 : make_float4(0.f, 0.f, 0.f, 0.f);
+          }
+        };
+        const bool gated = EXT && p.e.gate != nullptr && !p.e.gate_per_head;
+        if constexpr (EXT) {
+          if (p.e.sinks != nullptr) {   // the sink joins the denominator only
+            const float sk = __ldg(p.e.sinks + head) * 1.4426950408889634f, mn = fmaxf(m_ref, sk), oc = fast_exp2(m_ref - mn);
+            const float ll = l_run * oc + fast_exp2(sk - mn);
+            inv = ll > 0.f ? oc / ll : 0.f;
+          }
+          if (p.e.gate != nullptr && p.e.gate_per_head)
+            inv *= 1.0f / (1.0f + __expf(-__ldg(p.e.gate + static_cast<int64_t>(it.q0 + min(row, it.Lq - 1)) * p.e.ldg + head)));
+          if (gated) load_gate(0);
+        }
+        bf16* orow = p.out + static_cast<int64_t>(it.q0 + row) * p.out_stride + head * D;
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
           uint32_t orr[32];
           tmem_ld_32x32b_x32(tO + c * 32, orr);
-          tmem_ld_wait();
+          tmem_ld_wait(orr);
+          if constexpr (EXT) {
+            if (gated) {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const int r = i * 4 + (lane >> 3);
+                *reinterpret_cast<float4*>(stage + r * 128 + (((lane & 7) ^ (r & 7)) * 16)) = gate4[i];
+              }
+              __syncwarp();
+              if (c + 1 < D / 32) load_gate(c + 1);
+#pragma unroll
+              for (int e = 0; e < 8; ++e) {
+                const float4 v = *reinterpret_cast<const float4*>(stage + lane * 128 + ((e ^ (lane & 7)) * 16));
+                const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) orr[4 * e + k] = __float_as_uint(__uint_as_float(orr[4 * e + k]) * (1.0f / (1.0f + __expf(-x[k]))));
+              }
+              __syncwarp();
+            }
+          }
           if (row < it.Lq) {
 #pragma unroll
             for (int e = 0; e < 32; e += 8) {
@@ -504,6 +637,68 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     tc_fence_after();
     tmem_dealloc<512>(tmem_base);
   }
+}
+
+// (64 values, row, half of a head): a head's two halves come in one copy
+static int head_rows_map(CUtensorMap* map, const void* base, int64_t rows, int heads, int64_t ld, int box_rows) {
+  NVLLM_CHECK_ARG(ld % 8 == 0, NVLLM_ERR_ALIGN, "TMA: base must be 16-byte aligned and the row pitch a multiple of 16 bytes");
+  const uint64_t dims[3] = {64, (uint64_t)rows, 2 * (uint64_t)heads}, strides[2] = {(uint64_t)ld * 2, 128};
+  const uint32_t box[3] = {64, (uint32_t)box_rows, 2};
+  return make_tmap_bf16_nd(map, base, 3, dims, strides, box);
+}
+// (64 values, token, half, head, block) of a paged cache
+static int head_blocks_map(CUtensorMap* map, const void* base, int block_size, int kv_heads, int64_t token_stride, int64_t head_stride, int64_t block_stride,
+                           int box_tok) {
+  const uint64_t dims[5] = {64, (uint64_t)block_size, 2, (uint64_t)kv_heads, 0x3fffffull};
+  const uint64_t strides[4] = {(uint64_t)token_stride * 2, 128, (uint64_t)head_stride * 2, (uint64_t)block_stride * 2};
+  const uint32_t box[5] = {64, (uint32_t)box_tok, box_tok == pf::BN ? 2u : 1u, 1, 1};
+  return make_tmap_bf16_nd(map, base, 5, dims, strides, box);
+}
+static bool heads_pair(int heads, int kv_heads) { return (heads / kv_heads) % 2 == 0; }
+
+// From 96 tokens a sequence on: shorter ones leave the 128 rows of a block half empty (16/4 heads, us on mma.sync and here: 32 x 64 capped 37 and
+// 41, windowed 25 and 23; 24 x 130 69 and 67, 43 and 31; 8 x 1024 capped, gate per value 302 and 167, window of 512 180 and 71, dense keys of
+// 16 heads 198 and 76; 8192 tokens capped 1354 and 569).
+bool prompt_attention_applies(const PromptAttn& e, int n, int heads, int kv_heads, int dim, int vdim, int64_t ldq, int64_t k_row, int64_t v_row, int64_t ldo,
+                              const void* out, const void* q, const void* k, const void* v, bool paged, int block_size) {
+  return dim == pf::D && vdim == pf::D && e.n_seqs <= 4096 && n >= 96 * static_cast<int64_t>(e.n_seqs) && ldq % 8 == 0 && k_row % 8 == 0 && v_row % 8 == 0 &&
+         ldo % 8 == 0 && aligned16(out) && aligned16(q) && aligned16(k) && aligned16(v) && heads <= 65535 &&
+         (!paged || (block_size % 16 == 0 && (block_size >= pf::BN ? block_size % pf::BN == 0 : pf::BN % block_size == 0))) &&
+         (e.gate == nullptr || e.gate_per_head || (aligned16(e.gate) && e.ldg % 4 == 0)) && k_row >= static_cast<int64_t>(kv_heads) * dim &&
+         v_row >= static_cast<int64_t>(kv_heads) * vdim;
+}
+
+int prompt_attention(const PromptAttn& e, void* out, int64_t ldo, const void* q, int64_t ldq, const void* k, const void* v, int64_t k_row, int64_t v_row,
+                     const int32_t* cu_tokens, const int32_t* tables, int table_cap, int block_size, int n, int heads, int kv_heads, cudaStream_t st) {
+  CUtensorMap tq, tk, tv;
+  PrefillParams p{};
+  if (int rc = head_rows_map(&tq, q, n, heads, ldq, pf::BM)) return rc;
+  if (tables == nullptr) {
+    if (int rc = head_rows_map(&tk, k, n, kv_heads, k_row, pf::BN)) return rc;
+    if (int rc = head_rows_map(&tv, v, n, kv_heads, v_row, pf::BN)) return rc;
+    p.block_size = 1;
+  } else {
+    p.box_tok = block_size < pf::BN ? block_size : pf::BN;
+    if (int rc = head_blocks_map(&tk, k, block_size, kv_heads, k_row, pf::D, k_row * block_size, p.box_tok)) return rc;
+    if (int rc = head_blocks_map(&tv, v, block_size, kv_heads, v_row, pf::D, v_row * block_size, p.box_tok)) return rc;
+    p.block_size = block_size;
+    p.max_blocks = table_cap;
+  }
+  p.out = static_cast<bf16*>(out);
+  p.cu_q = p.cu_k = cu_tokens;
+  p.tables = tables;
+  p.H = heads;
+  p.Hkv = kv_heads;
+  p.out_stride = ldo;
+  p.e = e;
+  p.pair = heads_pair(heads, kv_heads) ? 1 : 0;
+  p.units = p.pair ? heads / 2 : heads;
+  p.z_blocks = 1;
+  const int rows = p.pair ? pf::BM : 2 * pf::BM;
+  NVLLM_SMEM_ATTR_ONCE(prefill_attn_kernel<true>, pf::kSmemBytesExt);
+  NVLLM_CUDA(launch_plain(prefill_attn_kernel<true>, dim3(p.units, (n + rows - 1) / rows + e.n_seqs), dim3(pf::kThreads), pf::kSmemBytesExt, st, tq, tk, tv, p));
+  NVLLM_LAUNCH_CHECK("prefill_attn_kernel");
+  return 0;
 }
 
 }  // namespace nvllm
@@ -531,20 +726,13 @@ extern "C" int nvllm_varlen_prefill_attention(void* out, const void* q, const vo
                   NVLLM_ERR_ALIGN, "prefill_attention: out alignment / stride");
   const bool paged = block_tables != nullptr;
   CUtensorMap tq, tk, tv;
-  // (64 values, row, half of a head): a head's two halves come in one copy
-  auto rows_map = [](CUtensorMap* map, const void* base, int64_t rows, int heads, int64_t ld, int box_rows) -> int {
-    NVLLM_CHECK_ARG(ld % 8 == 0, NVLLM_ERR_ALIGN, "TMA: base must be 16-byte aligned and the row pitch a multiple of 16 bytes");
-    const uint64_t dims[3] = {64, (uint64_t)rows, 2 * (uint64_t)heads}, strides[2] = {(uint64_t)ld * 2, 128};
-    const uint32_t box[3] = {64, (uint32_t)box_rows, 2};
-    return make_tmap_bf16_nd(map, base, 3, dims, strides, box);
-  };
-  if (int rc = rows_map(&tq, q, total_q, num_heads, q_token_stride, pf::BM)) return rc;
-  PrefillParams p;
+  if (int rc = head_rows_map(&tq, q, total_q, num_heads, q_token_stride, pf::BM)) return rc;
+  PrefillParams p{};
   p.box_tok = 0;
   if (!paged) {
     NVLLM_CHECK_ARG(k && v && total_k > 0, NVLLM_ERR_ARG, "prefill_attention: dense k/v missing");
-    if (int rc = rows_map(&tk, k, total_k, num_kv_heads, kv_token_stride, pf::BN)) return rc;
-    if (int rc = rows_map(&tv, v, total_k, num_kv_heads, kv_token_stride, pf::BN)) return rc;
+    if (int rc = head_rows_map(&tk, k, total_k, num_kv_heads, kv_token_stride, pf::BN)) return rc;
+    if (int rc = head_rows_map(&tv, v, total_k, num_kv_heads, kv_token_stride, pf::BN)) return rc;
     p.block_size = 1;
     p.max_blocks = 0;
   } else {
@@ -557,11 +745,8 @@ extern "C" int nvllm_varlen_prefill_attention(void* out, const void* q, const vo
     NVLLM_CHECK_ARG(bs % 16 == 0 && (bs >= kUnit ? bs % kUnit == 0 : kUnit % bs == 0), NVLLM_ERR_ARG,
                     "prefill_attention: block_size %d must divide or be a multiple of %d", bs, kUnit);
     p.box_tok = bs < pf::BN ? bs : pf::BN;
-    const uint64_t dims[5] = {64, (uint64_t)bs, 2, (uint64_t)num_kv_heads, 0x3fffffull};
-    const uint64_t strides[4] = {(uint64_t)layout->token_stride * 2, 128, (uint64_t)layout->head_stride * 2, (uint64_t)layout->block_stride * 2};
-    const uint32_t box[5] = {64, (uint32_t)p.box_tok, p.box_tok == pf::BN ? 2u : 1u, 1, 1};
-    if (int rc = make_tmap_bf16_nd(&tk, k_cache, 5, dims, strides, box)) return rc;
-    if (int rc = make_tmap_bf16_nd(&tv, v_cache, 5, dims, strides, box)) return rc;
+    if (int rc = head_blocks_map(&tk, k_cache, bs, num_kv_heads, layout->token_stride, layout->head_stride, layout->block_stride, p.box_tok)) return rc;
+    if (int rc = head_blocks_map(&tv, v_cache, bs, num_kv_heads, layout->token_stride, layout->head_stride, layout->block_stride, p.box_tok)) return rc;
     p.block_size = bs;
     p.max_blocks = max_blocks_per_seq;
   }
@@ -573,7 +758,7 @@ extern "C" int nvllm_varlen_prefill_attention(void* out, const void* q, const vo
   p.Hkv = num_kv_heads;
   p.out_stride = out_token_stride;
   p.scale_log2 = scale * 1.4426950408889634f;
-  const bool pair = (num_heads / num_kv_heads) % 2 == 0;
+  const bool pair = heads_pair(num_heads, num_kv_heads);
   p.pair = pair ? 1 : 0;
   p.units = pair ? num_heads / 2 : num_heads;
   const int rows = pair ? pf::BM : 2 * pf::BM;
@@ -581,7 +766,7 @@ extern "C" int nvllm_varlen_prefill_attention(void* out, const void* q, const vo
   p.z_blocks = (blocks + 65534) / 65535;
   (void)max_seqlen_k;
   const dim3 grid(p.units * p.z_blocks, batch, (blocks + p.z_blocks - 1) / p.z_blocks);
-  NVLLM_SMEM_ATTR_ONCE(prefill_attn_kernel, pf::kSmemBytes);
-  NVLLM_CUDA(launch_pdl(prefill_attn_kernel, grid, dim3(pf::kThreads), pf::kSmemBytes, static_cast<cudaStream_t>(stream), tq, tk, tv, p));
+  NVLLM_SMEM_ATTR_ONCE(prefill_attn_kernel<false>, pf::kSmemBytes);
+  NVLLM_CUDA(launch_pdl(prefill_attn_kernel<false>, grid, dim3(pf::kThreads), pf::kSmemBytes, static_cast<cudaStream_t>(stream), tq, tk, tv, p));
   return 0;
 }

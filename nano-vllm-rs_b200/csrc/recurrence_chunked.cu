@@ -419,10 +419,12 @@ __global__ void __launch_bounds__(kWarps * 32, 2) linear_recurrence_chunked_kern
 
 }  // namespace
 
-// From 16 tokens a sequence on: there a chunk, half empty, costs what 16 steps do (32 x 16 tokens: 85 and 83 us, 16 heads of 128 columns 47 and
-// 48); one decoded token costs it 10 times a step.
+// From 40 tokens a sequence on; from 16 on where all CTAs run at once and the steps' latency is what counts.  (32 x 33 tokens, two chunks
+// each: 16 heads of 128 columns 78 us here, 77 token by token; 32 x 16 tokens, 64 heads of 64: 85 and 83; 2 x 40 tokens 21 and 30.)  One decoded
+// token costs a chunk, 10 times a step.
 bool linear_recurrence_chunked_applies(const RecArgs& a, int n_seqs, int n_tokens) {
-  return a.dk == kDk && a.dv % kCols == 0 && static_cast<int64_t>(n_tokens) >= 16 * static_cast<int64_t>(n_seqs) && n_seqs <= 65535 &&
+  const bool at_once = static_cast<int64_t>(a.heads) * n_seqs * (a.dv / kCols) <= sm_count();
+  return a.dk == kDk && a.dv % kCols == 0 && static_cast<int64_t>(n_tokens) >= (at_once ? 16 : 40) * static_cast<int64_t>(n_seqs) && n_seqs <= 65535 &&
          a.ldq % 4 == 0 && a.ldk % 4 == 0 && a.ldy % 2 == 0 && aligned16(a.q) && aligned16(a.k) && aligned16(a.y);
 }
 
