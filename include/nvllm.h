@@ -660,6 +660,12 @@ int nvllm_head_delta_recurrence(float* y, int64_t ldy, const float* q, int64_t l
                                 int64_t ldv, const float* decay, int64_t ldd, const float* beta, int64_t ldb, float* state,
                                 const int32_t* seq_slot, const int32_t* cu_tokens, const int64_t* positions, int32_t n_seqs,
                                 int32_t heads, int32_t groups, int32_t dk, int32_t dv, void* stream);
+/* Both delta rules for a caller that knows how many tokens the batch holds (n; 0: not known): prompts are taken 16 tokens at a time as
+ * matrix products.  head_decay != 0: one decay per head (decay [n, heads]), else one per key channel. */
+int nvllm_delta_recurrence_step(float* y, int64_t ldy, const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v,
+                                int64_t ldv, const float* decay, int64_t ldd, int32_t head_decay, const float* beta, int64_t ldb,
+                                float* state, const int32_t* seq_slot, const int32_t* cu_tokens, const int64_t* positions,
+                                int32_t n, int32_t n_seqs, int32_t heads, int32_t groups, int32_t dk, int32_t dv, void* stream);
 /* Gated linear attention (sequence / slot conventions of nvllm_linear_recurrence): per head S <- diag(decay_t) S + k_t v_t^T,
  * y_t = q_scale S^T q_t.  decay: f32 [n, heads * dk], rows ldd apart.  dk <= 512. */
 int nvllm_channel_recurrence(float* y, int64_t ldy, const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v,

@@ -140,6 +140,8 @@ PROTOTYPES = {
     "nvllm_head_delta_prepare": (i32, [vp, i64, vp, i64, vp, i64, vp, i64, vp, vp, i32, i32, i32, i32, f32, f32, vp]),
     "nvllm_head_delta_recurrence": (i32, [vp, i64, vp, i64, vp, i64, vp, i64, vp, i64, vp, i64, vp, vp, vp, vp, i32, i32, i32, i32, i32,
                                           vp]),
+    "nvllm_delta_recurrence_step": (i32, [vp, i64, vp, i64, vp, i64, vp, i64, vp, i64, i32, vp, i64, vp, vp, vp, vp, i32, i32, i32, i32, i32,
+                                          i32, vp]),
     "nvllm_channel_recurrence": (i32, [vp, i64, vp, i64, vp, i64, vp, i64, vp, i64, f32, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp]),
     "nvllm_low_rank_decay": (i32, [vp, i64, vp, i64, vp, vp, i32, i32, i32, f32, vp]),
     "nvllm_gemm_glu_bf16": (i32, [vp, vp, vp, i32, i32, i32, i64, i64, i64, f32, vp, sz, vp]),

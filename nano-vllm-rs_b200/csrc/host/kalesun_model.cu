@@ -503,8 +503,8 @@ class Kalesun : public ModelBase {
                               st)); launches += L.taps > 1 ? 1 : 0; mk("causal_conv");
         RUN(nvllm_head_delta_prepare(conv_out_, qkv, conv_out_ + qc, qkv, beta, ld, dec, ld, L.a_log, L.dt_bias, N, L.H, L.G, L.D,
                                      1.0f / sqrtf(static_cast<float>(L.D)), 1e-6f, st)); mk("head_delta_prepare");
-        RUN(nvllm_head_delta_recurrence(y_, HV, conv_out_, qkv, conv_out_ + qc, qkv, conv_out_ + qc + kc, qkv, dec, ld, beta, ld, ls.S, v.seq_slots,
-                                        v.cu_tokens, v.positions, S, L.H, L.G, L.D, L.V, st)); mk("head_delta_recurrence");
+        RUN(nvllm_delta_recurrence_step(y_, HV, conv_out_, qkv, conv_out_ + qc, qkv, conv_out_ + qc + kc, qkv, dec, ld, 1, beta, ld, ls.S, v.seq_slots,
+                                        v.cu_tokens, v.positions, N, S, L.H, L.G, L.D, L.V, st)); mk("head_delta_recurrence");
         RUN(nvllm_gated_group_norm_act(mix_in_, HV, y_, HV, gate, ld, L.o_norm, 1, N, HV, L.H, eps_, 0, 0, dt_, st)); mk("gated_group_norm");
       } else {
         // [q | k | v | g | a1]; the second decay step; the recurrence; gated per-head norm

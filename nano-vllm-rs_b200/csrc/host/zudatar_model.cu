@@ -619,8 +619,8 @@ class Zudatar : public ModelImpl {
                               L.taps, 1, st)); launches += L.taps > 1 ? 2 : 1; mk("causal_conv");
         RUN(nvllm_delta_prepare(conv_out_, ch, conv_out_ + GD, ch, proj_ + ch, ldd, decay_, HD, L.a_log, L.dt_bias, N, L.H, L.G, L.D,
                                 1.0f / sqrtf(static_cast<float>(L.D)), 1e-6f, st)); ++launches; mk("delta_prepare");
-        RUN(nvllm_gated_delta_recurrence(y_, HV, conv_out_, ch, conv_out_ + GD, ch, conv_out_ + 2 * GD, ch, decay_, HD, proj_ + ch, ldd, ls.S,
-                                         v.seq_slots, v.cu_tokens, v.positions, S, L.H, L.G, L.D, L.V, st)); ++launches; mk("gated_delta_recurrence");
+        RUN(nvllm_delta_recurrence_step(y_, HV, conv_out_, ch, conv_out_ + GD, ch, conv_out_ + 2 * GD, ch, decay_, HD, 0, proj_ + ch, ldd, ls.S,
+                                        v.seq_slots, v.cu_tokens, v.positions, N, S, L.H, L.G, L.D, L.V, st)); ++launches; mk("gated_delta_recurrence");
         RUN(nvllm_gated_group_norm_act(mix_in_, HV, y_, HV, gate_, HV, L.o_norm, 1, N, HV, L.H, eps_, 0, 1, dt_, st)); ++launches; mk("gated_group_norm");
       }
       RUN(lin(sub_out_, mix_in_, L.o, W, HV, HV, W, dt_, "mixer output projection"));

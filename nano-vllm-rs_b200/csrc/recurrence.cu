@@ -174,17 +174,6 @@ __global__ void __launch_bounds__(512) linear_recurrence_kernel(const RecArgs a,
 }
 
 
-struct DeltaArgs {
-  float* y; int64_t ldy;
-  const float *q, *k, *v; int64_t ldq, ldk, ldv;
-  int group_div;                       // head h reads q / k of group h / group_div
-  const float* decay; int64_t ldd;     // [n, heads * dk]: decay of every key channel; HEADG: [n, heads]
-  const float* beta; int64_t ldb;      // [n, heads]
-  float* state;                        // [slots, heads, dk, dv]
-  const int32_t *seq_slot, *cu_tokens; const int64_t* positions;
-  int heads, dk, dv;
-};
-
 // The gated delta rule, laid out as linear_recurrence_kernel (CTA = (head, sequence, slice of dv); a thread keeps PP columns x NPT
 // rows of S in registers, NSL row slices of a column in neighbouring lanes; kRecTile tokens staged with cp.async two stages
 // deep).  Per token one pass over the registers decays S and accumulates both S^T k and S^T q of the DECAYED state; after the
@@ -949,29 +938,34 @@ extern "C" int nvllm_low_rank_decay(float* out, int64_t ldo, const float* x, int
   return 0;
 }
 
+extern "C" int nvllm_delta_recurrence_step(float* y, int64_t ldy, const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v,
+                                           int64_t ldv, const float* decay, int64_t ldd, int32_t head_decay, const float* beta, int64_t ldb,
+                                           float* state, const int32_t* seq_slot, const int32_t* cu_tokens, const int64_t* positions, int32_t n,
+                                           int32_t n_seqs, int32_t heads, int32_t groups, int32_t dk, int32_t dv, void* stream) {
+  NVLLM_CHECK_ARG(n_seqs >= 0 && heads > 0 && groups > 0 && heads % groups == 0 && dk > 0 && dk <= 512 && dv > 0, NVLLM_ERR_ARG,
+                  "delta_recurrence: seqs=%d heads=%d groups=%d dk=%d (<= 512) dv=%d", n_seqs, heads, groups, dk, dv);
+  if (n_seqs == 0) return 0;
+  NVLLM_CHECK_ARG(y && q && k && v && decay && beta && state && seq_slot && cu_tokens && positions, NVLLM_ERR_ARG, "delta_recurrence: NULL");
+  const DeltaArgs a{y, ldy, q, k, v, ldq, ldk, ldv, heads / groups, decay, ldd, beta, ldb, state, seq_slot, cu_tokens, positions, heads, dk, dv};
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (delta_chunked_applies(a, head_decay != 0, n_seqs, n)) return delta_chunked(a, head_decay != 0, n_seqs, st);
+  return head_decay ? launch_delta<true>(a, n_seqs, st) : launch_delta<false>(a, n_seqs, st);
+}
+
 extern "C" int nvllm_gated_delta_recurrence(float* y, int64_t ldy, const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v,
                                             int64_t ldv, const float* decay, int64_t ldd, const float* beta, int64_t ldb, float* state,
                                             const int32_t* seq_slot, const int32_t* cu_tokens, const int64_t* positions, int32_t n_seqs,
                                             int32_t heads, int32_t groups, int32_t dk, int32_t dv, void* stream) {
-  NVLLM_CHECK_ARG(n_seqs >= 0 && heads > 0 && groups > 0 && heads % groups == 0 && dk > 0 && dk <= 512 && dv > 0, NVLLM_ERR_ARG,
-                  "gated_delta_recurrence: seqs=%d heads=%d groups=%d dk=%d (<= 512) dv=%d", n_seqs, heads, groups, dk, dv);
-  if (n_seqs == 0) return 0;
-  NVLLM_CHECK_ARG(y && q && k && v && decay && beta && state && seq_slot && cu_tokens && positions, NVLLM_ERR_ARG, "gated_delta_recurrence: NULL");
-  DeltaArgs a{y, ldy, q, k, v, ldq, ldk, ldv, heads / groups, decay, ldd, beta, ldb, state, seq_slot, cu_tokens, positions, heads, dk, dv};
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  return launch_delta<false>(a, n_seqs, st);
+  return nvllm_delta_recurrence_step(y, ldy, q, ldq, k, ldk, v, ldv, decay, ldd, 0, beta, ldb, state, seq_slot, cu_tokens, positions, 0, n_seqs, heads,
+                                     groups, dk, dv, stream);
 }
 
 extern "C" int nvllm_head_delta_recurrence(float* y, int64_t ldy, const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v,
                                            int64_t ldv, const float* decay, int64_t ldd, const float* beta, int64_t ldb, float* state,
                                            const int32_t* seq_slot, const int32_t* cu_tokens, const int64_t* positions, int32_t n_seqs,
                                            int32_t heads, int32_t groups, int32_t dk, int32_t dv, void* stream) {
-  NVLLM_CHECK_ARG(n_seqs >= 0 && heads > 0 && groups > 0 && heads % groups == 0 && dk > 0 && dk <= 512 && dv > 0, NVLLM_ERR_ARG,
-                  "head_delta_recurrence: seqs=%d heads=%d groups=%d dk=%d (<= 512) dv=%d", n_seqs, heads, groups, dk, dv);
-  if (n_seqs == 0) return 0;
-  NVLLM_CHECK_ARG(y && q && k && v && decay && beta && state && seq_slot && cu_tokens && positions, NVLLM_ERR_ARG, "head_delta_recurrence: NULL");
-  const DeltaArgs a{y, ldy, q, k, v, ldq, ldk, ldv, heads / groups, decay, ldd, beta, ldb, state, seq_slot, cu_tokens, positions, heads, dk, dv};
-  return launch_delta<true>(a, n_seqs, static_cast<cudaStream_t>(stream));
+  return nvllm_delta_recurrence_step(y, ldy, q, ldq, k, ldk, v, ldv, decay, ldd, 1, beta, ldb, state, seq_slot, cu_tokens, positions, 0, n_seqs, heads,
+                                     groups, dk, dv, stream);
 }
 
 extern "C" int nvllm_channel_recurrence(float* y, int64_t ldy, const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v,

@@ -1,4 +1,4 @@
-// recurrence.cuh — the arguments of a linear recurrence, shared by its two kernels (recurrence.cu, recurrence_chunked.cu).
+// recurrence.cuh — the arguments of the recurrences, shared by their kernels (recurrence.cu; for prompts recurrence_chunked.cu, delta_chunked.cu).
 #pragma once
 
 #include "common.cuh"
@@ -21,5 +21,20 @@ struct RecArgs {
 // recurrence_chunked.cu: takes a recurrence with one decay per head if the sizes and the alignment suit it.
 bool linear_recurrence_chunked_applies(const RecArgs& a, int n_seqs, int n_tokens);
 int linear_recurrence_chunked(const RecArgs& a, int n_seqs, cudaStream_t st);
+
+struct DeltaArgs {
+  float* y; int64_t ldy;
+  const float *q, *k, *v; int64_t ldq, ldk, ldv;
+  int group_div;                       // head h reads q / k of group h / group_div
+  const float* decay; int64_t ldd;     // [n, heads * dk]: decay of every key channel; HEADG: [n, heads]
+  const float* beta; int64_t ldb;      // [n, heads]
+  float* state;                        // [slots, heads, dk, dv]
+  const int32_t *seq_slot, *cu_tokens; const int64_t* positions;
+  int heads, dk, dv;
+};
+
+// delta_chunked.cu: takes a gated delta rule (a decay per key channel, or one per head) if the sizes and the alignment suit it.
+bool delta_chunked_applies(const DeltaArgs& a, bool head_decay, int n_seqs, int n_tokens);
+int delta_chunked(const DeltaArgs& a, bool head_decay, int n_seqs, cudaStream_t st);
 
 }  // namespace nvllm

@@ -9,7 +9,7 @@
 // chunk and are added to the state in f32, so that the state is rounded once per 32 tokens instead of 32 times.  (Two fp16 values
 // and three products would need half the instructions, but their 22-bit products meet the truncation: 4.5e-7 from 64 bits.)  Relative
 // error of y and of the state against 64 bits, token by token and here: retention of 1024 tokens 2.3e-7, 2.1e-7 and 1.0e-7, 0.8e-7;
-// state-space duality 0.80e-7, 0.69e-7 and 0.82e-7, 0.71e-7.
+// state-space duality 0.80e-7, 0.69e-7 and 0.68e-7, 0.65e-7.
 // A chunk with a value that is no number, infinite, or far from the others' range (rows of q and k outside 2^-60 .. 2^40) is stepped
 // through token by token in f32 instead, by the warps that it concerns: what such a value reaches is then the same as there.
 //
@@ -20,14 +20,12 @@
 // around it; two CTAs an SM (91 KB each) hide each other's barriers.
 // Token by token and here (us): 16 heads of 128 x 128, 8 x 1024 tokens 551 and 296, 8192 tokens 3235 and 1730; 64 heads of 128 x 64, 8 x 1024
 // 876 and 575, 2 x 40 30 and 21, 32 x 16 83 and 85.
-#include "recurrence.cuh"
+#include "split_mma.cuh"
 
 namespace nvllm {
 namespace {
 
-__device__ __forceinline__ void cp_async_4(uint32_t smem_addr, const void* gptr) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(smem_addr), "l"(gptr) : "memory");
-}
+using namespace split;
 
 constexpr int kC = 32, kDk = 128, kCols = 64, kWarps = 4;
 constexpr int kRow = kDk * 2 + 16;               // bytes of a row of pieces: 16 more, so that ldmatrix rows fall into different banks
@@ -39,53 +37,6 @@ constexpr int kSmK = kSmQ + 3 * kPiece;
 constexpr int kSmP = kSmK + 3 * kPiece;          // D_ij, overwritten in place by the middle factor
 constexpr int kSmVec = kSmP + kC * kPs * 4;      // floats: pre, w [32 each], a [2][32], b [2][32], flag, low part of the product of all decays
 constexpr int kSmBytes = kSmVec + 6 * kC * 4 + 16;
-
-__device__ __forceinline__ uint32_t abs_bits(float x) { return __float_as_uint(x) & 0x7fffffffu; }
-
-// max(|a|, |b|, m), no number if one of them is none
-__device__ __forceinline__ float abs_max(float a, float b, float m) {
-  float r;
-  asm("max.NaN.f32 %0, %1, %2, %3;\n" : "=f"(r) : "f"(fabsf(a)), "f"(fabsf(b)), "f"(m));
-  return r;
-}
-__device__ __forceinline__ bool far_off(uint32_t bits, int lo, int hi) {   // not zero and outside [2^lo, 2^hi)
-  return bits != 0u && (bits < (static_cast<uint32_t>(127 + lo) << 23) || bits >= (static_cast<uint32_t>(127 + hi) << 23));
-}
-// (x0, x1) -> three bf16 pairs, hi + mid + lo = x to 2^-25 of it
-__device__ __forceinline__ void split3(float x0, float x1, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  hi = pack_bf16x2(x0, x1);
-  x0 -= bf16_lo(hi);
-  x1 -= bf16_hi(hi);
-  mid = pack_bf16x2(x0, x1);
-  lo = pack_bf16x2(x0 - bf16_lo(mid), x1 - bf16_hi(mid));
-}
-// (not volatile: the compiler may interleave independent accumulators)
-__device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-template <int M, int N>
-__device__ __forceinline__ void zero(float (&d)[M][N][4]) {
-#pragma unroll
-  for (int m = 0; m < M; ++m)
-#pragma unroll
-    for (int n = 0; n < N; ++n)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) d[m][n][i] = 0.f;
-}
-// The six products of M tiles (16 x 16) of A with N tiles (16 x 8) of B (a[tile][piece], b[piece][tile][half]): hi.hi into dh, the others into
-// dl.  An accumulator comes up again after M x N others at the least: dependent ones are about four issues apart.
-template <int M, int N>
-__device__ __forceinline__ void mma6(float (&dh)[M][N][4], float (&dl)[M][N][4], const uint32_t (&a)[M][3][4], const uint32_t (&b)[3][N][2]) {
-  constexpr int order[6][2] = {{2, 0}, {0, 2}, {0, 0}, {1, 1}, {1, 0}, {0, 1}};
-#pragma unroll
-  for (int i = 0; i < 6; ++i)
-#pragma unroll
-    for (int m = 0; m < M; ++m)
-#pragma unroll
-      for (int n = 0; n < N; ++n) mma(i == 2 ? dh[m][n] : dl[m][n], a[m][order[i][0]], b[order[i][1]][n][0], b[order[i][1]][n][1]);
-}
 
 __global__ void __launch_bounds__(kWarps * 32, 2) linear_recurrence_chunked_kernel(const RecArgs a) {
   pdl_wait();
@@ -267,7 +218,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) linear_recurrence_chunked_kern
         for (int i = 0; i < 4; ++i) {
           const int row = mt * 16 + r + (i >> 1) * 8, key = nt * 16 + n * 8 + c2 + (i & 1);
           float* m = mid + row * kPs + key;
-          *m = fmaf((sum[n][i] + (al[0][0][n][i] + al[1][0][n][i])) * bs[key], *m, row == key ? d : 0.f);      // D is zero above the diagonal
+          *m = fmaf(join(sum[n][i], al[0][0][n][i] + al[1][0][n][i]) * bs[key], *m, row == key ? d : 0.f);      // D is zero above the diagonal
         }
     }
     // v and the state: their largest magnitude decides whether the warp takes the products
@@ -312,7 +263,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) linear_recurrence_chunked_kern
 #pragma unroll
         for (int n = 0; n < 2; ++n)
 #pragma unroll
-          for (int i = 0; i < 4; ++i) yi[m][n][i] += yl[m][n][i];
+          for (int i = 0; i < 4; ++i) yi[m][n][i] = join(yi[m][n][i], yl[m][n][i]);
     }
     uint32_t vf[2][3][2][2];           // v as B: [token step][piece][8 columns][half of the 16 tokens]
 #pragma unroll
@@ -344,7 +295,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) linear_recurrence_chunked_kern
 #pragma unroll
             for (int n = 0; n < 2; ++n)
               *reinterpret_cast<float2*>(yh + t * a.ldy + n * 8 + c2) =
-                  make_float2(fmaf(yi[m][n][2 * e], fi, ah[0][n][2 * e] + al[0][n][2 * e]), fmaf(yi[m][n][2 * e + 1], fi, ah[0][n][2 * e + 1] + al[0][n][2 * e + 1]));
+                  make_float2(fmaf(yi[m][n][2 * e], fi, join(ah[0][n][2 * e], al[0][n][2 * e])), fmaf(yi[m][n][2 * e + 1], fi, join(ah[0][n][2 * e + 1], al[0][n][2 * e + 1])));
           }
         }
       }
@@ -377,7 +328,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) linear_recurrence_chunked_kern
 #pragma unroll
         for (int n = 0; n < 4; ++n)
 #pragma unroll
-          for (int i = 0; i < 4; ++i) S[4 * np + n][i] = fmaf(S[4 * np + n][i], at, fmaf(S[4 * np + n][i], at_lo, (ah[0][0][n][i] + ah[1][0][n][i]) + al[0][n][i]));
+          for (int i = 0; i < 4; ++i) S[4 * np + n][i] = fmaf(S[4 * np + n][i], at, fmaf(S[4 * np + n][i], at_lo, join(ah[0][0][n][i] + ah[1][0][n][i], al[0][n][i])));
       }
     } else {
       // ---- token by token, as the general kernel does it ---------------------------------------------------------------

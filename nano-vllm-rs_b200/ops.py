@@ -560,9 +560,9 @@ def gated_delta_recurrence(q, k, v, decay, beta, state, seq_slot, cu_tokens, pos
     """S <- diag(g) S, u = beta (v - S^T k), S <- S + k u^T, y = S^T q over the sequences of a step; state [slots, heads, dk, dv]."""
     n = v.shape[0]
     y = torch.empty((n, heads * dv), dtype=torch.float32, device=v.device)
-    check(_ffi.lib().nvllm_gated_delta_recurrence(_p(y), y.stride(0), _p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(decay),
-                                                  decay.stride(0), _p(beta), beta.stride(0), _p(state), _p(seq_slot), _p(cu_tokens),
-                                                  _p(positions), seq_slot.shape[0], heads, groups, dk, dv, _stream()))
+    check(_ffi.lib().nvllm_delta_recurrence_step(_p(y), y.stride(0), _p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(decay),
+                                                 decay.stride(0), 0, _p(beta), beta.stride(0), _p(state), _p(seq_slot), _p(cu_tokens),
+                                                 _p(positions), n, seq_slot.shape[0], heads, groups, dk, dv, _stream()))
     return y
 
 
@@ -716,9 +716,9 @@ def head_delta_recurrence(q, k, v, decay, beta, state, seq_slot, cu_tokens, posi
     """gated_delta_recurrence with one decay per head: decay [n, heads]."""
     n = v.shape[0]
     y = torch.empty((n, heads * dv), dtype=torch.float32, device=v.device)
-    check(_ffi.lib().nvllm_head_delta_recurrence(_p(y), y.stride(0), _p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(decay),
-                                                 decay.stride(0), _p(beta), beta.stride(0), _p(state), _p(seq_slot), _p(cu_tokens),
-                                                 _p(positions), seq_slot.shape[0], heads, groups, dk, dv, _stream()))
+    check(_ffi.lib().nvllm_delta_recurrence_step(_p(y), y.stride(0), _p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(decay),
+                                                 decay.stride(0), 1, _p(beta), beta.stride(0), _p(state), _p(seq_slot), _p(cu_tokens),
+                                                 _p(positions), n, seq_slot.shape[0], heads, groups, dk, dv, _stream()))
     return y
 
 

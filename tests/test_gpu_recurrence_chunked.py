@@ -1,4 +1,4 @@
-"""-m gpu tests of the linear recurrence's kernel for prompts (32 tokens at a time as matrix products) against the token-by-token
+"""-m gpu tests of the recurrences' kernels for prompts (32 or 16 tokens at a time as matrix products) against the token-by-token
 recurrence in float64."""
 import numpy as np
 import pytest
@@ -100,3 +100,93 @@ def test_odd_values(cuda, what):
     st = state.cpu().numpy()
     for i in range(2):
         _check(seqs[i], np.zeros((heads, DK, dv)), ys[i], st[i], heads, groups, np.zeros(heads))
+
+
+# ------------------------------------------------------------------------------------------------------------ the gated delta rule
+def _delta_reference(q, k, v, g, b, S):
+    """One sequence in float64: y, the final state, and the largest column norm that the state had (the error's scale)."""
+    n, H, dv = v.shape
+    y, S, top = np.empty_like(v), S.copy(), np.zeros((H, dv))
+    with np.errstate(all="ignore"):
+        for t in range(n):
+            S = g[t][:, :, None] * S
+            u = b[t][:, None] * (v[t] - np.einsum("hkv,hk->hv", S, k[t]))
+            S = S + k[t][:, :, None] * u[:, None, :]
+            y[t] = np.einsum("hkv,hk->hv", S, q[t])
+            top = np.fmax(top, np.sqrt((S * S).sum(1)))
+    return y, S, top
+
+
+def _delta_seq(rng, n, heads, groups, dv, head_decay, lo=0.5):
+    f = lambda x: np.asarray(x, np.float32)
+    unit = lambda x: x / np.sqrt((x * x).sum(-1, keepdims=True))
+    return {"q": f(unit(rng.standard_normal((n, groups, DK)))), "k": f(unit(rng.standard_normal((n, groups, DK)))), "v": f(rng.standard_normal((n, heads, dv))),
+            "g": f(rng.uniform(lo, 1.0, (n, heads, 1 if head_decay else DK))), "b": f(rng.uniform(0.1, 1.0, (n, heads)))}
+
+
+def _delta_run(cuda, seqs, heads, groups, dv, state, starts, head_decay):
+    from nano_vllm_rs_b200 import ops
+    cat = lambda x: torch.from_numpy(np.concatenate([s[x].reshape(len(s["v"]), -1) for s in seqs])).to(cuda)
+    lens = [len(s["v"]) for s in seqs]
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32, device=cuda)
+    pos = torch.cat([torch.arange(p, p + n) for p, n in zip(starts, lens)]).to(cuda)
+    slots = torch.arange(len(seqs), dtype=torch.int32, device=cuda)
+    fn = ops.head_delta_recurrence if head_decay else ops.gated_delta_recurrence
+    y = fn(cat("q"), cat("k"), cat("v"), cat("g"), cat("b"), state, slots, cu, pos, heads, groups, DK, dv)
+    return np.split(y.cpu().numpy().reshape(-1, heads, dv), np.cumsum(lens)[:-1])
+
+
+def _delta_check(seq, S0, got, state, heads, groups, tokens):
+    """With unit keys and beta <= 1 a step never enlarges an error that the state carries, so the errors of the tokens so far add up at the
+    worst; each is a handful (16 are allowed) of roundings of 2^-24 on the scale of a state's column."""
+    w = {x: s.astype(np.float64) for x, s in seq.items()}
+    rep = heads // groups
+    y, S, top = _delta_reference(w["q"].repeat(rep, 1), w["k"].repeat(rep, 1), w["v"], np.broadcast_to(w["g"], w["g"].shape[:2] + (DK,)), w["b"], S0)
+    tol = tokens * 16 * 2.0 ** -24 * np.where(np.isfinite(top), np.maximum(top, 1e-30), 1.0)
+    np.testing.assert_array_equal(np.isfinite(got), np.isfinite(y))
+    ok = np.isfinite(y)
+    with np.errstate(invalid="ignore"):
+        assert (np.abs(got - y)[ok] <= np.broadcast_to(tol, y.shape)[ok]).all(), np.max((np.abs(got - y) / tol)[ok])
+        ok = np.isfinite(S)
+        np.testing.assert_array_equal(np.isfinite(state), ok)
+        assert (np.abs(state - S)[ok] <= np.broadcast_to(tol[:, None], S.shape)[ok]).all()
+
+
+@pytest.mark.parametrize("heads,groups,dv,lens,head_decay,lo", [
+    (2, 2, 64, [16], False, 0.5), (4, 2, 64, [31, 1, 64], False, 0.9), (8, 1, 64, [17, 97], True, 0.5), (3, 3, 128, [33, 130], False, 0.02), (2, 1, 192, [65, 40], True, 0.99)])
+def test_delta_prompts_and_portions(cuda, heads, groups, dv, lens, head_decay, lo):
+    """Chunk edges and tails, single tokens beside prompts, decays from next to nothing to next to one, a second portion that goes on from the slots."""
+    rng = np.random.default_rng(sum(lens) + dv)
+    state = torch.full((len(lens), heads, DK, dv), 7.0, device=cuda)
+    S = [np.zeros((heads, DK, dv))] * len(lens)
+    for portion in range(2):
+        seqs = [_delta_seq(rng, n, heads, groups, dv, head_decay, lo) for n in lens]
+        ys = _delta_run(cuda, seqs, heads, groups, dv, state, [portion * n for n in lens], head_decay)
+        st = state.cpu().numpy()
+        for i, (q, y) in enumerate(zip(seqs, ys)):
+            _delta_check(q, S[i], y, st[i], heads, groups, lens[i])
+        S = [st[i].astype(np.float64) for i in range(len(lens))]
+
+
+@pytest.mark.parametrize("what", ["v nan", "v inf", "k nan", "q inf", "g zero", "g above one", "g nan", "beta nan", "k large", "all zero"])
+def test_delta_odd_values(cuda, what):
+    heads, groups, dv, n, at = 4, 2, 64, 60, 21
+    rng = np.random.default_rng(9)
+    seqs = [_delta_seq(rng, n, heads, groups, dv, False), _delta_seq(rng, n, heads, groups, dv, False)]
+    s = seqs[0]
+    if what == "v nan": s["v"][at, 1, 5] = np.nan
+    elif what == "v inf": s["v"][at, 1, 5] = np.inf
+    elif what == "k nan": s["k"][at, 0, 3] = np.nan
+    elif what == "q inf": s["q"][at, 1, 9] = np.inf
+    elif what == "g zero": s["g"][at] = 0.0
+    elif what == "g above one": s["g"][at] = 1.25
+    elif what == "g nan": s["g"][at, 2, 7] = np.nan
+    elif what == "beta nan": s["b"][at, 0] = np.nan
+    elif what == "k large": s["k"][n - 1] *= np.float32(2.0 ** 40)
+    else:
+        for x in "qkv": s[x][:] = 0.0
+    state = torch.zeros((2, heads, DK, dv), device=cuda)
+    ys = _delta_run(cuda, seqs, heads, groups, dv, state, [0, 0], False)
+    st = state.cpu().numpy()
+    for i in range(2):
+        _delta_check(seqs[i], np.zeros((heads, DK, dv)), ys[i], st[i], heads, groups, n)
