@@ -88,6 +88,55 @@ add_rmsnorm_kernel(bf16* __restrict__ out, const bf16* __restrict__ x, bf16* __r
   }
 }
 
+// The same with a warp per row, for batches of rows of up to 1024 values: all of a row's 16-byte pieces (four per lane) are requested at
+// once and the sum needs no barrier.  Back to back on rows that stay in L2, with a CTA per row and so: 13.4 K x 1024 15.0 -> 10.1 us (without
+// a residual 14.5 -> 6.5), 2400 x 1024 4.6 -> 4.1.  Rows of 2048 (eight pieces per lane) took 18.2 -> 19.3 at 8192 rows, so those keep the CTA.
+template <bool HAS_RES>
+__global__ void __launch_bounds__(256)
+add_rmsnorm_rows_kernel(bf16* __restrict__ out, const bf16* __restrict__ x, bf16* __restrict__ residual, const bf16* __restrict__ weight, int rows, int hidden,
+                        float eps) {
+  constexpr int NV = 4;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, nvec = hidden >> 3;
+  if (row >= rows) return;
+  const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<int64_t>(row) * hidden);
+  uint4* rr = HAS_RES ? reinterpret_cast<uint4*>(residual + static_cast<int64_t>(row) * hidden) : nullptr;
+  uint4 a[NV], r[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const bool in = lane + 32 * k < nvec;
+    a[k] = in ? xr[lane + 32 * k] : make_uint4(0, 0, 0, 0);
+    if (HAS_RES) r[k] = in ? rr[lane + 32 * k] : make_uint4(0, 0, 0, 0);
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    uint32_t u[4] = {a[k].x, a[k].y, a[k].z, a[k].w};
+    if (HAS_RES) {
+      const uint32_t w[4] = {r[k].x, r[k].y, r[k].z, r[k].w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) u[j] = pack_bf16x2(bf16_lo(u[j]) + bf16_lo(w[j]), bf16_hi(u[j]) + bf16_hi(w[j]));   // bf16 tensor add
+      a[k] = make_uint4(u[0], u[1], u[2], u[3]);
+      if (lane + 32 * k < nvec) rr[lane + 32 * k] = a[k];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) ss += bf16_lo(u[j]) * bf16_lo(u[j]) + bf16_hi(u[j]) * bf16_hi(u[j]);
+  }
+  const float inv = 1.0f / sqrtf(warp_sum(ss) / static_cast<float>(hidden) + eps);
+  uint4* orow = reinterpret_cast<uint4*>(out + static_cast<int64_t>(row) * hidden);
+#pragma unroll
+  for (int k = 0; k < NV; ++k)
+    if (lane + 32 * k < nvec) {
+      const uint4 wv = __ldg(reinterpret_cast<const uint4*>(weight) + lane + 32 * k);
+      const uint32_t w[4] = {wv.x, wv.y, wv.z, wv.w}, u[4] = {a[k].x, a[k].y, a[k].z, a[k].w};
+      uint32_t o[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) o[j] = pack_bf16x2(bf16_lo(u[j]) * inv * bf16_lo(w[j]), bf16_hi(u[j]) * inv * bf16_hi(w[j]));
+      orow[lane + 32 * k] = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+}
+
 // ------------------------------------------------------------------------------------------------
 // K7 (+K1): one warp per (token, head) of the packed qkv row.  Lane l owns elements
 // [EPL*l, EPL*l+EPL) of each half (EPL = D/64), i.e. exactly the RoPE pairs (j, j + D/2).
@@ -493,6 +542,17 @@ extern "C" int nvllm_add_rmsnorm(void* out, const void* x, void* residual, const
   if (nvec <= 256) threads = (nvec + 31) / 32 * 32;
   if (threads > 1024) threads = 1024;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  // short rows, enough of them that eight to a CTA still give every SM two CTAs
+  if (nvec <= 128 && num_tokens >= 16 * sm_count()) {
+    const dim3 grid(static_cast<unsigned>((num_tokens + 7) / 8));
+    auto rows = [&](auto kern) -> int {
+      NVLLM_CUDA(launch_pdl(kern, grid, dim3(256), 0, st, static_cast<bf16*>(out), static_cast<const bf16*>(x), static_cast<bf16*>(residual),
+                            static_cast<const bf16*>(weight), num_tokens, hidden, eps));
+      NVLLM_LAUNCH_CHECK("add_rmsnorm_rows_kernel");
+      return 0;
+    };
+    return residual ? rows(add_rmsnorm_rows_kernel<true>) : rows(add_rmsnorm_rows_kernel<false>);
+  }
   if (residual)
     NVLLM_CUDA(launch_pdl(add_rmsnorm_kernel<true>, dim3(num_tokens), dim3(threads), 0, st, static_cast<bf16*>(out),
                           static_cast<const bf16*>(x), static_cast<bf16*>(residual), static_cast<const bf16*>(weight),

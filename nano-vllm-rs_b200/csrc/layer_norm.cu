@@ -218,6 +218,34 @@ extern "C" int nvllm_concat_cast(void* out, const float* a, const float* b, int3
   return 0;
 }
 
+namespace nvllm {
+namespace {
+// The same four values at a time, a CTA per row.  8192 rows of 2048 bf16 into two copies (134 MB written, 20 us): 58 us value by value, 24 so.
+template <typename T>
+__global__ void __launch_bounds__(256) embedding_scaled_rows_kernel(float* __restrict__ h, float* __restrict__ h2, const T* __restrict__ table,
+                                                                   const int64_t* __restrict__ ids, int hidden, int vocab, float scale) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int64_t r = blockIdx.x;
+  int64_t id = ids[r];
+  id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);
+  const T* src = table + id * hidden;
+  for (int c = 4 * threadIdx.x; c < hidden; c += 4 * blockDim.x) {
+    float4 v;
+    if constexpr (sizeof(T) == 2) {
+      const uint2 u = __ldg(reinterpret_cast<const uint2*>(src + c));
+      v = make_float4(bf16_lo(u.x), bf16_hi(u.x), bf16_lo(u.y), bf16_hi(u.y));
+    } else {
+      v = __ldg(reinterpret_cast<const float4*>(src + c));
+    }
+    v = make_float4(v.x * scale, v.y * scale, v.z * scale, v.w * scale);
+    *reinterpret_cast<float4*>(h + r * hidden + c) = v;
+    if (h2) *reinterpret_cast<float4*>(h2 + r * hidden + c) = v;
+  }
+}
+}  // namespace
+}  // namespace nvllm
+
 extern "C" int nvllm_embedding_gather_scaled(float* h, float* h_copy, const void* table, const int64_t* ids, int32_t n,
                                              int32_t hidden, int32_t vocab, float scale, int32_t table_dtype, void* stream) {
   NVLLM_CHECK_ARG(n >= 0 && hidden > 0 && vocab > 0, NVLLM_ERR_ARG, "embedding_gather_scaled: sizes");
@@ -226,6 +254,12 @@ extern "C" int nvllm_embedding_gather_scaled(float* h, float* h_copy, const void
   NVLLM_CHECK_ARG(h && table && ids, NVLLM_ERR_ARG, "embedding_gather_scaled: NULL");
   const int64_t total = static_cast<int64_t>(n) * hidden;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (hidden % 4 == 0 && aligned16(h) && aligned16(h_copy) && aligned16(table)) {
+    if (table_dtype == NVLLM_BF16) NVLLM_CUDA(launch_pdl(embedding_scaled_rows_kernel<bf16>, dim3(n), dim3(256), 0, st, h, h_copy, static_cast<const bf16*>(table), ids, hidden, vocab, scale));
+    else NVLLM_CUDA(launch_pdl(embedding_scaled_rows_kernel<float>, dim3(n), dim3(256), 0, st, h, h_copy, static_cast<const float*>(table), ids, hidden, vocab, scale));
+    NVLLM_LAUNCH_CHECK("embedding_scaled_rows_kernel");
+    return 0;
+  }
   if (table_dtype == NVLLM_BF16) NVLLM_CUDA(launch_pdl(embedding_scaled_kernel<bf16>, dim3(grid_for(total)), dim3(256), 0, st, h, h_copy, static_cast<const bf16*>(table), ids, n, hidden, vocab, scale));
   else NVLLM_CUDA(launch_pdl(embedding_scaled_kernel<float>, dim3(grid_for(total)), dim3(256), 0, st, h, h_copy, static_cast<const float*>(table), ids, n, hidden, vocab, scale));
   NVLLM_LAUNCH_CHECK("embedding_scaled_kernel");
