@@ -408,8 +408,8 @@ int32_t nvllm_moe_max_rows(int32_t n_tokens, int32_t top, int32_t experts, int32
 int nvllm_moe_sort(int32_t* row_token, int32_t* tile_expert, int32_t* slot_row, const int32_t* topk_idx, int32_t n,
                    int32_t top, int32_t experts, int32_t max_rows, int32_t tile_rows, void* stream);
 /* Tensor-core grouped product (bf16): rows in 128-row tiles, tile i times the weight block of group tile_group[i], i.e.
- * rows [group * n, (group + 1) * n) of w ([groups * n, k]); an unused tile (group < 0) is computed against group 0 and its
- * rows mean nothing.  k % 64 == 0, n % 8 == 0, 16-byte aligned rows. */
+ * rows [group * n, (group + 1) * n) of w ([groups * n, k]); the rows of an unused tile (group < 0)
+ * mean nothing.  k % 64 == 0, n % 8 == 0, 16-byte aligned rows. */
 int nvllm_gemm_bf16_grouped(void* y, const void* x, const void* w, int32_t max_rows, int32_t n, int32_t k, int32_t groups,
                             int64_t ldx, int64_t ldw, int64_t ldy, const int32_t* tile_group, void* stream);
 /* out[t] = sum_k topk_w[t, k] * (slot_row[t, k] >= 0 ? expert_out[slot_row[t, k]] : x[t]) + shared_out[t] (nullable). */

@@ -85,7 +85,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                     const int32_t* __restrict__ tile_group = nullptr, int group_rows = 0, float glu_limit = 0.f,
                     const float* __restrict__ row_scale = nullptr) {
   // tile_group != nullptr (expert layers): 128-row tile m uses the weight block of group tile_group[m], i.e. rows
-  // [group * group_rows, ...) of w; an unused tile (group < 0) runs against group 0 and its rows are never read.
+  // [group * group_rows, ...) of w; an unused tile (group < 0) runs against group 0 and its rows are never read.  Large products of this
+  // kind go to CTA pairs (gemm_tcgen05_2cta.cu, which also says what the order of the tiles is worth).
   using C = GemmCfg<BN>;  // STAGES <= C::kStages: ring depth of this launch (fewer stages -> two CTAs per SM, see launch_gemm)
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;  // SWIZZLE_128B tiles: 1024-byte aligned
@@ -102,6 +103,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // (uniform)
   const int lane = threadIdx.x & 31;
   const int num_kb = K / C::BK;
+  const int n_fast = tile_group != nullptr ? num_tiles / num_m_tiles : 0;   // grouped: n-tiles run fastest
   const int cta0 = static_cast<int>(blockIdx.x), cta_stride = static_cast<int>(gridDim.x);
   pdl_launch_dependents();  // everything up to pdl_wait() below is independent of the previous kernel
 
@@ -155,7 +157,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     uint32_t phase = 0;
     bool first = true;
     for (int tile = cta0; tile < num_tiles; tile += cta_stride) {
-      const int m_tile = tile % num_m_tiles, n_tile = tile / num_m_tiles;
+      const int m_tile = n_fast ? tile / n_fast : tile % num_m_tiles, n_tile = n_fast ? tile % n_fast : tile / num_m_tiles;
       int goff = 0;
       if (tile_group != nullptr) { const int g = tile_group[m_tile]; goff = (g > 0 ? g : 0) * group_rows; }
       for (int kb = 0; kb < num_kb; ++kb) {
@@ -205,7 +207,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int tile = cta0; tile < num_tiles; tile += cta_stride) {
-      const int m_tile = tile % num_m_tiles, n_tile = tile / num_m_tiles;
+      const int m_tile = n_fast ? tile / n_fast : tile % num_m_tiles, n_tile = n_fast ? tile % n_fast : tile / num_m_tiles;
       mbar_wait(tfull_bar(acc), acc_phase);
       tc_fence_after();
       const int row = m_tile * C::BM + q * 32 + lane;
@@ -400,6 +402,10 @@ bool splitk_choose(int m, int n_acc, int k, bool silu, int bn_default, int* out_
 int gemm_splitk_dispatch(void* y, const void* x, const void* w, int m, int n, int k, int64_t ldx, int64_t ldw, int64_t ldy,
                          int gate, int bn, int sk, cudaStream_t st, const RowPush& ps = RowPush{}, float glu_limit = 0.f, int out_dtype = NVLLM_BF16);
 
+bool grouped_2cta(int max_rows, int n, int groups);                                                           // gemm_tcgen05_2cta.cu
+int gemm_grouped_2cta_dispatch(void* y, const void* x, const void* w, int max_rows, int n, int k, int groups, int64_t ldx, int64_t ldw, int64_t ldy,
+                               const int32_t* tile_group, cudaStream_t st);
+
 static bool use_2cta();
 // CTA pairs pay off once there are at least two 256-row tiles or the problem is large enough to fill the machine with
 // 256 x 256 tiles; between 129 and 511 rows the single-CTA kernel (more, narrower, single-wave tiles) measured faster
@@ -473,7 +479,7 @@ extern "C" int nvllm_gemm_bf16(void* y, const void* x, const void* w, int32_t m,
 }
 
 // Grouped GEMM for expert layers: rows come in 128-row tiles, tile i multiplies with the weight block of group
-// tile_group[i] (rows [group * n, (group + 1) * n) of w).  Same kernel as nvllm_gemm_bf16, single-CTA tiles.
+// tile_group[i] (rows [group * n, (group + 1) * n) of w).  Same kernels as nvllm_gemm_bf16.
 extern "C" int nvllm_gemm_bf16_grouped(void* y, const void* x, const void* w, int32_t max_rows, int32_t n, int32_t k,
                                        int32_t groups, int64_t ldx, int64_t ldw, int64_t ldy, const int32_t* tile_group,
                                        void* stream) {
@@ -485,6 +491,7 @@ extern "C" int nvllm_gemm_bf16_grouped(void* y, const void* x, const void* w, in
   if (max_rows == 0) return 0;
   NVLLM_CHECK_ARG(y && x && w && tile_group && aligned16(y) && aligned16(x) && aligned16(w), NVLLM_ERR_ALIGN, "gemm_grouped: pointers");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (grouped_2cta(max_rows, n, groups)) return gemm_grouped_2cta_dispatch(y, x, w, max_rows, n, k, groups, ldx, ldw, ldy, tile_group, st);
   const int bn = n >= 256 ? 256 : (n >= 128 ? 128 : (n >= 64 ? 64 : 32));
   CUtensorMap tx, tw;
   if (int rc = make_tmap_bf16_2d(&tx, x, max_rows, k, ldx, 128)) return rc;

@@ -160,11 +160,17 @@ __device__ __forceinline__ void rope_rows(bf16* __restrict__ y, int64_t ldy, con
 // [BN/2, BN) are up for the same BN/2 output features, and the epilogue writes y[:, n_tile*BN/2 + c] = silu(gate)*up
 // (SiluAndMul::forward, activation.rs:46-63; or another gate of gated_pair) without the [M, 2N] intermediate ever reaching HBM.  N = output features.
 // ROPE: the qkv epilogue that RopeEpi describes, on the two heads of a tile; see rope_rows.
-template <int BN, typename OutT, int GATE, bool ROPE>
+// GROUPED: the experts' product.  tile_group names the weight block (group_rows rows of w) of each 128-row tile, in device memory; a pair
+// takes two neighbouring tiles of one group, the last of an odd run alone (its second half multiplies the next group's rows and stores
+// nothing).  Every CTA makes the list of pairs itself.  n-tiles run fastest: the pairs at work then share a dozen groups' weights and x
+// comes from HBM once, where the other order reads it again for every n-tile (8192 tokens x 6 of 64 experts, 2048 -> 1408: single CTAs 356 us
+// with m-tiles fastest, 297 with n-tiles, pairs 259; 1408 -> 2048: 341, 286, 245).  Bound by the L2 -> SM feed like the plain product, and by
+// the rows that fill up tiles and pairs.
+template <int BN, typename OutT, int GATE, bool ROPE, bool GROUPED>
 __global__ void __launch_bounds__(gemm2_threads<GATE, ROPE>(), 1)
 gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                          OutT* __restrict__ y, int M, int N, int K, int64_t ldy, int num_m_tiles, int num_tiles, float glu_limit,
-                         const RopeEpi re) {
+                         const RopeEpi re, const int32_t* __restrict__ tile_group, int group_rows) {
   using C = Gemm2Cfg<BN>;
   constexpr int STAGES = C::kStages - (ROPE ? 1 : 0);   // (the qkv epilogue takes a stage's room)
   extern __shared__ uint8_t smem_raw[];
@@ -206,6 +212,45 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
   cluster_sync_all();  // barriers of BOTH CTAs are initialised before any remote signal can arrive
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
+  [[maybe_unused]] uint32_t* const pairs = tmem_slot_ptr + 4;   // GROUPED: m-tile | second half live << 12 | group << 13
+  if constexpr (GROUPED) {
+    // num_m_tiles: 128-row tiles (at most kMaxGroupedTiles); num_tiles: n-tiles
+    pdl_wait();
+    for (int i = threadIdx.x; i < num_m_tiles; i += blockDim.x) pairs[i] = static_cast<uint32_t>(tile_group[i]);
+    __syncthreads();
+    if (warp == 3) {
+      int count = 0, start = 0, prev = -1;                      // (in place: a pair's entry never lies behind the tile that it starts at)
+      for (int i0 = 0; i0 < num_m_tiles; i0 += 32) {
+        const int i = i0 + lane;
+        const int g = i < num_m_tiles ? static_cast<int>(pairs[i]) : -1, next = i + 1 < num_m_tiles ? static_cast<int>(pairs[i + 1]) : -1;
+        const int up = __shfl_up_sync(0xffffffffu, g, 1);
+        const uint32_t breaks = __ballot_sync(0xffffffffu, g != (lane == 0 ? prev : up)) & (0xffffffffu >> (31 - lane));
+        const int run = breaks ? i0 + 31 - __clz(breaks) : start;
+        const bool first = g >= 0 && ((i - run) & 1) == 0;
+        const uint32_t firsts = __ballot_sync(0xffffffffu, first);
+        if (first) pairs[count + __popc(firsts & ((1u << lane) - 1))] = static_cast<uint32_t>(i) | (next == g ? 1u << 12 : 0u) | static_cast<uint32_t>(g) << 13;
+        count += __popc(firsts);
+        start = __shfl_sync(0xffffffffu, run, 31);
+        prev = __shfl_sync(0xffffffffu, g, 31);
+        __syncwarp();
+      }
+      if (lane == 0) tmem_slot_ptr[1] = static_cast<uint32_t>(count);
+    }
+    __syncthreads();
+    num_m_tiles = num_tiles;                                    // (now the divisor of a tile's number)
+    num_tiles = __reduce_max_sync(0xffffffffu, static_cast<int>(tmem_slot_ptr[1])) * num_m_tiles;
+  }
+  // a tile's first row for this CTA, its n-tile, the first row that holds nothing of it, and its weight block's first row
+  struct Where { int row0, n_tile, m_end, w0; };
+  auto where = [&](int tile) {
+    if constexpr (GROUPED) {
+      const uint32_t p = pairs[tile / num_m_tiles];
+      const int row0 = static_cast<int>(p & 0xfffu) * C::BM_CTA;
+      return Where{row0 + static_cast<int>(rank) * C::BM_CTA, tile % num_m_tiles, row0 + (p & 0x1000u ? C::BM : C::BM_CTA), static_cast<int>(p >> 13) * group_rows};
+    } else {
+      return Where{tile % num_m_tiles * C::BM + static_cast<int>(rank) * C::BM_CTA, tile / num_m_tiles, M, 0};
+    }
+  };
 
   if (warp == 0 && lane == 0) {
     // ===== TMA producer (both CTAs) =====
@@ -213,13 +258,13 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
     int stage = 0;
     uint32_t phase = 0;
     for (int tile = cluster_id; tile < num_tiles; tile += num_clusters) {
-      const int m_tile = tile % num_m_tiles, n_tile = tile / num_m_tiles;
+      const Where at = where(tile);
       for (int kb = 0; kb < num_kb; ++kb) {
         mbar_wait(empty_bar(stage), phase ^ 1);
         if (leader) mbar_expect_tx(full_bar(stage), 2 * C::kStageBytes);
-        tma_load_2d_cg2(sA + stage * C::kABytes, &tmap_x, full_bar(stage), kb * C::BK, m_tile * C::BM + rank * C::BM_CTA);
+        tma_load_2d_cg2(sA + stage * C::kABytes, &tmap_x, full_bar(stage), kb * C::BK, at.row0);
         tma_load_2d_cg2(sB + stage * C::kBBytes, &tmap_w, full_bar(stage), kb * C::BK,
-                        GATE != kGateNone ? static_cast<int>(rank) * N + n_tile * (BN / 2) : n_tile * BN + static_cast<int>(rank) * (BN / 2));
+                        at.w0 + (GATE != kGateNone ? static_cast<int>(rank) * N + at.n_tile * (BN / 2) : at.n_tile * BN + static_cast<int>(rank) * (BN / 2)));
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
@@ -257,16 +302,17 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int tile = cluster_id; tile < num_tiles; tile += num_clusters) {
-      const int m_tile = tile % num_m_tiles, n_tile = tile / num_m_tiles;
+      const Where at = where(tile);
+      const int n_tile = at.n_tile;
       [[maybe_unused]] RopeAngles angles;
-      [[maybe_unused]] const int rope_row0 = m_tile * C::BM + static_cast<int>(rank) * C::BM_CTA + q * 32 + (warp < 8 ? 0 : 16);
+      [[maybe_unused]] const int rope_row0 = at.row0 + q * 32 + (warp < 8 ? 0 : 16);
       if constexpr (ROPE) {
         static_assert(!ROPE || BN == 256, "two heads a tile");
         rope_angles(angles, re, rope_row0, M, n_tile * 2 < re.H + re.Hkv);
       }
       mbar_wait(tfull_bar(acc), acc_phase);
       tc_fence_after();
-      const int row = m_tile * C::BM + rank * C::BM_CTA + q * 32 + lane;
+      const int row = at.row0 + q * 32 + lane;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
       if constexpr (ROPE) {
         rope_rows(y, ldy, re, angles, taddr, smem_raw + (smem_base - smem_u32(smem_raw)) + STAGES * C::kStageBytes + (warp - 4) * kRopeStage, rope_row0, M,
@@ -288,7 +334,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
             g[e + 1] = __float_as_uint(p.y);
           }
           const int col0 = n_tile * (BN / 2) + c * 32;
-          if (row < M && col0 < N) store_row32_2<OutT>(y + row * ldy + col0, g, col0, N);
+          if (row < at.m_end && col0 < N) store_row32_2<OutT>(y + row * ldy + col0, g, col0, N);
         }
       } else {
 #pragma unroll 1
@@ -297,7 +343,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
           tmem_ld_32x32b_x32(taddr + c * 32, r);
           tmem_ld_wait();
           const int col0 = n_tile * BN + c * 32;
-          if (row < M && col0 < N) store_row32_2<OutT>(y + row * ldy + col0, r, col0, N);
+          if (row < at.m_end && col0 < N) store_row32_2<OutT>(y + row * ldy + col0, r, col0, N);
         }
       }
       tc_fence_before();
@@ -314,14 +360,18 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
   }
 }
 
-template <int BN, typename OutT, int GATE = kGateNone, bool ROPE = false>
+constexpr int kMaxGroupedTiles = 4096;   // (the list's entries hold 12 bits of tile and 19 of group)
+
+template <int BN, typename OutT, int GATE = kGateNone, bool ROPE = false, bool GROUPED = false>
 static int launch_gemm2(const CUtensorMap& tx, const CUtensorMap& tw, void* y, int M, int N, int K, int64_t ldy,
-                        cudaStream_t st, float glu_limit = 0.f, const RopeEpi& re = RopeEpi{}) {
+                        cudaStream_t st, float glu_limit = 0.f, const RopeEpi& re = RopeEpi{}, const int32_t* tile_group = nullptr, int group_rows = 0) {
   using C = Gemm2Cfg<BN>;
-  auto kern = gemm_tcgen05_2cta_kernel<BN, OutT, GATE, ROPE>;
-  constexpr int smem = C::kSmemBytes + (ROPE ? 8 * kRopeStage - C::kStageBytes : 0);
-  NVLLM_SMEM_ATTR_ONCE(kern, smem);
-  const int num_m_tiles = (M + C::BM - 1) / C::BM;
+  auto kern = gemm_tcgen05_2cta_kernel<BN, OutT, GATE, ROPE, GROUPED>;
+  constexpr int smem_max = C::kSmemBytes + (ROPE ? 8 * kRopeStage - C::kStageBytes : 0) + (GROUPED ? 4 * kMaxGroupedTiles : 0);
+  static_assert(smem_max <= 227 * 1024, "");
+  NVLLM_SMEM_ATTR_ONCE(kern, smem_max);
+  const int num_m_tiles = GROUPED ? M / C::BM_CTA : (M + C::BM - 1) / C::BM;
+  const int smem = smem_max - (GROUPED ? 4 * (kMaxGroupedTiles - num_m_tiles) : 0);
   const int num_n_tiles = GATE != kGateNone ? (N + BN / 2 - 1) / (BN / 2) : (N + BN - 1) / BN;
   const int num_tiles = num_m_tiles * num_n_tiles;
   const int max_clusters = sm_count() / 2;
@@ -338,7 +388,8 @@ static int launch_gemm2(const CUtensorMap& tx, const CUtensorMap& tw, void* y, i
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  NVLLM_CUDA(cudaLaunchKernelEx(&cfg, kern, tx, tw, static_cast<OutT*>(y), M, N, K, ldy, num_m_tiles, num_tiles, glu_limit, re));
+  NVLLM_CUDA(cudaLaunchKernelEx(&cfg, kern, tx, tw, static_cast<OutT*>(y), M, N, K, ldy, num_m_tiles, GROUPED ? num_n_tiles : num_tiles, glu_limit, re, tile_group,
+                                group_rows));
   return 0;
 }
 
@@ -389,6 +440,21 @@ int gemm_qkv_2cta_dispatch(void* qkv, const void* x, const void* w, int m, int n
   if (int rc = make_tmap_bf16_2d(&tx, x, m, k, ldx, 128)) return rc;
   if (int rc = make_tmap_bf16_2d(&tw, w, n, k, ldw, 128)) return rc;
   return launch_gemm2<256, bf16, kGateNone, true>(tx, tw, qkv, m, n, k, n, st, 0.f, re);
+}
+
+// The experts' product of nvllm_gemm_bf16_grouped on CTA pairs.  A group of one tile wastes half a pair, but a tile that no group uses costs
+// nothing: 64 experts' tiles of 2048 -> 1408 take, on single CTAs and on pairs, 76 and 89 us at 67 tiles' room, 86 and 88 at 76, 103 and 88 at
+// 112; 8 experts, 2048 -> 2048, 18.5 and 18.3 at 10, 20 and 18 at 16.  Hence a quarter more tiles than groups.
+bool grouped_2cta(int max_rows, int n, int groups) {
+  const int tiles = max_rows / 128;
+  return knobs().gemm_2cta != 0 && n >= 256 && groups <= (1 << 19) && tiles <= kMaxGroupedTiles && 4 * static_cast<int64_t>(tiles) >= 5 * static_cast<int64_t>(groups);
+}
+int gemm_grouped_2cta_dispatch(void* y, const void* x, const void* w, int max_rows, int n, int k, int groups, int64_t ldx, int64_t ldw, int64_t ldy,
+                               const int32_t* tile_group, cudaStream_t st) {
+  CUtensorMap tx, tw;
+  if (int rc = make_tmap_bf16_2d(&tx, x, max_rows, k, ldx, 128)) return rc;
+  if (int rc = make_tmap_bf16_2d(&tw, w, static_cast<int64_t>(groups) * n, k, ldw, 128)) return rc;
+  return launch_gemm2<256, bf16, kGateNone, false, true>(tx, tw, y, max_rows, n, k, ldy, st, 0.f, RopeEpi{}, tile_group, n);
 }
 
 // y[M, inter] = silu(x . Wgate^T) * (x . Wup^T) (or another gate) with w = [Wgate | Wup] packed row-wise ([2*inter, K]).
