@@ -412,6 +412,9 @@ int nvllm_moe_sort(int32_t* row_token, int32_t* tile_expert, int32_t* slot_row, 
  * mean nothing.  k % 64 == 0, n % 8 == 0, 16-byte aligned rows. */
 int nvllm_gemm_bf16_grouped(void* y, const void* x, const void* w, int32_t max_rows, int32_t n, int32_t k, int32_t groups,
                             int64_t ldx, int64_t ldw, int64_t ldy, const int32_t* tile_group, void* stream);
+/* The same with y = relu(v)^2, v the product rounded to bf16 (nvllm_ff_activation's kind 1 in the epilogue). */
+int nvllm_gemm_relu2_bf16_grouped(void* y, const void* x, const void* w, int32_t max_rows, int32_t n, int32_t k, int32_t groups,
+                                  int64_t ldx, int64_t ldw, int64_t ldy, const int32_t* tile_group, void* stream);
 /* out[t] = sum_k topk_w[t, k] * (slot_row[t, k] >= 0 ? expert_out[slot_row[t, k]] : x[t]) + shared_out[t] (nullable). */
 int nvllm_moe_combine(void* out, const void* expert_out, const void* x, const void* shared_out, const int32_t* topk_idx,
                       const float* topk_w, const int32_t* slot_row, int32_t n, int32_t hidden, int32_t top, int32_t experts,

@@ -106,6 +106,7 @@ PROTOTYPES = {
     "nvllm_moe_max_rows": (i32, [i32, i32, i32, i32]),
     "nvllm_moe_sort": (i32, [vp, vp, vp, vp, i32, i32, i32, i32, i32, vp]),
     "nvllm_gemm_bf16_grouped": (i32, [vp, vp, vp, i32, i32, i32, i32, i64, i64, i64, vp, vp]),
+    "nvllm_gemm_relu2_bf16_grouped": (i32, [vp, vp, vp, i32, i32, i32, i32, i64, i64, i64, vp, vp]),
     "nvllm_moe_combine": (i32, [vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp]),
     "nvllm_rms_residual_norm": (i32, [vp, vp, vp, i32, vp, vp, i32, i32, f32, i32, vp]),
     "nvllm_rms_norm_rows": (i32, [vp, i64, vp, i64, vp, vp, i32, i32, f32, i32, vp]),

@@ -170,7 +170,7 @@ template <int BN, typename OutT, int GATE, bool ROPE, bool GROUPED>
 __global__ void __launch_bounds__(gemm2_threads<GATE, ROPE>(), 1)
 gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                          OutT* __restrict__ y, int M, int N, int K, int64_t ldy, int num_m_tiles, int num_tiles, float glu_limit,
-                         const RopeEpi re, const int32_t* __restrict__ tile_group, int group_rows) {
+                         const RopeEpi re, const int32_t* __restrict__ tile_group, int group_rows, bool relu2) {
   using C = Gemm2Cfg<BN>;
   constexpr int STAGES = C::kStages - (ROPE ? 1 : 0);   // (the qkv epilogue takes a stage's room)
   extern __shared__ uint8_t smem_raw[];
@@ -342,6 +342,9 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
           uint32_t r[32];
           tmem_ld_32x32b_x32(taddr + c * 32, r);
           tmem_ld_wait();
+          if constexpr (GROUPED) {
+            if (relu2) relu2_row32(r);
+          }
           const int col0 = n_tile * BN + c * 32;
           if (row < at.m_end && col0 < N) store_row32_2<OutT>(y + row * ldy + col0, r, col0, N);
         }
@@ -364,7 +367,7 @@ constexpr int kMaxGroupedTiles = 4096;   // (the list's entries hold 12 bits of 
 
 template <int BN, typename OutT, int GATE = kGateNone, bool ROPE = false, bool GROUPED = false>
 static int launch_gemm2(const CUtensorMap& tx, const CUtensorMap& tw, void* y, int M, int N, int K, int64_t ldy,
-                        cudaStream_t st, float glu_limit = 0.f, const RopeEpi& re = RopeEpi{}, const int32_t* tile_group = nullptr, int group_rows = 0) {
+                        cudaStream_t st, float glu_limit = 0.f, const RopeEpi& re = RopeEpi{}, const int32_t* tile_group = nullptr, int group_rows = 0, bool relu2 = false) {
   using C = Gemm2Cfg<BN>;
   auto kern = gemm_tcgen05_2cta_kernel<BN, OutT, GATE, ROPE, GROUPED>;
   constexpr int smem_max = C::kSmemBytes + (ROPE ? 8 * kRopeStage - C::kStageBytes : 0) + (GROUPED ? 4 * kMaxGroupedTiles : 0);
@@ -389,7 +392,7 @@ static int launch_gemm2(const CUtensorMap& tx, const CUtensorMap& tw, void* y, i
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
   NVLLM_CUDA(cudaLaunchKernelEx(&cfg, kern, tx, tw, static_cast<OutT*>(y), M, N, K, ldy, num_m_tiles, GROUPED ? num_n_tiles : num_tiles, glu_limit, re, tile_group,
-                                group_rows));
+                                group_rows, relu2));
   return 0;
 }
 
@@ -450,11 +453,11 @@ bool grouped_2cta(int max_rows, int n, int groups) {
   return knobs().gemm_2cta != 0 && n >= 256 && groups <= (1 << 19) && tiles <= kMaxGroupedTiles && 4 * static_cast<int64_t>(tiles) >= 5 * static_cast<int64_t>(groups);
 }
 int gemm_grouped_2cta_dispatch(void* y, const void* x, const void* w, int max_rows, int n, int k, int groups, int64_t ldx, int64_t ldw, int64_t ldy,
-                               const int32_t* tile_group, cudaStream_t st) {
+                               const int32_t* tile_group, bool relu2, cudaStream_t st) {
   CUtensorMap tx, tw;
   if (int rc = make_tmap_bf16_2d(&tx, x, max_rows, k, ldx, 128)) return rc;
   if (int rc = make_tmap_bf16_2d(&tw, w, static_cast<int64_t>(groups) * n, k, ldw, 128)) return rc;
-  return launch_gemm2<256, bf16, kGateNone, false, true>(tx, tw, y, max_rows, n, k, ldy, st, 0.f, RopeEpi{}, tile_group, n);
+  return launch_gemm2<256, bf16, kGateNone, false, true>(tx, tw, y, max_rows, n, k, ldy, st, 0.f, RopeEpi{}, tile_group, n, relu2);
 }
 
 // y[M, inter] = silu(x . Wgate^T) * (x . Wup^T) (or another gate) with w = [Wgate | Wup] packed row-wise ([2*inter, K]).

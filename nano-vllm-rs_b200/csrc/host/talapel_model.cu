@@ -100,7 +100,7 @@ class Talapel : public ModelImpl {
   float *h_ = nullptr, *x0_ = nullptr, *proj_ = nullptr, *left_out_ = nullptr, *right_out_ = nullptr, *conv_out_ = nullptr,
         *step_ = nullptr, *decay_t_ = nullptr, *y_ = nullptr, *topk_w_ = nullptr;
   void *normed_ = nullptr, *cat_ = nullptr, *q_ = nullptr, *mix_in_ = nullptr, *gu_buf_ = nullptr, *act_ = nullptr, *ff_out_ = nullptr,
-       *eout_ = nullptr, *xg_ = nullptr, *eup_buf_ = nullptr, *head_in_ = nullptr;
+       *eout_ = nullptr, *xg_ = nullptr, *head_in_ = nullptr;
   int32_t *topk_idx_ = nullptr, *row_token_ = nullptr, *tile_expert_ = nullptr, *slot_row_ = nullptr;
   int max_rows_ = 0, head_rows_ = 0;
   std::vector<void*> allocs_;
@@ -300,7 +300,6 @@ class Talapel : public ModelImpl {
       RUN(dalloc(&topk_w_, T * m_top)); RUN(dalloc(&topk_idx_, T * m_top)); RUN(dalloc(&slot_row_, T * m_top));
       RUN(dalloc(&row_token_, static_cast<size_t>(max_rows_) + 32)); RUN(dalloc(&tile_expert_, static_cast<size_t>(max_rows_) / 32 + 1));
       RUN(oalloc(&eout_, static_cast<size_t>(max_rows_) * W)); RUN(oalloc(&xg_, static_cast<size_t>(max_rows_) * W));
-      RUN(oalloc(&eup_buf_, static_cast<size_t>(max_rows_) * m_eff));
     }
     if (m_act > 0) RUN(oalloc(&act_, std::max(T, static_cast<size_t>(max_rows_)) * m_act));
     NVLLM_CUDA(cudaStreamSynchronize(stream));
@@ -570,8 +569,7 @@ class Talapel : public ModelImpl {
         RUN(nvllm_moe_sort(row_token_, tile_expert_, slot_row_, topk_idx_, N, L.top, L.experts, rows, L.tile_rows, st)); ++launches; mk("moe_sort");
         if (L.tile_rows == 128) {
           RUN(nvllm_gather_rows(xg_, normed_, row_token_, rows, W, N, dt_, st)); ++launches; mk("expert row gather");
-          RUN(nvllm_gemm_bf16_grouped(eup_buf_, xg_, L.eup, rows, L.ff, W, L.experts, W, W, L.ff, tile_expert_, st)); ++launches; mk("expert up grouped GEMM");
-          RUN(nvllm_ff_activation(act_, eup_buf_, rows, L.ff, 1, dt_, st)); ++launches; mk("ff_activation (relu^2)");
+          RUN(nvllm_gemm_relu2_bf16_grouped(act_, xg_, L.eup, rows, L.ff, W, L.experts, W, W, L.ff, tile_expert_, st)); ++launches; mk("expert up + relu^2 grouped GEMM");
           RUN(nvllm_gemm_bf16_grouped(eout_, act_, L.edown, rows, W, L.ff, L.experts, L.ff, L.ff, W, tile_expert_, st)); ++launches; mk("expert down grouped GEMM");
         } else {
           RUN(nvllm_linear_grouped(act_, normed_, L.eup, rows, L.ff, W, W, W, L.ff, static_cast<int64_t>(L.ff) * W, row_token_, tile_expert_, 2,

@@ -17,6 +17,15 @@ int make_tmap_bf16_2d(CUtensorMap* map, const void* base, int64_t rows, int64_t 
 int make_tmap_bf16_nd(CUtensorMap* map, const void* base, int rank, const uint64_t* dims,
                       const uint64_t* strides_bytes, const uint32_t* box);  // tc_host.cu
 
+// relu(v)^2 of 32 accumulator values, v rounded to bf16 first (the product as a tensor of its own would be).
+__device__ __forceinline__ void relu2_row32(uint32_t (&r)[32]) {
+#pragma unroll
+  for (int e = 0; e < 32; ++e) {
+    const float v = fmaxf(__bfloat162float(__float2bfloat16_rn(__uint_as_float(r[e]))), 0.f);
+    r[e] = __float_as_uint(v * v);
+  }
+}
+
 // ---- qkv epilogue of the GEMMs ---------------------------------------------------------------------
 // What Qwen3Attention::forward does between qkv_proj and Attention::forward (qwen3.rs:219-229) plus Attention::store_kv_cache
 // (attention.rs:150-174), on the accumulators of x . Wqkv^T: round to bf16 (the qkv tensor), per-head RMSNorm (q/k), bf16, half-split
