@@ -786,46 +786,69 @@ __global__ void __launch_bounds__(128) gated_group_norm_vec_kernel(TO* __restric
 }
 
 // Parts of up to 512 values: one WARP per (token, part), four parts per CTA, the part's values in registers.
-template <typename TO>
+// NV: 16-byte pieces per lane, PER: parts per warp.  Parts of up to 128 values have one piece a lane, so a warp takes four of them and
+// requests all before it uses any (8192 x 2048 values in parts of 128, 168 MB or 26 us at the copy rate: 57 us with a part a warp, 36 so).
+// In larger parts requesting y and z together is what counts (8192 x 4096 in parts of 512, 335 MB or 51 us: 69 -> 52 us).
+template <typename TO, int NV, int PER>
 __global__ void __launch_bounds__(128) gated_group_norm_warp_kernel(TO* __restrict__ out, int64_t ldo, const float* __restrict__ y, int64_t ldy,
                                                                     const float* __restrict__ z, int64_t ldz, const float* __restrict__ w, int gs,
                                                                     int parts, int64_t items, float eps, int gate_first, int act, int wst) {
   pdl_wait();
   pdl_launch_dependents();
   const int lane = threadIdx.x & 31, nv = gs / 4;
-  const int64_t item = static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5);
-  if (item >= items) return;
-  const int64_t t = item / parts;
-  const int g = static_cast<int>(item - t * parts);
-  const float4* yr = reinterpret_cast<const float4*>(y + t * ldy + static_cast<int64_t>(g) * gs);
-  const float4* zr = reinterpret_cast<const float4*>(z + t * ldz + static_cast<int64_t>(g) * gs);
-  float4 v[4], sg[4];
-  float sq = 0.f;
+  const int64_t item0 = (static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5)) * PER;
+  if (item0 >= items) return;
+  float4 v[PER][NV], sg[PER][NV];
+  int64_t t[PER];
+  int g[PER];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int c = lane + 32 * k;
-    if (c < nv) {
-      v[k] = yr[c];
-      const float4 zz = zr[c];
-      sg[k] = make_float4(gate_f(zz.x, act), gate_f(zz.y, act), gate_f(zz.z, act), gate_f(zz.w, act));
-      if (gate_first) { v[k].x *= sg[k].x; v[k].y *= sg[k].y; v[k].z *= sg[k].z; v[k].w *= sg[k].w; }
-      sq += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
+  for (int p = 0; p < PER; ++p) {
+    if (p == 0) {
+      t[0] = items <= INT32_MAX ? static_cast<uint32_t>(item0) / static_cast<uint32_t>(parts) : item0 / parts;
+      g[0] = static_cast<int>(item0 - t[0] * parts);
+    } else {
+      const bool more = item0 + p < items, wrap = more && g[p - 1] + 1 == parts;   // (past the end: the last part again, not stored)
+      t[p] = t[p - 1] + (wrap ? 1 : 0);
+      g[p] = wrap ? 0 : g[p - 1] + (more ? 1 : 0);
+    }
+    const float4* yr = reinterpret_cast<const float4*>(y + t[p] * ldy + static_cast<int64_t>(g[p]) * gs);
+    const float4* zr = reinterpret_cast<const float4*>(z + t[p] * ldz + static_cast<int64_t>(g[p]) * gs);
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const int c = lane + 32 * k;
+      if (c < nv) { v[p][k] = yr[c]; sg[p][k] = zr[c]; }
     }
   }
-  const float r = rsqrtf(warp_sum(sq) / gs + eps);
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int c = lane + 32 * k;
-    if (c < nv) {
-      float4 o = make_float4(v[k].x * r, v[k].y * r, v[k].z * r, v[k].w * r);
-      if (!gate_first) { o.x *= sg[k].x; o.y *= sg[k].y; o.z *= sg[k].z; o.w *= sg[k].w; }
-      if (w) {
-        const float4 ww = reinterpret_cast<const float4*>(w + static_cast<int64_t>(g) * wst)[c];
-        o.x *= ww.x; o.y *= ww.y; o.z *= ww.z; o.w *= ww.w;
+  for (int p = 0; p < PER; ++p) {
+    if (item0 + p >= items) return;
+    float sq = 0.f;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      if (lane + 32 * k < nv) {
+        float4& x = v[p][k];
+        float4& s = sg[p][k];
+        s = make_float4(gate_f(s.x, act), gate_f(s.y, act), gate_f(s.z, act), gate_f(s.w, act));
+        if (gate_first) { x.x *= s.x; x.y *= s.y; x.z *= s.z; x.w *= s.w; }
+        sq += x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;
       }
-      const int64_t at = t * ldo + static_cast<int64_t>(g) * gs + 4 * c;
-      if (sizeof(TO) == 2) *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(out) + at) = make_uint2(pack_bf16x2(o.x, o.y), pack_bf16x2(o.z, o.w));
-      else *reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + at) = o;
+    }
+    const float r = rsqrtf(warp_sum(sq) / gs + eps);
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const int c = lane + 32 * k;
+      if (c < nv) {
+        const float4 x = v[p][k], s = sg[p][k];
+        float4 o = make_float4(x.x * r, x.y * r, x.z * r, x.w * r);
+        if (!gate_first) { o.x *= s.x; o.y *= s.y; o.z *= s.z; o.w *= s.w; }
+        if (w) {
+          const float4 ww = reinterpret_cast<const float4*>(w + static_cast<int64_t>(g[p]) * wst)[c];
+          o.x *= ww.x; o.y *= ww.y; o.z *= ww.z; o.w *= ww.w;
+        }
+        const int64_t at = t[p] * ldo + static_cast<int64_t>(g[p]) * gs + 4 * c;
+        if (sizeof(TO) == 2) *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(out) + at) = make_uint2(pack_bf16x2(o.x, o.y), pack_bf16x2(o.z, o.w));
+        else *reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + at) = o;
+      }
     }
   }
 }
@@ -1113,11 +1136,15 @@ extern "C" int nvllm_gated_group_norm_act(void* out, int64_t ldo, const float* y
   const bool vec_ok = gs % 4 == 0 && ldo % 4 == 0 && ldy % 4 == 0 && ldg % 4 == 0 && aligned16(out) && aligned16(y) && aligned16(gate) && aligned16(w);
   if (vec_ok && gs <= 512) {
     const int64_t items = static_cast<int64_t>(n) * parts;
-    const unsigned wgrid = static_cast<unsigned>((items + 3) / 4);
+    // few parts: one a warp, so that they spread over the chip (parts of 128, one and four a warp: 5.4 and 6.2 us at 11200, 12.3 and 9.7 at 32768)
+    const bool four = gs <= 128 && items >= 128 * sm_count();
+    const unsigned wgrid = static_cast<unsigned>(four ? (items + 15) / 16 : (items + 3) / 4);
     if (out_dtype == NVLLM_BF16)
-      NVLLM_CUDA(launch_pdl(gated_group_norm_warp_kernel<bf16>, dim3(wgrid), dim3(128), 0, st, static_cast<bf16*>(out), ldo, y, ldy, gate, ldg, w, gs, parts, items, eps, gate_first, gate_act, wst));
+      NVLLM_CUDA(launch_pdl(four ? gated_group_norm_warp_kernel<bf16, 1, 4> : gated_group_norm_warp_kernel<bf16, 4, 1>, dim3(wgrid), dim3(128), 0, st, static_cast<bf16*>(out), ldo, y,
+                            ldy, gate, ldg, w, gs, parts, items, eps, gate_first, gate_act, wst));
     else
-      NVLLM_CUDA(launch_pdl(gated_group_norm_warp_kernel<float>, dim3(wgrid), dim3(128), 0, st, static_cast<float*>(out), ldo, y, ldy, gate, ldg, w, gs, parts, items, eps, gate_first, gate_act, wst));
+      NVLLM_CUDA(launch_pdl(four ? gated_group_norm_warp_kernel<float, 1, 4> : gated_group_norm_warp_kernel<float, 4, 1>, dim3(wgrid), dim3(128), 0, st, static_cast<float*>(out), ldo, y,
+                            ldy, gate, ldg, w, gs, parts, items, eps, gate_first, gate_act, wst));
     NVLLM_LAUNCH_CHECK("gated_group_norm_warp_kernel");
     return 0;
   }

@@ -76,3 +76,20 @@ def test_store_with_some_biases(cuda, q, k, v, which, dtype):
         ref = torch.zeros(20, w.shape[1]); ref[slots[live].long()] = w[live]
         assert torch.equal(cache.cpu(), ref.to(dtype))
     assert torch.equal(got.cpu(), want[0].to(dtype))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("gs", [4, 100, 128, 132])                                                 # up to 128: four parts a warp
+@pytest.mark.parametrize("rows,parts", [(18943, 1), (18945, 1), (1723, 11)])                       # 128 parts per SM of 148; last warps of 1 and 3 parts
+@pytest.mark.parametrize("gate_first", [False, True])
+def test_gated_norm_of_many_parts(cuda, rows, parts, gs, gate_first, dtype):
+    from nano_vllm_rs_b200 import ops
+    g = torch.Generator(device=cuda).manual_seed(rows + gs)
+    y, z = [torch.randn(rows, parts * gs, generator=g, device=cuda) for _ in range(2)]
+    w = 1 + 0.1 * torch.randn(parts * gs, generator=g, device=cuda)
+    got = ops.gated_group_norm(y, z, w, parts, 1e-5, gate_first, dtype).double()
+    s = torch.nn.functional.silu(z.double())
+    v = (y.double() * s if gate_first else y.double()).reshape(rows, parts, gs)
+    ref = (v / (v.square().mean(-1, keepdim=True) + 1e-5).sqrt()).reshape(rows, -1) * (1 if gate_first else s) * w.double()
+    tol = 2e-6 + (2.0 ** -8 if dtype == torch.bfloat16 else 0)      # expf and a quotient (3 ulp), rsqrtf (2), the sum and four products: 16 * 2^-23
+    assert ((got - ref).abs() <= tol * ref.abs() + 1e-30).all()
