@@ -111,16 +111,7 @@ __device__ __forceinline__ void tma_load_2d(uint32_t smem_dst, const CUtensorMap
       "l"(m), "r"(bar), "r"(c0), "r"(c1)
       : "memory");
 }
-// 4-D tile load (paged KV: d, head, token-in-block, block).
-__device__ __forceinline__ void tma_load_4d(uint32_t smem_dst, const CUtensorMap* m, uint32_t bar,
-                                            int c0, int c1, int c2, int c3) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];\n" ::"r"(smem_dst),
-      "l"(m), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-      : "memory");
-}
-
-// The same as predicated instructions of a whole converged warp (see umma_bf16_ss_warp).
+// Loads (tiles of 3 and 5 dimensions) and the bytes to expect, as predicated instructions of a whole converged warp (see umma_bf16_ss_warp).
 __device__ __forceinline__ void mbar_expect_tx_warp(uint32_t bar, uint32_t bytes, uint32_t elected) {
   asm volatile(
       "{\n\t.reg .pred q;\n\t"
@@ -161,34 +152,22 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "n"(NCOLS) : "memory");
 }
 
-// D[tmem] (+)= A[smem desc] . B[smem desc];  accumulate == 0 overwrites D.
-__device__ __forceinline__ void umma_bf16_ss(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                             uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// D[tmem] (+)= A[tmem] . B[smem desc]: A (M = 128 lanes x K, 16-bit elements packed two per 32-bit column, K-major)
-// is read straight from tensor memory — used for P of the attention kernels.
-__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(tmem_d),
-      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// The same as predicated instructions of a whole converged warp: `elected` is 1 in the one lane that issues (elect_one(), always the same
+// D[tmem] (+)= A[smem desc] . B[smem desc], accumulate == 0 overwrites D; _ts: A (M = 128 lanes x K, 16-bit elements packed two per 32-bit
+// column, K-major) is read straight from tensor memory, for P of the attention kernels; commit: arrives (count 1) on `bar` once every
+// MMA that this thread issued before has completed.
+// These are predicated instructions of a whole converged warp: `elected` is 1 in the one lane that issues (elect_one(), always the same
 // lane).  Addresses and descriptors are then computed once per warp in uniform registers, where the instruction takes them; under an
 // `if (lane == 0)` every MMA first moves its own, and a thread issues one in about 130 clocks, twice what an M128 N128 K16 one runs for.
 // Descriptors come as their lower words (umma_desc_lo); the upper one is the same for all SWIZZLE_128B tiles here.  Before and after, in
 // turn on one GPU: 8192 x 4096 x 12288 672 and 583 us, 8192 x 6144 x 4096 322 and 286, 13420 x 1024 x 2048 42.3 and 39.9, 256 x 4096 x 1024
 // 10.6 and 8.1, 64 x 2048 x 8192 15.2 and 11.2; latent attention of 8 x 1024 tokens, 16 heads 472 and 390.
-constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);   // stride of 8 rows, version, SWIZZLE_128B (see umma_desc_sw128)
+// Shared-memory matrix descriptor (64-bit): start address [0,14) >>4, LBO [16,30) >>4, SBO [32,46) >>4,
+// version [46,48) = 1 on sm_100, base offset [49,52) = 0 (tiles are 1024-byte aligned), layout [61,64):
+// 2 = SWIZZLE_128B.
+//   K-major, SW128 (rows of 64 bf16 = 128 B, as TMA writes them): SBO = 8 rows * 128 B = 1024, LBO unused.
+//   MN-major, SW128 (rows = k index, 64 contiguous MN elements per row): SBO = 1024 (next 8 k),
+//   LBO = byte distance between consecutive 64-element MN groups.
+constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);   // SBO 1024, version 1, SWIZZLE_128B
 __device__ __forceinline__ uint32_t umma_desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) {
   return ((smem_addr & 0x3FFFFu) >> 4) | (lbo_bytes >> 4) << 16;
 }
@@ -222,11 +201,6 @@ __device__ __forceinline__ void umma_commit_warp(uint32_t bar, uint32_t elected)
       "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(bar), "r"(elected)
       : "memory");
 }
-// Arrives (count 1) on `bar` once every previously issued tcgen05.mma of this thread has completed.
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
-}
-
 // TMEM -> registers: this warp's 32 lanes x 32 consecutive fp32 columns (thread i <- lane base+i).
 __device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
@@ -310,16 +284,6 @@ __device__ __forceinline__ void tmem_dealloc_cg2(uint32_t taddr) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "n"(NCOLS) : "memory");
 }
 // D[tmem of both CTAs, 256 rows] (+)= A[128 rows from each CTA] . B[N/2 rows from each CTA]; leader CTA only.
-__device__ __forceinline__ void umma_bf16_ss_cg2(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                                 uint32_t accumulate) {
-  const uint32_t z = 0;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(z)
-      : "memory");
-}
 __device__ __forceinline__ void umma_bf16_ss_cg2_warp(uint32_t tmem_d, uint32_t adesc_lo, uint32_t bdesc_lo, uint32_t idesc,
                                                       uint32_t accumulate, uint32_t elected) {
   asm volatile(
@@ -332,6 +296,7 @@ __device__ __forceinline__ void umma_bf16_ss_cg2_warp(uint32_t tmem_d, uint32_t 
       "r"(adesc_lo), "r"(bdesc_lo), "r"(idesc), "r"(accumulate), "r"(elected), "r"(kDescHi)
       : "memory");
 }
+// Arrives on the barrier at this offset in every CTA of `cta_mask` once the issued cta_group::2 MMAs have completed.
 __device__ __forceinline__ void umma_commit_cg2_warp(uint32_t bar, uint16_t cta_mask, uint32_t elected) {
   asm volatile(
       "{\n\t.reg .pred q;\n\t"
@@ -340,29 +305,7 @@ __device__ __forceinline__ void umma_commit_cg2_warp(uint32_t bar, uint16_t cta_
       "h"(cta_mask), "r"(elected)
       : "memory");
 }
-// Arrives on the barrier at this offset in every CTA of `cta_mask` once the issued cta_group::2 MMAs have completed.
-__device__ __forceinline__ void umma_commit_cg2(uint32_t bar, uint16_t cta_mask) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(bar),
-               "h"(cta_mask)
-               : "memory");
-}
-
 // ---- descriptors -----------------------------------------------------------------------------------
-// Shared-memory matrix descriptor (64-bit): start address [0,14) >>4, LBO [16,30) >>4, SBO [32,46) >>4,
-// version [46,48) = 1 on sm_100, base offset [49,52) = 0 (tiles are 1024-byte aligned), layout [61,64):
-// 2 = SWIZZLE_128B.
-//   K-major, SW128 (rows of 64 bf16 = 128 B, as TMA writes them): SBO = 8 rows * 128 B = 1024, LBO unused.
-//   MN-major, SW128 (rows = k index, 64 contiguous MN elements per row): SBO = 1024 (next 8 k),
-//   LBO = byte distance between consecutive 64-element MN groups.
-__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);
-  d |= static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFFu) << 16;
-  d |= static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFFu) << 32;
-  d |= static_cast<uint64_t>(1) << 46;
-  d |= static_cast<uint64_t>(2) << 61;
-  return d;
-}
 // Instruction descriptor for kind::f16, bf16 x bf16 -> f32: c_format[4,6)=1, a_format[7,10)=1,
 // b_format[10,13)=1, a_major[15], b_major[16] (0 = K-major, 1 = MN-major), N>>3 [17,23), M>>4 [24,29).
 __host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n, int a_mn_major, int b_mn_major) {
