@@ -401,6 +401,7 @@ extern "C" int nvllm_moe_sort_weighted(int32_t* row_token, float* row_weight, in
   // A cluster from the size on where its two barriers cost less than they save (8 experts, one CTA and eight: 4.1 and 4.4 us at 1024
   // assignments, 4.6 and 4.5 at 2048, 5.8 and 4.6 at 4096); a thread of it holds one expert's counts.
   const bool cluster = static_cast<int64_t>(n) * top >= 2048 && experts <= 1024;
+  NVLLM_SMEM_ATTR_ONCE(moe_sort_kernel<1>, 48 * 1024);   // (up to 6143 experts beside the scan's 128 bytes)
   NVLLM_CUDA(launch_pdl_cluster(cluster ? moe_sort_kernel<8> : moe_sort_kernel<1>, dim3(cluster ? 8 : 1), dim3(1024), cluster ? 8 : 1, smem,
                                 static_cast<cudaStream_t>(stream), row_token, tile_expert, slot_row, row_weight, topk_idx, topk_w, n * top, top, experts, max_rows, tile_rows));
   NVLLM_LAUNCH_CHECK("moe_sort_kernel");
