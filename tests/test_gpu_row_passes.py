@@ -93,3 +93,22 @@ def test_gated_norm_of_many_parts(cuda, rows, parts, gs, gate_first, dtype):
     ref = (v / (v.square().mean(-1, keepdim=True) + 1e-5).sqrt()).reshape(rows, -1) * (1 if gate_first else s) * w.double()
     tol = 2e-6 + (2.0 ** -8 if dtype == torch.bfloat16 else 0)      # expf and a quotient (3 ulp), rsqrtf (2), the sum and four products: 16 * 2^-23
     assert ((got - ref).abs() <= tol * ref.abs() + 1e-30).all()
+
+
+@pytest.mark.parametrize("n", [1, 592, 593])                                                       # up to four tokens per SM of 148: two CTAs a token
+def test_delta_preparation(cuda, n):
+    from nano_vllm_rs_b200 import ops
+    H, G, D = 3, 2, 128
+    g = torch.Generator(device=cuda).manual_seed(n)
+    rn = lambda *s: torch.randn(*s, generator=g, device=cuda)
+    q, k, beta, raw, alog, bias = rn(n, G * D), rn(n, G * D), rn(n, H), 2 * rn(n, H * D), rn(H), rn(H * D)
+    want = []
+    for x, scale in ((q, 0.5), (k, 1.0)):
+        v = x.double().reshape(n, G, D)
+        want.append((v * scale / (v.square().sum(-1, keepdim=True) + 1e-6).sqrt()).reshape(n, -1))
+    want.append(beta.double().sigmoid())
+    want.append((-alog.double().exp().repeat_interleave(D) * torch.nn.functional.softplus(raw.double() + bias.double())).exp())
+    ops.delta_prepare(q, k, beta, raw, alog, bias, H, G, D, 0.5)
+    for got, ref in zip((q, k, beta, raw), want):
+        # unit vectors and sigmoids: a few roundings each; a decay exp(-x) has x's relative error (8 * 2^-24) times x, at most 745
+        assert ((got.double() - ref).abs() <= 2e-6 * ref.abs() * (1 + ref.abs().clamp(min=1e-300).log().abs()) + 1e-37).all()
