@@ -60,6 +60,8 @@ static_assert(kSmemClaim % 16 == 0, "the claim's answer is written as 16 bytes")
 
 struct PrefillParams {
   bf16* out;
+  const bf16 *q, *k, *v;   // what the maps cover, for rows that are computed alone (row_alone)
+  int64_t ldq, k_tok, k_head, k_blk, v_tok, v_head, v_blk, rows_k;   // strides in elements; rows_k: rows of dense K/V
   const int32_t* cu_q;
   const int32_t* cu_k;
   const int32_t* tables;  // NULL: dense K/V
@@ -203,6 +205,76 @@ __device__ __forceinline__ void exp_chunk(uint32_t (&s)[32], uint32_t (&pk)[16],
 // tanh(x) = 1 - 2 / (2^(2 x log2 e) + 1): absolute error ~1e-6, exact at both saturations (as in the kernels of capped_attn.cu)
 __device__ __forceinline__ float ratio_tanh(float x) { return 1.0f - __fdividef(2.0f, fast_exp2(x * 2.8853900817779268f) + 1.0f); }
 
+// EXT: the factor on a row's accumulated values, from its maximum (log2 units) and sum: 1 / sum, with the sink and the head's gate.
+__device__ __forceinline__ float row_factor(const PrefillParams& p, int64_t tok, int head, float m, float l) {
+  float inv = l > 0.f ? 1.0f / l : 0.f;
+  if (p.e.sinks != nullptr) {   // the sink joins the denominator only
+    const float sk = __ldg(p.e.sinks + head) * 1.4426950408889634f, mn = fmaxf(m, sk), oc = fast_exp2(m - mn);
+    const float ll = l * oc + fast_exp2(sk - mn);
+    inv = ll > 0.f ? oc / ll : 0.f;
+  }
+  if (p.e.gate != nullptr && p.e.gate_per_head) inv *= 1.0f / (1.0f + __expf(-__ldg(p.e.gate + tok * p.e.ldg + head)));
+  return inv;
+}
+
+// One row by one warp, over the keys [from, vis) that it sees and no others.  P is 0 for the keys of a tile that a row does not see (later
+// tokens, keys before its window, rows of the next sequence, the unwritten rest of a block), but 0 x NaN and 0 x Inf are NaN: a value there
+// that is no number would reach the row through the tile's P.V.  So rows whose O is not finite are computed again here; inputs
+// that are numbers never get here.  The test is 64 instructions a row beside the 192 and more of every tile (two prompts of 4096 tokens at the
+// 8B widths, whole steps without and with it: 27.79 and 27.83 ms, runs of one side 1.4 % apart).  qscale: factor on the score before the cap, or to
+// log2 units.
+template <bool EXT>
+__device__ __noinline__ void row_alone(const PrefillParams& p, int seq, int64_t tok, int head, int kvh, int k0, int from, int vis, float qscale) {
+  const int lane = threadIdx.x & 31;
+  auto load4 = [&](const bf16* at, float (&x)[4]) {
+    const uint2 u = *reinterpret_cast<const uint2*>(at + 4 * lane);
+    x[0] = bf16_lo(u.x); x[1] = bf16_hi(u.x); x[2] = bf16_lo(u.y); x[3] = bf16_hi(u.y);
+  };
+  const int32_t* table = p.tables ? p.tables + static_cast<int64_t>(seq) * p.max_blocks : nullptr;
+  float q[4], acc[4] = {}, m = -INFINITY, l = 0.f;
+  load4(p.q + tok * p.ldq + static_cast<int64_t>(head) * D, q);
+#pragma unroll 4
+  for (int j = from; j < vis; ++j) {
+    int64_t blk = 0, at = static_cast<int64_t>(k0) + j;
+    bool there = at < p.rows_k;
+    if (table != nullptr) {
+      const int b = j / p.block_size;
+      blk = b < p.max_blocks ? table[b] : -1;
+      at = j - b * p.block_size;
+      there = blk >= 0;
+    }
+    float k[4] = {}, v[4] = {};   // (a block that is not there: zeros, as in the tiles)
+    if (there) {
+      load4(p.k + blk * p.k_blk + at * p.k_tok + kvh * p.k_head, k);
+      load4(p.v + blk * p.v_blk + at * p.v_tok + kvh * p.v_head, v);
+    }
+    float s = fmaf(q[0], k[0], fmaf(q[1], k[1], fmaf(q[2], k[2], q[3] * k[3])));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    s *= qscale;
+    if constexpr (EXT) {
+      if (p.e.softcap > 0.f) s = p.e.softcap * 1.4426950408889634f * ratio_tanh(s);
+    }
+    const float mn = fmaxf(m, s), corr = m == -INFINITY ? 0.f : fast_exp2(m - mn), w = fast_exp2(s - (mn == -INFINITY ? 0.f : mn));
+    m = mn;
+    l = l * corr + w;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[e] = fmaf(w, v[e], j == from ? 0.f : acc[e] * corr);
+  }
+  float inv = l > 0.f ? 1.0f / l : 0.f;
+  if constexpr (EXT) {
+    inv = row_factor(p, tok, head, m, l);
+    if (p.e.gate != nullptr && !p.e.gate_per_head) {
+      const float4 g = __ldg(reinterpret_cast<const float4*>(p.e.gate + tok * p.e.ldg + head * D) + lane);
+      const float x[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[e] *= 1.0f / (1.0f + __expf(-x[e]));
+    }
+  }
+  *reinterpret_cast<uint2*>(p.out + tok * p.out_stride + static_cast<int64_t>(head) * D + 4 * lane) =
+      make_uint2(pack_bf16x2(acc[0] * inv, acc[1] * inv), pack_bf16x2(acc[2] * inv, acc[3] * inv));
+}
+
 __device__ __forceinline__ float max3(uint32_t a, uint32_t b, float m) {
   float r;
   asm("max.f32 %0, %1, %2, %3;\n" : "=f"(r) : "f"(__uint_as_float(a)), "f"(__uint_as_float(b)), "f"(m));
@@ -229,7 +301,7 @@ __device__ __forceinline__ uint64_t sum32(const uint32_t (&s)[32], uint64_t acc)
 template <bool EXT>
 __global__ void __launch_bounds__(pf::kThreads, 1)
 prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                    const __grid_constant__ CUtensorMap tmap_v, const PrefillParams p) {
+                    const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ PrefillParams p) {
   using namespace pf;
   pdl_launch_dependents();
   extern __shared__ uint8_t smem_raw[];
@@ -580,21 +652,18 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         };
         const bool gated = EXT && p.e.gate != nullptr && !p.e.gate_per_head;
         if constexpr (EXT) {
-          if (p.e.sinks != nullptr) {   // the sink joins the denominator only
-            const float sk = __ldg(p.e.sinks + head) * 1.4426950408889634f, mn = fmaxf(m_ref, sk), oc = fast_exp2(m_ref - mn);
-            const float ll = l_run * oc + fast_exp2(sk - mn);
-            inv = ll > 0.f ? oc / ll : 0.f;
-          }
-          if (p.e.gate != nullptr && p.e.gate_per_head)
-            inv *= 1.0f / (1.0f + __expf(-__ldg(p.e.gate + static_cast<int64_t>(it.q0 + min(row, it.Lq - 1)) * p.e.ldg + head)));
+          inv = row_factor(p, it.q0 + min(row, it.Lq - 1), head, m_ref, l_run);
           if (gated) load_gate(0);
         }
         bf16* orow = p.out + static_cast<int64_t>(it.q0 + row) * p.out_stride + head * D;
+        float most = 0.f;   // largest |O| of the row, no number if one of them is none
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
           uint32_t orr[32];
           tmem_ld_32x32b_x32(tO + c * 32, orr);
           tmem_ld_wait(orr);
+#pragma unroll
+          for (int e = 0; e < 32; e += 2) most = abs_max(__uint_as_float(orr[e]), __uint_as_float(orr[e + 1]), most);
           if constexpr (EXT) {
             if (gated) {
 #pragma unroll
@@ -627,6 +696,12 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           }
         }
         tc_fence_before();   // ordered before the first P of the next item, whose P.V overwrites O
+        for (uint32_t odd = __ballot_sync(0xffffffffu, row < it.Lq && !(most < INFINITY)); odd != 0u; odd &= odd - 1) {   // (stored above: stored again)
+          const int src = __ffs(odd) - 1;
+          __syncwarp();
+          row_alone<EXT>(p, it.seq, it.q0 + row - lane + src, head, it.kvh, it.k0, __shfl_sync(0xffffffffu, from, src), __shfl_sync(0xffffffffu, vis, src),
+                         EXT ? __shfl_sync(0xffffffffu, qscale, src) : p.scale_log2);
+        }
       }
     }
   }
@@ -685,6 +760,16 @@ int prompt_attention(const PromptAttn& e, void* out, int64_t ldo, const void* q,
     p.max_blocks = table_cap;
   }
   p.out = static_cast<bf16*>(out);
+  p.q = static_cast<const bf16*>(q);
+  p.k = static_cast<const bf16*>(k);
+  p.v = static_cast<const bf16*>(v);
+  p.ldq = ldq;
+  p.k_tok = k_row;
+  p.v_tok = v_row;
+  p.k_head = p.v_head = pf::D;
+  p.k_blk = k_row * block_size;
+  p.v_blk = v_row * block_size;
+  p.rows_k = n;
   p.cu_q = p.cu_k = cu_tokens;
   p.tables = tables;
   p.H = heads;
@@ -751,6 +836,14 @@ extern "C" int nvllm_varlen_prefill_attention(void* out, const void* q, const vo
     p.max_blocks = max_blocks_per_seq;
   }
   p.out = static_cast<bf16*>(out);
+  p.q = static_cast<const bf16*>(q);
+  p.k = static_cast<const bf16*>(paged ? k_cache : k);
+  p.v = static_cast<const bf16*>(paged ? v_cache : v);
+  p.ldq = q_token_stride;
+  p.k_tok = p.v_tok = paged ? layout->token_stride : kv_token_stride;
+  p.k_head = p.v_head = paged ? layout->head_stride : pf::D;
+  p.k_blk = p.v_blk = paged ? layout->block_stride : 0;
+  p.rows_k = total_k;
   p.cu_q = cu_seqlens_q;
   p.cu_k = cu_seqlens_k;
   p.tables = block_tables;

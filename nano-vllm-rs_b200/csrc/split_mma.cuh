@@ -13,12 +13,6 @@ __device__ __forceinline__ void cp_async_4(uint32_t smem_addr, const void* gptr)
 
 __device__ __forceinline__ uint32_t abs_bits(float x) { return __float_as_uint(x) & 0x7fffffffu; }
 
-// max(|a|, |b|, m), no number if one of them is none
-__device__ __forceinline__ float abs_max(float a, float b, float m) {
-  float r;
-  asm("max.NaN.f32 %0, %1, %2, %3;\n" : "=f"(r) : "f"(fabsf(a)), "f"(fabsf(b)), "f"(m));
-  return r;
-}
 __device__ __forceinline__ bool far_off(uint32_t bits, int lo, int hi) {   // not zero and outside [2^lo, 2^hi)
   return bits != 0u && (bits < (static_cast<uint32_t>(127 + lo) << 23) || bits >= (static_cast<uint32_t>(127 + hi) << 23));
 }

@@ -138,3 +138,40 @@ def test_varlen_prefill_many_ragged_items(cuda, H, Hkv, top, paged):
             ref = torch.einsum("hqk,khd->qhd", s.masked_fill(hidden, -float("inf")).softmax(-1), vs[b].float().repeat_interleave(H // Hkv, 1))
             assert_close(to_np_f32(out[at:at + n]), to_np_f32(ref), ATT_ATOL, ATT_RTOL, f"sequence {b}: {n} of {tot[b]}")
         at += n
+
+
+@pytest.mark.parametrize("paged", [False, True])
+@pytest.mark.parametrize("H,Hkv", [(4, 2), (3, 3)])
+def test_no_number_reaches_only_the_tokens_that_see_it(cuda, H, Hkv, paged):
+    """NaN in the second sequence's keys and values, in one value in the middle of the first, and behind its last token in its block: rows that see
+    none of them are what they are without them."""
+    from nano_vllm_rs_b200 import ops
+    from nano_vllm_rs_b200._ffi import KvLayout
+    D, bs, lens, mid = 128, 256, [300, 200], 170
+    rng = np.random.default_rng(3)
+    kc, vc, tables, ks, vs = make_paged_kv(rng, lens, bs, Hkv, D)
+    cu = torch.from_numpy(_cu(lens)).to(cuda)
+    q = to_dev_bf16(randn_bf16(rng, (sum(lens), H, D)), cuda)
+    if paged:
+        kd, vd = (cache_to_layout(x, "reference", cuda) for x in (kc, vc))
+        flat = lambda x: x.view(-1, Hkv, D)
+        row = lambda s, j: int(tables[s, j // bs]) * bs + j % bs
+        call = lambda: ops.varlen_prefill_attention(q, None, None, cu, cu, max(lens), max(lens), k_cache=kd, v_cache=vd,
+                                                    block_tables=torch.from_numpy(tables).to(cuda), layout=KvLayout.reference(bs, Hkv, D))
+    else:
+        kd, vd = (to_dev_bf16(np.concatenate(x), cuda) for x in (ks, vs))
+        flat = lambda x: x
+        row = lambda s, j: sum(lens[:s]) + j
+        call = lambda: ops.varlen_prefill_attention(q, kd, vd, cu, cu, max(lens), max(lens))
+    clean = call()
+    for j in range(lens[1]): flat(kd)[row(1, j)], flat(vd)[row(1, j)] = float("nan"), float("nan")
+    flat(vd)[row(0, mid), 0, 5] = float("nan")
+    if paged:
+        for j in range(lens[0], -(-lens[0] // bs) * bs): flat(kd)[row(0, j)], flat(vd)[row(0, j)] = float("nan"), float("inf")
+    out = call()
+    torch.cuda.synchronize()
+    hit = torch.zeros_like(out, dtype=torch.bool)
+    hit[mid:lens[0], :H // Hkv, 5] = True
+    hit[lens[0]:] = True
+    assert torch.equal(torch.isnan(out), hit)
+    assert_close(to_np_f32(out[~hit]), to_np_f32(clean[~hit]), ATT_ATOL, ATT_RTOL, "rows that do not see it")

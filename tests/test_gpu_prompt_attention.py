@@ -89,3 +89,60 @@ def test_prompt_attention_against_torch(cuda, case, monkeypatch):
         assert_close(to_np_f32(out[at:at + n]), ref, ATOL, RTOL, f"sequence {s}")
         assert_close(to_np_f32(other[at:at + n]), ref, ATOL, RTOL, f"sequence {s} on mma.sync")
         at += n
+
+
+def _causal(q, k, v, starts, window):
+    """Plain causal (and windowed) attention of one sequence in f32: q [n, heads, D], k / v [keys, kv heads, D]; what a row does not see never touches it."""
+    n, heads = q.shape[:2]
+    pos, j = torch.arange(starts, starts + n, device=q.device), torch.arange(len(k), device=q.device)
+    hidden = j[None] > pos[:, None]
+    if window:
+        hidden = hidden | (j[None] <= pos[:, None] - window)
+    rep = heads // k.shape[1]
+    x = (torch.einsum("qhd,khd->hqk", q.float(), k.float().repeat_interleave(rep, 1)) * D ** -0.5).masked_fill(hidden, -float("inf"))
+    return torch.einsum("hqk,khd->qhd", x.softmax(-1), v.float().repeat_interleave(rep, 1)), ~hidden
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("heads,kv_heads,lens,starts,bs,window,sinks,gate", [
+    (4, 2, [300, 77, 200], None, 0, 0, False, 0), (3, 3, [257, 130], None, 0, 100, True, 2), (8, 2, [130, 100, 333], None, 256, 0, True, 1),
+    (4, 1, [200, 100], [300, 63], 16, 70, False, 2), (2, 1, [128, 128], [0, 0], 64, 0, False, 0)])
+def test_no_number_reaches_only_the_tokens_that_see_it(cuda, heads, kv_heads, lens, starts, bs, window, sinks, gate, bad):
+    """NaN or infinity in the values (and NaN in the keys) of every sequence's first token but the first sequence's, of one token in the middle of the
+    first sequence, and in whatever its blocks hold behind its last token: a row that sees none of them is what it is without them, one that sees
+    a value is not finite in that column and the same elsewhere."""
+    from nano_vllm_rs_b200 import ops
+    q, ks, vs, kc, vc, tables, meta, gates, sink, starts = _inputs(cuda, heads, kv_heads, lens, starts, bs, 0.0, 0.0, sinks, gate)
+
+    def call():
+        return ops.window_attention(q, gates, kc, vc, meta["tok_seq"], meta["positions"], tables, bs or 256, heads, kv_heads, D, D, D ** -0.5, window=window,
+                                    sinks=sink, gate_per_head=gate == 1, cu_tokens=meta["cu"])
+
+    clean = call()
+    cu, mid, col = meta["cu"].tolist(), starts[0] + lens[0] // 2 + 3, 21
+    row = lambda s, j: int(tables[s, j // bs]) * bs + j % bs if bs else cu[s] + j
+    for s in range(1, len(lens)):
+        kc[row(s, 0)], vc[row(s, 0)] = float("nan"), bad
+    vc[row(0, mid), col] = bad                                   # one column of the first kv head
+    if bs:
+        for s, n in enumerate(lens):
+            for j in range(starts[s] + n, -(-(starts[s] + n) // bs) * bs):
+                kc[row(s, j)], vc[row(s, j)] = float("nan"), bad
+    out = call()
+    torch.cuda.synchronize()
+    ref, seen = _causal(q[:lens[0]].view(lens[0], heads, D), ks[0], vs[0], starts[0], window)
+    got, was = out[:lens[0]].view(lens[0], heads, D), clean[:lens[0]].view(lens[0], heads, D)
+    hit = torch.zeros_like(got, dtype=torch.bool)
+    hit[seen[:, mid], :heads // kv_heads, col] = True
+    assert hit.any() and not hit.all(0).any()
+    assert not torch.isfinite(got[hit]).any() and torch.isfinite(got[~hit]).all()
+    assert_close(to_np_f32(got[~hit]), to_np_f32(was[~hit]), ATOL, RTOL, "rows that do not see it")
+    if not sinks and not gate:
+        assert_close(to_np_f32(got[~hit]), to_np_f32(ref[~hit]), ATOL, RTOL, "against torch")
+    for s in range(1, len(lens)):                               # the others: rows whose window has left their first token behind
+        pos = torch.arange(starts[s], starts[s] + lens[s], device=cuda)
+        free = (pos >= window) if window else torch.zeros_like(pos, dtype=torch.bool)
+        a, b = out[cu[s]:cu[s + 1]], clean[cu[s]:cu[s + 1]]
+        assert torch.isnan(a[~free].float()).all()
+        assert torch.equal(torch.isfinite(a).all(1), free)
+        assert_close(to_np_f32(a[free]), to_np_f32(b[free]), ATOL, RTOL, f"sequence {s}")
