@@ -109,9 +109,9 @@ __device__ __forceinline__ bool decode_item(const PrefillParams& p, int bx, int 
   return true;
 }
 
-// EXT: blocks of all sequences in one row (by), the last block of the last sequence first.  A whole converged warp; lane i looks at sequence i of 32.
-__device__ __forceinline__ bool decode_prompt_item(const PrefillParams& p, int bx, int by, Item& it) {
-  const int lane = threadIdx.x & 31, rows = p.pair ? BM : 2 * BM;
+// EXT: grid.x = units * blocks of all sequences, the last block of the last sequence first.  A whole converged warp; lane i looks at sequence i of 32.
+__device__ __forceinline__ bool decode_prompt_item(const PrefillParams& p, int index, Item& it) {
+  const int by = index / p.units, bx = index - by * p.units, lane = threadIdx.x & 31, rows = p.pair ? BM : 2 * BM;
   auto blocks_of = [&](int s) { return s < p.e.n_seqs ? (__ldg(p.cu_q + s + 1) - __ldg(p.cu_q + s) + rows - 1) / rows : 0; };
   int total = 0;
   for (int s = lane; s < p.e.n_seqs; s += 32) total += blocks_of(s);
@@ -338,7 +338,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   pdl_wait();  // q / k / v (and the cache) come from the previous kernel
 
   auto item_of = [&](int x, int y, int z, Item& it) {
-    if constexpr (EXT) return decode_prompt_item(p, x, y, it);
+    if constexpr (EXT) return decode_prompt_item(p, x, it);
     else return decode_item(p, x, y, z, it);
   };
   // Every role walks the same list of items: its own block index, then what warp 10 publishes.
@@ -736,7 +736,8 @@ static bool heads_pair(int heads, int kv_heads) { return (heads / kv_heads) % 2 
 // 16 heads 198 and 76; 8192 tokens capped 1354 and 569).
 bool prompt_attention_applies(const PromptAttn& e, int n, int heads, int kv_heads, int dim, int vdim, int64_t ldq, int64_t k_row, int64_t v_row, int64_t ldo,
                               const void* out, const void* q, const void* k, const void* v, bool paged, int block_size) {
-  return dim == pf::D && vdim == pf::D && e.n_seqs <= 4096 && n >= 96 * static_cast<int64_t>(e.n_seqs) && ldq % 8 == 0 && k_row % 8 == 0 && v_row % 8 == 0 &&
+  const int64_t blocks = n / pf::BM + 1 + e.n_seqs;   // at the most; a grid's first dimension holds 2^31 - 1 CTAs
+  return dim == pf::D && vdim == pf::D && e.n_seqs <= 4096 && blocks * heads <= INT32_MAX && n >= 96 * static_cast<int64_t>(e.n_seqs) && ldq % 8 == 0 && k_row % 8 == 0 && v_row % 8 == 0 &&
          ldo % 8 == 0 && aligned16(out) && aligned16(q) && aligned16(k) && aligned16(v) && heads <= 65535 &&
          (!paged || (block_size % 16 == 0 && (block_size >= pf::BN ? block_size % pf::BN == 0 : pf::BN % block_size == 0))) &&
          (e.gate == nullptr || e.gate_per_head || (aligned16(e.gate) && e.ldg % 4 == 0)) && k_row >= static_cast<int64_t>(kv_heads) * dim &&
@@ -780,8 +781,9 @@ int prompt_attention(const PromptAttn& e, void* out, int64_t ldo, const void* q,
   p.units = p.pair ? heads / 2 : heads;
   p.z_blocks = 1;
   const int rows = p.pair ? pf::BM : 2 * pf::BM;
+  const int64_t blocks = (static_cast<int64_t>(n) + rows - 1) / rows + e.n_seqs;
   NVLLM_SMEM_ATTR_ONCE(prefill_attn_kernel<true>, pf::kSmemBytesExt);
-  NVLLM_CUDA(launch_plain(prefill_attn_kernel<true>, dim3(p.units, (n + rows - 1) / rows + e.n_seqs), dim3(pf::kThreads), pf::kSmemBytesExt, st, tq, tk, tv, p));
+  NVLLM_CUDA(launch_plain(prefill_attn_kernel<true>, dim3(static_cast<unsigned>(p.units * blocks)), dim3(pf::kThreads), pf::kSmemBytesExt, st, tq, tk, tv, p));
   NVLLM_LAUNCH_CHECK("prefill_attn_kernel");
   return 0;
 }

@@ -146,3 +146,21 @@ def test_no_number_reaches_only_the_tokens_that_see_it(cuda, heads, kv_heads, le
         assert torch.isnan(a[~free].float()).all()
         assert torch.equal(torch.isfinite(a).all(1), free)
         assert_close(to_np_f32(a[free]), to_np_f32(b[free]), ATOL, RTOL, f"sequence {s}")
+
+
+def test_more_blocks_than_a_grid_has_rows(cuda):
+    """7.9 million tokens in 4000 sequences: more blocks of 128 rows than the 65535 of gridDim.y."""
+    from nano_vllm_rs_b200 import ops
+    heads, n_seqs, L, window = 2, 4000, 1970, 64
+    n = n_seqs * L
+    assert n // 128 + n_seqs > 65535
+    g = torch.Generator(device="cuda").manual_seed(0)
+    q, k, v = (torch.randn(n, w * D, generator=g, device=cuda, dtype=torch.bfloat16) for w in (heads, 1, 1))
+    cu = torch.arange(0, n + 1, L, dtype=torch.int32, device=cuda)
+    out = ops.window_attention(q, None, k, v, torch.arange(n_seqs, dtype=torch.int32, device=cuda).repeat_interleave(L), torch.arange(L, device=cuda).repeat(n_seqs),
+                               None, 256, heads, 1, D, D, D ** -0.5, window=window, cu_tokens=cu)
+    torch.cuda.synchronize()
+    for s in (0, 1999, 3999):
+        rows = slice(s * L, (s + 1) * L)
+        ref, _ = _causal(q[rows].view(L, heads, D), k[rows].view(L, 1, D), v[rows].view(L, 1, D), 0, window)
+        assert_close(to_np_f32(out[rows]), to_np_f32(ref.flatten(1)), ATOL, RTOL, f"sequence {s}")
