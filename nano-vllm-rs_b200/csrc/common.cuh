@@ -119,8 +119,9 @@ namespace nvllm {
 // Most kernels of a step are launched with cudaLaunchAttributeProgrammaticStreamSerialization (launch_pdl): such a kernel may start while
 // its predecessor is still running.  Contract: before pdl_wait() only work that does not depend on the predecessor (barrier init, TMEM
 // alloc, descriptor / weight prefetch), after it everything that a previous kernel wrote or still reads.  pdl_launch_dependents() lets the
-// successor be scheduled: first thing in most kernels; after pdl_wait() where CTAs of several kernels of the chain on one SM cost more than
-// the overlap gives (the kernel says so).  Kernels that launch_plain starts wait for their predecessor in stream order; pdl_wait()
+// successor be scheduled: first thing in most kernels; behind the allocation in those that use tensor memory (tcgen05.alloc waits for columns
+// without a limit: a successor's CTA that took them first would wait for this kernel, which would wait for it); after pdl_wait() where CTAs of
+// several kernels of the chain on one SM cost more than the overlap gives (the kernel says so).  Kernels that launch_plain starts wait for their predecessor in stream order; pdl_wait()
 // returns at once in them.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }

@@ -78,7 +78,6 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
   const int tile = static_cast<int>(blockIdx.x) / SK;
   const int m_tile = tile % num_m_tiles, n_tile = tile / num_m_tiles;
   const int kb_per = (K / C::BK) / SK, kb0 = rank * kb_per;
-  pdl_launch_dependents();
 
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tmap_x);
@@ -92,6 +91,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
   if (warp == 2) tmem_alloc<C::kTmemCols>(tmem_slot);
   tc_fence_before();
   __syncthreads();
+  pdl_launch_dependents();   // (behind the allocation)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
 

@@ -105,7 +105,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
   const int num_kb = K / C::BK;
   const int n_fast = tile_group != nullptr ? num_tiles / num_m_tiles : 0;   // grouped: n-tiles run fastest
   const int cta0 = static_cast<int>(blockIdx.x), cta_stride = static_cast<int>(gridDim.x);
-  pdl_launch_dependents();  // everything up to pdl_wait() below is independent of the previous kernel
 
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tmap_x);
@@ -125,6 +124,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
   if (warp == 2) tmem_alloc<C::kTmemCols>(tmem_slot);
   tc_fence_before();
   __syncthreads();
+  pdl_launch_dependents();  // (behind the allocation; everything up to pdl_wait() below is independent of the previous kernel)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
 

@@ -190,7 +190,6 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
   const bool leader = rank == 0;
   const int num_kb = K / C::BK;
   const int cluster_id = blockIdx.x >> 1, num_clusters = gridDim.x >> 1;
-  pdl_launch_dependents();
 
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tmap_x);
@@ -210,6 +209,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
   if (warp == 2) tmem_alloc_cg2<C::kTmemCols>(tmem_slot);
   tc_fence_before();
   cluster_sync_all();  // barriers of BOTH CTAs are initialised before any remote signal can arrive
+  pdl_launch_dependents();   // (behind the allocation)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
   [[maybe_unused]] uint32_t* const pairs = tmem_slot_ptr + 4;   // GROUPED: m-tile | second half live << 12 | group << 13

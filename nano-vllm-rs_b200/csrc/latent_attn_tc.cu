@@ -117,7 +117,6 @@ __device__ __noinline__ void row_alone(const LatentAttnArgs& a, int tok, int hea
 
 __global__ void __launch_bounds__(kThreads, 1) latent_attn_tc_kernel(const __grid_constant__ LatentAttnArgs a, int halves) {
   pdl_wait();
-  pdl_launch_dependents();
   extern __shared__ uint8_t smem_raw[];
   const int tile = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);   // late tokens of the batch (most keys) first
   if (!latent_tile_dense(a.tok_seq, a.n, tile)) return;
@@ -143,6 +142,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_attn_tc_kernel(const __gri
   if (warp == 8) tmem_alloc<512>(tmem_slot);
   tc_fence_before();
   __syncthreads();
+  pdl_launch_dependents();   // (behind the allocation)
   tc_fence_after();
   const uint32_t tmem = *reinterpret_cast<uint32_t*>(gen + kSmemBar + 9 * 8);
   const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;

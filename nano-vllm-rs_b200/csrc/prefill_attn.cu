@@ -303,7 +303,6 @@ __global__ void __launch_bounds__(pf::kThreads, 1)
 prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ PrefillParams p) {
   using namespace pf;
-  pdl_launch_dependents();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -334,6 +333,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_launch_dependents();   // (behind the allocation)
   const uint32_t tmem_base = *reinterpret_cast<uint32_t*>(smem_gen + kSmemTmem);
   pdl_wait();  // q / k / v (and the cache) come from the previous kernel
 
