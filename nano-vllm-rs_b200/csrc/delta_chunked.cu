@@ -8,8 +8,9 @@
 //
 // Precision: as in recurrence_chunked.cu, three bf16 pieces and six products of every f32 operand, hi.hi summed apart; the solve is f32.
 // A chunk with a decay outside [0, 1] or a product of decays below 2^-90, or with a value that is no number, infinite or far from the
-// others' range (q outside 2^-30 .. 2^30, k outside 2^-30 .. 2^8, beta, v or the state beyond 2^4, 2^20), is stepped through token by token in f32 by the warps that it concerns: what such a value
-// reaches is then the same as in the general kernel.
+// others' range (q outside 2^-30 .. 2^30, k outside 2^-30 .. 2^8, beta, v or the state beyond 2^4, 2^20), or where U grows beyond 2^64 (keys
+// far from unit vectors), is stepped through token by token in f32 by the warps that it concerns: what such a value reaches is then the same as
+// in the general kernel.  (P is 0 where a token does not see a later one's u, but 0 x Inf is NaN.)
 //
 // CTA = (head, sequence, 64 columns of v), 4 warps; a warp keeps 16 columns of the state, transposed, in the accumulator layout of m16n8k16
 // (64 registers), which is also that of the B operand of (G * K) S and (G * q) S.  q, k and the decays of the next chunk fly (cp.async) under the
@@ -236,7 +237,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) delta_chunked_kernel(const Del
       smax[0] = abs_max(S[n][0], S[n][1], smax[0]);
       smax[1] = abs_max(S[n][2], S[n][3], smax[1]);
     }
-    const bool step = __any_sync(0xffffffffu, slow || !(smax[0] < 1.0e6f && smax[1] < 1.0e6f));      // 2^20: k / G reaches 2^98
+    bool step = __any_sync(0xffffffffu, slow || !(smax[0] < 1.0e6f && smax[1] < 1.0e6f));      // 2^20: k / G reaches 2^98
     float sy[2][2][4] = {};            // [G * k, G * q] . S: [16 tokens][8 columns]
     if (!step) {
       float hh[2][2][4], lo[2][2][4] = {};
@@ -295,6 +296,10 @@ __global__ void __launch_bounds__(kWarps * 32, 2) delta_chunked_kernel(const Del
             if (4 * q4 + 3 > j) u[4 * q4 + 3] = fmaf(-c.w, u[j], u[4 * q4 + 3]);
           }
         }
+        float umax = 0.f;
+#pragma unroll
+        for (int i = 0; i < kC; i += 2) umax = abs_max(u[i], u[i + 1], umax);
+        step = __any_sync(0xffffffffu, !(umax < 1.8e19f));     // 2^64: P reaches 2^45
         __syncwarp();
         if (lane < 16) {
 #pragma unroll
@@ -302,6 +307,8 @@ __global__ void __launch_bounds__(kWarps * 32, 2) delta_chunked_kernel(const Del
         }
         __syncwarp();
       }
+    }
+    if (!step) {
       uint32_t uf[3][2][2], ua[1][3][4];   // U as B (16 tokens x 8 columns) and, the same values, U^T as A
 #pragma unroll
       for (int n = 0; n < 2; ++n)

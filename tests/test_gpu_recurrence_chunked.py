@@ -104,17 +104,18 @@ def test_odd_values(cuda, what):
 
 # ------------------------------------------------------------------------------------------------------------ the gated delta rule
 def _delta_reference(q, k, v, g, b, S):
-    """One sequence in float64: y, the final state, and the largest column norm that the state had (the error's scale)."""
-    n, H, dv = v.shape
-    y, S, top = np.empty_like(v), S.copy(), np.zeros((H, dv))
-    with np.errstate(all="ignore"):
-        for t in range(n):
-            S = g[t][:, :, None] * S
-            u = b[t][:, None] * (v[t] - np.einsum("hkv,hk->hv", S, k[t]))
-            S = S + k[t][:, :, None] * u[:, None, :]
-            y[t] = np.einsum("hkv,hk->hv", S, q[t])
-            top = np.fmax(top, np.sqrt((S * S).sum(1)))
-    return y, S, top
+    """One sequence in float64: y, the final state, and the error's scale: the largest column norm that the state had, times what a step does to an error that
+    the state carries (I - beta k k^T has norm 1 for unit keys and beta <= 1, else at most beta |k|^2 - 1)."""
+    q, k, v, g, b, S = (torch.from_numpy(np.array(x)).cuda() for x in (q, k, v, g, b, S))
+    y, top = torch.empty_like(v), torch.zeros_like(S[:, 0])
+    for t in range(len(v)):
+        S = g[t][:, :, None] * S
+        u = b[t][:, None] * (v[t] - (S * k[t][:, :, None]).sum(1))
+        S = S + k[t][:, :, None] * u[:, None, :]
+        y[t] = (S * q[t][:, :, None]).sum(1)
+        grow = (b[t] * k[t].square().sum(1) - 1).nan_to_num(1.0, 1.0, 1.0).clamp(min=1.0)
+        top = torch.fmax(top * grow[:, None], S.square().sum(1).sqrt())
+    return y.cpu().numpy(), S.cpu().numpy(), top.cpu().numpy()
 
 
 def _delta_seq(rng, n, heads, groups, dv, head_decay, lo=0.5):
@@ -124,21 +125,34 @@ def _delta_seq(rng, n, heads, groups, dv, head_decay, lo=0.5):
             "g": f(rng.uniform(lo, 1.0, (n, heads, 1 if head_decay else DK))), "b": f(rng.uniform(0.1, 1.0, (n, heads)))}
 
 
-def _delta_run(cuda, seqs, heads, groups, dv, state, starts, head_decay):
+def _delta_run(cuda, seqs, heads, groups, dv, state, starts, head_decay, tokenwise=False, slots=None):
     from nano_vllm_rs_b200 import ops
     cat = lambda x: torch.from_numpy(np.concatenate([s[x].reshape(len(s["v"]), -1) for s in seqs])).to(cuda)
     lens = [len(s["v"]) for s in seqs]
     cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32, device=cuda)
     pos = torch.cat([torch.arange(p, p + n) for p, n in zip(starts, lens)]).to(cuda)
-    slots = torch.arange(len(seqs), dtype=torch.int32, device=cuda)
-    fn = ops.head_delta_recurrence if head_decay else ops.gated_delta_recurrence
-    y = fn(cat("q"), cat("k"), cat("v"), cat("g"), cat("b"), state, slots, cu, pos, heads, groups, DK, dv)
+    slots = torch.tensor(range(len(seqs)) if slots is None else slots, dtype=torch.int32, device=cuda)
+    x = [cat(c) for c in "qkvgb"]
+    if tokenwise:      # the entries that are not told the number of tokens never take chunks
+        from nano_vllm_rs_b200 import _ffi
+        fn = _ffi.lib().nvllm_head_delta_recurrence if head_decay else _ffi.lib().nvllm_gated_delta_recurrence
+        y = torch.empty_like(x[2])
+        _ffi.check(fn(y.data_ptr(), y.stride(0), *(z for t in x for z in (t.data_ptr(), t.stride(0))), state.data_ptr(), slots.data_ptr(), cu.data_ptr(),
+                      pos.data_ptr(), len(seqs), heads, groups, DK, dv, torch.cuda.current_stream().cuda_stream))
+    else:
+        y = (ops.head_delta_recurrence if head_decay else ops.gated_delta_recurrence)(*x, state, slots, cu, pos, heads, groups, DK, dv)
     return np.split(y.cpu().numpy().reshape(-1, heads, dv), np.cumsum(lens)[:-1])
 
 
+def _takes_chunks(seqs, heads, dv):
+    """The rule of delta_chunked_applies for these tests' sizes: the CTAs, one per head, sequence and 64 columns, take half the SMs."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    return 2 * heads * len(seqs) * (dv // 64) >= sms and sum(len(s["v"]) for s in seqs) >= 16 * len(seqs)
+
+
 def _delta_check(seq, S0, got, state, heads, groups, tokens):
-    """With unit keys and beta <= 1 a step never enlarges an error that the state carries, so the errors of the tokens so far add up at the
-    worst; each is a handful (16 are allowed) of roundings of 2^-24 on the scale of a state's column."""
+    """The errors of the tokens so far add up at the worst; each is a handful (16 are allowed) of roundings of 2^-24 on the scale that
+    _delta_reference gives."""
     w = {x: s.astype(np.float64) for x, s in seq.items()}
     rep = heads // groups
     y, S, top = _delta_reference(w["q"].repeat(rep, 1), w["k"].repeat(rep, 1), w["v"], np.broadcast_to(w["g"], w["g"].shape[:2] + (DK,)), w["b"], S0)
@@ -152,15 +166,19 @@ def _delta_check(seq, S0, got, state, heads, groups, tokens):
         assert (np.abs(state - S)[ok] <= np.broadcast_to(tol[:, None], S.shape)[ok]).all()
 
 
-@pytest.mark.parametrize("heads,groups,dv,lens,head_decay,lo", [
-    (2, 2, 64, [16], False, 0.5), (4, 2, 64, [31, 1, 64], False, 0.9), (8, 1, 64, [17, 97], True, 0.5), (3, 3, 128, [33, 130], False, 0.02), (2, 1, 192, [65, 40], True, 0.99)])
-def test_delta_prompts_and_portions(cuda, heads, groups, dv, lens, head_decay, lo):
+@pytest.mark.parametrize("heads,groups,dv,lens,head_decay,lo,chunks", [
+    (2, 2, 64, [16], False, 0.5, False), (4, 2, 64, [31, 1, 64], False, 0.9, False), (8, 1, 64, [17, 97], True, 0.5, False),
+    (3, 3, 128, [33, 130], False, 0.02, False), (2, 1, 192, [65, 40], True, 0.99, False),
+    (16, 16, 128, [33, 16, 1, 64], False, 0.5, True), (16, 4, 128, [31, 1, 64, 20], False, 0.9, True), (40, 8, 64, [17, 97], True, 0.5, True),
+    (16, 2, 192, [15, 40, 33], False, 0.02, True), (37, 37, 64, [65, 40], True, 0.99, True), (16, 16, 128, [130, 48, 16], True, 0.02, True)])
+def test_delta_prompts_and_portions(cuda, heads, groups, dv, lens, head_decay, lo, chunks):
     """Chunk edges and tails, single tokens beside prompts, decays from next to nothing to next to one, a second portion that goes on from the slots."""
     rng = np.random.default_rng(sum(lens) + dv)
     state = torch.full((len(lens), heads, DK, dv), 7.0, device=cuda)
     S = [np.zeros((heads, DK, dv))] * len(lens)
     for portion in range(2):
         seqs = [_delta_seq(rng, n, heads, groups, dv, head_decay, lo) for n in lens]
+        assert _takes_chunks(seqs, heads, dv) == chunks
         ys = _delta_run(cuda, seqs, heads, groups, dv, state, [portion * n for n in lens], head_decay)
         st = state.cpu().numpy()
         for i, (q, y) in enumerate(zip(seqs, ys)):
@@ -168,11 +186,13 @@ def test_delta_prompts_and_portions(cuda, heads, groups, dv, lens, head_decay, l
         S = [st[i].astype(np.float64) for i in range(len(lens))]
 
 
+@pytest.mark.parametrize("heads,groups,dv,head_decay", [(4, 2, 64, False), (20, 10, 128, False), (20, 10, 128, True)], ids=["tokens", "chunks per channel", "chunks per head"])
 @pytest.mark.parametrize("what", ["v nan", "v inf", "k nan", "q inf", "g zero", "g above one", "g nan", "beta nan", "k large", "all zero"])
-def test_delta_odd_values(cuda, what):
-    heads, groups, dv, n, at = 4, 2, 64, 60, 21
+def test_delta_odd_values(cuda, what, heads, groups, dv, head_decay):
+    n, at = 60, 21
     rng = np.random.default_rng(9)
-    seqs = [_delta_seq(rng, n, heads, groups, dv, False), _delta_seq(rng, n, heads, groups, dv, False)]
+    seqs = [_delta_seq(rng, n, heads, groups, dv, head_decay), _delta_seq(rng, n, heads, groups, dv, head_decay)]
+    assert _takes_chunks(seqs, heads, dv) == (heads > 4)
     s = seqs[0]
     if what == "v nan": s["v"][at, 1, 5] = np.nan
     elif what == "v inf": s["v"][at, 1, 5] = np.inf
@@ -180,13 +200,52 @@ def test_delta_odd_values(cuda, what):
     elif what == "q inf": s["q"][at, 1, 9] = np.inf
     elif what == "g zero": s["g"][at] = 0.0
     elif what == "g above one": s["g"][at] = 1.25
-    elif what == "g nan": s["g"][at, 2, 7] = np.nan
+    elif what == "g nan": s["g"][at, 2, -1] = np.nan
     elif what == "beta nan": s["b"][at, 0] = np.nan
     elif what == "k large": s["k"][n - 1] *= np.float32(2.0 ** 40)
     else:
         for x in "qkv": s[x][:] = 0.0
     state = torch.zeros((2, heads, DK, dv), device=cuda)
-    ys = _delta_run(cuda, seqs, heads, groups, dv, state, [0, 0], False)
+    ys = _delta_run(cuda, seqs, heads, groups, dv, state, [0, 0], head_decay)
     st = state.cpu().numpy()
     for i in range(2):
         _delta_check(seqs[i], np.zeros((heads, DK, dv)), ys[i], st[i], heads, groups, n)
+
+
+def test_delta_padding_sequences(cuda):
+    """A sequence without a slot: zeros, no state touched."""
+    heads, dv, lens = 40, 128, [20, 40]
+    rng = np.random.default_rng(2)
+    seqs = [_delta_seq(rng, n, heads, heads, dv, False) for n in lens]
+    assert _takes_chunks(seqs, heads, dv)
+    state = torch.full((2, heads, DK, dv), 3.0, device=cuda)
+    ys = _delta_run(cuda, seqs, heads, heads, dv, state, [0, 0], False, slots=[-1, 1])
+    assert (ys[0] == 0).all() and (state[0] == 3).all()
+    _delta_check(seqs[1], np.zeros((heads, DK, dv)), ys[1], state[1].cpu().numpy(), heads, heads, lens[1])
+
+
+@pytest.mark.parametrize("size,beta", [(2.0 ** 7.5, 12.0), (2.0 ** 6, 8.0), (1.6, 1.9)])
+def test_delta_keys_that_make_u_grow(cuda, size, beta):
+    """Keys far from unit vectors, from the middle of a chunk on: u grows with every token, beyond f32 in the larger two.  What came before stays
+    finite and right, and what overflows is what overflows token by token."""
+    heads, dv, n, at = 40, 128, 32, 23
+    rng = np.random.default_rng(4)
+    seqs = [_delta_seq(rng, n, heads, heads, dv, False, 0.9) for _ in range(2)]
+    assert _takes_chunks(seqs, heads, dv)
+    s = seqs[0]
+    s["k"][at:] = s["k"][at] * np.float32(size)      # one direction: every token's A is beta |k|^2
+    s["b"][at:] = beta
+    state = torch.zeros((2, heads, DK, dv), device=cuda)
+    other = torch.zeros_like(state)
+    ys = _delta_run(cuda, seqs, heads, heads, dv, state, [0, 0], False)
+    ts = _delta_run(cuda, seqs, heads, heads, dv, other, [0, 0], False, tokenwise=True)
+    for i in range(2):
+        np.testing.assert_array_equal(np.isfinite(ys[i]), np.isfinite(ts[i]))
+        sure = at if i == 0 else n                   # tokens whose values come from unit keys
+        w = {x: v[:sure] for x, v in seqs[i].items()}
+        assert np.isfinite(ys[i][:sure]).all()
+        y, _, top = _delta_reference(*(w[x].astype(np.float64) for x in "qkv"), np.broadcast_to(w["g"].astype(np.float64), (sure, heads, DK)),
+                                     w["b"].astype(np.float64), np.zeros((heads, DK, dv)))
+        assert (np.abs(ys[i][:sure] - y) <= n * 16 * 2.0 ** -24 * top).all()
+    if size > 2: assert not np.isfinite(ys[0][-1]).all()
+    np.testing.assert_array_equal(torch.isfinite(state).cpu().numpy(), torch.isfinite(other).cpu().numpy())
