@@ -1,12 +1,17 @@
 // delta_chunked.cu — the gated delta rule with a decay per key channel,  S <- diag(g_t) S,  u_t = beta_t (v_t - S^T k_t),  S <- S + k_t u_t^T,
-// y_t = S^T q_t,  for prompts: 16 tokens at a time as matrix products and one triangular solve.  With G_t = g_1 ... g_t (per channel, from
+// y_t = S^T q_t,  for prompts: 16 tokens at a time as matrix products and one triangular inverse.  With G_t = g_1 ... g_t (per channel, from
 // the chunk's start; * and / per channel) and S the state before the chunk,
-//   A_ij = beta_i (G_i * k_i) . (k_j / G_j)  (j < i),   (I + A) U = beta (V - (G * K) S),
+//   A_ij = beta_i (G_i * k_i) . (k_j / G_j)  (j < i),   X = V - (G * K) S,   U = beta X + ((I + A)^-1 - I) beta X,
 //   y_i = (G_i * q_i)^T S + sum_(j <= i) ((G_i * q_i) . (k_j / G_j)) u_j,   S <- G_16 * S + sum_j (R_j * k_j) u_j^T,  R_j = g_(j+1) ... g_16.
 // The quotients pair with products of the same channel, so every term carries G_i / G_j <= 1 whatever the decays are; only the range of f32
 // limits them.  (R_j and not G_16 / G_j for the state: two roundings fewer in what stays.)
 //
-// Precision: as in recurrence_chunked.cu, three bf16 pieces and six products of every f32 operand, hi.hi summed apart; the solve is f32.
+// Precision: as in recurrence_chunked.cu, three bf16 pieces and six products of every f32 operand, hi.hi summed apart.  What the state keeps is rounded
+// as rarely as token by token: the inverse without its diagonal is small, so u is beta X with a small correction (solving for u
+// column by column rounds every u fifteen times), and u, R * k and k / G are split from values in two parts.  Relative error of y and the
+// state against 64 bits, token by token and here, 1e-7: decays per channel as the models make them 0.84, 0.95 and 0.67, 0.60; per head 0.81,
+// 0.84 and 0.70, 0.61; near one 2.01, 3.09 and 0.83, 0.89; 0.6 a token 0.78, 0.66 and 0.72, 0.60; inputs of one sign 0.57, 1.01 and 0.55, 0.60.
+// (With the solve per column and operands of one part: 0.93, 0.97; 0.97, 0.99; 1.10, 1.21; 1.00, 0.96; 0.73, 0.84; 10 % less time.)
 // A chunk with a decay outside [0, 1] or a product of decays below 2^-90, or with a value that is no number, infinite or far from the
 // others' range (q outside 2^-30 .. 2^30, k outside 2^-30 .. 2^8, beta, v or the state beyond 2^4, 2^20), or where U grows beyond 2^64 (keys
 // far from unit vectors), is stepped through token by token in f32 by the warps that it concerns: what such a value reaches is then the same as
@@ -14,10 +19,9 @@
 //
 // CTA = (head, sequence, 64 columns of v), 4 warps; a warp keeps 16 columns of the state, transposed, in the accumulator layout of m16n8k16
 // (64 registers), which is also that of the B operand of (G * K) S and (G * q) S.  q, k and the decays of the next chunk fly (cp.async) under the
-// products of this one.  Bound by mma.sync issue (348 a warp and chunk) and the conversions around it (a chunk of 16 tokens takes 10 K clocks, 2.6 K of
-// them for the operands' pieces, 2.5 K for the products with S, 1.5 K for the state).
-// Token by token and here, 16 heads of 128 x 128 (us): 8 x 1024 tokens 784 and 471, 32 x 256 641 and 469, 32 x 16 60 and 42, 8 x 40 44 and 32;
-// relative error against 64 bits of y and the state 0.96e-7, 0.94e-7 and 0.94e-7, 1.05e-7, with decays near one 2.7e-7, 3.6e-7 and 1.2e-7, 1.3e-7.
+// products of this one.  Bound by mma.sync issue (360 a warp and chunk) and the conversions around it; two CTAs an SM (94 KB each).
+// Token by token and here, 16 heads of 128 x 128 (us): 8 x 1024 tokens 784 and 520, with a decay per head 692 and 525; 32 x 256 642 and 510, 32 x 16
+// 60 and 46, 8 x 40 44 and 33.
 #include "split_mma.cuh"
 
 namespace nvllm {
@@ -29,7 +33,7 @@ constexpr int kC = 16, kDk = 128, kCols = 64, kWarps = 4;
 constexpr int kRow = kDk * 2 + 16;               // bytes of a row of pieces: 16 more, so that ldmatrix rows fall into different banks
 constexpr int kPiece = kC * kRow;
 constexpr int kPs = 24;                          // floats of a row of A and P (8-byte reads of 4 rows of a quarter warp: 24 r + 2 c, no conflicts)
-constexpr int kUs = 17;                          // floats of a row of a warp's R / U
+constexpr int kUs = 17;                          // floats of a row of a warp's X / U
 constexpr int kSmRaw = 0;                        // q, k, g of a chunk as they come: [16][128] f32 each
 constexpr int kSmQ = kSmRaw + 3 * kC * kDk * 4;  // G * q, G * k, k / G, R * k: three pieces each
 constexpr int kSmKu = kSmQ + 3 * kPiece;
@@ -37,19 +41,10 @@ constexpr int kSmKd = kSmKu + 3 * kPiece;
 constexpr int kSmKr = kSmKd + 3 * kPiece;
 constexpr int kSmA = kSmKr + 3 * kPiece;         // A transposed: row j holds A_ij over i
 constexpr int kSmP = kSmA + kC * kPs * 4;
-constexpr int kSmU = kSmP + kC * kPs * 4;        // per warp [16 tokens][16 columns]
-constexpr int kSmVec = kSmU + kWarps * kC * kUs * 4;   // floats: G_16 in two parts [2][128], beta [2][16], flag
+constexpr int kSmU = kSmP + kC * kPs * 4;        // per warp [two parts][16 tokens][16 columns]
+constexpr int kSmT = kSmU + kWarps * 2 * kC * kUs * 4;   // per warp: T beta below the diagonal
+constexpr int kSmVec = kSmT + kWarps * kC * kPs * 4;   // floats: G_16 in two parts [2][128], beta [2][16], flag
 constexpr int kSmBytes = kSmVec + (2 * kDk + 2 * kC) * 4 + 16;
-
-// x / y to an ulp for normal y (a division's slow path is for what is stepped through here): one Newton step on the approximate reciprocal
-// and one on the quotient.
-__device__ __forceinline__ float quotient(float x, float y) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(y));
-  r = fmaf(fmaf(-y, r, 1.f), r, r);
-  const float q = x * r;
-  return fmaf(fmaf(-y, q, x), r, q);
-}
 
 template <bool HEADG>
 __global__ void __launch_bounds__(kWarps * 32, 2) delta_chunked_kernel(const DeltaArgs a) {
@@ -66,7 +61,9 @@ __global__ void __launch_bounds__(kWarps * 32, 2) delta_chunked_kernel(const Del
   const int h = blockIdx.x, s = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int col0 = blockIdx.z * kCols + warp * 16;       // the warp's first column of the head
   const int r = lane >> 2, c2 = (lane & 3) * 2;          // row and first column of the lane in an accumulator tile
-  float* const U = reinterpret_cast<float*>(smem + kSmU) + warp * kC * kUs;
+  float* const U = reinterpret_cast<float*>(smem + kSmU) + warp * 2 * kC * kUs;
+  float* const Ul = U + kC * kUs;
+  float* const T = reinterpret_cast<float*>(smem + kSmT) + warp * kC * kPs;
   const int t0 = a.cu_tokens[s], t1 = a.cu_tokens[s + 1];
   const int slot = a.seq_slot[s];
   if (t1 <= t0) return;
@@ -136,8 +133,8 @@ __global__ void __launch_bounds__(kWarps * 32, 2) delta_chunked_kernel(const Del
     bool bad = false;
     {
       const int ch = 2 * (tid & 63), first = (tid >> 6) * 8;
-      // products of decays in two parts each, rounded once where they are used
-      float2 x[3][8], y[8], G = make_float2(1.f, 1.f), Gl = make_float2(0.f, 0.f), R[8], Rh = G, Rl = Gl;
+      // products of decays in two parts each
+      float2 x[3][8], y[8], G = make_float2(1.f, 1.f), Gl = make_float2(0.f, 0.f), R = G, Rl = Gl;
       auto times = [](float2& hi, float2& lo, float2 g) {
         const float px = hi.x * g.x, py = hi.y * g.y;
         lo.x = fmaf(lo.x, g.x, fmaf(hi.x, g.x, -px));
@@ -155,12 +152,21 @@ __global__ void __launch_bounds__(kWarps * 32, 2) delta_chunked_kernel(const Del
         for (int i = 0; i < 8; ++i) times(G, Gl, y[i]);
       } else {
 #pragma unroll
-        for (int i = 7; i >= 0; --i) times(Rh, Rl, y[i]);
+        for (int i = 7; i >= 0; --i) times(R, Rl, y[i]);
       }
+      auto put = [&](int operand, int i, const uint32_t (&p)[3]) {
+        uint8_t* dst = smem + kSmQ + (first + i) * kRow + ch * 2;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) *reinterpret_cast<uint32_t*>(dst + (3 * operand + j) * kPiece) = p[j];
+      };
+      uint32_t p[3];
 #pragma unroll
       for (int i = 7; i >= 0; --i) {
-        R[i] = make_float2(Rh.x + Rl.x, Rh.y + Rl.y);
-        times(Rh, Rl, x[2][i]);
+        const float2 k = x[1][i];      // R * k, the pieces of the unrounded value
+        const float px = __fmul_rn(k.x, R.x), py = __fmul_rn(k.y, R.y);
+        split3(px, py, fmaf(k.x, Rl.x, fmaf(k.x, R.x, -px)), fmaf(k.y, Rl.y, fmaf(k.y, R.y, -py)), p[0], p[1], p[2]);
+        put(3, i, p);
+        times(R, Rl, x[2][i]);
       }
       uint32_t most[2] = {0u, 0u};
 #pragma unroll
@@ -169,18 +175,16 @@ __global__ void __launch_bounds__(kWarps * 32, 2) delta_chunked_kernel(const Del
         bad |= !(x[2][i].x >= 0.f && x[2][i].x <= 1.f && x[2][i].y >= 0.f && x[2][i].y <= 1.f);
         const float2 P = make_float2(G.x + Gl.x, G.y + Gl.y);
 #pragma unroll
-        for (int op = 0; op < 2; ++op) most[op] = max(most[op], max(abs_bits(x[op][i].x), abs_bits(x[op][i].y)));
-        uint8_t* dst = smem + kSmQ + (first + i) * kRow + ch * 2;
-        auto put = [&](int operand, float a0, float a1) {
-          uint32_t p[3];
-          split3(a0, a1, p[0], p[1], p[2]);
-#pragma unroll
-          for (int j = 0; j < 3; ++j) *reinterpret_cast<uint32_t*>(dst + (3 * operand + j) * kPiece) = p[j];
-        };
-        put(0, x[0][i].x * P.x, x[0][i].y * P.y);
-        put(1, x[1][i].x * P.x, x[1][i].y * P.y);
-        put(2, quotient(x[1][i].x, P.x), quotient(x[1][i].y, P.y));
-        put(3, x[1][i].x * R[i].x, x[1][i].y * R[i].y);
+        for (int op = 0; op < 2; ++op) {
+          most[op] = max(most[op], max(abs_bits(x[op][i].x), abs_bits(x[op][i].y)));
+          split3(x[op][i].x * P.x, x[op][i].y * P.y, p[0], p[1], p[2]);
+          put(op, i, p);
+        }
+        // k / G: a quotient and, divided again, what it leaves over (the quotient of two-part numbers, Dekker 1971)
+        const float2 k = x[1][i];
+        const float qx = __fdividef(k.x, G.x), qy = __fdividef(k.y, G.y);
+        split3(qx, qy, __fdividef(fmaf(-qx, Gl.x, fmaf(-qx, G.x, k.x)), G.x), __fdividef(fmaf(-qy, Gl.y, fmaf(-qy, G.y, k.y)), G.y), p[0], p[1], p[2]);
+        put(2, i, p);
       }
       if (first != 0) {
         const float2 P = make_float2(G.x + Gl.x, G.y + Gl.y);
@@ -206,15 +210,17 @@ __global__ void __launch_bounds__(kWarps * 32, 2) delta_chunked_kernel(const Del
 #pragma unroll
       for (int kk = 0; kk < kDk / 16; ++kk) {
         uint32_t af[1][3][4], kf[3][1][2];
-        zero(hh);
+        if (kk % 2 == 0) zero(hh);
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
           ldmatrix_x4(af[0][j], a_addr + (warp < 2 ? kSmKu : kSmQ) + kk * 32 + j * kPiece);
           ldmatrix_x2(kf[j][0], k_addr + kk * 32 + j * kPiece);
         }
         mma6<1, 1>(hh, al[kk & 3], af, kf);
+        if (kk % 2 == 1) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) sum[i] += hh[0][0][i];
+          for (int i = 0; i < 4; ++i) sum[i] += hh[0][0][i];
+        }
       }
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -238,12 +244,12 @@ __global__ void __launch_bounds__(kWarps * 32, 2) delta_chunked_kernel(const Del
       smax[1] = abs_max(S[n][2], S[n][3], smax[1]);
     }
     bool step = __any_sync(0xffffffffu, slow || !(smax[0] < 1.0e6f && smax[1] < 1.0e6f));      // 2^20: k / G reaches 2^98
-    float sy[2][2][4] = {};            // [G * k, G * q] . S: [16 tokens][8 columns]
+    float sy[2][2][4] = {}, lo[2][2][4] = {};            // [G * k, G * q] . S in two parts: [16 tokens][8 columns]
     if (!step) {
-      float hh[2][2][4], lo[2][2][4] = {};
+      float hh[2][2][4];
 #pragma unroll
       for (int kk = 0; kk < kDk / 16; ++kk) {
-        zero(hh);
+        if (kk % 2 == 0) zero(hh);
         uint32_t sf[3][2][2], af[2][3][4];
 #pragma unroll
         for (int n = 0; n < 2; ++n)
@@ -255,36 +261,38 @@ __global__ void __launch_bounds__(kWarps * 32, 2) delta_chunked_kernel(const Del
           ldmatrix_x4(af[1][j], a_addr + kSmQ + kk * 32 + j * kPiece);
         }
         mma6<2, 2>(hh, lo, af, sf);
+        if (kk % 2 == 1) {
 #pragma unroll
-        for (int m = 0; m < 2; ++m)
+          for (int m = 0; m < 2; ++m)
 #pragma unroll
-          for (int n = 0; n < 2; ++n)
+            for (int n = 0; n < 2; ++n)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) sy[m][n][i] += hh[m][n][i];
+              for (int i = 0; i < 4; ++i) sy[m][n][i] += hh[m][n][i];
+        }
       }
 #pragma unroll
       for (int m = 0; m < 2; ++m)
 #pragma unroll
         for (int n = 0; n < 2; ++n)
 #pragma unroll
-          for (int i = 0; i < 4; ++i) sy[m][n][i] = join(sy[m][n][i], lo[m][n][i]);
-      // right side of the solve, token by column
+          for (int i = 0; i < 4; ++i) lo[m][n][i] = small_part(sy[m][n][i], lo[m][n][i]);
+      // X = V - (G * K) S, token by column
 #pragma unroll
       for (int n = 0; n < 2; ++n)
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const float b = bs[r + 8 * e];
-          U[(r + 8 * e) * kUs + 8 * n + c2] = b * (vr[n][e].x - sy[0][n][2 * e]);
-          U[(r + 8 * e) * kUs + 8 * n + c2 + 1] = b * (vr[n][e].y - sy[0][n][2 * e + 1]);
+        for (int i = 0; i < 4; ++i) {
+          const float2 v = vr[n][i >> 1];
+          U[(r + 8 * (i >> 1)) * kUs + 8 * n + c2 + (i & 1)] = ((i & 1 ? v.y : v.x) - sy[0][n][i]) - lo[0][n][i];
         }
     }
     __syncthreads();                   // A and P are complete
     if (!step) {
-      // ---- (I + A) U = R, a lane per column (the upper half repeats the lower) ------------------------------------------
+      // ---- T = (I + A)^-1, a lane per column; U = beta X + (T - I) beta X -----------------------------------------------------------
       {
         float u[kC];
+        const int col = lane & 15;
 #pragma unroll
-        for (int i = 0; i < kC; ++i) u[i] = U[i * kUs + (lane & 15)];
+        for (int i = 0; i < kC; ++i) u[i] = i == col ? 1.f : 0.f;
 #pragma unroll
         for (int j = 0; j < kC - 1; ++j) {
 #pragma unroll
@@ -296,15 +304,44 @@ __global__ void __launch_bounds__(kWarps * 32, 2) delta_chunked_kernel(const Del
             if (4 * q4 + 3 > j) u[4 * q4 + 3] = fmaf(-c.w, u[j], u[4 * q4 + 3]);
           }
         }
+        const int half = (lane >> 4) * 8;      // the lower half of the lanes stores the first eight rows, the upper the others
+        const float b = bs[col];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) T[(half + i) * kPs + col] = half + i > col ? (half ? u[8 + i] : u[i]) * b : 0.f;
+        __syncwarp();
+      }
+      {
+        float hh[1][2][4] = {}, rest[1][2][4] = {};
+        uint32_t tf[1][3][4], xf[3][2][2];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float2 x = *reinterpret_cast<const float2*>(T + (r + (i & 1) * 8) * kPs + (i >> 1) * 8 + c2);
+          split3(x.x, x.y, tf[0][0][i], tf[0][1][i], tf[0][2][i]);
+        }
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int at = (c2 + 8 * e) * kUs + r + 8 * n;
+            split3(U[at], U[at + kUs], xf[0][n][e], xf[1][n][e], xf[2][n][e]);
+          }
+        mma6<1, 2>(hh, rest, tf, xf);
+        __syncwarp();
         float umax = 0.f;
 #pragma unroll
-        for (int i = 0; i < kC; i += 2) umax = abs_max(u[i], u[i + 1], umax);
-        step = __any_sync(0xffffffffu, !(umax < 1.8e19f));     // 2^64: P reaches 2^45
-        __syncwarp();
-        if (lane < 16) {
+        for (int n = 0; n < 2; ++n)
 #pragma unroll
-          for (int i = 0; i < kC; ++i) U[i * kUs + lane] = u[i];
-        }
+          for (int i = 0; i < 4; ++i) {
+            const int row = r + 8 * (i >> 1), at = row * kUs + 8 * n + c2 + (i & 1);
+            const float b = bs[row], x = U[at], p = __fmul_rn(b, x), e = fmaf(b, x, -p);
+            float err;
+            float u = two_sum(p, hh[0][n][i], err);
+            u = two_sum(u, (err + e) + small_part(hh[0][n][i], rest[0][n][i]), err);
+            U[at] = u;
+            Ul[at] = err;
+            umax = abs_max(u, u, umax);
+          }
+        step = __any_sync(0xffffffffu, !(umax < 1.8e19f));     // 2^64: P reaches 2^45
         __syncwarp();
       }
     }
@@ -314,27 +351,32 @@ __global__ void __launch_bounds__(kWarps * 32, 2) delta_chunked_kernel(const Del
       for (int n = 0; n < 2; ++n)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          split3(U[(c2 + 8 * e) * kUs + r + 8 * n], U[(c2 + 8 * e + 1) * kUs + r + 8 * n], uf[0][n][e], uf[1][n][e], uf[2][n][e]);
+          const int at = (c2 + 8 * e) * kUs + r + 8 * n;
+          split3(U[at], U[at + kUs], Ul[at], Ul[at + kUs], uf[0][n][e], uf[1][n][e], uf[2][n][e]);
 #pragma unroll
           for (int j = 0; j < 3; ++j) ua[0][j][2 * e + n] = uf[j][n][e];
         }
       // ---- y ---------------------------------------------------------------------------------------------------------------
       {
-        float hh[1][2][4] = {}, lo[1][2][4] = {};
+        float hh[1][2][4] = {}, rest[1][2][4] = {};
         uint32_t pf[1][3][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const float2 x = *reinterpret_cast<const float2*>(Pm + (r + (i & 1) * 8) * kPs + (i >> 1) * 8 + c2);
           split3(x.x, x.y, pf[0][0][i], pf[0][1][i], pf[0][2][i]);
         }
-        mma6<1, 2>(hh, lo, pf, uf);
+        mma6<1, 2>(hh, rest, pf, uf);
+        auto sum = [&](int n, int i) {
+          float err;
+          const float s1 = two_sum(sy[1][n][i], hh[0][n][i], err);
+          return s1 + (err + (lo[1][n][i] + small_part(hh[0][n][i], rest[0][n][i])));
+        };
 #pragma unroll
         for (int e = 0; e < 2; ++e)
           if (r + 8 * e < cnt) {
 #pragma unroll
             for (int n = 0; n < 2; ++n)
-              *reinterpret_cast<float2*>(yh + static_cast<int64_t>(tb + r + 8 * e) * a.ldy + n * 8 + c2) =
-                  make_float2(sy[1][n][2 * e] + join(hh[0][n][2 * e], lo[0][n][2 * e]), sy[1][n][2 * e + 1] + join(hh[0][n][2 * e + 1], lo[0][n][2 * e + 1]));
+              *reinterpret_cast<float2*>(yh + static_cast<int64_t>(tb + r + 8 * e) * a.ldy + n * 8 + c2) = make_float2(sum(n, 2 * e), sum(n, 2 * e + 1));
           }
       }
       if (tb + kC < t1) load_v(tb + kC);
@@ -342,19 +384,19 @@ __global__ void __launch_bounds__(kWarps * 32, 2) delta_chunked_kernel(const Del
       // B of 16 tokens x 16 dims, transposed on the way: lanes 0-15 tokens 0-15 of dims 0-7, lanes 16-31 of dims 8-15
 #pragma unroll
       for (int np = 0; np < kDk / 32; ++np) {
-        float hh[1][4][4] = {}, lo[1][4][4] = {};
+        float hh[1][4][4] = {}, rest[1][4][4] = {};
         uint32_t kf[3][4][2];
 #pragma unroll
         for (int j = 0; j < 3; ++j)
 #pragma unroll
           for (int u = 0; u < 2; ++u)
             ldmatrix_x4_trans(reinterpret_cast<uint32_t(&)[4]>(kf[j][2 * u]), a_addr + kSmKr + np * 64 + u * 32 + j * kPiece);
-        mma6<1, 4>(hh, lo, ua, kf);
+        mma6<1, 4>(hh, rest, ua, kf);
 #pragma unroll
         for (int n = 0; n < 4; ++n) {
           const float2 G = *reinterpret_cast<const float2*>(gam + 8 * (4 * np + n) + c2), Gl = *reinterpret_cast<const float2*>(gam + kDk + 8 * (4 * np + n) + c2);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) S[4 * np + n][i] = fmaf(S[4 * np + n][i], i & 1 ? G.y : G.x, fmaf(S[4 * np + n][i], i & 1 ? Gl.y : Gl.x, join(hh[0][n][i], lo[0][n][i])));
+          for (int i = 0; i < 4; ++i) S[4 * np + n][i] = fmaf(S[4 * np + n][i], i & 1 ? G.y : G.x, fmaf(S[4 * np + n][i], i & 1 ? Gl.y : Gl.x, join(hh[0][n][i], rest[0][n][i])));
         }
       }
     } else {

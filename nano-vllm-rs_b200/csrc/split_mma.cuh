@@ -24,6 +24,20 @@ __device__ __forceinline__ void split3(float x0, float x1, uint32_t& hi, uint32_
   mid = pack_bf16x2(x0, x1);
   lo = pack_bf16x2(x0 - bf16_lo(mid), x1 - bf16_hi(mid));
 }
+// The same of x0 + e0 and x1 + e1, the second parts some ulps of the first at the most.
+__device__ __forceinline__ void split3(float x0, float x1, float e0, float e1, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  hi = pack_bf16x2(x0, x1);
+  x0 -= bf16_lo(hi);
+  x1 -= bf16_hi(hi);
+  mid = pack_bf16x2(x0, x1);
+  lo = pack_bf16x2((x0 - bf16_lo(mid)) + e0, (x1 - bf16_hi(mid)) + e1);
+}
+// a + b = result + err (Knuth 1969)
+__device__ __forceinline__ float two_sum(float a, float b, float& err) {
+  const float s = a + b, t = s - a;
+  err = (a - (s - t)) + (b - t);
+  return s;
+}
 // (not volatile: the compiler may interleave independent accumulators)
 __device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
@@ -54,7 +68,8 @@ __device__ __forceinline__ void mma6(float (&dh)[M][N][4], float (&dl)[M][N][4],
 
 // hi.hi and the other products together.  mma.sync cuts off where an addition rounds, always towards zero: measured over the recurrences' chunks,
 // sums of hi.hi come out 0.36 x 2^-24 too small on the average.  That mean is put back here, beside the small products, where it can be represented.
-__device__ __forceinline__ float join(float hh, float rest) { return hh + fmaf(hh, 0.36f * 5.9604645e-8f, rest); }
+__device__ __forceinline__ float small_part(float hh, float rest) { return fmaf(hh, 0.36f * 5.9604645e-8f, rest); }
+__device__ __forceinline__ float join(float hh, float rest) { return hh + small_part(hh, rest); }
 
 }  // namespace split
 }  // namespace nvllm
