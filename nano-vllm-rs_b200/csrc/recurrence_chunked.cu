@@ -10,7 +10,7 @@
 // and three products would need half the instructions, but their 22-bit products meet the truncation: 4.5e-7 from 64 bits.)  Relative
 // error of y and of the state against 64 bits, token by token and here: retention of 1024 tokens 2.3e-7, 2.1e-7 and 1.0e-7, 0.8e-7;
 // state-space duality 0.80e-7, 0.69e-7 and 0.68e-7, 0.65e-7.
-// A chunk with a value that is no number, infinite, or far from the others' range (rows of q and k outside 2^-60 .. 2^40) is stepped
+// A chunk with a value that is no number, infinite, or far from the others' range (rows of q and k outside 2^-60 .. 2^40, d beyond 2^40) is stepped
 // through token by token in f32 instead, by the warps that it concerns: what such a value reaches is then the same as there.
 //
 // CTA = (head, sequence, 64 columns of v), 4 warps; a warp keeps 16 columns of the state, transposed, in the accumulator layout of
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) linear_recurrence_chunked_kern
         if (lane == 31) wgt[31] = bv;
       }
       // decays above 1 are rare enough to step through: D then stays in [0, 1]
-      bad |= !(av >= 0.f && av <= 1.f) || far_off(abs_bits(bv), -60, 40);
+      bad |= !(av >= 0.f && av <= 1.f) || far_off(abs_bits(bv), -60, 40) || !(fabsf(d) < 1.1e12f);
     }
     if (bad) *flag = 1u;
     __syncthreads();
