@@ -4,12 +4,15 @@
 //
 // Precision: inputs, state and results are f32, and the products lose nothing that the token-by-token form (recurrence.cu) keeps.
 // Every operand is split into three bf16 values (8 bits each, f32's range), and six products on mma.sync keep what is above 2^-24:
-// hi.hi, hi.mid, mid.hi, mid.mid, hi.lo, lo.hi.  mma.sync truncates when it adds to its accumulator; products of 8-bit values are short
-// enough for one hi.hi to lose next to nothing to that; they are added up in f32 outside, and the rest, 2^-8 and smaller, is summed apart.  Accumulators start from zero in every
-// chunk and are added to the state in f32, so that the state is rounded once per 32 tokens instead of 32 times.  (Two fp16 values
-// and three products would need half the instructions, but their 22-bit products meet the truncation: 4.5e-7 from 64 bits.)  Relative
-// error of y and of the state against 64 bits, token by token and here: retention of 1024 tokens 2.3e-7, 2.1e-7 and 1.0e-7, 0.8e-7;
-// state-space duality 0.80e-7, 0.69e-7 and 0.68e-7, 0.65e-7.
+// hi.hi, hi.mid, mid.hi, mid.mid, hi.lo, lo.hi.  mma.sync cuts off: it aligns its addends to 2^-26 of the largest and its sum to 24 bits.  So hi.hi
+// of one or two steps is added up in f32 outside (four in a row lose more than the additions do), and the rest, 2^-8 and smaller, is summed apart.
+// Accumulators start from zero in every chunk and are added to the state in f32, so that the state is rounded once per 32 tokens instead of 32
+// times; D_(32)j b_j v_j is split from a value in two parts.  A state that keeps less than 2^-8 of the chunk's start is made of this one rounding,
+// so there the products of hi.hi run once more on top of the negated sum and give what was cut off (for every chunk 7 % more time; without
+// it the state's error reaches 1.04 times the other form's).  (Two fp16 values
+// and three products would need half the instructions, but their 22-bit products meet the cut: 4.5e-7 from 64 bits.)  Relative
+// error of y and of the state against 64 bits, token by token and here, 1e-7: retention 1.99, 1.89 and 0.83, 0.60; state-space duality as the models
+// have it 0.81, 0.68 and 0.67, 0.51; decays of 0.3 a token 0.79, 0.46 and 0.74, 0.45; any decay from 0 to 1 1.22, 0.47 and 0.82, 0.46.
 // A chunk with a value that is no number, infinite, or far from the others' range (rows of q and k outside 2^-60 .. 2^40, d beyond 2^40) is stepped
 // through token by token in f32 instead, by the warps that it concerns: what such a value reaches is then the same as there.
 //
@@ -18,8 +21,8 @@
 // global memory straight into the layout that serves as A (v^T of the update) and as B (of the middle product).  q and k of the
 // next chunk fly (cp.async) under the products of this one.  Bound by mma.sync issue (about 520 of them per warp and chunk) and the conversions
 // around it; two CTAs an SM (91 KB each) hide each other's barriers.
-// Token by token and here (us): 16 heads of 128 x 128, 8 x 1024 tokens 551 and 296, 8192 tokens 3235 and 1730; 64 heads of 128 x 64, 8 x 1024
-// 876 and 575, 2 x 40 30 and 21, 32 x 16 83 and 85.
+// Token by token and here (us): 16 heads of 128 x 128, 8 x 1024 tokens 548 and 297, 500 tokens 210 and 107; 64 heads of 128 x 64, 8 x 1024
+// 875 and 594, 2 x 40 30 and 21.
 #include "split_mma.cuh"
 
 namespace nvllm {
@@ -35,8 +38,8 @@ constexpr int kSmRaw = 0;                        // q, then k of a chunk as they
 constexpr int kSmQ = kSmRaw + 2 * kC * kDk * 4;  // hi, mid, lo
 constexpr int kSmK = kSmQ + 3 * kPiece;
 constexpr int kSmP = kSmK + 3 * kPiece;          // D_ij, overwritten in place by the middle factor
-constexpr int kSmVec = kSmP + kC * kPs * 4;      // floats: pre, w [32 each], a [2][32], b [2][32], flag, low part of the product of all decays
-constexpr int kSmBytes = kSmVec + 6 * kC * 4 + 16;
+constexpr int kSmVec = kSmP + kC * kPs * 4;      // floats: pre, w [32 each], a [2][32], b [2][32], second part of w [32], flag, that of the product of all decays
+constexpr int kSmBytes = kSmVec + 7 * kC * 4 + 16;
 
 __global__ void __launch_bounds__(kWarps * 32, 2) linear_recurrence_chunked_kernel(const RecArgs a) {
   pdl_wait();
@@ -46,8 +49,8 @@ __global__ void __launch_bounds__(kWarps * 32, 2) linear_recurrence_chunked_kern
   float* raw = reinterpret_cast<float*>(smem + kSmRaw);
   float* mid = reinterpret_cast<float*>(smem + kSmP);
   float* vec = reinterpret_cast<float*>(smem + kSmVec);
-  float *pre = vec, *wgt = vec + kC;
-  volatile uint32_t* flag = reinterpret_cast<volatile uint32_t*>(vec + 6 * kC);
+  float *pre = vec, *wgt = vec + kC, *wgt_lo = vec + 6 * kC;
+  volatile uint32_t* flag = reinterpret_cast<volatile uint32_t*>(vec + 7 * kC);
   const int h = blockIdx.x, s = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int col0 = blockIdx.z * kCols + warp * 16;       // the warp's first column of the head
   const int r = lane >> 2, c2 = (lane & 3) * 2;          // row and first column of the lane in an accumulator tile
@@ -180,8 +183,14 @@ __global__ void __launch_bounds__(kWarps * 32, 2) linear_recurrence_chunked_kern
       }
       if (warp == kWarps - 1) {
         const float all = hi + lo;
-        if (lane == 0) vec[6 * kC + 1] = (hi - all) + lo; else wgt[lane - 1] = b_prev * all;
-        if (lane == 31) wgt[31] = bv;
+        if (lane == 0) {
+          vec[7 * kC + 1] = (hi - all) + lo;
+        } else {
+          const float p = __fmul_rn(b_prev, hi);
+          wgt[lane - 1] = p;
+          wgt_lo[lane - 1] = fmaf(b_prev, lo, fmaf(b_prev, hi, -p));
+        }
+        if (lane == 31) { wgt[31] = bv; wgt_lo[31] = 0.f; }
       }
       // decays above 1 are rare enough to step through: D then stays in [0, 1]
       bad |= !(av >= 0.f && av <= 1.f) || far_off(abs_bits(bv), -60, 40) || !(fabsf(d) < 1.1e12f);
@@ -200,17 +209,19 @@ __global__ void __launch_bounds__(kWarps * 32, 2) linear_recurrence_chunked_kern
 #pragma unroll
       for (int kk = 0; kk < kDk / 16; ++kk) {
         uint32_t qf[1][3][4], kf[3][2][2];
-        zero(ah);
+        if (kk % 2 == 0) zero(ah);
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
           ldmatrix_x4(qf[0][j], q_addr + mt * 16 * kRow + kk * 32 + j * kPiece);
           ldmatrix_x4(reinterpret_cast<uint32_t(&)[4]>(kf[j]), k_addr + kk * 32 + j * kPiece);
         }
         mma6<1, 2>(ah, al[kk & 1], qf, kf);
+        if (kk % 2 == 1) {
 #pragma unroll
-        for (int n = 0; n < 2; ++n)
+          for (int n = 0; n < 2; ++n)
 #pragma unroll
-          for (int i = 0; i < 4; ++i) sum[n][i] += ah[0][n][i];
+            for (int i = 0; i < 4; ++i) sum[n][i] += ah[0][n][i];
+        }
       }
 #pragma unroll
       for (int n = 0; n < 2; ++n)
@@ -239,7 +250,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) linear_recurrence_chunked_kern
       float yl[2][2][4] = {}, hh[2][2][4];
 #pragma unroll
       for (int kk = 0; kk < kDk / 16; ++kk) {
-        zero(hh);
+        if (kk % 2 == 0) zero(hh);
         uint32_t sf[3][2][2];          // [piece][8 columns][half of the 16 keys]
 #pragma unroll
         for (int n = 0; n < 2; ++n)
@@ -251,12 +262,14 @@ __global__ void __launch_bounds__(kWarps * 32, 2) linear_recurrence_chunked_kern
 #pragma unroll
           for (int j = 0; j < 3; ++j) ldmatrix_x4(qf[m][j], q_addr + m * 16 * kRow + kk * 32 + j * kPiece);
         mma6<2, 2>(hh, yl, qf, sf);
+        if (kk % 2 == 1) {
 #pragma unroll
-        for (int m = 0; m < 2; ++m)
+          for (int m = 0; m < 2; ++m)
 #pragma unroll
-          for (int n = 0; n < 2; ++n)
+            for (int n = 0; n < 2; ++n)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) yi[m][n][i] += hh[m][n][i];
+              for (int i = 0; i < 4; ++i) yi[m][n][i] += hh[m][n][i];
+        }
       }
 #pragma unroll
       for (int m = 0; m < 2; ++m)
@@ -305,11 +318,15 @@ __global__ void __launch_bounds__(kWarps * 32, 2) linear_recurrence_chunked_kern
       for (int ks = 0; ks < 2; ++ks)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const float2 w = *reinterpret_cast<const float2*>(wgt + ks * 16 + (i >> 1) * 8 + c2);
-          split3(vr[ks][i][0] * w.x, vr[ks][i][1] * w.y, wf[ks][0][0][i], wf[ks][0][1][i], wf[ks][0][2][i]);
+          const float2 w = *reinterpret_cast<const float2*>(wgt + ks * 16 + (i >> 1) * 8 + c2), wl = *reinterpret_cast<const float2*>(wgt_lo + ks * 16 + (i >> 1) * 8 + c2);
+          const float p0 = __fmul_rn(vr[ks][i][0], w.x), p1 = __fmul_rn(vr[ks][i][1], w.y);   // (not to be fused with what follows: the second parts are p0's and p1's)
+          split3(p0, p1, fmaf(vr[ks][i][0], wl.x, fmaf(vr[ks][i][0], w.x, -p0)), fmaf(vr[ks][i][1], wl.y, fmaf(vr[ks][i][1], w.y, -p1)), wf[ks][0][0][i],
+                 wf[ks][0][1][i], wf[ks][0][2][i]);
         }
       if (tb + kC < t1) load_v(tb + kC);
-      const float at = pre[kC - 1], at_lo = vec[6 * kC + 1];   // the product of the decays in two parts
+      const float at = pre[kC - 1], at_lo = vec[7 * kC + 1];   // the product of the decays in two parts
+      // the state is nearly all of this chunk's making: the mean that small_part() puts back is not enough
+      const bool forgets = at < 0.00390625f;
       // B of 16 tokens x 16 dims, transposed on the way: lanes 0-15 tokens 0-15 of dims 0-7, lanes 16-31 of dims 8-15
       const uint32_t k_addr = sbase + kSmK + (lane & 15) * kRow + (lane >> 4) * 16;
 #pragma unroll
@@ -324,11 +341,31 @@ __global__ void __launch_bounds__(kWarps * 32, 2) linear_recurrence_chunked_kern
             for (int u = 0; u < 2; ++u)
               ldmatrix_x4_trans(reinterpret_cast<uint32_t(&)[4]>(kf[j][2 * u]), k_addr + ks * 16 * kRow + np * 64 + u * 32 + j * kPiece);
           mma6<1, 4>(ah[ks], al, wf[ks], kf);
+          if (forgets) {   // what mma.sync cut off of hi.hi: the same products once more, on top of the negated sum
+#pragma unroll
+            for (int n = 0; n < 4; ++n) {
+              float cut[4];
+#pragma unroll
+              for (int i = 0; i < 4; ++i) cut[i] = -ah[ks][0][n][i];
+              mma(cut, wf[ks][0][0], kf[0][n][0], kf[0][n][1]);
+#pragma unroll
+              for (int i = 0; i < 4; ++i) al[0][n][i] += cut[i];
+            }
+          } else
+          {
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+#pragma unroll
+              for (int i = 0; i < 4; ++i) al[0][n][i] = small_part(ah[ks][0][n][i], al[0][n][i]);
+          }
         }
 #pragma unroll
         for (int n = 0; n < 4; ++n)
 #pragma unroll
-          for (int i = 0; i < 4; ++i) S[4 * np + n][i] = fmaf(S[4 * np + n][i], at, fmaf(S[4 * np + n][i], at_lo, join(ah[0][0][n][i] + ah[1][0][n][i], al[0][n][i])));
+          for (int i = 0; i < 4; ++i) {
+            const float s = S[4 * np + n][i];
+            S[4 * np + n][i] = fmaf(s, at, (ah[0][0][n][i] + ah[1][0][n][i]) + fmaf(s, at_lo, al[0][n][i]));
+          }
       }
     } else {
       // ---- token by token, as the general kernel does it ---------------------------------------------------------------

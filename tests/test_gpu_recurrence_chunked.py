@@ -258,6 +258,7 @@ def test_delta_keys_that_make_u_grow(cuda, size, beta):
 # the sizes below an RMS over 10^5 values and more repeats itself within a few percent, hence the 5 % between what is claimed (no larger) and what
 # is asserted.
 SLACK = 1.05
+LINEAR = ["state space", "retention", "near one", "same sign", "strong decay", "any decay"]
 DELTA = ["per channel", "per head", "near one", "same sign", "strong decay", "long keys"]
 
 
@@ -270,8 +271,40 @@ def _batch(cuda, lens):
             torch.cat([torch.arange(m) for m in lens]).to(cuda))
 
 
-def delta_errors(cuda, kind, seed, lens=(300, 161)):
+def linear_errors(cuda, kind, seed, lens=(300, 161)):
     """Relative RMS errors of y and the state against float64: ((chunks), (token by token)), and whether the two kernels' bits differ."""
+    from nano_vllm_rs_b200 import _ffi, ops
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    rn = lambda *s: torch.randn(*s, generator=gen, device=cuda)
+    heads, groups, dv, n = (16, 16, 128, sum(lens)) if kind == "retention" else (16, 2, 64, sum(lens))
+    q, k, v = rn(n, groups * DK), rn(n, groups * DK), rn(n, heads * dv)
+    dt, d = torch.nn.functional.softplus(rn(n, heads) - 1 + 0.5 * rn(heads)), 1 + 0.2 * rn(heads)
+    if kind == "retention":
+        a, b, d = (1.0 - 2.0 ** (-5 - 3 * torch.arange(heads, device=cuda) / heads)).expand(n, heads), torch.full((n, heads), DK ** -0.5, device=cuda), 0 * d
+    elif kind == "any decay":
+        a, b = torch.rand(n, heads, generator=gen, device=cuda), torch.rand(n, heads, generator=gen, device=cuda) + 0.1
+    else:
+        q, k, v = (torch.nn.functional.silu(x) for x in (q, k, v))
+        a, b = torch.exp(-torch.exp(0.5 * rn(heads) + {"near one": -7.0, "strong decay": 1.0}.get(kind, -1.0)) * dt), dt
+        if kind == "same sign": q, k, v, d = q.abs(), k.abs(), v.abs(), d.abs()
+    a, b = a.contiguous(), b.contiguous()
+    slots, cu, pos = _batch(cuda, lens)
+    state, other = (torch.zeros(len(lens), heads, DK, dv, device=cuda) for _ in range(2))
+    y, z = ops.linear_recurrence(q, k, v, a, state, slots, cu, pos, heads, groups, DK, dv, step=b, skip=d), torch.empty_like(v)
+    _ffi.check(_ffi.lib().nvllm_linear_recurrence(z.data_ptr(), z.stride(0), q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), a.data_ptr(), 1,
+                                                  b.data_ptr(), 1, d.data_ptr(), other.data_ptr(), slots.data_ptr(), cu.data_ptr(), pos.data_ptr(), len(lens), heads, groups, DK,
+                                                  dv, torch.cuda.current_stream().cuda_stream))
+    y64, S64 = torch.empty(n, heads, dv, dtype=torch.float64, device=cuda), torch.zeros(len(lens), heads, DK, dv, dtype=torch.float64, device=cuda)
+    wide = lambda x, t: x[t].double().view(groups, DK).repeat_interleave(heads // groups, 0)
+    for s in range(len(lens)):
+        for t in range(int(cu[s]), int(cu[s + 1])):
+            vt = v[t].double().view(heads, dv)
+            S64[s] = S64[s] * a[t].double()[:, None, None] + (b[t].double()[:, None] * wide(k, t))[:, :, None] * vt[:, None]
+            y64[t] = (S64[s] * wide(q, t)[:, :, None]).sum(1) + d.double()[:, None] * vt
+    return (_rel(y.view_as(y64), y64), _rel(state, S64)), (_rel(z.view_as(y64), y64), _rel(other, S64)), not torch.equal(y, z)
+
+
+def delta_errors(cuda, kind, seed, lens=(300, 161)):
     from nano_vllm_rs_b200 import _ffi, ops
     gen = torch.Generator(device="cuda").manual_seed(seed)
     rn = lambda *s: torch.randn(*s, generator=gen, device=cuda)
@@ -299,7 +332,7 @@ def delta_errors(cuda, kind, seed, lens=(300, 161)):
     return (_rel(y.view_as(y64), y64), _rel(state, S64)), (_rel(z.view_as(y64), y64), _rel(other, S64)), not torch.equal(y, z)
 
 
-@pytest.mark.parametrize("errors,kind", [(delta_errors, k) for k in DELTA], ids=["delta " + k for k in DELTA])
+@pytest.mark.parametrize("errors,kind", [(linear_errors, k) for k in LINEAR] + [(delta_errors, k) for k in DELTA], ids=["linear " + k for k in LINEAR] + ["delta " + k for k in DELTA])
 def test_error_against_float64_is_no_larger(cuda, errors, kind):
     rows = [errors(cuda, kind, seed) for seed in range(3)]
     assert all(r[2] for r in rows), "both entries gave the same bits: the chunked kernel did not run"
