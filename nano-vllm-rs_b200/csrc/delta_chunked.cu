@@ -462,11 +462,17 @@ int launch(const DeltaArgs& a, int n_seqs, cudaStream_t st) {
 }  // namespace
 
 // Where the CTAs take half the SMs at the least: fewer wait for a chunk's chain of phases as long as for its 16 steps (one prompt of 8192 tokens
-// 2.68 and 2.69 ms, 2 x 40 tokens 25 and 24 us).  From 16 tokens a sequence on; one decoded token costs a chunk.
+// 2.68 and 2.69 ms, 2 x 40 tokens 25 and 24 us).  From 16 tokens a sequence on, if they fill three quarters of their chunks (five sixths with a decay
+// per head, where the steps load less): a chunk takes its time however few its tokens are.  Token by token and here (us), 16 heads of 128 x 128, 32
+// sequences, a decay per channel: 16 tokens 58 and 43, 17 62 and 75, 23 76 and 75, 24 79 and 75, 33 101 and 106, 36 108 and 106, 49 141 and 138;
+// per head: 17 57 and 75, 24 71 and 76, 28 81 and 76, 33 92 and 108, 40 108 and 108, 49 128 and 138, 56 143 and 139, 65 163 and 171, 80 196 and 171;
+// 5 and 16 sequences have the same crossings.  (Of a batch of mixed lengths only the mean is known here.)  One decoded token costs a chunk.
 bool delta_chunked_applies(const DeltaArgs& a, bool head_decay, int n_seqs, int n_tokens) {
-  return a.dk == kDk && a.dv % kCols == 0 && 2 * static_cast<int64_t>(a.heads) * n_seqs * (a.dv / kCols) >= sm_count() && static_cast<int64_t>(n_tokens) >= 16 * static_cast<int64_t>(n_seqs) && n_seqs <= 65535 && a.ldq % 4 == 0 &&
-         a.ldk % 4 == 0 && a.ldv % 2 == 0 && a.ldy % 2 == 0 && aligned16(a.q) && aligned16(a.k) && aligned16(a.v) && aligned16(a.y) &&
-         (head_decay || (a.ldd % 4 == 0 && aligned16(a.decay)));
+  const int64_t per_chunk = kC * static_cast<int64_t>(n_seqs), chunks = (n_tokens + per_chunk - 1) / per_chunk;   // of a sequence of the mean length
+  const bool full = head_decay ? 6 * static_cast<int64_t>(n_tokens) >= 5 * chunks * per_chunk : 4 * static_cast<int64_t>(n_tokens) >= 3 * chunks * per_chunk;
+  return a.dk == kDk && a.dv % kCols == 0 && 2 * static_cast<int64_t>(a.heads) * n_seqs * (a.dv / kCols) >= sm_count() && n_tokens >= per_chunk && full &&
+         n_seqs <= 65535 && a.ldq % 4 == 0 && a.ldk % 4 == 0 && a.ldv % 2 == 0 && a.ldy % 2 == 0 && aligned16(a.q) && aligned16(a.k) && aligned16(a.v) &&
+         aligned16(a.y) && (head_decay || (a.ldd % 4 == 0 && aligned16(a.decay)));
 }
 
 int delta_chunked(const DeltaArgs& a, bool head_decay, int n_seqs, cudaStream_t st) {

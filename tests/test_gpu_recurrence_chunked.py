@@ -146,10 +146,12 @@ def _delta_run(cuda, seqs, heads, groups, dv, state, starts, head_decay, tokenwi
     return np.split(y.cpu().numpy().reshape(-1, heads, dv), np.cumsum(lens)[:-1])
 
 
-def _takes_chunks(seqs, heads, dv):
-    """The rule of delta_chunked_applies for these tests' sizes: the CTAs, one per head, sequence and 64 columns, take half the SMs."""
+def _takes_chunks(seqs, heads, dv, head_decay):
+    """The rule of delta_chunked_applies for these tests' sizes: the CTAs, one per head, sequence and 64 columns, take half the SMs, and the tokens fill
+    three quarters of the chunks (five sixths with a decay per head) of sequences of their mean length."""
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    return 2 * heads * len(seqs) * (dv // 64) >= sms and sum(len(s["v"]) for s in seqs) >= 16 * len(seqs)
+    n, slots = sum(len(s["v"]) for s in seqs), 16 * len(seqs)
+    return 2 * heads * len(seqs) * (dv // 64) >= sms and n >= slots and n >= (5 / 6 if head_decay else 3 / 4) * slots * -(-n // slots)
 
 
 def _delta_check(seq, S0, got, state, heads, groups, tokens):
@@ -172,7 +174,8 @@ def _delta_check(seq, S0, got, state, heads, groups, tokens):
     (2, 2, 64, [16], False, 0.5, False), (4, 2, 64, [31, 1, 64], False, 0.9, False), (8, 1, 64, [17, 97], True, 0.5, False),
     (3, 3, 128, [33, 130], False, 0.02, False), (2, 1, 192, [65, 40], True, 0.99, False),
     (16, 16, 128, [33, 16, 1, 64], False, 0.5, True), (16, 4, 128, [31, 1, 64, 20], False, 0.9, True), (40, 8, 64, [17, 97], True, 0.5, True),
-    (16, 2, 192, [15, 40, 33], False, 0.02, True), (37, 37, 64, [65, 40], True, 0.99, True), (16, 16, 128, [130, 48, 16], True, 0.02, True)])
+    (16, 2, 192, [15, 40, 33], False, 0.02, True), (37, 37, 64, [65, 48], True, 0.99, True), (16, 16, 128, [130, 48, 23], True, 0.02, True),
+    (16, 16, 128, [17] * 5, False, 0.5, False), (16, 16, 128, [24] * 5, False, 0.5, True), (16, 8, 128, [24] * 5, True, 0.5, False), (16, 8, 128, [27] * 5, True, 0.5, True)])
 def test_delta_prompts_and_portions(cuda, heads, groups, dv, lens, head_decay, lo, chunks):
     """Chunk edges and tails, single tokens beside prompts, decays from next to nothing to next to one, a second portion that goes on from the slots."""
     rng = np.random.default_rng(sum(lens) + dv)
@@ -180,8 +183,11 @@ def test_delta_prompts_and_portions(cuda, heads, groups, dv, lens, head_decay, l
     S = [np.zeros((heads, DK, dv))] * len(lens)
     for portion in range(2):
         seqs = [_delta_seq(rng, n, heads, groups, dv, head_decay, lo) for n in lens]
-        assert _takes_chunks(seqs, heads, dv) == chunks
+        assert _takes_chunks(seqs, heads, dv, head_decay) == chunks
+        other = state.clone()
         ys = _delta_run(cuda, seqs, heads, groups, dv, state, [portion * n for n in lens], head_decay)
+        ts = _delta_run(cuda, seqs, heads, groups, dv, other, [portion * n for n in lens], head_decay, tokenwise=True)
+        assert chunks == (not torch.equal(state, other)) == any((a != b).any() for a, b in zip(ys, ts)), "the bits tell which kernel ran"
         st = state.cpu().numpy()
         for i, (q, y) in enumerate(zip(seqs, ys)):
             _delta_check(q, S[i], y, st[i], heads, groups, lens[i])
@@ -194,7 +200,7 @@ def test_delta_odd_values(cuda, what, heads, groups, dv, head_decay):
     n, at = 60, 21
     rng = np.random.default_rng(9)
     seqs = [_delta_seq(rng, n, heads, groups, dv, head_decay), _delta_seq(rng, n, heads, groups, dv, head_decay)]
-    assert _takes_chunks(seqs, heads, dv) == (heads > 4)
+    assert _takes_chunks(seqs, heads, dv, head_decay) == (heads > 4)
     s = seqs[0]
     if what == "v nan": s["v"][at, 1, 5] = np.nan
     elif what == "v inf": s["v"][at, 1, 5] = np.inf
@@ -219,7 +225,7 @@ def test_delta_padding_sequences(cuda):
     heads, dv, lens = 40, 128, [20, 40]
     rng = np.random.default_rng(2)
     seqs = [_delta_seq(rng, n, heads, heads, dv, False) for n in lens]
-    assert _takes_chunks(seqs, heads, dv)
+    assert _takes_chunks(seqs, heads, dv, False)
     state = torch.full((2, heads, DK, dv), 3.0, device=cuda)
     ys = _delta_run(cuda, seqs, heads, heads, dv, state, [0, 0], False, slots=[-1, 1])
     assert (ys[0] == 0).all() and (state[0] == 3).all()
@@ -233,7 +239,7 @@ def test_delta_keys_that_make_u_grow(cuda, size, beta):
     heads, dv, n, at = 40, 128, 32, 23
     rng = np.random.default_rng(4)
     seqs = [_delta_seq(rng, n, heads, heads, dv, False, 0.9) for _ in range(2)]
-    assert _takes_chunks(seqs, heads, dv)
+    assert _takes_chunks(seqs, heads, dv, False)
     s = seqs[0]
     s["k"][at:] = s["k"][at] * np.float32(size)      # one direction: every token's A is beta |k|^2
     s["b"][at:] = beta
