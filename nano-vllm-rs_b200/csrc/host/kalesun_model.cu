@@ -32,6 +32,7 @@
 #include <array>
 #include <map>
 
+#include "../recurrence.cuh"
 #include "model_base.hpp"
 
 namespace nvllm {
@@ -500,7 +501,7 @@ class Kalesun : public ModelBase {
         float *gate = proj_ + qkv, *beta = gate + HV, *dec = beta + L.H;
         RUN(lin(proj_, x_, L.in, ld, W, ld, NVLLM_F32, "delta q k v g b a projection"));
         RUN(nvllm_causal_conv(conv_out_, qkv, proj_, ld, L.conv_w, nullptr, ls.conv, v.tok_seq, v.seq_slots, v.cu_tokens, v.positions, N, S, qkv, L.taps, 1,
-                              st)); launches += conv_launches(N, S, qkv, L.taps) - 1; mk("causal_conv");
+                              st)); launches += causal_conv_launches(conv_out_, qkv, proj_, ld, ls.conv, N, S, qkv, L.taps) - 1; mk("causal_conv");
         RUN(nvllm_head_delta_prepare(conv_out_, qkv, conv_out_ + qc, qkv, beta, ld, dec, ld, L.a_log, L.dt_bias, N, L.H, L.G, L.D,
                                      1.0f / sqrtf(static_cast<float>(L.D)), 1e-6f, st)); mk("head_delta_prepare");
         RUN(nvllm_delta_recurrence_step(y_, HV, conv_out_, qkv, conv_out_ + qc, qkv, conv_out_ + qc + kc, qkv, dec, ld, 1, beta, ld, ls.S, v.seq_slots,

@@ -75,9 +75,4 @@ ModelImpl* make_zasorax(const json::Value& cfg);  // zasorax_model.cu
 ModelImpl* make_kalesun(const json::Value& cfg);  // kalesun_model.cu
 ModelImpl* make_fomerax(const json::Value& cfg);  // fomerax_model.cu
 
-// Launches of nvllm_causal_conv over a step: its kernel and the state's, or one for both (single tokens).
-inline int conv_launches(int tokens, int seqs, int channels, int taps) {
-  return taps == 1 || (tokens == seqs && taps <= 4 && channels % 4 == 0) ? 1 : 2;
-}
-
 }  // namespace nvllm

@@ -30,7 +30,7 @@
 #include <string>
 #include <vector>
 
-#include "../common.cuh"
+#include "../recurrence.cuh"
 #include "model.hpp"
 
 namespace nvllm {
@@ -533,7 +533,7 @@ class Talapel : public ModelImpl {
         const int inner = L.s_inner(), gns = L.sG * L.sN, ch = L.s_ch(), lds = pad8(L.s_cols());
         RUN(lin(proj_, normed_, L.s_in, lds, W, lds, NVLLM_F32, "ssd input projection"));
         RUN(nvllm_causal_conv(conv_out_, ch, proj_ + inner, lds, L.conv_w, L.conv_b, rs.conv, v.tok_seq, v.seq_slots, v.cu_tokens, v.positions, N, S,
-                              ch, L.taps, 1, st)); launches += conv_launches(N, S, ch, L.taps); mk("causal_conv");
+                              ch, L.taps, 1, st)); launches += causal_conv_launches(conv_out_, ch, proj_ + inner, lds, rs.conv, N, S, ch, L.taps); mk("causal_conv");
         RUN(nvllm_ssd_prepare(step_, decay_t_, proj_ + inner + ch, lds, L.dt_bias, L.a_log, N, L.sH, st)); ++launches; mk("ssd_prepare");
         RUN(nvllm_linear_recurrence_step(y_, inner, conv_out_ + inner + gns, ch, conv_out_ + inner, ch, conv_out_, ch, decay_t_, 1, step_, 1, L.skip,
                                     rs.ssd, v.seq_slots, v.cu_tokens, v.positions, N, S, L.sH, L.sG, L.sN, L.sP, st)); ++launches; mk("linear_recurrence (ssd)");

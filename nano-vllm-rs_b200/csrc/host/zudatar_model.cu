@@ -33,7 +33,7 @@
 #include <string>
 #include <vector>
 
-#include "../common.cuh"
+#include "../recurrence.cuh"
 #include "model.hpp"
 
 namespace nvllm {
@@ -616,7 +616,7 @@ class Zudatar : public ModelImpl {
         RUN(lin(decay_, lr_out_, L.a2, HD, L.ra, ldlr, HD, NVLLM_F32, "delta decay second step"));
         RUN(lin(gate_, off(lr_out_, pad8(L.ra)), L.g2, HV, L.rg, ldlr, HV, NVLLM_F32, "delta gate second step"));
         RUN(nvllm_causal_conv(conv_out_, ch, proj_, ldd, L.conv_w, nullptr, ls.conv, v.tok_seq, v.seq_slots, v.cu_tokens, v.positions, N, S, ch,
-                              L.taps, 1, st)); launches += conv_launches(N, S, ch, L.taps); mk("causal_conv");
+                              L.taps, 1, st)); launches += causal_conv_launches(conv_out_, ch, proj_, ldd, ls.conv, N, S, ch, L.taps); mk("causal_conv");
         RUN(nvllm_delta_prepare(conv_out_, ch, conv_out_ + GD, ch, proj_ + ch, ldd, decay_, HD, L.a_log, L.dt_bias, N, L.H, L.G, L.D,
                                 1.0f / sqrtf(static_cast<float>(L.D)), 1e-6f, st)); ++launches; mk("delta_prepare");
         RUN(nvllm_delta_recurrence_step(y_, HV, conv_out_, ch, conv_out_ + GD, ch, conv_out_ + 2 * GD, ch, decay_, HD, 0, proj_ + ch, ldd, ls.S,

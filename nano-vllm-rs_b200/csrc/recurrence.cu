@@ -1119,8 +1119,7 @@ extern "C" int nvllm_causal_conv(float* out, int64_t ldo, const float* in, int64
   NVLLM_CHECK_ARG(out && in && w && state && tok_seq && seq_slot && cu_tokens && positions && out != in, NVLLM_ERR_ARG, "causal_conv: NULL");
   ConvArgs a{out, ldo, in, ldi, w, bias, state, tok_seq, seq_slot, cu_tokens, positions, n, channels, taps, silu};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // as many tokens as sequences: single tokens
-  if (n == n_seqs && taps >= 2 && taps <= 4 && channels % 4 == 0 && ldi % 4 == 0 && ldo % 4 == 0 && aligned16(in) && aligned16(out) && aligned16(state)) {
+  if (causal_conv_single(out, ldo, in, ldi, state, n, n_seqs, channels, taps)) {
     NVLLM_CUDA(launch_pdl(taps == 2 ? causal_conv_single_kernel<2> : (taps == 3 ? causal_conv_single_kernel<3> : causal_conv_single_kernel<4>),
                           dim3(static_cast<unsigned>(n), static_cast<unsigned>((channels / 4 + 127) / 128)), dim3(128), 0, st, a));
     NVLLM_LAUNCH_CHECK("causal_conv_single_kernel");

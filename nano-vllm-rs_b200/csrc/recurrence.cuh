@@ -1,4 +1,5 @@
-// recurrence.cuh — the arguments of the recurrences, shared by their kernels (recurrence.cu; for prompts recurrence_chunked.cu, delta_chunked.cu).
+// recurrence.cuh — the arguments of the recurrences, shared by their kernels (recurrence.cu; for prompts recurrence_chunked.cu, delta_chunked.cu), and
+// what of their dispatch the models count launches by.
 #pragma once
 
 #include "common.cuh"
@@ -36,5 +37,14 @@ struct DeltaArgs {
 // delta_chunked.cu: takes a gated delta rule (a decay per key channel, or one per head) if the sizes and the alignment suit it.
 bool delta_chunked_applies(const DeltaArgs& a, bool head_decay, int n_seqs, int n_tokens);
 int delta_chunked(const DeltaArgs& a, bool head_decay, int n_seqs, cudaStream_t st);
+
+// nvllm_causal_conv over a step of single tokens (as many tokens as sequences): one launch for the convolution and its state.
+inline bool causal_conv_single(const float* out, int64_t ldo, const float* in, int64_t ldi, const float* state, int n, int n_seqs, int channels, int taps) {
+  return n == n_seqs && taps >= 2 && taps <= 4 && channels % 4 == 0 && ldi % 4 == 0 && ldo % 4 == 0 && aligned16(in) && aligned16(out) && aligned16(state);
+}
+// Launches of nvllm_causal_conv over any step: its kernel and the state's, or one.
+inline int causal_conv_launches(const float* out, int64_t ldo, const float* in, int64_t ldi, const float* state, int n, int n_seqs, int channels, int taps) {
+  return taps == 1 || causal_conv_single(out, ldo, in, ldi, state, n, n_seqs, channels, taps) ? 1 : 2;
+}
 
 }  // namespace nvllm
