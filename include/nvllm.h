@@ -4,7 +4,7 @@
  * This is the drop-in boundary for ssvgopal/nano-vllm-rs.  The reference has no FFI of its own
  * (pure Rust on candle); each entry point below replaces one Rust method on the hot path and cites
  * it as  <file>:<lines>  relative to the reference tree.  The Rust-side binding a maintainer
- * would add is shown in INTEGRATION.md and rust/ffi.rs.
+ * would add is shown in rust/ffi.rs.
  *
  * Conventions (all entry points):
  *   - return 0 on success, <0 for an argument error (shape / alignment / dtype), >0 = cudaError_t;

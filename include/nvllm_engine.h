@@ -2,7 +2,7 @@
  * nvllm_engine.h — C ABI of the C++ host runtime that mirrors the reference's Rust engine types for the
  * paged-attention decode hot path: Config / Qwen3Config, SamplingParams, Sequence, BlockManager, Scheduler,
  * ModelRunner, LLMEngine.  The reference toolchain (Rust) is absent from this image, so the host side above the
- * kernel ABI (nvllm.h) is C++; a Rust crate would bind either level (rust/ffi.rs, INTEGRATION.md).
+ * kernel ABI (nvllm.h) is C++; a Rust crate would bind either level (rust/ffi.rs).
  * Citations are file:line under the reference's src/.
  *
  * Error convention: as nvllm.h (0 OK, <0 argument/state error, >0 cudaError_t, nvllm_last_error()).
@@ -192,7 +192,7 @@ int64_t nvllm_runner_profile_report(nvllm_runner* r, char* h_buf, size_t cap);
 int nvllm_runner_set_eager(nvllm_runner* r, int32_t eager);
 /* Number of kernels launched by the last execute (decode graph node count, or eager launches). */
 int64_t nvllm_runner_last_launches(const nvllm_runner* r);
-/* Device pointers of layer `layer`'s K / V cache and the layout in use (tests). */
+/* Device pointers of layer `layer`'s K / V cache and the layout in use (tests, hosts that bind layers). */
 int nvllm_runner_kv_cache(nvllm_runner* r, int32_t layer, void** k_cache, void** v_cache, nvllm_kv_layout* layout);
 /* Re-runs only the paged decode attention of layer 0 on the last decode batch `iters` times between two CUDA
  * events (for the roofline line of bench.py); returns the average milliseconds per launch. */

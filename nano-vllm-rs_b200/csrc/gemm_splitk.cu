@@ -291,7 +291,7 @@ int launch_splitk(const CUtensorMap& tx, const CUtensorMap& tw, void* y, int M, 
 }
 
 // Cost of one CTA in "bytes through the SM's TMA port" (~40-60 B/clk): the operands, plus the reduce-scatter of the
-// partial tile over DSMEM — (SK-1)/SK of a BN x 128 f32 tile per CTA at ~20 B/clk (B300_MICROARCH.md: 17-21 B/clk), i.e.
+// partial tile over DSMEM — (SK-1)/SK of a BN x 128 f32 tile per CTA at ~20 B/clk (measured 17 to 21), i.e.
 // weighted x4 — which is why narrow tiles with SK = 4 win for the 0.6B projections.  Clusters of 8 measured 3-6 us
 // slower than clusters of 4 at equal bytes (fewer can be co-scheduled per GPC): flat penalty.
 long splitk_cost(int bn, int sk, int k) {

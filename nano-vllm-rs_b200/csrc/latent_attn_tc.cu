@@ -10,10 +10,10 @@
 // columns that a 256-wide O and two S tiles leave hold the first 256 query values as the A operand (read from TMEM, not from
 // shared memory); the other 320 sit in shared memory beside two 64-key tiles (80 + 2 x 72 KB).
 // Roles: warps 0-3 own a row each thread (softmax, P back into the S columns, output), warps 4-7 copy key tiles (cp.async in 16-byte
-// steps through the block table, zeros past the sequence's keys), one lane of warp 8 issues the MMAs.  S of the next tile runs
-// while a tile's softmax does.
-// Measured, 8 x 1024 tokens x 16 heads: 464 us (mma.sync kernel: 1526).  Per 64-key tile the MMAs take ~4100 clocks (S 36 x ~75: an
-// N64 step costs what an N128 one does; PV 4 x ~180), the rest of the ~5000 is S waiting for a tile's copies.
+// steps through the block table, zeros past the sequence's keys), warp 8 issues the MMAs (converged, one elected lane).  S of the next
+// tile runs while a tile's softmax does.
+// Measured, 8 x 1024 tokens x 16 heads: 387 us (mma.sync kernel: 1526; with a diverged issuing lane 470).  An N64 step of S costs what an N128 one
+// does; what the MMAs leave of a tile's time is S waiting for its copies.
 #include "latent_attn.cuh"
 #include "tc.cuh"
 

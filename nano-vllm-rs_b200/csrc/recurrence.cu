@@ -28,10 +28,6 @@ namespace {
 
 constexpr int kRecTile = 16;  // tokens per stage
 
-__device__ __forceinline__ void cp_async_4(uint32_t smem_addr, const void* gptr) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(smem_addr), "l"(gptr) : "memory");
-}
-
 // CTA = (head, sequence, slice of dv).  Thread (pc, ns): PP neighbouring columns of the state, rows [ns * NPT, (ns + 1) * NPT) of
 // each in registers (every k / q value read from shared memory serves PP columns: the broadcast reads are what binds).
 // kRecTile tokens' k, q (rows of dk), v, a, b are staged in shared memory with cp.async, two stages deep: the copies of the
@@ -735,7 +731,6 @@ __global__ void rotate_half_kernel(float* __restrict__ x, int64_t ldx, const int
   }
 }
 
-// One CTA per (token, part): parts of `gs` values.  gate_first: t = y * silu(z), out = rms(t) * w;  else out = rms(y) * silu(z) [* w].
 // The same in 16-byte pieces, a CTA per token: a piece of the first half with its partner of the second, four pairs.  8192 tokens x 32 heads
 // of 128 (a 268 MB pass, 41 us at the copy rate): 76 us value by value, 42 so; half of each head rotated, all scaled: 98 and 52.
 __global__ void __launch_bounds__(256) rotate_half_vec_kernel(float* __restrict__ x, int64_t ldx, const int64_t* __restrict__ positions,
@@ -761,6 +756,7 @@ __global__ void __launch_bounds__(256) rotate_half_vec_kernel(float* __restrict_
   }
 }
 
+// One CTA per (token, part): parts of `gs` values.  gate_first: t = y * silu(z), out = rms(t) * w;  else out = rms(y) * silu(z) [* w].
 template <typename TO>
 __global__ void __launch_bounds__(128) gated_group_norm_kernel(TO* __restrict__ out, int64_t ldo, const float* __restrict__ y, int64_t ldy,
                                                                const float* __restrict__ z, int64_t ldz, const float* __restrict__ w, int gs,

@@ -6,6 +6,10 @@
 
 namespace nvllm {
 
+__device__ __forceinline__ void cp_async_4(uint32_t smem_addr, const void* gptr) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(smem_addr), "l"(gptr) : "memory");
+}
+
 struct RecArgs {
   float* y; int64_t ldy;
   const float *q, *k, *v; int64_t ldq, ldk, ldv;

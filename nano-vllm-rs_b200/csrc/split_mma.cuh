@@ -7,10 +7,6 @@
 namespace nvllm {
 namespace split {
 
-__device__ __forceinline__ void cp_async_4(uint32_t smem_addr, const void* gptr) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(smem_addr), "l"(gptr) : "memory");
-}
-
 __device__ __forceinline__ uint32_t abs_bits(float x) { return __float_as_uint(x) & 0x7fffffffu; }
 
 __device__ __forceinline__ bool far_off(uint32_t bits, int lo, int hi) {   // not zero and outside [2^lo, 2^hi)

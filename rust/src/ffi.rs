@@ -1,6 +1,6 @@
 //! Safe(r) wrappers with the reference's method surface over the generated `extern "C"` declarations (ffi_gen.rs): one
-//! type per layer of nano-vllm-rs whose `forward` the B200 library replaces (INTEGRATION.md §1), plus RAII handles for the
-//! host-runtime level (§2).  Tensors stay owned by Rust (candle); the wrappers borrow raw device pointers for the duration
+//! type per layer of nano-vllm-rs whose `forward` the B200 library replaces, plus RAII handles for the
+//! host-runtime level.  Tensors stay owned by Rust (candle); the wrappers borrow raw device pointers for the duration
 //! of the enqueued work, so every call is `unsafe` and takes the CUDA stream explicitly.
 //! COMPILE-UNVERIFIED (no Rust toolchain in the build image); the same ABI is exercised through ctypes by
 //! nano-vllm-rs_b200/_ffi.py and every test under tests/.
