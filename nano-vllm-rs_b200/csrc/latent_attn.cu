@@ -808,8 +808,8 @@ int launch_attn_mma(const AttnArgs& a, cudaStream_t st) {
     return a.skip_dense ? launch_attn_mma_tq<NT2, 2, true>(b, st) : launch_attn_mma_tq<NT2, 2, false>(b, st);
   }
   // Single tokens without a window on fewer CTAs than SMs: a cluster shares the key tiles of a token, as many CTAs as give each (at the
-  // longest context the tables allow; the kernel looks at the token's own) kShareTiles tiles.  Measured, 16 heads, rank 512 (us, one CTA a
-  // token -> so): 1 token at 4001 keys 218 -> 36, 32 at 4001 221 -> 68, 11 at 279 22.0 -> 16.2, 40 at 33 9.0 -> 9.2.  With partials in
+  // longest context the tables allow; the kernel looks at the token's own) kShareTiles tiles.  Measured, 16 heads, at rank 512 before that
+  // rank had a kernel of its own (us, one CTA a token -> so): 1 token at 4001 keys 218 -> 36, 32 at 4001 221 -> 68, 11 at 279 22.0 -> 16.2, 40 at 33 9.0 -> 9.2.  With partials in
   // memory and a second kernel, whose cost follows the splits that the tables allow, 1 token at 33 keys in tables for 4096 took 36.
   AttnArgs b = a;
   if (a.n <= 256 && a.window == 0) {
@@ -970,9 +970,11 @@ int run_attention(const AttnArgs& a, size_t workspace_bytes, int dtype, int n_se
       if (int rc = latent_attn_tc_launch(a, st)) return rc;
       b.skip_dense = 1;   // tiles of many sequences are left to the kernel below
     }
+    // rank 512, up to 256 tokens (single tokens, or what the tcgen05 kernel leaves of prompts): a kernel of its own, each token by itself
+    if ((a.n <= 256 || knobs().latent_mma == 2) && latent_attn_decode_applies(a)) return latent_attn_decode_launch(b, st);
     // Single tokens with a bounded key range (a window) and fewer CTAs than SMs: split every token's key tiles over up to 4
     // CTAs, as many as fill the SMs once and leave each at least eight tiles; the partials meet in latent_attn_merge_kernel.
-    // (Measured, 64 tokens x 16 heads, rank 512: a window of 2048 keys 118 -> 79 us; at 512 keys the second launch costs what
+    // (Measured, 64 tokens x 16 heads, rank 512 on this kernel: a window of 2048 keys 118 -> 79 us; at 512 keys the second launch costs what
     // the shorter loop saves, 39 -> 37 us, so short windows stay on one CTA.)
     if (a.part != nullptr && a.n <= 256 && a.window > 0) {
       const int64_t ctas = static_cast<int64_t>(a.n) * ((a.heads + 15) / 16);

@@ -35,5 +35,7 @@ __device__ __forceinline__ bool latent_tile_dense(const int32_t* __restrict__ to
 
 bool latent_attn_tc_applies(const LatentAttnArgs& a);                 // latent_attn_tc.cu
 int latent_attn_tc_launch(const LatentAttnArgs& a, cudaStream_t st);
+bool latent_attn_decode_applies(const LatentAttnArgs& a);             // latent_attn_decode.cu
+int latent_attn_decode_launch(const LatentAttnArgs& a, cudaStream_t st);
 
 }  // namespace nvllm
