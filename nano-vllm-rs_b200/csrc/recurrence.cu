@@ -1048,6 +1048,7 @@ extern "C" int nvllm_delta_recurrence_step(float* y, int64_t ldy, const float* q
   NVLLM_CHECK_ARG(y && q && k && v && decay && beta && state && seq_slot && cu_tokens && positions, NVLLM_ERR_ARG, "delta_recurrence: NULL");
   const DeltaArgs a{y, ldy, q, k, v, ldq, ldk, ldv, heads / groups, decay, ldd, beta, ldb, state, seq_slot, cu_tokens, positions, heads, dk, dv};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (delta_single_applies(a, n_seqs, n)) return delta_single(a, head_decay != 0, n_seqs, st);
   if (delta_chunked_applies(a, head_decay != 0, n_seqs, n)) return delta_chunked(a, head_decay != 0, n_seqs, st);
   return head_decay ? launch_delta<true>(a, n_seqs, st) : launch_delta<false>(a, n_seqs, st);
 }
@@ -1093,6 +1094,7 @@ extern "C" int nvllm_linear_recurrence_step(float* y, int64_t ldy, const float* 
   RecArgs a{y, ldy, q, k, v, ldq, ldk, ldv, heads / groups, decay, decay_per_token ? heads : 0, step, step_per_token ? heads : 0,
             skip, state, seq_slot, cu_tokens, positions, heads, dk, dv, 1.0f};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (linear_recurrence_single_applies(a, n_seqs, n)) return linear_recurrence_single(a, n_seqs, st);
   if (linear_recurrence_chunked_applies(a, n_seqs, n)) return linear_recurrence_chunked(a, n_seqs, st);
   return launch_recurrence<false>(a, n_seqs, st);
 }

@@ -42,6 +42,12 @@ struct DeltaArgs {
 bool delta_chunked_applies(const DeltaArgs& a, bool head_decay, int n_seqs, int n_tokens);
 int delta_chunked(const DeltaArgs& a, bool head_decay, int n_seqs, cudaStream_t st);
 
+// recurrence_step.cu: take steps of single tokens (as many tokens as sequences; linear recurrences with a decay per head) if the sizes and the alignment suit them.
+bool linear_recurrence_single_applies(const RecArgs& a, int n_seqs, int n_tokens);
+int linear_recurrence_single(const RecArgs& a, int n_seqs, cudaStream_t st);
+bool delta_single_applies(const DeltaArgs& a, int n_seqs, int n_tokens);
+int delta_single(const DeltaArgs& a, bool head_decay, int n_seqs, cudaStream_t st);
+
 // nvllm_causal_conv over a step of single tokens (as many tokens as sequences): one launch for the convolution and its state.
 inline bool causal_conv_single(const float* out, int64_t ldo, const float* in, int64_t ldi, const float* state, int n, int n_seqs, int channels, int taps) {
   return n == n_seqs && taps >= 2 && taps <= 4 && channels % 4 == 0 && ldi % 4 == 0 && ldo % 4 == 0 && aligned16(in) && aligned16(out) && aligned16(state);
