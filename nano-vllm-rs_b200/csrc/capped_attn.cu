@@ -17,7 +17,7 @@
 // of neighbouring dimensions, a weightless per-head RMS norm after the rotation, and values that are the un-rotated keys.
 // nvllm_attn_norm_rotary_store: a weighted per-head RMS norm before the rotation, values mixed with an earlier layer's.
 // Scores, softmax and the accumulation of P.V are f32.
-#include "common.cuh"
+#include "capped_attn.cuh"
 #include "prefill_attn.cuh"
 
 namespace nvllm {
@@ -478,38 +478,10 @@ __global__ void __launch_bounds__(128) attn_norm_rotary_store_vec_kernel(const N
   }
 }
 
-struct AttnArgs {
-  void* out; int64_t ldo;
-  const void* q; int64_t ldq;
-  const float* gate; int64_t ldg;
-  const void *kc, *vc; int64_t k_row, v_row;
-  const int32_t* tok_seq; const int64_t* positions; const int32_t* tables;
-  int table_cap, block_size, n, heads, kv_heads, dim, vdim;
-  float scale, softcap, temp_coef; int temp_every;
-  int window; const float* sinks; int gate_per_head;
-  const int32_t* dense_cu;   // non-null (and tables null): keys are not paged, key j of sequence s is row dense_cu[s] + j
-  // positional options of nvllm_biased_attention (all off when zero / null)
-  int keep;                  // > 0: the keys 0 .. keep - 1 stay visible outside the window (or chunk), at their true positions
-  int chunk;                 // > 0: position p sees only the keys of its own chunk, floor(p / chunk) * chunk .. p
-  const float* head_scale;   // [heads]: a factor per head on the scaled score
-  const float* dist_bias;    // [heads, dist_rows]: added to the score of key j: dist_bias[h, min(p - j, dist_rows - 1)]
-  int dist_rows;
-  const float2* out_rot;     // [max_pos, vdim / 2] (cos, sin): every head's output is turned by -p, value m paired with m + vdim / 2
-  int max_pos;
-  int bias_staged;           // tensor-core kernel: the CTA copies its heads' rows of dist_bias into shared memory first
-  const float* slopes;       // [heads]: slopes[h] * (p - j) is taken off the score of key j, after the cap
-  const void* ks; int64_t ks_row; int shared;   // shared > 0: the last `shared` values of every head's key are row `slot` of ks
-};
-
 // shared memory the tensor-core kernel may spend on the distance-bias rows of a CTA's heads (two CTAs per SM still fit)
 constexpr int kBiasSmemBytes = 9216;
 
-// first key a row at position p sees
-__device__ __forceinline__ int first_key(const AttnArgs& a, int p) {
-  int lo = a.window > 0 ? max(0, p - a.window + 1) : 0;
-  if (a.chunk > 0) lo = max(lo, p / a.chunk * a.chunk);
-  return lo;
-}
+using AttnArgs = CappedAttnArgs;
 
 // With a cap and a slope the keys further back than this carry exactly no weight: scores lie within +-cap before the slope, so a
 // key d tokens back is at least slope d - 2 cap below the row's own key, and exp(-104) is below the smallest f32 number.
@@ -645,13 +617,7 @@ __global__ void __launch_bounds__(128) capped_attn_warp_kernel(const AttnArgs a)
 // cap, mask and the online softmax in f32.  Key tiles start at multiples of 64 from the sequence's first key whatever the
 // portion, so a row's result does not depend on how the prompt was cut.  Head sizes are padded to DMAX / VMAX with zeros in
 // shared memory.
-constexpr float kLog2e = 1.4426950408889634f;
 constexpr int kWarps = 8, kRows = 16 * kWarps, kKeys = 64;   // (heads beyond 128 values: 16 warps, see launch_mma)
-
-// tanh(x) = 1 - 2 / (2^(2 x log2 e) + 1): two MUFU operations (ex2, rcp), absolute error ~1e-6; exact at both saturations
-// (2^inf -> 1, 2^-inf -> -1).  The one-instruction tanh.approx is 2^-11 relative: too coarse where two scores near the cap
-// compete (cap x 5e-4 apart in the exponent).
-__device__ __forceinline__ float fast_tanh(float x) { return 1.0f - __fdividef(2.0f, fast_exp2(x * (2.0f * kLog2e)) + 1.0f); }
 
 // One warp's share of a key tile: 16 rows x (16 NP) keys -> S on tensor cores, cap / mask / online softmax in f32, then
 // O[:, 0 .. 16 VP) += P . V.  k_addr / v_addr are the warp's ldmatrix lane addresses of its first key (and first value column).
@@ -1237,6 +1203,7 @@ extern "C" int nvllm_extended_attention(void* out, int64_t ldo, const void* q, i
     if (prompt_attention_applies(e, n, heads, kv_heads, dim, vdim, ldq, k_row, v_row, ldo, out, q, k_cache, v_cache, block_tables != nullptr, block_size))
       return prompt_attention(e, out, ldo, q, ldq, k_cache, v_cache, k_row, v_row, cu_tokens, block_tables, table_cap, block_size, n, heads, kv_heads, st);
   }
+  if (dtype == NVLLM_BF16 && cu_tokens != nullptr && knobs().capped_mma == 1 && capped_decode_applies(a, n_seqs)) return capped_decode(a, st);
   // bf16 with 16-byte rows and a token range per sequence: tensor cores; everything else (f32, odd sizes): one warp per row
   const int group = heads / kv_heads;
   if (dtype == NVLLM_BF16 && cu_tokens != nullptr && n_seqs > 0 && knobs().capped_mma && group <= kRows && dim % 8 == 0 && vdim % 8 == 0 &&
