@@ -263,6 +263,18 @@ __device__ __forceinline__ float glu_clamped_fast(float g, float u, float limit)
 }
 // silu where a bf16 result follows: fast exponential and division (the division's divisor must stay below 2^126).
 __device__ __forceinline__ float silu_fast(float g) { return __fdividef(g, 1.0f + __expf(fminf(-g, 80.0f))); }
+// silu of a bf16 value, rounded to bf16 by the caller: what g / (1 + expf(-g)) rounds to for every one of the 65536 values, without the calls
+// and branches of expf and the division, which keep an epilogue's one warp per scheduler from overlapping its elements (64 x 8192 x 2048, gated:
+// 31.6 us with them, 19.9 so).  The quotient's scale of 2^-8 keeps its reciprocal a normal number up to where the exponential
+// overflows; behind that the maximum with 0 (which drops a NaN of inf x 0) leaves 0.
+__device__ __forceinline__ float fast_exp2(float x);
+__device__ __forceinline__ float silu_bf16(float g) {
+  const float d = fmaf(fast_exp2(g * -1.4426950408889634f), 0.00390625f, 0.00390625f);   // (1 + e^-g) / 256
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  r *= fmaxf(fmaf(-d, r, 2.0f), 0.0f);   // a Newton step
+  return g * (r * 0.00390625f);
+}
 // The tanh form of gelu, 0.5 z (1 + tanh(a)) with a = sqrt(2 / pi) (z + 0.044715 z^3), written as z sigmoid(2 a): one exponential,
 // saturating cleanly at both ends.
 constexpr float kGeluA = 1.5957691216057308f;   // 2 sqrt(2 / pi)
@@ -282,7 +294,7 @@ __device__ __forceinline__ float2 gated_pair(uint32_t gb, uint32_t ub, float lim
   if (GATE == kGateClamped) return make_float2(glu_clamped_fast(g0, bf16_lo(ub), limit), glu_clamped_fast(g1, bf16_hi(ub), limit));
   if (GATE == kGateGelu) return make_float2(gelu_tanh_fast(g0) * bf16_lo(ub), gelu_tanh_fast(g1) * bf16_hi(ub));
   if (GATE == kGateSiluRow) return make_float2(silu_fast(g0) * bf16_lo(ub), silu_fast(g1) * bf16_hi(ub));
-  const uint32_t sb = pack_bf16x2(g0 / (1.0f + expf(-g0)), g1 / (1.0f + expf(-g1)));
+  const uint32_t sb = pack_bf16x2(silu_bf16(g0), silu_bf16(g1));
   return make_float2(bf16_lo(sb) * bf16_lo(ub), bf16_hi(sb) * bf16_hi(ub));
 }
 

@@ -349,7 +349,7 @@ silu_mul_kernel(uint4* __restrict__ out, const uint4* __restrict__ x, int64_t to
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const float g0 = bf16_lo(gw[k]), g1 = bf16_hi(gw[k]);
-      const uint32_t s = pack_bf16x2(g0 / (1.0f + expf(-g0)), g1 / (1.0f + expf(-g1)));
+      const uint32_t s = pack_bf16x2(silu_bf16(g0), silu_bf16(g1));
       o[k] = pack_bf16x2(bf16_lo(s) * bf16_lo(uw[k]), bf16_hi(s) * bf16_hi(uw[k]));
     }
     out[i] = make_uint4(o[0], o[1], o[2], o[3]);
