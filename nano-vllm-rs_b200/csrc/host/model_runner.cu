@@ -719,7 +719,10 @@ int nvllm_runner::forward(int N, int S, bool is_prefill, bool paged_prefill, con
       }
     }
     if (!is_prefill) {
-      if (!roped) {  // one launch: q/k-norm + RoPE + KV store + split-K paged attention (qwen3.rs:219-233)
+      if (!roped && few) {   // one launch: q/k-norm + RoPE + KV store + split-K paged attention (qwen3.rs:219-233)
+        RUN(paged_decode_fused_in_step(attn, qkv, d_pos, rope, qnw, knw, eps, cfg.max_position_embeddings, kc[l], vc[l], d_slots, d_tables, d_ctx, N, H,
+                                       table_cap, qkv_dim, HD, &layout, scale, decode_ws, decode_ws_bytes, splits, stream));
+      } else if (!roped) {
         RUN(nvllm_paged_decode_attention_fused(attn, qkv, d_pos, rope, qnw, knw, eps, cfg.max_position_embeddings, kc[l], vc[l],
                                                d_slots, d_tables, d_ctx, N, H, table_cap, qkv_dim, HD, &layout, scale,
                                                decode_ws, decode_ws_bytes, splits, NVLLM_BF16, st));

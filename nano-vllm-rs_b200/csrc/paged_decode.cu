@@ -57,8 +57,12 @@ struct DecodeParams {
   const int32_t* slots;
   float eps;
   int max_position;
+  int early = 0;    // FUSE: tables, lengths and all earlier tokens' rows were written before the chain of programmatic launches that this
+                    // launch belongs to began (paged_decode_fused_in_step): they are read before the wait for the predecessor
   int cluster = 0;  // FUSE: the splits of an item are one cluster and merge over distributed shared memory (no partials, no second kernel)
 };
+
+constexpr int kMaxClusterSplits = 16;   // CTAs of a cluster that merges inside the kernel
 
 template <int D, int STAGES, int NWARPS>
 struct DecodeCfg {
@@ -95,8 +99,7 @@ paged_decode_kernel(const DecodeParams p) {
   const int b = blockIdx.z;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  pdl_wait();  // q and the newest KV row were written by the previous kernel
-  if (FUSE) pdl_launch_dependents();   // (steps of few tokens: not earlier, see gemm_skinny.cu)
+  if (!FUSE || !p.early) pdl_wait();  // q and the newest KV row were written by the previous kernel
   const int ctx_all = __ldg(p.ctx + b);        // tokens attended to, including (FUSE) this step's own
   const int ctx = FUSE ? max(ctx_all - 1, 0) : ctx_all;  // tokens read from the cache
   const int gvalid = min(8, p.g - grp * 8);   // q heads handled by this CTA
@@ -148,6 +151,30 @@ paged_decode_kernel(const DecodeParams p) {
 
   // ---- Q^T B-fragments: head n = lane/4, dims 16ks + 2(lane%4) + {0,1} (+8) --------------------
   uint32_t qb[KS][2];
+  // FUSE: what the norm and the rotation of q need besides q
+  uint32_t nw[FUSE ? KS : 1][2];
+  float rc[FUSE ? KS / 2 : 1][4], rs[FUSE ? KS / 2 : 1][4];
+  if constexpr (FUSE) {
+    static_assert(!FUSE || D == 128, "fused q/k-norm + RoPE: head_dim 128");
+    int64_t pos = __ldg(p.pos + b);
+    pos = pos < 0 ? 0 : (pos >= p.max_position ? p.max_position - 1 : pos);
+    const float* cs = p.cos_sin + pos * D;
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) {
+      const int d0 = ks * 16 + (lane & 3) * 2;
+      nw[ks][0] = p.qnw != nullptr ? __ldg(reinterpret_cast<const uint32_t*>(p.qnw + d0)) : 0u;
+      nw[ks][1] = p.qnw != nullptr ? __ldg(reinterpret_cast<const uint32_t*>(p.qnw + d0 + 8)) : 0u;
+      if (ks < KS / 2) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {   // d0 < 64
+          rc[ks][e] = __ldg(cs + d0 + (e & 1) + (e >> 1) * 8);
+          rs[ks][e] = __ldg(cs + D / 2 + d0 + (e & 1) + (e >> 1) * 8);
+        }
+      }
+    }
+    if (p.early) pdl_wait();
+    pdl_launch_dependents();   // (steps of few tokens: not earlier, see gemm_skinny.cu)
+  }
   {
     const int hn = lane >> 2;
     const bool hv = hn < gvalid;
@@ -159,7 +186,6 @@ paged_decode_kernel(const DecodeParams p) {
       qb[ks][1] = hv ? *reinterpret_cast<const uint32_t*>(qrow + d0 + 8) : 0u;
     }
     if constexpr (FUSE) {
-      static_assert(!FUSE || D == 128, "fused q/k-norm + RoPE: head_dim 128");
       // this lane holds dims 16ks + 2(lane%4) + {0,1} (+8) of head lane/4: the 4 lanes of a quad hold the whole head,
       // and the RoPE partner d + 64 of every dim sits in the same lane at ks + 4
       float x[KS][4];
@@ -177,25 +203,18 @@ paged_decode_kernel(const DecodeParams p) {
         const float inv = 1.0f / sqrtf(ss / static_cast<float>(D) + p.eps);
 #pragma unroll
         for (int ks = 0; ks < KS; ++ks) {
-          const int d0 = ks * 16 + (lane & 3) * 2;
-          const uint32_t w0 = __ldg(reinterpret_cast<const uint32_t*>(p.qnw + d0));
-          const uint32_t w1 = __ldg(reinterpret_cast<const uint32_t*>(p.qnw + d0 + 8));
+          const uint32_t w0 = nw[ks][0], w1 = nw[ks][1];
           x[ks][0] = __bfloat162float(__float2bfloat16_rn(x[ks][0] * inv * bf16_lo(w0)));
           x[ks][1] = __bfloat162float(__float2bfloat16_rn(x[ks][1] * inv * bf16_hi(w0)));
           x[ks][2] = __bfloat162float(__float2bfloat16_rn(x[ks][2] * inv * bf16_lo(w1)));
           x[ks][3] = __bfloat162float(__float2bfloat16_rn(x[ks][3] * inv * bf16_hi(w1)));
         }
       }
-      int64_t pos = __ldg(p.pos + b);
-      pos = pos < 0 ? 0 : (pos >= p.max_position ? p.max_position - 1 : pos);
-      const float* cs = p.cos_sin + pos * D;
 #pragma unroll
       for (int ks = 0; ks < KS / 2; ++ks) {
-        const int d0 = ks * 16 + (lane & 3) * 2;   // < 64
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const int d = d0 + (e & 1) + (e >> 1) * 8;
-          const float c = __ldg(cs + d), sn = __ldg(cs + D / 2 + d);
+          const float c = rc[ks][e], sn = rs[ks][e];
           const float x1 = x[ks][e], x2 = x[ks + KS / 2][e];
           x[ks][e] = x1 * c - x2 * sn;
           x[ks + KS / 2][e] = x2 * c + x1 * sn;
@@ -424,16 +443,24 @@ paged_decode_kernel(const DecodeParams p) {
     const uint32_t mine = smem_u32(smem) + C::kMergeBytes;
     for (int idx = split * NWARPS * 32 + threadIdx.x; idx < gvalid * D; idx += p.num_splits * NWARPS * 32) {
       const int hn = idx / D;
-      float M = -INFINITY;
-      for (int s = 0; s < p.num_splits; ++s) M = fmaxf(M, ld_peer_f32(mine + (8 * D + 2 * hn) * 4, s));
+      float ms[kMaxClusterSplits], ls[kMaxClusterSplits], os[kMaxClusterSplits], M = -INFINITY;   // all requested at once
+#pragma unroll
+      for (int s = 0; s < kMaxClusterSplits; ++s)
+        if (s < p.num_splits) {
+          ms[s] = ld_peer_f32(mine + (8 * D + 2 * hn) * 4, s);
+          ls[s] = ld_peer_f32(mine + (8 * D + 2 * hn + 1) * 4, s);
+          os[s] = ld_peer_f32(mine + idx * 4, s);
+        }
+#pragma unroll
+      for (int s = 0; s < kMaxClusterSplits; ++s)
+        if (s < p.num_splits) M = fmaxf(M, ms[s]);
       float o = 0.f, L = 0.f;
-      if (M != -INFINITY)
-        for (int s = 0; s < p.num_splits; ++s) {
-          const float ms = ld_peer_f32(mine + (8 * D + 2 * hn) * 4, s);
-          if (ms == -INFINITY) continue;
-          const float f = fast_exp2(ms - M);
-          o += ld_peer_f32(mine + idx * 4, s) * f;
-          L += ld_peer_f32(mine + (8 * D + 2 * hn + 1) * 4, s) * f;
+#pragma unroll
+      for (int s = 0; s < kMaxClusterSplits; ++s)
+        if (s < p.num_splits && ms[s] != -INFINITY) {
+          const float f = fast_exp2(ms[s] - M);
+          o += os[s] * f;
+          L += ls[s] * f;
         }
       p.out[b * p.out_stride + static_cast<int64_t>(qh0) * D + idx] = __float2bfloat16_rn(L > 0.f ? o / L : 0.f);
     }
@@ -712,7 +739,6 @@ __global__ void __launch_bounds__(D) paged_decode_reduce_kernel(const DecodePara
 // ------------------------------------------------------------------------------------------------
 namespace nvllm {
 
-constexpr int kMaxClusterSplits = 16;
 
 // Whether clusters of `splits` CTAs merge inside the kernel: steps of few tokens (FUSE; in a chain of other kernels the second launch is
 // hidden), few splits, and clusters that all run at once.  A GPC holds whole clusters only, so that the grid may not fit although its
@@ -838,6 +864,7 @@ struct FuseArgs {  // non-NULL positions == fused entry point
   const int32_t* slot_mapping = nullptr;
   float eps = 0.f;
   int max_position = 0;
+  bool early = false;   // DecodeParams::early
 };
 
 static int decode_dispatch(void* out, const void* q, void* k_cache, void* v_cache, const int32_t* block_tables,
@@ -889,6 +916,7 @@ static int decode_dispatch(void* out, const void* q, void* k_cache, void* v_cach
   p.slots = fa.slot_mapping;
   p.eps = fa.eps;
   p.max_position = fa.max_position;
+  p.early = fa.early ? 1 : 0;
   p.tables = block_tables;
   p.ctx = context_lens;
   p.ws_o = nullptr;
@@ -966,6 +994,19 @@ extern "C" int nvllm_paged_decode_attention_fused(void* out, const void* qkv, co
                                 qkv_token_stride, out_token_stride, layout, scale, workspace, workspace_bytes, num_splits, dtype,
                                 stream, fa);
 }
+
+namespace nvllm {
+int paged_decode_fused_in_step(void* out, const void* qkv, const int64_t* positions, const float* cos_sin, const void* q_norm_w, const void* k_norm_w, float eps,
+                             int32_t max_position, void* k_cache, void* v_cache, const int32_t* slot_mapping, const int32_t* block_tables, const int32_t* context_lens,
+                             int32_t batch, int32_t num_heads, int32_t max_blocks_per_seq, int64_t qkv_token_stride, int64_t out_token_stride,
+                             const nvllm_kv_layout* layout, float scale, void* workspace, size_t workspace_bytes, int32_t num_splits, cudaStream_t st) {
+  FuseArgs fa;
+  fa.positions = positions; fa.cos_sin = cos_sin; fa.q_norm_w = q_norm_w; fa.k_norm_w = k_norm_w;
+  fa.slot_mapping = slot_mapping; fa.eps = eps; fa.max_position = max_position; fa.early = true;
+  return decode_dispatch(out, qkv, k_cache, v_cache, block_tables, context_lens, batch, num_heads, max_blocks_per_seq, qkv_token_stride, out_token_stride,
+                         layout, scale, workspace, workspace_bytes, num_splits, NVLLM_BF16, st, fa);
+}
+}  // namespace nvllm
 
 // ------------------------------------------------------------------------------------------------
 // Split-K decode attention for callers that cannot hand us a workspace.
