@@ -14,6 +14,7 @@
 //                              K = 1024: 13.4 K x 6144 x 1024 215 us, with eight 157 (K = 4096: no difference).  A plain epilogue only
 //                              stores, and eight warps storing at once are slower than four: 32768 x 6144 x 1024 f32 512 us with four,
 //                              560 with eight; 13.4 K x 4096 x 1024 bf16 94 and 99.
+#include <algorithm>
 #include "tc.cuh"
 
 namespace nvllm {
@@ -170,7 +171,7 @@ template <int BN, typename OutT, int GATE, bool ROPE, bool GROUPED>
 __global__ void __launch_bounds__(gemm2_threads<GATE, ROPE>(), 1)
 gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                          OutT* __restrict__ y, int M, int N, int K, int64_t ldy, int num_m_tiles, int num_tiles, float glu_limit,
-                         const RopeEpi re, const int32_t* __restrict__ tile_group, int group_rows, bool relu2) {
+                         const RopeEpi re, const int32_t* __restrict__ tile_group, int group_rows, bool relu2, int panel) {
   using C = Gemm2Cfg<BN>;
   constexpr int STAGES = C::kStages - (ROPE ? 1 : 0);   // (the qkv epilogue takes a stage's room)
   extern __shared__ uint8_t smem_raw[];
@@ -248,7 +249,8 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
       const int row0 = static_cast<int>(p & 0xfffu) * C::BM_CTA;
       return Where{row0 + static_cast<int>(rank) * C::BM_CTA, tile % num_m_tiles, row0 + (p & 0x1000u ? C::BM : C::BM_CTA), static_cast<int>(p >> 13) * group_rows};
     } else {
-      return Where{tile % num_m_tiles * C::BM + static_cast<int>(rank) * C::BM_CTA, tile / num_m_tiles, M, 0};
+      const int p = tile / (panel * num_m_tiles), n0 = p * panel, in = tile - n0 * num_m_tiles, wide = min(panel, num_tiles / num_m_tiles - n0);
+      return Where{in / wide * C::BM + static_cast<int>(rank) * C::BM_CTA, n0 + in % wide, M, 0};
     }
   };
 
@@ -363,6 +365,14 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
   }
 }
 
+// The order of the tiles: panels of this many n-tiles, n fastest within a panel.  Up to K = 2048 one n-tile after the other (a w tile is read
+// once, x stays in L2): 8192 x 8192 x 2048 (gated) 401 us, 407 in panels of 12.  Longer rows of x leave L2 again before the next n-tile reads
+// them; in panels of 12 a wave of 74 tiles reads 12 tiles of w and 6 of x.  Measured (us, one n-tile after the other -> in panels of 12):
+// 8192 x 4096 x 12288 684 -> 629, 8192 x 24576 x 4096 1322 -> 1224, 8192 x 6144 x 4096 340 -> 314, 8192 x 2048 x 8192 247 -> 223, 12400 x 1024 x 3072
+// 73 -> 68.  Where a few m-tiles are no more than a wave anyway, panels of 2 do best: 3000 x 24576 x 4096 497 -> 461 (12: 470),
+// 1500 x 24576 x 4096 (gated) 247 -> 230 (237), 1500 x 4096 x 12288 161 -> 160 (161).
+static int panel_tiles(int num_m_tiles, int k) { return k < 3072 ? 1 : (num_m_tiles >= 16 ? 12 : 2); }
+
 constexpr int kMaxGroupedTiles = 4096;   // (the list's entries hold 12 bits of tile and 19 of group)
 
 template <int BN, typename OutT, int GATE = kGateNone, bool ROPE = false, bool GROUPED = false>
@@ -392,7 +402,7 @@ static int launch_gemm2(const CUtensorMap& tx, const CUtensorMap& tw, void* y, i
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
   NVLLM_CUDA(cudaLaunchKernelEx(&cfg, kern, tx, tw, static_cast<OutT*>(y), M, N, K, ldy, num_m_tiles, GROUPED ? num_n_tiles : num_tiles, glu_limit, re, tile_group,
-                                group_rows, relu2));
+                                group_rows, relu2, std::min(num_n_tiles, panel_tiles(num_m_tiles, K))));
   return 0;
 }
 
