@@ -62,6 +62,13 @@ int paged_decode_fused_in_step(void* out, const void* qkv, const int64_t* positi
                                int64_t out_token_stride, const nvllm_kv_layout* layout, float scale, void* workspace, size_t workspace_bytes,
                                int32_t num_splits, cudaStream_t st);
 
+// y = bf16(y + bf16(x . w^T)) in place, on CTA pairs (gemm_tcgen05_2cta.cu): the residual add of a prompt's projections rides in their epilogue,
+// where it hides behind the next tile's products, and the norm that follows moves half as much (12.4 K x 1024 16.8 -> 10.5 us beside 0.5 to 1
+// more in the product).  Prefill of Qwen3-0.6B, ragged prompts 14500 -> 14270 us, of Qwen3-8B (9 layers, 8192 tokens) 25000 -> 24770.
+// Rows of 16-byte pieces as nvllm_gemm_bf16 wants them.
+bool gemm_add_applies(int m, int n, int k);
+int gemm_add(void* y, const void* x, const void* w, int m, int n, int k, int64_t ldx, int64_t ldw, int64_t ldy, cudaStream_t st);
+
 // Projections of up to 16 tokens (gemm_skinny.cu): y = x . w^T as nvllm_gemm_bf16 / nvllm_gemm_silu_mul_bf16; norm_w: x is normed
 // first (bf16 weights, k columns); residual: y += the bf16 product, in place.
 bool gemm_skinny_applies(int m, int n, int k, int64_t ldx, int64_t ldw, bool f32_out, bool gate);

@@ -9,9 +9,9 @@
 //   leader,    warp 1 lane 0   MMA issuer; tcgen05.commit ... multicast releases the smem stage / publishes the tile in BOTH CTAs
 //   both CTAs, warp 2          TMEM allocator (cta_group::2)
 //   both CTAs, warps 4-7       epilogue on the CTA's own 128 TMEM lanes; drained-signal goes to the leader (remote mbarrier arrive).
-//                              Gated outputs have warps 8-11 besides, on the upper half of the columns: with four warps their epilogue
-//                              (an exponential and a division per output, one warp per scheduler) outlasted a tile's 16 k-blocks at
-//                              K = 1024: 13.4 K x 6144 x 1024 215 us, with eight 157 (K = 4096: no difference).  A plain epilogue only
+//                              Gated outputs and those that are added to y have warps 8-11 besides, on the upper half of the columns: with
+//                              four warps their epilogue outlasts a tile's k-blocks (added, 12.4 K x 1024 x 2048 and 3072 in a prefill 63 us
+//                              in the mean, with eight 54).  A plain epilogue only
 //                              stores, and eight warps storing at once are slower than four: 32768 x 6144 x 1024 f32 512 us with four,
 //                              560 with eight; 13.4 K x 4096 x 1024 bf16 94 and 99.
 #include <algorithm>
@@ -19,10 +19,10 @@
 
 namespace nvllm {
 
-template <int GATE, bool ROPE = false>
-constexpr int gemm2_epilogue_warps() { return GATE != kGateNone || ROPE ? 8 : 4; }
-template <int GATE, bool ROPE = false>
-constexpr int gemm2_threads() { return 128 + 32 * gemm2_epilogue_warps<GATE, ROPE>(); }
+template <int GATE, bool ROPE = false, bool ADD = false>
+constexpr int gemm2_epilogue_warps() { return GATE != kGateNone || ROPE || ADD ? 8 : 4; }
+template <int GATE, bool ROPE = false, bool ADD = false>
+constexpr int gemm2_threads() { return 128 + 32 * gemm2_epilogue_warps<GATE, ROPE, ADD>(); }
 
 constexpr int kRopeStage = 2 * 16 * 256;   // bytes of shared memory of an epilogue warp of the qkv form
 
@@ -167,8 +167,8 @@ __device__ __forceinline__ void rope_rows(bf16* __restrict__ y, int64_t ldy, con
 // comes from HBM once, where the other order reads it again for every n-tile (8192 tokens x 6 of 64 experts, 2048 -> 1408: single CTAs 356 us
 // with m-tiles fastest, 297 with n-tiles, pairs 259; 1408 -> 2048: 341, 286, 245).  Bound by the L2 -> SM feed like the plain product, and by
 // the rows that fill up tiles and pairs.
-template <int BN, typename OutT, int GATE, bool ROPE, bool GROUPED>
-__global__ void __launch_bounds__(gemm2_threads<GATE, ROPE>(), 1)
+template <int BN, typename OutT, int GATE, bool ROPE, bool GROUPED, bool ADD>
+__global__ void __launch_bounds__(gemm2_threads<GATE, ROPE, ADD>(), 1)
 gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                          OutT* __restrict__ y, int M, int N, int K, int64_t ldy, int num_m_tiles, int num_tiles, float glu_limit,
                          const RopeEpi re, const int32_t* __restrict__ tile_group, int group_rows, bool relu2, int panel) {
@@ -203,7 +203,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tfull_bar(a), 1);     // each CTA: multicast commit
-      mbar_init(tempty_bar(a), 64 * gemm2_epilogue_warps<GATE, ROPE>());  // leader: the epilogue threads of both CTAs
+      mbar_init(tempty_bar(a), 64 * gemm2_epilogue_warps<GATE, ROPE, ADD>());  // leader: the epilogue threads of both CTAs
     }
     fence_barrier_init();
   }
@@ -339,13 +339,37 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
           if (row < at.m_end && col0 < N) store_row32_2<OutT>(y + row * ldy + col0, g, col0, N);
         }
       } else {
+        // add: y holds the residual stream, and the product's bf16 values are added to it in place.  A chunk's old values are requested
+        // while the chunk before it is on its way.
+        [[maybe_unused]] uint4 old[4];
+        auto request = [&](int c) {
+          const int col0 = n_tile * BN + c * 32;
+          const bf16* src = reinterpret_cast<const bf16*>(y) + row * ldy + col0;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) old[j] = row < at.m_end && col0 + j * 8 < N ? *reinterpret_cast<const uint4*>(src + j * 8) : make_uint4(0, 0, 0, 0);
+        };
+        const int c0 = ADD && warp >= 8 ? BN / 64 : 0, c1 = ADD && warp < 8 ? BN / 64 : BN / 32;
+        if constexpr (ADD) request(c0);
 #pragma unroll 1
-        for (int c = 0; c < BN / 32; ++c) {
+        for (int c = c0; c < c1; ++c) {
           uint32_t r[32];
           tmem_ld_32x32b_x32(taddr + c * 32, r);
           tmem_ld_wait();
           if constexpr (GROUPED) {
             if (relu2) relu2_row32(r);
+          }
+          if constexpr (ADD) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const uint32_t o[4] = {old[j].x, old[j].y, old[j].z, old[j].w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const uint32_t b = pack_bf16x2(__uint_as_float(r[8 * j + 2 * e]), __uint_as_float(r[8 * j + 2 * e + 1]));
+                r[8 * j + 2 * e] = __float_as_uint(bf16_lo(b) + bf16_lo(o[e]));
+                r[8 * j + 2 * e + 1] = __float_as_uint(bf16_hi(b) + bf16_hi(o[e]));
+              }
+            }
+            if (c + 1 < c1) request(c + 1);
           }
           const int col0 = n_tile * BN + c * 32;
           if (row < at.m_end && col0 < N) store_row32_2<OutT>(y + row * ldy + col0, r, col0, N);
@@ -375,11 +399,11 @@ static int panel_tiles(int num_m_tiles, int k) { return k < 3072 ? 1 : (num_m_ti
 
 constexpr int kMaxGroupedTiles = 4096;   // (the list's entries hold 12 bits of tile and 19 of group)
 
-template <int BN, typename OutT, int GATE = kGateNone, bool ROPE = false, bool GROUPED = false>
+template <int BN, typename OutT, int GATE = kGateNone, bool ROPE = false, bool GROUPED = false, bool ADD = false>
 static int launch_gemm2(const CUtensorMap& tx, const CUtensorMap& tw, void* y, int M, int N, int K, int64_t ldy,
                         cudaStream_t st, float glu_limit = 0.f, const RopeEpi& re = RopeEpi{}, const int32_t* tile_group = nullptr, int group_rows = 0, bool relu2 = false) {
   using C = Gemm2Cfg<BN>;
-  auto kern = gemm_tcgen05_2cta_kernel<BN, OutT, GATE, ROPE, GROUPED>;
+  auto kern = gemm_tcgen05_2cta_kernel<BN, OutT, GATE, ROPE, GROUPED, ADD>;
   constexpr int smem_max = C::kSmemBytes + (ROPE ? 8 * kRopeStage - C::kStageBytes : 0) + (GROUPED ? 4 * kMaxGroupedTiles : 0);
   static_assert(smem_max <= 227 * 1024, "");
   NVLLM_SMEM_ATTR_ONCE(kern, smem_max);
@@ -391,7 +415,7 @@ static int launch_gemm2(const CUtensorMap& tx, const CUtensorMap& tw, void* y, i
   const int clusters = num_tiles < max_clusters ? num_tiles : max_clusters;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(2 * clusters);
-  cfg.blockDim = dim3(gemm2_threads<GATE, ROPE>());
+  cfg.blockDim = dim3(gemm2_threads<GATE, ROPE, ADD>());
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
@@ -428,7 +452,7 @@ static int pick_bn_2cta(int M, int N) {
 }
 
 int gemm_2cta_dispatch(void* y, const void* x, const void* w, int m, int n, int k, int64_t ldx, int64_t ldw,
-                       int64_t ldy, int out_dtype, cudaStream_t st) {
+                       int64_t ldy, int out_dtype, cudaStream_t st, bool add) {
   const int forced = knobs().gemm_bn;
   const int bn = (forced == 64 || forced == 128 || forced == 256) ? forced : pick_bn_2cta(m, n);
   CUtensorMap tx, tw;
@@ -436,6 +460,7 @@ int gemm_2cta_dispatch(void* y, const void* x, const void* w, int m, int n, int 
   if (int rc = make_tmap_bf16_2d(&tw, w, n, k, ldw, bn / 2)) return rc;
 #define NVLLM_G2(BNV)                                                                            \
   case BNV:                                                                                      \
+    if (add) return launch_gemm2<BNV, bf16, kGateNone, false, false, true>(tx, tw, y, m, n, k, ldy, st); \
     return out_dtype == NVLLM_BF16 ? launch_gemm2<BNV, bf16>(tx, tw, y, m, n, k, ldy, st)        \
                                    : launch_gemm2<BNV, float>(tx, tw, y, m, n, k, ldy, st)
   switch (bn) {

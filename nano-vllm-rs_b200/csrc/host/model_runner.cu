@@ -680,6 +680,22 @@ int nvllm_runner::forward(int N, int S, bool is_prefill, bool paged_prefill, con
     mark("add_rmsnorm");
     return rc;
   };
+  // prompts on one GPU: o_proj / down_proj add to the stream h themselves, the norm behind them only reads it
+  const bool adds = tp == 1 && gemm_add_applies(N, hidden, HD) && gemm_add_applies(N, hidden, inter);
+  auto close_block = [&](const void* x, const void* w, int k, const bf16* norm, const char* what) -> int {
+    if (!adds) {
+      RUN(row_gemm(x, w, k, what));
+      return norm != nullptr ? add_norm(norm) : 0;
+    }
+    ++launches;
+    RUN(gemm_add(h, x, w, N, hidden, k, k, k, hidden, stream));
+    mark(what);
+    if (norm == nullptr) return 0;
+    ++launches;
+    RUN(nvllm_add_rmsnorm(normed, h, nullptr, norm, N, hidden, eps, NVLLM_BF16, st));
+    mark("rmsnorm");
+    return 0;
+  };
   const bool few = few_tokens(N, S);   // no norm and no residual add of its own
   auto few_gemm = [&](void* y, const void* x, const void* w, int rows_n, int n, int k, int64_t ldy, int out_dt, bool gate, const bf16* norm, bool residual, const char* what) {
     ++launches;
@@ -692,11 +708,8 @@ int nvllm_runner::forward(int N, int S, bool is_prefill, bool paged_prefill, con
   if (!is_prefill) last_decode_splits = splits;
   for (int l = 0; l < layers; ++l) {
     const LayerWeights& w = lw[l];
-    // input_layernorm; for l > 0 fused with the residual add of the previous MLP output (qwen3.rs:389 -> :378)
-    // (and, under TP, with the all-reduce of that output: see add_norm below)
-    if (few) {}
-    else if (l == 0) { RUN(nvllm_add_rmsnorm(normed, h, nullptr, w.input_ln, N, hidden, eps, NVLLM_BF16, st)); ++launches; mark("add_rmsnorm"); }
-    else RUN(add_norm(w.input_ln));
+    // input_layernorm; for l > 0 it follows the residual add of the previous MLP output (qwen3.rs:389 -> :378), see close_block
+    if (!few && l == 0) { RUN(nvllm_add_rmsnorm(normed, h, nullptr, w.input_ln, N, hidden, eps, NVLLM_BF16, st)); ++launches; mark("add_rmsnorm"); }
     const bf16* qnw = cfg.qk_norm ? w.q_norm : nullptr;
     const bf16* knw = cfg.qk_norm ? w.k_norm : nullptr;
     bool roped = false;  // q/k-norm + RoPE + KV store already applied to the qkv buffer / cache
@@ -745,16 +758,15 @@ int nvllm_runner::forward(int N, int S, bool is_prefill, bool paged_prefill, con
       RUN(few_gemm(h, act, w.down, N, hidden, inter, hidden, NVLLM_BF16, false, nullptr, true, "down_proj + residual"));
       continue;
     }
-    RUN(row_gemm(attn, w.o, HD, "o_proj GEMM"));
-    RUN(add_norm(w.post_ln));                                                                                          // qwen3.rs:382-385
+    RUN(close_block(attn, w.o, HD, w.post_ln, "o_proj GEMM"));   // qwen3.rs:382-385
     // gate_up GEMM with the SiLU*mul in its epilogue (MergedColumnParallelLinear + SiluAndMul, qwen3.rs:307-310)
     RUN(nvllm_gemm_silu_mul_bf16(act, normed, w.gate_up, N, inter, hidden, hidden, hidden, inter, gate_up,
                                  static_cast<size_t>(max_tokens) * 2 * inter * 2, st));
     launches += (inter % 128 == 0) ? 1 : 2;
     mark("gate_up_proj GEMM + SiLU*mul");
-    RUN(row_gemm(act, w.down, inter, "down_proj GEMM"));
+    // with the norm of the next layer, or the final one
+    RUN(close_block(act, w.down, inter, l + 1 < layers ? lw[l + 1].input_ln : final_norm, "down_proj GEMM"));   // qwen3.rs:389,501
   }
-  if (!few) RUN(add_norm(final_norm));                                                                                           // qwen3.rs:389,501
   const bf16* last_rows = few ? h : normed;   // few: the final norm rides in the head's projection
   const bf16* head_in = last_rows;
   int rows = N;
