@@ -12,8 +12,10 @@
 // Roles: warps 0-3 own a row each thread (softmax, P back into the S columns, output), warps 4-7 copy key tiles (cp.async in 16-byte
 // steps through the block table, zeros past the sequence's keys), warp 8 issues the MMAs (converged, one elected lane).  S of the next
 // tile runs while a tile's softmax does.
-// Measured, 8 x 1024 tokens x 16 heads: 387 us (mma.sync kernel: 1526; with a diverged issuing lane 470).  An N64 step of S costs what an N128 one
-// does; what the MMAs leave of a tile's time is S waiting for its copies.
+// Measured, 8 x 1024 tokens x 16 heads, back to back: 380 us (411 before the queries were asked into L2 first and the output left in 32-byte
+// pieces; mma.sync kernel: 1526).  An N64 step of S costs what an N128 one does.  The copies bind: 74 KB a tile and half come in at 47 GB/s an
+// SM (7 TB/s from L2 over all), 1.6 of the 1.8 us of a tile.  CTAs that stay (clusterlaunchcontrol) with TMA copies, the chunks that only S
+// reads released early and a warp each for S and P . C took 394 us here, 6 to 10 % more than these for long portions.
 #include "latent_attn.cuh"
 #include "tc.cuh"
 
@@ -33,23 +35,40 @@ constexpr int kColO = 0, kColQ = kHalf, kColS = kColQ + kQTmem / 2;   // TMEM co
 
 struct Span { int seq, t0, t1, jstart, nkeys; };   // tokens [t0, t1) of one sequence; keys [jstart, nkeys), jstart a multiple of 64
 
-// The tile's one or two runs of tokens (every thread computes the same).
-__device__ __forceinline__ Span span_of(const LatentAttnArgs& a, int t0, int tend) {
+// What a CTA asks about its tile's tokens, requested at once (8 x 1024 tokens 383 -> 380 us).
+struct Tokens { int seq[kLatentTileTokens], nkeys[kLatentTileTokens]; };
+__device__ __forceinline__ Tokens tokens_of(const LatentAttnArgs& a, int tile0, int tend) {
+  Tokens t;
+#pragma unroll
+  for (int i = 0; i < kLatentTileTokens; ++i) t.seq[i] = tile0 + i < tend ? a.tok_seq[tile0 + i] : -1;
+#pragma unroll
+  for (int i = 0; i < kLatentTileTokens; ++i) t.nkeys[i] = tile0 + i < tend ? static_cast<int>(a.positions[tile0 + i]) + 1 : 0;
+  return t;
+}
+
+// The tile's one or two runs of tokens, from token t0 on (a whole warp; every lane computes the same).
+__device__ __forceinline__ Span span_of(const LatentAttnArgs& a, const Tokens& tok, int tile0, int t0, int tend) {
   Span s;
-  s.t0 = t0;
-  s.seq = a.tok_seq[t0];
-  int t1 = t0 + 1;
-  while (t1 < tend && a.tok_seq[t1] == s.seq) ++t1;
-  s.t1 = t1;
+  s.t0 = s.t1 = t0;
+  s.seq = -1;
   int nkeys = 0, first = 1 << 30;
-  for (int t = t0; t < t1; ++t) {
-    const int nk = static_cast<int>(a.positions[t]) + 1;
-    nkeys = max(nkeys, nk);
-    first = min(first, a.window > 0 && nk > a.window ? nk - a.window : 0);
+#pragma unroll
+  for (int i = 0; i < kLatentTileTokens; ++i) {
+    const int t = tile0 + i;
+    if (t == t0) s.seq = tok.seq[i];
+    if (t == s.t1 && t < tend && tok.seq[i] == s.seq) {
+      const int nk = tok.nkeys[i];
+      nkeys = max(nkeys, nk);
+      first = min(first, a.window > 0 && nk > a.window ? nk - a.window : 0);
+      s.t1 = t + 1;
+    }
   }
   const int32_t* table = a.tables + static_cast<int64_t>(s.seq) * a.table_cap;
-  for (int b = 0; b * a.block_size < nkeys; ++b)   // a missing block ends the sequence's keys
-    if (table[b] < 0) { nkeys = b * a.block_size; break; }
+  const int lane = threadIdx.x & 31, blocks = (nkeys + a.block_size - 1) / a.block_size;
+  for (int b = 0; b < blocks; b += 32) {   // a missing block ends the sequence's keys
+    const unsigned miss = __ballot_sync(0xffffffffu, b + lane < blocks && table[b + lane] < 0);
+    if (miss != 0) { nkeys = (b + __ffs(miss) - 1) * a.block_size; break; }
+  }
   s.nkeys = nkeys;
   s.jstart = min(first, nkeys) & ~(kKeys - 1);
   return s;
@@ -115,11 +134,34 @@ __device__ __noinline__ void row_alone(const LatentAttnArgs& a, int tok, int hea
   *reinterpret_cast<uint4*>(static_cast<bf16*>(a.out) + static_cast<int64_t>(tok) * a.ldo + static_cast<int64_t>(head) * kRank + half * kHalf + 8 * lane) = w;
 }
 
-__global__ void __launch_bounds__(kThreads, 1) latent_attn_tc_kernel(const __grid_constant__ LatentAttnArgs a, int halves) {
+__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(p), "r"(bytes) : "memory");
+}
+// 32 bytes at once: a whole sector of the one row that a lane writes
+__device__ __forceinline__ void st_32(void* p, const uint32_t (&v)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]),
+               "r"(v[7])
+               : "memory");
+}
+
+// wide: rows of the output lie on 32 bytes
+__global__ void __launch_bounds__(kThreads, 1) latent_attn_tc_kernel(const __grid_constant__ LatentAttnArgs a, int halves, bool wide) {
   pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   const int tile = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);   // late tokens of the batch (most keys) first
-  if (!latent_tile_dense(a.tok_seq, a.n, tile)) return;
+  // all of the queries set out for L2 while the CTA finds its way (8 tokens x 32 KB; they are read a quarter at a time)
+  if (threadIdx.x < kLatentTileTokens && tile * kLatentTileTokens + static_cast<int>(threadIdx.x) < a.n)
+    prefetch_l2(a.q_abs + static_cast<int64_t>(tile * kLatentTileTokens + threadIdx.x) * a.ldqa + static_cast<int64_t>(blockIdx.y) * kHeads * kRank, kHeads * kRank * 4);
+  const int tile0 = tile * kLatentTileTokens, tend = min(a.n, tile0 + kLatentTileTokens);
+  const Tokens tok = tokens_of(a, tile0, tend);
+  if (tend - tile0 < kLatentTileTokens) {
+    if (!latent_tile_dense(a.tok_seq, a.n, tile)) return;
+  } else {   // (the same)
+    int runs = 1;
+#pragma unroll
+    for (int i = 1; i < kLatentTileTokens; ++i) runs += tok.seq[i] != tok.seq[i - 1];
+    if (runs > 2) return;
+  }
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
   const uint32_t sQ = base, sK = base + kSmemK, bars = base + kSmemBar;
@@ -130,7 +172,6 @@ __global__ void __launch_bounds__(kThreads, 1) latent_attn_tc_kernel(const __gri
   const uint32_t o_done = bars + 8 * 8;
   const uint32_t tmem_slot = bars + 9 * 8;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;   // (warp: uniform)
-  const int tile0 = tile * kLatentTileTokens, tend = min(a.n, tile0 + kLatentTileTokens);
   const int hbase = blockIdx.y * kHeads;
   const int half0 = halves == 2 ? 0 : static_cast<int>(blockIdx.z);   // this CTA's halves of the latent values: half0 .. half0 + halves - 1
 
@@ -215,7 +256,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_attn_tc_kernel(const __gri
     const bf16* cache = static_cast<const bf16*>(a.cache);
     int it = 0;
     for (int t = tile0; t < tend;) {
-      const Span s = span_of(a, t, tend);
+      const Span s = span_of(a, tok, tile0, t, tend);
       const int32_t* table = a.tables + static_cast<int64_t>(s.seq) * a.table_cap;
       for (int h = 0; h < halves; ++h)
         for (int j0 = s.jstart; j0 < s.nkeys; j0 += kKeys, ++it) {
@@ -279,7 +320,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_attn_tc_kernel(const __gri
       // The key tiles of the two spans (the second may be empty), each walked once per half of the values.
       int tiles[2] = {0, 0}, ns = 0;
       for (int t = tile0; t < tend; ++ns) {
-        const Span s = span_of(a, t, tend);
+        const Span s = span_of(a, tok, tile0, t, tend);
         tiles[ns] = static_cast<int>(uni((s.nkeys - s.jstart + kKeys - 1) / kKeys));
         t = static_cast<int>(uni(s.t1));
       }
@@ -309,7 +350,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_attn_tc_kernel(const __gri
     int it = 0, again_lo = 0, again_hi = 0;
     bool again = false;
     for (int t = tile0; t < tend;) {
-      const Span s = span_of(a, t, tend);
+      const Span s = span_of(a, tok, tile0, t, tend);
       const bool mine = my_tok >= s.t0 && my_tok < s.t1;
       const int pos = mine ? static_cast<int>(a.positions[my_tok]) : -1;
       const int hi = min(pos + 1, s.nkeys), lo = a.window > 0 && pos + 1 > a.window ? pos + 1 - a.window : 0;   // the row sees the keys [lo, hi)
@@ -394,13 +435,16 @@ __global__ void __launch_bounds__(kThreads, 1) latent_attn_tc_kernel(const __gri
           }
           if (mine) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              uint4 v;
-              v.x = pack_bf16x2(__uint_as_float(o[8 * e]) * inv, __uint_as_float(o[8 * e + 1]) * inv);
-              v.y = pack_bf16x2(__uint_as_float(o[8 * e + 2]) * inv, __uint_as_float(o[8 * e + 3]) * inv);
-              v.z = pack_bf16x2(__uint_as_float(o[8 * e + 4]) * inv, __uint_as_float(o[8 * e + 5]) * inv);
-              v.w = pack_bf16x2(__uint_as_float(o[8 * e + 6]) * inv, __uint_as_float(o[8 * e + 7]) * inv);
-              *reinterpret_cast<uint4*>(out + c * 32 + e * 8) = v;
+            for (int e = 0; e < 2; ++e) {
+              uint32_t v[8];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) v[i] = pack_bf16x2(__uint_as_float(o[16 * e + 2 * i]) * inv, __uint_as_float(o[16 * e + 2 * i + 1]) * inv);
+              if (wide) {
+                st_32(out + c * 32 + e * 16, v);
+              } else {
+                *reinterpret_cast<uint4*>(out + c * 32 + e * 16) = make_uint4(v[0], v[1], v[2], v[3]);
+                *reinterpret_cast<uint4*>(out + c * 32 + e * 16 + 8) = make_uint4(v[4], v[5], v[6], v[7]);
+              }
             }
           }
         }
@@ -441,7 +485,8 @@ int latent_attn_tc_launch(const LatentAttnArgs& a, cudaStream_t st) {
   // One CTA per (tile, head group) walks both halves of the latent values on one copy of the queries; where that leaves SMs without
   // a CTA the halves are CTAs of their own.
   const bool split = static_cast<int64_t>(tiles) * groups * 2 <= sm_count();
-  NVLLM_CUDA(launch_pdl(latent_attn_tc_kernel, dim3(tiles, groups, split ? 2 : 1), dim3(kThreads), kSmemBytes, st, a, split ? 1 : 2));
+  NVLLM_CUDA(launch_pdl(latent_attn_tc_kernel, dim3(tiles, groups, split ? 2 : 1), dim3(kThreads), kSmemBytes, st, a, split ? 1 : 2,
+                        a.ldo % 16 == 0 && (reinterpret_cast<uintptr_t>(a.out) & 31u) == 0));
   NVLLM_LAUNCH_CHECK("latent_attn_tc_kernel");
   return 0;
 }
