@@ -266,6 +266,17 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   bf162 v = __floats2bfloat162_rn(lo, hi);  // .x = lo (low 16 bits)
   return *reinterpret_cast<uint32_t*>(&v);
 }
+// 32 bytes at once, a whole sector, where each lane writes along a row of its own: two 16-byte stores to a sector leave the SM as two partial
+// writes of it, and the stores of an epilogue then bind the kernel (figures at store_row32).  rows_on_32: all rows start on 32 bytes.
+template <typename T>
+__host__ __device__ __forceinline__ bool rows_on_32(const T* p, int64_t ld) {
+  return ((reinterpret_cast<uintptr_t>(p) | static_cast<uint64_t>(ld) * sizeof(T)) & 31) == 0;
+}
+__device__ __forceinline__ void st_global_32(void* p, const uint32_t (&v)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]),
+               "r"(v[7])
+               : "memory");
+}
 // The clamped gate of a feed-forward: g' sigmoid(1.702 g') (u' + 1) with g' = min(g, limit), u' = u clamped to [-limit, limit].
 __device__ __forceinline__ float bf16_lo(uint32_t v);
 __device__ __forceinline__ float bf16_hi(uint32_t v);

@@ -10,7 +10,7 @@
 //                      accumulators in TMEM (2 x BN columns, double buffered); tcgen05.commit releases
 //                      the smem stage (`empty`) and, after the last k-block, publishes the tile (`tmem_full`)
 //   warp 2             TMEM allocator
-//   warps 4-7          epilogue: tcgen05.ld (32 lanes x 32 columns per warp) -> bf16/fp32 -> 16-byte global
+//   warps 4-7          epilogue: tcgen05.ld (32 lanes x 32 columns per warp) -> bf16/fp32 -> 32-byte global
 //                      stores, overlapped with the next tile's MMAs through the second TMEM buffer
 // Both operands are K-major (row-major x and row-major w), the canonical TN case: no transposes anywhere.
 // Tiles are enumerated m-fastest so CTAs running together share the same w tile in L2; w is read from
@@ -32,24 +32,7 @@ struct GemmCfg {
   static constexpr int kSmemBytes = kStages * kStageBytes + kBarBytes + 1024;  // + alignment slack
 };
 
-template <typename OutT>
-__device__ __forceinline__ void store_row32(OutT* dst, const uint32_t (&r)[32], int col0, int n);
-
-template <>
-__device__ __forceinline__ void store_row32<bf16>(bf16* dst, const uint32_t (&r)[32], int col0, int n) {
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    if (col0 + j * 8 < n) {
-      uint4 v;
-      v.x = pack_bf16x2(__uint_as_float(r[8 * j + 0]), __uint_as_float(r[8 * j + 1]));
-      v.y = pack_bf16x2(__uint_as_float(r[8 * j + 2]), __uint_as_float(r[8 * j + 3]));
-      v.z = pack_bf16x2(__uint_as_float(r[8 * j + 4]), __uint_as_float(r[8 * j + 5]));
-      v.w = pack_bf16x2(__uint_as_float(r[8 * j + 6]), __uint_as_float(r[8 * j + 7]));
-      *reinterpret_cast<uint4*>(dst + j * 8) = v;
-    }
-  }
-}
-// The same 32 columns into a peer's low-latency stage buffer (RowPush): scrubbed, system-scope stores.
+// store_row32 into a peer's low-latency stage buffer (RowPush): scrubbed, system-scope stores.
 __device__ __forceinline__ void push_row32(bf16* dst, const uint32_t (&r)[32], int col0, int n) {
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -60,15 +43,6 @@ __device__ __forceinline__ void push_row32(bf16* dst, const uint32_t (&r)[32], i
       v.z = pack_bf16x2(__uint_as_float(r[8 * j + 4]), __uint_as_float(r[8 * j + 5]));
       v.w = pack_bf16x2(__uint_as_float(r[8 * j + 6]), __uint_as_float(r[8 * j + 7]));
       st_sys_16(dst + j * 8, ll_scrub(v));
-    }
-  }
-}
-template <>
-__device__ __forceinline__ void store_row32<float>(float* dst, const uint32_t (&r)[32], int col0, int n) {
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    if (col0 + j * 4 < n) {
-      *reinterpret_cast<uint4*>(dst + j * 4) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
     }
   }
 }
@@ -202,6 +176,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     }
   } else if (warp >= 4) {
     // ===== epilogue: TMEM -> registers -> global =====
+    [[maybe_unused]] const bool wide = rows_on_32(y, ldy);
     pdl_wait();              // y may still be read by an earlier kernel until the predecessor has completed
     const int q = warp & 3;  // TMEM lane quadrant this warp may access
     int acc = 0;
@@ -295,7 +270,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             g[e + 1] = __float_as_uint(p.y);
           }
           const int col0 = n_tile * (BN / 2) + c * 32;
-          if (row < M && col0 < N) store_row32<OutT>(y + row * ldy + col0, g, col0, N);
+          if (row < M && col0 < N) store_row32<OutT>(y + row * ldy + col0, g, col0, N, wide);
         }
       } else {
         bf16* remote = nullptr;  // TP: this row is reduced by another rank -> straight into its stage buffer
@@ -313,7 +288,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
           const int col0 = n_tile * BN + c * 32;
           if (row < M && col0 < N) {
             if (remote != nullptr) push_row32(remote + col0, r, col0, N);
-            else store_row32<OutT>(y + row * ldy + col0, r, col0, N);
+            else store_row32<OutT>(y + row * ldy + col0, r, col0, N, wide);
           }
         }
       }

@@ -12,8 +12,7 @@
 //                              Gated outputs and those that are added to y have warps 8-11 besides, on the upper half of the columns: with
 //                              four warps their epilogue outlasts a tile's k-blocks (added, 12.4 K x 1024 x 2048 and 3072 in a prefill 63 us
 //                              in the mean, with eight 54).  A plain epilogue only
-//                              stores, and eight warps storing at once are slower than four: 32768 x 6144 x 1024 f32 512 us with four,
-//                              560 with eight; 13.4 K x 4096 x 1024 bf16 94 and 99.
+//                              stores; eight warps are no faster at it (8192 x 10304 x 2048 f32 256 us with either).
 #include <algorithm>
 #include "tc.cuh"
 
@@ -37,27 +36,6 @@ struct Gemm2Cfg {
   static constexpr int kTmemCols = (2 * BN <= 64) ? 64 : (2 * BN <= 128) ? 128 : (2 * BN <= 256) ? 256 : 512;
   static constexpr int kSmemBytes = kStages * kStageBytes + (2 * kStages + 4) * 8 + 16 + 1024;
 };
-
-template <typename OutT>
-__device__ __forceinline__ void store_row32_2(OutT* dst, const uint32_t (&r)[32], int col0, int n) {
-  if constexpr (sizeof(OutT) == 2) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (col0 + j * 8 < n) {
-        uint4 v;
-        v.x = pack_bf16x2(__uint_as_float(r[8 * j + 0]), __uint_as_float(r[8 * j + 1]));
-        v.y = pack_bf16x2(__uint_as_float(r[8 * j + 2]), __uint_as_float(r[8 * j + 3]));
-        v.z = pack_bf16x2(__uint_as_float(r[8 * j + 4]), __uint_as_float(r[8 * j + 5]));
-        v.w = pack_bf16x2(__uint_as_float(r[8 * j + 6]), __uint_as_float(r[8 * j + 7]));
-        *reinterpret_cast<uint4*>(dst + j * 8) = v;
-      }
-  } else {
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (col0 + j * 4 < n)
-        *reinterpret_cast<uint4*>(dst + j * 4) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
-  }
-}
 
 // The qkv epilogue of a warp: 16 tokens (from row0 on) of the tile's two heads.  In the accumulator's layout (a lane per token) it is bound
 // by the LSU: angles and rows are then 16-byte accesses to 32 different lines each (13.4 K tokens x 4096 x 1024: 168 us, against 96 + 67 for
@@ -301,6 +279,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
     // ===== epilogue (both CTAs): own 128 TMEM lanes -> global =====
     pdl_wait();
     const int q = warp & 3;
+    [[maybe_unused]] const bool wide = rows_on_32(y, ldy);
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int tile = cluster_id; tile < num_tiles; tile += num_clusters) {
@@ -336,7 +315,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
             g[e + 1] = __float_as_uint(p.y);
           }
           const int col0 = n_tile * (BN / 2) + c * 32;
-          if (row < at.m_end && col0 < N) store_row32_2<OutT>(y + row * ldy + col0, g, col0, N);
+          if (row < at.m_end && col0 < N) store_row32<OutT>(y + row * ldy + col0, g, col0, N, wide);
         }
       } else {
         // add: y holds the residual stream, and the product's bf16 values are added to it in place.  A chunk's old values are requested
@@ -372,7 +351,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
             if (c + 1 < c1) request(c + 1);
           }
           const int col0 = n_tile * BN + c * 32;
-          if (row < at.m_end && col0 < N) store_row32_2<OutT>(y + row * ldy + col0, r, col0, N);
+          if (row < at.m_end && col0 < N) store_row32<OutT>(y + row * ldy + col0, r, col0, N, wide);
         }
       }
       tc_fence_before();

@@ -137,12 +137,6 @@ __device__ __noinline__ void row_alone(const LatentAttnArgs& a, int tok, int hea
 __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(p), "r"(bytes) : "memory");
 }
-// 32 bytes at once: a whole sector of the one row that a lane writes
-__device__ __forceinline__ void st_32(void* p, const uint32_t (&v)[8]) {
-  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]),
-               "r"(v[7])
-               : "memory");
-}
 
 // wide: rows of the output lie on 32 bytes
 __global__ void __launch_bounds__(kThreads, 1) latent_attn_tc_kernel(const __grid_constant__ LatentAttnArgs a, int halves, bool wide) {
@@ -440,7 +434,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_attn_tc_kernel(const __gri
 #pragma unroll
               for (int i = 0; i < 8; ++i) v[i] = pack_bf16x2(__uint_as_float(o[16 * e + 2 * i]) * inv, __uint_as_float(o[16 * e + 2 * i + 1]) * inv);
               if (wide) {
-                st_32(out + c * 32 + e * 16, v);
+                st_global_32(out + c * 32 + e * 16, v);
               } else {
                 *reinterpret_cast<uint4*>(out + c * 32 + e * 16) = make_uint4(v[0], v[1], v[2], v[3]);
                 *reinterpret_cast<uint4*>(out + c * 32 + e * 16 + 8) = make_uint4(v[4], v[5], v[6], v[7]);

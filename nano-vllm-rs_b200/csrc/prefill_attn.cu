@@ -656,6 +656,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           if (gated) load_gate(0);
         }
         bf16* orow = p.out + static_cast<int64_t>(it.q0 + row) * p.out_stride + head * D;
+        const bool wide = rows_on_32(p.out, p.out_stride);
         float most = 0.f;   // largest |O| of the row, no number if one of them is none
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
@@ -685,13 +686,15 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           }
           if (row < it.Lq) {
 #pragma unroll
-            for (int e = 0; e < 32; e += 8) {
-              uint4 v;
-              v.x = pack_bf16x2(__uint_as_float(orr[e]) * inv, __uint_as_float(orr[e + 1]) * inv);
-              v.y = pack_bf16x2(__uint_as_float(orr[e + 2]) * inv, __uint_as_float(orr[e + 3]) * inv);
-              v.z = pack_bf16x2(__uint_as_float(orr[e + 4]) * inv, __uint_as_float(orr[e + 5]) * inv);
-              v.w = pack_bf16x2(__uint_as_float(orr[e + 6]) * inv, __uint_as_float(orr[e + 7]) * inv);
-              *reinterpret_cast<uint4*>(orow + c * 32 + e) = v;
+            for (int e = 0; e < 32; e += 16) {
+              uint32_t v[8];
+#pragma unroll
+              for (int k = 0; k < 8; ++k) v[k] = pack_bf16x2(__uint_as_float(orr[e + 2 * k]) * inv, __uint_as_float(orr[e + 2 * k + 1]) * inv);
+              if (wide) st_global_32(orow + c * 32 + e, v);
+              else {
+                *reinterpret_cast<uint4*>(orow + c * 32 + e) = make_uint4(v[0], v[1], v[2], v[3]);
+                *reinterpret_cast<uint4*>(orow + c * 32 + e + 8) = make_uint4(v[4], v[5], v[6], v[7]);
+              }
             }
           }
         }
