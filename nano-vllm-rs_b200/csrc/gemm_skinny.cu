@@ -10,8 +10,9 @@
 //   norm_w    x is the residual stream and every CTA normalises its own copy of the few rows (rms(x) * w rounded to bf16)
 //   GATE      w = [gate | up]; the CTA computes the matching rows of both and writes silu(gate) * up
 //   residual  y = bf16(y + bf16(x . w^T)): the projection's output goes into the stream in place
-// Measured, a decode step of one token (Qwen3-0.6B, 28 layers, graph replay): 1408 us on the tcgen05 kernels, 791 with these; 28 layers of
-// weights and the head take 180 us at the copy rate, the rest is latency: 143 dependent launches of 5-6 us.
+// Measured, a decode step of one token (Qwen3-0.6B, 28 layers, graph replay): 1408 us on the tcgen05 kernels, 760 with these; 28 layers of
+// weights and the head take 180 us at the copy rate, the rest is latency: 143 dependent launches of 5 us (all layers of one token in one
+// launch, where their weights fit the SMs: step_single.cu).
 #include "tc.cuh"
 
 namespace nvllm {

@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "../common.cuh"
+#include "../step_single.cuh"
 #include "model.hpp"
 #include "scheduler.hpp"
 
@@ -94,6 +95,9 @@ struct nvllm_runner {
   int64_t *local_ids = nullptr, *all_ids = nullptr, *tokens = nullptr;
   void* decode_ws = nullptr;
   size_t decode_ws_bytes = 0;
+  uint64_t* step_words = nullptr;   // step_single: what its CTAs exchange, its marks, its error (pinned)
+  unsigned* step_sync = nullptr;
+  int* h_step_error = nullptr;
   // step metadata: one device block + one pinned staging block
   uint8_t *d_meta = nullptr, *h_meta = nullptr;
   size_t meta_bytes = 0;
@@ -145,6 +149,7 @@ struct nvllm_runner {
     for (cudaEvent_t e : prof_pool) cudaEventDestroy(e);
     if (h_meta) cudaFreeHost(h_meta);
     if (h_tokens) cudaFreeHost(h_tokens);
+    if (h_step_error) cudaFreeHost(h_step_error);
     if (h_samp) cudaFreeHost(h_samp);
     if (h_logit_stage) cudaFreeHost(h_logit_stage);
     if (stream) cudaStreamDestroy(stream);
@@ -181,6 +186,8 @@ struct nvllm_runner {
            gemm_skinny_applies(N, qkv_dim, hidden, hidden, hidden, false, false) && gemm_skinny_applies(N, hidden, HD, HD, HD, false, false) &&
            gemm_skinny_applies(N, inter, hidden, hidden, hidden, false, true) && gemm_skinny_applies(N, hidden, inter, inter, inter, false, false);
   }
+  // a decode step of one token: all layers in one launch
+  bool single_token_step(int N, int S) const { return N == 1 && few_tokens(N, S) && step_single_applies(hidden, H, Hkv, D, inter, layers); }
   // where the q/k norm, the rotation and the store of a step's keys happen: in the qkv projection, or (decode) in the attention
   // (few tokens: a launch costs more than the attention's longer prologue)
   // Prefill: on CTA pairs the projection hides most of the pass over the qkv rows (Qwen3-0.6B, 13.4 K tokens 113 us a layer instead of 96 + 67,
@@ -390,6 +397,15 @@ int nvllm_runner::create(const nvllm_config& c, nvllm_comm* cm) {
     if (b >= max_seqs) break;
   }
   if (decode_ws_bytes) { uint8_t* p = nullptr; RUN(dalloc(&p, decode_ws_bytes)); decode_ws = p; }
+  if (single_token_step(1, 1)) {
+    const size_t words = static_cast<size_t>(step_single_words(hidden, H, Hkv, inter));
+    RUN(dalloc(&step_words, words));
+    RUN(dalloc(&step_sync, 3));
+    NVLLM_CUDA(cudaMemsetAsync(step_words, 0, words * sizeof(uint64_t), stream));
+    NVLLM_CUDA(cudaMemsetAsync(step_sync, 0, 3 * sizeof(unsigned), stream));
+    NVLLM_CUDA(cudaMallocHost(reinterpret_cast<void**>(&h_step_error), sizeof(int)));
+    *h_step_error = 0;
+  }
   // metadata
   const size_t S = max_seqs;
   const size_t prefill_meta = 28 * T + 8 * (S + 1) + 4 * S * table_cap + 4 * S;
@@ -706,7 +722,22 @@ int nvllm_runner::forward(int N, int S, bool is_prefill, bool paged_prefill, con
   RUN(nvllm_embedding_gather(h, embed, d_ids, N, hidden, vocab, NVLLM_BF16, st)); ++launches; mark("embedding_gather");
   const int splits = is_prefill ? 1 : nvllm_paged_decode_choose_splits(N, H, Hkv, table_cap * layout.block_size);
   if (!is_prefill) last_decode_splits = splits;
-  for (int l = 0; l < layers; ++l) {
+  const bool single = !is_prefill && step_words != nullptr && single_token_step(N, S);
+  if (single) {
+    StepArgs a{};
+    for (int l = 0; l < layers; ++l) {
+      const LayerWeights& w = lw[l];
+      a.layer[l] = {w.qkv, w.o, w.gate_up, w.down, w.input_ln, w.post_ln, cfg.qk_norm ? w.q_norm : nullptr, cfg.qk_norm ? w.k_norm : nullptr, kc[l], vc[l]};
+    }
+    a.h = h; a.sync = step_sync; a.error = h_step_error;
+    a.pos = d_pos; a.slots = d_slots; a.tables = d_tables; a.ctx = d_ctx; a.cos_sin = rope;
+    a.blk_stride = layout.block_stride; a.tok_stride = layout.token_stride; a.head_stride = layout.head_stride;
+    a.max_position = cfg.max_position_embeddings;
+    a.layers = layers; a.hidden = hidden; a.heads = H; a.kv_heads = Hkv; a.inter = inter; a.block_size = layout.block_size; a.table_cap = table_cap;
+    a.eps = eps; a.scale_log2 = scale * 1.4426950408889634f;
+    RUN(step_single(a, step_words, stream)); ++launches; mark("all layers (one token)");
+  }
+  for (int l = 0; l < layers && !single; ++l) {
     const LayerWeights& w = lw[l];
     // input_layernorm; for l > 0 it follows the residual add of the previous MLP output (qwen3.rs:389 -> :378), see close_block
     if (!few && l == 0) { RUN(nvllm_add_rmsnorm(normed, h, nullptr, w.input_ln, N, hidden, eps, NVLLM_BF16, st)); ++launches; mark("add_rmsnorm"); }
@@ -895,6 +926,10 @@ int nvllm_runner::sample(const nvllm_batch& b) {
 int nvllm_runner::fetch(int64_t* out, int n) {
   NVLLM_CUDA(cudaStreamSynchronize(stream));
   if (!prof_marks.empty()) prof_collect();
+  if (h_step_error != nullptr && *h_step_error != 0) {
+    *h_step_error = 0;
+    NVLLM_CHECK_ARG(false, NVLLM_ERR_STATE, "execute: the step's thread blocks waited for one another in vain");
+  }
   if (comm != nullptr) RUN(nvllm_comm_error(comm));  // a fused TP kernel gave up waiting for a peer: tokens are garbage
   if (out) memcpy(out, h_tokens, sizeof(int64_t) * n);
   return 0;

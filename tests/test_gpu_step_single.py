@@ -1,0 +1,96 @@
+"""Decode steps of one token in one launch (step_single.cu) against the general path, where its shares, parts and rounds can go wrong."""
+import threading
+
+import numpy as np
+import pytest
+
+from tests.test_gpu_engine import LOGIT_RTOL, LOGIT_SIGMA_PER_SQRT_LAYER
+
+pytestmark = pytest.mark.gpu
+VOCAB, LAYERS = 1024, 2
+
+
+def weights_of(W, H, kv, ff, device):
+    import torch
+    shapes = {"model.embed_tokens.weight": (VOCAB, W), "model.norm.weight": (W,)}
+    for l in range(LAYERS):
+        p = f"model.layers.{l}."
+        shapes.update({p + "input_layernorm.weight": (W,), p + "post_attention_layernorm.weight": (W,), p + "self_attn.q_norm.weight": (128,),
+                       p + "self_attn.k_norm.weight": (128,), p + "self_attn.q_proj.weight": (H * 128, W), p + "self_attn.k_proj.weight": (kv * 128, W),
+                       p + "self_attn.v_proj.weight": (kv * 128, W), p + "self_attn.o_proj.weight": (W, H * 128), p + "mlp.gate_proj.weight": (ff, W),
+                       p + "mlp.up_proj.weight": (ff, W), p + "mlp.down_proj.weight": (W, ff)})
+    gen = torch.Generator(device=device).manual_seed(W + H)
+    out = {}
+    for name, shape in shapes.items():
+        x = torch.randn(shape, generator=gen, device=device)
+        x = 1.0 + 0.3 * x if "norm" in name else (x if "embed" in name else x * shape[-1] ** -0.5)
+        out[name] = x.to(torch.bfloat16).view(torch.int16).cpu().numpy().view(np.uint16)
+    return out
+
+
+class Decoder:
+    def __init__(self, W, H, kv, ff, weights, bs, qk_norm=1, max_len=2304, eager=0):
+        from nano_vllm_rs_b200 import engine as E
+        self.E = E
+        cfg = E.Config("qwen3-0.6b", hidden_size=W, num_attention_heads=H, num_key_value_heads=kv, intermediate_size=ff, vocab_size=VOCAB, qk_norm=qk_norm,
+                       num_hidden_layers=LAYERS, max_num_seqs=2, max_num_batched_tokens=max_len, max_model_len=max_len, kvcache_block_size=bs,
+                       num_kvcache_blocks=max_len // bs + 2, enforce_eager=eager).validate()
+        self.sched, self.runner = E.Scheduler(cfg), E.ModelRunner(cfg)
+        for name, w in weights.items():
+            self.runner.load_weight(name, w)
+
+    def run(self, prompt, forced):
+        """Logits of the prompt's last token and of a decode step behind each forced token but the last."""
+        self.sched.add_sequence(prompt, self.E.SamplingParams(temperature=0.0, max_tokens=len(forced), ignore_eos=True))
+        out = []
+        for t in forced:
+            out.append(self.runner.execute_model(self.sched.schedule(), return_logits=True)[1][0])
+            self.sched.postprocess([int(t)])
+        return np.stack(out)
+
+
+# groups of 1, 2 and 4 heads; widths whose rows leave some lanes without a piece, more rows than warps, and CTAs with one row; a stream of four values a thread
+@pytest.mark.parametrize("W,H,kv,ff,bs,qk_norm", [
+    (1024, 16, 8, 3072, 256, 1), (1024, 16, 8, 3072, 16, 0), (1024, 8, 8, 2048, 16, 1), (1024, 16, 4, 3072, 32, 1), (960, 12, 6, 2560, 16, 1),
+    (192, 4, 2, 320, 16, 1), (2048, 4, 2, 1024, 256, 1), (512, 4, 4, 3072, 64, 1)])
+def test_one_token_in_one_launch(cuda, W, H, kv, ff, bs, qk_norm, monkeypatch):
+    """Contexts around a round of 32 keys, a part of 64, the four rounds that are asked for ahead (9 parts of 128 keys), and several times as many.  The
+    logits of the general path, up to the roundings that another order of the sums, and probabilities in f32, flip."""
+    rng = np.random.default_rng(W + kv)
+    weights = weights_of(W, H, kv, ff, cuda)
+    lens = [1, 30, 63, 126, 573, 1150, 2290]
+    prompts = [rng.integers(0, VOCAB, n).tolist() for n in lens]
+    forced = rng.integers(0, VOCAB, (len(lens), 6))
+    got = {}
+    for skinny in ("0", "1"):
+        monkeypatch.setenv("NVLLM_GEMM_SKINNY", skinny)
+        d = Decoder(W, H, kv, ff, weights, bs, qk_norm)
+        got[skinny] = np.stack([d.run(p, f) for p, f in zip(prompts, forced)])     # eager, captured, replayed: the fifth token comes from the graph
+        d = Decoder(W, H, kv, ff, weights, bs, qk_norm, eager=1)
+        d.runner.profile()
+        assert np.array_equal(d.run(prompts[1], forced[1]), got[skinny][1])
+        assert ("all layers (one token)" in d.runner.profile_report()) == (skinny == "1")
+    sig = got["0"].std(-1, keepdims=True)
+    err = np.abs(got["1"] - got["0"])
+    tol = LOGIT_SIGMA_PER_SQRT_LAYER * np.sqrt(LAYERS) * sig + LOGIT_RTOL * np.abs(got["0"])
+    assert (err <= tol).all(), float((err / tol).max())
+
+
+def test_two_threads(cuda):
+    """Two runners, each with a stream of its own, at the same time: what either gives alone."""
+    rng = np.random.default_rng(3)
+    dims = (1024, 16, 8, 3072)
+    weights = weights_of(*dims, cuda)
+    prompts, forced = [rng.integers(0, VOCAB, 100 + 50 * i).tolist() for i in range(2)], rng.integers(0, VOCAB, (2, 60))
+    alone = [Decoder(*dims, weights, 16).run(p, f) for p, f in zip(prompts, forced)]
+    decoders, both = [Decoder(*dims, weights, 16) for _ in range(2)], [None, None]
+
+    def work(i):
+        both[i] = decoders[i].run(prompts[i], forced[i])
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert all(np.array_equal(a, b) for a, b in zip(alone, both))
