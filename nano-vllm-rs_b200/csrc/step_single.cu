@@ -5,7 +5,7 @@
 // its share of a layer fits its shared memory the share of layer l + 1 is copied there, one bulk copy a matrix, as soon as layer l has left
 // the room, so that the weights stream whatever the CTAs wait for.  What they hand to one another, the stream, q / k / v, parts of the attention and the gated
 // values, travels as 8-byte words of a value and a mark that tells layer and launch: the reader asks for the word itself until it carries
-// the mark.  (With a barrier between the stages, a step took 601 us instead of 560: the release behind the stores, the wait for the counter and the read of the
+// the mark.  (With a barrier between the stages, a step took 601 us instead of 532: the release behind the stores, the wait for the counter and the read of the
 // data are three trips to L2 instead of one.)
 //   1  norm + q, k, v projection         every CTA norms its own copy of the token's row
 //   2  attention                         item = (kv head, part of the keys): q/k norm and rotation in the CTA, a half warp per key, the first keys
@@ -16,7 +16,7 @@
 // A word is written anew only behind a stage that every CTA takes part in and that needs what was read from it, so no reader can miss its mark; every CTA has
 // rows of every matrix for that reason.  Rounded to bf16 in the same places as by the separate kernels, but probabilities stay f32.
 // Bound by the chain of stages, 2 to 4 K clocks each: the trip of the words through L2, then the products' and sums' latency.
-// Measured, Qwen3-0.6B (28 layers, 151936 rows of the head, us, kernel by kernel and here): behind 300 tokens 798 and 560, 1000 900 and 607, 3900 920 and 844.
+// Measured, Qwen3-0.6B (28 layers, 151936 rows of the head, us, kernel by kernel and here): behind 300 tokens 798 and 532, 1000 900 and 603, 3900 920 and 791.
 #include <type_traits>
 
 #include "step_single.cuh"
@@ -62,8 +62,7 @@ template <int N, bool FIRST = true>
 __device__ __forceinline__ void take(uint32_t (&out)[N], const uint64_t* p, int stride, int n, uint32_t mark, const Waiting& wt) {
   long long t0 = 0;
   int tries = 0;
-  // Until its first word is there a warp asks for this word alone: asked for by all lanes of all CTAs again and again, the words take the
-  // bandwidth that the weights and the stores need.
+  // FIRST: a warp asks for its first word alone until that is there (see first_word)
   if (FIRST) {
     if ((threadIdx.x & 31) == 0 && n > 0)
       while (static_cast<uint32_t>(look(p) >> 32) != mark && !in_vain(tries, t0, wt)) {}
@@ -159,6 +158,16 @@ __global__ void __launch_bounds__(kThreads, 1) step_single_kernel(const __grid_c
     for (int i = 0; i < 4; ++i) fetch(i, 0);
   const uint32_t base = *reinterpret_cast<volatile unsigned*>(a.sync);   // the marks of this launch: base + 1 .. base + 2 layers
   const Waiting wt{a.sync + 2, base + 1, a.error};
+  // One thread asks for one word, then all ask for theirs: asked for again and again by many, the words are written later (a step behind 300 tokens: 640 us
+  // with all threads asking from the start, 582 with a lane of every warp, 549 with four, 532 so; copies of the words, or pauses, give nothing).
+  auto first_word = [&](const uint64_t* p, uint32_t mark) {
+    if (tid == 0) {
+      long long t0 = 0;
+      int tries = 0;
+      while (static_cast<uint32_t>(look(p) >> 32) != mark && !in_vain(tries, t0, wt)) {}
+    }
+    __syncthreads();
+  };
   // x = bf16(rms(h) * w) into shared memory; nw: the thread's values of w
   const int mine = (a.hidden - tid + kThreads - 1) / kThreads;           // values of h that the thread takes
   auto norm = [&](const bf16 (&nw)[kMine], uint32_t mark) {
@@ -167,7 +176,8 @@ __global__ void __launch_bounds__(kThreads, 1) step_single_kernel(const __grid_c
 #pragma unroll
       for (int i = 0; i < kMine; ++i) v[i] = i < mine ? __ldcg(reinterpret_cast<const unsigned short*>(a.h) + tid + i * kThreads) : 0u;
     } else {
-      take<kMine>(v, a.ll_h + tid, kThreads, mine, mark, wt);
+      first_word(a.ll_h + (cta * 7) % a.hidden, mark);
+      take<kMine, false>(v, a.ll_h + tid, kThreads, mine, mark, wt);
     }
     float f[kMine], s = 0.f;
 #pragma unroll
@@ -193,10 +203,11 @@ __global__ void __launch_bounds__(kThreads, 1) step_single_kernel(const __grid_c
   };
   // x = the 2 n values of n words
   auto gather = [&](const uint64_t* words, int n, uint32_t mark) {
+    first_word(words + (cta * 7) % n, mark);
     for (int i0 = 0; i0 < n; i0 += kMine * kThreads) {
       uint32_t v[kMine];
       const int cnt = (n - i0 - tid + kThreads - 1) / kThreads;
-      take<kMine>(v, words + i0 + tid, kThreads, cnt, mark, wt);
+      take<kMine, false>(v, words + i0 + tid, kThreads, cnt, mark, wt);
 #pragma unroll
       for (int i = 0; i < kMine; ++i)
         if (i < cnt) xw[i0 + tid + i * kThreads] = v[i];
