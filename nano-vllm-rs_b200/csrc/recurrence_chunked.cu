@@ -19,10 +19,10 @@
 // CTA = (head, sequence, 64 columns of v), 4 warps; a warp keeps 16 columns of the state, transposed, in the accumulator layout of
 // m16n8k16 (64 registers), which is also that of the B operand of S^T q, so the state never leaves its registers.  v comes from
 // global memory straight into the layout that serves as A (v^T of the update) and as B (of the middle product).  q and k of the
-// next chunk fly (cp.async) under the products of this one.  Bound by mma.sync issue (about 520 of them per warp and chunk) and the conversions
+// next chunk fly (cp.async) under the products of this one.  Bound by mma.sync issue (about 540 of them per warp and chunk) and the conversions
 // around it; two CTAs an SM (91 KB each) hide each other's barriers.
-// Token by token and here (us): 16 heads of 128 x 128, 8 x 1024 tokens 548 and 297, 500 tokens 210 and 107; 64 heads of 128 x 64, 8 x 1024
-// 875 and 594, 2 x 40 30 and 21.
+// Token by token and here (us): 16 heads of 128 x 128, 8 x 1024 tokens 548 and 274, 500 tokens 210 and 111; 64 heads of 128 x 64, 8 x 1024
+// 875 and 559, 2 x 40 30 and 24.
 #include "split_mma.cuh"
 
 namespace nvllm {
@@ -199,39 +199,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) linear_recurrence_chunked_kern
     __syncthreads();
     const bool slow = *flag != 0u;
     if (tb + kC < t1) issue(tb + kC, buf ^ 1);
-    // ---- middle factor (q_i . k_j) D_ij b_j (+ d on the diagonal): warp w computes tokens 16 (w / 2) .. + 15, keys 16 (w % 2) .. + 15 ---------------
     const uint32_t q_addr = sbase + kSmQ + (lane & 15) * kRow + (lane >> 4) * 16;
-    if (!slow && warp != 1) {       // warp 1's keys lie behind all of its tokens
-      const int mt = warp >> 1, nt = warp & 1;
-      float sum[2][4] = {}, ah[1][2][4], al[2][1][2][4] = {};   // (al: even and odd steps)
-      // B of 16 keys x 16 dims: lanes 0-7 keys 0-7 dims 0-7, 8-15 the same keys dims 8-15, 16-31 keys 8-15
-      const uint32_t k_addr = sbase + kSmK + (nt * 16 + (lane & 7) + (lane >> 4) * 8) * kRow + ((lane >> 3) & 1) * 16;
-#pragma unroll
-      for (int kk = 0; kk < kDk / 16; ++kk) {
-        uint32_t qf[1][3][4], kf[3][2][2];
-        if (kk % 2 == 0) zero(ah);
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          ldmatrix_x4(qf[0][j], q_addr + mt * 16 * kRow + kk * 32 + j * kPiece);
-          ldmatrix_x4(reinterpret_cast<uint32_t(&)[4]>(kf[j]), k_addr + kk * 32 + j * kPiece);
-        }
-        mma6<1, 2>(ah, al[kk & 1], qf, kf);
-        if (kk % 2 == 1) {
-#pragma unroll
-          for (int n = 0; n < 2; ++n)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) sum[n][i] += ah[0][n][i];
-        }
-      }
-#pragma unroll
-      for (int n = 0; n < 2; ++n)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int row = mt * 16 + r + (i >> 1) * 8, key = nt * 16 + n * 8 + c2 + (i & 1);
-          float* m = mid + row * kPs + key;
-          *m = fmaf(join(sum[n][i], al[0][0][n][i] + al[1][0][n][i]) * bs[key], *m, row == key ? d : 0.f);      // D is zero above the diagonal
-        }
-    }
     // v and the state: their largest magnitude decides whether the warp takes the products
     float vmax = 0.f;
 #pragma unroll
@@ -245,32 +213,54 @@ __global__ void __launch_bounds__(kWarps * 32, 2) linear_recurrence_chunked_kern
       smax[1] = abs_max(S[n][2], S[n][3], smax[1]);
     }
     const bool step = __any_sync(0xffffffffu, slow || !(smax[0] < 1.2e24f && smax[1] < 1.2e24f));      // 2^80
-    float yi[2][2][4] = {};           // S^T q of the chunk's start: [16 tokens][8 columns]
-    if (!step) {
+    // ---- middle factor (q_i . k_j) D_ij b_j (+ d on the diagonal): warp w computes tokens 16 (w / 2) .. + 15, keys 16 (w % 2) .. + 15 (warp 1's keys lie
+    // behind all of its tokens: it keeps nothing); and S^T q of the chunk's start.  Each alone is a chain of dependent products, the first of two at a time:
+    // one after the other, with the first left out by warp 1, 8 x 1024 tokens take 293 and 592 us instead of 274 and 559 (16 and 64 heads, see above).
+    float yi[2][2][4] = {};           // S^T q: [16 tokens][8 columns]
+    if (!slow) {                      // (also where this warp steps: the middle factor is for all)
+      const int mt = warp >> 1, nt = warp & 1;
+      float sum[2][4] = {}, ah[1][2][4], al[2][1][2][4] = {};   // (al: even and odd steps)
       float yl[2][2][4] = {}, hh[2][2][4];
+      // B of 16 keys x 16 dims: lanes 0-7 keys 0-7 dims 0-7, 8-15 the same keys dims 8-15, 16-31 keys 8-15
+      const uint32_t k_addr = sbase + kSmK + (nt * 16 + (lane & 7) + (lane >> 4) * 8) * kRow + ((lane >> 3) & 1) * 16;
 #pragma unroll
       for (int kk = 0; kk < kDk / 16; ++kk) {
-        if (kk % 2 == 0) zero(hh);
-        uint32_t sf[3][2][2];          // [piece][8 columns][half of the 16 keys]
+        uint32_t qm[1][3][4], kf[3][2][2], qf[2][3][4], sf[3][2][2];          // sf: [piece][8 columns][half of the 16 keys]
+        if (kk % 2 == 0) { zero(ah); zero(hh); }
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          ldmatrix_x4(qm[0][j], q_addr + mt * 16 * kRow + kk * 32 + j * kPiece);
+          ldmatrix_x4(reinterpret_cast<uint32_t(&)[4]>(kf[j]), k_addr + kk * 32 + j * kPiece);
+        }
 #pragma unroll
         for (int n = 0; n < 2; ++n)
 #pragma unroll
           for (int e = 0; e < 2; ++e) split3(S[2 * kk + e][2 * n], S[2 * kk + e][2 * n + 1], sf[0][n][e], sf[1][n][e], sf[2][n][e]);
-        uint32_t qf[2][3][4];
 #pragma unroll
         for (int m = 0; m < 2; ++m)
 #pragma unroll
           for (int j = 0; j < 3; ++j) ldmatrix_x4(qf[m][j], q_addr + m * 16 * kRow + kk * 32 + j * kPiece);
+        mma6<1, 2>(ah, al[kk & 1], qm, kf);
         mma6<2, 2>(hh, yl, qf, sf);
         if (kk % 2 == 1) {
 #pragma unroll
-          for (int m = 0; m < 2; ++m)
+          for (int n = 0; n < 2; ++n)
 #pragma unroll
-            for (int n = 0; n < 2; ++n)
-#pragma unroll
-              for (int i = 0; i < 4; ++i) yi[m][n][i] += hh[m][n][i];
+            for (int i = 0; i < 4; ++i) {
+              sum[n][i] += ah[0][n][i];
+              yi[0][n][i] += hh[0][n][i];
+              yi[1][n][i] += hh[1][n][i];
+            }
         }
       }
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int row = mt * 16 + r + (i >> 1) * 8, key = nt * 16 + n * 8 + c2 + (i & 1);
+          float* m = mid + row * kPs + key;
+          if (warp != 1) *m = fmaf(join(sum[n][i], al[0][0][n][i] + al[1][0][n][i]) * bs[key], *m, row == key ? d : 0.f);      // D is zero above the diagonal
+        }
 #pragma unroll
       for (int m = 0; m < 2; ++m)
 #pragma unroll
