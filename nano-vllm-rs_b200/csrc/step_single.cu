@@ -14,7 +14,8 @@
 //   4  norm + gate / up projection + SiLU gate
 //   5  down projection + residual
 // A word is written anew only behind a stage that every CTA takes part in and that needs what was read from it, so no reader can miss its mark; every CTA has
-// rows of every matrix for that reason.  Rounded to bf16 in the same places as by the separate kernels, but probabilities stay f32.
+// rows of every matrix for that reason.  Rounded to bf16 in the same places as by the separate kernels, but probabilities stay f32 (logits of
+// Qwen3-0.6B against 64 bits, mean of 24 steps: 0.0128 kernel by kernel, 0.0127 here).
 // Bound by the chain of stages, 2 to 4 K clocks each: the trip of the words through L2, then the products' and sums' latency.
 // Measured, Qwen3-0.6B (28 layers, 151936 rows of the head, us, kernel by kernel and here): behind 300 tokens 798 and 532, 1000 900 and 603, 3900 920 and 791.
 #include <type_traits>
