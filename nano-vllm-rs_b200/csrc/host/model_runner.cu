@@ -98,6 +98,7 @@ struct nvllm_runner {
   uint64_t* step_words = nullptr;   // step_single: what its CTAs exchange, its marks, its error (pinned)
   unsigned* step_sync = nullptr;
   int* h_step_error = nullptr;
+  bool one_launch = false;          // the decode step at hand is step_single's
   // step metadata: one device block + one pinned staging block
   uint8_t *d_meta = nullptr, *h_meta = nullptr;
   size_t meta_bytes = 0;
@@ -722,7 +723,7 @@ int nvllm_runner::forward(int N, int S, bool is_prefill, bool paged_prefill, con
   RUN(nvllm_embedding_gather(h, embed, d_ids, N, hidden, vocab, NVLLM_BF16, st)); ++launches; mark("embedding_gather");
   const int splits = is_prefill ? 1 : nvllm_paged_decode_choose_splits(N, H, Hkv, table_cap * layout.block_size);
   if (!is_prefill) last_decode_splits = splits;
-  const bool single = !is_prefill && step_words != nullptr && single_token_step(N, S);
+  const bool single = !is_prefill && one_launch;
   if (single) {
     StepArgs a{};
     for (int l = 0; l < layers; ++l) {
@@ -849,7 +850,9 @@ int nvllm_runner::execute_async(const nvllm_batch& b) {
   } else {
     const int padded = bucket_for(b.num_seqs, max_seqs);
     RUN(upload(b, padded));
-    Graph& g = graphs[padded];
+    // a step of one token has two routes (by its context), and a graph for either
+    one_launch = step_words != nullptr && padded == 1 && single_token_step(1, 1) && b.context_lens[0] <= kStepContext;
+    Graph& g = graphs[one_launch ? 0 : padded];
     ++g.uses;
     if (cfg.enforce_eager || g.uses == 1) {
       // first use of a bucket runs eagerly (lazy per-kernel attribute setup happens outside capture)
@@ -1079,7 +1082,7 @@ int nvllm_runner_replay_decode(nvllm_runner* r, int32_t iters, float* ms_total) 
   NVLLM_CHECK_ARG(r && iters > 0 && ms_total, NVLLM_ERR_ARG, "replay_decode: arguments");
   NVLLM_CHECK_ARG(r->last_decode_b > 0 && r->d_ctx != nullptr, NVLLM_ERR_STATE, "replay_decode: no decode step has run yet");
   const int P = r->last_decode_b;
-  auto it = r->graphs.find(P);
+  auto it = r->graphs.find(r->one_launch ? 0 : P);
   const bool use_graph = !r->cfg.enforce_eager && it != r->graphs.end() && it->second.exec != nullptr;
   nvllm_batch dummy;
   memset(&dummy, 0, sizeof(dummy));

@@ -17,7 +17,8 @@
 // rows of every matrix for that reason.  Rounded to bf16 in the same places as by the separate kernels, but probabilities stay f32 (logits of
 // Qwen3-0.6B against 64 bits, mean of 24 steps: 0.0128 kernel by kernel, 0.0127 here).
 // Bound by the chain of stages, 2 to 4 K clocks each: the trip of the words through L2, then the products' and sums' latency.
-// Measured, Qwen3-0.6B (28 layers, 151936 rows of the head, us, kernel by kernel and here): behind 300 tokens 798 and 532, 1000 900 and 603, 3900 920 and 791.
+// Measured, Qwen3-0.6B (28 layers, 151936 rows of the head, us, kernel by kernel and here): behind 300 tokens 798 and 532, 1000 900 and 603, 3900 937 and 759,
+// 10000 1118 and 982, 20000 1285 and 1335: contexts of more than 16384 stay with the separate kernels (the runner decides).
 #include <type_traits>
 
 #include "step_single.cuh"
@@ -26,6 +27,9 @@
 namespace nvllm {
 namespace {
 
+// Parts of 64 keys and more: up to 9, of which one collects the other 8 in one go, and from 2880 keys on 17 (a step behind 1000, 2500, 3900, 7000 tokens, us: 9 parts
+// 605, 702, 795, 1019; 17 parts 629, 713, 759, 882).
+constexpr int kFewKeys = 2880, kFewParts = 9;
 constexpr int kThreads = 512, kWarps = 16, kD = 128, kParts = kStepParts, kSplitKeys = 64, kAhead = 4, kMine = 4;
 
 __device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
@@ -235,7 +239,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_single_kernel(const __grid_c
   if (tid < hn) own[tid] = a.h[h0 + tid];
 
   // attention: this CTA's item
-  const int ctx_all = __ldg(a.ctx), ctx = max(ctx_all - 1, 0), splits = min(max((ctx_all + kSplitKeys - 1) / kSplitKeys, 1), a.max_splits);
+  const int ctx_all = __ldg(a.ctx), ctx = max(ctx_all - 1, 0), splits = min(max((ctx_all + kSplitKeys - 1) / kSplitKeys, 1), ctx_all <= kFewKeys ? min(kFewParts, a.max_splits) : a.max_splits);
   const int kvh = cta % a.kv_heads, split = cta / a.kv_heads;
   const bool item = split < splits;
   const int per = (ctx_all + splits - 1) / splits, key0 = min(split * per, ctx_all), key1 = min(key0 + per, ctx_all);   // (key ctx: the step's own)

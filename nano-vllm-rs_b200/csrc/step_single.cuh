@@ -6,7 +6,8 @@
 namespace nvllm {
 
 constexpr int kStepLayers = 64, kStepRows = 128;       // at the most: layers, rows of h of a CTA
-constexpr int kStepParts = 9, kStepPart = 130;         // parts of the keys at the most (8 besides the one that merges); words of one: 128 sums, maximum, sum of weights
+constexpr int kStepContext = 16384;                    // tokens of the context at the most
+constexpr int kStepParts = 17, kStepPart = 130;         // parts of the keys at the most; words of one: 128 sums, maximum, sum of weights
 
 struct StepLayer {
   const bf16 *qkv, *o, *gate_up, *down, *input_ln, *post_ln, *q_norm, *k_norm;   // (q_norm, k_norm: may be NULL)

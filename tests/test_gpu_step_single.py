@@ -29,7 +29,7 @@ def weights_of(W, H, kv, ff, device):
 
 
 class Decoder:
-    def __init__(self, W, H, kv, ff, weights, bs, qk_norm=1, max_len=2304, eager=0):
+    def __init__(self, W, H, kv, ff, weights, bs, qk_norm=1, max_len=3328, eager=0):
         from nano_vllm_rs_b200 import engine as E
         self.E = E
         cfg = E.Config("qwen3-0.6b", hidden_size=W, num_attention_heads=H, num_key_value_heads=kv, intermediate_size=ff, vocab_size=VOCAB, qk_norm=qk_norm,
@@ -54,11 +54,11 @@ class Decoder:
     (1024, 16, 8, 3072, 256, 1), (1024, 16, 8, 3072, 16, 0), (1024, 8, 8, 2048, 16, 1), (1024, 16, 4, 3072, 32, 1), (960, 12, 6, 2560, 16, 1),
     (192, 4, 2, 320, 16, 1), (2048, 4, 2, 1024, 256, 1), (512, 4, 4, 3072, 64, 1)])
 def test_one_token_in_one_launch(cuda, W, H, kv, ff, bs, qk_norm, monkeypatch):
-    """Contexts around a round of 32 keys, a part of 64, the four rounds that are asked for ahead (9 parts of 128 keys), and several times as many.  The
+    """Contexts around a round of 32 keys, a part of 64, the four rounds that are asked for ahead (9 parts of 128 keys), several times as many, and around the step to 17 parts.  The
     logits of the general path, up to the roundings that another order of the sums, and probabilities in f32, flip."""
     rng = np.random.default_rng(W + kv)
     weights = weights_of(W, H, kv, ff, cuda)
-    lens = [1, 30, 63, 126, 573, 1150, 2290]
+    lens = [1, 30, 63, 126, 573, 1150, 2290, 2877, 3300]
     prompts = [rng.integers(0, VOCAB, n).tolist() for n in lens]
     forced = rng.integers(0, VOCAB, (len(lens), 6))
     got = {}
@@ -74,6 +74,20 @@ def test_one_token_in_one_launch(cuda, W, H, kv, ff, bs, qk_norm, monkeypatch):
     err = np.abs(got["1"] - got["0"])
     tol = LOGIT_SIGMA_PER_SQRT_LAYER * np.sqrt(LAYERS) * sig + LOGIT_RTOL * np.abs(got["0"])
     assert (err <= tol).all(), float((err / tol).max())
+
+
+def test_long_contexts_take_the_separate_kernels(cuda, monkeypatch):
+    """Steps on both sides of the longest context, as replayed graphs of either route: the logits of the general path."""
+    rng = np.random.default_rng(9)
+    dims = (1024, 4, 2, 640)
+    weights, prompt, forced = weights_of(*dims, cuda), rng.integers(0, VOCAB, 16378).tolist(), rng.integers(0, VOCAB, 12)
+    got = {}
+    for skinny in ("0", "1"):
+        monkeypatch.setenv("NVLLM_GEMM_SKINNY", skinny)
+        got[skinny] = Decoder(*dims, weights, 256, max_len=16640).run(prompt, forced)
+    sig = got["0"].std(-1, keepdims=True)
+    tol = LOGIT_SIGMA_PER_SQRT_LAYER * np.sqrt(LAYERS) * sig + LOGIT_RTOL * np.abs(got["0"])
+    assert (np.abs(got["1"] - got["0"]) <= tol).all()
 
 
 def test_two_threads(cuda):
