@@ -194,8 +194,8 @@ int nvllm_runner_set_eager(nvllm_runner* r, int32_t eager);
 int64_t nvllm_runner_last_launches(const nvllm_runner* r);
 /* Device pointers of layer `layer`'s K / V cache and the layout in use (tests, hosts that bind layers). */
 int nvllm_runner_kv_cache(nvllm_runner* r, int32_t layer, void** k_cache, void** v_cache, nvllm_kv_layout* layout);
-/* Re-runs only the paged decode attention of layer 0 on the last decode batch `iters` times between two CUDA
- * events (for the roofline line of bench.py); returns the average milliseconds per launch. */
+/* Re-runs only the paged decode attention, layer after layer, on the last decode batch `iters` times between two CUDA
+ * events (for the roofline line of bench.py); returns the average milliseconds per launch.  The caches stay as they are. */
 int nvllm_runner_time_decode_attention(nvllm_runner* r, int32_t iters, float* ms_per_launch, int64_t* alg_bytes);
 
 /* Replays the last decode step `iters` times with its inputs already resident in HBM (graph launches only; no host

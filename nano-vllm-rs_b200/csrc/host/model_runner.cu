@@ -1104,19 +1104,29 @@ int nvllm_runner_replay_decode(nvllm_runner* r, int32_t iters, float* ms_total) 
 
 // Re-launches the paged decode attention on the last decode batch's metadata (still resident), cycling through the
 // layers' caches so that consecutive launches never re-read the same KV from L2; CUDA events on the runner's stream.
+// Nothing is stored: qkv holds the rows of the last layer, or, behind a step in one launch, nothing of it at all (zeros then).
 int nvllm_runner_time_decode_attention(nvllm_runner* r, int32_t iters, float* ms_per_launch, int64_t* alg_bytes) {
   NVLLM_CHECK_ARG(r && iters > 0 && ms_per_launch, NVLLM_ERR_ARG, "time_decode_attention: arguments");
   NVLLM_CHECK_ARG(!r->model, NVLLM_ERR_STATE, "time_decode_attention: built-in Qwen3 runner only");
   NVLLM_CHECK_ARG(r->last_decode_b > 0 && r->d_ctx != nullptr, NVLLM_ERR_STATE, "time_decode_attention: no decode step has run yet");
   const int B = r->last_decode_b, HD = r->H * r->D;
   const float scale = 1.0f / sqrtf(static_cast<float>(r->D));
-  const bool fused = r->rope_in_decode(B, B);  // the kernel the decode step launches
+  const bool fused = r->rope_in_decode(B, B);  // the kernel that a step of this many tokens launches (one token in one launch aside)
+  struct Slots {
+    int32_t* p = nullptr;
+    ~Slots() { if (p) cudaFree(p); }
+  } none;   // a slot of -1: the token's key and value are not stored
+  if (fused) {
+    NVLLM_CUDA(cudaMalloc(reinterpret_cast<void**>(&none.p), sizeof(int32_t) * B));
+    NVLLM_CUDA(cudaMemsetAsync(none.p, 0xff, sizeof(int32_t) * B, r->stream));
+  }
+  if (r->one_launch) NVLLM_CUDA(cudaMemsetAsync(r->qkv, 0, sizeof(bf16) * B * r->qkv_dim, r->stream));
   auto launch = [&](int l) {
-    if (fused) {  // re-stores the step's K/V rows into the same slots: idempotent
+    if (fused) {
       const auto& w = r->lw[l];
       return nvllm_paged_decode_attention_fused(r->attn, r->qkv, r->d_pos, r->rope, r->cfg.qk_norm ? w.q_norm : nullptr,
                                                 r->cfg.qk_norm ? w.k_norm : nullptr, r->cfg.rms_norm_eps,
-                                                r->cfg.max_position_embeddings, r->kc[l], r->vc[l], r->d_slots, r->d_tables,
+                                                r->cfg.max_position_embeddings, r->kc[l], r->vc[l], none.p, r->d_tables,
                                                 r->d_ctx, B, r->H, r->table_cap, r->qkv_dim, HD, &r->layout, scale,
                                                 r->decode_ws, r->decode_ws_bytes, r->last_decode_splits, NVLLM_BF16, r->stream);
     }
