@@ -98,6 +98,8 @@ struct nvllm_runner {
   uint64_t* step_words = nullptr;   // step_single: what its CTAs exchange, its marks, its error (pinned)
   unsigned* step_sync = nullptr;
   int* h_step_error = nullptr;
+  int64_t step_wait_clocks = kStepWaitClocks;
+  int step_silent = -1;
   bool one_launch = false;          // the decode step at hand is step_single's
   // step metadata: one device block + one pinned staging block
   uint8_t *d_meta = nullptr, *h_meta = nullptr;
@@ -200,6 +202,7 @@ struct nvllm_runner {
   int forward(int n_tokens, int n_seqs, bool is_prefill, bool paged_prefill, const nvllm_batch& b);
   int execute_async(const nvllm_batch& b);
   int fetch(int64_t* out, int n);
+  int step_error();
   int sample(const nvllm_batch& b);
   void mark(const char* name) {  // after a launch: no-op unless profiling an eager (non-captured) step
     if (!profiling) return;
@@ -730,7 +733,7 @@ int nvllm_runner::forward(int N, int S, bool is_prefill, bool paged_prefill, con
       const LayerWeights& w = lw[l];
       a.layer[l] = {w.qkv, w.o, w.gate_up, w.down, w.input_ln, w.post_ln, cfg.qk_norm ? w.q_norm : nullptr, cfg.qk_norm ? w.k_norm : nullptr, kc[l], vc[l]};
     }
-    a.h = h; a.sync = step_sync; a.error = h_step_error;
+    a.h = h; a.sync = step_sync; a.error = h_step_error; a.wait_clocks = step_wait_clocks; a.silent = step_silent;
     a.pos = d_pos; a.slots = d_slots; a.tables = d_tables; a.ctx = d_ctx; a.cos_sin = rope;
     a.blk_stride = layout.block_stride; a.tok_stride = layout.token_stride; a.head_stride = layout.head_stride;
     a.max_position = cfg.max_position_embeddings;
@@ -926,13 +929,18 @@ int nvllm_runner::sample(const nvllm_batch& b) {
                       reinterpret_cast<const uint64_t*>(d_samp + 16 * S), nullptr, nullptr, stream);
 }
 
+// Behind a synchronisation: whether a step in one launch gave up since the last look.
+int nvllm_runner::step_error() {
+  if (h_step_error == nullptr || *h_step_error == 0) return 0;
+  *h_step_error = 0;
+  NVLLM_CHECK_ARG(false, NVLLM_ERR_STATE, "decode step: its thread blocks waited for one another in vain");
+  return 0;
+}
+
 int nvllm_runner::fetch(int64_t* out, int n) {
   NVLLM_CUDA(cudaStreamSynchronize(stream));
   if (!prof_marks.empty()) prof_collect();
-  if (h_step_error != nullptr && *h_step_error != 0) {
-    *h_step_error = 0;
-    NVLLM_CHECK_ARG(false, NVLLM_ERR_STATE, "execute: the step's thread blocks waited for one another in vain");
-  }
+  RUN(step_error());
   if (comm != nullptr) RUN(nvllm_comm_error(comm));  // a fused TP kernel gave up waiting for a peer: tokens are garbage
   if (out) memcpy(out, h_tokens, sizeof(int64_t) * n);
   return 0;
@@ -1066,6 +1074,18 @@ int nvllm_runner_set_eager(nvllm_runner* r, int32_t eager) {
   r->cfg.enforce_eager = eager != 0;
   return 0;
 }
+int nvllm_runner_step_wait(nvllm_runner* r, int64_t clocks, int32_t silent_block) {
+  NVLLM_CHECK_ARG(r && clocks >= 0, NVLLM_ERR_ARG, "runner_step_wait: arguments");
+  NVLLM_CUDA(cudaStreamSynchronize(r->stream));
+  r->step_wait_clocks = clocks > 0 ? clocks : kStepWaitClocks;
+  r->step_silent = silent_block;
+  auto it = r->graphs.find(0);   // (captured with what held before)
+  if (it != r->graphs.end()) {
+    if (it->second.exec != nullptr) cudaGraphExecDestroy(it->second.exec);
+    r->graphs.erase(it);
+  }
+  return 0;
+}
 int64_t nvllm_runner_last_launches(const nvllm_runner* r) { return r ? r->last_launches : 0; }
 int nvllm_runner_kv_cache(nvllm_runner* r, int32_t layer, void** k_cache, void** v_cache, nvllm_kv_layout* layout) {
   NVLLM_CHECK_ARG(r && !r->model, NVLLM_ERR_STATE, "runner_kv_cache: built-in Qwen3 runner only");
@@ -1099,7 +1119,7 @@ int nvllm_runner_replay_decode(nvllm_runner* r, int32_t iters, float* ms_total) 
   NVLLM_CUDA(cudaEventElapsedTime(ms_total, e0, e1));
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  return 0;
+  return r->step_error();
 }
 
 // Re-launches the paged decode attention on the last decode batch's metadata (still resident), cycling through the

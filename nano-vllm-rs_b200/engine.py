@@ -87,6 +87,7 @@ ENGINE_PROTOTYPES = {
     "nvllm_runner_last_launches": (i64, [vp]),
     "nvllm_runner_kv_cache": (i32, [vp, i32, C.POINTER(vp), C.POINTER(vp), C.POINTER(_ffi.KvLayout)]),
     "nvllm_runner_time_decode_attention": (i32, [vp, i32, C.POINTER(f32), C.POINTER(i64)]),
+    "nvllm_runner_step_wait": (i32, [vp, i64, i32]),
     "nvllm_runner_replay_decode": (i32, [vp, i32, C.POINTER(f32)]),
     "nvllm_engine_create": (i32, [C.POINTER(vp), C.POINTER(CConfig), vp]),
     "nvllm_engine_destroy": (i32, [vp]),
