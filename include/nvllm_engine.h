@@ -192,7 +192,7 @@ int64_t nvllm_runner_profile_report(nvllm_runner* r, char* h_buf, size_t cap);
 int nvllm_runner_set_eager(nvllm_runner* r, int32_t eager);
 /* A decode step of one token may run in one launch, whose thread blocks wait for one another: for `clocks` SM clocks at the most
  * (0: the default, about a second), after which execute, fetch_tokens or replay_decode returns an error; the step's keys are then
- * undefined, and executing the step again gives what it should have given.  silent_block (tests): a block that hands nothing on,
+ * undefined, and executing the step again gives what it should have given.  silent_block (tests): a block that leaves out its rows,
  * -1 for none. */
 int nvllm_runner_step_wait(nvllm_runner* r, int64_t clocks, int32_t silent_block);
 /* Number of kernels launched by the last execute (decode graph node count, or eager launches). */

@@ -98,7 +98,7 @@ struct nvllm_runner {
   uint64_t* step_words = nullptr;   // step_single: what its CTAs exchange, its marks, its error (pinned)
   unsigned* step_sync = nullptr;
   int* h_step_error = nullptr;
-  int64_t step_wait_clocks = kStepWaitClocks;
+  unsigned step_wait = kStepWait;
   int step_silent = -1;
   bool one_launch = false;          // the decode step at hand is step_single's
   // step metadata: one device block + one pinned staging block
@@ -733,7 +733,7 @@ int nvllm_runner::forward(int N, int S, bool is_prefill, bool paged_prefill, con
       const LayerWeights& w = lw[l];
       a.layer[l] = {w.qkv, w.o, w.gate_up, w.down, w.input_ln, w.post_ln, cfg.qk_norm ? w.q_norm : nullptr, cfg.qk_norm ? w.k_norm : nullptr, kc[l], vc[l]};
     }
-    a.h = h; a.sync = step_sync; a.error = h_step_error; a.wait_clocks = step_wait_clocks; a.silent = step_silent;
+    a.h = h; a.sync = step_sync; a.error = h_step_error; a.wait = step_wait; a.silent = step_silent;
     a.pos = d_pos; a.slots = d_slots; a.tables = d_tables; a.ctx = d_ctx; a.cos_sin = rope;
     a.blk_stride = layout.block_stride; a.tok_stride = layout.token_stride; a.head_stride = layout.head_stride;
     a.max_position = cfg.max_position_embeddings;
@@ -1077,7 +1077,7 @@ int nvllm_runner_set_eager(nvllm_runner* r, int32_t eager) {
 int nvllm_runner_step_wait(nvllm_runner* r, int64_t clocks, int32_t silent_block) {
   NVLLM_CHECK_ARG(r && clocks >= 0, NVLLM_ERR_ARG, "runner_step_wait: arguments");
   NVLLM_CUDA(cudaStreamSynchronize(r->stream));
-  r->step_wait_clocks = clocks > 0 ? clocks : kStepWaitClocks;
+  r->step_wait = clocks > 0 ? static_cast<unsigned>(std::min<int64_t>((clocks + 1023) / 1024, 0xffffffffll)) : kStepWait;
   r->step_silent = silent_block;
   auto it = r->graphs.find(0);   // (captured with what held before)
   if (it != r->graphs.end()) {

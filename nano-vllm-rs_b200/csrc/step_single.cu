@@ -45,7 +45,7 @@ __device__ __forceinline__ void put(uint64_t* p, uint32_t value, uint32_t mark) 
 }
 // N words of which the first n of the thread count, `stride` apart, once they carry the mark.  Bounded: where one does not come, the step ends with an
 // error; the abort word then ends the waits of all CTAs.
-struct Waiting { unsigned* abort; unsigned aborted; int* error; long long clocks; };   // aborted: what the abort word is set to by this launch
+struct Waiting { unsigned* abort; unsigned aborted; int* error; long long limit; };   // aborted: what the abort word is set to by this launch
 
 __device__ __forceinline__ uint64_t look(const uint64_t* p) {
   uint64_t v;
@@ -57,7 +57,7 @@ __device__ __forceinline__ bool in_vain(int& tries, long long& t0, const Waiting
   if ((++tries & 255) != 0) return false;
   if (t0 == 0) t0 = clock64();
   if (*reinterpret_cast<volatile unsigned*>(wt.abort) == wt.aborted) return true;
-  if (clock64() - t0 < wt.clocks) return false;
+  if (((clock64() - t0) >> 10) < wt.limit) return false;   // (a 64-bit argument, or a word in memory, takes registers and 3 us a step)
   *reinterpret_cast<volatile unsigned*>(wt.abort) = wt.aborted;
   *wt.error = 1;
   return true;
@@ -130,6 +130,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_single_kernel(const __grid_c
   share(a.hidden, h0, hn);
   share(a.inter / 2, f0, fn);
   q0 *= 2; qn *= 2; f0 *= 2; fn *= 2;
+  if (cta == a.silent) hn = 0;   // (asked once: at the rows themselves it takes 4 us a step)
   uint8_t* const w_qkv = smem;
   uint8_t* const w_o = w_qkv + a.off_o;
   uint8_t* const w_gu = w_qkv + a.off_gu;
@@ -152,17 +153,17 @@ __global__ void __launch_bounds__(kThreads, 1) step_single_kernel(const __grid_c
     const uint32_t rows = which == 0 ? qn : (which == 2 ? fn : hn), bytes = rows * row;
     mbar_expect_tx(bar, which == 2 ? 2 * bytes : bytes);
     if (which == 0) bulk_load(smem_u32(w_qkv), w.qkv + static_cast<int64_t>(q0) * a.hidden, bytes, bar);
-    if (which == 1) bulk_load(smem_u32(w_o), w.o + static_cast<int64_t>(h0) * HD, bytes, bar);
+    if (which == 1 && rows > 0) bulk_load(smem_u32(w_o), w.o + static_cast<int64_t>(h0) * HD, bytes, bar);
     if (which == 2) {
       bulk_load(smem_u32(w_gu), w.gate_up + static_cast<int64_t>(f0) * a.hidden, bytes, bar);
       bulk_load(smem_u32(w_gu) + bytes, w.gate_up + static_cast<int64_t>(a.inter + f0) * a.hidden, bytes, bar);
     }
-    if (which == 3) bulk_load(smem_u32(w_down), w.down + static_cast<int64_t>(h0) * a.inter, bytes, bar);
+    if (which == 3 && rows > 0) bulk_load(smem_u32(w_down), w.down + static_cast<int64_t>(h0) * a.inter, bytes, bar);
   };
   if (tid == 0)
     for (int i = 0; i < 4; ++i) fetch(i, 0);
   const uint32_t base = *reinterpret_cast<volatile unsigned*>(a.sync);   // the marks of this launch: base + 1 .. base + 2 layers
-  const Waiting wt{a.sync + 2, base + 1, a.error, a.wait_clocks};
+  const Waiting wt{a.sync + 2, base + 1, a.error, a.wait};
   // One thread asks for one word, then all ask for theirs: asked for again and again by many, the words are written later (a step behind 300 tokens: 640 us
   // with all threads asking from the start, 582 with a lane of every warp, 549 with four, 532 so; copies of the words, or pauses, give nothing).
   auto first_word = [&](const uint64_t* p, uint32_t mark) {
@@ -232,7 +233,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_single_kernel(const __grid_c
     if (tid < hn) {
       const bf16 v = __float2bfloat16_rn(__bfloat162float(own[tid]) + __bfloat162float(__float2bfloat16_rn(part_sum[2 * tid] + part_sum[2 * tid + 1])));
       own[tid] = v;
-      if (cta != a.silent) put(a.ll_h + h0 + tid, __bfloat16_as_ushort(v), mark);
+      put(a.ll_h + h0 + tid, __bfloat16_as_ushort(v), mark);
       if (last) a.h[h0 + tid] = v;
     }
   };

@@ -8,7 +8,7 @@ namespace nvllm {
 constexpr int kStepLayers = 64, kStepRows = 128;       // at the most: layers, rows of h of a CTA
 constexpr int kStepContext = 16384;                    // tokens of the context at the most
 constexpr int kStepParts = 17, kStepPart = 130;         // parts of the keys at the most; words of one: 128 sums, maximum, sum of weights
-constexpr int64_t kStepWaitClocks = 2000000000;         // ~1 s
+constexpr unsigned kStepWait = 2000000;                // the usual limit of a wait: ~1 s of 1024 clocks
 
 struct StepLayer {
   const bf16 *qkv, *o, *gate_up, *down, *input_ln, *post_ln, *q_norm, *k_norm;   // (q_norm, k_norm: may be NULL)
@@ -26,8 +26,8 @@ struct StepArgs {
   int64_t blk_stride, tok_stride, head_stride, max_position;
   int layers, hidden, heads, kv_heads, inter, block_size, table_cap;
   float eps, scale_log2;
-  int64_t wait_clocks = kStepWaitClocks;   // a CTA waits this long for a word at the most
-  int silent = -1;                         // a CTA that keeps its rows of the stream to itself (tests); -1: none
+  unsigned wait;               // 1024 clocks that a CTA waits for a word at the most
+  int silent;                  // a CTA that leaves its rows of the stream out (tests); -1: none
   int off_o, off_gu, off_down, off_x, max_splits;   // filled in by step_single
 };
 
