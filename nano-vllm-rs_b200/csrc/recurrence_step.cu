@@ -29,10 +29,13 @@ struct StepArgs {
   float q_scale;
 };
 
+// (128 columns: two CTAs an SM; left to itself the compiler may take a few registers too many for that, and 256 sequences of the delta rule with 16 heads
+// of 128 x 128 take 141 us instead of 100)
 template <bool DELTA, bool CHANNEL, int COLS>
-__global__ void __launch_bounds__(kThreads) recurrence_step_kernel(const StepArgs a) {
+__global__ void __launch_bounds__(kThreads, COLS == 128 ? 2 : 0) recurrence_step_kernel(const StepArgs a) {
   constexpr int CT = COLS / 4, RG = kThreads / CT, R = kDk / RG;   // threads of a row, row groups, rows of a thread
-  __shared__ float ks[kDk], qs[kDk], gs[CHANNEL ? kDk : 1], vs[COLS];
+  __shared__ float ks[kDk], qs[kDk], gs[CHANNEL ? kDk : 1];
+  __shared__ __align__(16) float vs[COLS];
   __shared__ float4 red[DELTA ? 2 : 1][kWarps][CT];
   __shared__ float kq_s[kWarps];
   pdl_wait();
