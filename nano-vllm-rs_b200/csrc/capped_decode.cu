@@ -248,11 +248,12 @@ int cluster_that_fits(int64_t clusters) {
 
 }  // namespace
 
-// The options that the prompt kernel takes too: a window, a cap, a temperature, sinks and a gate.
+// The options that the prompt kernel takes too: a window, a cap, a temperature, sinks and a gate; and the alignment with which a step goes to the tensor
+// cores at all (the kernel needs less of q and out): other calls have their probabilities in f32.
 bool capped_decode_applies(const CappedAttnArgs& a, int n_seqs) {
   return n_seqs > 0 && a.n == n_seqs && a.heads / a.kv_heads <= 2 * kHeads && a.dim == D && a.vdim == D && a.tables != nullptr && a.block_size % 16 == 0 && a.keep == 0 && a.chunk == 0 &&
-         a.head_scale == nullptr && a.dist_bias == nullptr && a.out_rot == nullptr && a.slopes == nullptr && a.shared == 0 && a.ldq % 2 == 0 &&
-         (reinterpret_cast<uintptr_t>(a.q) & 3u) == 0 && a.k_row % 8 == 0 && a.v_row % 8 == 0 && aligned16(a.kc) && aligned16(a.vc) &&
+         a.head_scale == nullptr && a.dist_bias == nullptr && a.out_rot == nullptr && a.slopes == nullptr && a.shared == 0 && a.ldq % 8 == 0 &&
+         aligned16(a.q) && a.ldo % 2 == 0 && (reinterpret_cast<uintptr_t>(a.out) & 3u) == 0 && a.k_row % 8 == 0 && a.v_row % 8 == 0 && aligned16(a.kc) && aligned16(a.vc) &&
          a.kv_heads * ((a.heads / a.kv_heads + kHeads - 1) / kHeads) <= 65535;
 }
 

@@ -57,3 +57,23 @@ def test_single_tokens_at_the_edges_of_tiles(cuda, heads, kv, bs, window, softca
             ref = ref * torch.sigmoid(gate[t].double().reshape(heads, -1))
         err = out[t].double().reshape(heads, D) - ref
         assert float(err.norm() / ref.norm()) < 6e-3, (t, pos[t])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("offset,pad", [(2, 6), (0, 2), (1, 7)])
+def test_queries_off_16_bytes_keep_their_probabilities_in_f32(cuda, offset, pad):
+    """Two keys of weights 1 and 1 - 2^-10 whose values cancel: what is left, 2^-11, is gone where the weights are rounded to bf16.  Tolerance: the output's own
+    rounding, 2^-9, and a key's value in bf16 (2^-9 of a score of 2^-10)."""
+    from nano_vllm_rs_b200 import ops
+    heads, kv, bs, n = 4, 2, 16, 2
+    kc, vc = (torch.zeros(4 * bs, kv * D, device="cuda", dtype=torch.bfloat16) for _ in "kv")
+    tabs = torch.tensor([[2, -1], [1, -1]], device="cuda", dtype=torch.int32)
+    for b in (1, 2):
+        kc[b * bs + 1, ::D] = -(2.0 ** -10)
+        vc[b * bs], vc[b * bs + 1] = 1.0, -1.0
+    q = torch.zeros(n, heads * D + pad + offset, device="cuda", dtype=torch.bfloat16)[:, offset:offset + heads * D]
+    q[:, ::D] = 1.0
+    out = ops.window_attention(q, None, kc, vc, torch.arange(n, device="cuda", dtype=torch.int32), torch.ones(n, device="cuda", dtype=torch.int64), tabs, bs, heads, kv, D, D, 1.0,
+                               cu_tokens=torch.arange(n + 1, device="cuda", dtype=torch.int32))
+    p = math.exp(-(2.0 ** -10))
+    assert ((out.double() / ((1 - p) / (1 + p)) - 1).abs() < 5e-3).all()
