@@ -223,3 +223,17 @@ def test_tokens_do_not_depend_on_what_else_is_asked_for(cuda, rows, V):
         tp = None if p is None else torch.full((rows,), p, device=cuda)
         ids, _, _ = ops.sample(x, T, seeds, tk, tp, debug=True)
         assert torch.equal(ids, ops.sample(x, T, seeds, tk, tp)), (k, p)
+
+
+@pytest.mark.parametrize("V", [3000, 20000, 151936])
+def test_top_k_of_values_close_to_one_another(cuda, V):
+    """Rows whose largest values differ by less than 2^-11 of themselves (the bound of the candidates then takes all 32 bits), on either side of it, and tied."""
+    rng = np.random.default_rng(V + 7)
+    spread = np.array([1e-2, 1e-3, 1e-4, 3e-6, 1e-2, 0.3])[:, None]
+    x = (np.array([10, 10, -10, 10, 1e4, 10])[:, None] + rng.standard_normal((6, V)) * spread).astype(np.float32)
+    temps, ks, seeds = [1.0, 0.8, 1.0, 1.0, 0.9, 1.0], [1, 50, 20, 200, 256, 9], seeds_for(6, 13)
+    ids, cnt, mask = run(cuda, x, temps, seeds, top_k=ks)
+    for b in range(6):
+        want = np.isfinite(O.sample_single(x[b], temps[b], None, ks[b], seeds[b])[1])
+        assert cnt[b] == want.sum() == ks[b] and (mask[b] == want).all()
+        check_token(x[b], temps[b], mask[b], seeds[b], ids[b])
