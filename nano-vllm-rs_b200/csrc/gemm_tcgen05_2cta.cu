@@ -371,10 +371,12 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
 // The order of the tiles: panels of this many n-tiles, n fastest within a panel.  Up to K = 2048 one n-tile after the other (a w tile is read
 // once, x stays in L2): 8192 x 8192 x 2048 (gated) 401 us, 407 in panels of 12.  Longer rows of x leave L2 again before the next n-tile reads
 // them; in panels of 12 a wave of 74 tiles reads 12 tiles of w and 6 of x.  Measured (us, one n-tile after the other -> in panels of 12):
-// 8192 x 4096 x 12288 684 -> 629, 8192 x 24576 x 4096 1322 -> 1224, 8192 x 6144 x 4096 340 -> 314, 8192 x 2048 x 8192 247 -> 223, 12400 x 1024 x 3072
-// 73 -> 68.  Where a few m-tiles are no more than a wave anyway, panels of 2 do best: 3000 x 24576 x 4096 497 -> 461 (12: 470),
-// 1500 x 24576 x 4096 (gated) 247 -> 230 (237), 1500 x 4096 x 12288 161 -> 160 (161).
-static int panel_tiles(int num_m_tiles, int k) { return k < 3072 ? 1 : (num_m_tiles >= 16 ? 12 : 2); }
+// 8192 x 4096 x 12288 568 -> 527, 8192 x 6144 x 4096 281 -> 262, 8192 x 2048 x 8192 202 -> 184, 12400 x 1024 x 3072 59 -> 55.
+// Where a few m-tiles are no more than a wave anyway, panels of 2 do best: 3000 x 24576 x 4096 497 -> 461 (12: 470),
+// 1500 x 24576 x 4096 (gated) 247 -> 230 (237), 1500 x 4096 x 12288 161 -> 160 (161).  From 16 to 23 m-tiles it depends on the length of the rows (one n-tile
+// after the other, panels of 2, of 12): 4400 x 6144 x 4096 142, 140, 144, 4400 x 12288 x 4096 (gated) 570, 560, 577; 4400 x 2048 x 8192 101.5, 100.5, 97.9, 5000 x 4096 x 12288
+// 357, 351, 349.
+static int panel_tiles(int num_m_tiles, int k) { return k < 3072 ? 1 : (num_m_tiles >= 24 || (num_m_tiles >= 16 && k >= 8192) ? 12 : 2); }
 
 constexpr int kMaxGroupedTiles = 4096;   // (the list's entries hold 12 bits of tile and 19 of group)
 

@@ -18,6 +18,13 @@ def test_panels_of_tiles_cover_the_product(cuda, m, n, k):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k", [(6200, 3400, 3072), (4200, 3400, 8192)])
+def test_panels_by_the_length_of_the_rows(cuda, m, n, k):
+    """Panels of 12 from 24 m-tiles on, and from 16 on where rows are long, with a narrower last one."""
+    test_panels_of_tiles_cover_the_product(cuda, m, n, k)
+
+
+@pytest.mark.gpu
 def test_prompts_give_the_same_logits_where_projections_add_to_the_stream(cuda):
     """Together the prompts have more tiles than pairs, and their o / down projections add to the stream; either half of them, on the same
     kernels otherwise, goes through the separate add.  Both round in the same places."""
