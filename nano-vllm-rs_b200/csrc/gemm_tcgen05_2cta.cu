@@ -227,6 +227,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gri
       const int row0 = static_cast<int>(p & 0xfffu) * C::BM_CTA;
       return Where{row0 + static_cast<int>(rank) * C::BM_CTA, tile % num_m_tiles, row0 + (p & 0x1000u ? C::BM : C::BM_CTA), static_cast<int>(p >> 13) * group_rows};
     } else {
+      if (panel == 1) return Where{tile % num_m_tiles * C::BM + static_cast<int>(rank) * C::BM_CTA, tile / num_m_tiles, M, 0};
       const int p = tile / (panel * num_m_tiles), n0 = p * panel, in = tile - n0 * num_m_tiles, wide = min(panel, num_tiles / num_m_tiles - n0);
       return Where{in / wide * C::BM + static_cast<int>(rank) * C::BM_CTA, n0 + in % wide, M, 0};
     }

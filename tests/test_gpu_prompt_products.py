@@ -18,9 +18,9 @@ def test_panels_of_tiles_cover_the_product(cuda, m, n, k):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("m,n,k", [(6200, 3400, 3072), (4200, 3400, 8192)])
+@pytest.mark.parametrize("m,n,k", [(6200, 3400, 3072), (4200, 3400, 8192), (6200, 2056, 3072), (4200, 1032, 1024)])
 def test_panels_by_the_length_of_the_rows(cuda, m, n, k):
-    """Panels of 12 from 24 m-tiles on, and from 16 on where rows are long, with a narrower last one."""
+    """Panels of 12 from 24 m-tiles on, and from 16 on where rows are long, with a narrower last one; rows of the product that do not lie on 32 bytes; no panels."""
     test_panels_of_tiles_cover_the_product(cuda, m, n, k)
 
 
