@@ -970,8 +970,13 @@ int run_attention(const AttnArgs& a, size_t workspace_bytes, int dtype, int n_se
       if (int rc = latent_attn_tc_launch(a, st)) return rc;
       b.skip_dense = 1;   // tiles of many sequences are left to the kernel below
     }
-    // rank 512, up to 256 tokens (single tokens, or what the tcgen05 kernel leaves of prompts): a kernel of its own, each token by itself
-    if ((a.n <= 256 || knobs().latent_mma == 2) && latent_attn_decode_applies(a)) return latent_attn_decode_launch(b, st);
+    // rank 512, up to 256 tokens (single tokens, or what the tcgen05 kernel leaves of prompts): a kernel of its own, each token by itself.  Behind the tcgen05
+    // kernel most of its CTAs have nothing to do, and more than two an SM of them take longer to come and go than the half as many below (256 tokens of a
+    // prompt, 32 and 64 heads: 22.9 and 35.1 us both kernels with this one, 21.5 and 31.4 with the one below; 16 heads 21.0 so).
+    // The limit of 256 tokens is that of the splits below and no measured one: 300 single tokens at 64, 500 and 2000 keys would take 21, 62 and 178 us here, and
+    // take 49, 175 and 556 below.
+    const bool mostly_idle = b.skip_dense && static_cast<int64_t>(a.n) * ((a.heads + 15) / 16) > 2 * sm_count();
+    if ((a.n <= 256 || knobs().latent_mma == 2) && !mostly_idle && latent_attn_decode_applies(a)) return latent_attn_decode_launch(b, st);
     // Single tokens with a bounded key range (a window) and fewer CTAs than SMs: split every token's key tiles over up to 4
     // CTAs, as many as fill the SMs once and leave each at least eight tiles; the partials meet in latent_attn_merge_kernel.
     // (Measured, 64 tokens x 16 heads, rank 512 on this kernel: a window of 2048 keys 118 -> 79 us; at 512 keys the second launch costs what

@@ -228,3 +228,10 @@ def test_clusters_share_the_keys_of_single_tokens(cuda, heads, rank, rot, n, ext
             ref = ref * torch.sigmoid(gate[t].double())[:, None]
         err = out[t].double().reshape(heads, rank) - ref
         assert float(err.norm() / ref.norm()) < 6e-3, (t, ctx[t])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,window,extras", [(48, 0, False), (64, 50, True)])
+def test_what_is_left_of_prompts_with_many_heads(cuda, heads, window, extras):
+    """Up to 256 tokens whose few tiles of many sequences go to the mma.sync kernel behind the prompts: more than two CTAs an SM would have nothing to do elsewhere."""
+    test_latent_prompts_portions_and_single_tokens(cuda, heads, 64, 64, window, extras, [(40, 1), (0, 100), (700, 1), (5, 1), (9, 1), (2, 1), (1000, 30)])
