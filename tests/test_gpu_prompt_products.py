@@ -46,3 +46,11 @@ def test_prompts_give_the_same_logits_where_projections_add_to_the_stream(cuda):
             out.append(eng.model_runner.execute_model(batch, return_logits=True)[1])
         return np.concatenate(out)
     assert np.array_equal(logits([prompts]), logits([prompts[:5], prompts[5:]]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("width", [64, 128, 256])
+def test_projections_add_to_the_stream_at_every_tile_width(cuda, width, monkeypatch):
+    """The 4900 tokens above take tiles 128 wide by themselves, large prompts 256."""
+    monkeypatch.setenv("NVLLM_GEMM_BN", str(width))
+    test_prompts_give_the_same_logits_where_projections_add_to_the_stream(cuda)
