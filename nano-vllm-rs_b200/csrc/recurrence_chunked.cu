@@ -21,8 +21,10 @@
 // global memory straight into the layout that serves as A (v^T of the update) and as B (of the middle product).  q and k of the
 // next chunk fly (cp.async) under the products of this one.  Bound by mma.sync issue (about 540 of them per warp and chunk) and the conversions
 // around it; two CTAs an SM (91 KB each) hide each other's barriers.
-// Token by token and here (us): 16 heads of 128 x 128, 8 x 1024 tokens 548 and 274, 500 tokens 210 and 111; 64 heads of 128 x 64, 8 x 1024
-// 875 and 559, 2 x 40 30 and 24.
+// Token by token and here (us, back to back on one GPU): 16 heads of 128 x 128, 8 x 1024 tokens 542 and 270, 500 tokens 205 and 100; 64 heads of 128 x 64,
+// 8 x 1024 868 and 531, 2 x 40 25 and 17.
+#include <type_traits>
+
 #include "split_mma.cuh"
 
 namespace nvllm {
@@ -41,6 +43,7 @@ constexpr int kSmP = kSmK + 3 * kPiece;          // D_ij, overwritten in place b
 constexpr int kSmVec = kSmP + kC * kPs * 4;      // floats: pre, w [32 each], a [2][32], b [2][32], second part of w [32], flag, that of the product of all decays
 constexpr int kSmBytes = kSmVec + 7 * kC * 4 + 16;
 
+template <bool TOGETHER>
 __global__ void __launch_bounds__(kWarps * 32, 2) linear_recurrence_chunked_kernel(const RecArgs a) {
   pdl_wait();
   pdl_launch_dependents();
@@ -200,6 +203,77 @@ __global__ void __launch_bounds__(kWarps * 32, 2) linear_recurrence_chunked_kern
     const bool slow = *flag != 0u;
     if (tb + kC < t1) issue(tb + kC, buf ^ 1);
     const uint32_t q_addr = sbase + kSmQ + (lane & 15) * kRow + (lane >> 4) * 16;
+    // ---- middle factor (q_i . k_j) D_ij b_j (+ d on the diagonal): warp w computes tokens 16 (w / 2) .. + 15, keys 16 (w % 2) .. + 15 (warp 1's keys lie
+    // behind all of its tokens: it keeps nothing); and S^T q of the chunk's start.  Each alone is a chain of dependent products, the first of two at a time.
+    // TOGETHER, step by step beside each other, 8 x 1024 tokens take 270 and 531 us (16 and 64 heads, see above), and one after the other, the first left out by
+    // warp 1, 292 and 576.  With one CTA an SM at the most it is the longest warp that counts, and one after the other is shorter: 500 tokens, 16 heads,
+    // 102.1 us together and 99.9 so, 4 x 300 72.7 and 72.2.
+    const int mt = warp >> 1, nt = warp & 1;
+    // B of 16 keys x 16 dims: lanes 0-7 keys 0-7 dims 0-7, 8-15 the same keys dims 8-15, 16-31 keys 8-15
+    const uint32_t mk_addr = sbase + kSmK + (nt * 16 + (lane & 7) + (lane >> 4) * 8) * kRow + ((lane >> 3) & 1) * 16;
+    float yi[2][2][4] = {};           // S^T q: [16 tokens][8 columns]
+    auto products = [&](auto which) {   // 1: the middle factor, 2: S^T q, 3: both
+      constexpr bool kMiddle = (decltype(which)::value & 1) != 0, kState = (decltype(which)::value & 2) != 0;
+      float sum[2][4] = {}, ah[1][2][4], al[2][1][2][4] = {};   // (al: even and odd steps)
+      float yl[2][2][4] = {}, hh[2][2][4];
+#pragma unroll
+      for (int kk = 0; kk < kDk / 16; ++kk) {
+        uint32_t qm[1][3][4], kf[3][2][2], qf[2][3][4], sf[3][2][2];          // sf: [piece][8 columns][half of the 16 keys]
+        if (kk % 2 == 0) { zero(ah); zero(hh); }
+        if constexpr (kMiddle) {
+#pragma unroll
+          for (int j = 0; j < 3; ++j) {
+            ldmatrix_x4(qm[0][j], q_addr + mt * 16 * kRow + kk * 32 + j * kPiece);
+            ldmatrix_x4(reinterpret_cast<uint32_t(&)[4]>(kf[j]), mk_addr + kk * 32 + j * kPiece);
+          }
+        }
+        if constexpr (kState) {
+#pragma unroll
+          for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) split3(S[2 * kk + e][2 * n], S[2 * kk + e][2 * n + 1], sf[0][n][e], sf[1][n][e], sf[2][n][e]);
+#pragma unroll
+          for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) ldmatrix_x4(qf[m][j], q_addr + m * 16 * kRow + kk * 32 + j * kPiece);
+        }
+        if constexpr (kMiddle) mma6<1, 2>(ah, al[kk & 1], qm, kf);
+        if constexpr (kState) mma6<2, 2>(hh, yl, qf, sf);
+        if (kk % 2 == 1) {
+#pragma unroll
+          for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              if constexpr (kMiddle) sum[n][i] += ah[0][n][i];
+              if constexpr (kState) {
+                yi[0][n][i] += hh[0][n][i];
+                yi[1][n][i] += hh[1][n][i];
+              }
+            }
+        }
+      }
+      if constexpr (kMiddle) {
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int row = mt * 16 + r + (i >> 1) * 8, key = nt * 16 + n * 8 + c2 + (i & 1);
+            float* m = mid + row * kPs + key;
+            if (warp != 1) *m = fmaf(join(sum[n][i], al[0][0][n][i] + al[1][0][n][i]) * bs[key], *m, row == key ? d : 0.f);      // D is zero above the diagonal
+          }
+      }
+      if constexpr (kState) {
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+          for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) yi[m][n][i] = join(yi[m][n][i], yl[m][n][i]);
+      }
+    };
+    if constexpr (!TOGETHER) {
+      if (!slow && warp != 1) products(std::integral_constant<int, 1>{});
+    }
     // v and the state: their largest magnitude decides whether the warp takes the products
     float vmax = 0.f;
 #pragma unroll
@@ -213,60 +287,10 @@ __global__ void __launch_bounds__(kWarps * 32, 2) linear_recurrence_chunked_kern
       smax[1] = abs_max(S[n][2], S[n][3], smax[1]);
     }
     const bool step = __any_sync(0xffffffffu, slow || !(smax[0] < 1.2e24f && smax[1] < 1.2e24f));      // 2^80
-    // ---- middle factor (q_i . k_j) D_ij b_j (+ d on the diagonal): warp w computes tokens 16 (w / 2) .. + 15, keys 16 (w % 2) .. + 15 (warp 1's keys lie
-    // behind all of its tokens: it keeps nothing); and S^T q of the chunk's start.  Each alone is a chain of dependent products, the first of two at a time:
-    // one after the other, with the first left out by warp 1, 8 x 1024 tokens take 293 and 592 us instead of 274 and 559 (16 and 64 heads, see above).
-    float yi[2][2][4] = {};           // S^T q: [16 tokens][8 columns]
-    if (!slow) {                      // (also where this warp steps: the middle factor is for all)
-      const int mt = warp >> 1, nt = warp & 1;
-      float sum[2][4] = {}, ah[1][2][4], al[2][1][2][4] = {};   // (al: even and odd steps)
-      float yl[2][2][4] = {}, hh[2][2][4];
-      // B of 16 keys x 16 dims: lanes 0-7 keys 0-7 dims 0-7, 8-15 the same keys dims 8-15, 16-31 keys 8-15
-      const uint32_t k_addr = sbase + kSmK + (nt * 16 + (lane & 7) + (lane >> 4) * 8) * kRow + ((lane >> 3) & 1) * 16;
-#pragma unroll
-      for (int kk = 0; kk < kDk / 16; ++kk) {
-        uint32_t qm[1][3][4], kf[3][2][2], qf[2][3][4], sf[3][2][2];          // sf: [piece][8 columns][half of the 16 keys]
-        if (kk % 2 == 0) { zero(ah); zero(hh); }
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          ldmatrix_x4(qm[0][j], q_addr + mt * 16 * kRow + kk * 32 + j * kPiece);
-          ldmatrix_x4(reinterpret_cast<uint32_t(&)[4]>(kf[j]), k_addr + kk * 32 + j * kPiece);
-        }
-#pragma unroll
-        for (int n = 0; n < 2; ++n)
-#pragma unroll
-          for (int e = 0; e < 2; ++e) split3(S[2 * kk + e][2 * n], S[2 * kk + e][2 * n + 1], sf[0][n][e], sf[1][n][e], sf[2][n][e]);
-#pragma unroll
-        for (int m = 0; m < 2; ++m)
-#pragma unroll
-          for (int j = 0; j < 3; ++j) ldmatrix_x4(qf[m][j], q_addr + m * 16 * kRow + kk * 32 + j * kPiece);
-        mma6<1, 2>(ah, al[kk & 1], qm, kf);
-        mma6<2, 2>(hh, yl, qf, sf);
-        if (kk % 2 == 1) {
-#pragma unroll
-          for (int n = 0; n < 2; ++n)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              sum[n][i] += ah[0][n][i];
-              yi[0][n][i] += hh[0][n][i];
-              yi[1][n][i] += hh[1][n][i];
-            }
-        }
-      }
-#pragma unroll
-      for (int n = 0; n < 2; ++n)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int row = mt * 16 + r + (i >> 1) * 8, key = nt * 16 + n * 8 + c2 + (i & 1);
-          float* m = mid + row * kPs + key;
-          if (warp != 1) *m = fmaf(join(sum[n][i], al[0][0][n][i] + al[1][0][n][i]) * bs[key], *m, row == key ? d : 0.f);      // D is zero above the diagonal
-        }
-#pragma unroll
-      for (int m = 0; m < 2; ++m)
-#pragma unroll
-        for (int n = 0; n < 2; ++n)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) yi[m][n][i] = join(yi[m][n][i], yl[m][n][i]);
+    if constexpr (TOGETHER) {
+      if (!slow) products(std::integral_constant<int, 3>{});   // (also where this warp steps: the middle factor is for all)
+    } else {
+      if (!step) products(std::integral_constant<int, 2>{});
     }
     uint32_t vf[2][3][2][2];           // v as B: [token step][piece][8 columns][half of the 16 tokens]
 #pragma unroll
@@ -397,18 +421,22 @@ __global__ void __launch_bounds__(kWarps * 32, 2) linear_recurrence_chunked_kern
 
 }  // namespace
 
+// a CTA an SM at the most
+static bool at_once(const RecArgs& a, int n_seqs) { return static_cast<int64_t>(a.heads) * n_seqs * (a.dv / kCols) <= sm_count(); }
+
 // From 40 tokens a sequence on; from 16 on where all CTAs run at once and the steps' latency is what counts.  (32 x 33 tokens, two chunks
 // each: 16 heads of 128 columns 78 us here, 77 token by token; 32 x 16 tokens, 64 heads of 64: 85 and 83; 2 x 40 tokens 21 and 30.)  One decoded
 // token costs a chunk, 10 times a step.
 bool linear_recurrence_chunked_applies(const RecArgs& a, int n_seqs, int n_tokens) {
-  const bool at_once = static_cast<int64_t>(a.heads) * n_seqs * (a.dv / kCols) <= sm_count();
-  return a.dk == kDk && a.dv % kCols == 0 && static_cast<int64_t>(n_tokens) >= (at_once ? 16 : 40) * static_cast<int64_t>(n_seqs) && n_seqs <= 65535 &&
+  return a.dk == kDk && a.dv % kCols == 0 && static_cast<int64_t>(n_tokens) >= (at_once(a, n_seqs) ? 16 : 40) * static_cast<int64_t>(n_seqs) && n_seqs <= 65535 &&
          a.ldq % 4 == 0 && a.ldk % 4 == 0 && a.ldy % 2 == 0 && aligned16(a.q) && aligned16(a.k) && aligned16(a.y);
 }
 
 int linear_recurrence_chunked(const RecArgs& a, int n_seqs, cudaStream_t st) {
-  NVLLM_SMEM_ATTR_ONCE(linear_recurrence_chunked_kernel, kSmBytes);
-  NVLLM_CUDA(launch_plain(linear_recurrence_chunked_kernel, dim3(a.heads, n_seqs, a.dv / kCols), dim3(kWarps * 32), kSmBytes, st, a));
+  NVLLM_SMEM_ATTR_ONCE(linear_recurrence_chunked_kernel<true>, kSmBytes);
+  NVLLM_SMEM_ATTR_ONCE(linear_recurrence_chunked_kernel<false>, kSmBytes);
+  const auto kern = at_once(a, n_seqs) ? linear_recurrence_chunked_kernel<false> : linear_recurrence_chunked_kernel<true>;   // (see the kernel)
+  NVLLM_CUDA(launch_plain(kern, dim3(a.heads, n_seqs, a.dv / kCols), dim3(kWarps * 32), kSmBytes, st, a));
   NVLLM_LAUNCH_CHECK("linear_recurrence_chunked_kernel");
   return 0;
 }

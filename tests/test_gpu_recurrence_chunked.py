@@ -345,3 +345,22 @@ def test_error_against_float64_is_no_larger(cuda, errors, kind):
     rms = lambda i, j: float(np.sqrt(np.mean([r[i][j] ** 2 for r in rows])))
     for j, what in enumerate(("y", "state")):
         assert rms(0, j) <= SLACK * rms(1, j), f"{what}: {rms(0, j):.3e} in chunks, {rms(1, j):.3e} token by token"
+
+
+@pytest.mark.parametrize("odd", [None, "v", "k"])
+def test_a_sequence_alone_is_one_of_many_to_the_bit(cuda, odd):
+    """With more CTAs than SMs the middle factor's products run beside those with the state, with fewer after one another: the same sums."""
+    heads, dv, lens = 16, 128, [97, 130, 41, 64, 33, 95, 32, 200]
+    assert len(lens) * heads * dv // 64 > torch.cuda.get_device_properties(0).multi_processor_count > heads * dv // 64 and sum(lens) >= 40 * len(lens)
+    rng = np.random.default_rng(11)
+    seqs = [_seq(rng, n, heads, heads, dv) for n in lens]
+    if odd is not None:   # a warp, or all of them, steps through a chunk
+        seqs[1][odd][50, 3, 7] = 1e30
+    skip = np.asarray(rng.standard_normal(heads), np.float32)
+    first = torch.randn(len(lens), heads, DK, dv, generator=torch.Generator().manual_seed(1)).to(cuda)
+    state = first.clone()
+    ys = _run(cuda, seqs, heads, heads, dv, state, [9] * len(lens), True, skip)
+    for i, s in enumerate(seqs):
+        alone = first[i:i + 1].clone()
+        y = _run(cuda, [s], heads, heads, dv, alone, [9], True, skip)[0]
+        assert np.array_equal(y, ys[i], equal_nan=True) and torch.equal(alone[0].view(torch.int32), state[i].view(torch.int32))
