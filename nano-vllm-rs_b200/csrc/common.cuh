@@ -54,7 +54,7 @@ int paged_decode_launches(int batch, int heads, int kv_heads, int splits, bool f
 // nvllm_paged_decode_attention_fused inside a step of the runner (paged_decode.cu).  The runner's chain of programmatic launches begins behind
 // a copy or the start of a graph, which waits for everything before it, and inside the chain nothing else writes block tables, lengths,
 // positions, or keys and values: the kernel reads those of earlier tokens before it waits for its predecessor.  A decode step of Qwen3-0.6B
-// (28 layers) of 1 token at 300 keys 850 -> 809 us, 16 at 300 1137 -> 1090, 8 at 4000 1394 -> 1345.  (The coming kernels' weights
+// (28 layers), kernel by kernel, of 1 token at 300 keys 764 -> 740 us, 4 at 300 866 -> 807, 16 at 300 1144 -> 1111, 8 at 4000 1380 -> 1361.  (The coming kernels' weights
 // asked into L2 from here as well take 2 us off their 18 a layer, but 24 CTAs request them for 12 us longer than the attention takes.)
 int paged_decode_fused_in_step(void* out, const void* qkv, const int64_t* positions, const float* cos_sin, const void* q_norm_w, const void* k_norm_w, float eps,
                                int32_t max_position, void* k_cache, void* v_cache, const int32_t* slot_mapping, const int32_t* block_tables,

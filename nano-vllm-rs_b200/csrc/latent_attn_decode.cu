@@ -13,8 +13,8 @@
 // Rows behind the last key repeat that key: what the unused columns of a tile multiply by zero is no other token's row.
 // Measured, 16 heads, back to back, before (one 64-key tile ahead, three barriers a tile) and so: 32 tokens at 4001 keys (147 MB, 23 us at the
 // copy rate) 66.3 and 38.3 us; with a launch's overhead in both, 1 at 4001 41 and 29, 150 at 500 72 and 45, 64 with a window of 512 41 and 20,
-// 40 at 33 14 and 14.  Of the 38 us the copies take 26 (5.6 TB/s on 128 SMs), the products alone 21; the first queries, tables and keys and
-// the merge take the rest.  Copied by cp.async.bulk, a row each lane, a tile takes as long (1.1 us on an SM).
+// 40 at 33 14 and 14.  Of the 38 us 33 are there without any product (queries, tables, the copies on 128 SMs, the merge).
+// Copied by cp.async.bulk, a row each lane, a tile takes as long (1.1 us on an SM).
 #include <algorithm>
 
 #include "latent_attn.cuh"
